@@ -640,12 +640,13 @@ def prefill_leg(D, B, torch, dev, dims, layers, fmt_main, fmt_alt, seed, n, tpea
             counted[0] += 1 if r == 0 else 0   # a refusal (the caller then splits the tokens) launched nothing
             return r
         return wrapped
-    LIB.call, LIB.status = counting(real_call), counting(real_status)   # every kernel launch goes through one of the two
+    LIB.call, LIB.status = counting(real_call), counting(real_status)   # a launch goes through one of the two,
+    native = LIB.hostops().launches()                                   # or is made by the native operators
     try:
         chunk()
     finally:
         LIB.call, LIB.status = real_call, real_status
-    launches[0] = counted[0] + 1   # + the copy of the hidden states
+    launches[0] = counted[0] + LIB.hostops().launches() - native + 1   # + the copy of the hidden states
     torch.cuda.synchronize()
     finite = bool(torch.isfinite(m["logits"]).all()) and bool(torch.isfinite(h).all())
     # parity, outside the timed region: the chunk product of the first layer's gate matrix against the one-token

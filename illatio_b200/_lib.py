@@ -6,6 +6,8 @@ is raised.
 import ctypes
 import os
 
+import torch
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libillatio_b200.so")
 
@@ -43,6 +45,7 @@ SIGNATURES = {
     "ill_mv_glu": (_I, [_I, _P, _P, _I, _I, _P, _P, _P, _P, _S]),
     "ill_moe_mv": (_I, [_I, _I, _I, _L, _P, _I, _P, _P, _P, _I, _P, _L, _S]),
     "ill_moe_glu": (_I, [_I, _I, _I, _L, _L, _P, _I, _P, _P, _P, _I, _F, _P, _P, _L, _S]),
+    "ill_silu_mul": (_I, [_L, _P, _P, _P, _S]),
     "ill_swiglu_w": (_I, [_L, _I, _F, _P, _P, _P, _P, _S]),
     "ill_moe_sum": (_I, [_I, _I, _L, _P, _P, _P, _P, _S]),
     "ill_swiglu_q8k_f16": (_I, [_L, _I, _F, _P, _P, _P, _P, _P, _P, _P, _S]),
@@ -118,15 +121,49 @@ def register(name, res, args):
         f.argtypes = args
 
 
+def fail(name, rc):
+    """Raise what status RC of entry point NAME stands for."""
+    L = lib()
+    raise IllatioError(name, rc, L.ill_error_string(rc).decode(), L.ill_last_cuda_error() if rc == 4 else 0)
+
+
 def call(name, *args):
     """Call entry point NAME; a non-zero status becomes an IllatioError."""
-    L = lib()
-    rc = getattr(L, name)(*args)
+    rc = getattr(lib(), name)(*args)
     if rc != 0:
-        raise IllatioError(name, rc, L.ill_error_string(rc).decode(), L.ill_last_cuda_error() if rc == 4 else 0)
+        fail(name, rc)
     return rc
 
 
 def status(name, *args):
     """Call entry point NAME and return its status code without raising."""
     return getattr(lib(), name)(*args)
+
+
+class _NotBuilt:
+    """Stands for the native operators where they have not been built: importing the package works, using them does not."""
+
+    def set_slow(self, fns):
+        pass
+
+    def __getattr__(self, name):
+        def missing(*args, **kw):
+            raise RuntimeError("illatio_b200._hostops is not built (run `python -m illatio_b200.build`); there is no fallback path")
+        return missing
+
+
+def hostops():
+    """The native operators of a decoded token (csrc/hostops.cpp)."""
+    try:
+        from . import _hostops
+    except ImportError:
+        if os.path.exists(os.path.join(HERE, "_hostops.so")):
+            raise
+        return _NotBuilt()
+    return _hostops
+
+
+def stream():
+    """The current stream of the current device, as an integer (a third of a microsecond; torch.cuda.current_stream()
+    builds an object in three)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())

@@ -1,0 +1,301 @@
+// hostops.cpp -- the operators of a decoded token as a CPython extension module (illatio_b200._hostops).
+//
+// A decode step is a few hundred launches of one to ten microseconds, so what the host spends on one decides the
+// token: through ctypes an operator cost 9.4 us (3.2 of them torch.cuda.current_stream(), 0.8 the conversion of
+// the arguments, the rest attribute look-ups and the launch itself at 2.4), here it costs 3 (a B200 box's Xeon,
+// D.cmat_mul of 896 x 896).  The functions have the signatures and the behaviour that cuda_dense.py and
+// cuda_ds4f.py document; they read the same objects (CMat, QAct, ExpertPool) and call the same C ABI.  What is
+// rare or long -- prefill chunks, activations whose fp16 form is in use, errors -- goes to the Python functions
+// registered with set_slow().
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/illatio_b200.h"
+
+namespace {
+
+PyObject* g_slow = nullptr;   // name -> Python function
+long long g_launches = 0;     // launches made from this module (the GIL is held): what bench.py counts
+
+// attribute names, interned once
+#define NAMES(X) \
+  X(type) X(rows) X(cols) X(qs) X(kind) X(xq) X(xs) X(xsum) X(_cf) X(w) X(act) X(y) X(n) X(bias) X(acc) X(x) X(f16_scale) X(d) X(eps) \
+  X(h) X(wq) X(wk) X(wv) X(q) X(k) X(v) X(bq) X(bk) X(bv) X(g) X(u) X(fa) X(fb) X(emb) X(tokens) X(quant_q8) X(rmsnorm_q8) \
+  X(cmat_mul) X(glu_mul) X(qkv_mul) X(error)
+#define DECL(s) PyObject* S_##s;
+NAMES(DECL)
+#undef DECL
+
+struct Failed {};  // a Python error is set
+
+inline ill_stream cur_stream() { return (ill_stream)c10::cuda::getCurrentCUDAStream().stream(); }
+
+inline bool capturing() {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing((cudaStream_t)cur_stream(), &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
+}
+
+// the address of a tensor's data (None: 0)
+inline ill_dptr ptr(PyObject* o) {
+  if (o == Py_None) return 0;
+  if (!THPVariable_Check(o)) {
+    PyErr_Format(PyExc_TypeError, "expected a tensor or None, got %s", Py_TYPE(o)->tp_name);
+    throw Failed();
+  }
+  return (ill_dptr)(uintptr_t)THPVariable_Unpack(o).data_ptr();
+}
+inline const at::Tensor& tensor(PyObject* o) {
+  if (!THPVariable_Check(o)) {
+    PyErr_Format(PyExc_TypeError, "expected a tensor, got %s", Py_TYPE(o)->tp_name);
+    throw Failed();
+  }
+  return THPVariable_Unpack(o);
+}
+
+struct Ref {  // an owned reference
+  PyObject* p;
+  explicit Ref(PyObject* o) : p(o) { if (!o) throw Failed(); }
+  ~Ref() { Py_XDECREF(p); }
+  Ref(const Ref&) = delete;
+  Ref& operator=(const Ref&) = delete;
+};
+inline long long as_int(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw Failed();
+  return v;
+}
+inline double as_float(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw Failed();
+  return v;
+}
+inline int as_bool(PyObject* o) {
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw Failed();
+  return v;
+}
+inline long long attr_int(PyObject* o, PyObject* name) { Ref r(PyObject_GetAttr(o, name)); return as_int(r.p); }
+inline ill_dptr attr_ptr(PyObject* o, PyObject* name) { Ref r(PyObject_GetAttr(o, name)); return ptr(r.p); }
+
+// a CMat
+struct Mat {
+  int type, rows, cols;
+  ill_dptr w;
+  explicit Mat(PyObject* o)
+      : type((int)attr_int(o, S_type)), rows((int)attr_int(o, S_rows)), cols((int)attr_int(o, S_cols)), w(attr_ptr(o, S_qs)) {}
+};
+// a QAct
+struct Act {
+  bool k;         // Q8_K super-blocks
+  bool has_f16;   // its fp16 form is in use
+  ill_dptr xq, xs, xsum;
+  explicit Act(PyObject* o) : xq(attr_ptr(o, S_xq)), xs(attr_ptr(o, S_xs)), xsum(attr_ptr(o, S_xsum)) {
+    Ref kind(PyObject_GetAttr(o, S_kind));
+    k = !(PyUnicode_Check(kind.p) && PyUnicode_GetLength(kind.p) == 2);
+    Ref cf(PyObject_GetAttr(o, S__cf));
+    has_f16 = cf.p != Py_None;
+  }
+};
+
+PyObject* slow(PyObject* name) {
+  PyObject* f = g_slow ? PyDict_GetItemWithError(g_slow, name) : nullptr;
+  if (!f && !PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "illatio_b200._hostops: set_slow() has not been called");
+  if (!f) throw Failed();
+  return f;
+}
+[[noreturn]] void raise_status(const char* fn, int rc) {
+  PyObject* r = PyObject_CallFunction(slow(S_error), "si", fn, rc);
+  Py_XDECREF(r);
+  if (r) PyErr_Format(PyExc_RuntimeError, "%s failed with status %d", fn, rc);
+  throw Failed();
+}
+inline void check(const char* fn, int rc) {
+  if (rc) raise_status(fn, rc);
+  ++g_launches;
+}
+
+// positional and keyword arguments into OUT (absent: null); the first REQUIRED must be there
+void parse(const char* fn, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames, PyObject* const* names, int n, int required,
+           PyObject** out) {
+  if (nargs > n) {
+    PyErr_Format(PyExc_TypeError, "%s() takes at most %d arguments (%zd given)", fn, n, nargs);
+    throw Failed();
+  }
+  for (int i = 0; i < n; ++i) out[i] = i < nargs ? args[i] : nullptr;
+  const Py_ssize_t nk = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
+  for (Py_ssize_t j = 0; j < nk; ++j) {
+    PyObject* key = PyTuple_GET_ITEM(kwnames, j);
+    int at = -1;
+    for (int i = 0; i < n && at < 0; ++i)
+      if (key == names[i]) at = i;
+    for (int i = 0; i < n && at < 0; ++i)  // a key that is not the interned string
+      if (PyUnicode_Compare(key, names[i]) == 0) at = i;
+    if (at < 0 || out[at]) {
+      PyErr_Format(PyExc_TypeError, "%s(): %s argument '%U'", fn, at < 0 ? "unexpected" : "repeated", key);
+      throw Failed();
+    }
+    out[at] = args[nargs + j];
+  }
+  for (int i = 0; i < required; ++i)
+    if (!out[i]) {
+      PyErr_Format(PyExc_TypeError, "%s(): missing argument '%U'", fn, names[i]);
+      throw Failed();
+    }
+}
+#define ARGS(FN, REQUIRED, ...)                                        \
+  PyObject* const names_[] = {__VA_ARGS__};                            \
+  constexpr int n_ = (int)(sizeof(names_) / sizeof(names_[0]));        \
+  PyObject* a[n_];                                                     \
+  parse(FN, args, nargs, kwnames, names_, n_, REQUIRED, a)
+#define OPT_INT(o, dflt) ((o) ? as_int(o) : (dflt))
+#define OPT_BOOL(o, dflt) ((o) ? as_bool(o) : (dflt))
+#define OPT_PTR(o) ((o) ? ptr(o) : 0)
+
+inline PyObject* ret(PyObject* o) { Py_INCREF(o); return o; }
+
+// ---- the operators ------------------------------------------------------------------
+
+PyObject* quant_q8(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
+  ARGS("quant_q8", 2, S_x, S_act, S_f16_scale);
+  const Act act(a[1]);
+  if (act.has_f16) return PyObject_Vectorcall(slow(S_quant_q8), args, nargs, kwnames);
+  const at::Tensor& x = tensor(a[0]);
+  const ill_dptr xp = (ill_dptr)(uintptr_t)x.data_ptr();
+  if (act.k) check("ill_quant_q8_k", ill_quant_q8_k(xp, act.xq, act.xs, act.xsum, x.numel() / 256, cur_stream()));
+  else check("ill_quant_q8_0", ill_quant_q8_0(xp, act.xq, act.xs, act.xsum, x.numel() / 32, OPT_BOOL(a[2], 1), cur_stream()));
+  return ret(a[1]);
+} catch (const Failed&) { return nullptr; }
+
+PyObject* rmsnorm_q8(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
+  ARGS("rmsnorm_q8", 5, S_x, S_w, S_act, S_d, S_eps, S_n, S_h, S_f16_scale);
+  const Act act(a[2]);
+  if (act.has_f16) return PyObject_Vectorcall(slow(S_rmsnorm_q8), args, nargs, kwnames);
+  check("ill_rmsnorm_q8", ill_rmsnorm_q8(act.k ? 1 : 0, ptr(a[0]), ptr(a[1]), OPT_PTR(a[6]), act.xq, act.xs, act.xsum, (int)as_int(a[3]),
+                                         (float)as_float(a[4]), OPT_INT(a[5], 1), OPT_BOOL(a[7], 1), cur_stream()));
+  return ret(a[2]);
+} catch (const Failed&) { return nullptr; }
+
+// Y = W X for up to 16 tokens in one launch; false when the shape wants the tokens split (the Python form does that)
+inline bool mul(const Mat& w, const Act& act, ill_dptr y, int n, ill_dptr bias, int acc) {
+  const int rc = ill_mv(w.type, w.w, w.rows, w.cols, act.xq, act.xs, act.k ? act.xsum : 0, y, bias, acc, n, cur_stream());
+  if (rc == ILL_ERR_UNSUPPORTED && n > 1) return false;
+  check("ill_mv", rc);
+  return true;
+}
+constexpr long long FEW = 16;  // more tokens are a chunk: the Python form picks the kernel
+
+PyObject* cmat_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
+  ARGS("cmat_mul", 3, S_w, S_act, S_y, S_n, S_bias, S_acc);
+  const long long n = OPT_INT(a[3], 1);
+  if (n < 1 || n > FEW || !mul(Mat(a[0]), Act(a[1]), ptr(a[2]), (int)n, OPT_PTR(a[4]), OPT_BOOL(a[5], 0)))
+    return PyObject_Vectorcall(slow(S_cmat_mul), args, nargs, kwnames);
+  return ret(a[2]);
+} catch (const Failed&) { return nullptr; }
+
+void mul_any(PyObject* w, PyObject* act, PyObject* y, long long n, PyObject* bias) {
+  if (n >= 1 && n <= FEW && mul(Mat(w), Act(act), ptr(y), (int)n, bias ? ptr(bias) : 0, 0)) return;
+  PyObject* nn = PyLong_FromLongLong(n);
+  Ref hold(nn);
+  PyObject* av[5] = {w, act, y, nn, bias ? bias : Py_None};
+  Ref r(PyObject_Vectorcall(slow(S_cmat_mul), av, 5, nullptr));
+}
+
+PyObject* qkv_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
+  ARGS("qkv_mul", 7, S_wq, S_wk, S_wv, S_act, S_q, S_k, S_v, S_bq, S_bk, S_bv, S_n);
+  const long long n = OPT_INT(a[10], 1);
+  if (n == 1) {
+    const Mat q(a[0]), k(a[1]), v(a[2]);
+    if (q.type == k.type) {
+      const Act x(a[3]);
+      const bool three = k.type == v.type;
+      // Q4_K_M files keep V in Q6_K: V in a launch of its own.  In a stream that is being captured the Python form runs
+      // it beside Q and K (a fork and a join cost a graph nothing: a 4B token 1.54 ms, 1.57 one after the other); launch
+      // by launch, the two events and four calls of a fork cost the host more than the overlap gives.
+      if (!three && capturing()) return PyObject_Vectorcall(slow(S_qkv_mul), args, nargs, kwnames);
+      check("ill_mv_3", ill_mv_3(q.type, q.w, k.w, three ? v.w : 0, q.rows, k.rows, three ? v.rows : 0, q.cols, x.xq, x.xs,
+                                 x.k ? x.xsum : 0, ptr(a[4]), ptr(a[5]), three ? ptr(a[6]) : 0, OPT_PTR(a[7]), OPT_PTR(a[8]),
+                                 three ? OPT_PTR(a[9]) : 0, cur_stream()));
+      if (!three) mul(v, x, ptr(a[6]), 1, OPT_PTR(a[9]), 0);
+      Py_RETURN_NONE;
+    }
+  }
+  for (int i = 0; i < 3; ++i) mul_any(a[i], a[3], a[4 + i], n, a[7 + i]);
+  Py_RETURN_NONE;
+} catch (const Failed&) { return nullptr; }
+
+PyObject* glu_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
+  ARGS("glu_mul", 4, S_g, S_u, S_act, S_fa, S_n, S_fb);
+  const long long n = OPT_INT(a[4], 1);
+  if (n == 1) {
+    const Mat g(a[0]), u(a[1]);
+    if (g.type == u.type) {
+      const Act x(a[2]);
+      check("ill_mv_glu", ill_mv_glu(g.type, g.w, u.w, g.rows, g.cols, x.xq, x.xs, x.k ? x.xsum : 0, ptr(a[3]), cur_stream()));
+      return ret(a[3]);
+    }
+  }
+  if (n >= 1 && a[5] && a[5] != Py_None) {
+    mul_any(a[0], a[2], a[3], n, nullptr);
+    mul_any(a[1], a[2], a[5], n, nullptr);
+    const at::Tensor& fa = tensor(a[3]);
+    const ill_dptr fp = (ill_dptr)(uintptr_t)fa.data_ptr();
+    check("ill_silu_mul", ill_silu_mul(fa.numel(), fp, ptr(a[5]), fp, cur_stream()));
+    return ret(a[3]);
+  }
+  return PyObject_Vectorcall(slow(S_glu_mul), args, nargs, kwnames);
+} catch (const Failed&) { return nullptr; }
+
+PyObject* embed(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
+  ARGS("embed", 3, S_emb, S_tokens, S_x);
+  const Mat m(a[0]);
+  const at::Tensor& t = tensor(a[1]);
+  check("ill_dequant_rows", ill_dequant_rows(m.type, m.w, m.cols, (ill_dptr)(uintptr_t)t.data_ptr(), 0, (int)t.numel(), ptr(a[2]), cur_stream()));
+  return ret(a[2]);
+} catch (const Failed&) { return nullptr; }
+
+PyObject* stream(PyObject*, PyObject*) { return PyLong_FromVoidPtr(cur_stream()); }
+PyObject* launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches); }
+
+PyObject* set_slow(PyObject*, PyObject* d) {
+  if (!PyDict_Check(d)) { PyErr_SetString(PyExc_TypeError, "set_slow() takes a dict"); return nullptr; }
+  Py_INCREF(d);
+  Py_XSETREF(g_slow, d);
+  Py_RETURN_NONE;
+}
+
+#define FAST(name, text) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL | METH_KEYWORDS, text}
+PyMethodDef methods[] = {
+    FAST(quant_q8,
+         "quant_q8(x, act, f16_scale=True)\n--\n\nX (float32, a whole number of blocks) quantized into ACT: the reference's quant_q8 launch\n"
+         "(src/cuda-dense.lisp:366,417), in the kind ACT holds."),
+    FAST(rmsnorm_q8,
+         "rmsnorm_q8(x, w, act, d, eps, n=1, h=None, f16_scale=True)\n--\n\nRMSNORM-Q8 (src/cuda-dense.lisp:260-264): RMSNORM! of N rows of X\n"
+         "(D wide) by W, quantized into ACT in the kind it holds; H, when given, also gets the floats."),
+    FAST(cmat_mul,
+         "cmat_mul(w, act, y, n=1, bias=None, acc=False)\n--\n\nCMAT-MUL (src/cuda-dense.lisp:220-248): Y = W X for N tokens (token t's X at\n"
+         "t*cols, its Y at t*rows), or Y += it when ACC."),
+    FAST(qkv_mul,
+         "qkv_mul(wq, wk, wv, act, q, k, v, bq=None, bk=None, bv=None, n=1)\n--\n\nQKV-MUL (src/cuda-dense.lisp:309-324): for one token one\n"
+         "launch when the three formats agree, two when those of Q and K do; else three products."),
+    FAST(glu_mul,
+         "glu_mul(g, u, act, fa, n=1, fb=None)\n--\n\nGLU-MUL (src/cuda-dense.lisp:326-339): silu(G x) * (U x) into FA."),
+    FAST(embed,
+         "embed(emb, tokens, x)\n--\n\nEMBED (src/cuda-dense.lisp:302-307): rows TOKENS (int32 on the device) of EMB as floats in X."),
+    {"stream", stream, METH_NOARGS, "The current stream of the current device, as an integer."},
+    {"launches", launches, METH_NOARGS, "Launches made by this module since it was loaded."},
+    {"set_slow", set_slow, METH_O, "Python functions for what this module leaves to Python: {name: function}."},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_hostops", "Native host side of the decode operators.", -1, methods,
+                      nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__hostops(void) {
+#define INTERN(s) if (!(S_##s = PyUnicode_InternFromString(#s))) return nullptr;
+  NAMES(INTERN)
+#undef INTERN
+  return PyModule_Create(&module);
+}

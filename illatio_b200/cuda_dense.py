@@ -25,8 +25,7 @@ def _ptr(t):
     return 0 if t is None else t.data_ptr()
 
 
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
+_stream = _lib.stream
 
 
 @dataclass
@@ -69,6 +68,8 @@ class QAct:
     xq: torch.Tensor     # int8 [n * cols]
     xs: torch.Tensor     # float32 per 32 (q8) or per 256 (q8k)
     xsum: torch.Tensor   # q8: int32 per 32 (or None); q8k: int16 per 16
+    _cf = None           # the fp16 form, once a tcgen05 product has used it (a ChunkF16)
+    _cf_fresh = False    # it is that of the quants
 
 
 def make_qact(n, kind, device="cuda", want_xsum=False):
@@ -87,47 +88,45 @@ def matrix_act_kind(w):
     return "q8k" if cmat_kquant_p(w) else "q8"
 
 
-def quant_q8(x, act, f16_scale=True):
-    """X (float32, a whole number of blocks) quantized into ACT: the reference's
-    quant_q8 launch (src/cuda-dense.lisp:366,417), in the kind ACT holds."""
-    n = x.numel()
-    if act.kind == "q8":
-        _lib.call("ill_quant_q8_0", _ptr(x), _ptr(act.xq), _ptr(act.xs), _ptr(act.xsum), n // 32,
-                  1 if f16_scale else 0, _stream())
-    else:
-        cf = getattr(act, "_cf", None)
-        if cf is not None and cf.n * cf.cols == n:
-            # ACT's fp16 form is in use by the tcgen05 products: renewed in the same launch
-            _lib.call("ill_quant_q8_k_f16", _ptr(x), _ptr(act.xq), _ptr(act.xs), _ptr(act.xsum), _ptr(cf.xh), _ptr(cf.xe), n // 256,
-                      _stream())
-            cf.xd = act.xs
-            act._cf_fresh = True
-            return act
-        _lib.call("ill_quant_q8_k", _ptr(x), _ptr(act.xq), _ptr(act.xs), _ptr(act.xsum), n // 256, _stream())
-    act._cf_fresh = False
+# The operators of a decoded token are native (csrc/hostops.cpp: the signatures and docstrings are there); the
+# functions below that begin with an underscore and share a name with one are what it leaves to Python.
+_H = _lib.hostops()
+quant_q8, rmsnorm_q8, cmat_mul, qkv_mul, glu_mul, embed = (getattr(_H, f) for f in (
+    "quant_q8", "rmsnorm_q8", "cmat_mul", "qkv_mul", "glu_mul", "embed"))
+
+
+def _quant_q8(x, act, f16_scale=True):
+    """quant_q8 of an ACT whose fp16 form is in use by the tcgen05 products: renewed in the same launch."""
+    n, cf = x.numel(), act._cf
+    if act.kind == "q8k" and cf.n * cf.cols == n:
+        _lib.call("ill_quant_q8_k_f16", _ptr(x), _ptr(act.xq), _ptr(act.xs), _ptr(act.xsum), _ptr(cf.xh), _ptr(cf.xe), n // 256,
+                  _stream())
+        cf.xd = act.xs
+        act._cf_fresh = True
+        return act
+    act._cf, act._cf_fresh = None, False
+    quant_q8(x, act, f16_scale)
+    act._cf = cf
     return act
 
 
-def rmsnorm_q8(x, w, act, d, eps, n=1, h=None, f16_scale=True):
-    """RMSNORM-Q8 (src/cuda-dense.lisp:260-264): RMSNORM! of N rows of X (D wide) by
-    W, quantized into ACT in the kind it holds; H, when given, also gets the floats."""
-    cf = getattr(act, "_cf", None)
-    if act.kind == "q8k" and cf is not None and cf.n == n and cf.cols == d:
-        # ACT's fp16 form is in use by the tcgen05 products: renewed in the same launch
+def _rmsnorm_q8(x, w, act, d, eps, n=1, h=None, f16_scale=True):
+    """rmsnorm_q8 of an ACT whose fp16 form is in use by the tcgen05 products: renewed in the same launch."""
+    cf = act._cf
+    if act.kind == "q8k" and cf.n == n and cf.cols == d:
         _lib.call("ill_rmsnorm_q8k_f16", _ptr(x), _ptr(w), _ptr(h), _ptr(act.xq), _ptr(act.xs), _ptr(act.xsum), _ptr(cf.xh),
                   _ptr(cf.xe), d, float(eps), n, _stream())
         cf.xd = act.xs
         act._cf_fresh = True
         return act
-    _lib.call("ill_rmsnorm_q8", 1 if act.kind == "q8k" else 0, _ptr(x), _ptr(w), _ptr(h), _ptr(act.xq), _ptr(act.xs),
-              _ptr(act.xsum), d, float(eps), n, 1 if f16_scale else 0, _stream())
-    act._cf_fresh = False
+    act._cf, act._cf_fresh = None, False
+    rmsnorm_q8(x, w, act, d, eps, n, h, f16_scale)
+    act._cf = cf
     return act
 
 
-def cmat_mul(w, act, y, n=1, bias=None, acc=False):
-    """CMAT-MUL (src/cuda-dense.lisp:220-248): Y = W X for N tokens (token t's X
-    at t*cols, its Y at t*rows), or Y += it when ACC."""
+def _cmat_mul(w, act, y, n=1, bias=None, acc=False):
+    """cmat_mul of a chunk, or of a few tokens that have to be split."""
     if ((w.type == 1 or (w.type == 2 and TC_Q6K)) and act.kind == "q8k" and n >= TC_MIN_TOKENS and w.rows >= TC_MIN_ROWS and w.rows % 4 == 0 and bias is None
             and w.qs.data_ptr() % 16 == 0 and act.xq.numel() == n * w.cols):
         # a prefill chunk of a Q4_K / Q6_K matrix: the tcgen05 kernel (the activations' fp16 form is made once per quantization)
@@ -165,43 +164,31 @@ def _side_stream(device):
     return s
 
 
-def qkv_mul(wq, wk, wv, act, q, k, v, bq=None, bk=None, bv=None, n=1):
-    """QKV-MUL (src/cuda-dense.lisp:309-324): one launch when the three formats
-    agree and there is one token, else three products."""
-    if n == 1 and wq.type == wk.type == wv.type:
-        _lib.call("ill_mv_3", wq.type, _ptr(wq.qs), _ptr(wk.qs), _ptr(wv.qs), wq.rows, wk.rows, wv.rows, wq.cols,
-                  _ptr(act.xq), _ptr(act.xs), _ptr(act.xsum) if act.kind == "q8k" else 0,
-                  _ptr(q), _ptr(k), _ptr(v), _ptr(bq), _ptr(bk), _ptr(bv), _stream())
-    elif n == 1 and wq.type == wk.type:
-        # Q4_K_M files keep V in Q6_K: Q and K in one launch, V in its own -- beside it, on a second
-        # stream (both read the same activations; in a captured graph this is a fork and a join)
-        cur = torch.cuda.current_stream()
-        side = _side_stream(cur.device)
-        side.wait_stream(cur)
-        with torch.cuda.stream(side):
-            cmat_mul(wv, act, v, n, bias=bv)
-        _lib.call("ill_mv_3", wq.type, _ptr(wq.qs), _ptr(wk.qs), 0, wq.rows, wk.rows, 0, wq.cols,
-                  _ptr(act.xq), _ptr(act.xs), _ptr(act.xsum) if act.kind == "q8k" else 0,
-                  _ptr(q), _ptr(k), 0, _ptr(bq), _ptr(bk), 0, _stream())
-        cur.wait_stream(side)
-    else:
-        cmat_mul(wq, act, q, n, bias=bq)
-        cmat_mul(wk, act, k, n, bias=bk)
+def _qkv_mul(wq, wk, wv, act, q, k, v, bq=None, bk=None, bv=None, n=1):
+    """qkv_mul of one token with a V in a format of its own, in a stream that is being captured: Q and K in one
+    launch, V in its own beside it (both read the same activations; in the graph this is a fork and a join)."""
+    cur = torch.cuda.current_stream()
+    side = _side_stream(cur.device)
+    side.wait_stream(cur)
+    with torch.cuda.stream(side):
         cmat_mul(wv, act, v, n, bias=bv)
+    _lib.call("ill_mv_3", wq.type, _ptr(wq.qs), _ptr(wk.qs), 0, wq.rows, wk.rows, 0, wq.cols,
+              _ptr(act.xq), _ptr(act.xs), _ptr(act.xsum) if act.kind == "q8k" else 0,
+              _ptr(q), _ptr(k), 0, _ptr(bq), _ptr(bk), 0, _stream())
+    cur.wait_stream(side)
 
 
-def glu_mul(g, u, act, fa, n=1, fb=None):
-    """GLU-MUL (src/cuda-dense.lisp:326-339): silu(G x) * (U x) into FA."""
-    if n == 1 and g.type == u.type:
-        _lib.call("ill_mv_glu", g.type, _ptr(g.qs), _ptr(u.qs), g.rows, g.cols, _ptr(act.xq), _ptr(act.xs),
-                  _ptr(act.xsum) if act.kind == "q8k" else 0, _ptr(fa), _stream())
-        return fa
+def _glu_mul(g, u, act, fa, n=1, fb=None):
+    """glu_mul of several tokens, or of two formats."""
     if fb is None:
         fb = torch.empty_like(fa)
     cmat_mul(g, act, fa, n)
     cmat_mul(u, act, fb, n)
-    fa.copy_((fa / (1.0 + torch.exp(-fa))) * fb)  # the reference's swiglu kernel; not on the decode path
+    _lib.call("ill_silu_mul", fa.numel(), _ptr(fa), _ptr(fb), _ptr(fa), _stream())
     return fa
+
+
+_H.set_slow({"quant_q8": _quant_q8, "rmsnorm_q8": _rmsnorm_q8, "cmat_mul": _cmat_mul, "qkv_mul": _qkv_mul, "glu_mul": _glu_mul, "error": _lib.fail})
 
 
 class ChunkF16:
@@ -264,11 +251,11 @@ TC_Q6K = True
 
 def _chunk_f16_of(act, n, cols):
     """ACT's fp16 form for the tcgen05 product, made once per quantization of ACT (quant_q8 / rmsnorm_q8 mark it stale)."""
-    cf = getattr(act, "_cf", None)
+    cf = act._cf
     if cf is None or cf.n != n or cf.cols != cols:
         cf = act._cf = ChunkF16(n, cols, device=act.xq.device)
         act._cf_fresh = False
-    if not getattr(act, "_cf_fresh", False):
+    if not act._cf_fresh:
         cf.fill(act)
         act._cf_fresh = True
     return cf
@@ -318,14 +305,6 @@ class DecodePlan:
 
     def run(self):
         _lib.call("ill_decode_run", self.base, self.launch, _stream())
-
-
-def embed(emb, tokens, x):
-    """EMBED (src/cuda-dense.lisp:302-307): rows TOKENS (int32 on the device) of
-    EMB as floats in X."""
-    _lib.call("ill_dequant_rows", emb.type, _ptr(emb.qs), emb.cols, _ptr(tokens), 0, tokens.numel(), _ptr(x),
-              _stream())
-    return x
 
 
 def dequant_rows(w, first_row, nrows, out=None):

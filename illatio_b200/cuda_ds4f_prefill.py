@@ -20,8 +20,7 @@ def _ptr(t):
     return 0 if t is None else t.data_ptr()
 
 
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
+_stream = _lib.stream
 
 
 @dataclass
