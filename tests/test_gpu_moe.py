@@ -130,3 +130,19 @@ def test_mv_dense_matches_f32mv(oracle, dtype, rows, cols, n):
     y1 = torch.empty(rows, device="cuda")
     M.dk_mv16(wd, xd[:1], y1)
     assert torch.equal(y1, y[0, :rows])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols,n", [(1, 8, 1), (3, 5128, 1), (8, 256, 5), (9, 264, 16), (33, 8, 17), (250, 520, 601), (288, 5120, 33)])
+def test_mv_dense_tiles(cuda_lib, dtype, rows, cols, n):
+    """The tiled chunk kernel and the one-token kernel at the edges of their tiles, slabs and row batches: the bits of
+    the token loop (taken two tokens at a time, which is what runs it), and nothing written past a row's end."""
+    g = torch.Generator(device="cuda").manual_seed(rows * cols + n)
+    w = torch.randn(rows, cols, device="cuda", generator=g).to(dtype)
+    x = torch.randn(n + n % 2, cols, device="cuda", generator=g)
+    y = torch.full((n, rows + 3), 5.0, device="cuda")
+    _lib.call("ill_mv_dense", M._DENSE_TYPES[dtype], w.data_ptr(), rows, cols, x.data_ptr(), y.data_ptr(), n, rows + 3, None)
+    want = torch.empty(n + n % 2, rows, device="cuda")
+    for t in range(0, n, 2):
+        M.dk_mv16(w, x[t:t + 2], want[t:t + 2], n=2)
+    assert torch.equal(y[:, :rows], want[:n]) and (y[:, rows:] == 5.0).all()
