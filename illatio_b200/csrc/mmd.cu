@@ -12,6 +12,7 @@
 //   * activations: the step's TN x 256 quants and their scales are brought by all threads with cp.async into one
 //     of two buffers while the other is being used -- one __syncthreads a step; a token tile's quants reach the
 //     registers as B fragments through ldmatrix.
+// This is mmd_kernel, for Q4_K and Q6_K; Q8_0 has a kernel of its own (mmq8_kernel).
 // Token tiles are the fastest-varying CTA index: the CTAs that share a tile of rows run together and the weights
 // come from HBM once.  Waits are bounded (status word, ST_MV_WAIT + 0x40 + format); a warp that gave up keeps
 // meeting the CTA's barriers and lets its copies land before the CTA leaves.
@@ -24,7 +25,7 @@
 
 namespace ill {
 
-constexpr int MD_WARPS = 8, MD_THREADS = 32 * MD_WARPS, MD_ROWS = 16 * MD_WARPS, MD_MAX_STAGES = 3;
+constexpr int MD_WARPS = 8, MD_THREADS = 32 * MD_WARPS, MD_MAX_STAGES = 3;
 constexpr int MD_XPITCH = 272;  // bytes between the tokens' 256 quants of a step: 68 words, so eight tokens x four words hit 32 banks
 
 struct MdParams {
@@ -234,7 +235,6 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
   extern __shared__ __align__(128) u8 smem[];
   constexpr int TN = 8 * NT8, SB = MdFrag<FMT>::SB, MD_SPITCH = MdFrag<FMT>::SPITCH;
   const int MD_STAGES = p.stages;
-  constexpr bool KQ = FMT != ILL_Q8_0;  // Q8_K activations: one scale a step (Q8_0: eight)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int ntt = (p.n + TN - 1) / TN, nthreads = blockDim.x;  // eight warps, or fewer when the matrix has few rows
   const int tok0 = (int)(blockIdx.x % ntt) * TN, row_base = (int)(blockIdx.x / ntt) * (nthreads / 2) + warp * 16;
@@ -272,27 +272,19 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
       if (tok0 + tk < p.n && c0 + 16 * ch < p.cols)
         cp_async16(xb + tk * MD_XPITCH + 16 * ch, p.xq + (long long)(tok0 + tk) * p.cols + c0 + 16 * ch);
     }
-    if constexpr (KQ) {
-      for (int i = tid; i < TN; i += nthreads)
-        if (tok0 + i < p.n) cp_async4(xb + p.xs_off + 4 * i, p.xs + (long long)(tok0 + i) * nsteps + step);
-      if constexpr (FMT == ILL_Q4_K) {
-        for (int i = tid; i < TN * 2; i += nthreads) {
-          const int tk = i >> 1, ch = i & 1;
-          if (tok0 + tk < p.n)
-            cp_async16(xb + p.xsum_off + tk * MD_SPITCH + 16 * ch, p.xsum + (long long)(tok0 + tk) * (p.cols / 16) + 16 * step + 8 * ch);
-        }
-      }
-    } else {
+    for (int i = tid; i < TN; i += nthreads)
+      if (tok0 + i < p.n) cp_async4(xb + p.xs_off + 4 * i, p.xs + (long long)(tok0 + i) * nsteps + step);
+    if constexpr (FMT == ILL_Q4_K) {
       for (int i = tid; i < TN * 2; i += nthreads) {
         const int tk = i >> 1, ch = i & 1;
-        if (tok0 + tk < p.n && c0 + 128 * ch < p.cols)
-          cp_async16(xb + p.xs_off + tk * MD_SPITCH + 16 * ch, p.xs + (long long)(tok0 + tk) * (p.cols / 32) + 8 * step + 4 * ch);
+        if (tok0 + tk < p.n)
+          cp_async16(xb + p.xsum_off + tk * MD_SPITCH + 16 * ch, p.xsum + (long long)(tok0 + tk) * (p.cols / 16) + 16 * step + 8 * ch);
       }
     }
     cp_async_commit();
   };
 
-  // both activation buffers start as zeros: the tokens past the last, and the columns past a Q8_0 row's end, stay so
+  // both activation buffers start as zeros: the tokens past the last stay so
   for (uint32_t i = 16u * tid; i < 2u * p.xbuf_bytes; i += 16u * nthreads) *(uint4*)(smem + i) = make_uint4(0, 0, 0, 0);
   if (lane == 0) {
     for (int s = 0; s < MD_STAGES; ++s) mbar_init(&full[s], 1);
@@ -329,23 +321,20 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
       const long long o8 = o0 + 8ll * p.row_bytes;
       const u8* row0 = piece + (size_t)g * p.pitch + (((uintptr_t)p.w + o0) & 15);
       const u8* row8 = piece + (size_t)(g + 8) * p.pitch + (((uintptr_t)p.w + o8) & 15);
-      f.load(row0, row8, lane, min(8, (p.cols - 256 * step) / 32));
+      f.load(row0, row8, lane, 8);
     }
     __syncwarp();
     issue_w();  // the stage is free: its block sits in registers
     const u8* xb = smem + (size_t)(step & 1) * p.xbuf_bytes;
     const u8* xl = xb + (lane & 7) * MD_XPITCH + 16 * (lane >> 3);  // this lane's row of the four matrices ldsm4 reads
-    // Q8_0: the eight scales of token 2 t (+ 8 nt); Q4_K: its sixteen sums of 16
-    const u8* scl = xb + (FMT == ILL_Q4_K ? p.xsum_off : p.xs_off) + 2 * t * MD_SPITCH;
+    const u8* scl = xb + p.xsum_off + 2 * t * MD_SPITCH;  // Q4_K: the sixteen sums of 16 of token 2 t (+ 8 nt)
     const float* ys = (const float*)(xb + p.xs_off) + 2 * t;
 #pragma unroll
     for (int nt = 0; nt < NT8; ++nt) {
       uint32_t x[4][4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) ldsm4(x[j], xl + 8 * nt * MD_XPITCH + 64 * j);
-      float ya = 0.0f, yb = 0.0f;
-      if constexpr (KQ) { ya = ys[8 * nt]; yb = ys[8 * nt + 1]; }
-      f.apply(x, scl + 8 * nt * MD_SPITCH, scl + (8 * nt + 1) * MD_SPITCH, ya, yb, acc[nt]);
+      f.apply(x, scl + 8 * nt * MD_SPITCH, scl + (8 * nt + 1) * MD_SPITCH, ys[8 * nt], ys[8 * nt + 1], acc[nt]);
     }
   }
   if (dead) {
@@ -365,6 +354,224 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
         if (p.bias) v += p.bias[row];
         float* yp = p.y + (long long)tok * p.rows + row;
         *yp = p.acc ? *yp + v : v;
+      }
+    }
+}
+
+// ---- Q8_0 chunks ---------------------------------------------------------------------------------------------
+// What bounds a Q8_0 chunk is not the tensor pipe but what every m16n8k32 product needs after it: its four integers
+// become floats and meet d_w * d_x, because Q8_0's scales are per 32 columns on both sides.  So the kernel is built
+// around those instructions -- four conversions, two packed multiplies and two packed fused multiply-adds
+// (fma.rn.f32x2: each half rounds as the scalar instruction does) a product -- and keeps everything else off the
+// issue slots:
+//   * columns in steps of 128 (four blocks; a row's step is 136 bytes), weights and activations both by 16-byte
+//     cp.async into a ring of two or three stages, one __syncthreads a step;
+//   * what a thread copies lies at fixed distances from one step to the next: a step's copies are an add and a few
+//     predicates beside the copies themselves;
+//   * the activations' scales are staged in the order a lane reads them: the four of a token pair's two blocks are one
+//     16-byte load for two products;
+//   * two blocks of weights sit in registers at a time (mmd_kernel holds eight): 80 tokens a CTA fit 128 registers and
+//     two CTAs share an SM.
+// A CTA of eight warps takes 16 RW rows x 8 NT8 tokens; with RW < 8 the warps are 8 / RW groups that take every
+// (8 / RW)-th step each and meet in shared memory in group order (few rows of many columns).
+//
+// Measured against mmd_kernel, which took Q8_0 before: 2048 x 4096 x 4096 tokens 412 -> 277 us (248 int8 TOPS), 5120 x 1536
+// x 8192 728 -> 492, 4864 x 896 x 777 58 -> 36, 896 x 4864 x 777 129 -> 48, 2048 x 4096 x 64 62 -> 14, 896 x 4864 x 17
+// 64 -> 9.  What is left: about 23 cycles a product of a scheduler where the packed arithmetic alone takes 8 and the int8
+// mma.sync 8.2, and 1.1 us a step for unpacking, copying and the barrier.  Measured and dropped: 32 rows a warp (half the
+// ldmatrix traffic, the same time), the integers turned into floats by adding 1.5 * 2^23 in the product (4 % slower).
+template <int NT8, int RW>
+struct Mq {
+  static constexpr int TN = 8 * NT8, KS = MD_WARPS / RW;
+  static constexpr int WPITCH = 176;  // ten chunks of 16 bytes a row's step; 44 words: eight rows x four words on 32 banks
+  static constexpr int XPITCH = 144;  // 36 words: ldmatrix's eight rows on 32 banks
+  static constexpr int W_BYTES = MD_WARPS * 16 * WPITCH, X_BYTES = KS * TN * XPITCH, S_BYTES = KS * TN * 16;
+  static constexpr int STAGE = W_BYTES + X_BYTES + S_BYTES;
+  static constexpr int TWO_CTAS = 233472 / 2 - 1024;  // shared memory a CTA may have for two to share an SM
+  static constexpr int PER_SM = 2 * STAGE <= TWO_CTAS ? 2 : 1, STAGES = PER_SM == 2 && 3 * STAGE > TWO_CTAS ? 2 : 3;
+};
+
+__device__ __forceinline__ uint64_t md_mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ void md_fma2(uint64_t& d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t md_pack(float a, float b) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+
+template <int NT8, int RW>
+__global__ void __launch_bounds__(MD_THREADS, 2) mmq8_kernel(const MdParams p) {
+  extern __shared__ __align__(128) u8 smem[];
+  using C = Mq<NT8, RW>;
+  constexpr int TN = C::TN, KS = C::KS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int rw = warp % RW, kg = warp / RW;
+  const int ntt = (p.n + TN - 1) / TN;
+  const int tok0 = (int)(blockIdx.x % ntt) * TN, row_base = (int)(blockIdx.x / ntt) * (16 * RW) + rw * 16;
+  const int nsteps = p.nsteps, nit = (nsteps + KS - 1) / KS;
+  const bool live = row_base < p.rows;  // a warp whose rows are all past the end only helps to bring the activations
+  const u8* wrow0 = p.w + (long long)row_base * p.row_bytes;
+
+  // Weights: four lanes a row, chunks lane % 4, + 4 and + 8 of its 16-byte aligned span (nine or ten chunks).
+  const u8* wsrc = wrow0 + (long long)g * p.row_bytes + (long long)kg * 136;  // row g's bytes of the step copied next
+  const long long w8 = 8ll * p.row_bytes;
+  const bool in0 = live && row_base + g < p.rows, in8 = live && row_base + g + 8 < p.rows;
+  const uint32_t wdst = (uint32_t)((warp * 16 + g) * C::WPITCH + 16 * t);
+  // Activations: eight threads a token's 128 quants, 32 tokens at a time; a thread a scale.
+  constexpr int XJ = (TN + 31) / 32, SJ = (TN * 4 + MD_THREADS - 1) / MD_THREADS;
+  const int xtk = tid >> 3, stk = tid >> 2;
+  const i8* xsrc = p.xq + (long long)(tok0 + xtk) * p.cols + 16 * (tid & 7);
+  const float* ssrc = p.xs + (long long)(tok0 + stk) * (p.cols / 32) + (tid & 3);
+  const uint32_t xdst = (uint32_t)(C::W_BYTES + xtk * C::XPITCH + 16 * (tid & 7));
+  // scale of token 2 j + h, block 2 b + o of the step -> float [b][j][o][h]
+  const uint32_t sdst = (uint32_t)(C::W_BYTES + C::X_BYTES + 4 * ((((tid & 3) >> 1) * (TN / 2) + (stk >> 1)) * 4 + 2 * (tid & 1) + (stk & 1)));
+  int w_step = kg, x_step = 0;  // the steps copied next
+  auto fill_w = [&](u8* st) {
+    if (w_step < nsteps) {
+      auto row = [&](const u8* src, u8* dst) {
+        const u8* a = (const u8*)((uintptr_t)src & ~(uintptr_t)15) + 16 * t;
+        cp_async16(dst, a);
+        cp_async16(dst + 64, a + 64);
+        if (t == 0 || (t == 1 && ((uintptr_t)src & 15) > 8)) cp_async16(dst + 128, a + 128);
+      };
+      if (in0) row(wsrc, st + wdst);
+      if (in8) row(wsrc + w8, st + wdst + 8 * C::WPITCH);
+    }
+    wsrc += KS * 136;
+    w_step += KS;
+  };
+  auto fill_x = [&](u8* st) {
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      if (x_step + ks < nsteps) {
+#pragma unroll
+        for (int j = 0; j < XJ; ++j)
+          if ((TN % 32 == 0 || 32 * j + xtk < TN) && tok0 + 32 * j + xtk < p.n)
+            cp_async16(st + xdst + (ks * TN + 32 * j) * C::XPITCH, xsrc + 128 * ks + 32ll * j * p.cols);
+#pragma unroll
+        for (int j = 0; j < SJ; ++j)
+          if ((TN % 64 == 0 || 64 * j + stk < TN) && tok0 + 64 * j + stk < p.n)
+            cp_async4(st + sdst + ks * TN * 16 + 512 * j, ssrc + 4 * ks + 2ll * j * p.cols);
+      }
+    }
+    xsrc += 128 * KS;
+    ssrc += 4 * KS;
+    x_step += KS;
+  };
+
+  fill_w(smem);  // the weights do not depend on the previous kernel
+  if (p.stages == 3) fill_w(smem + C::STAGE);
+  pdl_launch_dependents();
+  pdl_wait();
+  fill_x(smem);
+  cp_async_commit();
+  if (p.stages == 3) {
+    fill_x(smem + C::STAGE);
+    cp_async_commit();
+  }
+
+  uint64_t acc[NT8][2];  // [tile of eight tokens][row g / g + 8]: tokens 2 t and 2 t + 1
+#pragma unroll
+  for (int nt = 0; nt < NT8; ++nt) acc[nt][0] = acc[nt][1] = 0ull;
+  const bool even_off = ((uintptr_t)p.w & 2) == 0;  // a row is a multiple of four bytes: which blocks' quants are word-aligned
+  const uint32_t last = (uint32_t)(p.stages - 1) * C::STAGE;
+  uint32_t use_at = 0, fill_at = last, w_off = (uint32_t)(uintptr_t)wrow0 + (uint32_t)g * p.row_bytes + 136u * kg;
+  for (int it = 0; it < nit; ++it) {
+    if (p.stages == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");  // this iteration's copies are in
+    else cp_async_wait_all();
+    __syncthreads();  // ... everyone's; and everyone is through with the stage refilled next
+    fill_w(smem + fill_at);
+    fill_x(smem + fill_at);
+    cp_async_commit();
+    const u8* st = smem + use_at;
+    use_at = use_at == last ? 0 : use_at + C::STAGE;
+    fill_at = fill_at == last ? 0 : fill_at + C::STAGE;
+    const uint32_t o0 = w_off;
+    w_off += KS * 136;
+    if (!live || it * KS + kg >= nsteps) continue;
+    const u8* r0 = st + (warp * 16 + g) * C::WPITCH + (o0 & 15);
+    const u8* r8 = st + (warp * 16 + g + 8) * C::WPITCH + ((o0 + 8u * p.row_bytes) & 15);
+    const u8* xl = st + C::W_BYTES + (kg * TN + (lane & 7)) * C::XPITCH + 16 * (lane >> 3);
+    const u8* sl = st + C::W_BYTES + C::X_BYTES + kg * TN * 16 + 16 * t;
+#pragma unroll
+    for (int b2 = 0; b2 < 2; ++b2) {  // blocks 2 b2 and 2 b2 + 1 of the step
+      uint32_t a[2][4];
+      uint64_t d0[2], d8[2];
+#pragma unroll
+      for (int o = 0; o < 2; ++o) {
+        const u8 *q0 = r0 + 34 * (2 * b2 + o) + 2 + 4 * t, *q8 = r8 + 34 * (2 * b2 + o) + 2 + 4 * t;
+        if ((o == 1) == even_off) {
+          a[o][0] = *(const uint32_t*)q0; a[o][1] = *(const uint32_t*)q8;
+          a[o][2] = *(const uint32_t*)(q0 + 16); a[o][3] = *(const uint32_t*)(q8 + 16);
+        } else {
+          a[o][0] = __funnelshift_r(*(const uint32_t*)(q0 - 2), *(const uint32_t*)(q0 + 2), 16);
+          a[o][1] = __funnelshift_r(*(const uint32_t*)(q8 - 2), *(const uint32_t*)(q8 + 2), 16);
+          a[o][2] = __funnelshift_r(*(const uint32_t*)(q0 + 14), *(const uint32_t*)(q0 + 18), 16);
+          a[o][3] = __funnelshift_r(*(const uint32_t*)(q8 + 14), *(const uint32_t*)(q8 + 18), 16);
+        }
+        const float f0 = ldh(q0 - 2 - 4 * t), f8 = ldh(q8 - 2 - 4 * t);
+        d0[o] = md_pack(f0, f0);
+        d8[o] = md_pack(f8, f8);
+      }
+#pragma unroll
+      for (int nt = 0; nt < NT8; ++nt) {
+        uint32_t x[4];
+        ldsm4(x, xl + 8 * nt * C::XPITCH + 64 * b2);
+        const ulonglong2 s = *(const ulonglong2*)(sl + (b2 * (TN / 2) + 4 * nt) * 16);
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+          const uint64_t xs = o ? s.y : s.x;
+          int c[4];
+          mma_k32_s8(c, a[o], x[2 * o], x[2 * o + 1]);
+          // Q8-ROW-DOT-AT: sum += float(isum) * (d_w * d_x)
+          md_fma2(acc[nt][0], md_pack((float)c[0], (float)c[1]), md_mul2(d0[o], xs));
+          md_fma2(acc[nt][1], md_pack((float)c[2], (float)c[3]), md_mul2(d8[o], xs));
+        }
+      }
+    }
+  }
+  float v[NT8][4];
+#pragma unroll
+  for (int nt = 0; nt < NT8; ++nt)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) asm("mov.b64 {%0, %1}, %2;" : "=f"(v[nt][2 * i]), "=f"(v[nt][2 * i + 1]) : "l"(acc[nt][i]));
+  if constexpr (KS > 1) {  // the groups' partial sums meet in the first group's warps, in group order
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float* part = (float*)smem;  // [group - 1][row warp][value][lane]
+    static_assert((KS - 1) * RW * NT8 * 4 * 32 * 4 <= 2 * C::STAGE, "");
+    if (kg > 0)
+#pragma unroll
+      for (int nt = 0; nt < NT8; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) part[((((kg - 1) * RW + rw) * NT8 + nt) * 4 + i) * 32 + lane] = v[nt][i];
+    __syncthreads();
+    if (kg > 0) return;
+#pragma unroll
+    for (int k = 0; k < KS - 1; ++k)
+#pragma unroll
+      for (int nt = 0; nt < NT8; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[nt][i] = __fadd_rn(v[nt][i], part[(((k * RW + rw) * NT8 + nt) * 4 + i) * 32 + lane]);
+  }
+  if (!live) return;
+#pragma unroll
+  for (int nt = 0; nt < NT8; ++nt)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const long long row = row_base + g + 8 * (i >> 1);
+      const int tok = tok0 + 8 * nt + 2 * t + (i & 1);
+      if (row < p.rows && tok < p.n) {
+        float r = v[nt][i];
+        if (p.bias) r += p.bias[row];
+        float* yp = p.y + (long long)tok * p.rows + row;
+        *yp = p.acc ? *yp + r : r;
       }
     }
 }
@@ -535,6 +742,49 @@ static int mmd_launch(const MdParams& p, int tn, size_t smem, int grid, cudaStre
   return launch_kernel(k, dim3(grid), dim3(32 * p.warps), smem, args, st);
 }
 
+// The launch of a Q8_0 chunk.  Which tile: the one with the least of (steps a CTA goes through) x (CTAs one after
+// another on an SM) x (time a step).  STEP is that time in us with two CTAs on an SM (alone on it a CTA takes about
+// 0.65 of it), or with the one that fits, measured on 2048 x 4096 x 4096 tokens.  Over 20 shapes of 17 to 8192 tokens the
+// tile that it picks is the fastest measured or within 12 % of it (128 x 896 x 777: 9 us against 6.4).
+struct MqTile {
+  float step;
+  int rn, tn, ks, per_sm, stages;
+  uint32_t stage;
+  const void* kernel;
+};
+template <int NT8, int RW>
+static MqTile mq_tile(float step) {
+  using C = Mq<NT8, RW>;
+  return {step, 16 * RW, C::TN, C::KS, C::PER_SM, C::STAGES, (uint32_t)C::STAGE, (const void*)mmq8_kernel<NT8, RW>};
+}
+
+static int mmq8_launch(MdParams p, int sms, cudaStream_t st) {
+  static const MqTile tiles[] = {
+      mq_tile<4, 8>(1.91f), mq_tile<4, 4>(2.05f), mq_tile<4, 2>(2.33f), mq_tile<4, 1>(2.03f),
+      mq_tile<6, 8>(2.39f), mq_tile<6, 4>(2.49f), mq_tile<6, 2>(2.84f),
+      mq_tile<8, 8>(2.67f), mq_tile<8, 4>(2.92f), mq_tile<8, 2>(2.24f),
+      mq_tile<10, 8>(3.08f), mq_tile<10, 4>(3.42f), mq_tile<10, 2>(2.56f),
+  };
+  p.nsteps = p.cols / 128;
+  const MqTile* best = nullptr;
+  double best_us = 0.0;
+  long long grid = 0;
+  for (const MqTile& t : tiles) {
+    const long long ctas = (long long)((p.rows + t.rn - 1) / t.rn) * ((p.n + t.tn - 1) / t.tn);
+    const long long full = ctas / ((long long)t.per_sm * sms), rest = ctas % ((long long)t.per_sm * sms);
+    const double waves = (double)full + (rest == 0 ? 0.0 : t.per_sm == 2 && rest <= sms ? 0.65 : 1.0);
+    const double us = waves * ((p.nsteps + t.ks - 1) / t.ks) * t.step;
+    if (!best || us < best_us) { best = &t; best_us = us; grid = ctas; }
+  }
+  if (grid > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
+  p.stages = grid <= sms ? 3 : best->stages;  // a CTA that has the SM to itself has room for three
+  const size_t smem = (size_t)p.stages * best->stage;
+  cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(3 * best->stage));
+  if (e != cudaSuccess) return cuda_fail(e);
+  void* args[] = {&p};
+  return launch_kernel(best->kernel, dim3((unsigned)grid), dim3(MD_THREADS), smem, args, st);
+}
+
 // The chunk product on the tensor cores, for the formats and layouts it is written for; ILL_ERR_UNSUPPORTED
 // otherwise (the caller then takes the token loop of the CUDA-core kernel).
 int mmd_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum, uint64_t y, uint64_t bias, int acc,
@@ -563,6 +813,7 @@ int mmd_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+  if (!kq) return mmq8_launch(p, sms, (cudaStream_t)stream);
   // Tokens a CTA: 128 amortize a block's unpacking best (one CTA of eight warps an SM, up to 255 registers); tiles
   // of 64 keep a thread within 128 registers so that two CTAs share an SM -- measured equal to slower where both
   // fill the machine, so they are for chunks of up to 64 tokens and for matrices with so few rows that tiles of 128
@@ -574,12 +825,11 @@ int mmd_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
   while (p.warps > 1 && (long long)((rows + 16 * p.warps - 1) / (16 * p.warps)) * ((n + tn - 1) / tn) < sms) p.warps >>= 1;
   // a row's step: its 16-byte aligned span (a block is read from its stage once a step, so the rows' pitch need not
   // spread them over the banks); 16 bytes after the last row for the unaligned loads' second word
-  const int sb = fmt == ILL_Q8_0 ? 272 : bb;
-  p.pitch = (sb + 15 + 15) / 16 * 16;
+  p.pitch = (bb + 15 + 15) / 16 * 16;
   p.stage_bytes = (uint32_t)(16 * p.pitch + 16);
   uint32_t off = (uint32_t)tn * MD_XPITCH;
   p.xs_off = off;
-  off += kq ? 4u * tn : (uint32_t)tn * MdFrag<ILL_Q8_0>::SPITCH;
+  off += 4u * tn;
   off = (off + 15) / 16 * 16;
   p.xsum_off = off;
   if (fmt == ILL_Q4_K) off += (uint32_t)tn * MdFrag<ILL_Q4_K>::SPITCH;
@@ -595,7 +845,6 @@ int mmd_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
   if (grid > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
   switch (fmt) {
-    case ILL_Q8_0: return mmd_launch<ILL_Q8_0>(p, tn, smem, (int)grid, st);
     case ILL_Q4_K: return mmd_launch<ILL_Q4_K>(p, tn, smem, (int)grid, st);
     default: return mmd_launch<ILL_Q6_K>(p, tn, smem, (int)grid, st);
   }

@@ -49,6 +49,31 @@ def test_chunk_product_equals_token_by_token(fmt, rows, cols, n):
     assert err < 2e-6, err
 
 
+@pytest.mark.parametrize("rows,cols,n,base", [
+    (1, 128, 17, 0), (129, 128, 33, 2), (64, 384, 81, 6), (31, 4864, 17, 14), (896, 896, 161, 0), (1000, 4864, 200, 2),
+    (300, 640, 385, 10), (2048, 4096, 65, 0), (4864, 896, 777, 8), (5121, 256, 400, 4),
+])
+def test_q8_0_chunk_tiles(rows, cols, n, base):
+    """Q8_0's chunk kernel at the edges of its tiles (32 to 80 tokens, 16 to 128 rows, columns dealt to one to eight groups
+    of warps), blocks at every 2-byte alignment, with a bias, adding to Y: against the one-token product."""
+    nbytes = B.matrix_bytes(B.Q8_0, rows, cols)
+    buf = torch.zeros(nbytes + 32, dtype=torch.uint8, device="cuda")
+    buf[base:base + nbytes] = B.synth_matrix_torch(B.Q8_0, rows, cols, seed=rows)
+    w = D.CMat("w", B.Q8_0, rows, cols, buf[base:base + nbytes])
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x, y, bias = (torch.randn(k, device="cuda", generator=g) for k in (n * cols, n * rows, rows))
+    want = y.clone()
+    D.cmat_mul(w, D.quant_q8(x, D.make_qact(n * cols, "q8")), y, n, bias=bias, acc=True)
+    one = torch.empty(rows, device="cuda")
+    top = 0.0
+    for t in range(n):
+        D.cmat_mul(w, D.quant_q8(x[t * cols:(t + 1) * cols], D.make_qact(cols, "q8")), one, 1)
+        top = max(top, one.abs().max().item())
+        want[t * rows:(t + 1) * rows] += one + bias
+    # the same integers; cols / 32 float terms added in another order: a few units of 2^-24 of the largest sum
+    assert (y - want).abs().max().item() < 2e-6 * max(top, want.abs().max().item())
+
+
 @pytest.mark.parametrize("fmt", [B.Q8_0, B.Q4_K, B.Q6_K])
 def test_chunk_product_against_the_oracle(oracle, fmt):
     rows, cols, n = 200, 1024, 70
