@@ -37,6 +37,17 @@ __device__ __forceinline__ uint32_t lds32u(const u8* p) {
   const uint32_t* b = (const uint32_t*)(p - mis);
   return __funnelshift_r(b[0], b[1], 8u * mis);
 }
+// The same for many words at distances of a multiple of four from one address: the alignment is looked at once.
+struct LdsWords {
+  const uint32_t* b;
+  uint32_t sh;
+  __device__ __forceinline__ explicit LdsWords(const u8* p) {
+    const uint32_t mis = (uint32_t)(uintptr_t)p & 3u;
+    b = (const uint32_t*)(p - mis);
+    sh = 8u * mis;
+  }
+  __device__ __forceinline__ uint32_t operator()(int off) const { return __funnelshift_r(b[off / 4], b[off / 4 + 1], sh); }
+};
 __device__ __forceinline__ float ldh(const u8* p) { return h2f(*(const u16*)p); }  // p is 2-byte aligned
 
 __device__ __forceinline__ void mma_k16_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0, bool b_unsigned) {
@@ -48,6 +59,28 @@ __device__ __forceinline__ void mma_k16_s8(int (&c)[4], uint32_t a0, uint32_t a1
     asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                  : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                  : "r"(a0), "r"(a1), "r"(b0));
+}
+
+// 16 / 4 bytes global -> shared, asynchronously; a group of them is waited for with cp.async.wait_group
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// A row segment's bytes SRC .. SRC + LEN -> shared memory by the four lanes T = 0..3 of a quad: the 16-byte aligned span
+// that covers them, NCH chunks at most (the segment starts SRC % 16 bytes into it).  One instruction brings 64 bytes of
+// each of eight rows; a bulk copy a segment costs its lane a turn of its own through the copy unit.
+template <int NCH>
+__device__ __forceinline__ void copy_segment(u8* dst, const u8* src, uint32_t len, int t) {
+  const u8* a = (const u8*)((uintptr_t)src & ~(uintptr_t)15) + 16 * t;
+  const u8* end = src + len;
+#pragma unroll
+  for (int k = 0; k < (NCH + 3) / 4; ++k)
+    if (a + 64 * k < end) cp_async16(dst + 16 * t + 64 * k, a + 64 * k);
 }
 
 // get_scale_min_k4 (src/kquant.lisp:64-72) for group J of the 12 packed bytes at Q

@@ -46,15 +46,6 @@ struct MdParams {
   unsigned* status;
 };
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
 // four 8 x 16-byte matrices of shared memory -> each lane its four bytes of row lane / 4 of each: lane l gives the
 // address of row l % 8 of matrix l / 8.  For a token tile's 64 bytes of quants this is the B fragment of two k32
 // (or four k16) steps: r[0], r[1] = b0, b1 of the first k32 step, r[2], r[3] of the second.
@@ -122,10 +113,11 @@ template <> struct MdFrag<ILL_Q4_K> {
   float d0, m0, d8, m8;
   __device__ __forceinline__ void load(const u8* row0, const u8* row8, int lane, int) {
     const int t4 = 4 * (lane & 3);
+    const LdsWords q0(row0 + t4), q8(row8 + t4);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {  // 64 weights: groups 2k (low nibbles) and 2k + 1 (high)
-      const uint32_t w0 = lds32u(row0 + 16 + 32 * k + t4), w1 = lds32u(row8 + 16 + 32 * k + t4);
-      const uint32_t w2 = lds32u(row0 + 32 + 32 * k + t4), w3 = lds32u(row8 + 32 + 32 * k + t4);
+      const uint32_t w0 = q0(16 + 32 * k), w1 = q8(16 + 32 * k);
+      const uint32_t w2 = q0(32 + 32 * k), w3 = q8(32 + 32 * k);
       lo[k][0] = w0 & 0x0F0F0F0Fu; lo[k][1] = w1 & 0x0F0F0F0Fu; lo[k][2] = w2 & 0x0F0F0F0Fu; lo[k][3] = w3 & 0x0F0F0F0Fu;
       hi[k][0] = (w0 >> 4) & 0x0F0F0F0Fu; hi[k][1] = (w1 >> 4) & 0x0F0F0F0Fu;
       hi[k][2] = (w2 >> 4) & 0x0F0F0F0Fu; hi[k][3] = (w3 >> 4) & 0x0F0F0F0Fu;
@@ -185,16 +177,15 @@ template <> struct MdFrag<ILL_Q6_K> {
   int sc0[16], sc8[16];
   float d0, d8;
   __device__ __forceinline__ void load(const u8* row0, const u8* row8, int lane, int) {
-    const int t4 = 4 * (lane & 3);
+    const LdsWords w0s(row0), w8s(row8), q0(row0 + 4 * (lane & 3)), q8(row8 + 4 * (lane & 3));
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
       for (int is = 0; is < 2; ++is) {
-        const int l = 16 * is + t4;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const u8* row = r ? row8 : row0;
-          const uint32_t A = lds32u(row + 64 * c + l), B = lds32u(row + 64 * c + 32 + l), H = lds32u(row + 128 + 32 * c + l);
+          const LdsWords& row = r ? q8 : q0;
+          const uint32_t A = row(64 * c + 16 * is), B = row(64 * c + 32 + 16 * is), H = row(128 + 32 * c + 16 * is);
           // run RUN of the half covers weights 128 c + 32 run ..: its group of 16 is 8 c + 2 run + is
           q[8 * c + 0 + is][r] = q6_signed((A & 0x0F0F0F0Fu) | ((H << 4) & 0x30303030u));
           q[8 * c + 2 + is][r] = q6_signed((B & 0x0F0F0F0Fu) | ((H << 2) & 0x30303030u));
@@ -204,7 +195,7 @@ template <> struct MdFrag<ILL_Q6_K> {
       }
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      const uint32_t w0 = lds32u(row0 + 192 + 4 * w), w8 = lds32u(row8 + 192 + 4 * w);
+      const uint32_t w0 = w0s(192 + 4 * w), w8 = w8s(192 + 4 * w);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         sc0[4 * w + j] = (int)(signed char)(w0 >> (8 * j));
@@ -578,8 +569,8 @@ __global__ void __launch_bounds__(MD_THREADS, 2) mmq8_kernel(const MdParams p) {
 
 // ---- up to sixteen tokens of rows too long for mvt.cu to keep the activations resident ------------------------
 // One 16-row tile a CTA, its column steps dealt to the eight warps (warp w takes steps w, w + 8, ...): each warp
-// streams its own steps' weights (its ring) AND its own steps' activations (cp.async by its lanes into two buffers of
-// its own), so the warps never wait for one another until the end, where their partial sums meet in shared memory
+// streams its own steps' weights (its ring of three stages) AND its own steps' activations (two buffers of its own), all
+// by 16-byte cp.async of its lanes (Q6_K 5120 x 17408, 4 tokens: 40 us; 59 with a bulk copy a row segment), so the warps never wait for one another until the end, where their partial sums meet in shared memory
 // in warp order.  A matrix of few rows and many columns (5120 x 17408) thus fills the machine with rows / 16 CTAs
 // of eight busy warps, where the chunk kernel above would run two warps a CTA through all 68 steps.
 template <int FMT, int NT8>
@@ -587,37 +578,25 @@ __global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
   extern __shared__ __align__(128) u8 smem[];
   constexpr int TN = 8 * NT8, SB = MdFrag<FMT>::SB, SP = MdFrag<FMT>::SPITCH;
   constexpr bool KQ = FMT != ILL_Q8_0;
-  const int stages = p.stages;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int ntt = (p.n + TN - 1) / TN;
   const int tok0 = (int)(blockIdx.x % ntt) * TN, row_base = (int)(blockIdx.x / ntt) * 16;
   const int nsteps = p.nsteps;
   u8* xw = smem + (size_t)warp * 2 * p.xbuf_bytes;  // this warp's two activation buffers
-  u8* ring = smem + p.ring_off + (size_t)warp * stages * p.stage_bytes;
+  u8* ring = smem + p.ring_off + (size_t)warp * MD_MAX_STAGES * p.stage_bytes;
   float* part = (float*)(smem + p.part_off);        // [warp][16 rows][TN]
-  __shared__ uint64_t full_s[MD_WARPS * MD_MAX_STAGES];
-  uint64_t* full = full_s + warp * MD_MAX_STAGES;
 
-  int issued = 0;  // of this warp's steps
-  auto issue_w = [&]() {
-    const int step = warp + MD_WARPS * issued;
-    if (step >= nsteps) return;
-    const int s = issued % stages;
-    const int row = row_base + lane;
-    uint32_t bytes = 0;
-    const u8* src = nullptr;
-    if (lane < 16 && row < p.rows) {
-      src = p.w + (long long)row * p.row_bytes + (long long)step * SB;
+  auto fill_w = [&](int k) {  // this warp's K-th step's weights -> stage k % 3 (a group of cp.async, possibly empty)
+    const int step = warp + MD_WARPS * k;
+    if (step < nsteps) {
       const uint32_t len = (uint32_t)min(SB, p.row_bytes - step * SB);
-      bytes = (uint32_t)((((uintptr_t)src + len + 15) & ~(uintptr_t)15) - ((uintptr_t)src & ~(uintptr_t)15));
-    }
-    uint32_t total = bytes;
+      u8* st = ring + (size_t)(k % MD_MAX_STAGES) * p.stage_bytes;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-    if (lane == 0) mbar_expect_tx(&full[s], total);
-    __syncwarp();
-    if (bytes) bulk_g2s(ring + (size_t)s * p.stage_bytes + (size_t)lane * p.pitch, (const void*)((uintptr_t)src & ~(uintptr_t)15), bytes, &full[s]);
-    ++issued;
+      for (int h = 0; h < 16; h += 8)
+        if (row_base + h + g < p.rows)
+          copy_segment<(SB + 30) / 16>(st + (size_t)(h + g) * p.pitch, p.w + (long long)(row_base + h + g) * p.row_bytes + (long long)step * SB, len, t);
+    }
+    cp_async_commit();
   };
   auto fill_x = [&](int k) {  // this warp's K-th step -> its buffer k % 2 (a group of cp.async, possibly empty)
     const int step = warp + MD_WARPS * k;
@@ -652,12 +631,8 @@ __global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
 
   // the warp's activation buffers start as zeros (tokens past the last, columns past a Q8_0 row's end)
   for (uint32_t i = 16u * lane; i < 2u * p.xbuf_bytes; i += 16u * 32u) *(uint4*)(xw + i) = make_uint4(0, 0, 0, 0);
-  if (lane == 0) {
-    for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
-    mbar_fence_init();
-  }
   __syncwarp();
-  for (int s = 0; s < stages; ++s) issue_w();  // the weights do not depend on the previous kernel
+  for (int s = 0; s < MD_MAX_STAGES; ++s) fill_w(s);  // the weights do not depend on the previous kernel
   pdl_launch_dependents();
   pdl_wait();
   fill_x(0);
@@ -667,18 +642,12 @@ __global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
   for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[nt][i] = 0.0f;
-  bool dead = false;
-  int done = 0;
-  for (int k = 0; warp + MD_WARPS * k < nsteps && !dead; ++k) {
+  for (int k = 0; warp + MD_WARPS * k < nsteps; ++k) {
     const int step = warp + MD_WARPS * k;
     fill_x(k + 1);                                          // the other buffer: its readers are through (the __syncwarp below)
-    asm volatile("cp.async.wait_group 1;" ::: "memory");   // all but that newest group: step k's activations are in
+    asm volatile("cp.async.wait_group 2;" ::: "memory");   // all but that group and the next-but-one step's weights: step k is in
     __syncwarp();
-    const int s = k % stages;
-    bool ok = mbar_wait(&full[s], (uint32_t)(k / stages) & 1u, p.status, ST_MV_WAIT + 0x48 + FMT);
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) { dead = true; break; }
-    ++done;
+    const int s = k % MD_MAX_STAGES;
     MdFrag<FMT> f;
     {
       const u8* piece = ring + (size_t)s * p.stage_bytes;
@@ -689,7 +658,7 @@ __global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
       f.load(row0, row8, lane, min(8, (p.cols - 256 * step) / 32));
     }
     __syncwarp();
-    issue_w();
+    fill_w(k + MD_MAX_STAGES);
     const u8* xb = xw + (size_t)(k & 1) * p.xbuf_bytes;
     const u8* xl = xb + (lane & 7) * MD_XPITCH + 16 * (lane >> 3);
     const u8* scl = xb + (FMT == ILL_Q4_K ? p.xsum_off : p.xs_off) + 2 * t * SP;
@@ -706,17 +675,13 @@ __global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
     __syncwarp();  // every lane is through with buffer k % 2 before the next iteration's copies into it are issued
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (dead) {
-    // copies still in flight into this warp's stages get a bounded time to land before shared memory is released
-    for (int k = done; k < issued; ++k) mbar_wait(&full[k % stages], (uint32_t)(k / stages) & 1u, nullptr, 0);
-  }
   // the warps' partial sums meet: thread (row, token) adds them in warp order
 #pragma unroll
   for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-      part[(warp * 16 + g + 8 * (i >> 1)) * TN + 8 * nt + 2 * t + (i & 1)] = dead ? 0.0f : acc[nt][i];
-  if (__syncthreads_or(dead)) return;  // a warp gave up (status word set): the tile is not stored
+      part[(warp * 16 + g + 8 * (i >> 1)) * TN + 8 * nt + 2 * t + (i & 1)] = acc[nt][i];
+  __syncthreads();
   for (int o = tid; o < 16 * TN; o += MD_THREADS) {
     const int r = o / TN, tk = o - r * TN;
     const long long row = row_base + r;

@@ -11,8 +11,11 @@
 //   * A persistent CTA of eight warps stages the tokens' quantized activations in shared memory once (token
 //     stride padded by 16 bytes, so that the eight tokens of a B fragment sit on different banks), then walks
 //     tiles of 16 rows.  The eight warps share a tile's blocks (warp w takes blocks w, w + 8, ...): small matrices
-//     still fill the SMs.  Each warp streams its (tile, block) pieces -- 16 row segments, a bulk copy each, issued
-//     by 16 lanes -- through its own ring of stages, across tile boundaries.
+//     still fill the SMs.  Each warp streams its (tile, block) pieces -- 16 row segments, by 16-byte
+//     cp.async, four lanes a segment -- through its own ring of stages, across tile boundaries.  (A bulk copy a segment
+//     took its lanes one after another through the copy unit, which cost more issue slots than the products: Q6_K
+//     17408 x 5120, 4 tokens 37 -> 33 us and 16 tokens 59 -> 42, Q8_0 151936 x 896 136 -> 75, Q4_K 9728 x 2560 13.3 -> 9.9;
+//     the alignment of a row's words is looked at once a block for the same reason.)
 //   * A tile's partial sums (a float per row, token and warp) meet in shared memory in a fixed order.
 //
 // mma.sync is the legacy tensor path: right here, where N is 8 or 16 and the bound is HBM; the chunk-sized
@@ -45,7 +48,6 @@ struct MtParams {
   int stages, groups;   // stages a warp's ring; groups of eight warps a CTA
   int x_stride;         // bytes between the tokens' quants in shared memory
   uint32_t xs_off, bs_off, ring_off, part_off;
-  unsigned* status;
 };
 
 
@@ -72,7 +74,8 @@ template <int NT8> struct MtBlock<ILL_Q8_0, NT8> {
   __device__ static void run(const u8* row0, const u8* row8, int blk, const MtX& x, int lane, float (&acc)[NT8][4]) {
     const int g = lane >> 2, t4 = 4 * (lane & 3);
     uint32_t a[4];
-    a[0] = lds32u(row0 + 2 + t4); a[1] = lds32u(row8 + 2 + t4); a[2] = lds32u(row0 + 18 + t4); a[3] = lds32u(row8 + 18 + t4);
+    const LdsWords q0(row0 + 2 + t4), q8(row8 + 2 + t4);
+    a[0] = q0(0); a[1] = q8(0); a[2] = q0(16); a[3] = q8(16);
     const float d0 = ldh(row0), d8 = ldh(row8);
 #pragma unroll
     for (int nt = 0; nt < NT8; ++nt) {
@@ -99,10 +102,11 @@ template <int NT8> struct MtBlock<ILL_Q4_K, NT8> {
     for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) isum[nt][i] = imin[nt][i] = 0;
+    const LdsWords q0(row0 + t4), q8(row8 + t4);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {  // 64 weights: groups 2k (low nibbles) and 2k + 1 (high)
-      const uint32_t w0 = lds32u(row0 + 16 + 32 * k + t4), w1 = lds32u(row8 + 16 + 32 * k + t4);
-      const uint32_t w2 = lds32u(row0 + 32 + 32 * k + t4), w3 = lds32u(row8 + 32 + 32 * k + t4);
+      const uint32_t w0 = q0(16 + 32 * k), w1 = q8(16 + 32 * k);
+      const uint32_t w2 = q0(32 + 32 * k), w3 = q8(32 + 32 * k);
       const uint32_t lo[4] = {w0 & 0x0F0F0F0Fu, w1 & 0x0F0F0F0Fu, w2 & 0x0F0F0F0Fu, w3 & 0x0F0F0F0Fu};
       const uint32_t hi[4] = {(w0 >> 4) & 0x0F0F0F0Fu, (w1 >> 4) & 0x0F0F0F0Fu, (w2 >> 4) & 0x0F0F0F0Fu, (w3 >> 4) & 0x0F0F0F0Fu};
       int sc0[2], mn0[2], sc8[2], mn8[2];
@@ -146,11 +150,12 @@ template <int NT8> struct MtBlock<ILL_Q6_K, NT8> {
     int isum[NT8][4];
     const signed char* sc0 = (const signed char*)(row0 + 192);
     const signed char* sc8 = (const signed char*)(row8 + 192);
+    const LdsWords q0(row0 + t4), q8(row8 + t4);
     {
       // The quants are 0..63: their -32 comes off as 32 * sum over the groups of scale * (the activations' sum of
       // the group) -- itself a product of the block's 16 x 16 scales with the tokens' sums, taken on the tensor
       // cores with each sum split in two int8 halves: sum = 16 * (sum >> 4) + (sum & 15).
-      const uint32_t s0 = lds32u(row0 + 192 + t4), s8 = lds32u(row8 + 192 + t4);
+      const uint32_t s0 = q0(192), s8 = q8(192);
       const u8* hl = (const u8*)x.bs;
 #pragma unroll
       for (int nt = 0; nt < NT8; ++nt) {
@@ -170,8 +175,8 @@ template <int NT8> struct MtBlock<ILL_Q6_K, NT8> {
         uint32_t q[2][4];  // [row g / g + 8][run]: the lane's four 6-bit quants of each run
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const u8* row = r ? row8 : row0;
-          const uint32_t A = lds32u(row + 64 * c + l), B = lds32u(row + 64 * c + 32 + l), H = lds32u(row + 128 + 32 * c + l);
+          const LdsWords& row = r ? q8 : q0;
+          const uint32_t A = row(64 * c + 16 * is), B = row(64 * c + 32 + 16 * is), H = row(128 + 32 * c + 16 * is);
           q[r][0] = (A & 0x0F0F0F0Fu) | ((H << 4) & 0x30303030u);
           q[r][1] = (B & 0x0F0F0F0Fu) | ((H << 2) & 0x30303030u);
           q[r][2] = ((A >> 4) & 0x0F0F0F0Fu) | (H & 0x30303030u);
@@ -203,16 +208,9 @@ template <int NT8> struct MtBlock<ILL_Q6_K, NT8> {
   }
 };
 
-// the meeting of one group's eight warps (barrier 1 + group), with an OR over a flag
-__device__ __forceinline__ bool group_sync_or(int grp, bool flag) {
-  uint32_t out;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %2, 0;\n\t"
-      "barrier.cta.red.or.pred.aligned p, %1, %3, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(out)
-      : "r"(1 + grp), "r"((uint32_t)flag), "n"(MT_GROUP_THREADS)
-      : "memory");
-  return out != 0;
+// the meeting of one group's eight warps (barrier 1 + group)
+__device__ __forceinline__ void group_sync(int grp) {
+  asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(1 + grp), "n"(MT_GROUP_THREADS) : "memory");
 }
 
 template <int FMT, int NT8>
@@ -228,39 +226,29 @@ __global__ void __launch_bounds__(MT_GROUP_THREADS * MT_MAX_GROUPS) mvt_kernel(c
   int16_t* bs_s = (int16_t*)(smem + p.bs_off);
   u8* ring = smem + p.ring_off + (size_t)cwarp * stages * p.stage_bytes;
   float* part = (float*)(smem + p.part_off) + (size_t)grp * 2 * MT_WARPS * 256;  // [group][2][warps][16 rows][16 tokens]
-  __shared__ uint64_t full_s[MT_MAX_GROUPS * MT_WARPS * MT_MAX_STAGES];
-  uint64_t* full = full_s + cwarp * MT_MAX_STAGES;
 
   const int ntiles = (p.rows + MT_ROWS - 1) / MT_ROWS;
   const int nb = p.nblocks, cb = p.cb, np = p.npieces;
   // this warp's pieces in order: its group's tiles tile0, + tile_step, ...; of each the pieces warp, warp + 8, ...
-  int i_tile = tile0, i_blk = warp, issued = 0;  // i_blk counts pieces
-  auto issue_next = [&]() {  // all lanes; lanes 0..15 copy a row segment each
+  int i_tile = tile0, i_blk = warp, i_slot = 0;  // i_blk counts pieces
+  constexpr int MAXB = FMT == ILL_Q8_0 ? 8 : FMT == ILL_Q4_K ? 2 : 1;  // most blocks a piece
+  const int g = lane >> 2, t = lane & 3;
+  auto issue_next = [&]() {  // all lanes: four a row segment, eight rows at a time; a group of cp.async, possibly empty
     while (i_tile < ntiles && i_blk >= np) { i_tile += tile_step; i_blk = warp; }
-    if (i_tile >= ntiles) return;
-    const int s = issued % stages;
-    const int row = i_tile * MT_ROWS + lane;
-    uint32_t bytes = 0;
-    const u8* src = nullptr;
-    if (lane < MT_ROWS && row < p.rows) {
-      src = p.w + (long long)row * p.row_bytes + (long long)i_blk * cb * BB;
+    if (i_tile < ntiles) {
+      u8* st = ring + (size_t)i_slot * p.stage_bytes;
       const uint32_t len = (uint32_t)min(cb, nb - i_blk * cb) * BB;
-      bytes = (uint32_t)((((uintptr_t)src + len + 15) & ~(uintptr_t)15) - ((uintptr_t)src & ~(uintptr_t)15));
-    }
-    uint32_t total = bytes;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-    if (lane == 0) mbar_expect_tx(&full[s], total);
-    __syncwarp();
-    if (bytes) bulk_g2s(ring + (size_t)s * p.stage_bytes + (size_t)lane * p.pitch, (const void*)((uintptr_t)src & ~(uintptr_t)15), bytes, &full[s]);
-    ++issued;
-    i_blk += MT_WARPS;
+      for (int h = 0; h < MT_ROWS; h += 8) {
+        const int row = i_tile * MT_ROWS + h + g;
+        if (row < p.rows)
+          copy_segment<(MAXB * BB + 30) / 16>(st + (size_t)(h + g) * p.pitch, p.w + (long long)row * p.row_bytes + (long long)i_blk * cb * BB, len, t);
+      }
+      i_slot = i_slot + 1 == stages ? 0 : i_slot + 1;
+      i_blk += MT_WARPS;
+    }
+    cp_async_commit();
   };
-  if (lane == 0) {
-    for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
-    mbar_fence_init();
-  }
-  __syncwarp();
   for (int s = 0; s < stages; ++s) issue_next();  // the weights do not depend on the previous kernel
   pdl_launch_dependents();
   pdl_wait();
@@ -293,21 +281,21 @@ __global__ void __launch_bounds__(MT_GROUP_THREADS * MT_MAX_GROUPS) mvt_kernel(c
   MtX x;
   x.q = xq_s; x.stride = p.x_stride; x.s = xs_s; x.bs = bs_s; x.nsc = nsc; x.nbs = nbs; x.n = p.n;
 
-  const int g = lane >> 2;
-  int done = 0, it = 0;
-  bool dead = false;
+  int slot = 0, it = 0;
   for (int tile = tile0; tile < ntiles; tile += tile_step, ++it) {
     float acc[NT8][4];
 #pragma unroll
     for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[nt][i] = 0.0f;
-    for (int pc = warp; pc < np && !dead; pc += MT_WARPS) {
-      const int s = done % stages;
-      bool ok = mbar_wait(&full[s], (uint32_t)(done / stages) & 1u, p.status, ST_MV_WAIT + 0x20 + FMT);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) { dead = true; break; }
-      const u8* piece = ring + (size_t)s * p.stage_bytes;
+    for (int pc = warp; pc < np; pc += MT_WARPS) {
+      // all but the newer stages' groups: this piece is in
+      if (stages == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
+      else if (stages == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+      else asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncwarp();
+      const u8* piece = ring + (size_t)slot * p.stage_bytes;
+      slot = slot + 1 == stages ? 0 : slot + 1;
       // a row's segment starts where its block starts inside the 16-byte aligned span that was copied
       const long long o0 = (long long)(tile * MT_ROWS + g) * p.row_bytes + (long long)pc * cb * BB;
       const long long o8 = o0 + 8ll * p.row_bytes;
@@ -316,7 +304,6 @@ __global__ void __launch_bounds__(MT_GROUP_THREADS * MT_MAX_GROUPS) mvt_kernel(c
       const int nhere = min(cb, nb - pc * cb);
       for (int j = 0; j < nhere; ++j) MtBlock<FMT, NT8>::run(row0 + j * BB, row8 + j * BB, pc * cb + j, x, lane, acc);
       __syncwarp();
-      ++done;
       issue_next();
     }
     // the eight warps' partial sums meet: thread (row, token) adds them in warp order
@@ -325,24 +312,20 @@ __global__ void __launch_bounds__(MT_GROUP_THREADS * MT_MAX_GROUPS) mvt_kernel(c
     for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) mine[(g + 8 * (i >> 1)) * 16 + 8 * nt + 2 * (lane & 3) + (i & 1)] = acc[nt][i];
-    if (group_sync_or(grp, dead)) { dead = true; break; }
+    group_sync(grp);
     {
-      const int r = gtid >> 4, t = gtid & 15;
+      const int r = gtid >> 4, tk = gtid & 15;
       const long long row = (long long)tile * MT_ROWS + r;
-      if (t < p.n && row < p.rows) {
-        const float* all = part + (size_t)(it & 1) * MT_WARPS * 256 + r * 16 + t;
+      if (tk < p.n && row < p.rows) {
+        const float* all = part + (size_t)(it & 1) * MT_WARPS * 256 + r * 16 + tk;
         float v = 0.0f;
 #pragma unroll
         for (int w = 0; w < MT_WARPS; ++w) v = __fadd_rn(v, all[w * 256]);
         if (p.bias) v += p.bias[row];
-        float* yp = p.y + (long long)t * p.rows + row;
+        float* yp = p.y + (long long)tk * p.rows + row;
         *yp = p.acc ? *yp + v : v;
       }
     }
-  }
-  if (dead) {
-    // copies still in flight into this warp's stages get a bounded time to land before shared memory is released
-    for (int k = done + 1; k < issued; ++k) mbar_wait(&full[k % stages], (uint32_t)(k / stages) & 1u, nullptr, 0);
   }
 }
 
@@ -425,7 +408,6 @@ int mvt_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
   p.part_off = off;
   off += (uint32_t)p.groups * part_bytes;
   const size_t smem = off;
-  p.status = device_status_word();
   const int per_sm = (int)((227u * 1024u) / (smem + 1024u)) >= 2 ? 2 : 1;
   int grid = sms * per_sm;
   if (grid * p.groups > ntiles) grid = (ntiles + p.groups - 1) / p.groups;
