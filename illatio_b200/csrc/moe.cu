@@ -36,6 +36,27 @@ __global__ void __launch_bounds__(256) swiglu_w_kernel(long long n, int ff, floa
   const float wv = w ? w[i / ff] : 1.0f;
   mid[i] = __fmul_rn(__fmul_rn(__fmul_rn(gv, d4_sigmoid(gv)), uv), wv);
 }
+// The same, four values a thread, where G, U and MID lie on 16-byte boundaries and a row is a multiple of four: four
+// independent sigmoids a thread instead of one (777 x 4864 values: 15.6 -> 5.6 us, 4096 x 4096 69 -> 30, HBM's time).
+__global__ void __launch_bounds__(256) swiglu_w_vec_kernel(long long n, int ff, float clamp, const float4* __restrict__ g,
+                                                           const float4* __restrict__ u, const float* __restrict__ w,
+                                                           float4* __restrict__ mid) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (4 * i >= n) return;
+  const float4 g4 = g[i], u4 = u[i];
+  const float wv = w ? w[4 * i / ff] : 1.0f;
+  const float gs[4] = {g4.x, g4.y, g4.z, g4.w}, us[4] = {u4.x, u4.y, u4.z, u4.w};
+  float m[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float gv = gs[j], uv = us[j];
+    if (clamp > 1e-6f) { gv = fminf(gv, clamp); uv = fmaxf(-clamp, fminf(uv, clamp)); }
+    m[j] = __fmul_rn(__fmul_rn(__fmul_rn(gv, d4_sigmoid(gv)), uv), wv);
+  }
+  mid[i] = make_float4(m[0], m[1], m[2], m[3]);
+}
 
 // OUT = silu(G) * U with the gated product's own formula, g / (1 + exp(-g)), four values a thread (VEC: all three
 // pointers on 16-byte boundaries).  Bound by HBM: 12 bytes a value.
@@ -409,6 +430,9 @@ extern "C" int ill_swiglu_w(int64_t n, int ff, float clamp, ill_dptr g, ill_dptr
   const float *gp = (const float*)(uintptr_t)g, *up = (const float*)(uintptr_t)u, *wp = (const float*)(uintptr_t)w;
   float* mp = (float*)(uintptr_t)mid;
   void* args[] = {&nn, &ff, &clamp, &gp, &up, &wp, &mp};
+  if (((g | u | mid) & 15) == 0 && ff % 4 == 0 && n % 4 == 0)
+    return launch_kernel((const void*)swiglu_w_vec_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, args,
+                         (cudaStream_t)stream);
   return launch_kernel((const void*)swiglu_w_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, args,
                        (cudaStream_t)stream);
 }

@@ -24,6 +24,43 @@ __global__ void __launch_bounds__(256) quant_q8_0_kernel(const float* __restrict
   quant_block_q8_0(x[b * 32 + lane], lane, b, xq, xs, xsum, f16_scale);
 }
 
+// Four values of a Q8_0 block in each of its eight lanes (all 32 lanes take part; IN: the lane has values): the block's
+// maximum takes three shuffles for four blocks where a value a lane takes five for one, its bytes leave as a word a lane.
+// The same bits (a maximum and a sum of whole numbers do not depend on the order).  I4 numbers the fours from XQ's start.
+__device__ __forceinline__ void quant_four_q8_0(float4 v, bool in, long long i4, uint32_t* xq, float* xs, int* xsum, int f16_scale) {
+  float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float d = __fdiv_rn(amax, 127.0f);
+  const float id = d == 0.0f ? 0.0f : __fdiv_rn(1.0f, d);
+  const int q[4] = {__float2int_rn(__fmul_rn(v.x, id)), __float2int_rn(__fmul_rn(v.y, id)), __float2int_rn(__fmul_rn(v.z, id)),
+                    __float2int_rn(__fmul_rn(v.w, id))};
+  int t = q[0] + q[1] + q[2] + q[3];
+  if (xsum) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  }
+  if (!in) return;
+  xq[i4] = (uint32_t)(q[0] & 0xff) | (uint32_t)(q[1] & 0xff) << 8 | (uint32_t)(q[2] & 0xff) << 16 | (uint32_t)(q[3] & 0xff) << 24;
+  if ((threadIdx.x & 7) == 0) {
+    xs[i4 >> 3] = f16_scale ? __half2float(__float2half_rn(d)) : d;
+    if (xsum) xsum[i4 >> 3] = t;
+  }
+}
+
+// quant_q8_0_kernel where X and XQ lie on 16- and 4-byte boundaries.  A value a lane was bound by the issue of its divisions
+// and shuffles (777 x 4864 values 15.6 us, 4096 x 4096 68); four a lane are bound by memory (4.6 and 18 us).
+__global__ void __launch_bounds__(256) quant_q8_0_vec_kernel(const float4* __restrict__ x, uint32_t* __restrict__ xq,
+                                                             float* __restrict__ xs, int* __restrict__ xsum,
+                                                             long long nblocks, int f16_scale) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  const bool in = i < 8 * nblocks;
+  const float4 v = in ? x[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  quant_four_q8_0(v, in, i, xq, xs, xsum, f16_scale);
+}
+
 // A warp a super-block; lane l holds elements 8l .. 8l+7.  F16: also the block's fp16 forms (XH, XE).
 template <bool F16>
 __global__ void __launch_bounds__(256) quant_q8_k_kernel(const float* __restrict__ x, i8* __restrict__ xq,
@@ -47,45 +84,67 @@ __global__ void __launch_bounds__(256) quant_q8_k_kernel(const float* __restrict
 // row's scale out for itself (the row comes from L2) and takes a slice of its blocks, so that one token's
 // norm is not one CTA's serial work.  The double sum is taken in the order quantdev.cuh fixes, not in the
 // CPU loop's; the two agree until the float the sum is rounded to sits within 1e-16 of a rounding boundary.
-template <int K8K, bool F16>
+// Bound by latency: the norm's weights are on their way before the kernel waits for the row, a warp asks for four of its
+// groups and its first block's values at once, and a few rows are spread over their blocks too (16 rows of 2560: 3.9 -> 2.6 us; 4
+// of 5120 5.2 -> 2.9; one of 2560 3.1 -> 2.5).  VEC: Q8_0 blocks by four values a lane (X, W, H and XQ aligned for it).
+template <int K8K, bool F16, bool VEC>
 __global__ void __launch_bounds__(256) rmsnorm_q8_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                          float* __restrict__ h, i8* __restrict__ xq, float* __restrict__ xs,
                                                          void* __restrict__ xsum, int d, float eps, int f16_scale,
                                                          __half* __restrict__ xh, __half* __restrict__ xe) {
   __shared__ double group_s[RMS_MAX_GROUPS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // a unit is a warp's turn: a Q8_K block, a Q8_0 block, or (VEC) four Q8_0 blocks, the last unit perhaps fewer
+  constexpr int BW = K8K ? 256 : VEC ? 128 : 32, VL = BW / 32;  // a unit's values, a lane's
+  const int nb = (d + BW - 1) / BW, b0 = blockIdx.x * 8 + warp;
+  float wv[VL], x0[VL];  // of the warp's first block; the weights do not depend on the previous kernel
+  auto load = [&](const float* src, int b, float (&v)[VL]) {
+    if constexpr (K8K) rms_load8<false>(src, d, b * 256 + 8 * lane, v);
+    else if constexpr (VEC) {
+      const float4 f = b * 128 + 4 * lane < d ? ((const float4*)src)[b * 32 + lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    } else v[0] = src[b * 32 + lane];
+  };
+  if (b0 < nb) load(w, b0, wv);
   pdl_launch_dependents();
   pdl_wait();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long base = (long long)blockIdx.y * d;
   const float* xr = x + base;
+  if (b0 < nb) load(xr, b0, x0);
   const int ng = (d + 255) / 256;
-  for (int g = warp; g < ng; g += 8) {
-    float v[8];
-    rms_load8<false>(xr, d, g * 256 + 8 * lane, v);
-    const double s = rms_group_sum(v);
-    if (lane == 0) group_s[g] = s;
+  for (int g0 = warp; g0 < ng; g0 += 32) {
+    float v[4][8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (g0 + 8 * k < ng) rms_load8<false>(xr, d, (g0 + 8 * k) * 256 + 8 * lane, v[k]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (g0 + 8 * k < ng) {
+        const double s = rms_group_sum(v[k]);
+        if (lane == 0) group_s[g0 + 8 * k] = s;
+      }
   }
   __syncthreads();
   const float sc = rms_scale(rms_total(group_s, ng, lane), d, eps);
-  constexpr int BW = K8K ? 256 : 32;
-  const int nb = d / BW;
-  for (int b = blockIdx.x * 8 + warp; b < nb; b += gridDim.x * 8) {
-    const long long gb = base / BW + b;
-    if constexpr (K8K) {
-      float v[8];
+  for (int b = b0; b < nb; b += gridDim.x * 8) {
+    if (b != b0) { load(w, b, wv); load(xr, b, x0); }
+    float v[VL];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int i = b * 256 + 8 * lane + j;
-        v[j] = __fmul_rn(__fmul_rn(xr[i], sc), w[i]);
-        if (h) h[base + i] = v[j];
-      }
-      if constexpr (F16) quant_block_q8_k_f16(v, lane, gb, xq, xs, (int16_t*)xsum, xh, xe);
-      else quant_block_q8_k(v, lane, gb, xq, xs, (int16_t*)xsum);
+    for (int j = 0; j < VL; ++j) v[j] = __fmul_rn(__fmul_rn(x0[j], sc), wv[j]);
+    const long long at = base + (long long)b * BW + VL * lane;  // the lane's first value
+    if constexpr (VEC) {
+      const bool in = b * 128 + 4 * lane < d;
+      const float4 f = make_float4(v[0], v[1], v[2], v[3]);
+      if (h && in) *(float4*)(h + at) = f;
+      quant_four_q8_0(f, in, at / 4, (uint32_t*)xq, xs, (int*)xsum, f16_scale);
     } else {
-      const int i = b * 32 + lane;
-      const float v = __fmul_rn(__fmul_rn(xr[i], sc), w[i]);
-      if (h) h[base + i] = v;
-      quant_block_q8_0(v, lane, gb, xq, xs, (int*)xsum, f16_scale);
+      if (h)
+#pragma unroll
+        for (int j = 0; j < VL; ++j) h[at + j] = v[j];
+      const long long gb = base / BW + b;
+      if constexpr (!K8K) quant_block_q8_0(v[0], lane, gb, xq, xs, (int*)xsum, f16_scale);
+      else if constexpr (F16) quant_block_q8_k_f16(v, lane, gb, xq, xs, (int16_t*)xsum, xh, xe);
+      else quant_block_q8_k(v, lane, gb, xq, xs, (int16_t*)xsum);
     }
   }
 }
@@ -116,6 +175,9 @@ extern "C" int ill_quant_q8_0(ill_dptr x, ill_dptr xq, ill_dptr xs, ill_dptr xsu
   int* sump = (int*)(uintptr_t)xsum;
   long long nb = nblocks;
   void* args[] = {&xp, &qp, &sp, &sump, &nb, &f16_scale};
+  if (((x & 15) | (xq & 3)) == 0)
+    return launch_kernel((const void*)quant_q8_0_vec_kernel, dim3((unsigned)((nblocks + 31) / 32)), dim3(256), 0, args,
+                         (cudaStream_t)stream);
   return launch_kernel((const void*)quant_q8_0_kernel, dim3((unsigned)((nblocks + 7) / 8)), dim3(256), 0, args,
                        (cudaStream_t)stream);
 }
@@ -177,11 +239,12 @@ static int rmsnorm_q8_launch(int kind, ill_dptr x, ill_dptr w, ill_dptr h, ill_d
   void* bp = (void*)(uintptr_t)xsum;
   __half *fhp = (__half*)(uintptr_t)xh, *fep = (__half*)(uintptr_t)xe;
   void* args[] = {&xp, &wp, &hp, &qp, &sp, &bp, &d, &eps, &f16_scale, &fhp, &fep};
-  // a single row is spread over its blocks; many rows take a CTA each
-  const int nb = d / bw;
-  const unsigned slices = n == 1 ? (unsigned)((nb + 7) / 8) : 1u;
-  const void* k = kind == 1 ? (xh ? (const void*)rmsnorm_q8_kernel<1, true> : (const void*)rmsnorm_q8_kernel<1, false>)
-                            : (const void*)rmsnorm_q8_kernel<0, false>;
+  // few rows are spread over their blocks, as far as two CTAs an SM (148) go; many rows take a CTA each
+  const bool vec = kind == 0 && ((x | w | h) & 15) == 0 && (xq & 3) == 0;
+  const int nb = vec ? (d + 127) / 128 : d / bw, most = n < 296 ? (int)(296 / n) : 1;
+  const unsigned slices = (unsigned)((nb + 7) / 8 < most ? (nb + 7) / 8 : most);
+  const void* k = kind == 1 ? (xh ? (const void*)rmsnorm_q8_kernel<1, true, false> : (const void*)rmsnorm_q8_kernel<1, false, false>)
+                            : vec ? (const void*)rmsnorm_q8_kernel<0, false, true> : (const void*)rmsnorm_q8_kernel<0, false, false>;
   return launch_kernel(k, dim3(slices, (unsigned)n), dim3(256), 0, args, (cudaStream_t)stream);
 }
 

@@ -83,6 +83,37 @@ def test_rmsnorm_q8_matches_oracle(oracle, kind, d, n):
     assert np.array_equal(act.xs.cpu().numpy().view(np.uint32), s.view(np.uint32))
 
 
+@pytest.mark.parametrize("kind,d,n,off", [("q8", 32, 1, 0), ("q8", 160, 2, 0), ("q8", 4864, 17, 0), ("q8", 4864, 300, 0), ("q8", 896, 3, 1),
+                                          ("q8k", 256, 1, 0), ("q8k", 8448, 2, 0), ("q8k", 2560, 16, 1), ("q8k", 17408, 300, 0)])
+def test_norm_quantizer_and_swiglu_at_any_split_and_alignment(oracle, kind, d, n, off):
+    """Rows split over CTAs and not, vectors on 16-byte boundaries and (OFF floats past one) not: bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(d + n)
+    def dev(*shape):
+        k = int(np.prod(shape))
+        return torch.randn(k + off, device="cuda", generator=g)[off:].reshape(*shape)
+    x, w, h = dev(n, d), dev(d), dev(n, d)
+    act = D.make_qact(n * d, kind, want_xsum=True)
+    D.rmsnorm_q8(x, w, act, d, 1e-6, n, h=h)
+    quantize = oracle.quantize_q8_0 if kind == "q8" else oracle.quantize_q8k
+    want = np.stack([oracle.rmsnorm(r, w.cpu().numpy(), 1e-6) for r in x.cpu().numpy()])
+    assert np.array_equal(h.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    q, s = quantize(want)[:2]
+    assert np.array_equal(act.xq.cpu().numpy(), q)
+    assert np.array_equal(act.xs.cpu().numpy().view(np.uint32), s.view(np.uint32))
+    if kind == "q8":
+        again = D.make_qact(n * d, kind, want_xsum=True)
+        D.quant_q8(h.reshape(-1), again, f16_scale=False)
+        q, s = quantize(want, f16_scale=False)
+        assert np.array_equal(again.xq.cpu().numpy(), q)
+        assert np.array_equal(again.xs.cpu().numpy().view(np.uint32), s.view(np.uint32))
+        assert np.array_equal(again.xsum.cpu().numpy(), q.reshape(-1, 32).astype(np.int32).sum(1))
+    # the aligned and the unaligned form of one SwiGLU
+    a, b = dev(n, d), torch.empty(n * d + 1, device="cuda")[1:].reshape(n, d)
+    D.swiglu(x, h, a, d, clamp=1.5)
+    D.swiglu(x, h, b, d, clamp=1.5)
+    assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
 @pytest.mark.parametrize("fmt", FMTS)
 def test_dequant_rows_bit_exact_golden(fmt):
     z = np.load(os.path.join(GOLD, "dequant_%s.npz" % B.NAMES[fmt]))
