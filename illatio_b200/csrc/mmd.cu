@@ -645,7 +645,9 @@ __global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
   for (int k = 0; warp + MD_WARPS * k < nsteps; ++k) {
     const int step = warp + MD_WARPS * k;
     fill_x(k + 1);                                          // the other buffer: its readers are through (the __syncwarp below)
-    asm volatile("cp.async.wait_group 2;" ::: "memory");   // all but that group and the next-but-one step's weights: step k is in
+    // step k is in: all but that group and, after the first step, the weights asked for at the end of the last one
+    if (k == 0) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 2;" ::: "memory");
     __syncwarp();
     const int s = k % MD_MAX_STAGES;
     MdFrag<FMT> f;
