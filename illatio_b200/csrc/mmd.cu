@@ -44,6 +44,7 @@ struct MdParams {
   uint32_t xbuf_bytes, xs_off, xsum_off;  // one activation buffer: its size, where its scales and (Q4_K) sums start
   uint32_t ring_off, part_off;
   unsigned* status;
+  uint64_t neg_zeros;    // two floats -0.0 (mmq8_kernel)
 };
 
 // four 8 x 16-byte matrices of shared memory -> each lane its four bytes of row lane / 4 of each: lane l gives the
@@ -352,34 +353,34 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
 // ---- Q8_0 chunks ---------------------------------------------------------------------------------------------
 // What bounds a Q8_0 chunk is not the tensor pipe but what every m16n8k32 product needs after it: its four integers
 // become floats and meet d_w * d_x, because Q8_0's scales are per 32 columns on both sides.  So the kernel is built
-// around those instructions -- four conversions, two packed multiplies and two packed fused multiply-adds
-// (fma.rn.f32x2: each half rounds as the scalar instruction does) a product -- and keeps everything else off the
-// issue slots:
+// around those instructions -- four conversions, four packed multiplies and two packed additions (f32x2) a product -- and keeps everything else off the issue slots:
 //   * columns in steps of 128 (four blocks; a row's step is 136 bytes), weights and activations both by 16-byte
-//     cp.async into a ring of two or three stages, one __syncthreads a step;
+//     cp.async into a ring of three stages, one __syncthreads a step;
 //   * what a thread copies lies at fixed distances from one step to the next: a step's copies are an add and a few
 //     predicates beside the copies themselves;
 //   * the activations' scales are staged in the order a lane reads them: the four of a token pair's two blocks are one
 //     16-byte load for two products;
-//   * two blocks of weights sit in registers at a time (mmd_kernel holds eight): 80 tokens a CTA fit 128 registers and
-//     two CTAs share an SM.
-// A CTA of eight warps takes 16 RW rows x 8 NT8 tokens; with RW < 8 the warps are 8 / RW groups that take every
-// (8 / RW)-th step each and meet in shared memory in group order (few rows of many columns).
+//   * two blocks of weights sit in registers at a time (mmd_kernel holds a step's): 80 tokens a CTA fit 128 registers, and
+//     sixteen warps an SM.
+// A CTA of RW warps takes 16 RW rows x 8 NT8 tokens; few rows of many columns take small CTAs, several an SM.  A row's
+// blocks are added in order, each step rounded as in mmd_kernel: the same bits as it gave, whatever the tile.
 //
-// Measured against mmd_kernel, which took Q8_0 before: 2048 x 4096 x 4096 tokens 412 -> 277 us (248 int8 TOPS), 5120 x 1536
-// x 8192 728 -> 492, 4864 x 896 x 777 58 -> 36, 896 x 4864 x 777 129 -> 48, 2048 x 4096 x 64 62 -> 14, 896 x 4864 x 17
-// 64 -> 9.  What is left: about 23 cycles a product of a scheduler where the packed arithmetic alone takes 8 and the int8
-// mma.sync 8.2, and 1.1 us a step for unpacking, copying and the barrier.  Measured and dropped: 32 rows a warp (half the
-// ldmatrix traffic, the same time), the integers turned into floats by adding 1.5 * 2^23 in the product (4 % slower).
+// Measured against mmd_kernel, which took Q8_0 before: 2048 x 4096 x 4096 tokens 412 -> 298 us (231 int8 TOPS), 5120 x 1536
+// x 8192 728 -> 529, 4864 x 896 x 777 58 -> 39, 896 x 4864 x 777 129 -> 68, 2048 x 4096 x 64 62 -> 25.  What is left: about
+// 23 cycles a product of a scheduler where the packed arithmetic alone takes 12 and the int8 mma.sync 8.2, and 1.1 us a step
+// for unpacking, copying and the barrier.  Measured and dropped: 32 rows a warp (half the ldmatrix traffic, the same time);
+// the integers turned into floats by adding 1.5 * 2^23 in the product (4 % slower); the columns dealt to groups of a CTA's
+// warps (896 x 4864 x 777 in 40 us, but sums in another order: after a few layers' 8-bit activations that is a difference
+// of 1 % in a model's output); fused multiply-adds (5 % faster, other bits).
 template <int NT8, int RW>
 struct Mq {
-  static constexpr int TN = 8 * NT8, KS = MD_WARPS / RW;
+  static constexpr int TN = 8 * NT8, THREADS = 32 * RW;
   static constexpr int WPITCH = 176;  // ten chunks of 16 bytes a row's step; 44 words: eight rows x four words on 32 banks
   static constexpr int XPITCH = 144;  // 36 words: ldmatrix's eight rows on 32 banks
-  static constexpr int W_BYTES = MD_WARPS * 16 * WPITCH, X_BYTES = KS * TN * XPITCH, S_BYTES = KS * TN * 16;
+  static constexpr int W_BYTES = RW * 16 * WPITCH, X_BYTES = TN * XPITCH, S_BYTES = TN * 16;
   static constexpr int STAGE = W_BYTES + X_BYTES + S_BYTES;
-  static constexpr int TWO_CTAS = 233472 / 2 - 1024;  // shared memory a CTA may have for two to share an SM
-  static constexpr int PER_SM = 2 * STAGE <= TWO_CTAS ? 2 : 1, STAGES = PER_SM == 2 && 3 * STAGE > TWO_CTAS ? 2 : 3;
+  // CTAs an SM: sixteen warps of 128 registers, or what its shared memory holds
+  static constexpr int FIT = 233472 / (3 * STAGE + 1024), PER_SM = FIT < 16 / RW ? FIT : 16 / RW;
 };
 
 __device__ __forceinline__ uint64_t md_mul2(uint64_t a, uint64_t b) {
@@ -387,9 +388,14 @@ __device__ __forceinline__ uint64_t md_mul2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-__device__ __forceinline__ void md_fma2(uint64_t& d, uint64_t a, uint64_t b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+// A product rounded by itself: a * b + -0.0, with a -0.0 that the compiler does not know.  (It joins a mul.rn.f32x2 and the
+// add.rn.f32x2 after it into one fused instruction, .rn or not: other bits than the CPU's two roundings.)
+__device__ __forceinline__ uint64_t md_mul2_rounded(uint64_t a, uint64_t b, uint64_t neg_zeros) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(neg_zeros));
+  return d;
 }
+__device__ __forceinline__ void md_add2(uint64_t& d, uint64_t a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(a)); }
 __device__ __forceinline__ uint64_t md_pack(float a, float b) {
   uint64_t d;
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
@@ -397,32 +403,31 @@ __device__ __forceinline__ uint64_t md_pack(float a, float b) {
 }
 
 template <int NT8, int RW>
-__global__ void __launch_bounds__(MD_THREADS, 2) mmq8_kernel(const MdParams p) {
+__global__ void __launch_bounds__(Mq<NT8, RW>::THREADS, Mq<NT8, RW>::PER_SM) mmq8_kernel(const MdParams p) {
   extern __shared__ __align__(128) u8 smem[];
   using C = Mq<NT8, RW>;
-  constexpr int TN = C::TN, KS = C::KS;
+  constexpr int TN = C::TN;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int rw = warp % RW, kg = warp / RW;
   const int ntt = (p.n + TN - 1) / TN;
-  const int tok0 = (int)(blockIdx.x % ntt) * TN, row_base = (int)(blockIdx.x / ntt) * (16 * RW) + rw * 16;
-  const int nsteps = p.nsteps, nit = (nsteps + KS - 1) / KS;
+  const int tok0 = (int)(blockIdx.x % ntt) * TN, row_base = (int)(blockIdx.x / ntt) * (16 * RW) + warp * 16;
+  const int nsteps = p.nsteps;
   const bool live = row_base < p.rows;  // a warp whose rows are all past the end only helps to bring the activations
   const u8* wrow0 = p.w + (long long)row_base * p.row_bytes;
 
   // Weights: four lanes a row, chunks lane % 4, + 4 and + 8 of its 16-byte aligned span (nine or ten chunks).
-  const u8* wsrc = wrow0 + (long long)g * p.row_bytes + (long long)kg * 136;  // row g's bytes of the step copied next
+  const u8* wsrc = wrow0 + (long long)g * p.row_bytes;  // row g's bytes of the step copied next
   const long long w8 = 8ll * p.row_bytes;
   const bool in0 = live && row_base + g < p.rows, in8 = live && row_base + g + 8 < p.rows;
   const uint32_t wdst = (uint32_t)((warp * 16 + g) * C::WPITCH + 16 * t);
-  // Activations: eight threads a token's 128 quants, 32 tokens at a time; a thread a scale.
-  constexpr int XJ = (TN + 31) / 32, SJ = (TN * 4 + MD_THREADS - 1) / MD_THREADS;
+  // Activations: eight threads a token's 128 quants, XT tokens at a time; a thread a scale, ST tokens at a time.
+  constexpr int XT = C::THREADS / 8, ST = C::THREADS / 4, XJ = (TN + XT - 1) / XT, SJ = (TN + ST - 1) / ST;
   const int xtk = tid >> 3, stk = tid >> 2;
   const i8* xsrc = p.xq + (long long)(tok0 + xtk) * p.cols + 16 * (tid & 7);
   const float* ssrc = p.xs + (long long)(tok0 + stk) * (p.cols / 32) + (tid & 3);
   const uint32_t xdst = (uint32_t)(C::W_BYTES + xtk * C::XPITCH + 16 * (tid & 7));
   // scale of token 2 j + h, block 2 b + o of the step -> float [b][j][o][h]
   const uint32_t sdst = (uint32_t)(C::W_BYTES + C::X_BYTES + 4 * ((((tid & 3) >> 1) * (TN / 2) + (stk >> 1)) * 4 + 2 * (tid & 1) + (stk & 1)));
-  int w_step = kg, x_step = 0;  // the steps copied next
+  int w_step = 0, x_step = 0;  // the steps copied next
   auto fill_w = [&](u8* st) {
     if (w_step < nsteps) {
       auto row = [&](const u8* src, u8* dst) {
@@ -434,48 +439,42 @@ __global__ void __launch_bounds__(MD_THREADS, 2) mmq8_kernel(const MdParams p) {
       if (in0) row(wsrc, st + wdst);
       if (in8) row(wsrc + w8, st + wdst + 8 * C::WPITCH);
     }
-    wsrc += KS * 136;
-    w_step += KS;
+    wsrc += 136;
+    ++w_step;
   };
   auto fill_x = [&](u8* st) {
+    if (x_step < nsteps) {
 #pragma unroll
-    for (int ks = 0; ks < KS; ++ks) {
-      if (x_step + ks < nsteps) {
+      for (int j = 0; j < XJ; ++j)
+        if ((TN % XT == 0 || XT * j + xtk < TN) && tok0 + XT * j + xtk < p.n)
+          cp_async16(st + xdst + XT * j * C::XPITCH, xsrc + (long long)XT * j * p.cols);
 #pragma unroll
-        for (int j = 0; j < XJ; ++j)
-          if ((TN % 32 == 0 || 32 * j + xtk < TN) && tok0 + 32 * j + xtk < p.n)
-            cp_async16(st + xdst + (ks * TN + 32 * j) * C::XPITCH, xsrc + 128 * ks + 32ll * j * p.cols);
-#pragma unroll
-        for (int j = 0; j < SJ; ++j)
-          if ((TN % 64 == 0 || 64 * j + stk < TN) && tok0 + 64 * j + stk < p.n)
-            cp_async4(st + sdst + ks * TN * 16 + 512 * j, ssrc + 4 * ks + 2ll * j * p.cols);
-      }
+      for (int j = 0; j < SJ; ++j)
+        if ((TN % ST == 0 || ST * j + stk < TN) && tok0 + ST * j + stk < p.n)
+          cp_async4(st + sdst + 8 * ST * j, ssrc + (long long)ST * j * (p.cols / 32));
     }
-    xsrc += 128 * KS;
-    ssrc += 4 * KS;
-    x_step += KS;
+    xsrc += 128;
+    ssrc += 4;
+    ++x_step;
   };
 
   fill_w(smem);  // the weights do not depend on the previous kernel
-  if (p.stages == 3) fill_w(smem + C::STAGE);
+  fill_w(smem + C::STAGE);
   pdl_launch_dependents();
   pdl_wait();
   fill_x(smem);
   cp_async_commit();
-  if (p.stages == 3) {
-    fill_x(smem + C::STAGE);
-    cp_async_commit();
-  }
+  fill_x(smem + C::STAGE);
+  cp_async_commit();
 
   uint64_t acc[NT8][2];  // [tile of eight tokens][row g / g + 8]: tokens 2 t and 2 t + 1
 #pragma unroll
   for (int nt = 0; nt < NT8; ++nt) acc[nt][0] = acc[nt][1] = 0ull;
   const bool even_off = ((uintptr_t)p.w & 2) == 0;  // a row is a multiple of four bytes: which blocks' quants are word-aligned
-  const uint32_t last = (uint32_t)(p.stages - 1) * C::STAGE;
-  uint32_t use_at = 0, fill_at = last, w_off = (uint32_t)(uintptr_t)wrow0 + (uint32_t)g * p.row_bytes + 136u * kg;
-  for (int it = 0; it < nit; ++it) {
-    if (p.stages == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");  // this iteration's copies are in
-    else cp_async_wait_all();
+  constexpr uint32_t last = 2 * C::STAGE;
+  uint32_t use_at = 0, fill_at = last, w_off = (uint32_t)(uintptr_t)wrow0 + (uint32_t)g * p.row_bytes;
+  for (int step = 0; step < nsteps; ++step) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");  // all but the newest: this step's copies are in
     __syncthreads();  // ... everyone's; and everyone is through with the stage refilled next
     fill_w(smem + fill_at);
     fill_x(smem + fill_at);
@@ -484,12 +483,12 @@ __global__ void __launch_bounds__(MD_THREADS, 2) mmq8_kernel(const MdParams p) {
     use_at = use_at == last ? 0 : use_at + C::STAGE;
     fill_at = fill_at == last ? 0 : fill_at + C::STAGE;
     const uint32_t o0 = w_off;
-    w_off += KS * 136;
-    if (!live || it * KS + kg >= nsteps) continue;
+    w_off += 136;
+    if (!live) continue;
     const u8* r0 = st + (warp * 16 + g) * C::WPITCH + (o0 & 15);
     const u8* r8 = st + (warp * 16 + g + 8) * C::WPITCH + ((o0 + 8u * p.row_bytes) & 15);
-    const u8* xl = st + C::W_BYTES + (kg * TN + (lane & 7)) * C::XPITCH + 16 * (lane >> 3);
-    const u8* sl = st + C::W_BYTES + C::X_BYTES + kg * TN * 16 + 16 * t;
+    const u8* xl = st + C::W_BYTES + (lane & 7) * C::XPITCH + 16 * (lane >> 3);
+    const u8* sl = st + C::W_BYTES + C::X_BYTES + 16 * t;
 #pragma unroll
     for (int b2 = 0; b2 < 2; ++b2) {  // blocks 2 b2 and 2 b2 + 1 of the step
       uint32_t a[2][4];
@@ -521,8 +520,8 @@ __global__ void __launch_bounds__(MD_THREADS, 2) mmq8_kernel(const MdParams p) {
           int c[4];
           mma_k32_s8(c, a[o], x[2 * o], x[2 * o + 1]);
           // Q8-ROW-DOT-AT: sum += float(isum) * (d_w * d_x)
-          md_fma2(acc[nt][0], md_pack((float)c[0], (float)c[1]), md_mul2(d0[o], xs));
-          md_fma2(acc[nt][1], md_pack((float)c[2], (float)c[3]), md_mul2(d8[o], xs));
+          md_add2(acc[nt][0], md_mul2_rounded(md_pack((float)c[0], (float)c[1]), md_mul2(d0[o], xs), p.neg_zeros));
+          md_add2(acc[nt][1], md_mul2_rounded(md_pack((float)c[2], (float)c[3]), md_mul2(d8[o], xs), p.neg_zeros));
         }
       }
     }
@@ -532,25 +531,6 @@ __global__ void __launch_bounds__(MD_THREADS, 2) mmq8_kernel(const MdParams p) {
   for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
     for (int i = 0; i < 2; ++i) asm("mov.b64 {%0, %1}, %2;" : "=f"(v[nt][2 * i]), "=f"(v[nt][2 * i + 1]) : "l"(acc[nt][i]));
-  if constexpr (KS > 1) {  // the groups' partial sums meet in the first group's warps, in group order
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    float* part = (float*)smem;  // [group - 1][row warp][value][lane]
-    static_assert((KS - 1) * RW * NT8 * 4 * 32 * 4 <= 2 * C::STAGE, "");
-    if (kg > 0)
-#pragma unroll
-      for (int nt = 0; nt < NT8; ++nt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) part[((((kg - 1) * RW + rw) * NT8 + nt) * 4 + i) * 32 + lane] = v[nt][i];
-    __syncthreads();
-    if (kg > 0) return;
-#pragma unroll
-    for (int k = 0; k < KS - 1; ++k)
-#pragma unroll
-      for (int nt = 0; nt < NT8; ++nt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[nt][i] = __fadd_rn(v[nt][i], part[(((k * RW + rw) * NT8 + nt) * 4 + i) * 32 + lane]);
-  }
   if (!live) return;
 #pragma unroll
   for (int nt = 0; nt < NT8; ++nt)
@@ -709,47 +689,48 @@ static int mmd_launch(const MdParams& p, int tn, size_t smem, int grid, cudaStre
   return launch_kernel(k, dim3(grid), dim3(32 * p.warps), smem, args, st);
 }
 
-// The launch of a Q8_0 chunk.  Which tile: the one with the least of (steps a CTA goes through) x (CTAs one after
-// another on an SM) x (time a step).  STEP is that time in us with two CTAs on an SM (alone on it a CTA takes about
-// 0.65 of it), or with the one that fits, measured on 2048 x 4096 x 4096 tokens.  Over 20 shapes of 17 to 8192 tokens the
-// tile that it picks is the fastest measured or within 12 % of it (128 x 896 x 777: 9 us against 6.4).
+// The launch of a Q8_0 chunk.  Which tile: the one with the least estimated time, steps x (time a step) x (how often the
+// SMs are filled).  STEP is the time in us of a step with every SM full, measured on 2048 x 4096 x 4096 tokens.  CTAs that do
+// not fill the SMs take less of it, but not in proportion: what counts, over every tile, is how many warps the GPU holds --
+// 0.4 of STEP up to 256 warps, 0.55 at 512, 0.8 at 640, all of it at 2368 (sixteen an SM).  Over 20 shapes of 17 to 8192
+// tokens the tile it picks is the fastest measured or within 9 % of it (896 x 4864 x 17 tokens: 28 us against 23).
 struct MqTile {
   float step;
-  int rn, tn, ks, per_sm, stages;
-  uint32_t stage;
+  int rn, tn, threads, per_sm;
+  uint32_t smem;
   const void* kernel;
 };
 template <int NT8, int RW>
 static MqTile mq_tile(float step) {
   using C = Mq<NT8, RW>;
-  return {step, 16 * RW, C::TN, C::KS, C::PER_SM, C::STAGES, (uint32_t)C::STAGE, (const void*)mmq8_kernel<NT8, RW>};
+  return {step, 16 * RW, C::TN, C::THREADS, C::PER_SM, 3u * C::STAGE, (const void*)mmq8_kernel<NT8, RW>};
 }
 
 static int mmq8_launch(MdParams p, int sms, cudaStream_t st) {
   static const MqTile tiles[] = {
-      mq_tile<4, 8>(1.91f), mq_tile<4, 4>(2.05f), mq_tile<4, 2>(2.33f), mq_tile<4, 1>(2.03f),
-      mq_tile<6, 8>(2.39f), mq_tile<6, 4>(2.49f), mq_tile<6, 2>(2.84f),
-      mq_tile<8, 8>(2.67f), mq_tile<8, 4>(2.92f), mq_tile<8, 2>(2.24f),
-      mq_tile<10, 8>(3.08f), mq_tile<10, 4>(3.42f), mq_tile<10, 2>(2.56f),
+      mq_tile<4, 4>(1.78f), mq_tile<4, 2>(1.66f), mq_tile<6, 4>(2.19f), mq_tile<6, 2>(1.70f),
+      mq_tile<8, 4>(2.17f), mq_tile<10, 8>(3.13f), mq_tile<10, 4>(2.49f),
   };
   p.nsteps = p.cols / 128;
+  p.neg_zeros = 0x8000000080000000ull;
   const MqTile* best = nullptr;
   double best_us = 0.0;
   long long grid = 0;
   for (const MqTile& t : tiles) {
-    const long long ctas = (long long)((p.rows + t.rn - 1) / t.rn) * ((p.n + t.tn - 1) / t.tn);
-    const long long full = ctas / ((long long)t.per_sm * sms), rest = ctas % ((long long)t.per_sm * sms);
-    const double waves = (double)full + (rest == 0 ? 0.0 : t.per_sm == 2 && rest <= sms ? 0.65 : 1.0);
-    const double us = waves * ((p.nsteps + t.ks - 1) / t.ks) * t.step;
+    const long long ctas = (long long)((p.rows + t.rn - 1) / t.rn) * ((p.n + t.tn - 1) / t.tn), fit = (long long)t.per_sm * sms;
+    const double warps = (double)(ctas % fit) * (t.threads / 32);  // of the last, partial filling
+    double last = 0.0;
+    if (warps > 640.0) last = warps < 2368.0 ? 0.8 + 0.2 * (warps - 640.0) / 1728.0 : 1.0;
+    else if (warps > 512.0) last = 0.55 + 0.25 * (warps - 512.0) / 128.0;
+    else if (warps > 0.0) last = warps > 256.0 ? 0.4 + 0.15 * (warps - 256.0) / 256.0 : 0.4;
+    const double us = t.step * p.nsteps * ((double)(ctas / fit) + last);
     if (!best || us < best_us) { best = &t; best_us = us; grid = ctas; }
   }
   if (grid > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
-  p.stages = grid <= sms ? 3 : best->stages;  // a CTA that has the SM to itself has room for three
-  const size_t smem = (size_t)p.stages * best->stage;
-  cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(3 * best->stage));
+  cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best->smem);
   if (e != cudaSuccess) return cuda_fail(e);
   void* args[] = {&p};
-  return launch_kernel(best->kernel, dim3((unsigned)grid), dim3(MD_THREADS), smem, args, st);
+  return launch_kernel(best->kernel, dim3((unsigned)grid), dim3((unsigned)best->threads), best->smem, args, st);
 }
 
 // The chunk product on the tensor cores, for the formats and layouts it is written for; ILL_ERR_UNSUPPORTED

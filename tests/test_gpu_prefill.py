@@ -54,8 +54,8 @@ def test_chunk_product_equals_token_by_token(fmt, rows, cols, n):
     (300, 640, 385, 10), (2048, 4096, 65, 0), (4864, 896, 777, 8), (5121, 256, 400, 4),
 ])
 def test_q8_0_chunk_tiles(rows, cols, n, base):
-    """Q8_0's chunk kernel at the edges of its tiles (32 to 80 tokens, 16 to 128 rows, columns dealt to one to eight groups
-    of warps), blocks at every 2-byte alignment, with a bias, adding to Y: against the one-token product."""
+    """Q8_0's chunk kernel at the edges of its tiles (32 to 80 tokens, 32 to 128 rows), blocks at even alignments, with a
+    bias, adding to Y: against the one-token product."""
     nbytes = B.matrix_bytes(B.Q8_0, rows, cols)
     buf = torch.zeros(nbytes + 32, dtype=torch.uint8, device="cuda")
     buf[base:base + nbytes] = B.synth_matrix_torch(B.Q8_0, rows, cols, seed=rows)
@@ -72,6 +72,23 @@ def test_q8_0_chunk_tiles(rows, cols, n, base):
         want[t * rows:(t + 1) * rows] += one + bias
     # the same integers; cols / 32 float terms added in another order: a few units of 2^-24 of the largest sum
     assert (y - want).abs().max().item() < 2e-6 * max(top, want.abs().max().item())
+
+
+@pytest.mark.parametrize("rows,cols,n", [(40, 256, 33), (129, 384, 100), (300, 2048, 161)])
+def test_q8_0_chunk_adds_a_rows_blocks_in_order(rows, cols, n):
+    """Bit for bit: every block's float(sum) * (d_w * d_x), each step rounded, added in the row's order whatever the tile."""
+    w, x, act = _case(B.Q8_0, rows, cols, n)
+    y = torch.empty(n * rows, device="cuda")
+    D.cmat_mul(w, act, y, n)
+    nb = cols // 32
+    blk = w.qs[:rows * nb * 34].cpu().numpy().reshape(rows, nb, 34)
+    d = blk[:, :, :2].copy().view(np.float16)[:, :, 0].astype(np.float32)
+    q = blk[:, :, 2:].copy().view(np.int8).astype(np.int32)
+    xq, xs = act.xq.cpu().numpy()[:n * cols].reshape(n, nb, 32).astype(np.int32), act.xs.cpu().numpy()[:n * nb].reshape(n, nb)
+    want = np.zeros((n, rows), np.float32)
+    for b in range(nb):
+        want += (xq[:, b] @ q[:, b].T).astype(np.float32) * (d[None, :, b] * xs[:, b, None])
+    assert np.array_equal(y.cpu().numpy().reshape(n, rows).view(np.uint32), want.view(np.uint32))
 
 
 @pytest.mark.parametrize("fmt", [B.Q8_0, B.Q4_K, B.Q6_K])
