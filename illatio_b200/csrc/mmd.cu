@@ -7,7 +7,7 @@
 // against all TN tokens, so a block of weights is unpacked into tensor-core fragments once and used TN / 8 times
 // from registers.  The columns go by in steps of 256:
 //   * weights: every warp runs its own ring of stages, lanes 0..15 each copying one row's 256 columns of blocks
-//     (144 / 210 / 272 bytes, widened to 16-byte boundaries) with cp.async.bulk onto the stage's mbarrier; a stage
+//     (144 / 210 bytes, widened to 16-byte boundaries) with cp.async.bulk onto the stage's mbarrier; a stage
 //     is free again as soon as its block sits in registers, so the next copy is issued before the arithmetic;
 //   * activations: the step's TN x 256 quants and their scales are brought by all threads with cp.async into one
 //     of two buffers while the other is being used -- one __syncthreads a step; a token tile's quants reach the
