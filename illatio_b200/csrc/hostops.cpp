@@ -11,6 +11,7 @@
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/illatio_b200.h"
@@ -30,6 +31,11 @@ NAMES(DECL)
 #undef DECL
 
 struct Failed {};  // a Python error is set
+// What ends every operator: no C++ exception may reach the interpreter's C frames.  Tensors without storage (sparse, inside
+// vmap) and a stream that cannot be had throw c10::Error, which becomes the exception that torch's Python functions raise.
+#define CATCH_ERRORS                                                                                       \
+  catch (const Failed&) { return nullptr; }                                                                \
+  catch (...) { torch::translate_exception_to_python(std::current_exception()); return nullptr; }
 
 inline ill_stream cur_stream() { return (ill_stream)c10::cuda::getCurrentCUDAStream().stream(); }
 
@@ -167,7 +173,7 @@ PyObject* quant_q8(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject*
   if (act.k) check("ill_quant_q8_k", ill_quant_q8_k(xp, act.xq, act.xs, act.xsum, x.numel() / 256, cur_stream()));
   else check("ill_quant_q8_0", ill_quant_q8_0(xp, act.xq, act.xs, act.xsum, x.numel() / 32, OPT_BOOL(a[2], 1), cur_stream()));
   return ret(a[1]);
-} catch (const Failed&) { return nullptr; }
+} CATCH_ERRORS
 
 PyObject* rmsnorm_q8(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
   ARGS("rmsnorm_q8", 5, S_x, S_w, S_act, S_d, S_eps, S_n, S_h, S_f16_scale);
@@ -176,7 +182,7 @@ PyObject* rmsnorm_q8(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObjec
   check("ill_rmsnorm_q8", ill_rmsnorm_q8(act.k ? 1 : 0, ptr(a[0]), ptr(a[1]), OPT_PTR(a[6]), act.xq, act.xs, act.xsum, (int)as_int(a[3]),
                                          (float)as_float(a[4]), OPT_INT(a[5], 1), OPT_BOOL(a[7], 1), cur_stream()));
   return ret(a[2]);
-} catch (const Failed&) { return nullptr; }
+} CATCH_ERRORS
 
 // Y = W X for up to 16 tokens in one launch; false when the shape wants the tokens split (the Python form does that)
 inline bool mul(const Mat& w, const Act& act, ill_dptr y, int n, ill_dptr bias, int acc) {
@@ -193,7 +199,7 @@ PyObject* cmat_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject*
   if (n < 1 || n > FEW || !mul(Mat(a[0]), Act(a[1]), ptr(a[2]), (int)n, OPT_PTR(a[4]), OPT_BOOL(a[5], 0)))
     return PyObject_Vectorcall(slow(S_cmat_mul), args, nargs, kwnames);
   return ret(a[2]);
-} catch (const Failed&) { return nullptr; }
+} CATCH_ERRORS
 
 void mul_any(PyObject* w, PyObject* act, PyObject* y, long long n, PyObject* bias) {
   if (n >= 1 && n <= FEW && mul(Mat(w), Act(act), ptr(y), (int)n, bias ? ptr(bias) : 0, 0)) return;
@@ -224,7 +230,7 @@ PyObject* qkv_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
   }
   for (int i = 0; i < 3; ++i) mul_any(a[i], a[3], a[4 + i], n, a[7 + i]);
   Py_RETURN_NONE;
-} catch (const Failed&) { return nullptr; }
+} CATCH_ERRORS
 
 PyObject* glu_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
   ARGS("glu_mul", 4, S_g, S_u, S_act, S_fa, S_n, S_fb);
@@ -246,7 +252,7 @@ PyObject* glu_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
     return ret(a[3]);
   }
   return PyObject_Vectorcall(slow(S_glu_mul), args, nargs, kwnames);
-} catch (const Failed&) { return nullptr; }
+} CATCH_ERRORS
 
 PyObject* embed(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
   ARGS("embed", 3, S_emb, S_tokens, S_x);
@@ -254,9 +260,8 @@ PyObject* embed(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kw
   const at::Tensor& t = tensor(a[1]);
   check("ill_dequant_rows", ill_dequant_rows(m.type, m.w, m.cols, (ill_dptr)(uintptr_t)t.data_ptr(), 0, (int)t.numel(), ptr(a[2]), cur_stream()));
   return ret(a[2]);
-} catch (const Failed&) { return nullptr; }
+} CATCH_ERRORS
 
-PyObject* stream(PyObject*, PyObject*) { return PyLong_FromVoidPtr(cur_stream()); }
 PyObject* launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches); }
 
 PyObject* set_slow(PyObject*, PyObject* d) {
@@ -284,7 +289,6 @@ PyMethodDef methods[] = {
          "glu_mul(g, u, act, fa, n=1, fb=None)\n--\n\nGLU-MUL (src/cuda-dense.lisp:326-339): silu(G x) * (U x) into FA."),
     FAST(embed,
          "embed(emb, tokens, x)\n--\n\nEMBED (src/cuda-dense.lisp:302-307): rows TOKENS (int32 on the device) of EMB as floats in X."),
-    {"stream", stream, METH_NOARGS, "The current stream of the current device, as an integer."},
     {"launches", launches, METH_NOARGS, "Launches made by this module since it was loaded."},
     {"set_slow", set_slow, METH_O, "Python functions for what this module leaves to Python: {name: function}."},
     {nullptr, nullptr, 0, nullptr}};

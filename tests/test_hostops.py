@@ -1,0 +1,50 @@
+"""The native decode operators (csrc/hostops.cpp) where they raise before they launch anything: no GPU needed."""
+import os
+import subprocess
+import sys
+
+import pytest
+import torch
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SPARSE = "torch.sparse_coo_tensor([[0]], [1.0], (32,))"
+ACT = "D.make_qact(32, 'q8', device='cpu')"
+MAT = "D.CMat('w', 0, 1, 32, torch.zeros(34, dtype=torch.uint8))"
+NO_STORAGE = [
+    "D.quant_q8(%s, %s)" % (SPARSE, ACT),
+    "torch.func.vmap(lambda x: D.quant_q8(x, %s) and x)(torch.zeros(2, 32))" % ACT,
+    "D.rmsnorm_q8(%s, torch.ones(32), %s, 32, 1e-6)" % (SPARSE, ACT),
+    "D.cmat_mul(%s, %s, %s)" % (MAT, ACT, SPARSE),
+    "D.qkv_mul(%s, %s, %s, %s, %s, None, None)" % (MAT, MAT, MAT, ACT, SPARSE),
+    "D.glu_mul(%s, %s, %s, %s)" % (MAT, MAT, ACT, SPARSE),
+    "D.embed(%s, torch.zeros(1, dtype=torch.int32), %s)" % (MAT, SPARSE),
+]
+NO_DRIVER = [
+    "D.quant_q8(torch.zeros(32), %s)" % ACT,
+    "D.rmsnorm_q8(torch.zeros(32), torch.ones(32), %s, 32, 1e-6)" % ACT,
+    "D.cmat_mul(%s, %s, torch.zeros(1))" % (MAT, ACT),
+    "D.qkv_mul(%s, %s, %s, %s, torch.zeros(1), torch.zeros(1), torch.zeros(1))" % (MAT, MAT, MAT, ACT),
+    "D.glu_mul(%s, %s, %s, torch.zeros(1))" % (MAT, MAT, ACT),
+    "D.glu_mul(%s, %s, %s, torch.zeros(2), 2, torch.zeros(2))" % (MAT, MAT, ACT),
+    "D.embed(%s, torch.zeros(1, dtype=torch.int32), torch.zeros(32))" % MAT,
+]
+CODE = """
+import torch
+from illatio_b200 import cuda_dense as D
+for expr in %r:
+    try:
+        eval(expr)
+    except RuntimeError as e:
+        print("raised", flush=True)
+    else:
+        raise SystemExit(expr)
+"""
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="host tensors: only where nothing can be launched")
+@pytest.mark.parametrize("exprs", [NO_STORAGE, NO_DRIVER], ids=["no_storage", "no_driver"])
+def test_an_exception_of_torch_is_a_python_exception(exprs):
+    """In a process of its own: a C++ exception that is not caught ends the process."""
+    r = subprocess.run([sys.executable, "-c", CODE % exprs], capture_output=True, text=True, cwd=ROOT)
+    assert r.returncode == 0 and r.stdout.count("raised") == len(exprs), (r.returncode, r.stdout, r.stderr[-500:])
