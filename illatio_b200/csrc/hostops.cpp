@@ -10,6 +10,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/ExpandUtils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -244,11 +245,18 @@ PyObject* glu_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
     }
   }
   if (n >= 1 && a[5] && a[5] != Py_None) {
+    // the buffers may be longer than N tokens take (a serving loop's largest batch), but have to agree
+    const at::Tensor &fa = tensor(a[3]), &fb = tensor(a[5]);
+    const long long len = n * attr_int(a[0], S_rows);
+    if (!at::is_expandable_to(fb.sizes(), fa.sizes()) || fa.numel() < len || fb.numel() < len) {
+      PyErr_Format(PyExc_RuntimeError, "glu_mul(): FA of %lld values and FB of %lld do not agree, or hold fewer than N * ROWS = %lld",
+                   (long long)fa.numel(), (long long)fb.numel(), len);
+      throw Failed();
+    }
     mul_any(a[0], a[2], a[3], n, nullptr);
     mul_any(a[1], a[2], a[5], n, nullptr);
-    const at::Tensor& fa = tensor(a[3]);
-    const ill_dptr fp = (ill_dptr)(uintptr_t)fa.data_ptr();
-    check("ill_silu_mul", ill_silu_mul(fa.numel(), fp, ptr(a[5]), fp, cur_stream()));
+    const ill_dptr fp = ptr(a[3]);
+    check("ill_silu_mul", ill_silu_mul(len, fp, ptr(a[5]), fp, cur_stream()));
     return ret(a[3]);
   }
   return PyObject_Vectorcall(slow(S_glu_mul), args, nargs, kwnames);
@@ -286,7 +294,8 @@ PyMethodDef methods[] = {
          "qkv_mul(wq, wk, wv, act, q, k, v, bq=None, bk=None, bv=None, n=1)\n--\n\nQKV-MUL (src/cuda-dense.lisp:309-324): for one token one\n"
          "launch when the three formats agree, two when those of Q and K do; else three products."),
     FAST(glu_mul,
-         "glu_mul(g, u, act, fa, n=1, fb=None)\n--\n\nGLU-MUL (src/cuda-dense.lisp:326-339): silu(G x) * (U x) into FA."),
+         "glu_mul(g, u, act, fa, n=1, fb=None)\n--\n\nGLU-MUL (src/cuda-dense.lisp:326-339): silu(G x) * (U x) into FA; FB, of\n"
+         "FA's shape, is scratch for the products that one launch does not take."),
     FAST(embed,
          "embed(emb, tokens, x)\n--\n\nEMBED (src/cuda-dense.lisp:302-307): rows TOKENS (int32 on the device) of EMB as floats in X."),
     {"launches", launches, METH_NOARGS, "Launches made by this module since it was loaded."},

@@ -182,9 +182,12 @@ def _glu_mul(g, u, act, fa, n=1, fb=None):
     """glu_mul of several tokens, or of two formats."""
     if fb is None:
         fb = torch.empty_like(fa)
+    count = max(n, 0) * g.rows
+    if torch.broadcast_shapes(fa.shape, fb.shape) != fa.shape or min(fa.numel(), fb.numel()) < count:
+        raise RuntimeError("glu_mul(): FA of %d values and FB of %d do not agree, or hold fewer than N * ROWS = %d" % (fa.numel(), fb.numel(), count))
     cmat_mul(g, act, fa, n)
     cmat_mul(u, act, fb, n)
-    _lib.call("ill_silu_mul", fa.numel(), _ptr(fa), _ptr(fb), _ptr(fa), _stream())
+    _lib.call("ill_silu_mul", count, _ptr(fa), _ptr(fb), _ptr(fa), _stream())
     return fa
 
 

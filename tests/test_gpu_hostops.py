@@ -44,3 +44,31 @@ def test_arguments_and_errors(cuda_lib):
         D.cmat_mul(w, bad, y)
     assert e.value.code == 2
     assert D.device_status() == 0
+
+
+def _mat(fmt, rows, cols, seed):
+    return D.upload_gmat(B.synth_matrix(fmt, rows, cols, seed=seed), fmt, rows, cols)
+
+
+@pytest.mark.parametrize("n", [1, 2, 16, 17])
+@pytest.mark.parametrize("fmts", [(B.Q4_K, B.Q4_K), (B.Q4_K, B.Q6_K), (B.Q8_0, B.Q8_0)])
+@pytest.mark.parametrize("extra", [None, 0, 24])
+def test_glu_mul_of_several_tokens(cuda_lib, fmts, n, extra):
+    """glu_mul without FB (EXTRA None), with one, and with buffers EXTRA rows longer than the N tokens take: two products and
+    the formula, and nothing else of FA written."""
+    rows, cols = 40, 512
+    g, u = _mat(fmts[0], rows, cols, 1), _mat(fmts[1], rows, cols, 2)
+    x = torch.randn(n * cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n))
+    act = D.quant_q8(x, D.make_qact(n * cols, D.matrix_act_kind(g)))
+    a, b = (torch.empty(n * rows, device="cuda") for _ in range(2))
+    D.cmat_mul(g, act, a, n)
+    D.cmat_mul(u, act, b, n)
+    want = a.double() / (1.0 + torch.exp(-a.double())) * b.double()
+    fa = torch.full((n * rows + (extra or 0) * rows,), 7.0, device="cuda")
+    fb = None if extra is None else torch.full_like(fa, 9.0)
+    assert D.glu_mul(g, u, act, fa, n, fb=fb) is fa
+    # one token of one format takes its products in one launch (float terms in another order: 2e-6 of the largest, as the
+    # other products of two kernels here); else the same two products, six roundings of the formula apart
+    tol = 4e-6 * (a.abs().max() * b.abs().max() + want.abs().max()) if n == 1 and fmts[0] == fmts[1] else 6 * 2.0 ** -24 * want.abs() + 1e-30
+    assert ((fa[:n * rows].double() - want).abs() <= tol).all()
+    assert (fa[n * rows:] == 7.0).all()

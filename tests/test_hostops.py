@@ -6,6 +6,8 @@ import sys
 import pytest
 import torch
 
+from illatio_b200 import cuda_dense as D
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 SPARSE = "torch.sparse_coo_tensor([[0]], [1.0], (32,))"
@@ -48,3 +50,13 @@ def test_an_exception_of_torch_is_a_python_exception(exprs):
     """In a process of its own: a C++ exception that is not caught ends the process."""
     r = subprocess.run([sys.executable, "-c", CODE % exprs], capture_output=True, text=True, cwd=ROOT)
     assert r.returncode == 0 and r.stdout.count("raised") == len(exprs), (r.returncode, r.stdout, r.stderr[-500:])
+
+
+@pytest.mark.parametrize("fa,fb,n", [((16, 8), (4, 8), 4), ((128,), (32,), 4), ((4, 8), (16, 8), 4), ((32,), (4, 8), 4), ((2, 8), (2, 8), 4),
+                                     ((2, 8), None, 4), ((128,), (32,), 0)])
+def test_glu_mul_refuses_buffers_that_do_not_agree(fa, fb, n):
+    """FA and FB of different shapes, or shorter than the N tokens' rows: refused before anything is launched."""
+    m = D.CMat("w", 0, 8, 32, torch.zeros(8 * 34, dtype=torch.uint8))
+    act = D.make_qact(4 * 32, "q8", device="cpu")
+    with pytest.raises(RuntimeError, match="do not agree|broadcast"):
+        D.glu_mul(m, m, act, torch.zeros(fa), n, None if fb is None else torch.zeros(fb))
