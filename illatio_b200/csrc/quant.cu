@@ -239,9 +239,12 @@ static int rmsnorm_q8_launch(int kind, ill_dptr x, ill_dptr w, ill_dptr h, ill_d
   void* bp = (void*)(uintptr_t)xsum;
   __half *fhp = (__half*)(uintptr_t)xh, *fep = (__half*)(uintptr_t)xe;
   void* args[] = {&xp, &wp, &hp, &qp, &sp, &bp, &d, &eps, &f16_scale, &fhp, &fep};
-  // few rows are spread over their blocks, as far as two CTAs an SM (148) go; many rows take a CTA each
+  // few rows are spread over their blocks, as far as two CTAs an SM (148) go; many rows take a CTA each, and so do rows that
+  // are normalized in place: a CTA of a row that is shared would still be reading what another has written
   const bool vec = kind == 0 && ((x | w | h) & 15) == 0 && (xq & 3) == 0;
-  const int nb = vec ? (d + 127) / 128 : d / bw, most = n < 296 ? (int)(296 / n) : 1;
+  const uint64_t bytes = 4ull * (uint64_t)d * (uint64_t)n;
+  const bool in_place = h && h < x + bytes && x < h + bytes;
+  const int nb = vec ? (d + 127) / 128 : d / bw, most = n < 296 && !in_place ? (int)(296 / n) : 1;
   const unsigned slices = (unsigned)((nb + 7) / 8 < most ? (nb + 7) / 8 : most);
   const void* k = kind == 1 ? (xh ? (const void*)rmsnorm_q8_kernel<1, true, false> : (const void*)rmsnorm_q8_kernel<1, false, false>)
                             : vec ? (const void*)rmsnorm_q8_kernel<0, false, true> : (const void*)rmsnorm_q8_kernel<0, false, false>;

@@ -114,6 +114,17 @@ def test_norm_quantizer_and_swiglu_at_any_split_and_alignment(oracle, kind, d, n
     assert torch.equal(a.view(torch.int32), b.view(torch.int32))
 
 
+@pytest.mark.parametrize("kind,d,n", [("q8", 896, 1), ("q8", 4864, 4), ("q8", 4864, 400), ("q8k", 8448, 1), ("q8k", 2560, 16), ("q8k", 5120, 148)])
+def test_norm_in_place(kind, d, n):
+    """H the same memory as X: the bits of a separate H, where rows are otherwise split over CTAs and where they are not."""
+    g = torch.Generator(device="cuda").manual_seed(d)
+    x, w, h = torch.randn(n, d, device="cuda", generator=g), torch.randn(d, device="cuda", generator=g), torch.empty(n, d, device="cuda")
+    one, two = D.make_qact(n * d, kind), D.make_qact(n * d, kind)
+    D.rmsnorm_q8(x, w, one, d, 1e-6, n, h=h)
+    D.rmsnorm_q8(x, w, two, d, 1e-6, n, h=x)
+    assert torch.equal(x, h) and torch.equal(two.xq, one.xq) and torch.equal(two.xs, one.xs)
+
+
 @pytest.mark.parametrize("fmt", FMTS)
 def test_dequant_rows_bit_exact_golden(fmt):
     z = np.load(os.path.join(GOLD, "dequant_%s.npz" % B.NAMES[fmt]))
