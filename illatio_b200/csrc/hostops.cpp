@@ -20,7 +20,7 @@
 namespace {
 
 PyObject* g_slow = nullptr;   // name -> Python function
-long long g_launches = 0;     // launches made from this module (the GIL is held): what bench.py counts
+long long g_launches = 0;     // launches made from this module (counted under the GIL): what bench.py counts
 
 // attribute names, interned once
 #define NAMES(X) \
@@ -34,9 +34,9 @@ NAMES(DECL)
 struct Failed {};  // a Python error is set
 // What ends every operator: no C++ exception may reach the interpreter's C frames.  Tensors without storage (sparse, inside
 // vmap) and a stream that cannot be had throw c10::Error, which becomes the exception that torch's Python functions raise.
-#define CATCH_ERRORS                                                                                       \
-  catch (const Failed&) { return nullptr; }                                                                \
-  catch (...) { torch::translate_exception_to_python(std::current_exception()); return nullptr; }
+#define CATCH_ERRORS                        \
+  catch (const Failed&) { return nullptr; } \
+  catch (const std::exception&) { torch::translate_exception_to_python(std::current_exception()); return nullptr; }
 
 inline ill_stream cur_stream() { return (ill_stream)c10::cuda::getCurrentCUDAStream().stream(); }
 
@@ -119,10 +119,20 @@ PyObject* slow(PyObject* name) {
   if (r) PyErr_Format(PyExc_RuntimeError, "%s failed with status %d", fn, rc);
   throw Failed();
 }
-inline void check(const char* fn, int rc) {
-  if (rc) raise_status(fn, rc);
+// FN(ARGS...) without the GIL, which the arguments were made under: a launch waits while its stream's queue is full, and
+// other threads, and host functions queued before it, go on meanwhile.
+template <class... P, class... A>
+inline int launch(int (*fn)(P...), A... args) {
+  PyThreadState* const ts = PyEval_SaveThread();
+  const int rc = fn((P)args...);
+  PyEval_RestoreThread(ts);
+  return rc;
+}
+inline void check(const char* name, int rc) {
+  if (rc) raise_status(name, rc);
   ++g_launches;
 }
+#define LAUNCH(FN, ...) check(#FN, launch(FN, __VA_ARGS__))
 
 // positional and keyword arguments into OUT (absent: null); the first REQUIRED must be there
 void parse(const char* fn, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames, PyObject* const* names, int n, int required,
@@ -171,8 +181,8 @@ PyObject* quant_q8(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject*
   if (act.has_f16) return PyObject_Vectorcall(slow(S_quant_q8), args, nargs, kwnames);
   const at::Tensor& x = tensor(a[0]);
   const ill_dptr xp = (ill_dptr)(uintptr_t)x.data_ptr();
-  if (act.k) check("ill_quant_q8_k", ill_quant_q8_k(xp, act.xq, act.xs, act.xsum, x.numel() / 256, cur_stream()));
-  else check("ill_quant_q8_0", ill_quant_q8_0(xp, act.xq, act.xs, act.xsum, x.numel() / 32, OPT_BOOL(a[2], 1), cur_stream()));
+  if (act.k) LAUNCH(ill_quant_q8_k, xp, act.xq, act.xs, act.xsum, x.numel() / 256, cur_stream());
+  else LAUNCH(ill_quant_q8_0, xp, act.xq, act.xs, act.xsum, x.numel() / 32, OPT_BOOL(a[2], 1), cur_stream());
   return ret(a[1]);
 } CATCH_ERRORS
 
@@ -180,14 +190,14 @@ PyObject* rmsnorm_q8(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObjec
   ARGS("rmsnorm_q8", 5, S_x, S_w, S_act, S_d, S_eps, S_n, S_h, S_f16_scale);
   const Act act(a[2]);
   if (act.has_f16) return PyObject_Vectorcall(slow(S_rmsnorm_q8), args, nargs, kwnames);
-  check("ill_rmsnorm_q8", ill_rmsnorm_q8(act.k ? 1 : 0, ptr(a[0]), ptr(a[1]), OPT_PTR(a[6]), act.xq, act.xs, act.xsum, (int)as_int(a[3]),
-                                         (float)as_float(a[4]), OPT_INT(a[5], 1), OPT_BOOL(a[7], 1), cur_stream()));
+  LAUNCH(ill_rmsnorm_q8, act.k ? 1 : 0, ptr(a[0]), ptr(a[1]), OPT_PTR(a[6]), act.xq, act.xs, act.xsum, (int)as_int(a[3]), (float)as_float(a[4]),
+         OPT_INT(a[5], 1), OPT_BOOL(a[7], 1), cur_stream());
   return ret(a[2]);
 } CATCH_ERRORS
 
 // Y = W X for up to 16 tokens in one launch; false when the shape wants the tokens split (the Python form does that)
 inline bool mul(const Mat& w, const Act& act, ill_dptr y, int n, ill_dptr bias, int acc) {
-  const int rc = ill_mv(w.type, w.w, w.rows, w.cols, act.xq, act.xs, act.k ? act.xsum : 0, y, bias, acc, n, cur_stream());
+  const int rc = launch(ill_mv, w.type, w.w, w.rows, w.cols, act.xq, act.xs, act.k ? act.xsum : 0, y, bias, acc, n, cur_stream());
   if (rc == ILL_ERR_UNSUPPORTED && n > 1) return false;
   check("ill_mv", rc);
   return true;
@@ -222,9 +232,8 @@ PyObject* qkv_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
       // it beside Q and K (a fork and a join cost a graph nothing: a 4B token 1.54 ms, 1.57 one after the other); launch
       // by launch, the two events and four calls of a fork cost the host more than the overlap gives.
       if (!three && capturing()) return PyObject_Vectorcall(slow(S_qkv_mul), args, nargs, kwnames);
-      check("ill_mv_3", ill_mv_3(q.type, q.w, k.w, three ? v.w : 0, q.rows, k.rows, three ? v.rows : 0, q.cols, x.xq, x.xs,
-                                 x.k ? x.xsum : 0, ptr(a[4]), ptr(a[5]), three ? ptr(a[6]) : 0, OPT_PTR(a[7]), OPT_PTR(a[8]),
-                                 three ? OPT_PTR(a[9]) : 0, cur_stream()));
+      LAUNCH(ill_mv_3, q.type, q.w, k.w, three ? v.w : 0, q.rows, k.rows, three ? v.rows : 0, q.cols, x.xq, x.xs, x.k ? x.xsum : 0, ptr(a[4]),
+             ptr(a[5]), three ? ptr(a[6]) : 0, OPT_PTR(a[7]), OPT_PTR(a[8]), three ? OPT_PTR(a[9]) : 0, cur_stream());
       if (!three) mul(v, x, ptr(a[6]), 1, OPT_PTR(a[9]), 0);
       Py_RETURN_NONE;
     }
@@ -240,7 +249,7 @@ PyObject* glu_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
     const Mat g(a[0]), u(a[1]);
     if (g.type == u.type) {
       const Act x(a[2]);
-      check("ill_mv_glu", ill_mv_glu(g.type, g.w, u.w, g.rows, g.cols, x.xq, x.xs, x.k ? x.xsum : 0, ptr(a[3]), cur_stream()));
+      LAUNCH(ill_mv_glu, g.type, g.w, u.w, g.rows, g.cols, x.xq, x.xs, x.k ? x.xsum : 0, ptr(a[3]), cur_stream());
       return ret(a[3]);
     }
   }
@@ -256,7 +265,7 @@ PyObject* glu_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
     mul_any(a[0], a[2], a[3], n, nullptr);
     mul_any(a[1], a[2], a[5], n, nullptr);
     const ill_dptr fp = ptr(a[3]);
-    check("ill_silu_mul", ill_silu_mul(len, fp, ptr(a[5]), fp, cur_stream()));
+    LAUNCH(ill_silu_mul, len, fp, ptr(a[5]), fp, cur_stream());
     return ret(a[3]);
   }
   return PyObject_Vectorcall(slow(S_glu_mul), args, nargs, kwnames);
@@ -266,7 +275,7 @@ PyObject* embed(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kw
   ARGS("embed", 3, S_emb, S_tokens, S_x);
   const Mat m(a[0]);
   const at::Tensor& t = tensor(a[1]);
-  check("ill_dequant_rows", ill_dequant_rows(m.type, m.w, m.cols, (ill_dptr)(uintptr_t)t.data_ptr(), 0, (int)t.numel(), ptr(a[2]), cur_stream()));
+  LAUNCH(ill_dequant_rows, m.type, m.w, m.cols, (ill_dptr)(uintptr_t)t.data_ptr(), 0, (int)t.numel(), ptr(a[2]), cur_stream());
   return ret(a[2]);
 } CATCH_ERRORS
 

@@ -1,4 +1,7 @@
 """The native host side of the decode operators (csrc/hostops.cpp) and the kernel behind its several-token gated product."""
+import threading
+import time
+
 import pytest
 import torch
 
@@ -72,3 +75,31 @@ def test_glu_mul_of_several_tokens(cuda_lib, fmts, n, extra):
     tol = 4e-6 * (a.abs().max() * b.abs().max() + want.abs().max()) if n == 1 and fmts[0] == fmts[1] else 6 * 2.0 ** -24 * want.abs() + 1e-30
     assert ((fa[:n * rows].double() - want).abs() <= tol).all()
     assert (fa[n * rows:] == 7.0).all()
+
+
+def test_other_threads_run_while_a_launch_waits(cuda_lib):
+    """A launch into a full queue (thousands behind half a second's sleep on the device) leaves the interpreter to others."""
+    x, act = torch.randn(256, device="cuda"), D.make_qact(256, "q8k")
+    D.quant_q8(x, act)
+    torch.cuda.synchronize()
+    gap, stop = [0.0], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gap[0], last = max(gap[0], now - last), now
+
+    t = threading.Thread(target=tick)
+    t.start()
+    start = time.perf_counter()
+    torch.cuda._sleep(1_000_000_000)  # cycles
+    for _ in range(4000):
+        D.quant_q8(x, act)
+    took = time.perf_counter() - start
+    stop.set()
+    t.join()
+    torch.cuda.synchronize()
+    assert took > 0.3, "the queue never filled"
+    assert gap[0] < took / 3, (gap[0], took)
