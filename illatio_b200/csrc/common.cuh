@@ -145,6 +145,14 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 // prologue / wait until the previous kernel's memory is visible.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// P, for what a kernel before this one may have written: nothing is read through it ahead of the wait that it follows.
+template <class T>
+__device__ __forceinline__ T* after_wait(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
+// Asks for the 32 bytes at P to be brought into L2: a hint that returns nothing, so it may go ahead of the wait whoever writes P.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 __device__ __forceinline__ float h2f(uint32_t bits) { return __half2float(__ushort_as_half((unsigned short)bits)); }
 

@@ -84,9 +84,10 @@ __global__ void __launch_bounds__(256) quant_q8_k_kernel(const float* __restrict
 // row's scale out for itself (the row comes from L2) and takes a slice of its blocks, so that one token's
 // norm is not one CTA's serial work.  The double sum is taken in the order quantdev.cuh fixes, not in the
 // CPU loop's; the two agree until the float the sum is rounded to sits within 1e-16 of a rounding boundary.
-// Bound by latency: the norm's weights are on their way before the kernel waits for the row, a warp asks for four of its
-// groups and its first block's values at once, and a few rows are spread over their blocks too (16 rows of 2560: 3.9 -> 2.6 us; 4
-// of 5120 5.2 -> 2.9; one of 2560 3.1 -> 2.5).  VEC: Q8_0 blocks by four values a lane (X, W, H and XQ aligned for it).
+// Bound by latency: the norm's weights are on their way to L2 before the kernel waits for the one before it (which may have
+// written them), a warp asks for four of its groups and its first block's values at once, and a few rows are spread over their
+// blocks too (in a graph of norms, before and now: 16 rows of 2560 3.8 -> 2.6 us, 4 of 5120 5.1 -> 2.8, one of 2560 3.0 -> 2.5,
+// 512 of 5120 13.9 -> 7.1).  VEC: Q8_0 blocks by four values a lane (X, W, H and XQ aligned for it).
 template <int K8K, bool F16, bool VEC>
 __global__ void __launch_bounds__(256) rmsnorm_q8_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                          float* __restrict__ h, i8* __restrict__ xq, float* __restrict__ xs,
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(256) rmsnorm_q8_kernel(const float* __restrict
   // a unit is a warp's turn: a Q8_K block, a Q8_0 block, or (VEC) four Q8_0 blocks, the last unit perhaps fewer
   constexpr int BW = K8K ? 256 : VEC ? 128 : 32, VL = BW / 32;  // a unit's values, a lane's
   const int nb = (d + BW - 1) / BW, b0 = blockIdx.x * 8 + warp;
-  float wv[VL], x0[VL];  // of the warp's first block; the weights do not depend on the previous kernel
+  float wv[VL], x0[VL];  // of the warp's first block
   auto load = [&](const float* src, int b, float (&v)[VL]) {
     if constexpr (K8K) rms_load8<false>(src, d, b * 256 + 8 * lane, v);
     else if constexpr (VEC) {
@@ -105,12 +106,16 @@ __global__ void __launch_bounds__(256) rmsnorm_q8_kernel(const float* __restrict
       v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
     } else v[0] = src[b * 32 + lane];
   };
-  if (b0 < nb) load(w, b0, wv);
+  if (b0 < nb && b0 * BW + VL * lane < d) prefetch_l2(w + b0 * BW + VL * lane);
   pdl_launch_dependents();
   pdl_wait();
+  w = after_wait(w);
   const long long base = (long long)blockIdx.y * d;
-  const float* xr = x + base;
-  if (b0 < nb) load(xr, b0, x0);
+  const float* xr = after_wait(x + base);
+  if (b0 < nb) {
+    load(w, b0, wv);
+    load(xr, b0, x0);
+  }
   const int ng = (d + 255) / 256;
   for (int g0 = warp; g0 < ng; g0 += 32) {
     float v[4][8];

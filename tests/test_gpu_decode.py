@@ -254,3 +254,30 @@ def test_errors_are_reported_not_raised_as_faults():
                   act.xsum.data_ptr(), y.data_ptr(), 0, 0, 1, None)
     with pytest.raises(ValueError):
         D.upload_gmat(np.zeros(100, np.uint8), B.Q4_K, 4, 250)
+
+
+@pytest.mark.parametrize("kind", ["q8", "q8k"])
+def test_weights_that_the_kernel_before_has_written(kind):
+    """A norm's weights, and an unquantized matrix of one token, made by the kernel just before (whose launch lets the next
+    begin at once): read only after it is through."""
+    from illatio_b200 import cuda_ds4f as M
+    rows, cols = 2048, 2048
+    mats = [D.upload_gmat(B.synth_matrix(B.Q4_K, rows, cols, seed=s), B.Q4_K, rows, cols) for s in (1, 2)]
+    flat = [D.dequant_rows(m, 0, rows) for m in mats]
+    x = torch.randn(cols, device="cuda")
+    want = []
+    for f in flat:
+        torch.cuda.synchronize()
+        a, y = D.make_qact(cols, kind), torch.empty(rows, device="cuda")
+        D.rmsnorm_q8(x, f[rows - 1], a, cols, 1e-6)
+        M.dk_mv16(f, x.reshape(1, cols), y)
+        want.append((a.xq, a.xs, y))
+    buf = torch.empty(rows, cols, device="cuda")
+    for i in range(20):
+        a, b, y = D.make_qact(cols, kind), D.make_qact(cols, kind), torch.empty(rows, device="cuda")
+        D.dequant_rows(mats[i % 2], 0, rows, out=buf)
+        D.rmsnorm_q8(x, buf[rows - 1], a, cols, 1e-6)
+        D.dequant_rows(mats[(i + 1) % 2], 0, rows, out=buf)
+        M.dk_mv16(buf, x.reshape(1, cols), y)
+        assert torch.equal(a.xq, want[i % 2][0]) and torch.equal(a.xs, want[i % 2][1])
+        assert torch.equal(y, want[(i + 1) % 2][2])
