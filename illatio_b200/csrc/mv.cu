@@ -114,7 +114,11 @@ __global__ void __launch_bounds__(MV_THREADS) mvn_kernel(const MvParams p) {
   // this segment's matrices
   const u8* wbase[MV_MAX_MATS];
   if (p.ptrs) {
-    const u8* b = (const u8*)(uintptr_t)p.ptrs[z] + p.add;
+    // the table may come from a kernel before (ill_moe_row_ptrs, an index of the router's choice): no copy starts ahead of it
+    if (IQ) iq_tables_fill(iq_grid, iq_smask, ill_iq2xxs_grid, ill_ksigns_iq2xs);
+    pdl_launch_dependents();
+    pdl_wait();
+    const u8* b = (const u8*)(uintptr_t)after_wait(p.ptrs)[z] + p.add;
     wbase[0] = b;
     wbase[1] = b + p.up_add;
     wbase[2] = b;
@@ -153,7 +157,7 @@ __global__ void __launch_bounds__(MV_THREADS) mvn_kernel(const MvParams p) {
       if (tile < ntiles) issue(tile, s);
     }
   }
-  if (IQ) iq_tables_fill(iq_grid, iq_smask, ill_iq2xxs_grid, ill_ksigns_iq2xs);
+  if (IQ && !p.ptrs) iq_tables_fill(iq_grid, iq_smask, ill_iq2xxs_grid, ill_ksigns_iq2xs);
   pdl_launch_dependents();
   pdl_wait();  // activations may come from the previous kernel
 
@@ -322,7 +326,11 @@ __global__ void __launch_bounds__(MV_THREADS) mvw_kernel(const MvParams p) {
 
   const u8* wbase[MV_MAX_MATS];
   if (p.ptrs) {
-    const u8* b = (const u8*)(uintptr_t)p.ptrs[z] + p.add;
+    // the table may come from a kernel before (ill_moe_row_ptrs, an index of the router's choice): no copy starts ahead of it
+    if (IQ) iq_tables_fill(iq_grid, iq_smask, ill_iq2xxs_grid, ill_ksigns_iq2xs);
+    pdl_launch_dependents();
+    pdl_wait();
+    const u8* b = (const u8*)(uintptr_t)after_wait(p.ptrs)[z] + p.add;
     wbase[0] = b;
     wbase[1] = b + p.up_add;
     wbase[2] = b;
@@ -375,7 +383,7 @@ __global__ void __launch_bounds__(MV_THREADS) mvw_kernel(const MvParams p) {
     mbar_fence_init();
     for (int s = 0; s < p.nstages; ++s) issue_next(s);  // weights do not depend on the previous kernel
   }
-  if (IQ) iq_tables_fill(iq_grid, iq_smask, ill_iq2xxs_grid, ill_ksigns_iq2xs);
+  if (IQ && !p.ptrs) iq_tables_fill(iq_grid, iq_smask, ill_iq2xxs_grid, ill_ksigns_iq2xs);
   pdl_launch_dependents();
   pdl_wait();  // the activations may come from the previous kernel
 

@@ -146,3 +146,33 @@ def test_mv_dense_tiles(cuda_lib, dtype, rows, cols, n):
     for t in range(0, n, 2):
         M.dk_mv16(w, x[t:t + 2], want[t:t + 2], n=2)
     assert torch.equal(y[:, :rows], want[:n]) and (y[:, rows:] == 5.0).all()
+
+
+@pytest.mark.parametrize("fmt", [B.Q2_K, B.IQ2_XXS])
+def test_a_table_that_the_kernel_before_has_written(fmt):
+    """The experts' addresses made by ill_moe_row_ptrs just before the products (whose launch lets the next begin at once):
+    read only after it is through.  The table holds valid addresses throughout, those of the other expert before each turn."""
+    cols, rows, nz = 512, 256, 64
+    w = [to_dev(B.synth_matrix(fmt, rows, cols, seed=s)) for s in (1, 2)]
+    x = torch.randn(nz * cols, device="cuda")
+    act = D.quant_q8(x, D.make_qact(nz * cols, "q8k"))
+    ptrs = torch.tensor([t.data_ptr() for t in w], dtype=torch.int64, device="cuda")
+    counts = [torch.tensor(c, dtype=torch.int32, device="cuda") for c in ((nz, 0), (0, nz))]
+    bases = [torch.tensor(b, dtype=torch.int32, device="cuda") for b in ((0, nz), (0, 0))]
+    table = [torch.full((nz,), t.data_ptr(), dtype=torch.int64, device="cuda") for t in w]
+
+    def products(t, y):
+        _lib.call("ill_moe_mv", fmt, cols, rows, 0, t.data_ptr(), nz, act.xq.data_ptr(), act.xs.data_ptr(), act.xsum.data_ptr(), 1,
+                  y.data_ptr(), rows, _lib.stream())
+        return y
+    want = [torch.empty(nz, rows, device="cuda") for _ in range(2)]
+    for i in range(2):
+        torch.cuda.synchronize()
+        products(table[i], want[i])
+    torch.cuda.synchronize()
+    turning, y = table[1].clone(), torch.empty(20, nz, rows, device="cuda")
+    for i in range(20):
+        _lib.call("ill_moe_row_ptrs", 2, ptrs.data_ptr(), counts[i % 2].data_ptr(), bases[i % 2].data_ptr(), nz, turning.data_ptr(), _lib.stream())
+        products(turning, y[i])
+    for i in range(20):
+        assert torch.equal(y[i], want[i % 2])
