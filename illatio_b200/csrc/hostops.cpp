@@ -26,7 +26,7 @@ long long g_launches = 0;     // launches made from this module (counted under t
 #define NAMES(X) \
   X(type) X(rows) X(cols) X(qs) X(kind) X(xq) X(xs) X(xsum) X(_cf) X(w) X(act) X(y) X(n) X(bias) X(acc) X(x) X(f16_scale) X(d) X(eps) \
   X(h) X(wq) X(wk) X(wv) X(q) X(k) X(v) X(bq) X(bk) X(bv) X(g) X(u) X(fa) X(fb) X(emb) X(tokens) X(quant_q8) X(rmsnorm_q8) \
-  X(cmat_mul) X(glu_mul) X(qkv_mul) X(error)
+  X(cmat_mul) X(glu_mul) X(qkv_mul) X(error) X(vars) X(TC_MIN_TOKENS)
 #define DECL(s) PyObject* S_##s;
 NAMES(DECL)
 #undef DECL
@@ -202,18 +202,24 @@ inline bool mul(const Mat& w, const Act& act, ill_dptr y, int n, ill_dptr bias, 
   check("ill_mv", rc);
   return true;
 }
-constexpr long long FEW = 16;  // more tokens are a chunk: the Python form picks the kernel
+// Whether N tokens are few; more are a chunk, and the Python form picks the kernel.  So it does from cuda_dense.TC_MIN_TOKENS on.
+inline bool few(long long n) {
+  if (n < 1 || n > 16) return false;
+  PyObject* v = PyDict_GetItemWithError(slow(S_vars), S_TC_MIN_TOKENS);
+  if (!v && PyErr_Occurred()) throw Failed();
+  return !v || n < as_int(v);
+}
 
 PyObject* cmat_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
   ARGS("cmat_mul", 3, S_w, S_act, S_y, S_n, S_bias, S_acc);
   const long long n = OPT_INT(a[3], 1);
-  if (n < 1 || n > FEW || !mul(Mat(a[0]), Act(a[1]), ptr(a[2]), (int)n, OPT_PTR(a[4]), OPT_BOOL(a[5], 0)))
+  if (!few(n) || !mul(Mat(a[0]), Act(a[1]), ptr(a[2]), (int)n, OPT_PTR(a[4]), OPT_BOOL(a[5], 0)))
     return PyObject_Vectorcall(slow(S_cmat_mul), args, nargs, kwnames);
   return ret(a[2]);
 } CATCH_ERRORS
 
 void mul_any(PyObject* w, PyObject* act, PyObject* y, long long n, PyObject* bias) {
-  if (n >= 1 && n <= FEW && mul(Mat(w), Act(act), ptr(y), (int)n, bias ? ptr(bias) : 0, 0)) return;
+  if (few(n) && mul(Mat(w), Act(act), ptr(y), (int)n, bias ? ptr(bias) : 0, 0)) return;
   PyObject* nn = PyLong_FromLongLong(n);
   Ref hold(nn);
   PyObject* av[5] = {w, act, y, nn, bias ? bias : Py_None};

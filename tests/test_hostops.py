@@ -60,3 +60,20 @@ def test_glu_mul_refuses_buffers_that_do_not_agree(fa, fb, n):
     act = D.make_qact(4 * 32, "q8", device="cpu")
     with pytest.raises(RuntimeError, match="do not agree|broadcast"):
         D.glu_mul(m, m, act, torch.zeros(fa), n, None if fb is None else torch.zeros(fb))
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="host tensors: only where nothing can be launched")
+def test_few_tokens_follow_tc_min_tokens(monkeypatch):
+    """TC_MIN_TOKENS below 16: cmat_mul sends what tc_takes() says to the tcgen05 kernel."""
+    sent = []
+    monkeypatch.setattr(D, "TC_MIN_TOKENS", 4)
+    monkeypatch.setattr(D, "TC_MIN_ROWS", 8)
+    monkeypatch.setattr(D, "_chunk_f16_of", lambda act, n, cols: n)
+    monkeypatch.setattr(D, "cmat_mul_tc", lambda w, cf, y, acc=False: sent.append((cf, acc)) or y)
+    w = D.CMat("w", 1, 8, 256, torch.zeros(8 * 144, dtype=torch.uint8))
+    for n in (4, 16):
+        assert D.tc_takes(w, n)
+        D.cmat_mul(w, D.make_qact(n * 256, "q8k", device="cpu"), torch.zeros(n * 8), n, acc=True)
+    assert sent == [(4, True), (16, True)]
+    with pytest.raises(RuntimeError):  # three tokens: a launch
+        D.cmat_mul(w, D.make_qact(3 * 256, "q8k", device="cpu"), torch.zeros(24), 3)
