@@ -102,8 +102,13 @@ struct Act {
   explicit Act(PyObject* o) : xq(attr_ptr(o, S_xq)), xs(attr_ptr(o, S_xs)), xsum(attr_ptr(o, S_xsum)) {
     Ref kind(PyObject_GetAttr(o, S_kind));
     k = !(PyUnicode_Check(kind.p) && PyUnicode_GetLength(kind.p) == 2);
-    Ref cf(PyObject_GetAttr(o, S__cf));
-    has_f16 = cf.p != Py_None;
+    PyObject* cf = PyObject_GetAttr(o, S__cf);  // an object of the caller's own may lack it
+    if (!cf) {
+      if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw Failed();
+      PyErr_Clear();
+    }
+    has_f16 = cf && cf != Py_None;
+    Py_XDECREF(cf);
   }
 };
 

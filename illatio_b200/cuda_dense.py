@@ -255,11 +255,11 @@ TC_Q6K = True
 
 def _chunk_f16_of(act, n, cols):
     """ACT's fp16 form for the tcgen05 product, made once per quantization of ACT (quant_q8 / rmsnorm_q8 mark it stale)."""
-    cf = act._cf
+    cf = getattr(act, "_cf", None)
     if cf is None or cf.n != n or cf.cols != cols:
         cf = act._cf = ChunkF16(n, cols, device=act.xq.device)
         act._cf_fresh = False
-    if not act._cf_fresh:
+    if not getattr(act, "_cf_fresh", False):
         cf.fill(act)
         act._cf_fresh = True
     return cf

@@ -2,6 +2,7 @@
 import os
 import subprocess
 import sys
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -77,3 +78,15 @@ def test_few_tokens_follow_tc_min_tokens(monkeypatch):
     assert sent == [(4, True), (16, True)]
     with pytest.raises(RuntimeError):  # three tokens: a launch
         D.cmat_mul(w, D.make_qact(3 * 256, "q8k", device="cpu"), torch.zeros(24), 3)
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="host tensors: only where nothing can be launched")
+def test_activations_of_the_callers_own_class():
+    """An object with a QAct's four attributes gets as far as the launch, and its fp16 form is made on it."""
+    a = D.make_qact(256, "q8k", device="cpu")
+    own = SimpleNamespace(kind=a.kind, xq=a.xq, xs=a.xs, xsum=a.xsum)
+    w = D.CMat("w", 1, 1, 256, torch.zeros(144, dtype=torch.uint8))
+    for call in (lambda: D.quant_q8(torch.zeros(256), own), lambda: D.rmsnorm_q8(torch.zeros(256), torch.ones(256), own, 256, 1e-6),
+                 lambda: D.cmat_mul(w, own, torch.zeros(1)), lambda: D._chunk_f16_of(own, 1, 256)):
+        with pytest.raises(RuntimeError):
+            call()
