@@ -105,9 +105,10 @@ def _quant_q8(x, act, f16_scale=True):
         act._cf_fresh = True
         return act
     act._cf, act._cf_fresh = None, False
-    quant_q8(x, act, f16_scale)
-    act._cf = cf
-    return act
+    try:
+        return quant_q8(x, act, f16_scale)
+    finally:
+        act._cf = cf
 
 
 def _rmsnorm_q8(x, w, act, d, eps, n=1, h=None, f16_scale=True):
@@ -120,9 +121,10 @@ def _rmsnorm_q8(x, w, act, d, eps, n=1, h=None, f16_scale=True):
         act._cf_fresh = True
         return act
     act._cf, act._cf_fresh = None, False
-    rmsnorm_q8(x, w, act, d, eps, n, h, f16_scale)
-    act._cf = cf
-    return act
+    try:
+        return rmsnorm_q8(x, w, act, d, eps, n, h, f16_scale)
+    finally:
+        act._cf = cf
 
 
 def _cmat_mul(w, act, y, n=1, bias=None, acc=False):

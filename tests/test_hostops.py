@@ -90,3 +90,15 @@ def test_activations_of_the_callers_own_class():
                  lambda: D.cmat_mul(w, own, torch.zeros(1)), lambda: D._chunk_f16_of(own, 1, 256)):
         with pytest.raises(RuntimeError):
             call()
+
+
+@pytest.mark.parametrize("call", [lambda act: D.quant_q8(torch.sparse_coo_tensor([[0]], [1.0], (512,)), act),
+                                  lambda act: D.rmsnorm_q8(torch.sparse_coo_tensor([[0]], [1.0], (512,)), torch.ones(512), act, 512, 1e-6)])
+def test_an_activation_keeps_its_f16_buffers_past_an_exception(call):
+    """A captured token may still use them."""
+    act = D.make_qact(512, "q8k", device="cpu")
+    cf = act._cf = SimpleNamespace(n=1, cols=256)
+    act._cf_fresh = True
+    with pytest.raises(RuntimeError):
+        call(act)
+    assert act._cf is cf and not act._cf_fresh
