@@ -671,7 +671,7 @@ def prefill_leg(D, B, torch, dev, dims, layers, fmt_main, fmt_alt, seed, n, tpea
            "int8_TOPS": tops, "frac_of_bf16_tensor_peak": tops / tpeak[0] if tpeak and tpeak[0] else None,
            "weight_MB_read_once": body / 1e6,
            "kernel": "Q4_K matrices of 2048 rows and more: mm_id_kernel<Q4_K> (tcgen05, ill_mm_chunk; fp16 integer operands, the "
-                     "activations' fp16 form made once per quantization by ill_act_f16); k (1024 rows) and the Q6_K matrices (v, down): "
+                     "activations' fp16 form made once per quantization by ill_act_f16); k and v (1024 rows): "
                      "mmd_kernel (int8 mma.sync, 128 rows x 128 tokens a CTA)",
            "parity": {"finite": finite, "chunk_vs_one_token_max_rel": worst, "ok": finite and worst < 2e-6}}
     del m, g

@@ -3,10 +3,9 @@
 // A decode step is a few hundred launches of one to ten microseconds, so what the host spends on one decides the
 // token: through ctypes an operator cost 9.4 us (3.2 of them torch.cuda.current_stream(), 0.8 the conversion of
 // the arguments, the rest attribute look-ups and the launch itself at 2.4), here it costs 3 (a B200 box's Xeon,
-// D.cmat_mul of 896 x 896).  The functions have the signatures and the behaviour that cuda_dense.py and
-// cuda_ds4f.py document; they read the same objects (CMat, QAct, ExpertPool) and call the same C ABI.  What is
-// rare or long -- prefill chunks, activations whose fp16 form is in use, errors -- goes to the Python functions
-// registered with set_slow().
+// D.cmat_mul of 896 x 896).  They are cuda_dense.py's operators: they read its objects (CMat, QAct) and call the same C
+// ABI.  What is rare or long -- prefill chunks, activations whose fp16 form is in use, errors -- goes to the Python
+// functions registered with set_slow().
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -240,8 +239,10 @@ PyObject* qkv_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
       const Act x(a[3]);
       const bool three = k.type == v.type;
       // Q4_K_M files keep V in Q6_K: V in a launch of its own.  In a stream that is being captured the Python form runs
-      // it beside Q and K (a fork and a join cost a graph nothing: a 4B token 1.54 ms, 1.57 one after the other); launch
-      // by launch, the two events and four calls of a fork cost the host more than the overlap gives.
+      // it beside Q and K (a fork and a join cost a graph nothing: a 4B token 1.54 ms, 1.57 one after the other).  Launch
+      // by launch, the fork's events and calls cost the host 21 us, and where the GPU is the bound all the same the overlap
+      // gives nothing: a layer's products one after the other and with the fork take 26 and 45 us at a hidden size of
+      // 1024, 41 and 47 at 2560, 58.4 and 58.5 at 4096, 81.6 and 82.3 at 5120, 137.2 and 137.4 at 8192.
       if (!three && capturing()) return PyObject_Vectorcall(slow(S_qkv_mul), args, nargs, kwnames);
       LAUNCH(ill_mv_3, q.type, q.w, k.w, three ? v.w : 0, q.rows, k.rows, three ? v.rows : 0, q.cols, x.xq, x.xs, x.k ? x.xsum : 0, ptr(a[4]),
              ptr(a[5]), three ? ptr(a[6]) : 0, OPT_PTR(a[7]), OPT_PTR(a[8]), three ? OPT_PTR(a[9]) : 0, cur_stream());

@@ -353,7 +353,8 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
 // ---- Q8_0 chunks ---------------------------------------------------------------------------------------------
 // What bounds a Q8_0 chunk is not the tensor pipe but what every m16n8k32 product needs after it: its four integers
 // become floats and meet d_w * d_x, because Q8_0's scales are per 32 columns on both sides.  So the kernel is built
-// around those instructions -- four conversions, four packed multiplies and two packed additions (f32x2) a product -- and keeps everything else off the issue slots:
+// around those instructions -- four conversions, four packed multiplies and two packed additions (f32x2) a product -- and
+// keeps everything else off the issue slots:
 //   * columns in steps of 128 (four blocks; a row's step is 136 bytes), weights and activations both by 16-byte
 //     cp.async into a ring of three stages, one __syncthreads a step;
 //   * what a thread copies lies at fixed distances from one step to the next: a step's copies are an add and a few
@@ -365,13 +366,14 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
 // A CTA of RW warps takes 16 RW rows x 8 NT8 tokens; few rows of many columns take small CTAs, several an SM.  A row's
 // blocks are added in order, each step rounded as in mmd_kernel: the same bits as it gave, whatever the tile.
 //
-// Measured against mmd_kernel, which took Q8_0 before: 2048 x 4096 x 4096 tokens 412 -> 298 us (231 int8 TOPS), 5120 x 1536
-// x 8192 728 -> 529, 4864 x 896 x 777 58 -> 39, 896 x 4864 x 777 129 -> 68, 2048 x 4096 x 64 62 -> 25.  What is left: about
-// 23 cycles a product of a scheduler where the packed arithmetic alone takes 12 and the int8 mma.sync 8.2, and 1.1 us a step
-// for unpacking, copying and the barrier.  Measured and dropped: 32 rows a warp (half the ldmatrix traffic, the same time);
-// the integers turned into floats by adding 1.5 * 2^23 in the product (4 % slower); the columns dealt to groups of a CTA's
-// warps (896 x 4864 x 777 in 40 us, but sums in another order: after a few layers' 8-bit activations that is a difference
-// of 1 % in a model's output); fused multiply-adds (5 % faster, other bits).
+// Measured against mmd_kernel, which took Q8_0 before: 2048 x 4096 x 4096 tokens 412 -> 295 us (233 int8 TOPS), 5120 x 1536
+// x 8192 728 -> 529, 4864 x 896 x 777 58 -> 37, 896 x 4864 x 777 129 -> 66, 2048 x 4096 x 64 62 -> 25.  What is left (the
+// first of these shapes): about 40 cycles a product and scheduler, 18.5 instructions of it at 50 % issue, where the packed
+// arithmetic alone takes 12 and the int8 mma.sync 8.2; the largest stalls are the shared-memory loads and the products'
+// results (1.2 warps an issue), fixed latencies (0.9) and the arithmetic pipe (0.9).  Measured and dropped: 32 rows a warp
+// (half the ldmatrix traffic, the same time); the integers turned into floats by adding 1.5 * 2^23 in the product (4 %
+// slower); the columns dealt to groups of a CTA's warps (896 x 4864 x 777 in 40 us, but sums in another order: after a few
+// layers' 8-bit activations that is a difference of 1 % in a model's output); fused multiply-adds (5 % faster, other bits).
 template <int NT8, int RW>
 struct Mq {
   static constexpr int TN = 8 * NT8, THREADS = 32 * RW;
@@ -550,9 +552,10 @@ __global__ void __launch_bounds__(Mq<NT8, RW>::THREADS, Mq<NT8, RW>::PER_SM) mmq
 // ---- up to sixteen tokens of rows too long for mvt.cu to keep the activations resident ------------------------
 // One 16-row tile a CTA, its column steps dealt to the eight warps (warp w takes steps w, w + 8, ...): each warp
 // streams its own steps' weights (its ring of three stages) AND its own steps' activations (two buffers of its own), all
-// by 16-byte cp.async of its lanes (Q6_K 5120 x 17408, 4 tokens: 40 us; 59 with a bulk copy a row segment), so the warps never wait for one another until the end, where their partial sums meet in shared memory
-// in warp order.  A matrix of few rows and many columns (5120 x 17408) thus fills the machine with rows / 16 CTAs
-// of eight busy warps, where the chunk kernel above would run two warps a CTA through all 68 steps.
+// by 16-byte cp.async of its lanes (Q6_K 5120 x 17408, 4 tokens: 40 us; 59 with a bulk copy a row segment), so the warps
+// never wait for one another until the end, where their partial sums meet in shared memory in warp order.  A matrix of few
+// rows and many columns (5120 x 17408) thus fills the machine with rows / 16 CTAs of eight busy warps, where the chunk
+// kernel above would run two warps a CTA through all 68 steps.
 template <int FMT, int NT8>
 __global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
   extern __shared__ __align__(128) u8 smem[];
@@ -574,7 +577,8 @@ __global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
 #pragma unroll
       for (int h = 0; h < 16; h += 8)
         if (row_base + h + g < p.rows)
-          copy_segment<(SB + 30) / 16>(st + (size_t)(h + g) * p.pitch, p.w + (long long)(row_base + h + g) * p.row_bytes + (long long)step * SB, len, t);
+          copy_segment<(SB + 30) / 16>(st + (size_t)(h + g) * p.pitch,
+                                       p.w + (long long)(row_base + h + g) * p.row_bytes + (long long)step * SB, len, t);
     }
     cp_async_commit();
   };
@@ -692,8 +696,10 @@ static int mmd_launch(const MdParams& p, int tn, size_t smem, int grid, cudaStre
 // The launch of a Q8_0 chunk.  Which tile: the one with the least estimated time, steps x (time a step) x (how often the
 // SMs are filled).  STEP is the time in us of a step with every SM full, measured on 2048 x 4096 x 4096 tokens.  CTAs that do
 // not fill the SMs take less of it, but not in proportion: what counts, over every tile, is how many warps the GPU holds --
-// 0.4 of STEP up to 256 warps, 0.55 at 512, 0.8 at 640, all of it at 2368 (sixteen an SM).  Over 20 shapes of 17 to 8192
-// tokens the tile it picks is the fastest measured or within 9 % of it (896 x 4864 x 17 tokens: 28 us against 23).
+// 0.4 of STEP up to 256 warps, 0.55 at 512, 0.8 at 640, all of it at 2368 (sixteen on each of a B200's 148 SMs).  Over eight
+// matrices of 128 to 5120 rows at 17, 64, 200, 777 and 4096 tokens it takes the fastest tile or one within 5 % of it for 34
+// of the 40; it is furthest off at 200 tokens of 896 rows (x 4864: 51 us against 39, x 896: 9.6 against 7.3), then 128 x 896 x
+// 4096 (14.8 against 12.2), 2048 x 4096 x 200 (64 against 54), 5120 x 1536 x 17 and 1536 x 5120 x 200 (15 and 11 %).
 struct MqTile {
   float step;
   int rn, tn, threads, per_sm;
@@ -845,11 +851,9 @@ int mmk_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
   if (fmt == ILL_Q4_K) off += (uint32_t)tn * MdFrag<ILL_Q4_K>::SPITCH;
   p.xbuf_bytes = (off + 127) / 128 * 128;
   p.ring_off = 2 * MD_WARPS * p.xbuf_bytes;
-  p.stages = MD_MAX_STAGES;
-  p.part_off = (uint32_t)((p.ring_off + (size_t)MD_WARPS * p.stages * p.stage_bytes + 127) / 128 * 128);
+  p.part_off = (uint32_t)((p.ring_off + (size_t)MD_WARPS * MD_MAX_STAGES * p.stage_bytes + 127) / 128 * 128);
   const size_t smem = p.part_off + (size_t)MD_WARPS * 16 * tn * 4;
   if (smem > 226 * 1024) return ILL_ERR_UNSUPPORTED;
-  p.status = device_status_word();
   const long long grid = (long long)((rows + 15) / 16) * ((n + tn - 1) / tn);
   if (grid > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;

@@ -363,7 +363,7 @@ int mvt_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
   p.n = n;
   // a row's segment: its block's 16-byte aligned span, rows a multiple of 16 bytes apart that is an odd multiple
   // of 16 mod 128 (eight rows x four words then sit on 32 different banks)
-  // blocks a piece: about 200-300 bytes a row segment (a bulk copy each), but every warp should get a piece
+  // blocks a piece: about 200-300 bytes a row segment (four lanes' copies), but every warp should get a piece
   int cb = fmt == ILL_Q8_0 ? 8 : fmt == ILL_Q4_K ? 2 : 1;
   while (cb > 1 && (p.nblocks + cb - 1) / cb < MT_WARPS) cb >>= 1;
   p.cb = cb;

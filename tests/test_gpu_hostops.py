@@ -103,3 +103,37 @@ def test_other_threads_run_while_a_launch_waits(cuda_lib):
     torch.cuda.synchronize()
     assert took > 0.3, "the queue never filled"
     assert gap[0] < took / 3, (gap[0], took)
+
+
+@pytest.mark.parametrize("n", [1, 3, 17])
+@pytest.mark.parametrize("fmts", [(B.Q4_K, B.Q4_K, B.Q6_K), (B.Q4_K, B.Q4_K, B.Q4_K), (B.Q4_K, B.Q6_K, B.Q6_K)])
+def test_qkv_mul_of_mixed_formats_eager_and_captured(cuda_lib, fmts, n):
+    """Q, K and V with biases in one format, with V in another and with Q in another: three products' values, launched one by
+    one and replayed from a graph (where V runs beside Q and K) with other activations each time."""
+    cols, rows = 512, (96, 40, 24)
+    w = [_mat(f, r, cols, 3 + i) for i, (f, r) in enumerate(zip(fmts, rows))]
+    g = torch.Generator(device="cuda").manual_seed(n)
+    b = [torch.randn(r, device="cuda", generator=g) for r in rows]
+    x, act = torch.empty(n * cols, device="cuda"), D.make_qact(n * cols, "q8k")
+    y, want = ([torch.full((n * r,), -1.0, device="cuda") for r in rows] for _ in range(2))
+
+    def step():
+        D.quant_q8(x, act)
+        D.qkv_mul(*w, act, *y, bq=b[0], bk=b[1], bv=b[2], n=n)
+
+    x.normal_(generator=g)
+    step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    for run in (step, graph.replay, graph.replay):
+        x.normal_(generator=g)
+        for t in y:
+            t.fill_(-1.0)
+        run()
+        other = D.quant_q8(x, D.make_qact(n * cols, "q8k"))
+        for m, bias, t in zip(w, b, want):
+            D.cmat_mul(m, other, t, n, bias=bias)
+        for got, t in zip(y, want):  # (one launch for several matrices may add a row's float terms in another order)
+            assert (got - t).abs().max() <= 2e-6 * t.abs().max()
