@@ -85,9 +85,10 @@ __global__ void __launch_bounds__(256) quant_q8_k_kernel(const float* __restrict
 // norm is not one CTA's serial work.  The double sum is taken in the order quantdev.cuh fixes, not in the
 // CPU loop's; the two agree until the float the sum is rounded to sits within 1e-16 of a rounding boundary.
 // Bound by latency: the norm's weights are on their way to L2 before the kernel waits for the one before it (which may have
-// written them), a warp asks for four of its groups and its first block's values at once, and a few rows are spread over their
-// blocks too (in a graph of norms, before and now: 16 rows of 2560 3.8 -> 2.6 us, 4 of 5120 5.1 -> 2.8, one of 2560 3.0 -> 2.5,
-// 512 of 5120 13.9 -> 7.1).  VEC: Q8_0 blocks by four values a lane (X, W, H and XQ aligned for it).
+// written them; more rows than SMs find them there), a warp asks for four of its groups and its first block's values at once,
+// and a few rows are spread over their blocks too (in a graph of norms, before and now: 16 rows of 2560 3.8 -> 2.6 us, 4 of
+// 5120 5.1 -> 2.8, one of 2560 3.0 -> 2.4, 512 of 5120 13.9 -> 6.8).  VEC: Q8_0 blocks by four values a lane (X, W, H and XQ
+// aligned for it).
 template <int K8K, bool F16, bool VEC>
 __global__ void __launch_bounds__(256) rmsnorm_q8_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                          float* __restrict__ h, i8* __restrict__ xq, float* __restrict__ xs,
@@ -106,16 +107,14 @@ __global__ void __launch_bounds__(256) rmsnorm_q8_kernel(const float* __restrict
       v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
     } else v[0] = src[b * 32 + lane];
   };
-  if (b0 < nb && b0 * BW + VL * lane < d) prefetch_l2(w + b0 * BW + VL * lane);
+  if (gridDim.y <= 148 && b0 < nb && b0 * BW + VL * lane < d) prefetch_l2(w + b0 * BW + VL * lane);
   pdl_launch_dependents();
   pdl_wait();
   w = after_wait(w);
   const long long base = (long long)blockIdx.y * d;
   const float* xr = after_wait(x + base);
-  if (b0 < nb) {
-    load(w, b0, wv);
-    load(xr, b0, x0);
-  }
+  if (!K8K && b0 < nb) load(w, b0, wv);
+  if (b0 < nb) load(xr, b0, x0);
   const int ng = (d + 255) / 256;
   for (int g0 = warp; g0 < ng; g0 += 32) {
     float v[4][8];
@@ -129,6 +128,7 @@ __global__ void __launch_bounds__(256) rmsnorm_q8_kernel(const float* __restrict
         if (lane == 0) group_s[g0 + 8 * k] = s;
       }
   }
+  if (K8K && b0 < nb) load(w, b0, wv);  // (eight registers a lane less while the row's sum is taken)
   __syncthreads();
   const float sc = rms_scale(rms_total(group_s, ng, lane), d, eps);
   for (int b = b0; b < nb; b += gridDim.x * 8) {
