@@ -44,18 +44,33 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// Whether the phase of parity PARITY has completed, without waiting (about 60 cycles; a try_wait with a time hint about 90).
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // One poll: the thread may be suspended by the hardware for up to HINT_NS nanoseconds while the
 // phase is incomplete (it takes no issue slots meanwhile).
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity, uint32_t hint_ns) {
+__device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity, uint32_t hint_ns) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(hint_ns)
+      : "r"(bar), "r"(parity), "r"(hint_ns)
       : "memory");
   return ok != 0;
+}
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity, uint32_t hint_ns) {
+  return mbar_try_wait_at(smem_u32(bar), parity, hint_ns);
 }
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -68,7 +83,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // clock is read once in 64 polls.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned int* status, unsigned int code,
                                           unsigned sleep_ns = 0, unsigned long long limit_ns = ILL_WAIT_NS) {
-  if (mbar_try_wait(bar, parity, 0)) return true;
+  if (mbar_test(bar, parity)) return true;
   unsigned long long t0 = 0;
   for (unsigned it = 1;; ++it) {
     if (sleep_ns) __nanosleep(sleep_ns);

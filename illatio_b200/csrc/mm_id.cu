@@ -9,28 +9,27 @@
 // or Q2_K blocks at ptrs[e] + add -- or of Q4_K / Q6_K blocks: the dense prefill products run through the same
 // kernel with the matrix as its one expert (ill_mm_chunk; mm_q4k_mma / mm_q6k_mma, src/cuda/kquant.cu:316-466).
 //
-// A persistent grid (a CTA per SM) walks tiles of 128 weight rows x up to 128 rows of X.  The
+// A persistent grid (a CTA per SM) walks tiles of 128 weight rows x up to NT (64, 128 or 256) rows of X.  The
 // weights are the tensor core's A operand and live in tensor memory: the dequantizing warps write
 // their integer parts (exact in fp16) there with tcgen05.st, so they never pass through shared
 // memory; X is the B operand, brought by TMA (128-byte swizzle).  The accumulator
 // D[weight row, row of X] is drained once per 256-wide block of K and scaled by the block's two
-// float scales, which is the order the reference's CPU kernels multiply in.
-//   warp 0      one lane issues the TMA loads of the X tiles
+// float scales.
+//   warp 0      brings the X tiles by TMA, no more rows than the tile has (to the next 32)
 //   warp 1      allocates tensor memory; one lane issues tcgen05.mma (128 x N x 16, fp16 in,
 //               fp32 accumulate) and commits each step back to the producers
-//   warps 2-3   bring W_e's raw blocks and the X rows' block scales into rings in shared memory
-//               (cp.async)
-//   warps 4-7   drain the accumulators block by block (tcgen05.ld), scaling each block's integer
+//   warps 4-..  drain the accumulators block by block (tcgen05.ld), scaling each block's integer
 //               sums by the block's float scales; then store the tile (a lane = a weight row, so
 //               the 32 lanes of a warp write 128 contiguous bytes of a row of Y)
-//   warps 8-23  turn the raw blocks into the A operand (four threads a weight row, a K step each)
+//   the others  bring W_e's raw blocks into shared memory (cp.async) and turn them into the A operand
 // The roles' register needs differ widely, so the warp groups trade registers (setmaxnreg).
 // Every mbarrier wait is bounded; on a time-out the kernel records a code in the status
-// word, skips what depends on the wait, frees its tensor memory and returns.
+// word, skips what depends on the wait, lets copies and products in flight end, frees its tensor memory and returns.
 //
 // Replaces d4_mm_id_iq2_xxs / d4_mm_id_q2_k (src/cuda/ds4f_mm.cu:229-257: mma.sync
 // m16n8k16, 64x64 tiles) behind DK-FFN-ROUTED-CHUNK (src/cuda-ds4f-prefill.lisp:315-356).
 #include <cuda.h>
+#include <string.h>
 
 #include "formats.cuh"
 #include "iq2xxs_tables.cuh"
@@ -39,17 +38,9 @@
 
 namespace ill {
 
-constexpr int MM_BM = 128;                             // rows of X a tile (the MMA's N)
 constexpr int MM_BN = 128;                             // weight rows a tile (the MMA's M)
 constexpr int MM_BK = 64;                              // K step: one 128-byte row of the swizzled X tile
-constexpr int MM_RS = 3;                               // stages of the ring of raw weight blocks
-constexpr int MM_XSC = 16;                             // blocks of X scales kept (the loader runs < 16 blocks ahead of the drain)
-constexpr int MM_DR_WARPS = 4, MM_DQ_WARPS = 16, MM_LD_WARPS = 2;  // drain, dequantize, raw-load warps
-// Registers a thread after the roles part: the four warps of TMA / MMA / raw loads give theirs up, the
-// drain warps (a whole tile's row of 128 sums each) take them
-constexpr int MM_REGS_AUX = 40, MM_REGS_DRAIN = 184, MM_REGS_DQ = 64;
-constexpr int MM_THREADS = 32 * (2 + MM_LD_WARPS + MM_DR_WARPS + MM_DQ_WARPS);  // + the TMA warp and the MMA warp
-constexpr uint32_t MM_TILE_BYTES = MM_BM * MM_BK * 2;  // 16 KB
+constexpr int MM_XBOX = 32;                            // rows of X a load brings, or two, three or four times as many
 
 struct MmParams {
   int ncols, nrows;            // K and N of every expert matrix
@@ -73,6 +64,7 @@ struct MmParams {
   unsigned long long one_ptr;
   unsigned one_count;
   int acc;
+  int bm;                      // rows of X a tile, at most the kernel's NT
 };
 // (DENSE is a template argument of the kernel, so that the experts' launches compile to what they were without it)
 template <bool DENSE> __device__ __forceinline__ unsigned long long mm_ptr(const MmParams& p, int e) {
@@ -91,6 +83,13 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
           smem_u32(dst)),
       "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+          smem_u32(dst)),
+      "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
@@ -113,7 +112,7 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(acc)
       : "memory");
 }
-// the same with A in shared memory (K-major, 128-byte swizzle)
+// the same with A in shared memory (K-major)
 __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -122,9 +121,9 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t adesc, uin
       : "memory");
 }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// 16-byte chunk C of row ROW of a K-major tile with the 128-byte swizzle
-__device__ __forceinline__ void store_chunk(u8* tile, int row, int c, uint4 v) {
-  *(uint4*)(tile + (row >> 3) * 1024 + (row & 7) * 128 + ((c ^ (row & 7)) << 4)) = v;
+// 16-byte chunk C (0, 1) of row ROW of a K-major tile of 32-byte rows with the 32-byte swizzle
+__device__ __forceinline__ void store_chunk32(u8* tile, int row, int c, uint4 v) {
+  *(uint4*)(tile + row * 32 + ((c ^ ((row >> 2) & 1)) << 4)) = v;
 }
 // arrive on BAR once every tcgen05.mma issued so far by this thread has completed
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -137,19 +136,30 @@ __device__ __forceinline__ uint64_t umma_desc(const void* tile) {
   return addr | (1ull << 16) /* leading offset: 16 B, unused with a swizzle */ | ((uint64_t)(1024 >> 4) << 32) |
          (1ull << 46) /* descriptor version of sm_100 */ | (2ull << 61) /* SWIZZLE_128B */;
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+// the same for rows of 32 bytes, 32-byte swizzle: 8-row groups 256 bytes apart
+__device__ __forceinline__ uint64_t umma_desc32(const void* tile) {
+  const uint64_t addr = (uint64_t)(smem_u32(tile) >> 4) & 0x3fffu;
+  return addr | (1ull << 16) | ((uint64_t)(256 >> 4) << 32) | (1ull << 46) | (6ull << 61) /* SWIZZLE_32B */;
 }
-// this lane's 16 (4) words into 16 (4) consecutive columns of its tensor-memory lane
+// eight columns of this lane's row of tensor memory; the registers are filled only after the wait
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+// V passes through, so that nothing that uses it is moved ahead of the wait before this
+__device__ __forceinline__ void tmem_ld_done(uint32_t (&v)[8]) {
+  asm volatile("" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]));
+}
+// waits for this warp's loads
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
+               :
+               : "memory");
+}
+// this lane's 16 (8) words into 16 (8) consecutive columns of its tensor-memory lane
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
@@ -160,11 +170,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
                "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t* v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]),
-               "r"(v[3])
                : "memory");
 }
 // true in one lane of the (converged) warp
@@ -214,10 +219,7 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
   return d;
 }
 
-// 4 bytes global -> shared, asynchronously (both addresses 4-byte aligned)
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
+// 16 bytes global -> shared, asynchronously
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {  // both 16-byte aligned
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
@@ -232,38 +234,39 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // the 32 integers grid * sign * (2 LS + 1) (at most 43 * 31: exact in fp16).  The block's float
 // part is d / 8 (src/avx2.lisp:77-110 takes the products this way).  GRID points at this lane's copy
 // of the grid as halves (16 bytes an entry, eight interleaved copies: entry e of copy c at [8 e + c],
-// so the eight lanes of a 128-bit request's quarter never share a bank); SGN likewise at the table
-// that gives, for the seven stored sign bits, the sign bits of the eight halves (the eighth sign is
-// the parity of the seven: ksigns_iq2xs[i] = i | parity(i) << 7).
-__device__ __forceinline__ void w_iq2xxs(uint32_t idx, uint32_t aux, const uint4* grid, const uint4* sgn, uint32_t* out) {
+// so the eight lanes of a 128-bit request's quarter never share a bank).  SGN points at this lane's copy of the
+// signs (a word an entry, 32 copies: one wavefront a request): for the seven stored bits, the eight sign bits s (the
+// eighth is the parity of the seven: ksigns_iq2xs[i] = i | parity(i) << 7) as s << 9 | s << 24, so that a shift by
+// 6 - 2 k brings signs 2 k and 2 k + 1 to the sign bits of the k-th pair of halves.  (A table of the eight halves' sign
+// bits, 16 bytes an entry, costs four wavefronts a look-up.)
+__device__ __forceinline__ void w_iq2xxs(uint32_t idx, uint32_t aux, const uint4* grid, const uint32_t* sgn, uint32_t* out) {
   const uint32_t s2 = small_h2(2 * (aux >> 28) + 1);
-  uint4 g[4], m[4];
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
-    g[l] = grid[8 * ((idx >> (8 * l)) & 0xff)];
-    m[l] = sgn[8 * ((aux >> (7 * l)) & 127u)];
-  }
-#pragma unroll
-  for (int l = 0; l < 4; ++l) {
-    out[4 * l] = hmul2(g[l].x, s2) ^ m[l].x;
-    out[4 * l + 1] = hmul2(g[l].y, s2) ^ m[l].y;
-    out[4 * l + 2] = hmul2(g[l].z, s2) ^ m[l].z;
-    out[4 * l + 3] = hmul2(g[l].w, s2) ^ m[l].w;
+    const uint4 g = grid[8 * ((idx >> (8 * l)) & 0xff)];
+    const uint32_t m = sgn[32 * ((aux >> (7 * l)) & 127u)];
+    out[4 * l] = hmul2(g.x, s2) ^ ((m << 6) & 0x80008000u);
+    out[4 * l + 1] = hmul2(g.y, s2) ^ ((m << 4) & 0x80008000u);
+    out[4 * l + 2] = hmul2(g.z, s2) ^ ((m << 2) & 0x80008000u);
+    out[4 * l + 3] = hmul2(g.w, s2) ^ (m & 0x80008000u);
   }
 }
 
-// Q2_K: the 32 weights at shift K of a half's 32 quant bytes Q: (scale & 15) * q (at most 45), the
-// scales SC_LO for the first sixteen and SC_HI for the rest (src/kquant.lisp:DEQUANTIZE-ROW-Q2-K order).
-__device__ __forceinline__ void w_q2k(const uint32_t* q, int k, uint32_t sc_lo, uint32_t sc_hi, uint32_t* out) {
+// byte I of V as the half 1024 + byte, twice
+__device__ __forceinline__ uint32_t byte_h2_1024(uint32_t v, int i) { return __byte_perm(v, 0x64646464u, 0x4040u + 0x0101u * i); }
+// 4 NW weights from the NW words Q: their fields under MASK, 2^SH too large where they lie, times the scale in byte I of SC.
+// 1024 + 2^SH q has the byte's bits under the exponent of 1024; times s / 2^SH, less 1024 s / 2^SH, it is s q exactly (Q2_K: at
+// most 45, Q4_K: 945; the fused multiply-add rounds once): no shift, no conversion.
+template <int NW, int SH>
+__device__ __forceinline__ void w_fields(const uint32_t* q, uint32_t mask, uint32_t sc, int i, uint32_t* out) {
+  constexpr uint32_t inv = (uint32_t)(15 - SH) << 10, inv2 = inv | inv << 16;             // 2^-SH, twice
+  constexpr uint32_t off = 0x8000u | (uint32_t)(25 - SH) << 10, off2 = off | off << 16;  // -1024 / 2^SH, twice
+  const uint32_t s2 = hfma2(byte_h2_1024(sc, i), inv2, off2), bias = hmul2(s2, 0xe400e400u /* -1024 */);
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const uint32_t s2 = small_h2((half ? sc_hi : sc_lo) & 15u), bias = hmul2(s2, 0xe400e400u /* -1024 */);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t v = (q[4 * half + i] >> (2 * k)) & 0x03030303u;
-      out[8 * half + 2 * i] = hfma2(bytes_to_h2_1024(v, 0x4140), s2, bias);
-      out[8 * half + 2 * i + 1] = hfma2(bytes_to_h2_1024(v, 0x4342), s2, bias);
-    }
+  for (int k = 0; k < NW; ++k) {
+    const uint32_t v = q[k] & mask;
+    out[2 * k] = hfma2(bytes_to_h2_1024(v, 0x4140), s2, bias);
+    out[2 * k + 1] = hfma2(bytes_to_h2_1024(v, 0x4342), s2, bias);
   }
 }
 // Q2_K: eight mins (scale bytes M0, M1 >> 4) as four words
@@ -276,49 +279,28 @@ __device__ __forceinline__ void w_q2k_mins(uint32_t m0, uint32_t m1, uint32_t* v
   for (int i = 0; i < 4; ++i) asm("add.rn.f16x2 %0, %0, %1;" : "+r"(v[i]) : "r"(k1024));
 }
 
-// Per format.  A 256-wide block is four K steps; for Q2_K it also has a tile of the activations' sums
-// of 16, multiplied with the mins (one K = 16 MMA into a second accumulator).
-// Tensor memory, 512 columns: accumulators D[2] at 0 and 128 (a column = a row of X); then
-//   IQ2_XXS  the A ring, 8 K steps x 32 columns, at 256
-//   Q2_K     the mins' accumulator at 256; the A ring, 4 K steps, at 384 (the mins themselves, a
-//   Q4_K     128 x 16 operand, go through two tiles in shared memory)
-// Q4_K: byte I (0..11) of the block's packed scales and mins, held as the three words S
-__device__ __forceinline__ uint32_t q4k_sb(const uint32_t* s, int i) { return (s[i >> 2] >> (8 * (i & 3))) & 0xffu; }
-// get_scale_min_k4 (src/kquant.lisp:64-72): group J's 6-bit scale and min
-__device__ __forceinline__ void q4k_scale_min(const uint32_t* s, int j, uint32_t& sc, uint32_t& mn) {
-  if (j < 4) { sc = q4k_sb(s, j) & 63u; mn = q4k_sb(s, j + 4) & 63u; }
-  else { sc = (q4k_sb(s, j + 4) & 0xFu) | ((q4k_sb(s, j - 4) >> 6) << 4); mn = (q4k_sb(s, j + 4) >> 4) | ((q4k_sb(s, j) >> 6) << 4); }
-}
-// Q4_K: 4 NW weights of a group -- the low (HI = 0) or high nibbles of the NW words of quant bytes Q -- times the
-// group's scale: at most 15 * 63 = 945, exact in fp16 (the fused multiply-add rounds once)
-template <int NW>
-__device__ __forceinline__ void w_q4k(const uint32_t* q, int hi, uint32_t sc, uint32_t* out) {
-  const uint32_t s2 = small_h2(sc), bias = hmul2(s2, 0xe400e400u /* -1024 */);
-#pragma unroll
-  for (int i = 0; i < NW; ++i) {
-    const uint32_t v = (q[i] >> (4 * hi)) & 0x0f0f0f0fu;
-    out[2 * i] = hfma2(bytes_to_h2_1024(v, 0x4140), s2, bias);
-    out[2 * i + 1] = hfma2(bytes_to_h2_1024(v, 0x4342), s2, bias);
-  }
+// Q4_K: the four 6-bit scales and the four mins of half H of a block, a byte each, from the twelve packed bytes S
+// (get_scale_min_k4, src/kquant.lisp:64-72, four at a time)
+__device__ __forceinline__ void q4k_scales_mins(const uint32_t* s, int h, uint32_t& sc, uint32_t& mn) {
+  sc = h ? (s[2] & 0x0f0f0f0fu) | ((s[0] >> 2) & 0x30303030u) : s[0] & 0x3f3f3f3fu;
+  mn = h ? ((s[2] >> 4) & 0x0f0f0f0fu) | ((s[1] >> 2) & 0x30303030u) : s[1] & 0x3f3f3f3fu;
 }
 // Q4_K: four groups' mins, each twice (a group of 32 faces two of the activations' sums of 16), as four words
-__device__ __forceinline__ void w_q4k_mins(const uint32_t* s, int g0, uint32_t* v) {
+__device__ __forceinline__ void w_q4k_mins(uint32_t mn, uint32_t* v) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    uint32_t sc, mn;
-    q4k_scale_min(s, g0 + i, sc, mn);
-    v[i] = small_h2(mn);
+    v[i] = byte_h2_1024(mn, i);
+    asm("add.rn.f16x2 %0, %0, %1;" : "+r"(v[i]) : "r"(0xe400e400u));  // - 1024
   }
 }
 
-// N words starting BYTE_OFF bytes into the row's window RW (any 2-byte alignment of the offset is taken up by funnel shifts)
+// N words at RW of a row whose block starts SH / 8 (0 or 2) bytes into its first word
 template <int N>
-__device__ __forceinline__ void raw_words(const uint32_t* rw, uint32_t byte_off, uint32_t* out) {
-  const uint32_t w0 = byte_off >> 2, sh = (byte_off & 3u) * 8u;
-  uint32_t prev = rw[w0];
+__device__ __forceinline__ void raw_words(const uint32_t* rw, uint32_t sh, uint32_t* out) {
+  uint32_t prev = rw[0];
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const uint32_t next = rw[w0 + i + 1];
+    const uint32_t next = rw[i + 1];
     out[i] = __funnelshift_r(prev, next, sh);
     prev = next;
   }
@@ -345,73 +327,164 @@ __device__ __forceinline__ void w_q6k(const uint32_t* ql, const uint32_t* qh, in
   }
 }
 
-template <int FMT> struct MmGeom {
-  static constexpr bool KM = FMT == ILL_Q2_K || FMT == ILL_Q4_K;  // formats with mins: a second, small product a block
-  static constexpr int BB = FMT == ILL_Q2_K ? 84 : FMT == ILL_Q4_K ? 144 : FMT == ILL_Q6_K ? 210 : 66;
-  static constexpr int NSLOT = KM || FMT == ILL_Q6_K ? 4 : 8;  // a multiple of four: a slot is always written by the same warps
-  static constexpr int NX = FMT == ILL_Q4_K ? 5 : KM ? 6 : FMT == ILL_Q6_K ? 6 : 8;  // stages of the ring of X tiles = K steps in flight
-  // A dequantizing warp waits for K step st - NSLOT on barrier (st - NSLOT) % NX; the barrier's next phase (K step
-  // st - NSLOT + NX) must not be able to complete before that warp has passed, or the parity it waits for comes round again
-  static_assert(NX >= NSLOT, "the ring of K-step barriers must be at least as long as the ring of A slots");
-  static constexpr int NE = KM ? 4 : 0;     // Q2_K, Q4_K: two tiles of X's sums of 16, two of the mins
-  static constexpr uint32_t A_COL = KM ? 384 : 256, DM_COL = 256;
-  static constexpr uint32_t SLOTW = FMT == ILL_Q6_K ? 64 : 32;  // columns of an A slot (Q6_K: the even and the odd part)
-  // A row's raw block reaches shared memory as the WIN bytes from the 16-byte boundary at or before it,
-  // PITCH bytes apart (Q4_K: blocks of 144 bytes in rows that the launcher wants 16-byte aligned)
-  static constexpr uint32_t WIN = FMT == ILL_Q2_K ? 96 : FMT == ILL_Q4_K ? 144 : FMT == ILL_Q6_K ? 224 : 80;
-  static constexpr uint32_t PITCH = FMT == ILL_Q2_K ? 112 : FMT == ILL_Q4_K ? 160 : FMT == ILL_Q6_K ? 240 : 80;
-  static constexpr uint32_t RAW_BYTES = 128 * PITCH;
-  static constexpr size_t SMEM = (size_t)(NX + NE) * MM_TILE_BYTES + MM_RS * RAW_BYTES + 16 /* a word past the last row is read */ +
-                                 512 /* barriers */ + 4 * 256 * 4 /* weight scales */ + MM_XSC * 128 * 4 /* X scales */ +
-                                 2304 /* experts' first tiles */ + (FMT == ILL_IQ2_XXS ? 8 * 4096 + 8 * 2048 : 0) /* tables */ +
-                                 1024 /* alignment */;
+// The barriers that a role's lanes watch, one each: one poll shows all their phases.  Waiting is bounded as in mbar_wait.
+struct MmPoll {
+  unsigned int* status;
+  unsigned code, ready = 0;
+  __device__ __forceinline__ MmPoll(unsigned int* st, unsigned c) : status(st), code(c) {}
+  // until the phases of parity PAR of the BARs of the lanes in NEED have completed; the same answer in every lane
+  __device__ __forceinline__ bool until(uint64_t* bar, uint32_t par, uint32_t need) {
+    if ((ready & need) == need) return true;
+    unsigned long long t0 = 0;
+    for (unsigned it = 1;; ++it) {
+      ready = __ballot_sync(0xffffffffu, mbar_test(bar, par));
+      const uint32_t missing = need & ~ready;
+      if (!missing) return true;
+      // the warp sleeps on the first that is missing (and takes no issue slots meanwhile)
+      const int l = __ffs(missing) - 1;
+      mbar_try_wait_at(__shfl_sync(0xffffffffu, smem_u32(bar), l), __shfl_sync(0xffffffffu, par, l), 20000);
+      if ((it & 63u) == 0) {
+        const unsigned long long now = __shfl_sync(0xffffffffu, global_ns(), 0);
+        if (t0 == 0) t0 = now;
+        else if (now - t0 > ILL_WAIT_NS) break;
+      }
+    }
+    if (status) atomicCAS(status, 0u, code);
+    return false;
+  }
 };
 
-template <int FMT, bool DENSE>
-__global__ void __launch_bounds__(MM_THREADS) mm_id_kernel(const __grid_constant__ CUtensorMap xmap,
-                                                           const __grid_constant__ CUtensorMap emap, const MmParams p) {
-  typedef MmGeom<FMT> G;
-  constexpr int BB = G::BB, NSLOT = G::NSLOT, NX = G::NX;
+// The tensor maps of X (rows of 64 halves, two K steps a load) and of its sums of 16 for loads of 32, 64, 96 and 128 rows
+struct MmMaps {
+  CUtensorMap x[4], e[4];
+};
+__device__ __forceinline__ int mm_boxes(int rows) { return max(1, (rows + MM_XBOX - 1) / MM_XBOX); }
+
+// Geometry per format and per NT, the most rows of X a tile has (64, 128 or 256).  A 256-wide block is four K steps; the
+// formats with mins (KM) have a second, small product a block: the mins against the activations' sums of 16 (one K = 16 MMA).
+// A tile of up to 128 rows is one job a block (one accumulator); a tile of up to 256 is two, its halves, against the same
+// A operand: a block's weights are then unpacked once for twice the rows.
+// Tensor memory, 512 columns (an accumulator's column = a row of X):
+//   D[2] at 0, two accumulators that alternate job by job; KM: the mins' accumulator (two when NT is 64); then the ring
+//   of A slots, a K step each, to the end
+template <int FMT, int NT> struct MmGeom {
+  static constexpr bool KM = FMT == ILL_Q2_K || FMT == ILL_Q4_K;
+  static constexpr int BB = FMT == ILL_Q2_K ? 84 : FMT == ILL_Q4_K ? 144 : FMT == ILL_Q6_K ? 210 : 66;
+  static constexpr int HALVES = NT > 128 ? 2 : 1;
+  static constexpr int DC = NT < 128 ? NT : 128;            // columns of an accumulator
+  // Dequantizing warps: a set of eight makes a block -- four (32 weight rows each) its first half of K, four the second --
+  // and two sets take the CTA's blocks in turn.  In wide tiles, and in tiles of 128 with two accumulators a block, the way out
+  // of tensor memory takes longer than the way in, and a second set's registers go to it.
+  static constexpr int SETS = NT < 128 || (NT == 128 && !KM) ? 2 : 1, DQ_WARPS = 8 * SETS;
+  // Drain warps: DR_GROUPS times four (32 weight rows each); a group takes every DR_GROUPS-th eight columns
+  static constexpr int DR_GROUPS = NT == 128 && KM ? 4 : 2, DR_WARPS = 4 * DR_GROUPS;
+  static constexpr int THREADS = 32 * (4 + DR_WARPS + DQ_WARPS);
+  // registers a thread after the roles part (the sum must fit in what the CTA was launched with: checked by the host)
+  static constexpr int REGS_AUX = 40, REGS_DRAIN = NT > 128 ? 160 : DR_GROUPS == 4 ? 88 : 120, REGS_DQ = 56;
+  static constexpr int REGS_SUM = 128 * REGS_AUX + 32 * (DR_WARPS * REGS_DRAIN + DQ_WARPS * REGS_DQ);
+  static constexpr uint32_t SLOTW = FMT == ILL_Q6_K ? 64 : 32;  // columns of an A slot (Q6_K: the even and the odd part)
+  static constexpr int NDM = !KM ? 0 : NT < 128 ? 2 : 1;
+  static constexpr uint32_t DM_COL = 2 * DC, A_COL = NT < 128 ? 256 : KM ? 384 : 256;
+  static_assert(DM_COL + NDM * DC <= A_COL, "accumulators and the A ring overlap");
+  static constexpr int NSLOT = (512 - A_COL) / SLOTW;       // a block or two
+  static_assert(NSLOT == 4 || NSLOT == 8, "a block's slots are consecutive");
+  // Raw blocks: two warps (a block's halves, the same 32 rows) bring their rows' windows, the CPR 16-byte pieces from the
+  // boundary at or before the block, PITCH bytes apart (an odd number of 16-byte pieces: 32 rows' words lie in at most four
+  // lanes a bank), RPI rows a request, a block of theirs ahead
+  static constexpr int CPR = FMT == ILL_Q2_K ? 6 : FMT == ILL_Q4_K ? 9 : FMT == ILL_Q6_K ? 14 : 5;
+  static constexpr int PITCH = FMT == ILL_Q2_K ? 112 : FMT == ILL_Q4_K ? 144 : FMT == ILL_Q6_K ? 240 : 80;
+  static constexpr int RPI = 32 / CPR;
+  static constexpr uint32_t RAW_BYTES = 32 * PITCH;         // 32 rows'; there are DQ_WARPS of these
+  static constexpr uint32_t X_BYTES = 2 * DC * MM_BK * 2, E_BYTES = KM ? DC * 32 : 0, M_BYTES = KM ? 128 * 32 : 0;
+  static constexpr int NX = FMT == ILL_Q6_K && NT == 128 ? 3 : 4;  // stages of the ring of X tiles, two K steps each
+  static constexpr uint32_t TAIL = 768 /* barriers */ + 4 * 256 * 4 /* weight scales */ + 16 * NT /* X scales */;
+  static constexpr size_t SMEM = (size_t)NX * X_BYTES + 2 * E_BYTES + 2 * M_BYTES + (size_t)DQ_WARPS * RAW_BYTES + TAIL +
+                                 2304 /* experts' first tiles */ + (FMT == ILL_IQ2_XXS ? 8 * 4096 + 32 * 512 : 0) /* tables */ +
+                                 1024 /* alignment */;
+  static_assert(SMEM <= 227 * 1024, "shared memory of a CTA");
+};
+
+template <int FMT, bool DENSE, int NT>
+__global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(const __grid_constant__ MmMaps maps, const MmParams p) {
+  typedef MmGeom<FMT, NT> G;
+  constexpr int BB = G::BB, NSLOT = G::NSLOT, NX = G::NX, PITCH = G::PITCH, HALVES = G::HALVES, DC = G::DC;
   constexpr bool KM = G::KM;
   constexpr uint32_t TMEM_COLS = 512;
   extern __shared__ __align__(1024) u8 smem_raw[];
-  // [X ring][Q2_K: sums of 16 x 2, mins x 2] (each tile 1024-byte aligned, as the 128-byte swizzle needs), the
-  // ring of raw blocks, then barriers, scales, tables
+  // [X ring][KM: sums of 16 x 2, mins x 2] (the X tiles 1024-byte aligned, as the 128-byte swizzle needs), the
+  // dequantizing warps' raw blocks, then barriers, scales, tables
   u8* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   u8* x_tiles = smem;
-  u8* e_tiles = smem + NX * MM_TILE_BYTES;       // Q2_K: the sums of 16 of the tile's rows of X
-  u8* m_tiles = e_tiles + 2 * MM_TILE_BYTES;     // Q2_K: the mins
-  uint32_t* raw = (uint32_t*)(smem + (NX + G::NE) * MM_TILE_BYTES);
-  u8* tail = (u8*)raw + MM_RS * G::RAW_BYTES + 16;
-  // K step st of this CTA (four a block, counted over all its tiles) uses X stage st % NX, A slot st % NSLOT
-  // and the pair of barriers st % NX
-  uint64_t* kfull = (uint64_t*)tail;             // [NX] the X tile landed (TMA) and the K step of A is in tensor memory (4 warps)
-  uint64_t* kempty = kfull + NX;                 // [NX] the MMAs of the K step completed
-  uint64_t* mfull = kempty + NX;                 // [2] Q2_K: the block's sums of 16 landed and its mins are in their tile (8 warps)
-  uint64_t* mempty = mfull + 2;                  // [2] the MMA that read them completed
-  uint64_t* raw_full = mempty + 2;               // [RS] the raw-load lanes' copies landed
-  uint64_t* raw_empty = raw_full + MM_RS;        // [RS] the dequantizing warps have read the stage
-  uint64_t* acc_full = raw_empty + MM_RS;        // [2] a block's MMAs completed
-  uint64_t* acc_free = acc_full + 2;             // [2] the drain warps read the buffer
-  uint64_t* accm_free = acc_free + 2;            // [1] Q2_K: the drain warps read the mins' accumulator
-  uint32_t* tmem_slot = (uint32_t*)(accm_free + 1);
-  float* wsc = (float*)(tail + 512);             // [4 blocks in flight][2: d, dmin][128 weight rows]
-  float* xsc = wsc + 4 * 256;                    // [XSC blocks][128 rows of X] the activations' block scales
-  int* tile_first = (int*)(xsc + MM_XSC * 128);  // [ne + 1] first row tile of each expert; the total
+  u8* e_tiles = smem + NX * G::X_BYTES;          // KM: the sums of 16 of the job's rows of X
+  u8* m_tiles = e_tiles + 2 * G::E_BYTES;        // KM: the mins
+  u8* raw = m_tiles + 2 * G::M_BYTES;
+  u8* tail = raw + G::DQ_WARPS * G::RAW_BYTES;
+  uint64_t* xfull = (uint64_t*)tail;             // [NX] the X tile landed (TMA)
+  uint64_t* xempty = xfull + NX;                 // [NX] the MMAs that read it completed
+  uint64_t* afull = xempty + NX;                 // [NSLOT] the K step of A is in tensor memory (4 warps)
+  // [2][4] the MMAs that read block n's K steps completed, at n % 2: a barrier for each block that may be waited for, since
+  // a warp two blocks ahead could not tell a slot's phases apart by their parity
+  uint64_t* aempty = afull + NSLOT;
+  uint64_t* efull = aempty + 8;                  // [2] KM: the job's sums of 16 landed
+  uint64_t* eempty = efull + 2;                  // [2]
+  uint64_t* mfull = eempty + 2;                  // [2] KM: the block's mins are in their tile (8 warps)
+  uint64_t* mempty = mfull + 2;                  // [2]
+  uint64_t* acc_full = mempty + 2;               // [2] a job's MMAs completed
+  uint64_t* acc_free = acc_full + 2;             // [2] the drain warps have read the job's accumulators
+  uint64_t* raw_full = acc_free + 2;             // [DQ_WARPS] both warps' copies into a raw buffer landed
+  uint64_t* raw_empty = raw_full + G::DQ_WARPS;  // [DQ_WARPS] both warps have read it
+  uint64_t* fin = raw_empty + G::DQ_WARPS;       // [1] after a time-out: the MMAs issued so far completed
+  uint32_t* tmem_slot = (uint32_t*)(fin + 1);
+  static_assert((2 * NX + NSLOT + 8 + 13 + 2 * G::DQ_WARPS) * 8 + 4 <= 768, "barriers");
+  float* wsc = (float*)(tail + 768);             // [4 blocks in flight][2: d, dmin][128 weight rows]
+  float* xsc = wsc + 4 * 256;                    // [drain warps][HALVES * DC / DR_GROUPS] the block's scales of the warp's rows of X
+  int* tile_first = (int*)(tail + G::TAIL);      // [ne + 1] first row tile of each expert; the total
   uint4* iq_grid = (uint4*)((u8*)tile_first + 2304);  // [256 entries][8 copies] the grid as halves
-  uint4* iq_sgn = iq_grid + 8 * 256;             // [128 entries][8 copies] sign bits of the eight halves
+  uint32_t* iq_sgn = (uint32_t*)(iq_grid + 8 * 256);  // [128 entries][32 copies] the eight signs (w_iq2xxs)
 
   // the warp number through a shuffle: the compiler then knows that the role branches are warp-uniform
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 
-  // ---- once per CTA: the experts' row tiles counted (first tile of each expert, in shared memory),
-  // barriers, tables, tensor memory.  The CTA then walks tiles blockIdx.x, + gridDim.x, ...
+  // ---- once per CTA: barriers, tables, tensor memory; then, after the kernel before, the experts' row tiles counted
+  // (first tile of each expert, in shared memory).  The CTA then walks tiles blockIdx.x, + gridDim.x, ...
+  pdl_launch_dependents();
+  if (tid == 32) {
+    for (int s = 0; s < NX; ++s) { mbar_init(&xfull[s], 1); mbar_init(&xempty[s], 1); }
+    for (int s = 0; s < NSLOT; ++s) mbar_init(&afull[s], 4);
+    for (int s = 0; s < 8; ++s) mbar_init(&aempty[s], 1);
+    for (int s = 0; s < G::DQ_WARPS; ++s) { mbar_init(&raw_full[s], 64); mbar_init(&raw_empty[s], 2); }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&efull[s], 1); mbar_init(&eempty[s], 1);
+      mbar_init(&mfull[s], 8); mbar_init(&mempty[s], 1);
+      mbar_init(&acc_full[s], 1); mbar_init(&acc_free[s], G::DR_WARPS);
+    }
+    mbar_init(fin, 1);
+    mbar_fence_init();
+  }
+  if (FMT == ILL_IQ2_XXS) {
+    for (int i = tid; i < 8 * 256; i += G::THREADS) {
+      const uint64_t g = ill_iq2xxs_grid[i >> 3];
+      uint32_t h[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const __half2 hh = __floats2half2_rn((float)((g >> (16 * k)) & 0xff), (float)((g >> (16 * k + 8)) & 0xff));
+        h[k] = *(const uint32_t*)&hh;
+      }
+      iq_grid[i] = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+    for (int i = tid; i < 32 * 128; i += G::THREADS) {
+      const uint32_t s7 = (uint32_t)i >> 5, sg = s7 | ((__popc(s7) & 1u) << 7);
+      iq_sgn[i] = (sg << 9) | (sg << 24);
+    }
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
+  pdl_wait();
   if (warp == 0) {
     int before = 0;
     for (int e0 = 0; e0 < p.ne; e0 += 32) {
       const int e = e0 + lane;
       const int c = e < p.ne ? mm_count<DENSE>(p, e) : 0;
-      const int tiles = (c + MM_BM - 1) / MM_BM;
+      const int tiles = (c + p.bm - 1) / p.bm;
       int incl = tiles;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -423,34 +496,6 @@ __global__ void __launch_bounds__(MM_THREADS) mm_id_kernel(const __grid_constant
     }
     if (lane == 0) tile_first[p.ne] = before;  // row tiles in all
   }
-  if (tid == 32) {
-    for (int s = 0; s < NX; ++s) { mbar_init(&kfull[s], 1 + MM_DQ_WARPS / 4); mbar_init(&kempty[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&mfull[s], 1 + MM_DQ_WARPS / 2); mbar_init(&mempty[s], 1); }
-    for (int s = 0; s < MM_RS; ++s) { mbar_init(&raw_full[s], 32 * MM_LD_WARPS); mbar_init(&raw_empty[s], MM_DQ_WARPS); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_free[b], MM_DR_WARPS); }
-    mbar_init(accm_free, MM_DR_WARPS);
-    mbar_fence_init();
-  }
-  if (FMT == ILL_IQ2_XXS) {
-    for (int i = tid; i < 8 * 256; i += MM_THREADS) {
-      const uint64_t g = ill_iq2xxs_grid[i >> 3];
-      uint32_t h[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const __half2 hh = __floats2half2_rn((float)((g >> (16 * k)) & 0xff), (float)((g >> (16 * k + 8)) & 0xff));
-        h[k] = *(const uint32_t*)&hh;
-      }
-      iq_grid[i] = make_uint4(h[0], h[1], h[2], h[3]);
-    }
-    for (int i = tid; i < 8 * 128; i += MM_THREADS) {
-      const uint32_t s7 = (uint32_t)i >> 3, sg = s7 | ((__popc(s7) & 1u) << 7);
-      uint32_t h[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) h[k] = (((sg >> (2 * k)) & 1u) << 15) | (((sg >> (2 * k + 1)) & 1u) << 31);
-      iq_sgn[i] = make_uint4(h[0], h[1], h[2], h[3]);
-    }
-  }
-  if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -474,392 +519,464 @@ __global__ void __launch_bounds__(MM_THREADS) mm_id_kernel(const __grid_constant
     }
     expert = lo;
     const int m_in = mt - tile_first[lo];
-    row0 = mm_base<DENSE>(p, lo) + m_in * MM_BM;
-    nvalid = min(MM_BM, mm_count<DENSE>(p, lo) - m_in * MM_BM);
+    row0 = mm_base<DENSE>(p, lo) + m_in * p.bm;
+    nvalid = min(p.bm, mm_count<DENSE>(p, lo) - m_in * p.bm);
     // counts / bases come from the caller: a tile never reaches past the TOTAL_ROWS rows X and Y have
     if ((long long)row0 >= p.total_rows) { row0 = 0; nvalid = 0; }
     else nvalid = min(nvalid, (int)(p.total_rows - row0));
   };
 
-  if (warp < 2 + MM_LD_WARPS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(MM_REGS_AUX));
+  if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(G::REGS_AUX));
   if (warp == 0) {
-    // ---- TMA producer of the X tiles
-    if (lane == 0) {
-      int g_st = 0, g_kb = 0;  // K steps and blocks issued so far by this CTA
-      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        int expert, row0, nvalid, nt;
-        locate(tile, expert, row0, nvalid, nt);
-        for (int kb = 0; kb < nkb && ok; ++kb, ++g_kb) {
-          for (int j = 0; j < 4; ++j, ++g_st) {
-            const int s = g_st % NX;
-            if (g_st >= NX && !mbar_wait(&kempty[s], (uint32_t)(g_st / NX - 1) & 1u, p.status, ST_MM_WAIT_EMPTY, 0)) { ok = false; break; }
-            mbar_expect_tx(&kfull[s], MM_TILE_BYTES);
-            tma_load_2d(x_tiles + s * MM_TILE_BYTES, &xmap, kb * 256 + j * MM_BK, row0, &kfull[s]);
+    // ---- TMA producer of the X tiles: a load brings two K steps of the job's rows of X (up to 32, 64, 96 or 128).  Lanes 0
+    // and 1 watch a job's two stages, lane 2 (KM) the tile for its sums of 16: one poll looks at all of them.
+    int s = 0, g = 0;                              // stage of the ring; jobs so far
+    uint32_t ph = 1;                               // parity that a free stage's barrier has completed (a fresh barrier: 1)
+    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+      int expert, row0, nvalid, nt;
+      locate(tile, expert, row0, nvalid, nt);
+      for (int kb = 0; kb < nkb && ok; ++kb) {
+        for (int half = 0; half == 0 || (half < HALVES && 128 * half < nvalid); ++half, ++g) {
+          const int boxes = mm_boxes(min(DC, nvalid - 128 * half)), hrow = row0 + 128 * half, b = g & 1;
+          const bool wrap = s + lane >= NX;
+          uint64_t* bar = lane == 2 && KM ? &eempty[b] : &xempty[lane < 2 ? (wrap ? s + lane - NX : s + lane) : s];
+          const uint32_t par = lane == 2 && KM ? ((uint32_t)(g >> 1) & 1u) ^ 1u : ph ^ (wrap && lane < 2 ? 1u : 0u);
+          MmPoll poll(p.status, ST_MM_WAIT_EMPTY);
+#pragma unroll
+          for (int i = 0; i < (KM ? 3 : 2); ++i) {
+            if (!(ok = poll.until(bar, par, 1u << i))) break;
+            if (i < 2) {
+              if (elect_one()) {
+                mbar_expect_tx(&xfull[s], boxes * (2 * MM_XBOX * MM_BK * 2));
+                tma_load_3d(x_tiles + s * G::X_BYTES, &maps.x[boxes - 1], 0, hrow, kb * 4 + 2 * i, &xfull[s]);
+              }
+              __syncwarp();
+              if (++s == NX) { s = 0; ph ^= 1; }
+            } else {
+              if (elect_one()) {
+                mbar_expect_tx(&efull[b], boxes * (MM_XBOX * 32));
+                tma_load_2d(e_tiles + b * G::E_BYTES, &maps.e[boxes - 1], kb * MM_BK, hrow, &efull[b]);
+              }
+              __syncwarp();
+            }
           }
-          if (KM && ok) {
-            const int sm = g_kb & 1;
-            if (g_kb >= 2 && !mbar_wait(&mempty[sm], (uint32_t)((g_kb >> 1) - 1) & 1u, p.status, ST_MM_WAIT_EMPTY + 3, 0)) { ok = false; break; }
-            mbar_expect_tx(&mfull[sm], MM_TILE_BYTES);
-            tma_load_2d(e_tiles + sm * MM_TILE_BYTES, &emap, kb * MM_BK, row0, &mfull[sm]);  // the sums of 16
-          }
+          if (!ok) break;
         }
       }
     }
+    if (!ok) {
+      // a wait ran out: the copies that are in flight land before the CTA goes (a stage's last phase, if it had one)
+      for (int i = 0; i < NX; ++i) mbar_wait(&xfull[i], i < s ? ph ^ 1u : ph, nullptr, 0, 0, ILL_WAIT_NS / 20);
+      if (KM)
+        for (int j = max(0, g - 2); j < g; ++j) mbar_wait(&efull[j & 1], (uint32_t)(j >> 1) & 1u, nullptr, 0, 0, ILL_WAIT_NS / 20);
+    }
   } else if (warp == 1) {
     // ---- MMA issuer: the whole warp walks the loop (so that addresses and descriptors stay in uniform
-    // registers) and one elected lane issues
-    {
-      int g_st = 0, g_kb = 0;  // K steps and blocks consumed so far by this CTA
-      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        int expert, row0, nvalid, nt;
-        locate(tile, expert, row0, nvalid, nt);
-        nvalid = __shfl_sync(0xffffffffu, nvalid, 0);
-        // fp32 accumulate, fp16 A and B, both K-major, M = 128 weight rows, N = the tile's rows of X up to 16
-        const int nmma = max(16, (nvalid + 15) & ~15);
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(nmma >> 3) << 17) | ((uint32_t)(MM_BN >> 4) << 24);
-        for (int kb = 0; kb < nkb && ok; ++kb, ++g_kb) {
-          const int b = g_kb & 1;
-          if (g_kb >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&acc_free[b], (uint32_t)(g_kb / 2 - 1) & 1u, p.status, ST_MM_WAIT_EPI));
-          if (!ok) break;
-          const uint32_t d1 = tmem_base + (uint32_t)(b * MM_BM);
-          for (int j = 0; j < 4; ++j, ++g_st) {
-            const int s = g_st % NX, slot = g_st % NSLOT;
-            ok = __all_sync(0xffffffffu, mbar_wait(&kfull[s], (uint32_t)(g_st / NX) & 1u, p.status, ST_MM_WAIT_FULL));
-            if (!ok) break;
+    // registers) and one elected lane issues.  A barrier costs 60 to 90 cycles to look at, so each lane watches one of a
+    // job's: 0 and 1 its X stages, 4..7 its K steps of A, 8 its accumulator; KM: 9 its sums of 16, 10 the block's mins, 11 the
+    // mins' accumulator (when there is one, the job before must have been drained).
+    uint64_t* ring = lane < 2 ? xfull : lane < 4 ? acc_free : lane < 8 ? afull : lane == 9 ? efull : lane == 10 ? mfull : acc_free;
+    const int len = lane < 2 ? NX : lane < 4 ? 2 : lane < 8 ? NSLOT : 2, step = lane < 2 ? 2 : lane < 4 ? 1 : lane < 8 ? 4 : 1;
+    int idx = lane < 2 ? lane : lane < 4 ? 0 : lane < 8 ? lane - 4 : lane == 11 ? 1 : 0;
+    uint32_t par = lane == 8 || lane == 11 ? 1u : 0u;
+    const bool per_block = (lane >= 4 && lane < 8) || lane == 10;  // shared by a block's jobs
+    const uint64_t xdesc0 = umma_desc(x_tiles);
+    int s = 0, slot = 0, g = 0, g_kb = 0;          // X stage; first A slot of the block; jobs and blocks so far
+    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+      int expert, row0, nvalid, nt;
+      locate(tile, expert, row0, nvalid, nt);
+      nvalid = __shfl_sync(0xffffffffu, nvalid, 0);
+      const bool two = HALVES > 1 && nvalid > 128;
+      for (int kb = 0; kb < nkb && ok; ++kb, ++g_kb) {
+        for (int half = 0; half <= (two ? 1 : 0); ++half, ++g) {
+          const int b = g & 1, rows = min(DC, nvalid - 128 * half);
+          const bool last = half == (two ? 1 : 0);
+          // fp32 accumulate, fp16 A and B, both K-major, M = 128 weight rows, N = the job's rows of X up to 16
+          const int nmma = max(16, (rows + 15) & ~15);
+          const uint32_t idesc = (1u << 4) | ((uint32_t)(nmma >> 3) << 17) | ((uint32_t)(MM_BN >> 4) << 24);
+          const uint32_t d1 = tmem_base + (uint32_t)(b * DC);
+          const uint32_t xstep = mm_boxes(rows) * (MM_XBOX * MM_BK * 2 / 16);  // a K step's tile in a stage
+          uint64_t* aem = aempty + 4 * (g_kb & 1);
+          MmPoll poll(p.status, ST_MM_WAIT_FULL);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (!(ok = poll.until(ring + idx, par, (i ? 0u : 0x100u) | (1u << (i >> 1)) | (0x10u << i)))) break;
             tc_fence_after();
-            const uint64_t xdsc = umma_desc(x_tiles + s * MM_TILE_BYTES);
-            const uint32_t a0 = tmem_base + G::A_COL + G::SLOTW * slot;
+            const uint64_t xdsc = xdesc0 + (uint32_t)(s * (int)(G::X_BYTES >> 4)) + (i & 1 ? xstep : 0u);
+            const uint32_t a0 = tmem_base + G::A_COL + G::SLOTW * (slot + i);
             if (elect_one()) {
 #pragma unroll
               for (int k = 0; k < MM_BK / 16; ++k)  // 16 of K: 8 columns of A, 32 bytes inside X's swizzle atom
-                umma_f16_ts(d1, a0 + 8 * k, xdsc + 2 * k, idesc, (j | k) ? 1u : 0u);
+                umma_f16_ts(d1, a0 + 8 * k, xdsc + 2 * k, idesc, (i | k) ? 1u : 0u);
               if constexpr (FMT == ILL_Q6_K) {  // the weights' odd parts against the same activations
 #pragma unroll
                 for (int k = 0; k < MM_BK / 16; ++k) umma_f16_ts(d1, a0 + 32 + 8 * k, xdsc + 2 * k, idesc, 1u);
               }
-              umma_commit(&kempty[s]);  // the X stage and the A slot are free when these MMAs are done
+              if (i & 1) umma_commit(&xempty[s]);
+              if (last) umma_commit(&aem[i]);
+              if (!KM && i == 3) umma_commit(&acc_full[b]);
             }
             __syncwarp();
+            if ((i & 1) && ++s == NX) s = 0;
           }
           if (!ok) break;
           if constexpr (KM) {
-            const int sm = g_kb & 1;
-            ok = __all_sync(0xffffffffu, mbar_wait(&mfull[sm], (uint32_t)(g_kb >> 1) & 1u, p.status, ST_MM_WAIT_FULL + 3) &&
-                                             (g_kb < 1 || mbar_wait(accm_free, (uint32_t)(g_kb - 1) & 1u, p.status, ST_MM_WAIT_EPI + 2)));
-            if (!ok) break;
+            const int mb = g_kb & 1;
+            if (!(ok = poll.until(ring + idx, par, G::NDM == 1 ? 0xe00u : 0x600u))) break;
             tc_fence_after();
             // mins x sums of 16: one K = 16 product into the mins' accumulator
             if (elect_one()) {
-              umma_f16_ss(tmem_base + G::DM_COL, umma_desc(m_tiles + sm * MM_TILE_BYTES), umma_desc(e_tiles + sm * MM_TILE_BYTES), idesc, 0u);
-              umma_commit(&mempty[sm]);
+              umma_f16_ss(tmem_base + G::DM_COL + (G::NDM == 2 ? b * DC : 0), umma_desc32(m_tiles + mb * G::M_BYTES),
+                          umma_desc32(e_tiles + b * G::E_BYTES), idesc, 0u);
+              umma_commit(&eempty[b]);
+              if (last) umma_commit(&mempty[mb]);
+              umma_commit(&acc_full[b]);
             }
             __syncwarp();
           }
-          if (elect_one()) umma_commit(&acc_full[b]);
-          __syncwarp();
-        }
-      }
-    }
-  } else if (warp < 2 + MM_LD_WARPS) {
-    // ---- warps 2, 3 bring each block's raw bytes (for every weight row the 16-byte-aligned window
-    // around the row's block, 16 bytes a lane at a time: a warp's requests touch six or seven rows) and
-    // the block's scale of each of the tile's rows of X into shared memory
-    const int L = (warp - 2) * 32 + lane;
-    constexpr int NL = 32 * MM_LD_WARPS, CPR = G::WIN / 16;  // chunks of a row's window
-    int g_kb = 0;
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-      int expert, row0, nvalid, nt;
-      locate(tile, expert, row0, nvalid, nt);
-      const bool second = nt >= ntn1;
-      if (second) nt -= ntn1;
-      const u8* wbase = (const u8*)(uintptr_t)mm_ptr<DENSE>(p, expert) + (second ? p.add2 : p.add) + (long long)nt * MM_BN * p.row_bytes;
-      const int rows_here = min(MM_BN, p.nrows - nt * MM_BN);
-      // the tokens of the tile's rows L, L + NL of X (a row past the tile's last takes the first row's)
-      const float* xdp[128 / NL];
-#pragma unroll
-      for (int i = 0; i < 128 / NL; ++i) {
-        const long long place = (long long)row0 + (L + i * NL < nvalid ? L + i * NL : 0);
-        const long long tok = p.map ? (long long)p.map[place] : place;
-        xdp[i] = p.xd + tok * nkb;
-      }
-      for (int kb = 0; kb < nkb; ++kb, ++g_kb) {
-        const int s = g_kb % MM_RS, use = g_kb / MM_RS;
-        bool w_ok = true;
-        if (use > 0) w_ok = mbar_wait(&raw_empty[s], (uint32_t)(use - 1) & 1u, p.status, ST_MM_WAIT_EMPTY + 2, 200);
-        if (!__all_sync(0xffffffffu, w_ok)) { ok = false; break; }
-#pragma unroll
-        for (int i = 0; i < 128 / NL; ++i) {
-          cp_async4(xsc + (g_kb % MM_XSC) * 128 + L + i * NL, xdp[i] + kb);
-
-        }
-        u8* dst = (u8*)raw + s * G::RAW_BYTES;
-#pragma unroll 4
-        for (int c = L; c < 128 * CPR; c += NL) {
-          const int row = c / CPR, ch = c - row * CPR;
-          if (row < rows_here) {
-            const uintptr_t blk = (uintptr_t)(wbase + (long long)row * p.row_bytes + kb * BB);
-            cp_async16(dst + row * G::PITCH + 16 * ch, (const void*)((blk & ~(uintptr_t)15) + 16 * ch));
+          if (last || !per_block) {
+            idx += step;
+            if (idx >= len) { idx -= len; par ^= 1; }
           }
         }
-        cp_async_arrive(&raw_full[s]);
+        slot += 4;
+        if (slot == NSLOT) slot = 0;
       }
     }
-    cp_async_wait_all();
-  } else if (warp < 2 + MM_LD_WARPS + MM_DR_WARPS) {
-    // ---- warps 4..7 drain the accumulators block by block, scaling each block's integer sums by the
+    if (!ok) {
+      // a wait ran out: the products issued so far end before tensor memory is freed
+      if (elect_one()) umma_commit(fin);
+      __syncwarp();
+      mbar_wait(fin, 0, nullptr, 0, 0, ILL_WAIT_NS / 20);
+    }
+  } else if (warp < 4) {
+    // (two warps of the first warp group have no role)
+  } else if (warp < 4 + G::DR_WARPS) {
+    // ---- warps 4.. drain the accumulators job by job, scaling each block's integer sums by the
     // block's float scales, and store the finished tile.  A warp reads the 32 tensor-memory lanes
-    // its number gives it (warp % 4: 32 weight rows) and all the columns (rows of X).
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(MM_REGS_DRAIN));
-    const int q = warp & 3;
+    // its number gives it (warp % 4: 32 weight rows) and every DR_GROUPS-th eight columns (rows of X), so that
+    // the warps have the same share whatever the tile's rows.
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(G::REGS_DRAIN));
+    const int q = warp & 3, hh = (warp - 4) >> 2;
     const int m = q * 32 + lane;                   // accumulator lane = weight row in the tile
-    int d_kb = 0;                                  // blocks drained so far by this CTA
+    constexpr int STRIDE = 8 * G::DR_GROUPS, NP = DC / (32 * G::DR_GROUPS);  // a warp's eights of columns lie STRIDE apart; it has 32 NP columns of a job
+    constexpr bool PIPE = NT <= 128;
+    const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + 8 * hh;
+    int g = 0, d_kb = 0;                           // jobs and blocks drained so far by this CTA
+    float* xsw = xsc + (warp - 4) * (HALVES * NP * 32);
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
       int expert, row0, nvalid, nt;
       locate(tile, expert, row0, nvalid, nt);
-      uint64_t out[64];  // pairs of fp32: this weight row against the tile's 128 rows of X
+      // pairs of fp32: this weight row against the tile's rows of X 128 half + column(0 .. 32 NP - 1)
+      uint64_t out[HALVES * NP * 16];
+      auto column = [&](int i) { return STRIDE * (i >> 3) + 8 * hh + (i & 7); };
 #pragma unroll
-      for (int i = 0; i < 64; ++i) out[i] = 0ull;
-      for (int kb = 0; kb < nkb; ++kb, ++d_kb) {
-        const int b = d_kb & 1;
-        const bool e_ok = mbar_wait(&acc_full[b], (uint32_t)(d_kb / 2) & 1u, p.status, ST_MM_WAIT_ACC, 0);
-        if (!__all_sync(0xffffffffu, e_ok)) { ok = false; break; }
-        tc_fence_after();
-        // Two fp32 at a time (fma.rn.f32x2: each half rounds as the scalar instruction does).
-        // IQ2XXS-DOT-AVX2 (src/avx2.lisp:107-110): total += d * y.d * sum, the 1/8 at the end;
-        // Q2K-DOT-AVX2 (src/avx2.lisp:147-150): y.d * d * sum - y.d * dmin * mins
-        const float dw = wsc[(d_kb & 3) * 256 + m];
-        const uint64_t dw2 = pack2(dw, dw);
-        const float* xs = xsc + (d_kb % MM_XSC) * 128;
-        const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16);
-        if constexpr (KM) {
-          const float dm = -wsc[(d_kb & 3) * 256 + 128 + m];
-          const uint64_t dm2 = pack2(dm, dm);
+      for (int i = 0; i < HALVES * NP * 16; ++i) out[i] = 0ull;
+      // a lane fetches the scales of one row of X of 32 (a row past the tile's last: the first row's), a block ahead
+      int tok[HALVES * NP];
+      float dxn[HALVES * NP];
 #pragma unroll
-          for (int part = 0; part < 4; ++part) {
-            if (32 * part < nvalid) {  // columns past the tile's last row of X were not computed
-              uint32_t v[32];
-              tmem_ld32(t0 + G::DM_COL + 32 * part, v);
+      for (int i = 0; i < HALVES * NP; ++i) {
+        const int c = 128 * (i / NP) + column(32 * (i % NP) + lane);
+        const long long place = (long long)row0 + (c < nvalid ? c : 0);
+        tok[i] = !DENSE && p.map ? (int)p.map[place] : (int)place;
+        dxn[i] = p.xd[(long long)tok[i] * nkb];
+      }
+      for (int kb = 0; kb < nkb && ok; ++kb, ++d_kb) {
 #pragma unroll
-              for (int i = 0; i < 32; i += 4) {
-                const ulonglong2 dx = *(const ulonglong2*)(xs + 32 * part + i);
-                uint64_t* o = out + (32 * part + i) / 2;
-                o[0] = fma2(mul2(dx.x, dm2), pack2u(v[i], v[i + 1]), o[0]);
-                o[1] = fma2(mul2(dx.y, dm2), pack2u(v[i + 2], v[i + 3]), o[1]);
+        for (int i = 0; i < HALVES * NP; ++i) {
+          xsw[32 * i + lane] = dxn[i];
+          if (kb + 1 < nkb) dxn[i] = p.xd[(long long)tok[i] * nkb + kb + 1];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int half = 0; half < HALVES; ++half) {
+          if (half > 0 && (nvalid <= 128 * half || !ok)) break;
+          const int b = g & 1;
+          const bool e_ok = mbar_wait(&acc_full[b], (uint32_t)(g >> 1) & 1u, p.status, ST_MM_WAIT_ACC);
+          if (!__all_sync(0xffffffffu, e_ok)) { ok = false; break; }
+          tc_fence_after();
+          // Two fp32 at a time (each half of a packed instruction rounds as the scalar one does).
+          // IQ2XXS-DOT-AVX2 (src/avx2.lisp:107-110): total += d * y.d * sum, the 1/8 at the end;
+          // Q2K-DOT-AVX2 (src/avx2.lisp:147-150): y.d * d * sum - y.d * dmin * mins
+          const float dw = wsc[(d_kb & 3) * 256 + m];
+          const uint64_t dw2 = pack2(dw, dw);
+          uint64_t dm2 = 0;
+          if constexpr (KM) {
+            const float dm = -wsc[(d_kb & 3) * 256 + 128 + m];
+            dm2 = pack2(dm, dm);
+          }
+          const float* xp = xsw + half * NP * 32;
+          const int nv = nvalid - 128 * half - 8 * hh;  // columns past the tile's last row of X were not computed
+          const uint32_t td = t0 + b * DC, tm = t0 + G::DM_COL + (G::NDM == 2 ? b * DC : 0);
+          // eight columns at a time; in narrow tiles, where the registers allow it, the next eight are on their way meanwhile
+          uint32_t v[PIPE ? 2 : 1][8], w[PIPE ? 2 : 1][8];
+          if (PIPE && nv > 0) {
+            tmem_ld(td, v[0]);
+            if constexpr (KM) tmem_ld(tm, w[0]);
+          }
+#pragma unroll
+          for (int c = 0; c < NP * 32; c += 8) {
+            const int cur = PIPE ? (c >> 3) & 1 : 0, col = STRIDE * (c >> 3), nxt = col + STRIDE;
+            if (col < nv) {
+              if (!PIPE) {
+                tmem_ld(td + col, v[0]);
+                if constexpr (KM) tmem_ld(tm + col, w[0]);
+              }
+              tmem_ld_wait(v[cur]);
+              if constexpr (KM) tmem_ld_done(w[cur]);
+              if (PIPE && c + 8 < NP * 32 && nxt < nv) {
+                tmem_ld(td + nxt, v[PIPE ? cur ^ 1 : 0]);
+                if constexpr (KM) tmem_ld(tm + nxt, w[PIPE ? cur ^ 1 : 0]);
+              }
+#pragma unroll
+              for (int i = 0; i < 8; i += 4) {
+                const ulonglong2 dx = *(const ulonglong2*)(xp + c + i);
+                uint64_t* o = out + half * NP * 16 + (c + i) / 2;
+                if constexpr (KM) {
+                  o[0] = fma2(mul2(dx.x, dm2), pack2u(w[cur][i], w[cur][i + 1]), o[0]);
+                  o[1] = fma2(mul2(dx.y, dm2), pack2u(w[cur][i + 2], w[cur][i + 3]), o[1]);
+                }
+                o[0] = fma2(mul2(dw2, dx.x), pack2u(v[cur][i], v[cur][i + 1]), o[0]);
+                o[1] = fma2(mul2(dw2, dx.y), pack2u(v[cur][i + 2], v[cur][i + 3]), o[1]);
               }
             }
           }
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(accm_free);
+          if (lane == 0) mbar_arrive(&acc_free[b]);
+          ++g;
         }
-#pragma unroll
-        for (int part = 0; part < 4; ++part) {
-          if (32 * part < nvalid) {
-            uint32_t v[32];
-            tmem_ld32(t0 + b * MM_BM + 32 * part, v);
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const ulonglong2 dx = *(const ulonglong2*)(xs + 32 * part + i);
-              uint64_t* o = out + (32 * part + i) / 2;
-              o[0] = fma2(mul2(dw2, dx.x), pack2u(v[i], v[i + 1]), o[0]);
-              o[1] = fma2(mul2(dw2, dx.y), pack2u(v[i + 2], v[i + 3]), o[1]);
-            }
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_free[b]);
+        __syncwarp();                              // the scales of this block have been read
       }
       const bool second = nt >= ntn1;
       if (second) nt -= ntn1;
       const int n = nt * MM_BN + m;
       if (ok && n < p.nrows) {
-        const float fin = FMT == ILL_IQ2_XXS ? 0.125f : 1.0f;
+        const float fin_scale = FMT == ILL_IQ2_XXS ? 0.125f : 1.0f;
         float* ycol = (second ? p.y2 : p.y) + n;
         const unsigned ys = (unsigned)p.y_stride;
-        if (p.ymap) {
-          const unsigned* ym = p.ymap + row0;
+        // eight rows of X at a time: the rows of Y (or what is added to) first, then the stores: a load does not wait
+        // for the store before it
 #pragma unroll
-          for (int i0 = 0; i0 < 128; i0 += 8) {
-            if (i0 < nvalid) {
-              unsigned yr[8];  // the rows first, then the stores: a load does not wait for the store before it
+        for (int i0 = 0; i0 < HALVES * NP * 32; i0 += 8) {
+          const int c0 = 128 * (i0 / (32 * NP)) + column(i0 % (32 * NP));
+          if (c0 < nvalid) {
+            float v[8];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) yr[i] = i0 + i < nvalid ? __ldg(ym + i0 + i) : 0u;
+            for (int i = 0; i < 8; ++i) v[i] = __uint_as_float((uint32_t)(out[(i0 + i) >> 1] >> (32 * (i & 1)))) * fin_scale;
+            if (!DENSE && p.ymap) {
+              unsigned yr[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) yr[i] = c0 + i < nvalid ? __ldg(p.ymap + row0 + c0 + i) : 0u;
               if (p.ypeers) {
                 // the combine of an expert-parallel chunk, fused: the row goes straight into the memory of the
                 // rank that owns its token (a plain store over NVLink), tile by tile as the products finish
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                  if (i0 + i < nvalid) {
-                    float* dst = (float*)(uintptr_t)__ldg(p.ypeers + (yr[i] >> 24)) + (size_t)(yr[i] & 0xffffffu) * ys + n;
-                    *dst = __uint_as_float((uint32_t)(out[(i0 + i) >> 1] >> (32 * (i & 1)))) * fin;
-                  }
+                  if (c0 + i < nvalid)
+                    *((float*)(uintptr_t)__ldg(p.ypeers + (yr[i] >> 24)) + (size_t)(yr[i] & 0xffffffu) * ys + n) = v[i];
               } else {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                  if (i0 + i < nvalid)
-                    ycol[(size_t)yr[i] * ys] = __uint_as_float((uint32_t)(out[(i0 + i) >> 1] >> (32 * (i & 1)))) * fin;
+                  if (c0 + i < nvalid) ycol[(size_t)yr[i] * ys] = v[i];
+              }
+            } else {
+              float* yp = ycol + (size_t)(row0 + c0) * ys;
+              if (DENSE && p.acc) {
+                float old[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) old[i] = c0 + i < nvalid ? yp[(size_t)i * ys] : 0.0f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = old[i] + v[i];
+              }
+              if (c0 + 8 <= nvalid) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i, yp += ys) *yp = v[i];
+              } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                  if (c0 + i < nvalid) yp[(size_t)i * ys] = v[i];
               }
             }
-          }
-        } else {
-          ycol += (size_t)row0 * ys;
-#pragma unroll
-          for (int i = 0; i < 128; ++i) {
-            if (i < nvalid) {
-              const float v = __uint_as_float((uint32_t)(out[i >> 1] >> (32 * (i & 1)))) * fin;
-              if constexpr (DENSE) *ycol = p.acc ? *ycol + v : v;
-              else *ycol = v;
-            }
-            ycol += ys;
           }
         }
       }
     }
   } else {
-    // ---- warps 8..23 turn the raw blocks into the A operand in tensor memory: thread (row, j) makes K
-    // step j of its weight row in every block, so the tensor core can start on a block's first K
-    // step while the others are still being made.
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(MM_REGS_DQ));
-    const int t = tid - 32 * (2 + MM_LD_WARPS + MM_DR_WARPS);  // 0..511
-    const int row = t & 127, j = t >> 7;
-    const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's lanes: rows (warp % 4) * 32 ..
+    // ---- the other warps turn the raw blocks into the A operand in tensor memory: a thread makes two K steps (half H) of its
+    // weight row in every SETS-th block of the CTA, so the tensor core can start on a K step while the others are still being
+    // made.  The two warps with the same rows bring their raw windows (cp.async) a block of theirs ahead.  (Rows past the
+    // matrix's last: whatever lies in shared memory; they are not stored.)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(G::REGS_DQ));
+    const int wi = warp - (4 + G::DR_WARPS), wq = wi & 3, h = (wi >> 2) & 1, set = wi >> 3, row = 32 * wq + lane;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(wq * 32) << 16) + G::A_COL;  // this warp's lanes
+    u8* praw = raw + (set * 4 + wq) * 2 * G::RAW_BYTES;   // the two warps' two buffers
+    uint64_t* rfull = raw_full + (set * 4 + wq) * 2;
+    uint64_t* rempty = raw_empty + (set * 4 + wq) * 2;
     const uint4* grid = iq_grid + (lane & 7);
-    const uint4* sgn = iq_sgn + (lane & 7);
-    int g_kb = 0;                                  // blocks produced so far by this CTA
-
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    const uint32_t* sgn = iq_sgn + lane;
+    int tile = blockIdx.x, kb = set;               // the block that is fetched next: of the CTA's blocks, every SETS-th
+    const u8* wrow0 = nullptr;                     // the warp's first row of the tile's matrix
+    int rows_here = 0;
+    auto at_tile = [&]() {
+      if (tile >= ntiles) return;
       int expert, row0, nvalid, nt;
       locate(tile, expert, row0, nvalid, nt);
       const bool second = nt >= ntn1;
       if (second) nt -= ntn1;
-      const int n = nt * MM_BN + row;
-      const bool has_row = n < p.nrows;
-      // the low bits of the row's address: where its blocks start inside their first word
-      const uint32_t rowlow = (uint32_t)(mm_ptr<DENSE>(p, expert) + (unsigned long long)(second ? p.add2 : p.add) + (unsigned long long)n * p.row_bytes);
-      for (int kb = 0; kb < nkb && ok; ++kb, ++g_kb) {
-        const int rs = g_kb % MM_RS;
-        const bool r_ok = mbar_wait(&raw_full[rs], (uint32_t)(g_kb / MM_RS) & 1u, p.status, ST_MM_WAIT_FULL + 2, 50);
-        if (!__all_sync(0xffffffffu, r_ok)) { ok = false; break; }
-        // this thread's words of the block (it starts O16 bytes into the row's window), then the raw
-        // stage is free again
-        const uint32_t o16 = (rowlow + (uint32_t)kb * BB) & 15u;
-        const uint32_t* rw = raw + rs * (G::RAW_BYTES / 4) + row * (G::PITCH / 4);
-        uint32_t w[KM ? 8 : 4], sc4 = 0, m0 = 0, m1 = 0, dd = 0, s12[3] = {0, 0, 0};
+      wrow0 = (const u8*)(uintptr_t)mm_ptr<DENSE>(p, expert) + (second ? p.add2 : p.add) + (long long)(nt * MM_BN + 32 * wq) * p.row_bytes;
+      rows_here = min(32, p.nrows - nt * MM_BN - 32 * wq);
+    };
+    auto to_block = [&]() {                        // on to the tile that block kb falls in
+      while (kb >= nkb && tile < ntiles) { kb -= nkb; tile += gridDim.x; if (kb < nkb) at_tile(); }
+    };
+    auto fetch = [&](int buf) -> uint32_t {        // this warp's part of block kb's windows; where the lane's row starts in its own
+      const int r0 = lane / G::CPR, ch = lane - r0 * G::CPR;
+      if (r0 < G::RPI) {
+        const u8* src = wrow0 + (long long)(r0 + h * G::RPI) * p.row_bytes + (long long)kb * BB;
+        u8* dst = praw + buf * G::RAW_BYTES + (r0 + h * G::RPI) * PITCH + 16 * ch;
+        const long long rstep = 2ll * G::RPI * p.row_bytes;
 #pragma unroll
-        for (int i = 0; i < (KM ? 8 : 4); ++i) w[i] = 0;
-        if (has_row) {
-          if constexpr (FMT == ILL_IQ2_XXS) {
-            dd = (rw[o16 >> 2] >> (8 * (o16 & 2u))) & 0xffffu;
-            const uint32_t o = o16 + 2 + 16 * j, w0 = o >> 2, sh = (o & 3u) * 8u;
-            uint32_t prev = rw[w0];
+        for (int r = 0; r < 32; r += 2 * G::RPI, src += rstep)
+          if (r + r0 + h * G::RPI < rows_here) cp_async16(dst + r * PITCH, (const void*)(((uintptr_t)src & ~(uintptr_t)15) + 16 * ch));
+      }
+      cp_async_arrive(&rfull[buf]);
+      return ((uint32_t)(uintptr_t)wrow0 + (uint32_t)lane * (uint32_t)p.row_bytes + (uint32_t)kb * BB) & 15u;
+    };
+    at_tile();
+    to_block();
+    uint32_t o16n = 0;
+    bool more = tile < ntiles;
+    if (more) o16n = fetch(0);
+    for (int g_kb = set, it = 0; more; g_kb += G::SETS, ++it) {
+      const int buf = it & 1;
+      const uint32_t o16 = o16n;
+      // the next block into the other buffer, once both warps have read the block before from it
+      kb += G::SETS;
+      to_block();
+      more = tile < ntiles;
+      if (more) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&rempty[buf ^ 1], ((uint32_t)(it + 1) >> 1 & 1u) ^ 1u, p.status, ST_MM_WAIT_EMPTY + 2))) { ok = false; break; }
+        o16n = fetch(buf ^ 1);
+      }
+      if (!__all_sync(0xffffffffu, mbar_wait(&rfull[buf], (uint32_t)(it >> 1) & 1u, p.status, ST_MM_WAIT_FULL + 2))) { ok = false; break; }
+      const uint32_t sh = (o16 & 2u) * 8u;         // IQ2_XXS, Q6_K: the block may start in the middle of a word
+      const uint32_t* mine = (const uint32_t*)(praw + buf * G::RAW_BYTES + lane * PITCH);
+      const uint32_t* rw = mine + (o16 >> 2);
+      uint32_t dd, m4[2] = {0, 0};                 // d, dmin; Q4_K: the half's scales and mins, Q2_K: its eight scale bytes
+      if constexpr (FMT == ILL_IQ2_XXS) dd = rw[0] >> sh;
+      else if constexpr (FMT == ILL_Q6_K) dd = rw[52] >> sh;
+      else if constexpr (FMT == ILL_Q4_K) {        // (a Q4_K block is 16-byte aligned)
+        const uint4 hd = *(const uint4*)mine;
+        dd = hd.x;
+        const uint32_t s12[3] = {hd.y, hd.z, hd.w};
+        q4k_scales_mins(s12, h, m4[0], m4[1]);
+      } else {
+        dd = rw[20];
+        m4[0] = rw[2 * h]; m4[1] = rw[2 * h + 1];
+      }
+      const int slot = (4 * g_kb) % NSLOT;
+      const int prev = g_kb - NSLOT / 4;           // the block that was in the slots before
+      auto slot_free = [&](int j) {                // its MMAs of the K step must be done
+        if (prev >= 0)
+          ok = __all_sync(0xffffffffu, mbar_wait(&aempty[4 * (prev & 1) + j], (uint32_t)(prev >> 1) & 1u, p.status, ST_MM_WAIT_EMPTY + 1));
+        tc_fence_after();
+        if (j == 0) {
+          // The drain of four blocks back is over: the MMAs that freed this slot were issued after it.
+          wsc[(g_kb & 3) * 256 + row] = h2f(dd & 0xffff);
+          if (KM) wsc[(g_kb & 3) * 256 + 128 + row] = h2f(dd >> 16);
+        }
+        return ok;
+      };
+      const uint32_t a0 = lane_base + G::SLOTW * (slot + 2 * h);
+      if constexpr (FMT == ILL_Q6_K) {
+        // The half's two K steps together: step jj has the nibbles at shift 4 jj of ql[0 .. 63]; columns 32 sb .. of it go with
+        // the 2-bit fields at shift 2 (2 jj + sb) of qh.  Sixteen weights (a group) at a time.
+        uint32_t sc[2];
+        raw_words<2>(rw + 48 + 2 * h, sh, sc);
+        if (!slot_free(2 * h) || !slot_free(2 * h + 1)) break;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const uint32_t next = rw[w0 + i + 1];
-              w[i] = __funnelshift_r(prev, next, sh);
-              prev = next;
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t qh[4];
+          raw_words<4>(rw + 32 + 8 * h + 4 * hf, sh, qh);
+#pragma unroll
+          for (int sb = 0; sb < 2; ++sb) {
+            uint32_t ql[4];
+            raw_words<4>(rw + 16 * h + 8 * sb + 4 * hf, sh, ql);
+#pragma unroll
+            for (int jj = 0; jj < 2; ++jj) {
+              uint32_t ev[8], od[8];
+              w_q6k(ql, qh, jj, 2 * (2 * jj + sb), (int)(signed char)((sc[jj] >> (16 * sb + 8 * hf)) & 0xffu), ev, od);
+              tmem_st8(a0 + G::SLOTW * jj + 16 * sb + 8 * hf, ev);
+              tmem_st8(a0 + G::SLOTW * jj + 32 + 16 * sb + 8 * hf, od);
             }
-          } else if constexpr (FMT == ILL_Q6_K) {
-            // the block's scale and K step j's four group scales; the quants are read as they are unpacked (below)
-            dd = (rw[(o16 + 208) >> 2] >> (8 * ((o16 + 208) & 2u))) & 0xffffu;
-            raw_words<1>(rw, o16 + 192 + 4 * j, &sc4);
-          } else if constexpr (FMT == ILL_Q4_K) {
-            // K step j: the block's chunk j of 32 quant bytes (groups 2j and 2j + 1); the twelve bytes of scales and mins
-            const uint32_t* bw = rw + (o16 >> 2);  // a Q4_K block is 16-byte aligned
-            dd = bw[0];
-            s12[0] = bw[1]; s12[1] = bw[2]; s12[2] = bw[3];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] = bw[4 + 8 * j + i];
-          } else {
-            // K step j: half j / 2 of the block's quants at shifts 2 (j % 2) and 2 (j % 2) + 1; its four scale bytes
-            const uint32_t* bw = rw + (o16 >> 2);  // a Q2_K block is 4-byte aligned
-            sc4 = bw[j];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] = bw[4 + 8 * (j >> 1) + i];
-            if (j < 2) { m0 = bw[2 * j]; m1 = bw[2 * j + 1]; }
-            dd = bw[20];
           }
         }
+        tmem_st_wait();
+        tc_fence_before();
         __syncwarp();
-        if (FMT != ILL_Q6_K && lane == 0) mbar_arrive(&raw_empty[rs]);  // (Q6_K reads its quants from the stage while unpacking)
-        {
-          // the slot's last K step was st - NSLOT: its MMAs must be done
-          const int st = 4 * g_kb + j, slot = st % NSLOT, sp = st - NSLOT;
-          bool w_ok = true;
-          if (sp >= 0) w_ok = mbar_wait(&kempty[sp % NX], (uint32_t)(sp / NX) & 1u, p.status, ST_MM_WAIT_EMPTY + 1, 50);
-          if (!__all_sync(0xffffffffu, w_ok)) { ok = false; break; }
-          tc_fence_after();
-          if (j == 0) {
-            // The drain of four blocks back is over: the MMAs that freed this slot were issued after it.
-            wsc[(g_kb & 3) * 256 + row] = h2f(dd & 0xffff);
-            if (KM) wsc[(g_kb & 3) * 256 + 128 + row] = h2f(dd >> 16);
-          }
-          const uint32_t a0 = lane_base + G::A_COL + G::SLOTW * slot;
+        if (lane == 0) { mbar_arrive(&afull[slot + 2 * h]); mbar_arrive(&afull[slot + 2 * h + 1]); mbar_arrive(&rempty[buf]); }
+      } else {
+        uint32_t w[8];
 #pragma unroll
-          for (int sb = 0; sb < 2; ++sb) {  // 32 weights = 16 columns at a time
+        for (int jj = 0; jj < 2; ++jj) {           // K step j = 2 h + jj
+          const int j = 2 * h + jj;
+#pragma unroll
+          for (int sb = 0; sb < 2; ++sb) {         // 32 weights = 16 columns at a time
             uint32_t v[16];
-            if constexpr (FMT == ILL_IQ2_XXS) {
+            if constexpr (FMT == ILL_IQ2_XXS) {    // sub-block 2 j + sb
+              if (sb == 0) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w[i] = __funnelshift_rc(rw[4 * j + i], rw[4 * j + i + 1], 16 + sh);
+              }
               w_iq2xxs(w[2 * sb], w[2 * sb + 1], grid, sgn, v);
-              if (!has_row) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = 0;
+            } else if constexpr (FMT == ILL_Q4_K) {  // group 2 j + sb: the low or the high nibbles of chunk j
+              if (sb == 0) {
+                const uint4 a = *(const uint4*)(mine + 4 + 8 * j), c = *(const uint4*)(mine + 8 + 8 * j);
+                w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = c.x; w[5] = c.y; w[6] = c.z; w[7] = c.w;
               }
-            } else if constexpr (FMT == ILL_Q6_K) {
-              // K step j: half j / 2 of the block; columns 32 sb .. of the step are the nibbles at shift 4 (j % 2) of
-              // ql[32 sb ..] with the 2-bit fields at shift 2 (2 (j % 2) + sb) of qh; sixteen weights (a group) at a time
+              if (sb == 0) w_fields<8, 0>(w, 0x0f0f0f0fu, m4[0], 2 * jj, v);
+              else w_fields<8, 4>(w, 0xf0f0f0f0u, m4[0], 2 * jj + 1, v);
+            } else {                               // shift 2 (2 jj + sb) of the half's quants; scale bytes 4 j + 2 sb, + 1
+              if (jj == 0 && sb == 0) {
 #pragma unroll
-              for (int hf = 0; hf < 2; ++hf) {
-                uint32_t ev[8], od[8];
-                if (has_row) {
-                  uint32_t ql[4], qh[4];
-                  raw_words<4>(rw, o16 + 64 * (j >> 1) + 32 * sb + 16 * hf, ql);
-                  raw_words<4>(rw, o16 + 128 + 32 * (j >> 1) + 16 * hf, qh);
-                  w_q6k(ql, qh, j & 1, 2 * (2 * (j & 1) + sb), (int)(signed char)((sc4 >> (16 * sb + 8 * hf)) & 0xffu), ev, od);
-                } else {
-#pragma unroll
-                  for (int i = 0; i < 8; ++i) ev[i] = od[i] = 0;
-                }
-                tmem_st8(a0 + 16 * sb + 8 * hf, ev);
-                tmem_st8(a0 + 32 + 16 * sb + 8 * hf, od);
+                for (int i = 0; i < 8; ++i) w[i] = rw[4 + 8 * h + i];
               }
-            } else if constexpr (FMT == ILL_Q4_K) {
-              uint32_t sc, mn;
-              q4k_scale_min(s12, 2 * j + sb, sc, mn);
-#pragma unroll
-              for (int hf = 0; hf < 2; ++hf) {  // sixteen weights at a time: fewer live registers than all 32
-                uint32_t v8[8];
-                w_q4k<4>(w + 4 * hf, sb, sc, v8);
-                tmem_st8(a0 + 16 * sb + 8 * hf, v8);
-              }
-            } else {
-              w_q2k(w, 2 * (j & 1) + sb, sc4 >> (16 * sb), sc4 >> (16 * sb + 8), v);
+              const uint32_t sc = m4[jj] & 0x0f0f0f0fu;
+              if (jj == 0 && sb == 0) { w_fields<4, 0>(w, 0x03030303u, sc, 0, v); w_fields<4, 0>(w + 4, 0x03030303u, sc, 1, v + 8); }
+              else if (jj == 0) { w_fields<4, 2>(w, 0x0c0c0c0cu, sc, 2, v); w_fields<4, 2>(w + 4, 0x0c0c0c0cu, sc, 3, v + 8); }
+              else if (sb == 0) { w_fields<4, 4>(w, 0x30303030u, sc, 0, v); w_fields<4, 4>(w + 4, 0x30303030u, sc, 1, v + 8); }
+              else { w_fields<4, 6>(w, 0xc0c0c0c0u, sc, 2, v); w_fields<4, 6>(w + 4, 0xc0c0c0c0u, sc, 3, v + 8); }
             }
-            if constexpr (FMT != ILL_Q6_K && FMT != ILL_Q4_K) tmem_st16(a0 + 16 * sb, v);
+            if (sb == 0 && !slot_free(j)) break;   // (the first 32 weights are made before the slot is waited for)
+            tmem_st16(a0 + G::SLOTW * jj + 16 * sb, v);
           }
+          if (!ok) break;
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&kfull[st % NX]);
-          if (FMT == ILL_Q6_K && lane == 0) mbar_arrive(&raw_empty[rs]);
-        }
-        if constexpr (KM) {
-          if (j < 2) {  // warp-uniform: the eight warps of K steps 0 and 1 also make the mins
-            const int sm = g_kb & 1;
-            bool w_ok = true;
-            if (g_kb >= 2) w_ok = mbar_wait(&mempty[sm], (uint32_t)((g_kb >> 1) - 1) & 1u, p.status, ST_MM_WAIT_EMPTY + 3, 50);
-            if (!__all_sync(0xffffffffu, w_ok)) { ok = false; break; }
-            uint32_t v[4];
-            // half j's eight mins: K = 8j .. 8j + 7 of the 16, chunk j of the row (Q4_K: groups 4j .. 4j + 3, each twice)
-            if constexpr (FMT == ILL_Q4_K) w_q4k_mins(s12, 4 * j, v);
-            else w_q2k_mins(m0, m1, v);
-            store_chunk(m_tiles + sm * MM_TILE_BYTES, row, j, make_uint4(v[0], v[1], v[2], v[3]));
-            fence_async_smem();  // the tensor core reads the tile through the async proxy
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&mfull[sm]);
+          if (lane == 0) {
+            mbar_arrive(&afull[slot + j]);
+            if (jj == 1) mbar_arrive(&rempty[buf]);  // both K steps' words have been read
           }
         }
       }
+      if (!ok) break;
+      if constexpr (KM) {
+        const int mb = g_kb & 1;
+        if (!__all_sync(0xffffffffu, mbar_wait(&mempty[mb], ((uint32_t)(g_kb >> 1) & 1u) ^ 1u, p.status, ST_MM_WAIT_EMPTY + 3))) { ok = false; break; }
+        uint32_t v[4];
+        // half h's eight mins: K = 8 h .. 8 h + 7 of the 16, chunk h of the row (Q4_K: groups 4 h .. 4 h + 3, each twice)
+        if constexpr (FMT == ILL_Q4_K) w_q4k_mins(m4[1], v);
+        else w_q2k_mins(m4[0], m4[1], v);
+        store_chunk32(m_tiles + mb * G::M_BYTES, row, h, make_uint4(v[0], v[1], v[2], v[3]));
+        fence_async_smem();  // the tensor core reads the tile through the async proxy
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&mfull[mb]);
+      }
     }
+    cp_async_wait_all();
   }
   tc_fence_before();
   __syncthreads();
@@ -1338,18 +1455,24 @@ extern "C" int ill_ep_unpack(int64_t rows, int cols, ill_dptr packed, ill_dptr m
                         base + cols + cols / 256 * 4 + cols / 16 * 2, xd, w, stream, rows_dev);
 }
 
-static int encode_map(CUtensorMap* map, ill_dptr base, int64_t inner, int64_t rows) {
+// Rows of 64 K halves (X: a load brings two K steps of BOX_ROWS rows) or, SUMS, the first 16 of each 64 (a block's sums of 16)
+static int encode_map(CUtensorMap* map, ill_dptr base, int64_t cols, int64_t rows, bool sums, cuuint32_t box_rows) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return cuda_fail(cudaErrorNotSupported);
-  const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)inner * 2};
-  const cuuint32_t box[2] = {MM_BK, MM_BM};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)(uintptr_t)base, dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const cuuint64_t dims[3] = {sums ? (cuuint64_t)cols : MM_BK, (cuuint64_t)rows, (cuuint64_t)cols / MM_BK};
+  const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, MM_BK * 2};
+  const cuuint32_t box[3] = {sums ? 16u : MM_BK, box_rows, 2};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, sums ? 2 : 3, (void*)(uintptr_t)base, dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, sums ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? ILL_OK : cuda_fail(cudaErrorInvalidValue);
 }
+
+#ifdef ILL_TUNING
+static int g_nt = 0, g_bm = 0;
+extern "C" __attribute__((visibility("default"))) void ill_tune_mm(int nt, int bm) { g_nt = nt; g_bm = bm; }
+#endif
 
 static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
                         int64_t total_rows, ill_dptr xh, ill_dptr xe, ill_dptr xd, ill_dptr map, ill_dptr ymap, ill_dptr ypeers,
@@ -1398,6 +1521,43 @@ extern "C" int ill_mm_chunk2(int fmt, ill_dptr w, ill_dptr w2, int rows, int col
   return mm_id_launch(fmt, cols, rows, 0, 0, 0, 0, 1, n, xh, xe, xd, 0, 0, 0, y, rows, stream, add2, y2, w, 0);
 }
 
+struct MmVariant {
+  const void* k;
+  size_t smem;
+  int threads, regs_sum;
+};
+template <int FMT, bool DENSE, int NT>
+static MmVariant mm_one() {
+  typedef MmGeom<FMT, NT> G;
+  return MmVariant{(const void*)mm_id_kernel<FMT, DENSE, NT>, G::SMEM, G::THREADS, G::REGS_SUM};
+}
+template <int FMT>
+static MmVariant mm_variant(bool dense, int nt) {
+  if constexpr (FMT == ILL_Q6_K)
+    if (dense && nt == 256) return mm_one<FMT, true, 256>();
+  if constexpr (FMT == ILL_Q4_K || FMT == ILL_Q6_K)
+    if (dense) return nt == 64 ? mm_one<FMT, true, 64>() : mm_one<FMT, true, 128>();
+  return nt == 64 ? mm_one<FMT, false, 64>() : mm_one<FMT, false, 128>();
+}
+
+// Rows of X a tile.  Experts: what their mean number of rows asks for; with up to 24 the tiles of 64, whose A ring holds two
+// blocks (512 rows on 288 experts of 5120 x 1536, Q2_K, one chunk's three products 0.74 ms against 1.05 with tiles of 128),
+// else those of 128 (24576 rows on 256 experts: 2.09 ms against 3.14 with tiles of 64).
+// A dense matrix: the rounds of tiles on the SMs times a tile's measured time a block of 256 columns, us; tiles of up to 64, of
+// up to 128, and (Q6_K, which has one accumulator a block: with two, draining 256 columns takes longer than it saves) 256 rows.
+static int mm_pick_tile(int fmt, long long rows, int ne, bool dense, long long ntn, int sms) {
+  if (!dense) return rows / ne <= 24 ? 64 : 128;
+  const bool q6 = fmt == ILL_Q6_K;
+  double best = 1e30;
+  int bm = 16;
+  for (int b = 16; b <= (q6 ? 256 : 128); b += 16) {
+    const long long tiles = (rows + b - 1) / b * ntn, rounds = (tiles + sms - 1) / sms;
+    const double us = b <= 64 ? (q6 ? 1.5 + 0.0048 * b : 0.82 + 0.0045 * b) : b <= 128 ? (q6 ? 1.5 + 0.0042 * b : 1.05 + 0.0043 * b) : 2.6 + 0.0033 * b;
+    if (rounds * us < best) { best = rounds * us; bm = b; }
+  }
+  return bm;
+}
+
 static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
                         int64_t total_rows, ill_dptr xh, ill_dptr xe, ill_dptr xd, ill_dptr map, ill_dptr ymap, ill_dptr ypeers,
                         ill_dptr y, int64_t y_stride, ill_stream stream, int64_t add2, ill_dptr y2, ill_dptr one_ptr, int acc) {
@@ -1414,11 +1574,13 @@ static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptr
     return ILL_ERR_ALIGN;
   if (fmt == ILL_Q4_K && ((add | add2) & 15)) return ILL_ERR_ALIGN;  // (and every PTRS[e]: the kernel copies 16-byte pieces of the rows as they lie)
   if (total_rows == 0) return ILL_OK;
-  CUtensorMap xmap, emap;
-  int rc = encode_map(&xmap, xh, ncols, total_rows);
-  if (rc) return rc;
-  rc = km ? encode_map(&emap, xe, (int64_t)(ncols / 256) * 64, total_rows) : encode_map(&emap, xh, ncols, total_rows);
-  if (rc) return rc;
+  MmMaps maps;
+  for (int i = 0; i < 4; ++i) {
+    int rc = encode_map(&maps.x[i], xh, ncols, total_rows, false, MM_XBOX * (i + 1));
+    if (rc == ILL_OK && km) rc = encode_map(&maps.e[i], xe, (int64_t)(ncols / 256) * 64, total_rows, true, MM_XBOX * (i + 1));
+    if (rc) return rc;
+  }
+  if (!km) memcpy(maps.e, maps.x, sizeof maps.e);
   MmParams p;
   p.ncols = ncols;
   p.nrows = nrows;
@@ -1441,31 +1603,31 @@ static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptr
   p.one_count = (unsigned)total_rows;
   p.acc = acc;
   p.status = device_status_word();
-  const long long max_tiles = ((total_rows + MM_BM - 1) / MM_BM + ne) * ((nrows + MM_BN - 1) / MM_BN) * (y2 ? 2 : 1);  // an upper bound
-  const size_t smem = fmt == ILL_IQ2_XXS ? MmGeom<ILL_IQ2_XXS>::SMEM : fmt == ILL_Q2_K ? MmGeom<ILL_Q2_K>::SMEM
-                      : fmt == ILL_Q4_K ? MmGeom<ILL_Q4_K>::SMEM : MmGeom<ILL_Q6_K>::SMEM;
   if (ne > 512) return ILL_ERR_TOO_LARGE;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-  const void* k = fmt == ILL_IQ2_XXS ? (const void*)mm_id_kernel<ILL_IQ2_XXS, false>
-                  : fmt == ILL_Q2_K ? (const void*)mm_id_kernel<ILL_Q2_K, false>
-                  : fmt == ILL_Q4_K ? (one_ptr ? (const void*)mm_id_kernel<ILL_Q4_K, true> : (const void*)mm_id_kernel<ILL_Q4_K, false>)
-                                    : (one_ptr ? (const void*)mm_id_kernel<ILL_Q6_K, true> : (const void*)mm_id_kernel<ILL_Q6_K, false>);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const long long ntn = (nrows + MM_BN - 1) / MM_BN * (y2 ? 2 : 1);
+  p.bm = mm_pick_tile(fmt, total_rows, ne, one_ptr != 0, ntn, sms);
+#ifdef ILL_TUNING
+  if (g_bm) p.bm = g_bm;
+#endif
+  int nt = p.bm <= 64 ? 64 : p.bm <= 128 ? 128 : 256;
+#ifdef ILL_TUNING
+  if (g_nt) nt = g_nt;
+#endif
+  const long long max_tiles = ((total_rows + p.bm - 1) / p.bm + ne) * ntn;  // an upper bound
+  const MmVariant v = fmt == ILL_IQ2_XXS ? mm_variant<ILL_IQ2_XXS>(false, nt) : fmt == ILL_Q2_K ? mm_variant<ILL_Q2_K>(false, nt)
+                      : fmt == ILL_Q4_K ? mm_variant<ILL_Q4_K>(one_ptr != 0, nt) : mm_variant<ILL_Q6_K>(one_ptr != 0, nt);
+  cudaError_t e = cudaFuncSetAttribute(v.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem);
   if (e != cudaSuccess) return cuda_fail(e);
   // The warp groups trade registers after launch; what they ask for together must fit in what the
   // CTA was given, or the drain warps would wait for registers for ever.
   cudaFuncAttributes fa;
-  e = cudaFuncGetAttributes(&fa, k);
+  e = cudaFuncGetAttributes(&fa, v.k);
   if (e != cudaSuccess) return cuda_fail(e);
-  if (fa.numRegs * MM_THREADS < 128 * (MM_REGS_AUX + MM_REGS_DRAIN) + 32 * MM_DQ_WARPS * MM_REGS_DQ) return ILL_ERR_UNSUPPORTED;
-  void* args[] = {&xmap, &emap, &p};
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(max_tiles < sms ? max_tiles : sms), 1, 1);  // persistent: a CTA an SM, each walks tiles
-  cfg.blockDim = dim3(MM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = (cudaStream_t)stream;
-  e = cudaLaunchKernelExC(&cfg, k, args);
-  return e == cudaSuccess ? ILL_OK : cuda_fail(e);
+  if (fa.numRegs / 8 * 8 * v.threads < v.regs_sum) return ILL_ERR_UNSUPPORTED;
+  void* args[] = {&maps, &p};
+  // persistent: a CTA an SM, each walks tiles
+  return launch_kernel(v.k, dim3((unsigned)(max_tiles < sms ? max_tiles : sms)), dim3((unsigned)v.threads), v.smem, args, (cudaStream_t)stream);
 }

@@ -176,3 +176,45 @@ def test_a_table_that_the_kernel_before_has_written(fmt):
         products(turning, y[i])
     for i in range(20):
         assert torch.equal(y[i], want[i % 2])
+
+
+@pytest.mark.parametrize("fmt,base", [(B.IQ2_XXS, 2), (B.Q2_K, 4), (B.Q4_K, 16), (B.Q6_K, 6)])
+@pytest.mark.parametrize("rows,cols", [(200, 768), (128, 256), (260, 2048)])
+@pytest.mark.parametrize("counts", [(0, 1, 64, 65, 3, 0, 15), (33, 127, 128, 129, 1), (300, 0, 256, 257, 17)])
+def test_expert_chunk_tiles(fmt, base, rows, cols, counts):
+    """The chunk product at the edges of its tiles (of up to 64, 128 and 256 rows of X, by the experts' mean), rows that are no
+    multiple of a tile, blocks at the alignments a format may have, fewer and more blocks than are in flight: against the
+    one-token product of every row."""
+    ne, n = len(counts), sum(counts)
+    nbytes = B.matrix_bytes(fmt, rows, cols)
+    step = (nbytes + 64) // 16 * 16
+    buf = torch.zeros(ne * step + 32, dtype=torch.uint8, device="cuda")
+    for e in range(ne):
+        buf[base + e * step:base + e * step + nbytes] = B.synth_matrix_torch(fmt, rows, cols, seed=e + rows)
+    g = torch.Generator(device="cuda").manual_seed(n + cols)
+    act = D.quant_q8(torch.randn(n * cols, device="cuda", generator=g), D.make_qact(n * cols, "q8k"))
+    cf = D.ChunkF16(n, cols).fill(act)
+    ptrs = torch.tensor([buf.data_ptr() + base + e * step for e in range(ne)], dtype=torch.int64, device="cuda")
+    cnt = torch.tensor(counts, dtype=torch.int32, device="cuda")
+    bases = torch.tensor([sum(counts[:e]) for e in range(ne)], dtype=torch.int32, device="cuda")
+    stride = (rows + 3) // 4 * 4 + 4
+    y = torch.full((n + 1, stride), 5.0, device="cuda")
+    _lib.call("ill_moe_mm_id", fmt, cols, rows, 0, ptrs.data_ptr(), cnt.data_ptr(), bases.data_ptr(), ne, n, cf.xh.data_ptr(),
+              cf.xe.data_ptr(), cf.xd.data_ptr(), 0, 0, y.data_ptr(), stride, _lib.stream())
+    want = torch.empty(n, rows, device="cuda")
+    if fmt in (B.IQ2_XXS, B.Q2_K):
+        table = torch.empty(n, dtype=torch.int64, device="cuda")
+        _lib.call("ill_moe_row_ptrs", ne, ptrs.data_ptr(), cnt.data_ptr(), bases.data_ptr(), n, table.data_ptr(), _lib.stream())
+        _lib.call("ill_moe_mv", fmt, cols, rows, 0, table.data_ptr(), n, act.xq.data_ptr(), act.xs.data_ptr(), act.xsum.data_ptr(), 1,
+                  want.data_ptr(), rows, _lib.stream())
+    else:
+        for e, c in enumerate(counts):
+            at = sum(counts[:e])
+            for t in range(at, at + c):
+                _lib.call("ill_mv", fmt, buf.data_ptr() + base + e * step, rows, cols, act.xq.data_ptr() + t * cols,
+                          act.xs.data_ptr() + 4 * t * (cols // 256), act.xsum.data_ptr() + 2 * t * (cols // 16), want[t].data_ptr(), 0, 0, 1,
+                          _lib.stream())
+    # the same whole-number block sums; cols / 256 float terms in another order, a difference of two of them among the formats
+    # with mins: a few units of 2^-24 of the largest
+    assert (y[:n, :rows] - want).abs().max().item() < 2e-6 * want.abs().max().item()
+    assert (y[n] == 5.0).all() and (y[:, rows:] == 5.0).all()

@@ -269,3 +269,22 @@ def test_quantizers_that_also_leave_the_fp16_forms():
             assert torch.equal(act._cf.xh, fresh.xh) and torch.equal(act._cf.xe, fresh.xe)
             outs.append(y.clone())
         assert torch.isfinite(outs[1]).all()
+
+
+@pytest.mark.parametrize("fmt", [B.Q4_K, B.Q6_K])
+@pytest.mark.parametrize("rows,cols,n", [(128, 256, 1), (132, 768, 97), (1024, 2560, 513), (384, 2816, 31), (2560, 1024, 130), (19456, 256, 512)])
+def test_chunk_on_tcgen05_tiles(fmt, rows, cols, n):
+    """The tcgen05 chunk product at the edges of its tiles (16 to 256 tokens, by the number of tiles a matrix makes), with fewer
+    blocks than are in flight and matrices of one tile: against the one-token product, and adding to Y."""
+    w, x, act = _case(fmt, rows, cols, n, seed=n)
+    cf = D.ChunkF16(n, cols).fill(act)
+    y = torch.full((n * rows + 64,), -3.0, device="cuda")
+    D.cmat_mul_tc(w, cf, y)
+    want = torch.empty(n, rows, device="cuda")
+    for t in range(n):
+        D.cmat_mul(w, D.quant_q8(x[t * cols:(t + 1) * cols], D.make_qact(cols, "q8k")), want[t], 1)
+    top = want.abs().max().item()
+    assert (y[:n * rows].view(n, rows) - want).abs().max().item() < 2e-6 * top and (y[n * rows:] == -3.0).all()
+    y[:n * rows] = 1.0
+    D.cmat_mul_tc(w, cf, y, acc=True)
+    assert (y[:n * rows].view(n, rows) - 1.0 - want).abs().max().item() < 2e-6 * max(top, 1.0) + 2.0 ** -23 * (1.0 + top)
