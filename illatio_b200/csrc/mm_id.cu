@@ -388,9 +388,12 @@ template <int FMT, int NT> struct MmGeom {
   static_assert(DM_COL + NDM * DC <= A_COL, "accumulators and the A ring overlap");
   static constexpr int NSLOT = (512 - A_COL) / SLOTW;       // a block or two
   static_assert(NSLOT == 4 || NSLOT == 8, "a block's slots are consecutive");
-  // Raw blocks: two warps (a block's halves, the same 32 rows) bring their rows' windows, the CPR 16-byte pieces from the
+  // Raw blocks: the two warps that unpack them (a block's halves, the same 32 rows) bring their rows' windows -- or, LOADERS,
+  // in IQ2_XXS, whose unpacking bounds the kernel (gate and up of 24576 rows on 256 experts 1360 -> 1301 us; Q6_K was 7 %
+  // slower), the two warps that have no other role, for all -- the CPR 16-byte pieces from the
   // boundary at or before the block, PITCH bytes apart (an odd number of 16-byte pieces: 32 rows' words lie in at most four
   // lanes a bank), RPI rows a request, a block of theirs ahead
+  static constexpr bool LOADERS = FMT == ILL_IQ2_XXS;
   static constexpr int CPR = FMT == ILL_Q2_K ? 6 : FMT == ILL_Q4_K ? 9 : FMT == ILL_Q6_K ? 14 : 5;
   static constexpr int PITCH = FMT == ILL_Q2_K ? 112 : FMT == ILL_Q4_K ? 144 : FMT == ILL_Q6_K ? 240 : 80;
   static constexpr int RPI = 32 / CPR;
@@ -403,6 +406,23 @@ template <int FMT, int NT> struct MmGeom {
                                  1024 /* alignment */;
   static_assert(SMEM <= 227 * 1024, "shared memory of a CTA");
 };
+
+// One of two warps' (H) requests for the windows of a block of ROWS <= 32 rows (the first row's block at SRC) into the buffer DST;
+// FULL gets this warp's 32 arrivals once they have landed.
+template <int FMT, int NT>
+__device__ __forceinline__ void mm_fetch(const u8* src, int row_bytes, int rows, int h, int lane, u8* dst, uint64_t* full) {
+  typedef MmGeom<FMT, NT> G;
+  const int r0 = lane / G::CPR + h * G::RPI, ch = lane % G::CPR;
+  if (lane < G::CPR * G::RPI) {
+    src += (long long)r0 * row_bytes;
+    dst += r0 * G::PITCH + 16 * ch;
+    const long long step = 2ll * G::RPI * row_bytes;
+#pragma unroll
+    for (int r = 0; r < 32; r += 2 * G::RPI, src += step)
+      if (r + r0 < rows) cp_async16(dst + r * G::PITCH, (const void*)(((uintptr_t)src & ~(uintptr_t)15) + 16 * ch));
+  }
+  cp_async_arrive(full);
+}
 
 template <int FMT, bool DENSE, int NT>
 __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(const __grid_constant__ MmMaps maps, const MmParams p) {
@@ -650,7 +670,31 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
       mbar_wait(fin, 0, nullptr, 0, 0, ILL_WAIT_NS / 20);
     }
   } else if (warp < 4) {
-    // (two warps of the first warp group have no role)
+    // ---- warps 2, 3 (LOADERS) bring the raw windows of every block, half of each 32 rows' requests a warp
+    if constexpr (G::LOADERS) {
+      int g_kb = 0;
+      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        int expert, row0, nvalid, nt;
+        locate(tile, expert, row0, nvalid, nt);
+        const bool second = nt >= ntn1;
+        if (second) nt -= ntn1;
+        const u8* w0 = (const u8*)(uintptr_t)mm_ptr<DENSE>(p, expert) + (second ? p.add2 : p.add) + (long long)nt * MM_BN * p.row_bytes;
+        const int rows_here = p.nrows - nt * MM_BN;
+        for (int kb = 0; kb < nkb && ok; ++kb, ++g_kb) {
+          const int set = g_kb % G::SETS, it = g_kb / G::SETS, buf = it & 1;
+          // lane WQ < 4 watches the four warp pairs' buffers: the block two back must have been read from them
+          uint64_t* bar = raw_empty + (set * 4 + (lane & 3)) * 2 + buf;
+          MmPoll poll(p.status, ST_MM_WAIT_EMPTY + 2);
+#pragma unroll 1
+          for (int wq = 0; wq < 4; ++wq) {
+            if (!(ok = poll.until(bar, ((uint32_t)(it >> 1) & 1u) ^ 1u, 1u << wq))) break;
+            mm_fetch<FMT, NT>(w0 + (long long)(32 * wq) * p.row_bytes + (long long)kb * BB, p.row_bytes, min(32, rows_here - 32 * wq), warp & 1,
+                              lane, raw + ((set * 4 + wq) * 2 + buf) * G::RAW_BYTES, raw_full + (set * 4 + wq) * 2 + buf);
+          }
+        }
+      }
+      cp_async_wait_all();
+    }
   } else if (warp < 4 + G::DR_WARPS) {
     // ---- warps 4.. drain the accumulators job by job, scaling each block's integer sums by the
     // block's float scales, and store the finished tile.  A warp reads the 32 tensor-memory lanes
@@ -831,18 +875,10 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
     auto to_block = [&]() {                        // on to the tile that block kb falls in
       while (kb >= nkb && tile < ntiles) { kb -= nkb; tile += gridDim.x; if (kb < nkb) at_tile(); }
     };
+    auto start = [&]() { return ((uint32_t)(uintptr_t)wrow0 + (uint32_t)lane * (uint32_t)p.row_bytes + (uint32_t)kb * BB) & 15u; };
     auto fetch = [&](int buf) -> uint32_t {        // this warp's part of block kb's windows; where the lane's row starts in its own
-      const int r0 = lane / G::CPR, ch = lane - r0 * G::CPR;
-      if (r0 < G::RPI) {
-        const u8* src = wrow0 + (long long)(r0 + h * G::RPI) * p.row_bytes + (long long)kb * BB;
-        u8* dst = praw + buf * G::RAW_BYTES + (r0 + h * G::RPI) * PITCH + 16 * ch;
-        const long long rstep = 2ll * G::RPI * p.row_bytes;
-#pragma unroll
-        for (int r = 0; r < 32; r += 2 * G::RPI, src += rstep)
-          if (r + r0 + h * G::RPI < rows_here) cp_async16(dst + r * PITCH, (const void*)(((uintptr_t)src & ~(uintptr_t)15) + 16 * ch));
-      }
-      cp_async_arrive(&rfull[buf]);
-      return ((uint32_t)(uintptr_t)wrow0 + (uint32_t)lane * (uint32_t)p.row_bytes + (uint32_t)kb * BB) & 15u;
+      if (!G::LOADERS) mm_fetch<FMT, NT>(wrow0 + (long long)kb * BB, p.row_bytes, rows_here, h, lane, praw + buf * G::RAW_BYTES, &rfull[buf]);
+      return start();
     };
     at_tile();
     to_block();
@@ -857,7 +893,7 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
       to_block();
       more = tile < ntiles;
       if (more) {
-        if (!__all_sync(0xffffffffu, mbar_wait(&rempty[buf ^ 1], ((uint32_t)(it + 1) >> 1 & 1u) ^ 1u, p.status, ST_MM_WAIT_EMPTY + 2))) { ok = false; break; }
+        if (!G::LOADERS && !__all_sync(0xffffffffu, mbar_wait(&rempty[buf ^ 1], ((uint32_t)(it + 1) >> 1 & 1u) ^ 1u, p.status, ST_MM_WAIT_EMPTY + 2))) { ok = false; break; }
         o16n = fetch(buf ^ 1);
       }
       if (!__all_sync(0xffffffffu, mbar_wait(&rfull[buf], (uint32_t)(it >> 1) & 1u, p.status, ST_MM_WAIT_FULL + 2))) { ok = false; break; }
