@@ -23,6 +23,11 @@
 //               the 32 lanes of a warp write 128 contiguous bytes of a row of Y)
 //   the others  bring W_e's raw blocks into shared memory (cp.async) and turn them into the A operand
 // The roles' register needs differ widely, so the warp groups trade registers (setmaxnreg).
+// What bounds it: the drain beside the unpacking, by instructions and latency, not the tensor pipe or memory.  Left out for
+// timing: the drain's arithmetic 14-23 % of a launch, its stores 10 %, IQ2_XXS's unpacking 21 %, the X loads, the raw copies
+// and the products' width nothing.  us, with four drain warps, two raw-load warps and 128-row tiles throughout / now: gate and up
+// of 512 tokens x 2 x 9728 x 2560 (Q4_K) 151 / 81, 2560 x 9728 (Q6_K) 123 / 73, 512 rows on 288 experts of 5120 x 1536 (Q2_K, two
+// launches) 1249 / 740, 24576 rows on 256 experts, down 2048 x 4096 (Q2_K) 811 / 735, gate and up (IQ2_XXS) 1281 / 1301.
 // Every mbarrier wait is bounded; on a time-out the kernel records a code in the status
 // word, skips what depends on the wait, lets copies and products in flight end, frees its tensor memory and returns.
 //
@@ -1578,7 +1583,7 @@ static MmVariant mm_variant(bool dense, int nt) {
 
 // Rows of X a tile.  Experts: what their mean number of rows asks for; with up to 24 the tiles of 64, whose A ring holds two
 // blocks (512 rows on 288 experts of 5120 x 1536, Q2_K, one chunk's three products 0.74 ms against 1.05 with tiles of 128),
-// else those of 128 (24576 rows on 256 experts: 2.09 ms against 3.14 with tiles of 64).
+// else those of 128 (24576 rows on 256 experts, IQ2_XXS and Q2_K: 2.04 ms against 3.14 with tiles of 64).
 // A dense matrix: the rounds of tiles on the SMs times a tile's measured time a block of 256 columns, us; tiles of up to 64, of
 // up to 128, and (Q6_K, which has one accumulator a block: with two, draining 256 columns takes longer than it saves) 256 rows.
 static int mm_pick_tile(int fmt, long long rows, int ne, bool dense, long long ntn, int sms) {
