@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 import torch
 
+from illatio_b200 import _lib
 from illatio_b200 import blocks as B
 from illatio_b200 import cuda_dense as D
 from gpu_util import to_dev
@@ -288,3 +289,35 @@ def test_chunk_on_tcgen05_tiles(fmt, rows, cols, n):
     y[:n * rows] = 1.0
     D.cmat_mul_tc(w, cf, y, acc=True)
     assert (y[:n * rows].view(n, rows) - 1.0 - want).abs().max().item() < 2e-6 * max(top, 1.0) + 2.0 ** -23 * (1.0 + top)
+
+
+@pytest.mark.parametrize("fmt", [B.Q4_K, B.Q6_K])
+@pytest.mark.parametrize("rows", [256, 1024, 2044])
+def test_chunk_of_a_small_matrix(fmt, rows):
+    """Chunks of 64 tokens through matrices of fewer than 2048 rows (a layer's K and V): block sums past 2^24 are whole numbers
+    as in the one-token product, Y may lie at any float, and the quants count as they are when the product is enqueued."""
+    cols, n = 256, 64
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    wb = torch.randint(0, 256, (rows, B.BLOCK_BYTES[fmt]), dtype=torch.uint8, device="cuda", generator=g)
+    if fmt == B.Q6_K:   # quants 56 .. 63, scales 112 .. 127: sums up to 6.2 * 2^24
+        wb[:, :128] |= 0x88
+        wb[:, 128:192] = 0xff
+        wb[:, 192:208] = wb[:, 192:208] & 0x0f | 0x70
+    else:               # quants 12 .. 15, scales 48 .. 63, no mins: up to 1.6 * 2^24
+        wb[:, 4:8] |= 0xf0
+        wb[:, 8:12] = 0
+        wb[:, 12:16] &= 0x0f
+        wb[:, 16:] |= 0xcc
+    for off in B.SCALE_OFFSETS[fmt]:
+        wb[:, off:off + 2] = (torch.rand(rows, device="cuda", generator=g) + 0.5).to(torch.float16).view(torch.uint8).view(rows, 2)
+    w = D.CMat("w", fmt, rows, cols, wb.reshape(-1))
+    x = 1.0 + 0.03 * torch.randn(2, n * cols, device="cuda", generator=g).clamp(-2.0, 2.0)
+    act, one = D.make_qact(n * cols, "q8k"), D.make_qact(cols, "q8k")
+    y, want = torch.empty(n * rows + 1, device="cuda")[1:], torch.empty(n * rows, device="cuda")
+    for i in range(2):  # the second time the quants are written by the library's own entry point
+        _lib.call("ill_quant_q8_k", x[i].data_ptr(), act.xq.data_ptr(), act.xs.data_ptr(), act.xsum.data_ptr(), n, _lib.stream())
+        D.cmat_mul(w, act, y, n)
+        for t in range(n):
+            D.cmat_mul(w, D.quant_q8(x[i, t * cols:(t + 1) * cols], one), want[t * rows:(t + 1) * rows], 1)
+        # one block a row: the same whole number, rounded to the same float, times two scales -- two roundings of 2^-24 on either side
+        assert ((y - want).abs() <= 4.00001 * 2.0 ** -24 * want.abs()).all()
