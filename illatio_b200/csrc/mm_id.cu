@@ -1510,11 +1510,6 @@ static int encode_map(CUtensorMap* map, ill_dptr base, int64_t cols, int64_t row
   return r == CUDA_SUCCESS ? ILL_OK : cuda_fail(cudaErrorInvalidValue);
 }
 
-#ifdef ILL_TUNING
-static int g_nt = 0, g_bm = 0;
-extern "C" __attribute__((visibility("default"))) void ill_tune_mm(int nt, int bm) { g_nt = nt; g_bm = bm; }
-#endif
-
 static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
                         int64_t total_rows, ill_dptr xh, ill_dptr xe, ill_dptr xd, ill_dptr map, ill_dptr ymap, ill_dptr ypeers,
                         ill_dptr y, int64_t y_stride, ill_stream stream, int64_t add2 = 0, ill_dptr y2 = 0, ill_dptr one_ptr = 0,
@@ -1650,13 +1645,7 @@ static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptr
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   const long long ntn = (nrows + MM_BN - 1) / MM_BN * (y2 ? 2 : 1);
   p.bm = mm_pick_tile(fmt, total_rows, ne, one_ptr != 0, ntn, sms);
-#ifdef ILL_TUNING
-  if (g_bm) p.bm = g_bm;
-#endif
-  int nt = p.bm <= 64 ? 64 : p.bm <= 128 ? 128 : 256;
-#ifdef ILL_TUNING
-  if (g_nt) nt = g_nt;
-#endif
+  const int nt = p.bm <= 64 ? 64 : p.bm <= 128 ? 128 : 256;
   const long long max_tiles = ((total_rows + p.bm - 1) / p.bm + ne) * ntn;  // an upper bound
   const MmVariant v = fmt == ILL_IQ2_XXS ? mm_variant<ILL_IQ2_XXS>(false, nt) : fmt == ILL_Q2_K ? mm_variant<ILL_Q2_K>(false, nt)
                       : fmt == ILL_Q4_K ? mm_variant<ILL_Q4_K>(one_ptr != 0, nt) : mm_variant<ILL_Q6_K>(one_ptr != 0, nt);
