@@ -70,6 +70,7 @@ struct MmParams {
   unsigned one_count;
   int acc;
   int bm;                      // rows of X a tile, at most the kernel's NT
+  int min_rows, max_rows;      // experts with fewer or more rows are another launch's
 };
 // (DENSE is a template argument of the kernel, so that the experts' launches compile to what they were without it)
 template <bool DENSE> __device__ __forceinline__ unsigned long long mm_ptr(const MmParams& p, int e) {
@@ -509,7 +510,7 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
     for (int e0 = 0; e0 < p.ne; e0 += 32) {
       const int e = e0 + lane;
       const int c = e < p.ne ? mm_count<DENSE>(p, e) : 0;
-      const int tiles = (c + p.bm - 1) / p.bm;
+      const int tiles = c < p.min_rows || c > p.max_rows ? 0 : (c + p.bm - 1) / p.bm;
       int incl = tiles;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -1573,16 +1574,26 @@ static MmVariant mm_variant(bool dense, int nt) {
     if (dense && nt == 256) return mm_one<FMT, true, 256>();
   if constexpr (FMT == ILL_Q4_K || FMT == ILL_Q6_K)
     if (dense) return nt == 64 ? mm_one<FMT, true, 64>() : mm_one<FMT, true, 128>();
-  return nt == 64 ? mm_one<FMT, false, 64>() : mm_one<FMT, false, 128>();
+  if constexpr (FMT == ILL_Q2_K || FMT == ILL_Q4_K)
+    if (nt == 64) return mm_one<FMT, false, 64>();
+  return mm_one<FMT, false, 128>();
 }
 
-// Rows of X a tile.  Experts: what their mean number of rows asks for; with up to 24 the tiles of 64, whose A ring holds two
-// blocks (512 rows on 288 experts of 5120 x 1536, Q2_K, one chunk's three products 0.74 ms against 1.05 with tiles of 128),
-// else those of 128 (24576 rows on 256 experts, IQ2_XXS and Q2_K: 2.04 ms against 3.14 with tiles of 64).
-// A dense matrix: the rounds of tiles on the SMs times a tile's measured time a block of 256 columns, us; tiles of up to 64, of
-// up to 128, and (Q6_K, which has one accumulator a block: with two, draining 256 columns takes longer than it saves) 256 rows.
-static int mm_pick_tile(int fmt, long long rows, int ne, bool dense, long long ntn, int sms) {
-  if (!dense) return rows / ne <= 24 ? 64 : 128;
+// Whether experts of few rows get tiles of 64 (whose A ring holds two blocks) in a launch of their own.  Only the formats with mins
+// gain from them; IQ2_XXS and Q6_K, bound by their unpacking, take 0 to 2 % less time with 64 rows an expert or fewer and up to 1.9
+// times as long with more, each tile unpacking the weights again.  The host does not know an expert's rows, so the experts are
+// dealt out on the device: up to MM_FEW rows to tiles of 64, the others to tiles of 128.  The launch that finds none costs 4 to 6 us.
+// us, tiles of 128 / of 64 / dealt out: gate and up of 288 experts of 1536 x 5120 (Q2_K) for 64 tokens 999 / 705 / 709, 6912 rows
+// (24 an expert) skewed by 1 / rank^1.1 1334 / 1084 / 1042, 512 tokens that all choose the same eight 193 / 255 / 200.
+// Above a mean of 24 rows all take tiles of 128 in one launch: 96 rows each 1408 against 2079 (but with 32 each 1218 / 890, with 64
+// each 1323 / 1100: the line could lie higher).  TOTAL_ROWS may be a capacity of which fewer rows are in use; the mean is then the larger.
+constexpr int MM_FEW = 64;
+static bool mm_few_rows(int fmt, long long rows, int ne) { return (fmt == ILL_Q2_K || fmt == ILL_Q4_K) && rows / ne <= 24; }
+
+// Rows of X a tile of a dense matrix: the rounds of tiles on the SMs times a tile's measured time a block of 256 columns, us; tiles
+// of up to 64, of up to 128, and (Q6_K, which has one accumulator a block: with two, draining 256 columns takes longer than it
+// saves) 256 rows.
+static int mm_pick_tile(int fmt, long long rows, long long ntn, int sms) {
   const bool q6 = fmt == ILL_Q6_K;
   double best = 1e30;
   int bm = 16;
@@ -1644,20 +1655,29 @@ static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptr
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   const long long ntn = (nrows + MM_BN - 1) / MM_BN * (y2 ? 2 : 1);
-  p.bm = mm_pick_tile(fmt, total_rows, ne, one_ptr != 0, ntn, sms);
-  const int nt = p.bm <= 64 ? 64 : p.bm <= 128 ? 128 : 256;
-  const long long max_tiles = ((total_rows + p.bm - 1) / p.bm + ne) * ntn;  // an upper bound
-  const MmVariant v = fmt == ILL_IQ2_XXS ? mm_variant<ILL_IQ2_XXS>(false, nt) : fmt == ILL_Q2_K ? mm_variant<ILL_Q2_K>(false, nt)
-                      : fmt == ILL_Q4_K ? mm_variant<ILL_Q4_K>(one_ptr != 0, nt) : mm_variant<ILL_Q6_K>(one_ptr != 0, nt);
-  cudaError_t e = cudaFuncSetAttribute(v.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem);
-  if (e != cudaSuccess) return cuda_fail(e);
-  // The warp groups trade registers after launch; what they ask for together must fit in what the
-  // CTA was given, or the drain warps would wait for registers for ever.
-  cudaFuncAttributes fa;
-  e = cudaFuncGetAttributes(&fa, v.k);
-  if (e != cudaSuccess) return cuda_fail(e);
-  if (fa.numRegs / 8 * 8 * v.threads < v.regs_sum) return ILL_ERR_UNSUPPORTED;
-  void* args[] = {&maps, &p};
-  // persistent: a CTA an SM, each walks tiles
-  return launch_kernel(v.k, dim3((unsigned)(max_tiles < sms ? max_tiles : sms)), dim3((unsigned)v.threads), v.smem, args, (cudaStream_t)stream);
+  const auto launch = [&](int bm, int min_rows, int max_rows) -> int {
+    p.bm = bm;
+    p.min_rows = min_rows;
+    p.max_rows = max_rows;
+    const int nt = bm <= 64 ? 64 : bm <= 128 ? 128 : 256;
+    const long long max_tiles = ((total_rows + bm - 1) / bm + ne) * ntn;  // an upper bound
+    const MmVariant v = fmt == ILL_IQ2_XXS ? mm_variant<ILL_IQ2_XXS>(false, nt) : fmt == ILL_Q2_K ? mm_variant<ILL_Q2_K>(false, nt)
+                        : fmt == ILL_Q4_K ? mm_variant<ILL_Q4_K>(one_ptr != 0, nt) : mm_variant<ILL_Q6_K>(one_ptr != 0, nt);
+    cudaError_t e = cudaFuncSetAttribute(v.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem);
+    if (e != cudaSuccess) return cuda_fail(e);
+    // The warp groups trade registers after launch; what they ask for together must fit in what the
+    // CTA was given, or the drain warps would wait for registers for ever.
+    cudaFuncAttributes fa;
+    e = cudaFuncGetAttributes(&fa, v.k);
+    if (e != cudaSuccess) return cuda_fail(e);
+    if (fa.numRegs / 8 * 8 * v.threads < v.regs_sum) return ILL_ERR_UNSUPPORTED;
+    void* args[] = {&maps, &p};
+    // persistent: a CTA an SM, each walks tiles
+    return launch_kernel(v.k, dim3((unsigned)(max_tiles < sms ? max_tiles : sms)), dim3((unsigned)v.threads), v.smem, args, (cudaStream_t)stream);
+  };
+  const int all = 0x7fffffff;
+  if (one_ptr) return launch(mm_pick_tile(fmt, total_rows, ntn, sms), 0, all);
+  if (!mm_few_rows(fmt, total_rows, ne)) return launch(128, 0, all);
+  const int rc = launch(64, 0, MM_FEW);
+  return rc || total_rows <= MM_FEW ? rc : launch(128, MM_FEW + 1, all);
 }
