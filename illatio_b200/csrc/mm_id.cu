@@ -338,12 +338,14 @@ struct MmPoll {
   unsigned int* status;
   unsigned code, ready = 0;
   __device__ __forceinline__ MmPoll(unsigned int* st, unsigned c) : status(st), code(c) {}
-  // until the phases of parity PAR of the BARs of the lanes in NEED have completed; the same answer in every lane
+  // until the phases of parity PAR of the BARs of the lanes in NEED have completed; the same answer in every lane.  A lane sees
+  // (acquires) its own barrier only and a ballot orders no memory: the __syncwarp hands what the lanes saw to those that act on it.
   __device__ __forceinline__ bool until(uint64_t* bar, uint32_t par, uint32_t need) {
-    if ((ready & need) == need) return true;
+    if ((ready & need) == need) return true;  // (the ballot that showed it was followed by a __syncwarp)
     unsigned long long t0 = 0;
     for (unsigned it = 1;; ++it) {
       ready = __ballot_sync(0xffffffffu, mbar_test(bar, par));
+      __syncwarp();
       const uint32_t missing = need & ~ready;
       if (!missing) return true;
       // the warp sleeps on the first that is missing (and takes no issue slots meanwhile)
