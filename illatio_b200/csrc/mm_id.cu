@@ -9,7 +9,8 @@
 // or Q2_K blocks at ptrs[e] + add -- or of Q4_K / Q6_K blocks: the dense prefill products run through the same
 // kernel with the matrix as its one expert (ill_mm_chunk; mm_q4k_mma / mm_q6k_mma, src/cuda/kquant.cu:316-466).
 //
-// A persistent grid (a CTA per SM) walks tiles of 128 weight rows x up to NT (64, 128 or 256) rows of X.  The
+// A persistent grid (a CTA per SM) walks tiles of 128 weight rows x up to NT (64, 128 or 256) rows of X, picked on the host by the
+// sizes of a dense matrix and on the device by the rows of the experts.  The
 // weights are the tensor core's A operand and live in tensor memory: the dequantizing warps write
 // their integer parts (exact in fp16) there with tcgen05.st, so they never pass through shared
 // memory; X is the B operand, brought by TMA (128-byte swizzle).  The accumulator
@@ -69,8 +70,7 @@ struct MmParams {
   unsigned long long one_ptr;
   unsigned one_count;
   int acc;
-  int bm;                      // rows of X a tile, at most the kernel's NT
-  int min_rows, max_rows;      // experts with fewer or more rows are another launch's
+  int bm;                      // rows of X a tile of a dense matrix, at most the kernel's NT
 };
 // (DENSE is a template argument of the kernel, so that the experts' launches compile to what they were without it)
 template <bool DENSE> __device__ __forceinline__ unsigned long long mm_ptr(const MmParams& p, int e) {
@@ -408,10 +408,17 @@ template <int FMT, int NT> struct MmGeom {
   static constexpr uint32_t RAW_BYTES = 32 * PITCH;         // 32 rows'; there are DQ_WARPS of these
   static constexpr uint32_t X_BYTES = 2 * DC * MM_BK * 2, E_BYTES = KM ? DC * 32 : 0, M_BYTES = KM ? 128 * 32 : 0;
   static constexpr int NX = FMT == ILL_Q6_K && NT == 128 ? 3 : 4;  // stages of the ring of X tiles, two K steps each
-  static constexpr uint32_t TAIL = 768 /* barriers */ + 4 * 256 * 4 /* weight scales */ + 16 * NT /* X scales */;
-  static constexpr size_t SMEM = (size_t)NX * X_BYTES + 2 * E_BYTES + 2 * M_BYTES + (size_t)DQ_WARPS * RAW_BYTES + TAIL +
-                                 2304 /* experts' first tiles */ + (FMT == ILL_IQ2_XXS ? 8 * 4096 + 32 * 512 : 0) /* tables */ +
-                                 1024 /* alignment */;
+  static constexpr uint32_t BODY = NX * X_BYTES + 2 * E_BYTES + 2 * M_BYTES + DQ_WARPS * RAW_BYTES + 4 * 256 * 4 /* weight scales */ +
+                                   16 * NT /* X scales */;
+};
+// Shared memory of a kernel for tiles of up to NT rows of X or, when NT2 is not 0, of up to NT or of up to NT2
+constexpr uint32_t MM_BARS = 768;  // the barriers of one of them
+constexpr int MM_MAX_NE = 512;     // experts a launch
+template <int FMT, int NT, int NT2> struct MmSmem {
+  static constexpr uint32_t BODY2 = MmGeom<FMT, NT2 ? NT2 : NT>::BODY, BODY = MmGeom<FMT, NT>::BODY > BODY2 ? MmGeom<FMT, NT>::BODY : BODY2;
+  static constexpr uint32_t FIRST = BODY + (NT2 ? 2 : 1) * MM_BARS, SLOTS = FIRST + 4 * (MM_MAX_NE + 1) /* experts' first tiles */,
+                            TABLES = (SLOTS + 8 + 255) / 256 * 256;
+  static constexpr size_t SMEM = TABLES + (FMT == ILL_IQ2_XXS ? 8 * 4096 + 32 * 512 : 0) + 1024 /* alignment */;
   static_assert(SMEM <= 227 * 1024, "shared memory of a CTA");
 };
 
@@ -432,53 +439,27 @@ __device__ __forceinline__ void mm_fetch(const u8* src, int row_bytes, int rows,
   cp_async_arrive(full);
 }
 
-template <int FMT, bool DENSE, int NT>
-__global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(const __grid_constant__ MmMaps maps, const MmParams p) {
+// The mbarriers of a kernel for tiles of up to NT rows of X
+template <int FMT, int NT> struct MmBars {
   typedef MmGeom<FMT, NT> G;
-  constexpr int BB = G::BB, NSLOT = G::NSLOT, NX = G::NX, PITCH = G::PITCH, HALVES = G::HALVES, DC = G::DC;
-  constexpr bool KM = G::KM;
-  constexpr uint32_t TMEM_COLS = 512;
-  extern __shared__ __align__(1024) u8 smem_raw[];
-  // [X ring][KM: sums of 16 x 2, mins x 2] (the X tiles 1024-byte aligned, as the 128-byte swizzle needs), the
-  // dequantizing warps' raw blocks, then barriers, scales, tables
-  u8* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  u8* x_tiles = smem;
-  u8* e_tiles = smem + NX * G::X_BYTES;          // KM: the sums of 16 of the job's rows of X
-  u8* m_tiles = e_tiles + 2 * G::E_BYTES;        // KM: the mins
-  u8* raw = m_tiles + 2 * G::M_BYTES;
-  u8* tail = raw + G::DQ_WARPS * G::RAW_BYTES;
-  uint64_t* xfull = (uint64_t*)tail;             // [NX] the X tile landed (TMA)
-  uint64_t* xempty = xfull + NX;                 // [NX] the MMAs that read it completed
-  uint64_t* afull = xempty + NX;                 // [NSLOT] the K step of A is in tensor memory (4 warps)
+  uint64_t xfull[G::NX];      // the X tile landed (TMA)
+  uint64_t xempty[G::NX];     // the MMAs that read it completed
+  uint64_t afull[G::NSLOT];   // the K step of A is in tensor memory (4 warps)
   // [2][4] the MMAs that read block n's K steps completed, at n % 2: a barrier for each block that may be waited for, since
   // a warp two blocks ahead could not tell a slot's phases apart by their parity
-  uint64_t* aempty = afull + NSLOT;
-  uint64_t* efull = aempty + 8;                  // [2] KM: the job's sums of 16 landed
-  uint64_t* eempty = efull + 2;                  // [2]
-  uint64_t* mfull = eempty + 2;                  // [2] KM: the block's mins are in their tile (8 warps)
-  uint64_t* mempty = mfull + 2;                  // [2]
-  uint64_t* acc_full = mempty + 2;               // [2] a job's MMAs completed
-  uint64_t* acc_free = acc_full + 2;             // [2] the drain warps have read the job's accumulators
-  uint64_t* raw_full = acc_free + 2;             // [DQ_WARPS] both warps' copies into a raw buffer landed
-  uint64_t* raw_empty = raw_full + G::DQ_WARPS;  // [DQ_WARPS] both warps have read it
-  uint64_t* fin = raw_empty + G::DQ_WARPS;       // [1] after a time-out: the MMAs issued so far completed
-  uint32_t* tmem_slot = (uint32_t*)(fin + 1);
-  static_assert((2 * NX + NSLOT + 8 + 13 + 2 * G::DQ_WARPS) * 8 + 4 <= 768, "barriers");
-  float* wsc = (float*)(tail + 768);             // [4 blocks in flight][2: d, dmin][128 weight rows]
-  float* xsc = wsc + 4 * 256;                    // [drain warps][HALVES * DC / DR_GROUPS] the block's scales of the warp's rows of X
-  int* tile_first = (int*)(tail + G::TAIL);      // [ne + 1] first row tile of each expert; the total
-  uint4* iq_grid = (uint4*)((u8*)tile_first + 2304);  // [256 entries][8 copies] the grid as halves
-  uint32_t* iq_sgn = (uint32_t*)(iq_grid + 8 * 256);  // [128 entries][32 copies] the eight signs (w_iq2xxs)
-
-  // the warp number through a shuffle: the compiler then knows that the role branches are warp-uniform
-  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-
-  // ---- once per CTA: barriers, tables, tensor memory; then, after the kernel before, the experts' row tiles counted
-  // (first tile of each expert, in shared memory).  The CTA then walks tiles blockIdx.x, + gridDim.x, ...
-  pdl_launch_dependents();
-  if (tid == 32) {
-    for (int s = 0; s < NX; ++s) { mbar_init(&xfull[s], 1); mbar_init(&xempty[s], 1); }
-    for (int s = 0; s < NSLOT; ++s) mbar_init(&afull[s], 4);
+  uint64_t aempty[8];
+  uint64_t efull[2];          // KM: the job's sums of 16 landed
+  uint64_t eempty[2];
+  uint64_t mfull[2];          // KM: the block's mins are in their tile (8 warps)
+  uint64_t mempty[2];
+  uint64_t acc_full[2];       // a job's MMAs completed
+  uint64_t acc_free[2];       // the drain warps have read the job's accumulators
+  uint64_t raw_full[G::DQ_WARPS];   // both warps' copies into a raw buffer landed
+  uint64_t raw_empty[G::DQ_WARPS];  // both warps have read it
+  uint64_t fin;               // after a time-out: the MMAs issued so far completed
+  __device__ __forceinline__ void init() {
+    for (int s = 0; s < G::NX; ++s) { mbar_init(&xfull[s], 1); mbar_init(&xempty[s], 1); }
+    for (int s = 0; s < G::NSLOT; ++s) mbar_init(&afull[s], 4);
     for (int s = 0; s < 8; ++s) mbar_init(&aempty[s], 1);
     for (int s = 0; s < G::DQ_WARPS; ++s) { mbar_init(&raw_full[s], 64); mbar_init(&raw_empty[s], 2); }
     for (int s = 0; s < 2; ++s) {
@@ -486,48 +467,29 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
       mbar_init(&mfull[s], 8); mbar_init(&mempty[s], 1);
       mbar_init(&acc_full[s], 1); mbar_init(&acc_free[s], G::DR_WARPS);
     }
-    mbar_init(fin, 1);
-    mbar_fence_init();
+    mbar_init(&fin, 1);
   }
-  if (FMT == ILL_IQ2_XXS) {
-    for (int i = tid; i < 8 * 256; i += G::THREADS) {
-      const uint64_t g = ill_iq2xxs_grid[i >> 3];
-      uint32_t h[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const __half2 hh = __floats2half2_rn((float)((g >> (16 * k)) & 0xff), (float)((g >> (16 * k + 8)) & 0xff));
-        h[k] = *(const uint32_t*)&hh;
-      }
-      iq_grid[i] = make_uint4(h[0], h[1], h[2], h[3]);
-    }
-    for (int i = tid; i < 32 * 128; i += G::THREADS) {
-      const uint32_t s7 = (uint32_t)i >> 5, sg = s7 | ((__popc(s7) & 1u) << 7);
-      iq_sgn[i] = (sg << 9) | (sg << 24);
-    }
-  }
-  if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
-  pdl_wait();
-  if (warp == 0) {
-    int before = 0;
-    for (int e0 = 0; e0 < p.ne; e0 += 32) {
-      const int e = e0 + lane;
-      const int c = e < p.ne ? mm_count<DENSE>(p, e) : 0;
-      const int tiles = c < p.min_rows || c > p.max_rows ? 0 : (c + p.bm - 1) / p.bm;
-      int incl = tiles;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      if (e < p.ne) tile_first[e] = before + incl - tiles;
-      before += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) tile_first[p.ne] = before;  // row tiles in all
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+};
+
+// What a CTA does once its barriers, tables and tensor memory are there and the experts' tiles of up to BM rows of X are counted
+// (TILE_FIRST): tiles blockIdx.x, + gridDim.x, ...
+template <int FMT, bool DENSE, int NT>
+__device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, int bm, u8* smem, MmBars<FMT, NT>* bars, const int* tile_first,
+                                         const uint4* iq_grid, const uint32_t* iq_sgn, uint32_t tmem_base, int warp, int lane) {
+  typedef MmGeom<FMT, NT> G;
+  constexpr int BB = G::BB, NSLOT = G::NSLOT, NX = G::NX, PITCH = G::PITCH, HALVES = G::HALVES, DC = G::DC;
+  constexpr bool KM = G::KM;
+  // [X ring][KM: sums of 16 x 2, mins x 2] (the X tiles 1024-byte aligned, as the 128-byte swizzle needs), the
+  // dequantizing warps' raw blocks, scales
+  u8* x_tiles = smem;
+  u8* e_tiles = smem + NX * G::X_BYTES;          // KM: the sums of 16 of the job's rows of X
+  u8* m_tiles = e_tiles + 2 * G::E_BYTES;        // KM: the mins
+  u8* raw = m_tiles + 2 * G::M_BYTES;
+  float* wsc = (float*)(raw + G::DQ_WARPS * G::RAW_BYTES);  // [4 blocks in flight][2: d, dmin][128 weight rows]
+  float* xsc = wsc + 4 * 256;                    // [drain warps][HALVES * DC / DR_GROUPS] the block's scales of the warp's rows of X
+  uint64_t *xfull = bars->xfull, *xempty = bars->xempty, *afull = bars->afull, *aempty = bars->aempty, *efull = bars->efull,
+           *eempty = bars->eempty, *mfull = bars->mfull, *mempty = bars->mempty, *acc_full = bars->acc_full, *acc_free = bars->acc_free,
+           *raw_full = bars->raw_full, *raw_empty = bars->raw_empty, *fin = &bars->fin;
 
   const int nkb = p.ncols / 256;
   const int ntn1 = (p.nrows + MM_BN - 1) / MM_BN;
@@ -547,8 +509,8 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
     }
     expert = lo;
     const int m_in = mt - tile_first[lo];
-    row0 = mm_base<DENSE>(p, lo) + m_in * p.bm;
-    nvalid = min(p.bm, mm_count<DENSE>(p, lo) - m_in * p.bm);
+    row0 = mm_base<DENSE>(p, lo) + m_in * bm;
+    nvalid = min(bm, mm_count<DENSE>(p, lo) - m_in * bm);
     // counts / bases come from the caller: a tile never reaches past the TOTAL_ROWS rows X and Y have
     if ((long long)row0 >= p.total_rows) { row0 = 0; nvalid = 0; }
     else nvalid = min(nvalid, (int)(p.total_rows - row0));
@@ -1021,6 +983,108 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
       }
     }
     cp_async_wait_all();
+  }
+}
+
+// What an expert of C rows costs in tiles of up to 64 and of up to 128 rows of X (Q2_K, Q4_K), in hundredths of a tile of 64 with
+// 16 rows.  Measured on Q2_K, a tile an expert: of 64 with 16, 32, 48, 64 rows 100, 106, 114, 131; of 128 with 16, 64, 96, 128 rows
+// 142, 158, 168, 190.
+__device__ __forceinline__ int mm_cost64(int c) { return c / 64 * 131 + (c % 64 ? 92 + 6 * (c % 64) / 10 : 0); }
+__device__ __forceinline__ int mm_cost128(int c) { return c / 128 * 190 + (c % 128 ? 134 + 4 * (c % 128) / 10 : 0); }
+
+// NT2: tiles of up to NT2 rows of X in place of NT where the experts' rows ask for them.  Only the device knows the rows, and a mean
+// of what the host knows misleads where the tokens meet in few experts (or where TOTAL_ROWS is a capacity): every tile unpacks its
+// expert's weights again.  us, all tiles of 128 / of 64 / picked here, 288 experts, Q2_K, gate and up of 1536 x 5120: 64 tokens
+// 1000 / 665 / 660; 512 that all choose the same eight 193 / 251 / 190; 1400 skewed by 1 / rank^0.4 1241 / - / 1044, 4096 1756 / - / 1788.
+// Where the two are close tiles of 128 are taken: many small tiles of few columns cost more than the sum says (model 0.93, measured 1.03).
+template <int FMT, bool DENSE, int NT, int NT2>
+__global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(const __grid_constant__ MmMaps maps, const MmParams p) {
+  typedef MmGeom<FMT, NT> G;
+  typedef MmSmem<FMT, NT, NT2> S;
+  constexpr uint32_t TMEM_COLS = 512;
+  static_assert(!NT2 || MmGeom<FMT, NT2 ? NT2 : NT>::THREADS == G::THREADS, "one launch for both");
+  static_assert(sizeof(MmBars<FMT, NT>) <= MM_BARS && sizeof(MmBars<FMT, NT2 ? NT2 : NT>) <= MM_BARS, "barriers");
+  extern __shared__ __align__(1024) u8 smem_raw[];
+  u8* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  MmBars<FMT, NT>* bars = (MmBars<FMT, NT>*)(smem + S::BODY);
+  MmBars<FMT, NT2 ? NT2 : NT>* bars2 = (MmBars<FMT, NT2 ? NT2 : NT>*)(smem + S::BODY + MM_BARS);
+  int* tile_first = (int*)(smem + S::FIRST);          // [ne + 1] first row tile of each expert; the total
+  uint32_t* tmem_slot = (uint32_t*)(smem + S::SLOTS);
+  uint32_t* narrow = tmem_slot + 1;                   // NT2: tiles of up to NT2 rows
+  uint4* iq_grid = (uint4*)(smem + S::TABLES);        // [256 entries][8 copies] the grid as halves
+  uint32_t* iq_sgn = (uint32_t*)(iq_grid + 8 * 256);  // [128 entries][32 copies] the eight signs (w_iq2xxs)
+
+  // the warp number through a shuffle: the compiler then knows that the role branches are warp-uniform
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+
+  // ---- once per CTA: barriers, tables, tensor memory; then, after the kernel before, the experts' row tiles counted
+  // (first tile of each expert, in shared memory).
+  pdl_launch_dependents();
+  if (tid == 32) {
+    bars->init();
+    if constexpr (NT2 != 0) bars2->init();
+    mbar_fence_init();
+  }
+  if (FMT == ILL_IQ2_XXS) {
+    for (int i = tid; i < 8 * 256; i += G::THREADS) {
+      const uint64_t g = ill_iq2xxs_grid[i >> 3];
+      uint32_t h[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const __half2 hh = __floats2half2_rn((float)((g >> (16 * k)) & 0xff), (float)((g >> (16 * k + 8)) & 0xff));
+        h[k] = *(const uint32_t*)&hh;
+      }
+      iq_grid[i] = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+    for (int i = tid; i < 32 * 128; i += G::THREADS) {
+      const uint32_t s7 = (uint32_t)i >> 5, sg = s7 | ((__popc(s7) & 1u) << 7);
+      iq_sgn[i] = (sg << 9) | (sg << 24);
+    }
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
+  pdl_wait();
+  int bm = DENSE ? p.bm : NT;
+  if constexpr (NT2 != 0) {  // every expert's rows, all loads at once
+    for (int e = tid; e < p.ne; e += G::THREADS) tile_first[e] = min(max(mm_count<DENSE>(p, e), 0), 1 << 22);
+    __syncthreads();
+  }
+  if (warp == 0) {
+    if constexpr (NT2 != 0) {
+      float more = 0.0f;                         // what tiles of NT2 cost more, for a margin of a tenth
+      for (int e = lane; e < p.ne; e += 32) {
+        const int c = tile_first[e];
+        more += 1.1f * (float)mm_cost64(c) - (float)mm_cost128(c);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) more += __shfl_xor_sync(0xffffffffu, more, o);
+      if (more <= 0.0f) bm = NT2;
+      if (lane == 0) *narrow = bm == NT2;
+    }
+    int before = 0;
+    for (int e0 = 0; e0 < p.ne; e0 += 32) {
+      const int e = e0 + lane;
+      const int c = e >= p.ne ? 0 : NT2 ? tile_first[e] : mm_count<DENSE>(p, e);
+      const int tiles = (c + bm - 1) / bm;
+      int incl = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (e < p.ne) tile_first[e] = before + incl - tiles;
+      before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) tile_first[p.ne] = before;  // row tiles in all
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  if constexpr (NT2 != 0) {
+    if (__shfl_sync(0xffffffffu, *narrow, 0)) mm_tiles<FMT, DENSE, NT2>(maps, p, NT2, smem, bars2, tile_first, iq_grid, iq_sgn, tmem_base, warp, lane);
+    else mm_tiles<FMT, DENSE, NT>(maps, p, NT, smem, bars, tile_first, iq_grid, iq_sgn, tmem_base, warp, lane);
+  } else {
+    mm_tiles<FMT, DENSE, NT>(maps, p, DENSE ? p.bm : NT, smem, bars, tile_first, iq_grid, iq_sgn, tmem_base, warp, lane);
   }
   tc_fence_before();
   __syncthreads();
@@ -1565,32 +1629,24 @@ struct MmVariant {
   size_t smem;
   int threads, regs_sum;
 };
-template <int FMT, bool DENSE, int NT>
+template <int FMT, bool DENSE, int NT, int NT2 = 0>
 static MmVariant mm_one() {
   typedef MmGeom<FMT, NT> G;
-  return MmVariant{(const void*)mm_id_kernel<FMT, DENSE, NT>, G::SMEM, G::THREADS, G::REGS_SUM};
+  constexpr int sum2 = MmGeom<FMT, NT2 ? NT2 : NT>::REGS_SUM;
+  return MmVariant{(const void*)mm_id_kernel<FMT, DENSE, NT, NT2>, MmSmem<FMT, NT, NT2>::SMEM, G::THREADS, G::REGS_SUM > sum2 ? G::REGS_SUM : sum2};
 }
+// The kernel for tiles of up to NT rows of X of a dense matrix; for experts (NT 0) the formats with mins pick on the device between
+// tiles of 64, whose A ring holds two blocks, and of 128.  IQ2_XXS and Q6_K, bound by their unpacking, gain 0 to 2 % from tiles of
+// 64 where no expert has more rows and lose up to 90 % elsewhere: always 128.  (A kernel of both made IQ2_XXS's tiles of 128 10 % slower.)
 template <int FMT>
-static MmVariant mm_variant(bool dense, int nt) {
+static MmVariant mm_variant(int nt) {
   if constexpr (FMT == ILL_Q6_K)
-    if (dense && nt == 256) return mm_one<FMT, true, 256>();
+    if (nt == 256) return mm_one<FMT, true, 256>();
   if constexpr (FMT == ILL_Q4_K || FMT == ILL_Q6_K)
-    if (dense) return nt == 64 ? mm_one<FMT, true, 64>() : mm_one<FMT, true, 128>();
-  if constexpr (FMT == ILL_Q2_K || FMT == ILL_Q4_K)
-    if (nt == 64) return mm_one<FMT, false, 64>();
-  return mm_one<FMT, false, 128>();
+    if (nt) return nt == 64 ? mm_one<FMT, true, 64>() : mm_one<FMT, true, 128>();
+  if constexpr (FMT == ILL_Q2_K || FMT == ILL_Q4_K) return mm_one<FMT, false, 128, 64>();
+  else return mm_one<FMT, false, 128>();
 }
-
-// Whether experts of few rows get tiles of 64 (whose A ring holds two blocks) in a launch of their own.  Only the formats with mins
-// gain from them; IQ2_XXS and Q6_K, bound by their unpacking, take 0 to 2 % less time with 64 rows an expert or fewer and up to 1.9
-// times as long with more, each tile unpacking the weights again.  The host does not know an expert's rows, so the experts are
-// dealt out on the device: up to MM_FEW rows to tiles of 64, the others to tiles of 128.  The launch that finds none costs 4 to 6 us.
-// us, tiles of 128 / of 64 / dealt out: gate and up of 288 experts of 1536 x 5120 (Q2_K) for 64 tokens 999 / 705 / 709, 6912 rows
-// (24 an expert) skewed by 1 / rank^1.1 1334 / 1084 / 1042, 512 tokens that all choose the same eight 193 / 255 / 200.
-// Above a mean of 24 rows all take tiles of 128 in one launch: 96 rows each 1408 against 2079 (but with 32 each 1218 / 890, with 64
-// each 1323 / 1100: the line could lie higher).  TOTAL_ROWS may be a capacity of which fewer rows are in use; the mean is then the larger.
-constexpr int MM_FEW = 64;
-static bool mm_few_rows(int fmt, long long rows, int ne) { return (fmt == ILL_Q2_K || fmt == ILL_Q4_K) && rows / ne <= 24; }
 
 // Rows of X a tile of a dense matrix: the rounds of tiles on the SMs times a tile's measured time a block of 256 columns, us; tiles
 // of up to 64, of up to 128, and (Q6_K, which has one accumulator a block: with two, draining 256 columns takes longer than it
@@ -1652,34 +1708,30 @@ static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptr
   p.one_count = (unsigned)total_rows;
   p.acc = acc;
   p.status = device_status_word();
-  if (ne > 512) return ILL_ERR_TOO_LARGE;
+  if (ne > MM_MAX_NE) return ILL_ERR_TOO_LARGE;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   const long long ntn = (nrows + MM_BN - 1) / MM_BN * (y2 ? 2 : 1);
-  const auto launch = [&](int bm, int min_rows, int max_rows) -> int {
-    p.bm = bm;
-    p.min_rows = min_rows;
-    p.max_rows = max_rows;
-    const int nt = bm <= 64 ? 64 : bm <= 128 ? 128 : 256;
-    const long long max_tiles = ((total_rows + bm - 1) / bm + ne) * ntn;  // an upper bound
-    const MmVariant v = fmt == ILL_IQ2_XXS ? mm_variant<ILL_IQ2_XXS>(false, nt) : fmt == ILL_Q2_K ? mm_variant<ILL_Q2_K>(false, nt)
-                        : fmt == ILL_Q4_K ? mm_variant<ILL_Q4_K>(one_ptr != 0, nt) : mm_variant<ILL_Q6_K>(one_ptr != 0, nt);
-    cudaError_t e = cudaFuncSetAttribute(v.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem);
-    if (e != cudaSuccess) return cuda_fail(e);
-    // The warp groups trade registers after launch; what they ask for together must fit in what the
-    // CTA was given, or the drain warps would wait for registers for ever.
-    cudaFuncAttributes fa;
-    e = cudaFuncGetAttributes(&fa, v.k);
-    if (e != cudaSuccess) return cuda_fail(e);
-    if (fa.numRegs / 8 * 8 * v.threads < v.regs_sum) return ILL_ERR_UNSUPPORTED;
-    void* args[] = {&maps, &p};
-    // persistent: a CTA an SM, each walks tiles
-    return launch_kernel(v.k, dim3((unsigned)(max_tiles < sms ? max_tiles : sms)), dim3((unsigned)v.threads), v.smem, args, (cudaStream_t)stream);
-  };
-  const int all = 0x7fffffff;
-  if (one_ptr) return launch(mm_pick_tile(fmt, total_rows, ntn, sms), 0, all);
-  if (!mm_few_rows(fmt, total_rows, ne)) return launch(128, 0, all);
-  const int rc = launch(64, 0, MM_FEW);
-  return rc || total_rows <= MM_FEW ? rc : launch(128, MM_FEW + 1, all);
+  int nt = 0;
+  p.bm = MM_BN;
+  if (one_ptr) {
+    p.bm = mm_pick_tile(fmt, total_rows, ntn, sms);
+    nt = p.bm <= 64 ? 64 : p.bm <= 128 ? 128 : 256;
+  }
+  const int least = one_ptr ? p.bm : 64;         // rows of X a tile
+  const long long max_tiles = ((total_rows + least - 1) / least + ne) * ntn;  // an upper bound
+  const MmVariant v = fmt == ILL_IQ2_XXS ? mm_variant<ILL_IQ2_XXS>(nt) : fmt == ILL_Q2_K ? mm_variant<ILL_Q2_K>(nt)
+                      : fmt == ILL_Q4_K ? mm_variant<ILL_Q4_K>(nt) : mm_variant<ILL_Q6_K>(nt);
+  cudaError_t e = cudaFuncSetAttribute(v.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem);
+  if (e != cudaSuccess) return cuda_fail(e);
+  // The warp groups trade registers after launch; what they ask for together must fit in what the
+  // CTA was given, or the drain warps would wait for registers for ever.
+  cudaFuncAttributes fa;
+  e = cudaFuncGetAttributes(&fa, v.k);
+  if (e != cudaSuccess) return cuda_fail(e);
+  if (fa.numRegs / 8 * 8 * v.threads < v.regs_sum) return ILL_ERR_UNSUPPORTED;
+  void* args[] = {&maps, &p};
+  // persistent: a CTA an SM, each walks tiles
+  return launch_kernel(v.k, dim3((unsigned)(max_tiles < sms ? max_tiles : sms)), dim3((unsigned)v.threads), v.smem, args, (cudaStream_t)stream);
 }

@@ -223,7 +223,7 @@ def test_expert_chunk_tiles(fmt, base, rows, cols, counts):
 @pytest.mark.parametrize("fmt", [B.IQ2_XXS, B.Q2_K])
 def test_an_expert_of_many_rows_among_idle_ones(fmt):
     """All rows of a chunk on one of 32 experts: 799 rows (a mean of 24 an expert) take no longer than 800 (25), whatever tiles the
-    mean asks for.  Medians of 15 launches in turn; the margin is for a second launch and the clocks (0.99 and 1.02; with tiles of 64 for every expert 1.72 and 1.36)."""
+    mean asks for.  Medians of 15 launches in turn; the margin is for the clocks (1.00; with tiles of 64 for every expert 1.72 and 1.36)."""
     rows, cols, ne = 128 * 148, 4096, 32
     w = B.synth_matrix_torch(fmt, rows, cols, seed=1)
     ptrs = torch.full((ne,), w.data_ptr(), dtype=torch.int64, device="cuda")
