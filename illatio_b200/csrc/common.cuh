@@ -21,11 +21,14 @@ typedef signed char i8;
 typedef unsigned short u16;
 
 // device status codes (written once, first writer wins)
-enum { ST_OK = 0, ST_MV_WAIT = 0x100, ST_MM_WAIT_FULL = 0x200, ST_MM_WAIT_EMPTY = 0x300,
-       ST_MM_WAIT_ACC = 0x400, ST_MM_WAIT_EPI = 0x500,
+enum { ST_OK = 0, ST_MV_WAIT = 0x100,
+       ST_MM_WAIT_FULL = 0x200 /* the chunk kernel: X; + 1 a K step of A, + 2 raw blocks, + 3 the mins, + 4 the sums of 16 */,
+       ST_MM_WAIT_EMPTY = 0x300 /* a stage of X is free; + 1 a slot of A, + 2 a raw buffer, + 3 a tile of mins, + 4 one of sums */,
+       ST_MM_WAIT_ACC = 0x400 /* a block's products */,
+       ST_MM_WAIT_EPI = 0x500 /* an accumulator has been drained; + 2 the mins' */,
        ST_GROUP_SEL = 0x600 /* an expert number out of range in ill_moe_group's SEL */,
        ST_BARRIER_WAIT = 0x700 /* a barrier between CTAs or ranks never completed */,
-       ST_TEST_WAIT = 0x800 /* ill_test_wait_timeout: the wait that is meant to run out */ };
+       ST_TEST_WAIT = 0x800 /* ill_test_wait_timeout: the wait that is meant to run out; + 1 + l: lane l's of ill_test_poll_timeout */ };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -97,6 +100,39 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
   if (status) atomicCAS(status, 0u, code);
   return false;
 }
+
+// Barriers that a warp's lanes watch, one each: one poll shows all their phases.  Waiting is bounded as in mbar_wait; when it runs
+// out the status word gets the code of the first lane whose barrier is missing.
+struct BarPoll {
+  unsigned int* status;
+  unsigned code, ready = 0;    // the lane's own code
+  unsigned long long limit_ns;
+  __device__ __forceinline__ BarPoll(unsigned int* st, unsigned c, unsigned long long limit = ILL_WAIT_NS) : status(st), code(c), limit_ns(limit) {}
+  // until the phases of parity PAR of the BARs of the lanes in NEED have completed; the same answer in every lane.  A lane sees
+  // (acquires) its own barrier only and a ballot orders no memory: the __syncwarp hands what the lanes saw to those that act on it.
+  __device__ __forceinline__ bool until(uint64_t* bar, uint32_t par, uint32_t need) {
+    if ((ready & need) == need) return true;  // (the ballot that showed it was followed by a __syncwarp)
+    unsigned long long t0 = 0;
+    for (unsigned it = 1;; ++it) {
+      ready = __ballot_sync(0xffffffffu, mbar_test(bar, par));
+      __syncwarp();
+      const uint32_t missing = need & ~ready;
+      if (!missing) return true;
+      // the warp sleeps on the first that is missing (and takes no issue slots meanwhile)
+      const int l = __ffs(missing) - 1;
+      mbar_try_wait_at(__shfl_sync(0xffffffffu, smem_u32(bar), l), __shfl_sync(0xffffffffu, par, l), 20000);
+      if ((it & 63u) == 0) {
+        const unsigned long long now = __shfl_sync(0xffffffffu, global_ns(), 0);
+        if (t0 == 0) t0 = now;
+        else if (now - t0 > limit_ns) {
+          const unsigned c = __shfl_sync(0xffffffffu, code, l);
+          if (status) atomicCAS(status, 0u, c);
+          return false;
+        }
+      }
+    }
+  }
+};
 
 // ---- ranks meet without a collective: flags in peer memory -------------------------------------
 // Every rank owns an array of flags, EP_FLAG_SLOTS x EP_MAX_RANKS words, that its peers can store into

@@ -60,9 +60,33 @@ __global__ void __launch_bounds__(32) test_wait_kernel(unsigned long long limit_
   if (threadIdx.x == 0 && gave_up) *gave_up = ok ? 0u : 1u;
 }
 
+// A poll over 32 barriers, one a lane, of which those of the lanes in ARRIVED have completed their phase, until those in NEED have;
+// lane l's code is ST_TEST_WAIT + 1 + l.
+__global__ void __launch_bounds__(32) test_poll_kernel(unsigned long long limit_ns, unsigned arrived, unsigned need, unsigned int* status,
+                                                       unsigned int* gave_up) {
+  __shared__ uint64_t bar[32];
+  const unsigned l = threadIdx.x;
+  mbar_init(&bar[l], 1);
+  mbar_fence_init();
+  __syncwarp();
+  if (arrived >> l & 1u) mbar_arrive(&bar[l]);
+  BarPoll poll(status, ST_TEST_WAIT + 1 + l, limit_ns);
+  const bool ok = poll.until(&bar[l], 0u, need) && poll.until(&bar[l], 0u, need);  // (the second look finds what the first saw)
+  if (l == 0 && gave_up) *gave_up = ok ? 0u : 1u;
+}
+
 }  // namespace ill
 
 using namespace ill;
+
+extern "C" int ill_test_poll_timeout(int64_t limit_ns, uint32_t arrived, uint32_t need, ill_dptr gave_up, ill_stream stream) {
+  if (limit_ns < 1000 || limit_ns > 100000000ll || (gave_up & 3)) return ILL_ERR_ARG;  // 1 us .. 100 ms
+  unsigned long long lim = (unsigned long long)limit_ns;
+  unsigned int* st = device_status_word();
+  unsigned int* gu = (unsigned int*)(uintptr_t)gave_up;
+  void* args[] = {&lim, &arrived, &need, &st, &gu};
+  return launch_kernel((const void*)test_poll_kernel, dim3(1), dim3(32), 0, args, (cudaStream_t)stream);
+}
 
 extern "C" int ill_test_wait_timeout(int64_t limit_ns, ill_dptr gave_up, ill_stream stream) {
   if (limit_ns < 1000 || limit_ns > 100000000ll || (gave_up & 3)) return ILL_ERR_ARG;  // 1 us .. 100 ms

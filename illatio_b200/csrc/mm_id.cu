@@ -333,35 +333,6 @@ __device__ __forceinline__ void w_q6k(const uint32_t* ql, const uint32_t* qh, in
   }
 }
 
-// The barriers that a role's lanes watch, one each: one poll shows all their phases.  Waiting is bounded as in mbar_wait.
-struct MmPoll {
-  unsigned int* status;
-  unsigned code, ready = 0;
-  __device__ __forceinline__ MmPoll(unsigned int* st, unsigned c) : status(st), code(c) {}
-  // until the phases of parity PAR of the BARs of the lanes in NEED have completed; the same answer in every lane.  A lane sees
-  // (acquires) its own barrier only and a ballot orders no memory: the __syncwarp hands what the lanes saw to those that act on it.
-  __device__ __forceinline__ bool until(uint64_t* bar, uint32_t par, uint32_t need) {
-    if ((ready & need) == need) return true;  // (the ballot that showed it was followed by a __syncwarp)
-    unsigned long long t0 = 0;
-    for (unsigned it = 1;; ++it) {
-      ready = __ballot_sync(0xffffffffu, mbar_test(bar, par));
-      __syncwarp();
-      const uint32_t missing = need & ~ready;
-      if (!missing) return true;
-      // the warp sleeps on the first that is missing (and takes no issue slots meanwhile)
-      const int l = __ffs(missing) - 1;
-      mbar_try_wait_at(__shfl_sync(0xffffffffu, smem_u32(bar), l), __shfl_sync(0xffffffffu, par, l), 20000);
-      if ((it & 63u) == 0) {
-        const unsigned long long now = __shfl_sync(0xffffffffu, global_ns(), 0);
-        if (t0 == 0) t0 = now;
-        else if (now - t0 > ILL_WAIT_NS) break;
-      }
-    }
-    if (status) atomicCAS(status, 0u, code);
-    return false;
-  }
-};
-
 // The tensor maps of X (rows of 64 halves, two K steps a load) and of its sums of 16 for loads of 32, 64, 96 and 128 rows
 struct MmMaps {
   CUtensorMap x[4], e[4];
@@ -531,7 +502,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
           const bool wrap = s + lane >= NX;
           uint64_t* bar = lane == 2 && KM ? &eempty[b] : &xempty[lane < 2 ? (wrap ? s + lane - NX : s + lane) : s];
           const uint32_t par = lane == 2 && KM ? ((uint32_t)(g >> 1) & 1u) ^ 1u : ph ^ (wrap && lane < 2 ? 1u : 0u);
-          MmPoll poll(p.status, ST_MM_WAIT_EMPTY);
+          BarPoll poll(p.status, lane == 2 ? ST_MM_WAIT_EMPTY + 4 : ST_MM_WAIT_EMPTY);
 #pragma unroll
           for (int i = 0; i < (KM ? 3 : 2); ++i) {
             if (!(ok = poll.until(bar, par, 1u << i))) break;
@@ -570,6 +541,8 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
     int idx = lane < 2 ? lane : lane < 4 ? 0 : lane < 8 ? lane - 4 : lane == 11 ? 1 : 0;
     uint32_t par = lane == 8 || lane == 11 ? 1u : 0u;
     const bool per_block = (lane >= 4 && lane < 8) || lane == 10;  // shared by a block's jobs
+    const unsigned code = lane < 4 ? ST_MM_WAIT_FULL : lane < 8 ? ST_MM_WAIT_FULL + 1 : lane == 8 ? ST_MM_WAIT_EPI
+                          : lane == 9 ? ST_MM_WAIT_FULL + 4 : lane == 10 ? ST_MM_WAIT_FULL + 3 : ST_MM_WAIT_EPI + 2;
     const uint64_t xdesc0 = umma_desc(x_tiles);
     int s = 0, slot = 0, g = 0, g_kb = 0;          // X stage; first A slot of the block; jobs and blocks so far
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
@@ -587,7 +560,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
           const uint32_t d1 = tmem_base + (uint32_t)(b * DC);
           const uint32_t xstep = mm_boxes(rows) * (MM_XBOX * MM_BK * 2 / 16);  // a K step's tile in a stage
           uint64_t* aem = aempty + 4 * (g_kb & 1);
-          MmPoll poll(p.status, ST_MM_WAIT_FULL);
+          BarPoll poll(p.status, code);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             if (!(ok = poll.until(ring + idx, par, (i ? 0u : 0x100u) | (1u << (i >> 1)) | (0x10u << i)))) break;
@@ -654,7 +627,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
           const int set = g_kb % G::SETS, it = g_kb / G::SETS, buf = it & 1;
           // lane WQ < 4 watches the four warp pairs' buffers: the block two back must have been read from them
           uint64_t* bar = raw_empty + (set * 4 + (lane & 3)) * 2 + buf;
-          MmPoll poll(p.status, ST_MM_WAIT_EMPTY + 2);
+          BarPoll poll(p.status, ST_MM_WAIT_EMPTY + 2);
 #pragma unroll 1
           for (int wq = 0; wq < 4; ++wq) {
             if (!(ok = poll.until(bar, ((uint32_t)(it >> 1) & 1u) ^ 1u, 1u << wq))) break;

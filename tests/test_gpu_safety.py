@@ -52,6 +52,20 @@ def test_bounded_wait_runs_out_and_the_device_stays_usable(cuda_lib):
     assert _lib.status("ill_test_wait_timeout", 10, 0, None) == 1   # limits outside 1 us .. 100 ms are refused
 
 
+@pytest.mark.parametrize("arrived,need,code", [
+    (0xffffffff, 0x113, 0), (0x113, 0x113, 0), (0, 0, 0), (0x80000000, 0x80000000, 0),
+    (0x013, 0x113, 0x801 + 8), (0x112, 0x113, 0x801), (0, 0xffffffff, 0x801), (0x7fffffff, 0xffffffff, 0x801 + 31), (0x103, 0x630, 0x801 + 4),
+])
+def test_a_poll_that_runs_out_says_which_barrier_is_missing(cuda_lib, arrived, need, code):
+    """The wait of a warp whose lanes watch a barrier each: the status word names the first that is missing."""
+    assert _status() == (0, 0)
+    flag = torch.full((1,), 7, dtype=torch.int32, device="cuda")
+    _lib.call("ill_test_poll_timeout", 1_000_000, arrived, need, flag.data_ptr(), None)
+    torch.cuda.synchronize()
+    assert flag.item() == (1 if code else 0)
+    assert _status() == ((5, code) if code else (0, 0))
+
+
 def test_meeting_of_ranks_gives_up_when_a_peer_never_arrives(cuda_lib):
     """The flag barrier of the expert-parallel path, on one GPU: a world of two whose second rank never
     signals.  The meeting waits its millisecond, records the barrier's code and returns; once the missing
