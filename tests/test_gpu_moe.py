@@ -182,8 +182,8 @@ def test_a_table_that_the_kernel_before_has_written(fmt):
 @pytest.mark.parametrize("rows,cols", [(200, 768), (128, 256), (260, 2048)])
 @pytest.mark.parametrize("counts", [(0, 1, 64, 65, 3, 0, 15), (33, 127, 128, 129, 1), (300, 0, 256, 257, 17)])
 def test_expert_chunk_tiles(fmt, base, rows, cols, counts):
-    """The chunk product at the edges of its tiles (of up to 64, 128 and 256 rows of X, by the experts' mean), rows that are no
-    multiple of a tile, blocks at the alignments a format may have, fewer and more blocks than are in flight: against the
+    """The chunk product at the edges of its tiles (of up to 64 rows of X for the first counts, Q2_K and Q4_K, else 128), rows that
+    are no multiple of a tile, blocks at the alignments a format may have, fewer and more blocks than are in flight: against the
     one-token product of every row."""
     ne, n = len(counts), sum(counts)
     nbytes = B.matrix_bytes(fmt, rows, cols)
@@ -218,6 +218,51 @@ def test_expert_chunk_tiles(fmt, base, rows, cols, counts):
     # with mins: a few units of 2^-24 of the largest
     assert (y[:n, :rows] - want).abs().max().item() < 2e-6 * want.abs().max().item()
     assert (y[n] == 5.0).all() and (y[:, rows:] == 5.0).all()
+
+
+@pytest.mark.parametrize("fmt", [B.IQ2_XXS, B.Q2_K])
+@pytest.mark.parametrize("last", ["counts", "bases", "ptrs", "xh"])
+def test_chunk_tables_that_the_kernel_before_has_written(fmt, last):
+    """The experts' counts, first rows and addresses, and X, each written by the kernel just before the chunk product (whose launch lets
+    the product's begin at once).  The buffers hold valid values throughout, those of the other turn before each turn."""
+    cols, rows, n = 512, 256, 128
+    w = [B.synth_matrix_torch(fmt, rows, cols, seed=s) for s in (1, 2)]
+    acts = [D.quant_q8(torch.randn(n * cols, device="cuda"), D.make_qact(n * cols, "q8k")) for _ in range(2)]
+    acts[1].xs.copy_(acts[0].xs)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    src = dict(counts=[torch.tensor(c, **i32) for c in ((100, 28), (28, 100))], bases=[torch.tensor(b, **i32) for b in ((0, 100), (0, 28))],
+               ptrs=[torch.tensor([t.data_ptr() for t in o], dtype=torch.int64, device="cuda") for o in ((w[0], w[1]), (w[1], w[0]))], xh=acts)
+    now = dict(counts=src["counts"][1].clone(), bases=src["bases"][1].clone(), ptrs=src["ptrs"][1].clone())
+    own, ones, zero_one = torch.arange(2, **i32), torch.ones(2, **i32), torch.arange(2, **i32)
+    cf = D.ChunkF16(n, cols).fill(acts[1])
+
+    def write(what, i):
+        if what == "xh":
+            cf.fill(acts[i])
+        elif what == "ptrs":   # two rows of an expert each: the table of their addresses
+            _lib.call("ill_moe_row_ptrs", 2, src["ptrs"][i].data_ptr(), ones.data_ptr(), zero_one.data_ptr(), 2, now["ptrs"].data_ptr(), _lib.stream())
+        else:
+            _lib.call("ill_gather_rows", 2, 4, src[what][i].data_ptr(), own.data_ptr(), now[what].data_ptr(), _lib.stream())
+
+    def product(y):
+        _lib.call("ill_moe_mm_id", fmt, cols, rows, 0, now["ptrs"].data_ptr(), now["counts"].data_ptr(), now["bases"].data_ptr(), 2, n,
+                  cf.xh.data_ptr(), cf.xe.data_ptr(), acts[0].xs.data_ptr(), 0, 0, y.data_ptr(), rows, _lib.stream())
+        return y
+    order = [k for k in ("counts", "bases", "ptrs", "xh") if k != last] + [last]
+    want, y = [], torch.empty(20, n, rows, device="cuda")
+    for i in range(2):
+        for what in order:
+            write(what, i)
+        torch.cuda.synchronize()
+        want.append(product(torch.empty(n, rows, device="cuda")))
+        torch.cuda.synchronize()
+    assert not torch.equal(*want)
+    for i in range(20):
+        for what in order:
+            write(what, i % 2)
+        product(y[i])
+    for i in range(20):
+        assert torch.equal(y[i], want[i % 2])
 
 
 @pytest.mark.parametrize("fmt", [B.IQ2_XXS, B.Q2_K])

@@ -273,10 +273,12 @@ def test_quantizers_that_also_leave_the_fp16_forms():
 
 
 @pytest.mark.parametrize("fmt", [B.Q4_K, B.Q6_K])
-@pytest.mark.parametrize("rows,cols,n", [(128, 256, 1), (132, 768, 97), (1024, 2560, 513), (384, 2816, 31), (2560, 1024, 130), (19456, 256, 512)])
+@pytest.mark.parametrize("rows,cols,n", [(128, 256, 1), (132, 768, 97), (1024, 2560, 513), (384, 2816, 31), (2560, 1024, 130), (19456, 256, 512),
+                                         # on 148 SMs Q6_K takes tiles of two jobs here: 144, 176, 256, 256 and 208 rows, the last ones 97, 160, 256, 250 and 153
+                                         (5120, 256, 385), (5116, 768, 512), (17408, 256, 512), (18940, 256, 250), (4736, 512, 777)])
 def test_chunk_on_tcgen05_tiles(fmt, rows, cols, n):
-    """The tcgen05 chunk product at the edges of its tiles (16 to 256 tokens, by the number of tiles a matrix makes), with fewer
-    blocks than are in flight and matrices of one tile: against the one-token product, and adding to Y."""
+    """The tcgen05 chunk product at the edges of its tiles (16 to 128 tokens, Q6_K 16 to 256, by the number of tiles a matrix makes),
+    with fewer blocks than are in flight and matrices of one tile: against the one-token product, and adding to Y."""
     w, x, act = _case(fmt, rows, cols, n, seed=n)
     cf = D.ChunkF16(n, cols).fill(act)
     y = torch.full((n * rows + 64,), -3.0, device="cuda")
@@ -289,6 +291,22 @@ def test_chunk_on_tcgen05_tiles(fmt, rows, cols, n):
     y[:n * rows] = 1.0
     D.cmat_mul_tc(w, cf, y, acc=True)
     assert (y[:n * rows].view(n, rows) - 1.0 - want).abs().max().item() < 2e-6 * max(top, 1.0) + 2.0 ** -23 * (1.0 + top)
+
+
+@pytest.mark.parametrize("fmt", [B.Q4_K, B.Q6_K])
+@pytest.mark.parametrize("rows,cols,n", [(9472, 256, 512), (17408, 512, 512), (2176, 1024, 200), (9468, 256, 257), (132, 256, 3)])
+def test_gate_and_up_in_one_launch_tiles(fmt, rows, cols, n):
+    """Two matrices against one chunk, in tiles of one and (Q6_K, 9472 and 17408 rows: 256 rows each) of two jobs: the bits of two
+    launches, whatever tiles those take, and nothing past the last row."""
+    g, x, act = _case(fmt, rows, cols, n, seed=n)
+    u = D.CMat("u", fmt, rows, cols, B.synth_matrix_torch(fmt, rows, cols, seed=n + 7))
+    fa, fb = (torch.full((n * rows + 64,), -3.0, device="cuda") for _ in range(2))
+    D.glu_mul_tc(g, u, act, n, fa, fb)
+    cf = D.ChunkF16(n, cols).fill(act)
+    for w, y in ((g, fa), (u, fb)):
+        want = torch.empty(n * rows, device="cuda")
+        D.cmat_mul_tc(w, cf, want)
+        assert torch.equal(y[:n * rows], want) and (y[n * rows:] == -3.0).all()
 
 
 @pytest.mark.parametrize("fmt", [B.Q4_K, B.Q6_K])
