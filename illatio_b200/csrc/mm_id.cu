@@ -26,9 +26,10 @@
 // The roles' register needs differ widely, so the warp groups trade registers (setmaxnreg).
 // What bounds it: the drain beside the unpacking, by instructions and latency, not the tensor pipe or memory.  Left out for
 // timing: the drain's arithmetic 14-23 % of a launch, its stores 10 %, IQ2_XXS's unpacking 21 %, the X loads, the raw copies
-// and the products' width nothing.  us, with four drain warps, two raw-load warps and 128-row tiles throughout / now: gate and up
-// of 512 tokens x 2 x 9728 x 2560 (Q4_K) 151 / 81, 2560 x 9728 (Q6_K) 123 / 73, 512 rows on 288 experts of 5120 x 1536 (Q2_K, two
-// launches) 1249 / 740, 24576 rows on 256 experts, down 2048 x 4096 (Q2_K) 811 / 735, gate and up (IQ2_XXS) 1281 / 1301.
+// and the products' width nothing.  us, with four drain warps, two raw-load warps and 128-row tiles throughout / now, timed in turn:
+// gate and up of 512 tokens x 2 x 9728 x 2560 (Q4_K) 153 / 83, 2560 x 9728 (Q6_K) 123 / 74; 64 tokens on 288 experts (Q2_K), gate and
+// up of 1536 x 5120 1146 / 660, down 671 / 378; 96 rows each on 256 experts, down of 4096 x 2048 (Q2_K) 774 / 682, gate and up of 2048 x
+// 4096 (IQ2_XXS) 1292 / 1274.
 // Every mbarrier wait is bounded; on a time-out the kernel records a code in the status
 // word, skips what depends on the wait, lets copies and products in flight end, frees its tensor memory and returns.
 //
