@@ -1,0 +1,497 @@
+// mm_q8.cu -- Q8_0 products of a chunk of tokens (more than 16) on the 5th-generation tensor cores.
+//
+//   Y[token, row] (+)= sum over blocks b of 32 columns of  float(W_b[row] . X_b[token]) * (d_w * d_x)   (+ bias[row])
+//
+// Q8_0 has a scale for every 32 columns on both sides, so every 32-wide product of integers has to leave the tensor core and meet
+// its scales: tcgen05.mma.kind::i8 takes the int8 quants of both as they are (128 x N x 32, int32 accumulators: one instruction a
+// block, no conversion of either operand) and the drain turns the int32 sums into floats.  A row's blocks are added in order and each
+// step is rounded as the CPU path rounds it (Q8-ROW-DOT-AT, src/tensor.lisp:321-336: sum += float(isum) * (d_w * d_x)), so the bits do
+// not depend on the tile.
+//
+// A persistent CTA an SM walks tiles of 128 weight rows x BM (a multiple of 16, at most 128) tokens; columns go by in steps of 128.
+//   warp 0       brings X by TMA: a step of the tile's tokens, 128 bytes a token (128-byte swizzle), the MMA's B operand
+//   warp 1       allocates tensor memory; one lane issues the products
+//   warp 2       brings the weights' raw blocks by TMA: 176 bytes of each row, from the 16-byte boundary at or before the step's 136
+//   warp 3       brings the activations' scales (cp.async), transposed to [block][token]
+//   warps 4-19   drain: four warps for each 32 weight rows, a quarter of the tokens each
+//   warps 20-27  take the 34-byte blocks apart and store the quants to tensor memory, where they are the MMA's A operand: four warps,
+//                a row a lane, every second step
+// Tensor memory: three accumulators of 128 columns (a block of 128 tokens, two of 64 or four of 32 a job, so that a hand-over is
+// always about 128 columns' worth), four stages of A.
+//
+// What bounds it: the drain's instructions.  A sum takes a conversion, a multiplication d_w * d_x, one with the sum and an addition,
+// 512 issue slots a scheduler for 128 x 128 x 32 where the product itself takes 64 cycles (the packed f32x2 forms take two slots
+// each); with the loads of the scales, the hand-overs and the unpacking 830 are executed, at 72 % issue 1150 cycles.  us, int8
+// mma.sync (the kernel before) / now: 896 x 896 x 777 tokens 14.9 / 11.1, 896 x 4864 x 777 67 / 43, 4864 x 896 x 777 38 / 36,
+// 2048 x 4096 x 64 25 / 20, x 200 60 / 26, x 4096 297 / 288, 4096 x 2048 x 4096 298 / 277, 1536 x 5120 x 8192 548 / 548.
+// Measured and taken back: eight drain warps with the next half on its way while one is scaled (NT 128: 309 -> 398); 16 x 256-bit
+// loads of tensor memory, a quarter of the shared memory's traffic (309 -> 319: it was no bound); raw blocks by cp.async of the
+// warps that take them apart (a step 0.5 -> 1.1 us); quarters of the weight rows' tiles dealt evenly whatever the rounds
+// (4864 x 896 x 200 13.6 -> 16.3).
+//
+// Every mbarrier wait is bounded; on a time-out the kernel records a code in the status word, skips what depends on the wait, lets
+// copies and products in flight end, frees its tensor memory and returns.
+//
+// Replaces mm_q8_mma2 behind CMAT-MUL-N for prefill chunks (src/cuda-dense.lisp:220-255; src/cuda/dense.cu:885-1100).
+#include "formats.cuh"
+#include "tc05.cuh"
+#include "host.h"
+
+namespace ill {
+
+constexpr int MQ_ROWS = 128;                        // weight rows a tile (the MMA's M)
+constexpr int MQ_STEP = 128, MQ_WSTEP = 136;        // columns a step; a row's bytes of one (four blocks of 34)
+constexpr int MQ_NS = 4, MQ_NACC = 3, MQ_NRAW = 4;  // stages of X, A and scales; accumulators; stages of raw blocks
+constexpr int MQ_DRAIN = 16, MQ_UNPACK = 8, MQ_THREADS = 32 * (4 + MQ_DRAIN + MQ_UNPACK);
+constexpr int MQ_PITCH = 176;                       // bytes of a row in a raw stage: an odd number of 16-byte pieces
+constexpr uint32_t MQ_RAW_BYTES = MQ_ROWS * MQ_PITCH, MQ_A_COL = 128 * MQ_NACC;
+constexpr int MQ_REGS_AUX = 32, MQ_REGS_DRAIN = 88, MQ_REGS_UNPACK = 56;
+constexpr int MQ_REGS_SUM = 128 * MQ_REGS_AUX + 32 * (MQ_DRAIN * MQ_REGS_DRAIN + MQ_UNPACK * MQ_REGS_UNPACK);
+
+struct MqParams {
+  int rows, nsteps;
+  int split;           // rows are a multiple of 16 bytes apart only two by two: the even ones and the odd ones have a map each
+  int off[2];          // where the first row's bytes start in the (even, odd) map
+  int cols;
+  const float* xs;
+  float* y;
+  const float* bias;
+  int acc, n;
+  int bm;              // tokens a tile, a multiple of 16; a CTA takes every gridDim.x-th tile -- or, SHARE not 0,
+  int ncol, share;     // SHARE of the NCOL columns of 16 tokens of all the tiles of rows one after another, in tiles of up to BM
+  uint32_t zero;
+  unsigned* status;
+};
+struct MqMaps {
+  CUtensorMap x, w[2];
+};
+
+template <int NT> struct MqGeom {
+  static constexpr int G = 128 / NT, JOBS = 4 / G;  // blocks a job; jobs a step
+  static constexpr int TW = NT / 4;                 // tokens a drain warp
+  static constexpr uint32_t X_BYTES = NT * MQ_STEP;
+  static constexpr uint32_t RAW = MQ_NS * X_BYTES, WSC = RAW + MQ_NRAW * MQ_RAW_BYTES, XSC = WSC + MQ_NS * 4 * MQ_ROWS * 4,
+                            BARS = XSC + MQ_NS * 4 * NT * 4, SLOT = BARS + 8 * (2 * MQ_NS + 2 * MQ_NACC + 2 * MQ_NRAW + 1);
+  // at least what keeps a second CTA, which would wait for tensor memory, off the SM
+  static constexpr size_t NEED = SLOT + 16 + 1024 /* alignment */, SMEM = NEED > 118 * 1024 ? NEED : 118 * 1024;
+};
+
+// D[tmem] = A[tmem] * B[smem]^T, 128 x N x 32, int8 operands, int32 accumulators.  A: 128 lanes x 8 columns (four quants a column).
+__device__ __forceinline__ void umma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(bdesc), "r"(idesc)
+      : "memory");
+}
+__device__ __forceinline__ void mq_cp_async4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+// A CTA's tiles, in order
+struct MqWalk {
+  int pos, end, ntr;         // the tile, or column, next; past the last
+  int row0, tok0, nvalid;    // the tile
+  __device__ __forceinline__ explicit MqWalk(const MqParams& p) {
+    ntr = (p.rows + MQ_ROWS - 1) / MQ_ROWS;
+    pos = p.share ? blockIdx.x * p.share : blockIdx.x;
+    end = p.share ? min(pos + p.share, ntr * p.ncol) : ntr * ((p.n + p.bm - 1) / p.bm);
+  }
+  __device__ __forceinline__ bool next(const MqParams& p) {
+    if (pos >= end) return false;
+    if (p.share) {
+      const int rt = pos / p.ncol, col = pos - rt * p.ncol, take = min(min(p.bm / 16, end - pos), p.ncol - col);
+      row0 = rt * MQ_ROWS;
+      tok0 = 16 * col;
+      nvalid = min(16 * take, p.n - tok0);
+      pos += take;
+    } else {                 // tiles of rows vary fastest: CTAs running together share X
+      const int tt = pos / ntr;
+      row0 = (pos - tt * ntr) * MQ_ROWS;
+      tok0 = tt * p.bm;
+      nvalid = min(p.bm, p.n - tok0);
+      pos += gridDim.x;
+    }
+    return true;
+  }
+};
+
+template <int NT>
+__global__ void __launch_bounds__(MQ_THREADS, 1) mm_q8_kernel(const __grid_constant__ MqMaps maps, const MqParams p) {
+  typedef MqGeom<NT> G;
+  constexpr int JOBS = G::JOBS, GB = G::G, TW = G::TW;
+  extern __shared__ __align__(1024) u8 smem_raw[];
+  u8* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  u8* x_tiles = smem;                                // [MQ_NS][NT tokens][128 bytes], swizzled
+  u8* raw = smem + G::RAW;                           // [MQ_NRAW][128 rows][MQ_PITCH] (SPLIT: the even rows, then the odd ones)
+  float* wsc = (float*)(smem + G::WSC);              // [MQ_NS][4 blocks][128 weight rows]
+  float* xsc = (float*)(smem + G::XSC);              // [MQ_NS][4 blocks][NT tokens]
+  uint64_t* bars = (uint64_t*)(smem + G::BARS);
+  uint64_t *full = bars,                             // the step's X landed (TMA), its quants of the weights are in tensor memory (4 warps),
+                                                     // its scales in shared memory (those warps' and 32 lanes' copies)
+      *free = bars + MQ_NS,                          // the drain is through with the step (16 warps): so are the products
+      *acc_full = bars + 2 * MQ_NS,                  // a job's products completed
+      *acc_free = acc_full + MQ_NACC,                // the drain has read them (16 warps)
+      *raw_full = acc_free + MQ_NACC,                // the step's raw blocks landed (TMA)
+      *raw_free = raw_full + MQ_NRAW,                // they have been read (4 warps)
+      *fin = raw_free + MQ_NRAW;                     // after a time-out: the products issued so far completed
+  uint32_t* tmem_slot = (uint32_t*)(smem + G::SLOT);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+
+  pdl_launch_dependents();
+  if (tid == 32) {
+    for (int s = 0; s < MQ_NS; ++s) { mbar_init(&full[s], 1 + 4 + 32); mbar_init(&free[s], MQ_DRAIN); }
+    for (int b = 0; b < MQ_NACC; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_free[b], MQ_DRAIN); }
+    for (int r = 0; r < MQ_NRAW; ++r) { mbar_init(&raw_full[r], 1); mbar_init(&raw_free[r], 4); }
+    mbar_init(fin, 1);
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
+  const int nsteps = p.nsteps;
+  MqWalk tile(p);
+  bool ok = true;
+
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(MQ_REGS_AUX));
+    if (warp == 0) {
+      // ---- X by TMA
+      pdl_wait();
+      int k = 0;  // steps so far
+      while (ok && tile.next(p)) {
+        for (int st = 0; st < nsteps; ++st, ++k) {
+          const int s = k % MQ_NS;
+          ok = __all_sync(0xffffffffu, mbar_wait(&free[s], ((uint32_t)(k / MQ_NS) & 1u) ^ 1u, p.status, ST_MQ_WAIT));
+          if (!ok) break;
+          if (elect_one()) {
+            mbar_expect_tx(&full[s], p.bm * MQ_STEP);
+            tma_load_2d(x_tiles + s * G::X_BYTES, &maps.x, st * MQ_STEP, tile.tok0, &full[s]);
+          }
+          __syncwarp();
+        }
+      }
+      if (!ok)  // a wait ran out: the copies in flight land before the CTA goes
+        for (int j = max(0, k - MQ_NS); j < k; ++j) mbar_wait(&full[j % MQ_NS], (uint32_t)(j / MQ_NS) & 1u, nullptr, 0, 0, ILL_WAIT_NS / 20);
+    } else if (warp == 1) {
+      // ---- the products: the whole warp walks the loop, one elected lane issues.  Lane 0 watches the step, lane
+      // 1 the job's accumulator: one poll looks at both.
+      const uint64_t xdesc0 = umma_desc(x_tiles);
+      const unsigned code = ST_MQ_WAIT + 1 + (lane ? 1 : 0);
+      int k = 0, b = 0;
+      uint32_t bph = 1;  // parity that a free accumulator's barrier has completed (a fresh barrier: 1)
+      while (ok && tile.next(p)) {
+        // int32 accumulate, int8 A and B, both K-major, M = 128 weight rows, N = the tile's tokens up to 16
+        const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)((tile.nvalid + 15) >> 4) << 18) | ((uint32_t)(MQ_ROWS >> 4) << 24);
+        for (int st = 0; st < nsteps && ok; ++st, ++k) {
+          const int s = k % MQ_NS;
+#pragma unroll
+          for (int j = 0; j < JOBS; ++j) {
+            BarPoll poll(p.status, code);
+            uint64_t* bar = lane == 0 ? &full[s] : &acc_free[b];
+            if (!(ok = poll.until(bar, lane == 0 ? (uint32_t)(k / MQ_NS) & 1u : bph, j == 0 ? 3u : 2u))) break;
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+              for (int g = 0; g < GB; ++g)
+                umma_i8_ts(tmem_base + b * 128 + g * NT, tmem_base + MQ_A_COL + s * 32 + (j * GB + g) * 8,
+                           xdesc0 + (uint32_t)(s * (int)(G::X_BYTES >> 4)) + 2 * (j * GB + g), idesc);
+              umma_commit(&acc_full[b]);
+            }
+            __syncwarp();
+            if (++b == MQ_NACC) { b = 0; bph ^= 1; }
+          }
+        }
+      }
+      if (!ok) {
+        // a wait ran out: the products issued so far end before tensor memory is freed
+        if (elect_one()) umma_commit(fin);
+        __syncwarp();
+        mbar_wait(fin, 0, nullptr, 0, 0, ILL_WAIT_NS / 20);
+      }
+    } else if (warp == 2) {
+      // ---- the weights' raw blocks by TMA (they do not depend on the kernel before)
+      int k = 0;
+      while (ok && tile.next(p)) {
+        for (int st = 0; st < nsteps; ++st, ++k) {
+          const int r = k % MQ_NRAW;
+          ok = __all_sync(0xffffffffu, mbar_wait(&raw_free[r], ((uint32_t)(k / MQ_NRAW) & 1u) ^ 1u, p.status, ST_MQ_WAIT + 7));
+          if (!ok) break;
+          if (elect_one()) {
+            u8* dst = raw + r * MQ_RAW_BYTES;
+            mbar_expect_tx(&raw_full[r], MQ_RAW_BYTES);
+            if (p.split) {
+              tma_load_2d(dst, &maps.w[0], (p.off[0] + st * MQ_WSTEP) & ~15, tile.row0 / 2, &raw_full[r]);
+              tma_load_2d(dst + MQ_RAW_BYTES / 2, &maps.w[1], (p.off[1] + st * MQ_WSTEP) & ~15, tile.row0 / 2, &raw_full[r]);
+            } else {
+              tma_load_2d(dst, &maps.w[0], (p.off[0] + st * MQ_WSTEP) & ~15, tile.row0, &raw_full[r]);
+            }
+          }
+          __syncwarp();
+        }
+      }
+      if (!ok)
+        for (int j = max(0, k - MQ_NRAW); j < k; ++j)
+          mbar_wait(&raw_full[j % MQ_NRAW], (uint32_t)(j / MQ_NRAW) & 1u, nullptr, 0, 0, ILL_WAIT_NS / 20);
+    } else {
+      // ---- the activations' scales, [token][block] in memory, [block][token] in shared memory
+      pdl_wait();
+      const int nb = p.cols / 32;
+      int k = 0;
+      while (ok && tile.next(p)) {
+        const float* src0 = p.xs + (long long)(tile.tok0 + lane) * nb;
+        for (int st = 0; st < nsteps; ++st, ++k) {
+          const int s = k % MQ_NS;
+          ok = __all_sync(0xffffffffu, mbar_wait(&free[s], ((uint32_t)(k / MQ_NS) & 1u) ^ 1u, p.status, ST_MQ_WAIT + 4));
+          if (!ok) break;
+#pragma unroll
+          for (int t = 0; t < NT; t += 32)
+            if (t + lane < tile.nvalid) {
+              const float* src = src0 + (long long)t * nb + 4 * st;
+              float* dst = xsc + s * 4 * NT + t + lane;
+#pragma unroll
+              for (int b = 0; b < 4; ++b) mq_cp_async4(dst + b * NT, src + b);
+            }
+          cp_async_arrive(&full[s]);
+        }
+      }
+      cp_async_wait_all();
+    }
+  } else if (warp < 4 + MQ_DRAIN) {
+    // ---- drain.  A warp reads the 32 lanes of tensor memory that its number gives it (warp % 4: 32 weight rows) and a quarter of
+    // the tokens of every block: 32 columns a job.
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(MQ_REGS_DRAIN));
+    pdl_wait();
+    const int q = warp & 3, c0 = ((warp - 4) >> 2) * TW, m = q * 32 + lane;
+    const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + c0;
+    int s = 0, b = 0;
+    uint32_t sph = 0, bph = 0;
+    while (ok && tile.next(p)) {
+      const int nvalid = tile.nvalid;
+      float out[TW];
+#pragma unroll
+      for (int i = 0; i < TW; ++i) out[i] = 0.0f;
+      for (int st = 0; st < nsteps; ++st) {
+        // (complete as soon as the step's first products are: what makes the scales visible here)
+        bool lane_ok = mbar_wait(&full[s], sph, p.status, ST_MQ_WAIT + 5);
+        const float *ws = wsc + s * 4 * MQ_ROWS + m, *xs = xsc + s * 4 * NT + c0;
+#pragma unroll
+        for (int j = 0; j < JOBS; ++j) {
+          lane_ok = lane_ok && mbar_wait(&acc_full[b], bph, p.status, ST_MQ_WAIT + 6);
+          __syncwarp();
+          tc_fence_after();
+          uint32_t v[4][8];
+          if (c0 < nvalid) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) tmem_ld(t0 + b * 128 + (8 * r / TW) * NT + 8 * r % TW, v[r]);
+            tmem_ld_wait(v[0]);
+            tmem_ld_done(v[1]); tmem_ld_done(v[2]); tmem_ld_done(v[3]);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_free[b]);
+          if (++b == MQ_NACC) { b = 0; bph ^= 1; }
+          if (c0 < nvalid) {  // (columns past the tile's last token: whatever lies there; they are not stored)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              const int blk = j * GB + 8 * r / TW, c = 8 * r % TW;
+              const float dw = ws[blk * MQ_ROWS];
+#pragma unroll
+              for (int i = 0; i < 8; i += 4) {
+                const float4 dx = *(const float4*)(xs + blk * NT + c + i);
+                out[c + i] = __fadd_rn(out[c + i], __fmul_rn((float)(int)v[r][i], __fmul_rn(dw, dx.x)));
+                out[c + i + 1] = __fadd_rn(out[c + i + 1], __fmul_rn((float)(int)v[r][i + 1], __fmul_rn(dw, dx.y)));
+                out[c + i + 2] = __fadd_rn(out[c + i + 2], __fmul_rn((float)(int)v[r][i + 2], __fmul_rn(dw, dx.z)));
+                out[c + i + 3] = __fadd_rn(out[c + i + 3], __fmul_rn((float)(int)v[r][i + 3], __fmul_rn(dw, dx.w)));
+              }
+            }
+          }
+        }
+        if (!(ok = __all_sync(0xffffffffu, lane_ok))) break;
+        // (ZERO is none that the compiler knows: the step's last scales have been used, not only asked for, when it is given back)
+        if (lane == 0) mbar_arrive(free + s + (__float_as_uint(out[TW - 1]) & p.zero));
+        if (++s == MQ_NS) { s = 0; sph ^= 1; }
+      }
+      const int row = tile.row0 + m;
+      if (ok && row < p.rows) {
+        const float bias = p.bias ? p.bias[row] : 0.0f;
+        float* yp = p.y + (long long)(tile.tok0 + c0) * p.rows + row;
+#pragma unroll
+        for (int i0 = 0; i0 < TW; i0 += 8) {
+          if (c0 + i0 < nvalid) {
+            float old[8];
+            if (p.acc) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) old[i] = c0 + i0 + i < nvalid ? yp[(long long)(i0 + i) * p.rows] : 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              float r = out[i0 + i];
+              if (p.bias) r += bias;
+              if (p.acc) r = old[i] + r;
+              if (c0 + i0 + i < nvalid) yp[(long long)(i0 + i) * p.rows] = r;
+            }
+          }
+        }
+      }
+    }
+  } else {
+    // ---- the weights: a warp has 32 rows of every second step, a lane one of them
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(MQ_REGS_UNPACK));
+    const int q = warp & 3, set = (warp - 4 - MQ_DRAIN) >> 2, row = 32 * q + lane, odd = p.split & row & 1;
+    const uint32_t a0 = tmem_base + ((uint32_t)(q * 32) << 16) + MQ_A_COL;
+    const u8* mine = raw + (p.split ? odd * (MQ_RAW_BYTES / 2) + (row >> 1) * MQ_PITCH : row * MQ_PITCH);
+    const int off = odd ? p.off[1] : p.off[0];
+    const bool by8 = (off & 7) == 0;                 // (the same for all: rows lie a multiple of eight bytes apart)
+    int k = 0;
+    while (ok && tile.next(p)) {
+      for (int st = 0; st < nsteps; ++st, ++k) {
+        if ((k & 1) != set) continue;
+        const int s = k % MQ_NS, r = k % MQ_NRAW;
+        const uint32_t free_par = ((uint32_t)(k / MQ_NS) & 1u) ^ 1u;
+        ok = __all_sync(0xffffffffu, mbar_wait(&raw_full[r], (uint32_t)(k / MQ_NRAW) & 1u, p.status, ST_MQ_WAIT + 2));
+        if (!ok) break;
+        // the step's 34 words: four blocks of a half and 32 quants, 34 bytes apart
+        const uint32_t o16 = (uint32_t)(off + st * MQ_WSTEP) & 15u, sh = 8 * (o16 & 2u);
+        const u8* src = mine + r * MQ_RAW_BYTES + (o16 & ~3u);
+        auto words = [&](int w0, int n, uint32_t* w) {
+          if (by8) {
+#pragma unroll
+            for (int i = 0; i < 18; i += 2)
+              if (i < n) {
+                const uint2 v = *(const uint2*)(src + 4 * (w0 + i));
+                w[i] = v.x;
+                w[i + 1] = v.y;
+              }
+          } else {                                   // a row may start in the middle of a word
+#pragma unroll
+            for (int i = 0; i < 18; ++i)
+              if (i < n) w[i] = __funnelshift_r(*(const uint32_t*)(src + 4 * (w0 + i)), *(const uint32_t*)(src + 4 * (w0 + i) + 4), sh);
+          }
+        };
+        uint32_t w[18], a[16], d[4];
+        words(0, 18, w);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          a[i] = __funnelshift_r(w[i], w[i + 1], 16);
+          a[8 + i] = w[9 + i];
+        }
+        d[0] = w[0] & 0xffffu;
+        d[1] = w[8] >> 16;
+        const uint32_t w17 = w[17];
+        ok = __all_sync(0xffffffffu, mbar_wait(&free[s], free_par, p.status, ST_MQ_WAIT + 3));
+        if (!ok) break;
+        tc_fence_after();
+        tmem_st16(a0 + s * 32, a);
+        words(18, 16, w);
+        d[2] = w17 & 0xffffu;
+        d[3] = w[7] >> 16;
+        a[0] = __funnelshift_r(w17, w[0], 16);
+#pragma unroll
+        for (int i = 1; i < 8; ++i) a[i] = __funnelshift_r(w[i - 1], w[i], 16);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[8 + i] = w[8 + i];
+        tmem_st16(a0 + s * 32 + 16, a);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) wsc[(s * 4 + i) * MQ_ROWS + row] = h2f(d[i]);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        // (the raw words have been stored by now, not only asked for)
+        if (lane == 0) { mbar_arrive(&full[s]); mbar_arrive(&raw_free[r]); }
+      }
+    }
+    tmem_st_wait();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, 512);
+}
+
+template <int NT>
+static int mq_launch(const MqMaps& maps, const MqParams& p, int grid, cudaStream_t st) {
+  const void* k = (const void*)mm_q8_kernel<NT>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MqGeom<NT>::SMEM);
+  if (e != cudaSuccess) return cuda_fail(e);
+  // the warp groups trade registers after launch: what they ask for together must fit in what the CTA was given
+  static const int regs = [k] {
+    cudaFuncAttributes fa;
+    return cudaFuncGetAttributes(&fa, k) == cudaSuccess ? fa.numRegs : 0;
+  }();
+  if (regs / 8 * 8 * MQ_THREADS < MQ_REGS_SUM) return ILL_ERR_UNSUPPORTED;
+  MqMaps m = maps;
+  MqParams pp = p;
+  void* args[] = {&m, &pp};
+  return launch_kernel(k, dim3((unsigned)grid), dim3(MQ_THREADS), MqGeom<NT>::SMEM, args, st);
+}
+
+// A map of ROWS rows of BYTES bytes, STRIDE apart (a multiple of 16, as BASE), read in boxes of BOX_BYTES x BOX_ROWS
+static bool byte_map(CUtensorMap* map, uint64_t base, uint64_t bytes, uint64_t rows, uint64_t stride, uint32_t box_bytes, uint32_t box_rows,
+                     bool swizzle) {
+  EncodeTiledFn enc = encode_tiled_fn();
+  if (!enc) return false;
+  const cuuint64_t dims[2] = {bytes, rows}, strides[1] = {stride};
+  const cuuint32_t box[2] = {box_bytes, box_rows}, estr[2] = {1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)(uintptr_t)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// N tokens of a Q8_0 matrix; ILL_ERR_UNSUPPORTED for what it is not written for.
+int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t y, uint64_t bias, int acc, int n, void* stream) {
+  if (n < 2 || cols % MQ_STEP || (xq & 15) || (xs & 15) || (w & 1)) return ILL_ERR_UNSUPPORTED;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+  MqParams p = {};
+  p.rows = rows;
+  p.cols = cols;
+  p.nsteps = cols / MQ_STEP;
+  p.xs = (const float*)(uintptr_t)xs;
+  p.y = (float*)(uintptr_t)y;
+  p.bias = (const float*)(uintptr_t)bias;
+  p.acc = acc;
+  p.n = n;
+  p.status = device_status_word();
+  const long long ntr = (rows + MQ_ROWS - 1) / MQ_ROWS, ncol = (n + 15) / 16;
+  if (ntr * ncol > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
+  // Tokens a tile: the rounds of tiles on the SMs times a tile's measured time a step, us (2048 rows x 4096 columns, every SM busy).
+  // A step's hand-overs cost 16 tokens as much as its arithmetic; above 64 tokens a block is a job of its own.
+  static const float step_us[8] = {0.54f, 0.71f, 1.09f, 1.27f, 2.06f, 2.08f, 2.41f, 2.43f};
+  float best = 1e30f;
+  long long tiles = 0;
+  for (int bm = 16; bm <= 128; bm += 16) {
+    const long long count = ntr * ((n + bm - 1) / bm), rounds = (count + sms - 1) / sms;
+    const float us = (float)rounds * step_us[bm / 16 - 1];
+    if (us < best) { best = us; p.bm = bm; tiles = count; }
+  }
+  int grid = (int)(tiles < sms ? tiles : sms);
+  if (tiles > 8ll * sms) {
+    // many rounds: even shares instead of a last round that is half empty (1536 x 5120 x 8192 tokens, 11 rounds for 10.4:
+    // 562 -> 543 us; with fewer rounds the tile more at a share's ends costs what it saves)
+    p.bm = 64;
+    p.ncol = (int)ncol;
+    p.share = (int)((ntr * ncol + sms - 1) / sms);
+    grid = (int)((ntr * ncol + p.share - 1) / p.share);
+  }
+  MqMaps maps;
+  const uint64_t row_bytes = (uint64_t)cols / 32 * 34;
+  if (!byte_map(&maps.x, xq, cols, n, cols, MQ_STEP, p.bm, true)) return cuda_fail(cudaErrorInvalidValue);
+  // Rows lie a multiple of eight bytes apart; a map's have to lie a multiple of 16.  A row starts OFF bytes after a 16-byte boundary.
+  p.split = row_bytes % 16 != 0;
+  for (int i = 0; i < 2; ++i) {
+    const uint64_t base = w + (p.split && i && rows > 1 ? row_bytes : 0), count = p.split ? (rows > 1 ? (rows + 1 - i) / 2 : 1) : rows;
+    p.off[i] = (int)(base & 15);
+    if (!byte_map(&maps.w[i], base & ~15ull, p.off[i] + row_bytes, count, p.split ? 2 * row_bytes : row_bytes, MQ_PITCH,
+                  p.split ? MQ_ROWS / 2 : MQ_ROWS, false))
+      return cuda_fail(cudaErrorInvalidValue);
+  }
+  cudaStream_t st = (cudaStream_t)stream;
+  if (p.bm <= 32) return mq_launch<32>(maps, p, grid, st);
+  if (p.bm <= 64) return mq_launch<64>(maps, p, grid, st);
+  return mq_launch<128>(maps, p, grid, st);
+}
+
+}  // namespace ill
