@@ -43,6 +43,7 @@ SIGNATURES = {
     "ill_dequant_rows": (_I, [_I, _P, _I, _P, _L, _I, _P, _S]),
     "ill_mv": (_I, [_I, _P, _I, _I, _P, _P, _P, _P, _P, _I, _I, _S]),
     "ill_mv_3": (_I, [_I, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _S]),
+    "ill_mv_3n": (_I, [_I, _I, _I, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _S]),
     "ill_mv_glu": (_I, [_I, _P, _P, _I, _I, _P, _P, _P, _P, _S]),
     "ill_moe_mv": (_I, [_I, _I, _I, _L, _P, _I, _P, _P, _P, _I, _P, _L, _S]),
     "ill_moe_glu": (_I, [_I, _I, _I, _L, _L, _P, _I, _P, _P, _P, _I, _F, _P, _P, _L, _S]),

@@ -230,6 +230,18 @@ void mul_any(PyObject* w, PyObject* act, PyObject* y, long long n, PyObject* bia
   Ref r(PyObject_Vectorcall(slow(S_cmat_mul), av, 5, nullptr));
 }
 
+// Up to three products of up to 16 tokens that share the activations, in one launch (C null: two); false where that is not to be had
+inline bool mul_3(const Mat& a, const Mat& b, const Mat* c, const Act& x, ill_dptr ya, ill_dptr yb, ill_dptr yc, ill_dptr ba, ill_dptr bb,
+                  ill_dptr bc, int n) {
+  // (a Q8_0 matrix takes other activations than the K formats: not with them)
+  if ((a.type == 0) != (b.type == 0) || a.cols != b.cols || (c && ((c->type == 0) != (a.type == 0) || c->cols != a.cols))) return false;
+  const int rc = launch(ill_mv_3n, a.type, b.type, c ? c->type : 0, a.w, b.w, c ? c->w : 0, a.rows, b.rows, c ? c->rows : 0, a.cols, x.xq, x.xs, x.k ? x.xsum : 0, ya, yb,
+                        yc, ba, bb, bc, n, cur_stream());
+  if (rc == ILL_ERR_UNSUPPORTED) return false;
+  check("ill_mv_3n", rc);
+  return true;
+}
+
 PyObject* qkv_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
   ARGS("qkv_mul", 7, S_wq, S_wk, S_wv, S_act, S_q, S_k, S_v, S_bq, S_bk, S_bv, S_n);
   const long long n = OPT_INT(a[10], 1);
@@ -250,7 +262,14 @@ PyObject* qkv_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
       Py_RETURN_NONE;
     }
   }
-  for (int i = 0; i < 3; ++i) mul_any(a[i], a[3], a[4 + i], n, a[7 + i]);
+  int left = 0;
+  if (n > 1 && few(n)) {
+    const Mat q(a[0]), k(a[1]), v(a[2]);
+    const Act x(a[3]);
+    if (mul_3(q, k, &v, x, ptr(a[4]), ptr(a[5]), ptr(a[6]), OPT_PTR(a[7]), OPT_PTR(a[8]), OPT_PTR(a[9]), (int)n)) left = 3;
+    else if (mul_3(q, k, nullptr, x, ptr(a[4]), ptr(a[5]), 0, OPT_PTR(a[7]), OPT_PTR(a[8]), 0, (int)n)) left = 2;
+  }
+  for (int i = left; i < 3; ++i) mul_any(a[i], a[3], a[4 + i], n, a[7 + i]);
   Py_RETURN_NONE;
 } CATCH_ERRORS
 
@@ -274,8 +293,11 @@ PyObject* glu_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
                    (long long)fa.numel(), (long long)fb.numel(), len);
       throw Failed();
     }
-    mul_any(a[0], a[2], a[3], n, nullptr);
-    mul_any(a[1], a[2], a[5], n, nullptr);
+    const Mat g(a[0]), u(a[1]);
+    if (!(n > 1 && few(n) && g.rows == u.rows && g.type == u.type && mul_3(g, u, nullptr, Act(a[2]), ptr(a[3]), ptr(a[5]), 0, 0, 0, 0, (int)n))) {
+      mul_any(a[0], a[2], a[3], n, nullptr);
+      mul_any(a[1], a[2], a[5], n, nullptr);
+    }
     const ill_dptr fp = ptr(a[3]);
     LAUNCH(ill_silu_mul, len, fp, ptr(a[5]), fp, cur_stream());
     return ret(a[3]);
@@ -312,8 +334,9 @@ PyMethodDef methods[] = {
          "cmat_mul(w, act, y, n=1, bias=None, acc=False)\n--\n\nCMAT-MUL (src/cuda-dense.lisp:220-248): Y = W X for N tokens (token t's X at\n"
          "t*cols, its Y at t*rows), or Y += it when ACC."),
     FAST(qkv_mul,
-         "qkv_mul(wq, wk, wv, act, q, k, v, bq=None, bk=None, bv=None, n=1)\n--\n\nQKV-MUL (src/cuda-dense.lisp:309-324): for one token one\n"
-         "launch when the three formats agree, two when those of Q and K do; else three products."),
+         "qkv_mul(wq, wk, wv, act, q, k, v, bq=None, bk=None, bv=None, n=1)\n--\n\nQKV-MUL (src/cuda-dense.lisp:309-324): for up to 16\n"
+         "tokens one launch when the three formats agree (for several also when they are Q4_K and Q6_K), two when those of Q and\n"
+         "K do; else three products."),
     FAST(glu_mul,
          "glu_mul(g, u, act, fa, n=1, fb=None)\n--\n\nGLU-MUL (src/cuda-dense.lisp:326-339): silu(G x) * (U x) into FA; FB, of\n"
          "FA's shape, is scratch for the products that one launch does not take."),

@@ -840,7 +840,7 @@ int mv_common(int fmt, int mode, int nmat, const ill_dptr* w, const int* rows, i
     // several tokens: the tensor cores' int8 path where it is written (Q8_0, Q4_K, Q6_K; up to 16 tokens with the
     // activations resident, chunks with them streamed), else the token loop below
     int rc_t = ILL_ERR_UNSUPPORTED;
-    if (n <= 16) rc_t = mvt_try(fmt, w[0], rows[0], cols, xq, xs, xsum, y[0], bias ? bias[0] : 0, acc, n, stream);
+    if (n <= 16) rc_t = mvt_try(1, &fmt, w, rows, cols, xq, xs, xsum, y, bias, acc, n, stream);
     // a few tokens of rows too long for their activations to stay in shared memory
     if (rc_t == ILL_ERR_UNSUPPORTED && n <= 16) rc_t = mmk_try(fmt, w[0], rows[0], cols, xq, xs, xsum, y[0], bias ? bias[0] : 0, acc, n, stream);
     // a chunk
@@ -964,6 +964,21 @@ extern "C" int ill_mv_3(int fmt, ill_dptr w0, ill_dptr w1, ill_dptr w2, int rows
   const int rs[3] = {rows0, rows1, rows2};
   const int nmat = (rows2 == 0 && !w2) ? 2 : 3;
   return mv_common(fmt, MODE_PLAIN, nmat, ws, rs, cols, xq, xs, xsum, ys, bs, 0, 1, 0, 1, 0, 0, 0, 0, 0, 0.0f, stream);
+}
+
+extern "C" int ill_mv_3n(int fmt0, int fmt1, int fmt2, ill_dptr w0, ill_dptr w1, ill_dptr w2, int rows0, int rows1, int rows2, int cols,
+                         ill_dptr xq, ill_dptr xs, ill_dptr xsum, ill_dptr y0, ill_dptr y1, ill_dptr y2, ill_dptr b0,
+                         ill_dptr b1, ill_dptr b2, int n, ill_stream stream) {
+  const ill_dptr ws[3] = {w0, w1, w2}, ys[3] = {y0, y1, y2}, bs[3] = {b0, b1, b2};
+  const int rs[3] = {rows0, rows1, rows2}, fs[3] = {fmt0, fmt1, fmt2}, nmat = (rows2 == 0 && !w2) ? 2 : 3;
+  if (cols <= 0 || n < 2 || !xq || !xs) return ILL_ERR_ARG;
+  for (int i = 0; i < nmat; ++i) {
+    const int bw = fmt_block_weights(fs[i]);
+    if (!bw || cols % (bw == 32 ? 32 : 256) || rs[i] <= 0 || !ws[i] || !ys[i] || (needs_bsums(fs[i]) && !xsum)) return ILL_ERR_ARG;
+    if (ys[i] & 3) return ILL_ERR_ALIGN;
+  }
+  if (xq & 15 || xs & 3 || xsum & 7) return ILL_ERR_ALIGN;
+  return mvt_try(nmat, fs, ws, rs, cols, xq, xs, xsum, ys, bs, 0, n, stream);
 }
 
 extern "C" int ill_mv_glu(int fmt, ill_dptr wg, ill_dptr wu, int rows, int cols, ill_dptr xq, ill_dptr xs,

@@ -8,15 +8,21 @@
 // whatever the number of tokens.  The integers are the CPU kernels' (exact); each block's sum meets its float
 // scales as in the reference's portable loops (src/tensor.lisp:321-336, src/kquant.lisp:171-236).
 //
-//   * A persistent CTA of eight warps stages the tokens' quantized activations in shared memory once (token
-//     stride padded by 16 bytes, so that the eight tokens of a B fragment sit on different banks), then walks
-//     tiles of 16 rows.  The eight warps share a tile's blocks (warp w takes blocks w, w + 8, ...): small matrices
-//     still fill the SMs.  Each warp streams its (tile, block) pieces -- 16 row segments, by 16-byte
-//     cp.async, four lanes a segment -- through its own ring of stages, across tile boundaries.  (A bulk copy a segment
-//     took its lanes one after another through the copy unit, which cost more issue slots than the products: Q6_K
-//     17408 x 5120, 4 tokens 37 -> 33 us and 16 tokens 59 -> 42, Q8_0 151936 x 896 136 -> 75, Q4_K 9728 x 2560 13.3 -> 9.9;
-//     the alignment of a row's words is looked at once a block for the same reason.)
-//   * A tile's partial sums (a float per row, token and warp) meet in shared memory in a fixed order.
+//   * A persistent CTA stages the tokens' quantized activations in shared memory once (token stride padded by 16 bytes, so that the
+//     eight tokens of a B fragment sit on different banks), then walks tiles of 16 rows, of one matrix or of up to three that share
+//     the activations (Q, K and V; gate and up).  A tile's pieces -- 16 row segments of one or more blocks -- make up to eight partial
+//     sums (piece I goes to sum I % 8), dealt to the warps of a group so that they have as many pieces each: five warps for rows
+//     of ten Q4_K blocks, four for twenty of Q6_K; a CTA holds as many groups as its warps and shared memory allow.  Each warp
+//     streams its pieces by 16-byte cp.async, four lanes a segment, through its own ring of stages, across tile boundaries.
+//   * The partial sums (a float per row and token) meet in shared memory and are added in order: the bits do not depend on the groups.
+//
+// Bound by the chain from one launch to the next where the matrix is small (activations, one or two pieces a warp, the meeting), by
+// instruction issue where it is large: 48 % of cycles, then the shared-memory queue (Q6_K's blocks, every second of which starts in the
+// middle of a word).  us, weights cold and launches one behind the other, eight warps a tile and a launch a matrix / now: Q, K (Q4_K)
+// and V (Q6_K) of 4096 + 2 x 1024 x 2560, 16 tokens 20.6 / 7.3; gate and up of 2 x 9728 x 2560 (Q4_K), 16 tokens 25.4 / 14.0, 4 tokens - / 12.0;
+// of 2 x 17408 x 5120 (Q6_K), 4 tokens 66 / 42; 5120 x 5120 (Q6_K), 16 tokens 28.7 / 22.5; a head of 151936 x 2560 (Q6_K), 16 tokens
+// 142 / 117.  What gave it: one launch; activations that are all asked for before anything is waited for (4 us a launch); the deal;
+// Q4_K's mins against the sums of 16 by two products, its scales four at a time (half the instructions); ldmatrix.
 //
 // mma.sync is the legacy tensor path: right here, where N is 8 or 16 and the bound is HBM; the chunk-sized
 // products (hundreds of rows of X an expert) use tcgen05 (mm_id.cu).
@@ -29,48 +35,71 @@
 
 namespace ill {
 
-// A tile's columns are split over a group of eight warps; a CTA holds one or two groups (a tile each at a time)
-// that share the staged activations, and each warp a ring of two to four stages.
-constexpr int MT_WARPS = 8, MT_GROUP_THREADS = 32 * MT_WARPS, MT_ROWS = 16, MT_MAX_STAGES = 4, MT_MAX_GROUPS = 2;
+// A tile's pieces are dealt to eight partial sums (piece I to sum I % 8), and the sums to a group's warps; a CTA holds one to four
+// groups (a tile each at a time) that share the staged activations, and each warp a ring of two to four stages.
+constexpr int MT_SUMS = 8, MT_MAX_WARPS = 16, MT_ROWS = 16, MT_MAX_STAGES = 4, MT_MATS = 3;
 
-struct MtParams {
+struct MtMat {
   const u8* w;
-  int rows, cols, row_bytes, nblocks;  // blocks a row
+  float* y;
+  const float* bias;
+  int rows, tile_end;   // tiles of 16 rows of this matrix and those before it
+  int alt;              // in the kernel's second format
+};
+// a format's pieces
+struct MtFmt {
+  int row_bytes;
   int cb, npieces;      // blocks a staged piece (a warp's unit of copying); pieces a row
+  int pitch;            // bytes between the rows of a staged piece
+  u8 sums[MT_SUMS];     // the partial sums of a group's warp (bits)
+};
+struct MtParams {
+  MtMat m[MT_MATS];     // matrices that share the activations; the last ones may be empty
+  MtFmt f[2];           // the kernel's formats
+  int cols, nblocks;    // blocks a row
   const i8* xq;
   const float* xs;
   const int16_t* xsum;
-  float* y;
-  const float* bias;
   int acc, n;
-  int pitch;            // bytes between the rows of a staged piece
+  int nsums;            // partial sums a row, at most
   uint32_t stage_bytes;
-  int stages, groups;   // stages a warp's ring; groups of eight warps a CTA
+  int stages, groups;   // stages a warp's ring; groups of warps a CTA
+  int gw;               // warps a group
   int x_stride;         // bytes between the tokens' quants in shared memory
   uint32_t xs_off, bs_off, ring_off, part_off;
 };
-
 
 // The tokens' activations in shared memory.
 struct MtX {
   const i8* q;        // token t's quants at q + t * stride
   int stride;
   const float* s;     // [t][scales a token]
-  const int16_t* bs;  // [t][sums a token]: Q4_K sums of 32, Q6_K sums of 16
-  int nsc, nbs, n;
+  const u8* bs;       // K formats, [t][block][32]: the block's sixteen sums of 16 in two bytes each: sum >> 4 (signed), then sum & 15
+  int nsc, nb;
 };
-// the B fragment's word: token TOK's quants K .. K+3 (the tokens past the last are staged as zeros)
-__device__ __forceinline__ uint32_t xword(const MtX& x, int tok, int k) {
-  return *(const uint32_t*)(x.q + (size_t)tok * x.stride + k);
+// B fragments of 64 columns from K on against tokens 8 NT .. 8 NT + 7 (those past the last are staged as zeros): r[0], r[1] the first
+// 32 columns', r[2], r[3] the others'; of k16 products one each
+__device__ __forceinline__ void xfrag(uint32_t (&r)[4], const MtX& x, int nt, int k, int lane) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(x.q + (size_t)(8 * nt + (lane & 7)) * x.stride + k + 16 * (lane >> 3))));
+}
+// sums of 16 times sixteen bytes of the rows' (S0, S8: row g's and g + 8's bytes 4 t ..), each sum split in two int8 halves
+__device__ __forceinline__ void mul_sums(int (&c)[4], uint32_t s0, uint32_t s8, const MtX& x, int nt, int blk, int lane) {
+  const u8* b = x.bs + ((size_t)(8 * nt + (lane >> 2)) * x.nb + blk) * 32 + 4 * (lane & 3);
+  int hi[4] = {0, 0, 0, 0}, lo[4] = {0, 0, 0, 0};
+  mma_k16_s8(hi, s0, s8, *(const uint32_t*)b, false);
+  mma_k16_s8(lo, s0, s8, *(const uint32_t*)(b + 16), true);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) c[i] = 16 * hi[i] + lo[i];
 }
 
 // ---- one block of 16 rows against the tokens: ACC[nt][i] += ... --------------------------------------
 // ROW0 / ROW8: the block's bytes of rows g and g + 8 of the tile (g = lane / 4) in the staged piece; BLK the
 // block's number in the row; NT8 tiles of eight tokens.  Output i of a tile: row g + 8 (i / 2), token 8 nt + 2 (lane % 4) + i % 2.
-template <int FMT, int NT8> struct MtBlock;
+template <int FMT, int NT8, bool AL4> struct MtBlock;
 
-template <int NT8> struct MtBlock<ILL_Q8_0, NT8> {
-  static constexpr int BS_PER = 0;
+template <int NT8, bool AL4> struct MtBlock<ILL_Q8_0, NT8, AL4> {
   __device__ static void run(const u8* row0, const u8* row8, int blk, const MtX& x, int lane, float (&acc)[NT8][4]) {
     const int g = lane >> 2, t4 = 4 * (lane & 3);
     uint32_t a[4];
@@ -79,7 +108,8 @@ template <int NT8> struct MtBlock<ILL_Q8_0, NT8> {
     const float d0 = ldh(row0), d8 = ldh(row8);
 #pragma unroll
     for (int nt = 0; nt < NT8; ++nt) {
-      uint32_t b[2] = {xword(x, 8 * nt + g, 32 * blk + t4), xword(x, 8 * nt + g, 32 * blk + 16 + t4)};
+      const i8* xw = x.q + (size_t)(8 * nt + g) * x.stride + 32 * blk + t4;
+      const uint32_t b[2] = {*(const uint32_t*)xw, *(const uint32_t*)(xw + 16)};
       int c[4] = {0, 0, 0, 0};
       mma_k32(c, a, b, false);
 #pragma unroll
@@ -93,89 +123,118 @@ template <int NT8> struct MtBlock<ILL_Q8_0, NT8> {
   }
 };
 
-template <int NT8> struct MtBlock<ILL_Q4_K, NT8> {
-  static constexpr int BS_PER = 8;  // sums of 32 a block
+// words of a row: at multiples of four bytes from it where AL4, else at any two
+template <bool AL4> struct MtWords;
+template <> struct MtWords<false> : LdsWords {
+  __device__ __forceinline__ explicit MtWords(const u8* p) : LdsWords(p) {}
+};
+template <> struct MtWords<true> {
+  const u8* p;
+  __device__ __forceinline__ explicit MtWords(const u8* q) : p(q) {}
+  __device__ __forceinline__ uint32_t operator()(int off) const { return *(const uint32_t*)(p + off); }
+};
+
+template <int NT8, bool AL4> struct MtBlock<ILL_Q4_K, NT8, AL4> {
   __device__ static void run(const u8* row0, const u8* row8, int blk, const MtX& x, int lane, float (&acc)[NT8][4]) {
-    const int g = lane >> 2, t4 = 4 * (lane & 3);
-    int isum[NT8][4], imin[NT8][4];
+    const int t = lane & 3, t4 = 4 * t;
+    const MtWords<AL4> h0(row0), h8(row8), q0(row0 + t4), q8(row8 + t4);
+    // the 6-bit scales and mins of the eight groups, a byte each (get_scale_min_k4, src/kquant.lisp:64-72, four at a time)
+    uint32_t sc[2][2], mn[2][2];  // [row g / g + 8][groups 0-3 / 4-7]
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const uint32_t a = (r ? h8 : h0)(4), b = (r ? h8 : h0)(8), c = (r ? h8 : h0)(12);
+      sc[r][0] = a & 0x3f3f3f3fu;
+      sc[r][1] = (c & 0x0f0f0f0fu) | ((a >> 2) & 0x30303030u);
+      mn[r][0] = b & 0x3f3f3f3fu;
+      mn[r][1] = ((c >> 4) & 0x0f0f0f0fu) | ((b >> 2) & 0x30303030u);
+    }
+    int isum[NT8][4];
 #pragma unroll
     for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) isum[nt][i] = imin[nt][i] = 0;
-    const LdsWords q0(row0 + t4), q8(row8 + t4);
+      for (int i = 0; i < 4; ++i) isum[nt][i] = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {  // 64 weights: groups 2k (low nibbles) and 2k + 1 (high)
-      const uint32_t w0 = q0(16 + 32 * k), w1 = q8(16 + 32 * k);
-      const uint32_t w2 = q0(32 + 32 * k), w3 = q8(32 + 32 * k);
-      const uint32_t lo[4] = {w0 & 0x0F0F0F0Fu, w1 & 0x0F0F0F0Fu, w2 & 0x0F0F0F0Fu, w3 & 0x0F0F0F0Fu};
-      const uint32_t hi[4] = {(w0 >> 4) & 0x0F0F0F0Fu, (w1 >> 4) & 0x0F0F0F0Fu, (w2 >> 4) & 0x0F0F0F0Fu, (w3 >> 4) & 0x0F0F0F0Fu};
-      int sc0[2], mn0[2], sc8[2], mn8[2];
-      scale_min_k4(row0 + 4, 2 * k, sc0[0], mn0[0]); scale_min_k4(row0 + 4, 2 * k + 1, sc0[1], mn0[1]);
-      scale_min_k4(row8 + 4, 2 * k, sc8[0], mn8[0]); scale_min_k4(row8 + 4, 2 * k + 1, sc8[1], mn8[1]);
+      const uint32_t w[4] = {q0(16 + 32 * k), q8(16 + 32 * k), q0(32 + 32 * k), q8(32 + 32 * k)};
+      uint32_t lo[4], hi[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { lo[i] = w[i] & 0x0F0F0F0Fu; hi[i] = (w[i] >> 4) & 0x0F0F0F0Fu; }
+      int s[2][2];  // [row][group]
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) s[r][j] = (int)(sc[r][k >> 1] >> (16 * (k & 1) + 8 * j) & 0xffu);
 #pragma unroll
       for (int nt = 0; nt < NT8; ++nt) {
-        const int kb = 256 * blk + 64 * k + t4;
-        uint32_t b0[2] = {xword(x, 8 * nt + g, kb), xword(x, 8 * nt + g, kb + 16)};
-        uint32_t b1[2] = {xword(x, 8 * nt + g, kb + 32), xword(x, 8 * nt + g, kb + 48)};
+        uint32_t b[4];
+        xfrag(b, x, nt, 256 * blk + 64 * k, lane);
+        const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
         int c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
         mma_k32(c0, lo, b0, true);
         mma_k32(c1, hi, b1, true);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int tok = 8 * nt + 2 * (lane & 3) + (i & 1);
-          isum[nt][i] += c0[i] * (i < 2 ? sc0[0] : sc8[0]) + c1[i] * (i < 2 ? sc0[1] : sc8[1]);
-          const int bsp = *(const int*)(x.bs + tok * x.nbs + 8 * blk + 2 * k);  // the two groups' sums of 32
-          imin[nt][i] = dp2a_lo(bsp, (i < 2 ? mn0[0] : mn8[0]) | ((i < 2 ? mn0[1] : mn8[1]) << 8), imin[nt][i]);
-        }
+        for (int i = 0; i < 4; ++i) isum[nt][i] += c0[i] * s[i >> 1][0] + c1[i] * s[i >> 1][1];
       }
     }
-    const float d0 = ldh(row0), m0 = ldh(row0 + 2), d8 = ldh(row8), m8 = ldh(row8 + 2);
+    const uint32_t e0 = h0(0), e8 = h8(0);
+    const float d0 = h2f(e0 & 0xffffu), m0 = h2f(e0 >> 16), d8 = h2f(e8 & 0xffffu), m8 = h2f(e8 >> 16);
+    // the mins against the sums of 16: a group of 32 faces two of them, so bytes 4 t .. are mins 2 t, 2 t, 2 t + 1, 2 t + 1
+    const uint32_t sel = t & 1 ? 0x3322u : 0x1100u;
+    const uint32_t a0 = __byte_perm(t >> 1 ? mn[0][1] : mn[0][0], 0, sel), a8 = __byte_perm(t >> 1 ? mn[1][1] : mn[1][0], 0, sel);
 #pragma unroll
-    for (int nt = 0; nt < NT8; ++nt)
+    for (int nt = 0; nt < NT8; ++nt) {
+      int imin[4];
+      mul_sums(imin, a0, a8, x, nt, blk, lane);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int tok = 8 * nt + 2 * (lane & 3) + (i & 1);
+        const int tok = 8 * nt + 2 * t + (i & 1);
         const float yd = x.s[tok * x.nsc + blk];
         // Q4K-ROW-DOT: sum -= (yd * dmin) * imin; sum += (yd * d) * isum
-        float s = __fsub_rn(acc[nt][i], __fmul_rn(__fmul_rn(yd, i < 2 ? m0 : m8), (float)imin[nt][i]));
-        acc[nt][i] = __fadd_rn(s, __fmul_rn(__fmul_rn(yd, i < 2 ? d0 : d8), (float)isum[nt][i]));
+        const float v = __fsub_rn(acc[nt][i], __fmul_rn(__fmul_rn(yd, i < 2 ? m0 : m8), (float)imin[i]));
+        acc[nt][i] = __fadd_rn(v, __fmul_rn(__fmul_rn(yd, i < 2 ? d0 : d8), (float)isum[nt][i]));
       }
+    }
   }
 };
 
-template <int NT8> struct MtBlock<ILL_Q6_K, NT8> {
-  static constexpr int BS_PER = 16;  // a block's sixteen sums of 16, staged as two bytes each: (sum >> 4, sum & 15)
+template <int NT8, bool AL4> struct MtBlock<ILL_Q6_K, NT8, AL4> {
+  // every second block starts on a word, in all rows alike where they lie a multiple of four bytes apart
   __device__ static void run(const u8* row0, const u8* row8, int blk, const MtX& x, int lane, float (&acc)[NT8][4]) {
-    const int g = lane >> 2, t4 = 4 * (lane & 3);
+    if (__all_sync(0xffffffffu, (((uintptr_t)row0 | (uintptr_t)row8) & 3) == 0)) run_al<true>(row0, row8, blk, x, lane, acc);
+    else run_al<false>(row0, row8, blk, x, lane, acc);
+  }
+  template <bool W>
+  __device__ __forceinline__ static void run_al(const u8* row0, const u8* row8, int blk, const MtX& x, int lane, float (&acc)[NT8][4]) {
+    const int t4 = 4 * (lane & 3);
     int isum[NT8][4];
-    const signed char* sc0 = (const signed char*)(row0 + 192);
-    const signed char* sc8 = (const signed char*)(row8 + 192);
-    const LdsWords q0(row0 + t4), q8(row8 + t4);
+    const MtWords<W> q0(row0 + t4), q8(row8 + t4), h0(row0), h8(row8);
+    uint32_t sc[2][4];  // [row g / g + 8]: the sixteen scales
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { sc[0][j] = h0(192 + 4 * j); sc[1][j] = h8(192 + 4 * j); }
     {
       // The quants are 0..63: their -32 comes off as 32 * sum over the groups of scale * (the activations' sum of
-      // the group) -- itself a product of the block's 16 x 16 scales with the tokens' sums, taken on the tensor
-      // cores with each sum split in two int8 halves: sum = 16 * (sum >> 4) + (sum & 15).
+      // the group) -- itself a product of the block's 16 x 16 scales with the tokens' sums
       const uint32_t s0 = q0(192), s8 = q8(192);
-      const u8* hl = (const u8*)x.bs;
 #pragma unroll
       for (int nt = 0; nt < NT8; ++nt) {
-        const u8* b = hl + ((size_t)(8 * nt + g) * x.nbs + 16 * blk) * 2;
-        int hi[4] = {0, 0, 0, 0}, lo[4] = {0, 0, 0, 0};
-        mma_k16_s8(hi, s0, s8, *(const uint32_t*)(b + t4), false);
-        mma_k16_s8(lo, s0, s8, *(const uint32_t*)(b + 16 + t4), true);
+        mul_sums(isum[nt], s0, s8, x, nt, blk, lane);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) isum[nt][i] = -32 * (16 * hi[i] + lo[i]);
+        for (int i = 0; i < 4; ++i) isum[nt][i] *= -32;
       }
     }
 #pragma unroll
-    for (int c = 0; c < 2; ++c)      // half of the block: 128 weights
+    for (int c = 0; c < 2; ++c) {    // half of the block: 128 weights, two groups of 16 of each of the half's four runs of 32
+      uint32_t b[NT8][2][4];         // the tokens' quants of runs 0 and 1, 2 and 3: [run & 1][group]
 #pragma unroll
-      for (int is = 0; is < 2; ++is) {  // weights l = 16 is .. 16 is + 15 of each of the half's four runs of 32
-        const int l = 16 * is + t4;
+      for (int nt = 0; nt < NT8; ++nt)
+#pragma unroll
+        for (int r2 = 0; r2 < 2; ++r2) xfrag(b[nt][r2], x, nt, 256 * blk + 128 * c + 64 * r2, lane);
+#pragma unroll
+      for (int is = 0; is < 2; ++is) {
         uint32_t q[2][4];  // [row g / g + 8][run]: the lane's four 6-bit quants of each run
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const LdsWords& row = r ? q8 : q0;
+          const MtWords<W>& row = r ? q8 : q0;
           const uint32_t A = row(64 * c + 16 * is), B = row(64 * c + 32 + 16 * is), H = row(128 + 32 * c + 16 * is);
           q[r][0] = (A & 0x0F0F0F0Fu) | ((H << 4) & 0x30303030u);
           q[r][1] = (B & 0x0F0F0F0Fu) | ((H << 2) & 0x30303030u);
@@ -185,16 +244,17 @@ template <int NT8> struct MtBlock<ILL_Q6_K, NT8> {
 #pragma unroll
         for (int run = 0; run < 4; ++run) {
           const int grp = 8 * c + 2 * run + is;  // the group of 16 and its scale
-          const int s0 = sc0[grp], s8 = sc8[grp];
+          const int s0 = (int)(signed char)(sc[0][grp >> 2] >> (8 * (grp & 3))), s8 = (int)(signed char)(sc[1][grp >> 2] >> (8 * (grp & 3)));
 #pragma unroll
           for (int nt = 0; nt < NT8; ++nt) {
             int cc[4] = {0, 0, 0, 0};
-            mma_k16_u8(cc, q[0][run], q[1][run], xword(x, 8 * nt + g, 256 * blk + 128 * c + 32 * run + l));
+            mma_k16_u8(cc, q[0][run], q[1][run], b[nt][run >> 1][2 * (run & 1) + is]);
 #pragma unroll
             for (int i = 0; i < 4; ++i) isum[nt][i] += cc[i] * (i < 2 ? s0 : s8);
           }
         }
       }
+    }
     const float d0 = ldh(row0 + 208), d8 = ldh(row8 + 208);
 #pragma unroll
     for (int nt = 0; nt < NT8; ++nt)
@@ -208,44 +268,74 @@ template <int NT8> struct MtBlock<ILL_Q6_K, NT8> {
   }
 };
 
-// the meeting of one group's eight warps (barrier 1 + group)
-__device__ __forceinline__ void group_sync(int grp) {
-  asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(1 + grp), "n"(MT_GROUP_THREADS) : "memory");
+// 16 / 4 bytes global -> shared, asynchronously, or zeros
+__device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async4_or_zero(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+// the meeting of one group's warps (barrier 1 + group)
+__device__ __forceinline__ void group_sync(int grp, int threads) {
+  asm volatile("barrier.cta.sync %0, %1;" ::"r"(1 + grp), "r"(threads) : "memory");
 }
 
-template <int FMT, int NT8>
-__global__ void __launch_bounds__(MT_GROUP_THREADS * MT_MAX_GROUPS) mvt_kernel(const MtParams p) {
+template <int N> struct IntC { static constexpr int value = N; };
+
+// FMT2: the format of the matrices marked ALT (a file's V in Q6_K beside Q and K in Q4_K), or FMT
+template <int FMT, int FMT2, int NT8, bool AL4>
+__global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_constant__ MtParams p) {
   extern __shared__ __align__(128) u8 smem[];
-  constexpr int BB = Fmt<FMT>::BB, BW = Fmt<FMT>::BW;
+  constexpr int BW = Fmt<FMT>::BW, NTOK = 8 * NT8, PP = 20 /* floats a token's 16 rows of a partial sum are apart */;
+  constexpr bool TWO = FMT != FMT2;
   const int tid = threadIdx.x, lane = tid & 31, cwarp = tid >> 5;  // the warp's number in the CTA
-  const int warp = cwarp & (MT_WARPS - 1), grp = cwarp / MT_WARPS, gtid = tid & (MT_GROUP_THREADS - 1);
+  const int gw = p.gw, grp = cwarp / gw, wg = cwarp - gw * grp, gtid = tid - 32 * gw * grp;
   const int nthreads = blockDim.x, stages = p.stages;
-  const int tile0 = blockIdx.x * p.groups + grp, tile_step = gridDim.x * p.groups;
+  const int tile0 = grp * gridDim.x + blockIdx.x, tile_step = gridDim.x * p.groups;
   i8* xq_s = (i8*)smem;
   float* xs_s = (float*)(smem + p.xs_off);
-  int16_t* bs_s = (int16_t*)(smem + p.bs_off);
   u8* ring = smem + p.ring_off + (size_t)cwarp * stages * p.stage_bytes;
-  float* part = (float*)(smem + p.part_off) + (size_t)grp * 2 * MT_WARPS * 256;  // [group][2][warps][16 rows][16 tokens]
+  const int nb = p.nblocks;
+  float* part = (float*)(smem + p.part_off) + (size_t)grp * 2 * p.nsums * NTOK * PP;  // [group][2][sums][tokens][PP]
+  const int ntiles = p.m[MT_MATS - 1].tile_end;
 
-  const int ntiles = (p.rows + MT_ROWS - 1) / MT_ROWS;
-  const int nb = p.nblocks, cb = p.cb, np = p.npieces;
-  // this warp's pieces in order: its group's tiles tile0, + tile_step, ...; of each the pieces warp, warp + 8, ...
-  int i_tile = tile0, i_blk = warp, i_slot = 0;  // i_blk counts pieces
-  constexpr int MAXB = FMT == ILL_Q8_0 ? 8 : FMT == ILL_Q4_K ? 2 : 1;  // most blocks a piece
+  auto matrix = [&](int tile) { return (tile >= p.m[0].tile_end) + (tile >= p.m[1].tile_end); };
+  auto format = [&](int mi) { return TWO ? p.m[mi].alt : 0; };
+  // this warp's pieces in order: its group's tiles tile0, + tile_step, ...; of each, sum after sum, the pieces of its sums
+  int n_tile = tile0, n_pc = 0, n_mi = 0, i_slot = 0;
+  unsigned n_left = 0;
+  auto at_tile = [&]() {  // on to the first tile from n_tile on that this warp has a sum of
+    while (n_tile < ntiles) {
+      n_mi = matrix(n_tile);
+      n_left = p.f[format(n_mi)].sums[wg];
+      if (n_left) { n_pc = __ffs(n_left) - 1; return; }
+      n_tile += tile_step;
+    }
+  };
+  at_tile();
   const int g = lane >> 2, t = lane & 3;
   auto issue_next = [&]() {  // all lanes: four a row segment, eight rows at a time; a group of cp.async, possibly empty
-    while (i_tile < ntiles && i_blk >= np) { i_tile += tile_step; i_blk = warp; }
-    if (i_tile < ntiles) {
-      u8* st = ring + (size_t)i_slot * p.stage_bytes;
-      const uint32_t len = (uint32_t)min(cb, nb - i_blk * cb) * BB;
+    if (n_tile < ntiles) {
+      auto copy = [&](auto fmt_) {
+        constexpr int F = decltype(fmt_)::value, BB = Fmt<F>::BB, MAXB = F == ILL_Q8_0 ? 8 : F == ILL_Q4_K ? 2 : 1;  // most blocks a piece
+        const MtFmt& f = p.f[F != FMT];
+        const int row0 = (n_tile - (n_mi ? p.m[n_mi - 1].tile_end : 0)) * MT_ROWS;
+        u8* st = ring + (size_t)i_slot * p.stage_bytes;
+        const uint32_t len = (uint32_t)min(f.cb, nb - n_pc * f.cb) * BB;
+        const u8* src = p.m[n_mi].w + (long long)(row0 + g) * f.row_bytes + (long long)n_pc * f.cb * BB;
 #pragma unroll
-      for (int h = 0; h < MT_ROWS; h += 8) {
-        const int row = i_tile * MT_ROWS + h + g;
-        if (row < p.rows)
-          copy_segment<(MAXB * BB + 30) / 16>(st + (size_t)(h + g) * p.pitch, p.w + (long long)row * p.row_bytes + (long long)i_blk * cb * BB, len, t);
-      }
+        for (int h = 0; h < MT_ROWS; h += 8)
+          if (row0 + h + g < p.m[n_mi].rows)
+            copy_segment<(MAXB * BB + 30) / 16>(st + (size_t)(h + g) * f.pitch, src + (long long)h * f.row_bytes, len, t);
+        n_pc += MT_SUMS;
+        if (n_pc >= f.npieces) {
+          n_left &= n_left - 1;
+          if (n_left) n_pc = __ffs(n_left) - 1;
+          else { n_tile += tile_step; at_tile(); }
+        }
+      };
+      if (TWO && p.m[n_mi].alt) copy(IntC<FMT2>()); else copy(IntC<FMT>());
       i_slot = i_slot + 1 == stages ? 0 : i_slot + 1;
-      i_blk += MT_WARPS;
     }
     cp_async_commit();
   };
@@ -253,128 +343,178 @@ __global__ void __launch_bounds__(MT_GROUP_THREADS * MT_MAX_GROUPS) mvt_kernel(c
   pdl_launch_dependents();
   pdl_wait();
 
-  // the tokens' activations -> shared memory, the tokens past the last (up to a whole tile of eight) as zeros
-  const int nsc = p.cols / BW, nbs = MtBlock<FMT, NT8>::BS_PER * (p.cols / 256);
-  constexpr int NTOK = 8 * NT8;
-  for (int i = tid; i < NTOK * (p.cols / 16); i += nthreads) {
-    const int t = i / (p.cols / 16), j = i - t * (p.cols / 16);
-    *(uint4*)(xq_s + (size_t)t * p.x_stride + 16 * j) = t < p.n ? ((const uint4*)(p.xq + (size_t)t * p.cols))[j] : make_uint4(0, 0, 0, 0);
-  }
-  for (int i = tid; i < NTOK * nsc; i += nthreads) xs_s[i] = i < p.n * nsc ? p.xs[i] : 0.0f;
-  if constexpr (FMT == ILL_Q4_K) {
-    for (int i = tid; i < NTOK * nbs; i += nthreads) {  // sums of 32: pairs of the sums of 16
-      const int t = i / nbs, j = i - t * nbs;
-      const int16_t* b = p.xsum + (size_t)t * (p.cols / 16) + 2 * j;
-      bs_s[i] = t < p.n ? (int16_t)(b[0] + b[1]) : (int16_t)0;
+  // The tokens' activations -> shared memory, the tokens past the last (up to a whole tile of eight) as zeros: all asked for before
+  // anything is waited for.  (A load, a store and the next load a thread took 12 latencies of L2 one after another: four of the 15 us
+  // of gate and up, 2 x 9728 x 2560, of 16 tokens.)
+  const int nsc = p.cols / BW, per_tok = p.cols / 16;
+  uint4 sum8[2];            // K formats: eight sums of 16 a load; two loads a thread hold 16 tokens of 8192 columns
+  const int nsum8 = FMT == ILL_Q8_0 ? 0 : NTOK * per_tok / 8;
+  auto load_sums = [&](int i) { return i < nsum8 && 8 * i < p.n * per_tok ? ((const uint4*)p.xsum)[i] : make_uint4(0, 0, 0, 0); };
+#pragma unroll
+  for (int k = 0; k < 2; ++k) sum8[k] = load_sums(tid + k * nthreads);
+  for (int tk = cwarp; tk < NTOK; tk += nthreads / 32)  // a warp a token
+    for (int j = lane; j < per_tok; j += 32) {
+      const bool in = tk < p.n;
+      cp_async16_or_zero(xq_s + (size_t)tk * p.x_stride + 16 * j, in ? p.xq + (size_t)tk * p.cols + 16 * j : p.xq, in);
     }
-  } else if constexpr (FMT == ILL_Q6_K) {
+  for (int i = tid; i < NTOK * nsc; i += nthreads) {
+    const bool in = i < p.n * nsc;
+    cp_async4_or_zero(xs_s + i, in ? p.xs + i : p.xs, in);
+  }
+  cp_async_commit();
+  if constexpr (FMT != ILL_Q8_0) {
     // per block 32 bytes: the sixteen sums' high parts (sum >> 4, signed), then their low parts (sum & 15)
-    u8* hl = (u8*)bs_s;
-    for (int i = tid; i < NTOK * nbs; i += nthreads) {
-      const int t = i / nbs, j = i - t * nbs, b = j >> 4, gq = j & 15;
-      const int v = t < p.n ? (int)p.xsum[(size_t)t * (p.cols / 16) + j] : 0;
-      hl[((size_t)t * nbs + 16 * b) * 2 + gq] = (u8)(signed char)(v >> 4);
-      hl[((size_t)t * nbs + 16 * b) * 2 + 16 + gq] = (u8)(v & 15);
-    }
+    auto store_sums = [&](int i, const uint4& v) {
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};  // two sums each
+      uint32_t hi[2], lo[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        // bits 4..11 of the four 16-bit sums, a byte each; bits 0..3
+        hi[k] = __byte_perm(w[2 * k] >> 4, w[2 * k + 1] >> 4, 0x6420);
+        lo[k] = __byte_perm(w[2 * k], w[2 * k + 1], 0x6420) & 0x0f0f0f0fu;
+      }
+      u8* b = smem + p.bs_off + (i >> 1) * 32 + 8 * (i & 1);
+      *(uint2*)b = make_uint2(hi[0], hi[1]);
+      *(uint2*)(b + 16) = make_uint2(lo[0], lo[1]);
+    };
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if (tid + k * nthreads < nsum8) store_sums(tid + k * nthreads, sum8[k]);
+    for (int i = tid + 2 * nthreads; i < nsum8; i += nthreads) store_sums(i, load_sums(i));
   }
+  cp_async_wait_all();
   __syncthreads();
   MtX x;
-  x.q = xq_s; x.stride = p.x_stride; x.s = xs_s; x.bs = bs_s; x.nsc = nsc; x.nbs = nbs; x.n = p.n;
+  x.q = xq_s; x.stride = p.x_stride; x.s = xs_s; x.bs = smem + p.bs_off; x.nsc = nsc; x.nb = nb;
 
   int slot = 0, it = 0;
   for (int tile = tile0; tile < ntiles; tile += tile_step, ++it) {
-    float acc[NT8][4];
+    const int mi = matrix(tile), row0 = (tile - (mi ? p.m[mi - 1].tile_end : 0)) * MT_ROWS;
+    float* sums = part + (size_t)(it & 1) * p.nsums * NTOK * PP;
+    const u8* w = p.m[mi].w;
+    const MtFmt& f = p.f[format(mi)];
+    for (unsigned left = f.sums[wg]; left; left &= left - 1) {
+      const int sum = __ffs(left) - 1;
+      float acc[NT8][4];
 #pragma unroll
-    for (int nt = 0; nt < NT8; ++nt)
+      for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[nt][i] = 0.0f;
-    for (int pc = warp; pc < np; pc += MT_WARPS) {
-      // all but the newer stages' groups: this piece is in
-      if (stages == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
-      else if (stages == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
-      else asm volatile("cp.async.wait_group 1;" ::: "memory");
-      __syncwarp();
-      const u8* piece = ring + (size_t)slot * p.stage_bytes;
-      slot = slot + 1 == stages ? 0 : slot + 1;
-      // a row's segment starts where its block starts inside the 16-byte aligned span that was copied
-      const long long o0 = (long long)(tile * MT_ROWS + g) * p.row_bytes + (long long)pc * cb * BB;
-      const long long o8 = o0 + 8ll * p.row_bytes;
-      const u8* row0 = piece + (size_t)g * p.pitch + (((uintptr_t)p.w + o0) & 15);
-      const u8* row8 = piece + (size_t)(g + 8) * p.pitch + (((uintptr_t)p.w + o8) & 15);
-      const int nhere = min(cb, nb - pc * cb);
-      for (int j = 0; j < nhere; ++j) MtBlock<FMT, NT8>::run(row0 + j * BB, row8 + j * BB, pc * cb + j, x, lane, acc);
-      __syncwarp();
-      issue_next();
+        for (int i = 0; i < 4; ++i) acc[nt][i] = 0.0f;
+      for (int pc = sum; pc < f.npieces; pc += MT_SUMS) {
+        // all but the newer stages' groups: this piece is in
+        if (stages == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
+        else if (stages == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const u8* piece = ring + (size_t)slot * p.stage_bytes;
+        slot = slot + 1 == stages ? 0 : slot + 1;
+        auto use = [&](auto fmt_) {
+          constexpr int F = decltype(fmt_)::value, BB = Fmt<F>::BB;
+          // a row's segment starts where its block starts inside the 16-byte aligned span that was copied
+          const long long o0 = (long long)(row0 + g) * f.row_bytes + (long long)pc * f.cb * BB;
+          const long long o8 = o0 + 8ll * f.row_bytes;
+          const u8* s0 = piece + (size_t)g * f.pitch + (((uintptr_t)w + o0) & 15);
+          const u8* s8 = piece + (size_t)(g + 8) * f.pitch + (((uintptr_t)w + o8) & 15);
+          const int nhere = min(f.cb, nb - pc * f.cb);
+          for (int j = 0; j < nhere; ++j) MtBlock<F, NT8, AL4>::run(s0 + j * BB, s8 + j * BB, pc * f.cb + j, x, lane, acc);
+        };
+        if (TWO && p.m[mi].alt) use(IntC<FMT2>()); else use(IntC<FMT>());
+        __syncwarp();
+        issue_next();
+      }
+#pragma unroll
+      for (int nt = 0; nt < NT8; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sums[(sum * NTOK + 8 * nt + 2 * t + (i & 1)) * PP + g + 8 * (i >> 1)] = acc[nt][i];
     }
-    // the eight warps' partial sums meet: thread (row, token) adds them in warp order
-    float* mine = part + (size_t)(it & 1) * MT_WARPS * 256 + warp * 256;
-#pragma unroll
-    for (int nt = 0; nt < NT8; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) mine[(g + 8 * (i >> 1)) * 16 + 8 * nt + 2 * (lane & 3) + (i & 1)] = acc[nt][i];
-    group_sync(grp);
-    {
-      const int r = gtid >> 4, tk = gtid & 15;
-      const long long row = (long long)tile * MT_ROWS + r;
-      if (tk < p.n && row < p.rows) {
-        const float* all = part + (size_t)(it & 1) * MT_WARPS * 256 + r * 16 + tk;
+    // the partial sums meet: thread (token, row) adds them in order
+    group_sync(grp, 32 * gw);
+    const int nsums = min(MT_SUMS, f.npieces);
+    for (int o = gtid; o < MT_ROWS * p.n; o += 32 * gw) {
+      const int r = o & 15, tk = o >> 4, row = row0 + r;
+      if (row < p.m[mi].rows) {
         float v = 0.0f;
 #pragma unroll
-        for (int w = 0; w < MT_WARPS; ++w) v = __fadd_rn(v, all[w * 256]);
-        if (p.bias) v += p.bias[row];
-        float* yp = p.y + (long long)tk * p.rows + row;
+        for (int k = 0; k < MT_SUMS; ++k)
+          if (k < nsums) v = __fadd_rn(v, sums[(k * NTOK + tk) * PP + r]);
+        if (p.m[mi].bias) v += p.m[mi].bias[row];
+        float* yp = p.m[mi].y + (long long)tk * p.m[mi].rows + row;
         *yp = p.acc ? *yp + v : v;
       }
     }
   }
 }
 
-template <int FMT>
+template <int FMT, int FMT2, bool AL4>
 static int mvt_launch(const MtParams& p, size_t smem, int grid, cudaStream_t st) {
-  const void* k = p.n <= 8 ? (const void*)mvt_kernel<FMT, 1> : (const void*)mvt_kernel<FMT, 2>;
+  const void* k = p.n <= 8 ? (const void*)mvt_kernel<FMT, FMT2, 1, AL4> : (const void*)mvt_kernel<FMT, FMT2, 2, AL4>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e);
   }
   MtParams pp = p;
   void* args[] = {&pp};
-  return launch_kernel(k, dim3(grid), dim3(MT_GROUP_THREADS * p.groups), smem, args, st);
+  return launch_kernel(k, dim3(grid), dim3(32 * p.gw * p.groups), smem, args, st);
 }
 
-// The several-token product on the tensor cores, for the formats it is written for; ILL_ERR_UNSUPPORTED
-// otherwise (the caller then takes the CUDA-core kernel).
-int mvt_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum, uint64_t y, uint64_t bias, int acc,
-            int n, void* stream) {
-  if (fmt != ILL_Q8_0 && fmt != ILL_Q4_K && fmt != ILL_Q6_K) return ILL_ERR_UNSUPPORTED;
-  if (n < 2 || n > 16) return ILL_ERR_UNSUPPORTED;
-  const int bw = fmt_block_weights(fmt), bb = fmt_block_bytes(fmt);
+// Deals the eight sums of NP pieces to GW warps, the longest first to the warp with the fewest pieces; returns the most a warp gets.
+static int mt_deal(int np, int gw, u8* sums) {
+  int load[MT_SUMS] = {}, most = 0;
+  for (int i = 0; i < MT_SUMS; ++i) sums[i] = 0;
+  for (int k = 0; k < MT_SUMS && k < np; ++k) {  // (earlier sums have as many pieces or one more)
+    int w = 0;
+    for (int i = 1; i < gw; ++i)
+      if (load[i] < load[w]) w = i;
+    load[w] += (np - k + MT_SUMS - 1) / MT_SUMS;
+    sums[w] |= (u8)(1u << k);
+    if (load[w] > most) most = load[w];
+  }
+  return most;
+}
+
+#ifdef ILL_TUNING
+static int g_gw = 0, g_groups = 0, g_stages = 0;
+extern "C" __attribute__((visibility("default"))) void ill_set_mt(int gw, int groups, int stages) { g_gw = gw; g_groups = groups; g_stages = stages; }
+#else
+constexpr int g_gw = 0, g_groups = 0, g_stages = 0;
+#endif
+
+// The several-token product on the tensor cores, of NMAT matrices that share the activations -- of one format, or (FMTS) of Q4_K and
+// Q6_K --, for the formats it is written for; ILL_ERR_UNSUPPORTED otherwise (the caller then takes the CUDA-core kernel).
+int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum,
+            const uint64_t* y, const uint64_t* bias, int acc, int n, void* stream) {
+  if (n < 2 || n > 16 || nmat < 1 || nmat > MT_MATS) return ILL_ERR_UNSUPPORTED;
   MtParams p = {};
-  p.w = (const u8*)(uintptr_t)w;
-  p.rows = rows;
+  long long ntiles = 0, tiles[2] = {};
+  bool al4 = true, two = false;
+  for (int i = 0; i < nmat; ++i) two = two || fmts[i] != fmts[0];
+  const int fmt = two ? ILL_Q4_K : fmts[0];
+  if (fmt != ILL_Q8_0 && fmt != ILL_Q4_K && fmt != ILL_Q6_K) return ILL_ERR_UNSUPPORTED;
+  for (int i = 0; i < MT_MATS; ++i) {
+    if (i < nmat) {
+      if (two && fmts[i] != ILL_Q4_K && fmts[i] != ILL_Q6_K) return ILL_ERR_UNSUPPORTED;
+      p.m[i].w = (const u8*)(uintptr_t)w[i];
+      p.m[i].y = (float*)(uintptr_t)y[i];
+      p.m[i].bias = bias ? (const float*)(uintptr_t)bias[i] : nullptr;
+      p.m[i].rows = rows[i];
+      p.m[i].alt = fmts[i] != fmt;
+      const int t = (rows[i] + MT_ROWS - 1) / MT_ROWS;
+      ntiles += t;
+      tiles[p.m[i].alt] += t;
+      if (fmts[i] == ILL_Q4_K) al4 = al4 && (w[i] & 3) == 0;
+    }
+    if (ntiles > 0x3fffffff) return ILL_ERR_TOO_LARGE;
+    p.m[i].tile_end = (int)ntiles;
+  }
+  const int bw = fmt_block_weights(fmt), nsc = cols / bw;
   p.cols = cols;
-  p.nblocks = cols / bw;
-  p.row_bytes = p.nblocks * bb;
+  p.nblocks = nsc;
   p.xq = (const i8*)(uintptr_t)xq;
   p.xs = (const float*)(uintptr_t)xs;
   p.xsum = (const int16_t*)(uintptr_t)xsum;
-  p.y = (float*)(uintptr_t)y;
-  p.bias = (const float*)(uintptr_t)bias;
   p.acc = acc;
   p.n = n;
-  // a row's segment: its block's 16-byte aligned span, rows a multiple of 16 bytes apart that is an odd multiple
-  // of 16 mod 128 (eight rows x four words then sit on 32 different banks)
-  // blocks a piece: about 200-300 bytes a row segment (four lanes' copies), but every warp should get a piece
-  int cb = fmt == ILL_Q8_0 ? 8 : fmt == ILL_Q4_K ? 2 : 1;
-  while (cb > 1 && (p.nblocks + cb - 1) / cb < MT_WARPS) cb >>= 1;
-  p.cb = cb;
-  p.npieces = (p.nblocks + cb - 1) / cb;
-  int pitch = (cb * bb + 15 + 15) / 16 * 16;
-  while ((pitch / 16) % 8 % 2 == 0) pitch += 16;
-  p.pitch = pitch;
-  p.stage_bytes = (uint32_t)(MT_ROWS * pitch + 16);
-  p.stage_bytes = (p.stage_bytes + 127) / 128 * 128;
   p.x_stride = cols + 16;
-  const int nsc = cols / bw, bs_per = fmt == ILL_Q4_K ? 8 : fmt == ILL_Q6_K ? 16 : 0;
   const uint32_t ntok = n <= 8 ? 8 : 16;  // staged tokens: whole tiles of eight
   uint32_t off = ntok * (uint32_t)p.x_stride;
   off = (off + 15) / 16 * 16;
@@ -382,40 +522,76 @@ int mvt_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
   off += 4u * ntok * nsc;
   off = (off + 15) / 16 * 16;
   p.bs_off = off;
-  off += 2u * ntok * bs_per * (cols / 256);
+  for (int i = 0; i < (two ? 2 : 1); ++i) {
+    const int ft = i ? ILL_Q6_K : fmt, bb = fmt_block_bytes(ft);
+    MtFmt& f = p.f[i];
+    f.row_bytes = p.nblocks * bb;
+    // a row's segment: its block's 16-byte aligned span, rows a multiple of 16 bytes apart that is an odd multiple
+    // of 16 mod 128 (eight rows x four words then sit on 32 different banks)
+    // blocks a piece: about 200-300 bytes a row segment (four lanes' copies), but every sum should get a piece
+    int cb = ft == ILL_Q8_0 ? 8 : ft == ILL_Q4_K ? 2 : 1;
+    while (cb > 1 && (p.nblocks + cb - 1) / cb < MT_SUMS) cb >>= 1;
+    f.cb = cb;
+    f.npieces = (p.nblocks + cb - 1) / cb;
+    f.pitch = (cb * bb + 15 + 15) / 16 * 16;
+    while ((f.pitch / 16) % 8 % 2 == 0) f.pitch += 16;
+    const uint32_t stage = (uint32_t)(MT_ROWS * f.pitch + 16 + 127) / 128 * 128;
+    // Too many tokens of too many columns (no room for eight warps with two stages each): mmd.cu's form, which brings the
+    // activations step by step, is the faster one, and adds a row's blocks in another order
+    if (off + (ft == ILL_Q8_0 ? 0u : ft == ILL_Q4_K ? 16u : 32u) * ntok * (cols / 256) + 16384u + 2u * MT_SUMS * stage > 220u * 1024u)
+      return ILL_ERR_UNSUPPORTED;
+    if (stage > p.stage_bytes) p.stage_bytes = stage;
+    const int ns = f.npieces < MT_SUMS ? f.npieces : MT_SUMS;
+    if (ns > p.nsums) p.nsums = ns;
+  }
+  if (fmt != ILL_Q8_0) off += 32u * ntok * (cols / 256);
   off = (off + 127) / 128 * 128;
   p.ring_off = off;
-  // two groups with rings as deep as fit (four stages at most, two at least), else one group
-  const uint32_t budget = 220u * 1024u, part_bytes = 2u * MT_WARPS * 256 * 4, ring1 = (uint32_t)MT_WARPS * p.stage_bytes;
-  const int ntiles = (rows + MT_ROWS - 1) / MT_ROWS;
-  p.groups = 0;
-  for (int g = MT_MAX_GROUPS; g >= 1 && !p.groups; --g) {
-    if (off + g * (part_bytes + 2 * ring1) > budget) continue;
-    p.groups = g;
-    p.stages = (int)((budget - off - g * part_bytes) / (g * ring1));
-    if (p.stages > MT_MAX_STAGES) p.stages = MT_MAX_STAGES;
-  }
-  if (!p.groups) return ILL_ERR_UNSUPPORTED;  // too many tokens of too many columns: the caller splits them
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-  if (p.groups == 2 && ntiles < 2 * sms && p.stages < 3) {  // few tiles: a group a CTA spreads them over more SMs
-    p.groups = 1;
-    p.stages = (int)((budget - off - part_bytes) / ring1);
-    if (p.stages > MT_MAX_STAGES) p.stages = MT_MAX_STAGES;
+  // Warps a group and groups a CTA, for the least time: the tiles a group takes one after another, times the pieces of its busiest
+  // warp.  The rings are as deep as fits (four stages at most, two at least).
+  const uint32_t budget = 226u * 1024u, part_bytes = 2u * p.nsums * ntok * 20 * 4;
+  double best = 0;
+  for (int gw = p.nsums; gw >= 1; --gw) {
+    u8 sums[2][MT_SUMS];
+    int most[2] = {};
+    for (int i = 0; i < (two ? 2 : 1); ++i) most[i] = mt_deal(p.f[i].npieces, gw, sums[i]) * p.f[i].cb;
+    const uint32_t ring1 = (uint32_t)gw * p.stage_bytes;
+    for (int g = MT_MAX_WARPS / gw; g >= 1; --g) {
+      if (g > 1 && (g - 1) * sms >= ntiles) continue;      // (fewer groups have a tile each already)
+      if (off + g * (part_bytes + 2 * ring1) > budget) continue;
+      if (g_gw && (g_gw != gw || g_groups != g)) continue;
+      const long long rounds = (ntiles + (long long)g * sms - 1) / ((long long)g * sms);
+      const double a_tile = (double)(tiles[0] * most[0] + tiles[1] * most[1]) / ntiles, cost = rounds * a_tile * (24 + g * gw);
+      if (p.groups && cost >= best) continue;
+      best = cost;
+      p.groups = g;
+      p.gw = gw;
+      for (int i = 0; i < 2; ++i)
+        for (int k = 0; k < MT_SUMS; ++k) p.f[i].sums[k] = sums[i][k];
+      p.stages = (int)((budget - off - g * part_bytes) / (g * ring1));
+      if (p.stages > MT_MAX_STAGES) p.stages = MT_MAX_STAGES;
+      if (g_stages && p.stages > g_stages) p.stages = g_stages;
+    }
   }
-  off += (uint32_t)p.groups * p.stages * ring1;
+  if (!p.groups) return ILL_ERR_UNSUPPORTED;
+  off += (uint32_t)(p.groups * p.gw * p.stages) * p.stage_bytes;
   p.part_off = off;
   off += (uint32_t)p.groups * part_bytes;
   const size_t smem = off;
-  const int per_sm = (int)((227u * 1024u) / (smem + 1024u)) >= 2 ? 2 : 1;
-  int grid = sms * per_sm;
-  if (grid * p.groups > ntiles) grid = (ntiles + p.groups - 1) / p.groups;
+  // (two CTAs an SM where their registers fit too: up to 64 a thread, K formats up to 83 or 128)
+  const int threads = 32 * p.gw * p.groups, most2 = fmt == ILL_Q8_0 ? 512 : n <= 8 ? 384 : 256;
+  const int per_sm = (int)((227u * 1024u) / (smem + 1024u)) >= 2 && threads <= most2 ? 2 : 1;
+  long long grid = (long long)sms * per_sm;
+  if (grid > ntiles) grid = ntiles;
   cudaStream_t st = (cudaStream_t)stream;
+  if (two) return al4 ? mvt_launch<ILL_Q4_K, ILL_Q6_K, true>(p, smem, (int)grid, st) : mvt_launch<ILL_Q4_K, ILL_Q6_K, false>(p, smem, (int)grid, st);
   switch (fmt) {
-    case ILL_Q8_0: return mvt_launch<ILL_Q8_0>(p, smem, grid, st);
-    case ILL_Q4_K: return mvt_launch<ILL_Q4_K>(p, smem, grid, st);
-    default: return mvt_launch<ILL_Q6_K>(p, smem, grid, st);
+    case ILL_Q8_0: return mvt_launch<ILL_Q8_0, ILL_Q8_0, false>(p, smem, (int)grid, st);
+    case ILL_Q4_K: return al4 ? mvt_launch<ILL_Q4_K, ILL_Q4_K, true>(p, smem, (int)grid, st) : mvt_launch<ILL_Q4_K, ILL_Q4_K, false>(p, smem, (int)grid, st);
+    default: return mvt_launch<ILL_Q6_K, ILL_Q6_K, false>(p, smem, (int)grid, st);
   }
 }
 

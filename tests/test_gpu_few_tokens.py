@@ -1,0 +1,78 @@
+"""Products of two to sixteen tokens: two or three matrices in one launch (ill_mv_3n) give each matrix's own bits, whatever groups and
+sums the launch deals out; ragged rows, rows at every alignment, Q4_K beside Q6_K; and the product itself against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from illatio_b200 import _lib
+from illatio_b200 import blocks as B
+from illatio_b200 import cuda_dense as D
+
+from gpu_util import act_to_host, dev_act, rel_errors
+
+pytestmark = pytest.mark.gpu
+
+
+def _mat(fmt, rows, cols, seed, off):
+    w = B.synth_matrix(fmt, rows, cols, seed=seed)
+    buf = torch.zeros(w.size + 16, dtype=torch.uint8, device="cuda")
+    buf[off:off + w.size] = torch.as_tensor(np.ascontiguousarray(w)).cuda().reshape(-1)
+    return w, buf, buf.data_ptr() + off
+
+
+@pytest.mark.parametrize("fmts,rows,cols,n,off", [
+    ((B.Q8_0, B.Q8_0, B.Q8_0), (896, 128, 130), 896, 2, 2),
+    ((B.Q8_0, B.Q8_0), (17, 1), 32, 16, 0),            # one block a row: one partial sum
+    ((B.Q8_0, B.Q8_0), (300, 300), 4864, 9, 0),
+    ((B.Q4_K, B.Q4_K, B.Q4_K), (257, 16, 15), 256, 3, 0),
+    ((B.Q4_K, B.Q4_K), (2000, 2000), 2560, 16, 0),     # five partial sums
+    ((B.Q4_K, B.Q4_K), (40, 33), 1792, 7, 2),          # blocks that start in the middle of a word
+    ((B.Q6_K, B.Q6_K, B.Q6_K), (513, 100, 64), 5120, 4, 0),
+    ((B.Q6_K, B.Q6_K), (65, 65), 768, 16, 2),          # rows that start on words and between them in turn
+    ((B.Q4_K, B.Q4_K, B.Q6_K), (4096, 1024, 1024), 2560, 16, 0),
+    ((B.Q4_K, B.Q4_K, B.Q6_K), (33, 47, 5), 2048, 8, 2),
+    ((B.Q6_K, B.Q4_K), (31, 100), 512, 5, 0),
+    ((B.Q4_K, B.Q6_K, B.Q4_K), (3000, 2500, 20), 3072, 12, 0),
+])
+def test_matrices_in_one_launch_give_each_ones_bits(cuda_lib, fmts, rows, cols, n, off):
+    x = np.random.default_rng(rows[0] + cols).standard_normal(n * cols).astype(np.float32)
+    act = dev_act(fmts[0], x)
+    mats = [_mat(f, r, cols, 11 + i, off) for i, (f, r) in enumerate(zip(fmts, rows))]
+    bias = [torch.randn(r, device="cuda") if i != 1 else None for i, r in enumerate(rows)]
+    xsum = 0 if act.kind == "q8" else act.xsum.data_ptr()
+    want, got = [], []
+    for (w, keep, ptr), f, r, b in zip(mats, fmts, rows, bias):
+        y = torch.zeros(n * r, device="cuda")
+        _lib.call("ill_mv", f, ptr, r, cols, act.xq.data_ptr(), act.xs.data_ptr(), xsum, y.data_ptr(), b.data_ptr() if b is not None else 0, 0, n,
+                  _lib.stream())
+        want.append(y)
+        got.append(torch.full((n * r + 8,), 7.0, device="cuda"))
+    third = len(fmts) == 3
+    _lib.call("ill_mv_3n", fmts[0], fmts[1], fmts[2] if third else 0, mats[0][2], mats[1][2], mats[2][2] if third else 0, rows[0], rows[1],
+              rows[2] if third else 0, cols, act.xq.data_ptr(), act.xs.data_ptr(), xsum, got[0].data_ptr(), got[1].data_ptr(),
+              got[2].data_ptr() if third else 0, bias[0].data_ptr(), 0, bias[2].data_ptr() if third else 0, n, _lib.stream())
+    for g, w, r in zip(got, want, rows):
+        assert torch.equal(g[:n * r], w)
+        assert (g[n * r:] == 7.0).all()
+    assert D.device_status() == 0
+
+
+@pytest.mark.parametrize("fmt,rows,cols,n", [(B.Q8_0, 50, 1152, 16), (B.Q4_K, 40, 2560, 16), (B.Q4_K, 19, 1280, 3), (B.Q6_K, 40, 5120, 16),
+                                             (B.Q6_K, 23, 2304, 2)])
+def test_few_tokens_against_the_oracle(oracle, cuda_lib, fmt, rows, cols, n):
+    x = np.random.default_rng(cols).standard_normal(n * cols).astype(np.float32)
+    act = dev_act(fmt, x)
+    w, keep, ptr = _mat(fmt, rows, cols, 3, 0)
+    y = torch.zeros(n * rows, device="cuda")
+    _lib.call("ill_mv", fmt, ptr, rows, cols, act.xq.data_ptr(), act.xs.data_ptr(), 0 if act.kind == "q8" else act.xsum.data_ptr(),
+              y.data_ptr(), 0, 0, n, _lib.stream())
+    xq, xs, bs = act_to_host(act)
+    want = []
+    for t in range(n):
+        per = 32 if fmt == B.Q8_0 else 256
+        h = (xq[t * cols:(t + 1) * cols], xs[t * (cols // per):(t + 1) * (cols // per)])
+        h = h + ((bs[t * (cols // 16):(t + 1) * (cols // 16)],) if bs is not None else (None,))
+        want.append(oracle.matvec(fmt, w, rows, cols, h)[0])
+    # whole-number block sums: what differs is the order of at most 152 32-bit additions
+    err, _ = rel_errors(y.cpu().numpy().reshape(n, rows), np.stack(want))
+    assert err <= 1e-5
