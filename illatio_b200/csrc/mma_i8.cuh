@@ -48,6 +48,16 @@ struct LdsWords {
   }
   __device__ __forceinline__ uint32_t operator()(int off) const { return __funnelshift_r(b[off / 4], b[off / 4 + 1], sh); }
 };
+// Words of a row at multiples of four bytes from an address: one that lies on a word (AL4), or on any two bytes.
+template <bool AL4> struct RowWords;
+template <> struct RowWords<false> : LdsWords {
+  __device__ __forceinline__ explicit RowWords(const u8* p) : LdsWords(p) {}
+};
+template <> struct RowWords<true> {
+  const u8* p;
+  __device__ __forceinline__ explicit RowWords(const u8* q) : p(q) {}
+  __device__ __forceinline__ uint32_t operator()(int off) const { return *(const uint32_t*)(p + off); }
+};
 __device__ __forceinline__ float ldh(const u8* p) { return h2f(*(const u16*)p); }  // p is 2-byte aligned
 
 __device__ __forceinline__ void mma_k16_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0, bool b_unsigned) {

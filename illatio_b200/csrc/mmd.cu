@@ -176,15 +176,21 @@ template <> struct MdFrag<ILL_Q6_K> {
   uint32_t q[16][2];  // [group of 16][row g / g + 8]: the lane's four quants as signed bytes -32..31
   int sc0[16], sc8[16];
   float d0, d8;
+  // every second block starts on a word, in all rows alike where they lie a multiple of four bytes apart
   __device__ __forceinline__ void load(const u8* row0, const u8* row8, int lane, int) {
-    const LdsWords w0s(row0), w8s(row8), q0(row0 + 4 * (lane & 3)), q8(row8 + 4 * (lane & 3));
+    if (__all_sync(0xffffffffu, (((uintptr_t)row0 | (uintptr_t)row8) & 3) == 0)) load_al<true>(row0, row8, lane);
+    else load_al<false>(row0, row8, lane);
+  }
+  template <bool W>
+  __device__ __forceinline__ void load_al(const u8* row0, const u8* row8, int lane) {
+    const RowWords<W> w0s(row0), w8s(row8), q0(row0 + 4 * (lane & 3)), q8(row8 + 4 * (lane & 3));
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
       for (int is = 0; is < 2; ++is) {
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const LdsWords& row = r ? q8 : q0;
+          const RowWords<W>& row = r ? q8 : q0;
           const uint32_t A = row(64 * c + 16 * is), B = row(64 * c + 32 + 16 * is), H = row(128 + 32 * c + 16 * is);
           // run RUN of the half covers weights 128 c + 32 run ..: its group of 16 is 8 c + 2 run + is
           q[8 * c + 0 + is][r] = q6_signed((A & 0x0F0F0F0Fu) | ((H << 4) & 0x30303030u));
@@ -350,24 +356,42 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
 }
 
 // ---- up to sixteen tokens of rows too long for mvt.cu to keep the activations resident ------------------------
-// One 16-row tile a CTA, its column steps dealt to the eight warps (warp w takes steps w, w + 8, ...): each warp
-// streams its own steps' weights (its ring of three stages) AND its own steps' activations (two buffers of its own), all
+// A 16-row tile's column steps are dealt to eight warps (warp w takes steps w, w + 8, ...) in the four CTAs of a cluster, two each: each
+// warp streams its own steps' weights (its ring of three stages) AND its own steps' activations (two buffers of its own), all
 // by 16-byte cp.async of its lanes (Q6_K 5120 x 17408, 4 tokens: 40 us; 59 with a bulk copy a row segment), so the warps
-// never wait for one another until the end, where their partial sums meet in shared memory in warp order.  A matrix of few
-// rows and many columns (5120 x 17408) thus fills the machine with rows / 16 CTAs of eight busy warps, where the chunk
-// kernel above would run two warps a CTA through all 68 steps.
-template <int FMT, int NT8>
-__global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
-  extern __shared__ __align__(128) u8 smem[];
+// never wait for one another until the end, where their partial sums are read from the four CTAs' shared memory in warp order.  A matrix
+// of few rows and many columns (5120 x 17408) thus fills the machine where the chunk kernel above would run two warps a CTA
+// through all 68 steps.  With the eight warps in one CTA, which takes most of an SM's shared memory, 160 tiles were two rounds on 148
+// SMs and 320 three; CTAs of two warps spread over the SMs to a quarter of a tile.  us, one CTA a tile / a cluster, weights cold, launches
+// one behind the other: Q6_K 2560 x 9728, 16 tokens 19.8 / 15.1; 5120 x 17408, 4 tokens 40.6 / 34.7, 16 tokens 47.5 / 41.5; Q4_K
+// 5120 x 17408, 16 tokens 44.0 / 39.2.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+// the float that CTA RANK of the cluster has at P of its shared memory
+__device__ __forceinline__ float ld_cluster(const float* p, int rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+constexpr int MK_PP = 20;  // floats between the tokens of a partial sum: a fragment's stores lie on different banks
+
+template <int FMT, int NT8, int CTAS /* of a tile */>
+__device__ __forceinline__ void mmk_body(const MdParams& p, u8* smem) {
+  constexpr int WARPS = MD_WARPS / CTAS;
   constexpr int TN = 8 * NT8, SB = MdFrag<FMT>::SB, SP = MdFrag<FMT>::SPITCH;
   constexpr bool KQ = FMT != ILL_Q8_0;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int tid = threadIdx.x, lane = tid & 31, cwarp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int rank = blockIdx.x % CTAS, tile = blockIdx.x / CTAS, warp = rank * WARPS + cwarp;
   const int ntt = (p.n + TN - 1) / TN;
-  const int tok0 = (int)(blockIdx.x % ntt) * TN, row_base = (int)(blockIdx.x / ntt) * 16;
+  const int tok0 = (tile % ntt) * TN, row_base = (tile / ntt) * 16;
   const int nsteps = p.nsteps;
-  u8* xw = smem + (size_t)warp * 2 * p.xbuf_bytes;  // this warp's two activation buffers
-  u8* ring = smem + p.ring_off + (size_t)warp * MD_MAX_STAGES * p.stage_bytes;
-  float* part = (float*)(smem + p.part_off);        // [warp][16 rows][TN]
+  u8* xw = smem + (size_t)cwarp * 2 * p.xbuf_bytes;  // this warp's two activation buffers
+  u8* ring = smem + p.ring_off + (size_t)cwarp * MD_MAX_STAGES * p.stage_bytes;
+  float* part = (float*)(smem + p.part_off);        // [this CTA's warps][TN][MK_PP: 16 rows]
 
   auto fill_w = [&](int k) {  // this warp's K-th step's weights -> stage k % 3 (a group of cp.async, possibly empty)
     const int step = warp + MD_WARPS * k;
@@ -461,26 +485,37 @@ __global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
     __syncwarp();  // every lane is through with buffer k % 2 before the next iteration's copies into it are issued
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  // the warps' partial sums meet: thread (row, token) adds them in warp order
+  // the warps' partial sums meet: thread (row, token) adds them in warp order, a quarter of the tile's in each CTA
 #pragma unroll
   for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      part[(warp * 16 + g + 8 * (i >> 1)) * TN + 8 * nt + 2 * t + (i & 1)] = acc[nt][i];
-  __syncthreads();
-  for (int o = tid; o < 16 * TN; o += MD_THREADS) {
-    const int r = o / TN, tk = o - r * TN;
-    const long long row = row_base + r;
-    const int tok = tok0 + tk;
+    for (int i = 0; i < 4; ++i) part[(cwarp * TN + 8 * nt + 2 * t + (i & 1)) * MK_PP + g + 8 * (i >> 1)] = acc[nt][i];
+  if constexpr (CTAS > 1) cluster_sync(); else __syncthreads();
+#pragma unroll
+  for (int o = rank * (16 * TN / CTAS) + tid; o < (rank + 1) * (16 * TN / CTAS); o += 32 * WARPS) {
+    const long long row = row_base + (o & 15);
+    const int tok = tok0 + (o >> 4), at = (o >> 4) * MK_PP + (o & 15);
     if (row < p.rows && tok < p.n) {
       float v = 0.0f;
 #pragma unroll
-      for (int w = 0; w < MD_WARPS; ++w) v = __fadd_rn(v, part[(w * 16 + r) * TN + tk]);
+      for (int w = 0; w < MD_WARPS; ++w) v = __fadd_rn(v, CTAS > 1 ? ld_cluster(part + w % WARPS * TN * MK_PP + at, w / WARPS) : part[w * TN * MK_PP + at]);
       if (p.bias) v += p.bias[row];
       float* yp = p.y + (long long)tok * p.rows + row;
       *yp = p.acc ? *yp + v : v;
     }
   }
+  if constexpr (CTAS > 1) cluster_sync();  // nobody's partial sums go before everyone has read them
+}
+template <int FMT, int NT8>
+__global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
+  extern __shared__ __align__(128) u8 smem[];
+  mmk_body<FMT, NT8, 1>(p, smem);
+}
+constexpr int MK_CTAS = 4;
+template <int FMT, int NT8>
+__global__ void __cluster_dims__(MK_CTAS, 1, 1) __launch_bounds__(MD_THREADS / MK_CTAS) mmk_cluster_kernel(const MdParams p) {
+  extern __shared__ __align__(128) u8 smem[];
+  mmk_body<FMT, NT8, MK_CTAS>(p, smem);
 }
 
 template <int FMT>
@@ -557,13 +592,15 @@ int mmd_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
 }
 
 template <int FMT>
-static int mmk_launch(const MdParams& p, int tn, size_t smem, int grid, cudaStream_t st) {
-  const void* k = tn == 8 ? (const void*)mmk_kernel<FMT, 1> : (const void*)mmk_kernel<FMT, 2>;
+static int mmk_launch(const MdParams& p, int tn, int ctas, size_t smem, int grid, cudaStream_t st) {
+  const void* k = tn == 8 ? (const void*)mmk_cluster_kernel<FMT, 1> : (const void*)mmk_cluster_kernel<FMT, 2>;
+  if constexpr (FMT == ILL_Q4_K)
+    if (ctas == 1) k = (const void*)mmk_kernel<FMT, 1>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e);
   MdParams pp = p;
   void* args[] = {&pp};
-  return launch_kernel(k, dim3(grid), dim3(MD_THREADS), smem, args, st);
+  return launch_kernel(k, dim3(grid), dim3(32 * MD_WARPS / ctas), smem, args, st);
 }
 
 // Up to sixteen tokens with the columns dealt to a CTA's warps (mmk_kernel): for rows of many columns.
@@ -602,17 +639,18 @@ int mmk_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
   p.xsum_off = off;
   if (fmt == ILL_Q4_K) off += (uint32_t)tn * MdFrag<ILL_Q4_K>::SPITCH;
   p.xbuf_bytes = (off + 127) / 128 * 128;
-  p.ring_off = 2 * MD_WARPS * p.xbuf_bytes;
-  p.part_off = (uint32_t)((p.ring_off + (size_t)MD_WARPS * MD_MAX_STAGES * p.stage_bytes + 127) / 128 * 128);
-  const size_t smem = p.part_off + (size_t)MD_WARPS * 16 * tn * 4;
-  if (smem > 226 * 1024) return ILL_ERR_UNSUPPORTED;
-  const long long grid = (long long)((rows + 15) / 16) * ((n + tn - 1) / tn);
+  // One CTA a tile where two of them fit an SM (Q4_K, up to eight tokens: 5120 x 17408 28 us, a cluster of four 30)
+  const int ctas = fmt == ILL_Q4_K && tn == 8 ? 1 : MK_CTAS, warps = MD_WARPS / ctas;
+  p.ring_off = 2 * warps * p.xbuf_bytes;
+  p.part_off = (uint32_t)((p.ring_off + (size_t)warps * MD_MAX_STAGES * p.stage_bytes + 127) / 128 * 128);
+  const size_t smem = p.part_off + (size_t)warps * MK_PP * tn * 4;
+  const long long grid = ctas * (long long)((rows + 15) / 16) * ((n + tn - 1) / tn);
   if (grid > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
   switch (fmt) {
-    case ILL_Q8_0: return mmk_launch<ILL_Q8_0>(p, tn, smem, (int)grid, st);
-    case ILL_Q4_K: return mmk_launch<ILL_Q4_K>(p, tn, smem, (int)grid, st);
-    default: return mmk_launch<ILL_Q6_K>(p, tn, smem, (int)grid, st);
+    case ILL_Q8_0: return mmk_launch<ILL_Q8_0>(p, tn, ctas, smem, (int)grid, st);
+    case ILL_Q4_K: return mmk_launch<ILL_Q4_K>(p, tn, ctas, smem, (int)grid, st);
+    default: return mmk_launch<ILL_Q6_K>(p, tn, ctas, smem, (int)grid, st);
   }
 }
 

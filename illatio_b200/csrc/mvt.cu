@@ -123,21 +123,10 @@ template <int NT8, bool AL4> struct MtBlock<ILL_Q8_0, NT8, AL4> {
   }
 };
 
-// words of a row: at multiples of four bytes from it where AL4, else at any two
-template <bool AL4> struct MtWords;
-template <> struct MtWords<false> : LdsWords {
-  __device__ __forceinline__ explicit MtWords(const u8* p) : LdsWords(p) {}
-};
-template <> struct MtWords<true> {
-  const u8* p;
-  __device__ __forceinline__ explicit MtWords(const u8* q) : p(q) {}
-  __device__ __forceinline__ uint32_t operator()(int off) const { return *(const uint32_t*)(p + off); }
-};
-
 template <int NT8, bool AL4> struct MtBlock<ILL_Q4_K, NT8, AL4> {
   __device__ static void run(const u8* row0, const u8* row8, int blk, const MtX& x, int lane, float (&acc)[NT8][4]) {
     const int t = lane & 3, t4 = 4 * t;
-    const MtWords<AL4> h0(row0), h8(row8), q0(row0 + t4), q8(row8 + t4);
+    const RowWords<AL4> h0(row0), h8(row8), q0(row0 + t4), q8(row8 + t4);
     // the 6-bit scales and mins of the eight groups, a byte each (get_scale_min_k4, src/kquant.lisp:64-72, four at a time)
     uint32_t sc[2][2], mn[2][2];  // [row g / g + 8][groups 0-3 / 4-7]
 #pragma unroll
@@ -207,7 +196,7 @@ template <int NT8, bool AL4> struct MtBlock<ILL_Q6_K, NT8, AL4> {
   __device__ __forceinline__ static void run_al(const u8* row0, const u8* row8, int blk, const MtX& x, int lane, float (&acc)[NT8][4]) {
     const int t4 = 4 * (lane & 3);
     int isum[NT8][4];
-    const MtWords<W> q0(row0 + t4), q8(row8 + t4), h0(row0), h8(row8);
+    const RowWords<W> q0(row0 + t4), q8(row8 + t4), h0(row0), h8(row8);
     uint32_t sc[2][4];  // [row g / g + 8]: the sixteen scales
 #pragma unroll
     for (int j = 0; j < 4; ++j) { sc[0][j] = h0(192 + 4 * j); sc[1][j] = h8(192 + 4 * j); }
@@ -234,7 +223,7 @@ template <int NT8, bool AL4> struct MtBlock<ILL_Q6_K, NT8, AL4> {
         uint32_t q[2][4];  // [row g / g + 8][run]: the lane's four 6-bit quants of each run
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const MtWords<W>& row = r ? q8 : q0;
+          const RowWords<W>& row = r ? q8 : q0;
           const uint32_t A = row(64 * c + 16 * is), B = row(64 * c + 32 + 16 * is), H = row(128 + 32 * c + 16 * is);
           q[r][0] = (A & 0x0F0F0F0Fu) | ((H << 4) & 0x30303030u);
           q[r][1] = (B & 0x0F0F0F0Fu) | ((H << 2) & 0x30303030u);
