@@ -6,16 +6,18 @@
 // Design.  A CTA of eight warps takes 128 rows x TN tokens (TN = 32, 64 or 128); warp w owns rows 16 w .. 16 w + 15
 // against all TN tokens, so a block of weights is unpacked into tensor-core fragments once and used TN / 8 times
 // from registers.  The columns go by in steps of 256:
-//   * weights: every warp runs its own ring of stages, lanes 0..15 each copying one row's 256 columns of blocks
-//     (144 / 210 bytes, widened to 16-byte boundaries) with cp.async.bulk onto the stage's mbarrier; a stage
-//     is free again as soon as its block sits in registers, so the next copy is issued before the arithmetic;
-//   * activations: the step's TN x 256 quants and their scales are brought by all threads with cp.async into one
-//     of two buffers while the other is being used -- one __syncthreads a step; a token tile's quants reach the
-//     registers as B fragments through ldmatrix.
+//   * weights: every warp brings its own sixteen rows' blocks (144 / 210 bytes, widened to 16-byte boundaries) by cp.async, four
+//     lanes a row;
+//   * activations: the step's TN x 256 quants and their scales are brought by all threads with cp.async; a token tile's quants
+//     reach the registers as B fragments through ldmatrix.
+// Both go through a ring of two to four stages, one __syncthreads a step.  (With a bulk copy a row segment, sixteen a warp and step, the
+// copy unit took 2.7 us a step of eight warps whatever the tokens.  us, bulk copies / now: 1024 x 2560 of Q4_K, 17 tokens 26.8 / 18.8, 128
+// 33.6 / 19.7, 512 28.4 / 21.9, 2048 65.8 / 62.6; of Q6_K, 512 28.9 / 23.4; 1024 x 5120 of Q6_K, 512 56.3 / 45.1; 9728 x 2560 of Q4_K, 63
+// 56.1 / 45.3.)  Bound now by the chain of one warp's step where few rows and tokens leave a warp or two an SM (1.8 us a step: a
+// block's fragments, then its products), by instruction issue where they do not.
 // This is mmd_kernel, for Q4_K and Q6_K; Q8_0 has a kernel of its own (mm_q8.cu).
 // Token tiles are the fastest-varying CTA index: the CTAs that share a tile of rows run together and the weights
-// come from HBM once.  Waits are bounded (status word, ST_MV_WAIT + 0x40 + format); a warp that gave up keeps
-// meeting the CTA's barriers and lets its copies land before the CTA leaves.
+// come from HBM once.
 //
 // Replaces mm_q8_mma2 / mm_q4k_mma / mm_q6k_mma behind CMAT-MUL-N for prefill chunks
 // (src/cuda-dense.lisp:220-255; src/cuda/dense.cu:885-1100, src/cuda/kquant.cu:316-466).
@@ -25,7 +27,7 @@
 
 namespace ill {
 
-constexpr int MD_WARPS = 8, MD_THREADS = 32 * MD_WARPS, MD_MAX_STAGES = 3;
+constexpr int MD_WARPS = 8, MD_THREADS = 32 * MD_WARPS, MD_MAX_STAGES = 3 /* of mmk_kernel */;
 constexpr int MD_XPITCH = 272;  // bytes between the tokens' 256 quants of a step: 68 words, so eight tokens x four words hit 32 banks
 
 struct MdParams {
@@ -38,12 +40,11 @@ struct MdParams {
   const float* bias;
   int acc, n;
   int warps;             // warps a CTA (16 rows each)
-  int stages;            // stages of a warp's ring of weights (2 or 3)
+  int stages;            // mmd_kernel: stages of weights and activations (2 to 4)
   int pitch;             // bytes between the rows of a staged piece
   uint32_t stage_bytes;
   uint32_t xbuf_bytes, xs_off, xsum_off;  // one activation buffer: its size, where its scales and (Q4_K) sums start
   uint32_t ring_off, part_off;
-  unsigned* status;
 };
 
 // four 8 x 16-byte matrices of shared memory -> each lane its four bytes of row lane / 4 of each: lane l gives the
@@ -231,88 +232,80 @@ template <int FMT, int NT8, int MINB>
 __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p) {
   extern __shared__ __align__(128) u8 smem[];
   constexpr int TN = 8 * NT8, SB = MdFrag<FMT>::SB, MD_SPITCH = MdFrag<FMT>::SPITCH;
-  const int MD_STAGES = p.stages;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int ntt = (p.n + TN - 1) / TN, nthreads = blockDim.x;  // eight warps, or fewer when the matrix has few rows
   const int tok0 = (int)(blockIdx.x % ntt) * TN, row_base = (int)(blockIdx.x / ntt) * (nthreads / 2) + warp * 16;
-  const int nsteps = p.nsteps;
+  const int nsteps = p.nsteps, stages = p.stages;
   const bool live = row_base < p.rows;  // a warp whose rows are all past the end only helps to bring the activations
-  u8* ring = smem + p.ring_off + (size_t)warp * MD_STAGES * p.stage_bytes;
-  __shared__ uint64_t full_s[MD_WARPS * MD_MAX_STAGES];
-  uint64_t* full = full_s + warp * MD_MAX_STAGES;
+  u8* ring = smem + p.ring_off + (size_t)warp * stages * p.stage_bytes;
 
-  int issued = 0;
-  auto issue_w = [&]() {  // all lanes of the warp; lanes 0..15 copy a row's step each
-    if (!live || issued >= nsteps) return;
-    const int s = issued % MD_STAGES;
-    const int row = row_base + lane;
-    uint32_t bytes = 0;
-    const u8* src = nullptr;
-    if (lane < 16 && row < p.rows) {
-      src = p.w + (long long)row * p.row_bytes + (long long)issued * SB;
-      const uint32_t len = (uint32_t)min(SB, p.row_bytes - issued * SB);
-      bytes = (uint32_t)((((uintptr_t)src + len + 15) & ~(uintptr_t)15) - ((uintptr_t)src & ~(uintptr_t)15));
-    }
-    uint32_t total = bytes;
+  int w_step = 0, w_at = 0, x_step = 0, x_at = 0;  // the steps brought next, their stages
+  auto fill_w = [&]() {  // the warp's sixteen rows, four lanes a row segment
+    if (live && w_step < nsteps) {
+      u8* st = ring + (size_t)w_at * p.stage_bytes;
+      const u8* src = p.w + (long long)(row_base + g) * p.row_bytes + (long long)w_step * SB;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-    if (lane == 0) mbar_expect_tx(&full[s], total);
-    __syncwarp();
-    if (bytes) bulk_g2s(ring + (size_t)s * p.stage_bytes + (size_t)lane * p.pitch, (const void*)((uintptr_t)src & ~(uintptr_t)15), bytes, &full[s]);
-    ++issued;
-  };
-  auto fill_x = [&](int step) {  // all threads: the step's activations -> buffer step % 2
-    u8* xb = smem + (size_t)(step & 1) * p.xbuf_bytes;
-    const int c0 = 256 * step;
-    for (int i = tid; i < TN * 16; i += nthreads) {
-      const int tk = i >> 4, ch = i & 15;
-      if (tok0 + tk < p.n && c0 + 16 * ch < p.cols)
-        cp_async16(xb + tk * MD_XPITCH + 16 * ch, p.xq + (long long)(tok0 + tk) * p.cols + c0 + 16 * ch);
+      for (int h = 0; h < 16; h += 8)
+        if (row_base + h + g < p.rows)
+          copy_segment<(SB + 30) / 16>(st + (size_t)(h + g) * p.pitch, src + (long long)h * p.row_bytes, SB, t);
     }
-    for (int i = tid; i < TN; i += nthreads)
-      if (tok0 + i < p.n) cp_async4(xb + p.xs_off + 4 * i, p.xs + (long long)(tok0 + i) * nsteps + step);
-    if constexpr (FMT == ILL_Q4_K) {
-      for (int i = tid; i < TN * 2; i += nthreads) {
-        const int tk = i >> 1, ch = i & 1;
-        if (tok0 + tk < p.n)
-          cp_async16(xb + p.xsum_off + tk * MD_SPITCH + 16 * ch, p.xsum + (long long)(tok0 + tk) * (p.cols / 16) + 16 * step + 8 * ch);
+    ++w_step;
+    w_at = w_at + 1 == stages ? 0 : w_at + 1;
+  };
+  auto fill_x = [&]() {  // all threads
+    if (x_step < nsteps) {
+      u8* xb = smem + (size_t)x_at * p.xbuf_bytes;
+      const int c0 = 256 * x_step;
+      for (int i = tid; i < TN * 16; i += nthreads) {
+        const int tk = i >> 4, ch = i & 15;
+        if (tok0 + tk < p.n) cp_async16(xb + tk * MD_XPITCH + 16 * ch, p.xq + (long long)(tok0 + tk) * p.cols + c0 + 16 * ch);
+      }
+      for (int i = tid; i < TN; i += nthreads)
+        if (tok0 + i < p.n) cp_async4(xb + p.xs_off + 4 * i, p.xs + (long long)(tok0 + i) * nsteps + x_step);
+      if constexpr (FMT == ILL_Q4_K) {
+        for (int i = tid; i < TN * 2; i += nthreads) {
+          const int tk = i >> 1, ch = i & 1;
+          if (tok0 + tk < p.n)
+            cp_async16(xb + p.xsum_off + tk * MD_SPITCH + 16 * ch, p.xsum + (long long)(tok0 + tk) * (p.cols / 16) + 16 * x_step + 8 * ch);
+        }
       }
     }
-    cp_async_commit();
+    ++x_step;
+    x_at = x_at + 1 == stages ? 0 : x_at + 1;
   };
 
-  // both activation buffers start as zeros: the tokens past the last stay so
-  for (uint32_t i = 16u * tid; i < 2u * p.xbuf_bytes; i += 16u * nthreads) *(uint4*)(smem + i) = make_uint4(0, 0, 0, 0);
-  if (lane == 0) {
-    for (int s = 0; s < MD_STAGES; ++s) mbar_init(&full[s], 1);
-    mbar_fence_init();
-  }
+  // the activation buffers start as zeros: the tokens past the last stay so
+  for (uint32_t i = 16u * tid; i < stages * p.xbuf_bytes; i += 16u * nthreads) *(uint4*)(smem + i) = make_uint4(0, 0, 0, 0);
   __syncthreads();
-  for (int s = 0; s < MD_STAGES; ++s) issue_w();  // the weights do not depend on the previous kernel
+  for (int s = 0; s < stages - 1; ++s) fill_w();  // the weights do not depend on the previous kernel
   pdl_launch_dependents();
   pdl_wait();
-  fill_x(0);
+  for (int s = 0; s < stages - 1; ++s) {          // a group a step (the weights are in the first)
+    fill_x();
+    cp_async_commit();
+  }
 
   float acc[NT8][4];
 #pragma unroll
   for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[nt][i] = 0.0f;
-  bool dead = false;
-  int done = 0;
+  int at = 0;
   for (int step = 0; step < nsteps; ++step) {
-    cp_async_wait_all();
-    __syncthreads();  // the step's activations are in; everyone is through with the other buffer
-    if (step + 1 < nsteps) fill_x(step + 1);
-    if (!live || dead) continue;
-    const int s = step % MD_STAGES;
-    bool ok = mbar_wait(&full[s], (uint32_t)(step / MD_STAGES) & 1u, p.status, ST_MV_WAIT + 0x40 + FMT);
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) { dead = true; continue; }
-    ++done;
+    // all but the newer steps' copies: this step's are in
+    if (stages == 4) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else if (stages == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else cp_async_wait_all();
+    __syncthreads();  // ... everyone's; and everyone is through with the stages of the step before, which are filled next
+    fill_w();
+    fill_x();
+    cp_async_commit();
+    const u8* piece = ring + (size_t)at * p.stage_bytes;
+    const u8* xb = smem + (size_t)at * p.xbuf_bytes;
+    at = at + 1 == stages ? 0 : at + 1;
+    if (!live) continue;
     MdFrag<FMT> f;
     {
-      const u8* piece = ring + (size_t)s * p.stage_bytes;
       // a row's bytes start where its block starts inside the 16-byte aligned span that was copied
       const long long o0 = (long long)(row_base + g) * p.row_bytes + (long long)step * SB;
       const long long o8 = o0 + 8ll * p.row_bytes;
@@ -320,9 +313,6 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
       const u8* row8 = piece + (size_t)(g + 8) * p.pitch + (((uintptr_t)p.w + o8) & 15);
       f.load(row0, row8, lane, 8);
     }
-    __syncwarp();
-    issue_w();  // the stage is free: its block sits in registers
-    const u8* xb = smem + (size_t)(step & 1) * p.xbuf_bytes;
     const u8* xl = xb + (lane & 7) * MD_XPITCH + 16 * (lane >> 3);  // this lane's row of the four matrices ldsm4 reads
     const u8* scl = xb + p.xsum_off + 2 * t * MD_SPITCH;  // Q4_K: the sixteen sums of 16 of token 2 t (+ 8 nt)
     const float* ys = (const float*)(xb + p.xs_off) + 2 * t;
@@ -333,11 +323,6 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
       for (int j = 0; j < 4; ++j) ldsm4(x[j], xl + 8 * nt * MD_XPITCH + 64 * j);
       f.apply(x, scl + 8 * nt * MD_SPITCH, scl + (8 * nt + 1) * MD_SPITCH, ys[8 * nt], ys[8 * nt + 1], acc[nt]);
     }
-  }
-  if (dead) {
-    // copies still in flight into this warp's stages get a bounded time to land before shared memory is released
-    for (int k = done; k < issued; ++k) mbar_wait(&full[k % MD_STAGES], (uint32_t)(k / MD_STAGES) & 1u, nullptr, 0);
-    return;
   }
   if (!live) return;
 #pragma unroll
@@ -575,13 +560,12 @@ int mmd_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
   p.xsum_off = off;
   if (fmt == ILL_Q4_K) off += (uint32_t)tn * MdFrag<ILL_Q4_K>::SPITCH;
   p.xbuf_bytes = (off + 127) / 128 * 128;
-  p.ring_off = 2 * p.xbuf_bytes;
-  // three stages a ring where two CTAs still fit an SM with them (or where one CTA has the SM anyway), else two
-  const size_t ring1 = (size_t)p.warps * p.stage_bytes, two_ctas = (233472 / 2 - 1024 - 256);
-  p.stages = (tn == 128 || p.ring_off + 3 * ring1 <= two_ctas) ? 3 : 2;
-  const size_t smem = p.ring_off + (size_t)p.stages * ring1;
+  // stages of weights and activations: four, three where that is all that fits, two where two CTAs share an SM
+  const uint32_t stage = (uint32_t)p.warps * p.stage_bytes + p.xbuf_bytes;
+  p.stages = tn == 64 ? 2 : 226 * 1024 / stage < 4 ? 226 * 1024 / stage : 4;
+  p.ring_off = p.stages * p.xbuf_bytes;
+  const size_t smem = (size_t)p.stages * stage;
   if (smem > 226 * 1024) return ILL_ERR_UNSUPPORTED;
-  p.status = device_status_word();
   const long long grid = (long long)((rows + 16 * p.warps - 1) / (16 * p.warps)) * ((n + tn - 1) / tn);
   if (grid > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;

@@ -461,13 +461,6 @@ static int mt_deal(int np, int gw, u8* sums) {
   return most;
 }
 
-#ifdef ILL_TUNING
-static int g_gw = 0, g_groups = 0, g_stages = 0;
-extern "C" __attribute__((visibility("default"))) void ill_set_mt(int gw, int groups, int stages) { g_gw = gw; g_groups = groups; g_stages = stages; }
-#else
-constexpr int g_gw = 0, g_groups = 0, g_stages = 0;
-#endif
-
 // The several-token product on the tensor cores, of NMAT matrices that share the activations -- of one format, or (FMTS) of Q4_K and
 // Q6_K --, for the formats it is written for; ILL_ERR_UNSUPPORTED otherwise (the caller then takes the CUDA-core kernel).
 int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum,
@@ -539,8 +532,10 @@ int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-  // Warps a group and groups a CTA, for the least time: the tiles a group takes one after another, times the pieces of its busiest
-  // warp.  The rings are as deep as fits (four stages at most, two at least).
+  // Warps a group and groups a CTA, for the least time: the tiles a group takes one after another, times the blocks of its busiest
+  // warp, times what a block takes with that many warps an SM (a latency of 24, and 1 a warp).  The rings are as deep as fits (four
+  // stages at most, two at least).  Swept over every pair on nine launches of a 0.5B, a 4B and a 27B model at 2, 4 and 16 tokens: the
+  // fastest pair or one within 5 % of it but for a head of 151936 x 2560 at two tokens (10 %).
   const uint32_t budget = 226u * 1024u, part_bytes = 2u * p.nsums * ntok * 20 * 4;
   double best = 0;
   for (int gw = p.nsums; gw >= 1; --gw) {
@@ -551,7 +546,6 @@ int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
     for (int g = MT_MAX_WARPS / gw; g >= 1; --g) {
       if (g > 1 && (g - 1) * sms >= ntiles) continue;      // (fewer groups have a tile each already)
       if (off + g * (part_bytes + 2 * ring1) > budget) continue;
-      if (g_gw && (g_gw != gw || g_groups != g)) continue;
       const long long rounds = (ntiles + (long long)g * sms - 1) / ((long long)g * sms);
       const double a_tile = (double)(tiles[0] * most[0] + tiles[1] * most[1]) / ntiles, cost = rounds * a_tile * (24 + g * gw);
       if (p.groups && cost >= best) continue;
@@ -562,7 +556,6 @@ int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
         for (int k = 0; k < MT_SUMS; ++k) p.f[i].sums[k] = sums[i][k];
       p.stages = (int)((budget - off - g * part_bytes) / (g * ring1));
       if (p.stages > MT_MAX_STAGES) p.stages = MT_MAX_STAGES;
-      if (g_stages && p.stages > g_stages) p.stages = g_stages;
     }
   }
   if (!p.groups) return ILL_ERR_UNSUPPORTED;
