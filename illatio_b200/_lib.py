@@ -47,6 +47,8 @@ SIGNATURES = {
     "ill_mv_glu": (_I, [_I, _P, _P, _I, _I, _P, _P, _P, _P, _S]),
     "ill_moe_mv": (_I, [_I, _I, _I, _L, _P, _I, _P, _P, _P, _I, _P, _L, _S]),
     "ill_moe_glu": (_I, [_I, _I, _I, _L, _L, _P, _I, _P, _P, _P, _I, _F, _P, _P, _L, _S]),
+    "ill_moe_mv_sel": (_I, [_I, _I, _I, _L, _P, _I, _P, _I, _P, _P, _P, _I, _P, _L, _S]),
+    "ill_moe_glu_sel": (_I, [_I, _I, _I, _L, _L, _P, _I, _P, _I, _P, _P, _P, _I, _F, _P, _P, _L, _S]),
     "ill_silu_mul": (_I, [_L, _P, _P, _P, _S]),
     "ill_swiglu_w": (_I, [_L, _I, _F, _P, _P, _P, _P, _S]),
     "ill_moe_sum": (_I, [_I, _I, _L, _P, _P, _P, _P, _S]),

@@ -27,7 +27,8 @@ enum { MODE_PLAIN = 0, MODE_GLU = 1, MODE_MOE_GLU = 2,
 // is given.  See ill_mv / ill_moe_mv for the argument meaning.
 int mv_common(int fmt, int mode, int nmat, const uint64_t* w, const int* rows, int cols, uint64_t xq, uint64_t xs,
               uint64_t xsum, const uint64_t* y, const uint64_t* bias, int acc, int n, uint64_t ptrs, int nseg,
-              long long add, long long up_add, int x_seg, long long y_seg, uint64_t seg_w, float clamp, void* stream);
+              long long add, long long up_add, int x_seg, long long y_seg, uint64_t seg_w, float clamp, void* stream,
+              uint64_t sel = 0, int nptrs = 0);
 
 // Lanes a row and units a lane of the one-token product for rows of UNITS units (mv.cu); false when a row does
 // not fit in registers.  BIG: the launch moves 16 MB or more.

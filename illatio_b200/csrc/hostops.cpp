@@ -25,7 +25,9 @@ long long g_launches = 0;     // launches made from this module (counted under t
 #define NAMES(X) \
   X(type) X(rows) X(cols) X(qs) X(kind) X(xq) X(xs) X(xsum) X(_cf) X(w) X(act) X(y) X(n) X(bias) X(acc) X(x) X(f16_scale) X(d) X(eps) \
   X(h) X(wq) X(wk) X(wv) X(q) X(k) X(v) X(bq) X(bk) X(bv) X(g) X(u) X(fa) X(fb) X(emb) X(tokens) X(quant_q8) X(rmsnorm_q8) \
-  X(cmat_mul) X(glu_mul) X(qkv_mul) X(error) X(vars) X(TC_MIN_TOKENS)
+  X(cmat_mul) X(glu_mul) X(qkv_mul) X(error) X(vars) X(TC_MIN_TOKENS) X(dk_mv16) X(route) X(dk_shared) X(dk_ffn_tail) X(logits) X(nu) \
+  X(mode) X(scale) X(sh_gate) X(sh_up) X(sh_down) X(norm) X(clamp) X(out) X(pool) X(norm2) X(sel) X(shared) X(moe) X(ff) X(gate_fmt) \
+  X(down_fmt) X(gate_bytes) X(n_expert) X(ptrs_all)
 #define DECL(s) PyObject* S_##s;
 NAMES(DECL)
 #undef DECL
@@ -313,6 +315,90 @@ PyObject* embed(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kw
   return ret(a[2]);
 } CATCH_ERRORS
 
+// ---- a token's mixture-of-experts layer (cuda_ds4f.py) --------------------------------------
+// The Python forms' steps; what they do not take in one piece -- other types, shapes and layouts -- goes to those.
+
+// device memory of a call's own: N bytes each, 256 apart, from one allocation on the current stream
+struct Scratch {
+  at::Tensor t;
+  ill_dptr next;
+  Scratch(const at::Tensor& like, long long bytes)
+      : t(at::empty({bytes}, like.options().dtype(at::kByte).requires_grad(false))), next((ill_dptr)(uintptr_t)t.data_ptr()) {}
+  ill_dptr take(long long bytes) {
+    const ill_dptr p = next;
+    next += (bytes + 255) / 256 * 256;
+    return p;
+  }
+};
+inline bool plain(const at::Tensor& t, at::ScalarType type) { return t.is_cuda() && t.scalar_type() == type && t.is_contiguous(); }
+
+PyObject* dk_mv16(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
+  ARGS("dk_mv16", 3, S_w, S_x, S_y, S_n);
+  const at::Tensor& w = tensor(a[0]);
+  const int type = w.scalar_type() == at::kFloat ? 0 : w.scalar_type() == at::kHalf ? 1 : w.scalar_type() == at::kBFloat16 ? 2 : -1;
+  if (type < 0 || w.dim() != 2) return PyObject_Vectorcall(slow(S_dk_mv16), args, nargs, kwnames);
+  LAUNCH(ill_mv_dense, type, ptr(a[0]), (int)w.size(0), (int)w.size(1), ptr(a[1]), ptr(a[2]), (int)OPT_INT(a[3], 1), w.size(0), cur_stream());
+  return ret(a[2]);
+} CATCH_ERRORS
+
+PyObject* route(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
+  ARGS("route", 2, S_logits, S_nu, S_mode, S_bias, S_scale);
+  const at::Tensor& l = tensor(a[0]);
+  const long long nu = as_int(a[1]);
+  if (l.dim() != 2 || nu < 1) return PyObject_Vectorcall(slow(S_route), args, nargs, kwnames);
+  at::Tensor sel = at::empty({l.size(0), nu}, l.options().dtype(at::kInt).requires_grad(false)),
+             w = at::empty({l.size(0), nu}, l.options().dtype(at::kFloat).requires_grad(false));
+  LAUNCH(ill_moe_route, (int)l.size(1), (int)nu, (int)OPT_INT(a[2], 2), (float)(a[4] ? as_float(a[4]) : 1.0), l.size(0), ptr(a[0]), OPT_PTR(a[3]),
+         (ill_dptr)(uintptr_t)sel.data_ptr(), (ill_dptr)(uintptr_t)w.data_ptr(), cur_stream());
+  Ref ps(THPVariable_Wrap(sel)), pw(THPVariable_Wrap(w));
+  return PyTuple_Pack(2, ps.p, pw.p);
+} CATCH_ERRORS
+
+PyObject* dk_shared(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
+  ARGS("dk_shared", 6, S_sh_gate, S_sh_up, S_sh_down, S_norm, S_clamp, S_out);
+  const Mat g(a[0]), u(a[1]), d(a[2]);
+  const at::Tensor& x = tensor(a[3]);
+  if (g.type || u.type || d.type || u.rows != g.rows || u.cols != g.cols || d.cols != g.rows || x.numel() != g.cols || !plain(x, at::kFloat))
+    return PyObject_Vectorcall(slow(S_dk_shared), args, nargs, kwnames);
+  const long long c = g.cols, ff = g.rows;
+  Scratch s(x, c + c / 8 + ff + ff / 8 + 12 * ff + 7 * 256);
+  const ill_stream st = cur_stream();
+  const ill_dptr xq = s.take(c), xs = s.take(c / 8), yg = s.take(4 * ff), yu = s.take(4 * ff), mid = s.take(4 * ff), mq = s.take(ff), ms = s.take(ff / 8);
+  LAUNCH(ill_quant_q8_0, ptr(a[3]), xq, xs, 0, c / 32, 0, st);
+  LAUNCH(ill_mv_3, 0, g.w, u.w, 0, g.rows, u.rows, 0, g.cols, xq, xs, 0, yg, yu, 0, 0, 0, 0, st);
+  LAUNCH(ill_swiglu_w, ff, (int)ff, (float)as_float(a[4]), yg, yu, 0, mid, st);
+  LAUNCH(ill_quant_q8_0, mid, mq, ms, 0, ff / 32, 0, st);
+  LAUNCH(ill_mv, 0, d.w, d.rows, d.cols, mq, ms, 0, ptr(a[5]), 0, 0, 1, st);
+  return ret(a[5]);
+} CATCH_ERRORS
+
+PyObject* dk_ffn_tail(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
+  ARGS("dk_ffn_tail", 5, S_pool, S_norm2, S_sel, S_w, S_clamp, S_shared, S_moe);
+  const at::Tensor &x = tensor(a[1]), &sel = tensor(a[2]);
+  const long long d = attr_int(a[0], S_d), ff = attr_int(a[0], S_ff), k = sel.numel();
+  if (!plain(x, at::kFloat) || !plain(sel, at::kInt) || x.numel() != d || d % 256 || ff % 256 || k < 1)
+    return PyObject_Vectorcall(slow(S_dk_ffn_tail), args, nargs, kwnames);
+  const long long gb = attr_int(a[0], S_gate_bytes), ne = attr_int(a[0], S_n_expert);
+  const ill_dptr ptrs = attr_ptr(a[0], S_ptrs_all), sp = ptr(a[2]);
+  const ill_stream st = cur_stream();
+  const auto f32 = x.options().requires_grad(false);
+  Scratch s(x, d + d / 64 + d / 8 + k * (ff + ff / 64 + ff / 8) + 4 * k * d + 8 * 256);
+  const ill_dptr xq = s.take(d), xs = s.take(d / 64), xsum = s.take(d / 8), mq = s.take(k * ff), ms = s.take(k * ff / 64),
+                 msum = s.take(k * ff / 8), down = s.take(4 * k * d);
+  at::Tensor mid = at::empty({k * ff}, f32);
+  const ill_dptr mp = (ill_dptr)(uintptr_t)mid.data_ptr();
+  LAUNCH(ill_quant_q8_k, ptr(a[1]), xq, xs, xsum, d / 256, st);
+  LAUNCH(ill_moe_glu_sel, (int)attr_int(a[0], S_gate_fmt), (int)d, (int)ff, 0, gb, ptrs, (int)ne, sp, (int)k, xq, xs, xsum, 0, (float)as_float(a[4]),
+         ptr(a[3]), mp, ff, st);
+  // a slot's FF values are whole super-blocks: quantized apart (src/ds4f.lisp:1021-1022)
+  LAUNCH(ill_quant_q8_k, mp, mq, ms, msum, k * ff / 256, st);
+  LAUNCH(ill_moe_mv_sel, (int)attr_int(a[0], S_down_fmt), (int)ff, (int)d, 2 * gb, ptrs, (int)ne, sp, (int)k, mq, ms, msum, 1, down, d, st);
+  Ref moe(a[6] && a[6] != Py_None ? ret(a[6]) : THPVariable_Wrap(at::empty({d}, f32)));
+  LAUNCH(ill_moe_sum, (int)d, (int)k, 1, down, 0, OPT_PTR(a[5]), ptr(moe.p), st);
+  Ref pm(THPVariable_Wrap(mid));
+  return PyTuple_Pack(2, moe.p, pm.p);
+} CATCH_ERRORS
+
 PyObject* launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches); }
 
 PyObject* set_slow(PyObject*, PyObject* d) {
@@ -342,6 +428,18 @@ PyMethodDef methods[] = {
          "FA's shape, is scratch for the products that one launch does not take."),
     FAST(embed,
          "embed(emb, tokens, x)\n--\n\nEMBED (src/cuda-dense.lisp:302-307): rows TOKENS (int32 on the device) of EMB as floats in X."),
+    FAST(dk_mv16,
+         "dk_mv16(w, x, y, n=1)\n--\n\nDK-MV16 (src/cuda-ds4f.lisp:767-771): Y = W X for an unquantized tensor W [rows, cols]\n"
+         "(float32, float16 or bfloat16 on the device) and N tokens' float activations."),
+    FAST(route,
+         "route(logits, nu, mode=2, bias=None, scale=1.0)\n--\n\nD4-ROUTE / G53-ROUTE on the device for every row of LOGITS [n, ne]."),
+    FAST(dk_shared,
+         "dk_shared(sh_gate, sh_up, sh_down, norm, clamp, out)\n--\n\nThe shared expert as DK-FFN-HEAD runs it\n"
+         "(src/cuda-ds4f.lisp:900-906): D4-SHARED! (src/ds4f.lisp:1039-1048)."),
+    FAST(dk_ffn_tail,
+         "dk_ffn_tail(pool, norm2, sel, w, clamp, shared=None, moe=None)\n--\n\nDK-FFN-TAIL (src/cuda-ds4f.lisp:908-956) for one token:\n"
+         "the routed experts SEL (device int32 [k]) with weights W (device float [k]) on the FFN input NORM2, summed in SEL's order\n"
+         "with the shared expert's output SHARED."),
     {"launches", launches, METH_NOARGS, "Launches made by this module since it was loaded."},
     {"set_slow", set_slow, METH_O, "Python functions for what this module leaves to Python: {name: function}."},
     {nullptr, nullptr, 0, nullptr}};

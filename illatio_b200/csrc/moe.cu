@@ -402,24 +402,48 @@ using namespace ill;
 
 static int check_ptr(ill_dptr p, unsigned align) { return p && !(p & (align - 1)); }
 
-extern "C" int ill_moe_mv(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, int nz, ill_dptr xq, ill_dptr xs,
-                          ill_dptr xsum, int x_per_expert, ill_dptr y, int64_t y_stride, ill_stream stream) {
-  if (!ptrs || nz < 1 || (ptrs & 7) || (x_per_expert != 0 && x_per_expert != 1)) return ILL_ERR_ARG;
+static int moe_mv(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, int nz, ill_dptr xq, ill_dptr xs, ill_dptr xsum,
+                  int x_per_expert, ill_dptr y, int64_t y_stride, ill_stream stream, ill_dptr sel, int ne) {
+  if (!ptrs || nz < 1 || (ptrs & 7) || (sel & 3) || (x_per_expert != 0 && x_per_expert != 1)) return ILL_ERR_ARG;
   const uint64_t ws[1] = {0}, ys[1] = {y};
   const int rs[1] = {nrows};
   return mv_common(fmt, MODE_PLAIN, 1, ws, rs, ncols, xq, xs, xsum, ys, nullptr, 0, 1, ptrs, nz, add, 0, x_per_expert,
-                   y_stride, 0, 0.0f, stream);
+                   y_stride, 0, 0.0f, stream, sel, ne);
+}
+
+static int moe_glu(int fmt, int ncols, int nrows, int64_t gate_add, int64_t up_add, ill_dptr ptrs, int nz, ill_dptr xq, ill_dptr xs,
+                   ill_dptr xsum, int x_per_expert, float clamp, ill_dptr weights, ill_dptr mid, int64_t mid_stride, ill_stream stream,
+                   ill_dptr sel, int ne) {
+  if (!ptrs || nz < 1 || (ptrs & 7) || (sel & 3) || !weights || (weights & 3) || (x_per_expert != 0 && x_per_expert != 1))
+    return ILL_ERR_ARG;
+  const uint64_t ws[2] = {0, 0}, ys[2] = {mid, mid};
+  const int rs[2] = {nrows, nrows};
+  return mv_common(fmt, MODE_MOE_GLU, 2, ws, rs, ncols, xq, xs, xsum, ys, nullptr, 0, 1, ptrs, nz, gate_add,
+                   up_add - gate_add, x_per_expert, mid_stride, weights, clamp, stream, sel, ne);
+}
+
+extern "C" int ill_moe_mv(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, int nz, ill_dptr xq, ill_dptr xs,
+                          ill_dptr xsum, int x_per_expert, ill_dptr y, int64_t y_stride, ill_stream stream) {
+  return moe_mv(fmt, ncols, nrows, add, ptrs, nz, xq, xs, xsum, x_per_expert, y, y_stride, stream, 0, 0);
+}
+
+extern "C" int ill_moe_mv_sel(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, int ne, ill_dptr sel, int nz, ill_dptr xq,
+                              ill_dptr xs, ill_dptr xsum, int x_per_expert, ill_dptr y, int64_t y_stride, ill_stream stream) {
+  if (!sel || ne < 1) return ILL_ERR_ARG;
+  return moe_mv(fmt, ncols, nrows, add, ptrs, nz, xq, xs, xsum, x_per_expert, y, y_stride, stream, sel, ne);
 }
 
 extern "C" int ill_moe_glu(int fmt, int ncols, int nrows, int64_t gate_add, int64_t up_add, ill_dptr ptrs, int nz,
                            ill_dptr xq, ill_dptr xs, ill_dptr xsum, int x_per_expert, float clamp, ill_dptr weights,
                            ill_dptr mid, int64_t mid_stride, ill_stream stream) {
-  if (!ptrs || nz < 1 || (ptrs & 7) || !weights || (weights & 3) || (x_per_expert != 0 && x_per_expert != 1))
-    return ILL_ERR_ARG;
-  const uint64_t ws[2] = {0, 0}, ys[2] = {mid, mid};
-  const int rs[2] = {nrows, nrows};
-  return mv_common(fmt, MODE_MOE_GLU, 2, ws, rs, ncols, xq, xs, xsum, ys, nullptr, 0, 1, ptrs, nz, gate_add,
-                   up_add - gate_add, x_per_expert, mid_stride, weights, clamp, stream);
+  return moe_glu(fmt, ncols, nrows, gate_add, up_add, ptrs, nz, xq, xs, xsum, x_per_expert, clamp, weights, mid, mid_stride, stream, 0, 0);
+}
+
+extern "C" int ill_moe_glu_sel(int fmt, int ncols, int nrows, int64_t gate_add, int64_t up_add, ill_dptr ptrs, int ne, ill_dptr sel,
+                               int nz, ill_dptr xq, ill_dptr xs, ill_dptr xsum, int x_per_expert, float clamp, ill_dptr weights,
+                               ill_dptr mid, int64_t mid_stride, ill_stream stream) {
+  if (!sel || ne < 1) return ILL_ERR_ARG;
+  return moe_glu(fmt, ncols, nrows, gate_add, up_add, ptrs, nz, xq, xs, xsum, x_per_expert, clamp, weights, mid, mid_stride, stream, sel, ne);
 }
 
 extern "C" int ill_swiglu_w(int64_t n, int ff, float clamp, ill_dptr g, ill_dptr u, ill_dptr w, ill_dptr mid,

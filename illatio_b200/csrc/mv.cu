@@ -53,6 +53,8 @@ struct MvParams {
   // segments (grid.y): expert z's weights at ptrs[z] + add (+ up_add for "up"),
   // its activations at token z*x_seg (0: shared), its output at y + z*y_seg
   const unsigned long long* ptrs;
+  const int* sel;       // given: expert z is SEL[z] (from the end where below 0) of the NPTRS that PTRS holds
+  int nptrs;
   long long add, up_add;
   int x_seg;
   long long y_seg;
@@ -69,6 +71,18 @@ struct MvParams {
   unsigned epoch;
   unsigned long long wait_ns;
 };
+
+// The place in PTRS of segment Z.  An expert number out of range raises the status word and reads expert 0: inside the pool.
+__device__ __forceinline__ int mv_expert(const MvParams& p, int z) {
+  if (!p.sel) return z;
+  int e = after_wait(p.sel)[z];
+  if (e < 0) e += p.nptrs;
+  if ((unsigned)e >= (unsigned)p.nptrs) {
+    if (p.status) atomicCAS(p.status, 0u, (unsigned)ST_GROUP_SEL);
+    e = 0;
+  }
+  return e;
+}
 
 __device__ unsigned g_mv_ticket;  // CTAs of the running peer-storing product that are through (one such call at a time a device)
 
@@ -118,7 +132,7 @@ __global__ void __launch_bounds__(MV_THREADS) mvn_kernel(const MvParams p) {
     if (IQ) iq_tables_fill(iq_grid, iq_smask, ill_iq2xxs_grid, ill_ksigns_iq2xs);
     pdl_launch_dependents();
     pdl_wait();
-    const u8* b = (const u8*)(uintptr_t)after_wait(p.ptrs)[z] + p.add;
+    const u8* b = (const u8*)(uintptr_t)after_wait(p.ptrs)[mv_expert(p, z)] + p.add;
     wbase[0] = b;
     wbase[1] = b + p.up_add;
     wbase[2] = b;
@@ -330,7 +344,7 @@ __global__ void __launch_bounds__(MV_THREADS) mvw_kernel(const MvParams p) {
     if (IQ) iq_tables_fill(iq_grid, iq_smask, ill_iq2xxs_grid, ill_ksigns_iq2xs);
     pdl_launch_dependents();
     pdl_wait();
-    const u8* b = (const u8*)(uintptr_t)after_wait(p.ptrs)[z] + p.add;
+    const u8* b = (const u8*)(uintptr_t)after_wait(p.ptrs)[mv_expert(p, z)] + p.add;
     wbase[0] = b;
     wbase[1] = b + p.up_add;
     wbase[2] = b;
@@ -820,7 +834,7 @@ static thread_local const MvPeer* t_peer = nullptr;
 int mv_common(int fmt, int mode, int nmat, const ill_dptr* w, const int* rows, int cols, ill_dptr xq, ill_dptr xs,
               ill_dptr xsum, const ill_dptr* y, const ill_dptr* bias, int acc, int n, ill_dptr ptrs, int nseg,
               long long add, long long up_add, int x_seg, long long y_seg, ill_dptr seg_w, float clamp,
-              ill_stream stream) {
+              ill_stream stream, ill_dptr sel, int nptrs) {
   const int bw = fmt_block_weights(fmt);
   if (!bw || nmat < 1 || nmat > MV_MAX_MATS || cols <= 0 || cols % (bw == 32 ? 32 : 256)) return ILL_ERR_ARG;
   if (n < 1 || nseg < 1 || nseg > 65535) return ILL_ERR_ARG;
@@ -886,6 +900,8 @@ int mv_common(int fmt, int mode, int nmat, const ill_dptr* w, const int* rows, i
   p.xs_off = pl.xs_off;
   p.bs_off = pl.bs_off;
   p.ptrs = (const unsigned long long*)(uintptr_t)ptrs;
+  p.sel = (const int*)(uintptr_t)sel;
+  p.nptrs = nptrs;
   p.add = add;
   p.up_add = up_add;
   p.x_seg = x_seg;

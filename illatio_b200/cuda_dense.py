@@ -193,8 +193,9 @@ def _glu_mul(g, u, act, fa, n=1, fb=None):
     return fa
 
 
-_H.set_slow({"quant_q8": _quant_q8, "rmsnorm_q8": _rmsnorm_q8, "cmat_mul": _cmat_mul, "qkv_mul": _qkv_mul, "glu_mul": _glu_mul,
-             "error": _lib.fail, "vars": globals()})
+_SLOW = {"quant_q8": _quant_q8, "rmsnorm_q8": _rmsnorm_q8, "cmat_mul": _cmat_mul, "qkv_mul": _qkv_mul, "glu_mul": _glu_mul,
+             "error": _lib.fail, "vars": globals()}
+_H.set_slow(_SLOW)
 
 
 class ChunkF16:

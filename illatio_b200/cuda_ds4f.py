@@ -77,7 +77,7 @@ F32, F16, BF16 = 0, 1, 2
 _DENSE_TYPES = {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16}
 
 
-def dk_mv16(w, x, y, n=1):
+def _dk_mv16(w, x, y, n=1):
     """DK-MV16 (src/cuda-ds4f.lisp:767-771): Y = W X for an unquantized tensor W [rows, cols]
     (float32, float16 or bfloat16 on the device) and N tokens' float activations."""
     rows, cols = w.shape
@@ -91,7 +91,7 @@ def swiglu_w(g, u, w, mid, ff, clamp):
     return mid
 
 
-def dk_shared(sh_gate, sh_up, sh_down, norm, clamp, out):
+def _dk_shared(sh_gate, sh_up, sh_down, norm, clamp, out):
     """The shared expert as DK-FFN-HEAD runs it (src/cuda-ds4f.lisp:900-906):
     D4-SHARED! (src/ds4f.lisp:1039-1048)."""
     ff = sh_gate.rows
@@ -105,7 +105,7 @@ def dk_shared(sh_gate, sh_up, sh_down, norm, clamp, out):
     return out
 
 
-def route(logits, nu, mode=2, bias=None, scale=1.0):
+def _route(logits, nu, mode=2, bias=None, scale=1.0):
     """D4-ROUTE / G53-ROUTE on the device for every row of LOGITS [n, ne]."""
     n, ne = logits.shape
     sel = torch.empty(n, nu, dtype=torch.int32, device=logits.device)
@@ -114,7 +114,7 @@ def route(logits, nu, mode=2, bias=None, scale=1.0):
     return sel, w
 
 
-def dk_ffn_tail(pool, norm2, sel, w, clamp, shared=None, moe=None):
+def _dk_ffn_tail(pool, norm2, sel, w, clamp, shared=None, moe=None):
     """DK-FFN-TAIL (src/cuda-ds4f.lisp:908-956) for one token: the routed experts
     SEL (device int32 [k]) with weights W (device float [k]) on the FFN input
     NORM2, summed in SEL's order with the shared expert's output SHARED."""
@@ -135,3 +135,10 @@ def dk_ffn_tail(pool, norm2, sel, w, clamp, shared=None, moe=None):
         moe = torch.empty(d, device=dev)
     _lib.call("ill_moe_sum", d, k, 1, _ptr(bd), 0, _ptr(shared), _ptr(moe), _stream())
     return moe, mid
+
+
+# The operators of a decoded token's layer are native too (csrc/hostops.cpp); the functions above that begin with an underscore
+# and share a name with one are what it leaves to Python.
+_H = _lib.hostops()
+dk_mv16, route, dk_shared, dk_ffn_tail = (getattr(_H, f) for f in ("dk_mv16", "route", "dk_shared", "dk_ffn_tail"))
+D._SLOW.update({"dk_mv16": _dk_mv16, "route": _route, "dk_shared": _dk_shared, "dk_ffn_tail": _dk_ffn_tail})
