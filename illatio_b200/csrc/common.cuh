@@ -27,7 +27,8 @@ enum { ST_OK = 0, ST_MV_WAIT = 0x100,
        ST_MM_WAIT_ACC = 0x400 /* a block's products */,
        ST_MM_WAIT_EPI = 0x500 /* an accumulator has been drained; + 2 the mins' */,
        ST_GROUP_SEL = 0x600 /* an expert number out of range in ill_moe_group's SEL */,
-       ST_MQ_WAIT = 0x900 /* the Q8_0 chunk kernel, by wait: 0 X is free, + 1 X, 2 weights, 3 an accumulator free, 4 scales free, 5 scales, 6 products, 7 weights free, 8 scales free */,
+       ST_MQ_WAIT = 0x900 /* the Q8_0 chunk kernel: a stage of X is free; + 1 a step's operands, + 2 an accumulator is free, + 3 a slot of
+           A, + 4 room for scales, + 5 scales, + 6 products, + 7 a raw buffer is free, + 8 raw blocks */,
        ST_BARRIER_WAIT = 0x700 /* a barrier between CTAs or ranks never completed */,
        ST_TEST_WAIT = 0x800 /* ill_test_wait_timeout: the wait that is meant to run out; + 1 + l: lane l's of ill_test_poll_timeout */ };
 

@@ -21,13 +21,12 @@
 //
 // What bounds it: the drain's instructions.  A sum takes a conversion, a multiplication d_w * d_x, one with the sum and an addition,
 // 512 issue slots a scheduler for 128 x 128 x 32 where the product itself takes 64 cycles (the packed f32x2 forms take two slots
-// each); with the loads of the scales, the hand-overs and the unpacking 830 are executed, at 72 % issue 1150 cycles.  us, int8
+// each); with the loads of the scales, the hand-overs and the unpacking 830 are executed, at 78 % issue about 1100 cycles.  us, int8
 // mma.sync (the kernel before) / now: 896 x 896 x 777 tokens 14.9 / 11.1, 896 x 4864 x 777 67 / 43, 4864 x 896 x 777 38 / 36,
 // 2048 x 4096 x 64 25 / 20, x 200 60 / 26, x 4096 297 / 288, 4096 x 2048 x 4096 298 / 277, 1536 x 5120 x 8192 548 / 548.
 // Measured and taken back: eight drain warps with the next half on its way while one is scaled (NT 128: 309 -> 398); 16 x 256-bit
 // loads of tensor memory, a quarter of the shared memory's traffic (309 -> 319: it was no bound); raw blocks by cp.async of the
-// warps that take them apart (a step 0.5 -> 1.1 us); quarters of the weight rows' tiles dealt evenly whatever the rounds
-// (4864 x 896 x 200 13.6 -> 16.3).
+// warps that take them apart (a step 0.5 -> 1.1 us); even shares whatever the rounds (4864 x 896 x 200 13.6 -> 16.3).
 //
 // Every mbarrier wait is bounded; on a time-out the kernel records a code in the status word, skips what depends on the wait, lets
 // copies and products in flight end, frees its tensor memory and returns.
@@ -351,7 +350,7 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) mm_q8_kernel(const __grid_const
         if ((k & 1) != set) continue;
         const int s = k % MQ_NS, r = k % MQ_NRAW;
         const uint32_t free_par = ((uint32_t)(k / MQ_NS) & 1u) ^ 1u;
-        ok = __all_sync(0xffffffffu, mbar_wait(&raw_full[r], (uint32_t)(k / MQ_NRAW) & 1u, p.status, ST_MQ_WAIT + 2));
+        ok = __all_sync(0xffffffffu, mbar_wait(&raw_full[r], (uint32_t)(k / MQ_NRAW) & 1u, p.status, ST_MQ_WAIT + 8));
         if (!ok) break;
         // the step's 34 words: four blocks of a half and 32 quants, 34 bytes apart
         const uint32_t o16 = (uint32_t)(off + st * MQ_WSTEP) & 15u, sh = 8 * (o16 & 2u);
