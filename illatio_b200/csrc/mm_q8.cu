@@ -415,11 +415,10 @@ static int mq_launch(const MqMaps& maps, const MqParams& p, int grid, cudaStream
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MqGeom<NT>::SMEM);
   if (e != cudaSuccess) return cuda_fail(e);
   // the warp groups trade registers after launch: what they ask for together must fit in what the CTA was given
-  static const int regs = [k] {
-    cudaFuncAttributes fa;
-    return cudaFuncGetAttributes(&fa, k) == cudaSuccess ? fa.numRegs : 0;
-  }();
-  if (regs / 8 * 8 * MQ_THREADS < MQ_REGS_SUM) return ILL_ERR_UNSUPPORTED;
+  cudaFuncAttributes fa;
+  e = cudaFuncGetAttributes(&fa, k);
+  if (e != cudaSuccess) return cuda_fail(e);
+  if (fa.numRegs / 8 * 8 * MQ_THREADS < MQ_REGS_SUM) return ILL_ERR_UNSUPPORTED;
   MqMaps m = maps;
   MqParams pp = p;
   void* args[] = {&m, &pp};
