@@ -35,9 +35,14 @@
 
 namespace ill {
 
-// A tile's pieces are dealt to eight partial sums (piece I to sum I % 8), and the sums to a group's warps; a CTA holds one to four
-// groups (a tile each at a time) that share the staged activations, and each warp a ring of two to four stages.
+// A tile's pieces are dealt to eight partial sums (piece I to sum I % 8), and the sums to a group's warps; a CTA holds as many groups (a
+// tile each at a time) as make up to sixteen warps, which share the staged activations, and each warp a ring of two to four stages.
 constexpr int MT_SUMS = 8, MT_MAX_WARPS = 16, MT_ROWS = 16, MT_MAX_STAGES = 4, MT_MATS = 3;
+
+// The named barrier at which the warps of group GRP of GW warps meet, or 0: a group of one warp needs none.  A CTA has barriers 0 (that
+// of __syncthreads) to 15, and sixteen groups of one warp.
+__host__ __device__ constexpr int mt_barrier(int grp, int gw) { return gw == 1 ? 0 : 1 + grp; }
+static_assert(mt_barrier(MT_MAX_WARPS / 2 - 1, 2) <= 15, "groups of two warps are the most that meet at barriers");
 
 struct MtMat {
   const u8* w;
@@ -264,9 +269,10 @@ __device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, b
 __device__ __forceinline__ void cp_async4_or_zero(void* dst, const void* src, bool in) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 4 : 0) : "memory");
 }
-// the meeting of one group's warps (barrier 1 + group)
-__device__ __forceinline__ void group_sync(int grp, int threads) {
-  asm volatile("barrier.cta.sync %0, %1;" ::"r"(1 + grp), "r"(threads) : "memory");
+// the meeting of one group's warps
+__device__ __forceinline__ void group_sync(int grp, int gw) {
+  if (gw == 1) __syncwarp();
+  else asm volatile("barrier.cta.sync %0, %1;" ::"r"(mt_barrier(grp, gw)), "r"(32 * gw) : "memory");
 }
 
 template <int N> struct IntC { static constexpr int value = N; };
@@ -417,7 +423,7 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
         for (int i = 0; i < 4; ++i) sums[(sum * NTOK + 8 * nt + 2 * t + (i & 1)) * PP + g + 8 * (i >> 1)] = acc[nt][i];
     }
     // the partial sums meet: thread (token, row) adds them in order
-    group_sync(grp, 32 * gw);
+    group_sync(grp, gw);
     const int nsums = min(MT_SUMS, f.npieces);
     for (int o = gtid; o < MT_ROWS * p.n; o += 32 * gw) {
       const int r = o & 15, tk = o >> 4, row = row0 + r;
@@ -461,29 +467,34 @@ static int mt_deal(int np, int gw, u8* sums) {
   return most;
 }
 
-// The several-token product on the tensor cores, of NMAT matrices that share the activations -- of one format, or (FMTS) of Q4_K and
-// Q6_K --, for the formats it is written for; ILL_ERR_UNSUPPORTED otherwise (the caller then takes the CUDA-core kernel).
-int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum,
-            const uint64_t* y, const uint64_t* bias, int acc, int n, void* stream) {
+// A launch of mvt_kernel: everything but the pointers.
+struct MtPlan {
+  MtParams p;
+  int fmt;              // the kernel's (first) format
+  bool two;             // Q4_K and Q6_K
+  int grid;
+  size_t smem;
+};
+
+// The launch for NMAT matrices that share the activations -- of one format, or (FMTS) of Q4_K and Q6_K -- and N tokens on SMS SMs;
+// ILL_ERR_UNSUPPORTED where the kernel is not written for them.
+static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n, int sms, MtPlan* plan) {
   if (n < 2 || n > 16 || nmat < 1 || nmat > MT_MATS) return ILL_ERR_UNSUPPORTED;
-  MtParams p = {};
+  MtParams& p = plan->p;
+  p = {};
   long long ntiles = 0, tiles[2] = {};
-  bool al4 = true, two = false;
+  bool two = false;
   for (int i = 0; i < nmat; ++i) two = two || fmts[i] != fmts[0];
   const int fmt = two ? ILL_Q4_K : fmts[0];
   if (fmt != ILL_Q8_0 && fmt != ILL_Q4_K && fmt != ILL_Q6_K) return ILL_ERR_UNSUPPORTED;
   for (int i = 0; i < MT_MATS; ++i) {
     if (i < nmat) {
       if (two && fmts[i] != ILL_Q4_K && fmts[i] != ILL_Q6_K) return ILL_ERR_UNSUPPORTED;
-      p.m[i].w = (const u8*)(uintptr_t)w[i];
-      p.m[i].y = (float*)(uintptr_t)y[i];
-      p.m[i].bias = bias ? (const float*)(uintptr_t)bias[i] : nullptr;
       p.m[i].rows = rows[i];
       p.m[i].alt = fmts[i] != fmt;
       const int t = (rows[i] + MT_ROWS - 1) / MT_ROWS;
       ntiles += t;
       tiles[p.m[i].alt] += t;
-      if (fmts[i] == ILL_Q4_K) al4 = al4 && (w[i] & 3) == 0;
     }
     if (ntiles > 0x3fffffff) return ILL_ERR_TOO_LARGE;
     p.m[i].tile_end = (int)ntiles;
@@ -491,10 +502,6 @@ int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
   const int bw = fmt_block_weights(fmt), nsc = cols / bw;
   p.cols = cols;
   p.nblocks = nsc;
-  p.xq = (const i8*)(uintptr_t)xq;
-  p.xs = (const float*)(uintptr_t)xs;
-  p.xsum = (const int16_t*)(uintptr_t)xsum;
-  p.acc = acc;
   p.n = n;
   p.x_stride = cols + 16;
   const uint32_t ntok = n <= 8 ? 8 : 16;  // staged tokens: whole tiles of eight
@@ -529,9 +536,6 @@ int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
   if (fmt != ILL_Q8_0) off += 32u * ntok * (cols / 256);
   off = (off + 127) / 128 * 128;
   p.ring_off = off;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   // Warps a group and groups a CTA, for the least time: the tiles a group takes one after another, times the blocks of its busiest
   // warp, times what a block takes with that many warps an SM (a latency of 24, and 1 a warp).  The rings are as deep as fits (four
   // stages at most, two at least).  Swept over every pair on nine launches of a 0.5B, a 4B and a 27B model at 2, 4 and 16 tokens: the
@@ -562,19 +566,70 @@ int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
   off += (uint32_t)(p.groups * p.gw * p.stages) * p.stage_bytes;
   p.part_off = off;
   off += (uint32_t)p.groups * part_bytes;
-  const size_t smem = off;
   // (two CTAs an SM where their registers fit too: up to 64 a thread, K formats up to 83 or 128)
   const int threads = 32 * p.gw * p.groups, most2 = fmt == ILL_Q8_0 ? 512 : n <= 8 ? 384 : 256;
-  const int per_sm = (int)((227u * 1024u) / (smem + 1024u)) >= 2 && threads <= most2 ? 2 : 1;
-  long long grid = (long long)sms * per_sm;
-  if (grid > ntiles) grid = ntiles;
+  const int per_sm = (int)((227u * 1024u) / (off + 1024u)) >= 2 && threads <= most2 ? 2 : 1;
+  plan->grid = (int)((long long)sms * per_sm < ntiles ? (long long)sms * per_sm : ntiles);
+  plan->smem = off;
+  plan->fmt = fmt;
+  plan->two = two;
+  return ILL_OK;
+}
+
+// The several-token product on the tensor cores, for the formats it is written for; ILL_ERR_UNSUPPORTED otherwise (the caller then
+// takes the CUDA-core kernel).
+int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum,
+            const uint64_t* y, const uint64_t* bias, int acc, int n, void* stream) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+  MtPlan plan;
+  const int rc = mvt_plan(nmat, fmts, rows, cols, n, sms, &plan);
+  if (rc) return rc;
+  MtParams& p = plan.p;
+  bool al4 = true;
+  for (int i = 0; i < nmat; ++i) {
+    p.m[i].w = (const u8*)(uintptr_t)w[i];
+    p.m[i].y = (float*)(uintptr_t)y[i];
+    p.m[i].bias = bias ? (const float*)(uintptr_t)bias[i] : nullptr;
+    if (fmts[i] == ILL_Q4_K) al4 = al4 && (w[i] & 3) == 0;
+  }
+  p.xq = (const i8*)(uintptr_t)xq;
+  p.xs = (const float*)(uintptr_t)xs;
+  p.xsum = (const int16_t*)(uintptr_t)xsum;
+  p.acc = acc;
+  const size_t smem = plan.smem;
   cudaStream_t st = (cudaStream_t)stream;
-  if (two) return al4 ? mvt_launch<ILL_Q4_K, ILL_Q6_K, true>(p, smem, (int)grid, st) : mvt_launch<ILL_Q4_K, ILL_Q6_K, false>(p, smem, (int)grid, st);
-  switch (fmt) {
-    case ILL_Q8_0: return mvt_launch<ILL_Q8_0, ILL_Q8_0, false>(p, smem, (int)grid, st);
-    case ILL_Q4_K: return al4 ? mvt_launch<ILL_Q4_K, ILL_Q4_K, true>(p, smem, (int)grid, st) : mvt_launch<ILL_Q4_K, ILL_Q4_K, false>(p, smem, (int)grid, st);
-    default: return mvt_launch<ILL_Q6_K, ILL_Q6_K, false>(p, smem, (int)grid, st);
+  if (plan.two)
+    return al4 ? mvt_launch<ILL_Q4_K, ILL_Q6_K, true>(p, smem, plan.grid, st) : mvt_launch<ILL_Q4_K, ILL_Q6_K, false>(p, smem, plan.grid, st);
+  switch (plan.fmt) {
+    case ILL_Q8_0: return mvt_launch<ILL_Q8_0, ILL_Q8_0, false>(p, smem, plan.grid, st);
+    case ILL_Q4_K: return al4 ? mvt_launch<ILL_Q4_K, ILL_Q4_K, true>(p, smem, plan.grid, st) : mvt_launch<ILL_Q4_K, ILL_Q4_K, false>(p, smem, plan.grid, st);
+    default: return mvt_launch<ILL_Q6_K, ILL_Q6_K, false>(p, smem, plan.grid, st);
   }
 }
 
 }  // namespace ill
+
+using namespace ill;
+
+extern "C" int ill_test_few_tokens_plan(int nmat, int fmt0, int fmt1, int fmt2, int rows0, int rows1, int rows2, int cols, int n, int sms,
+                                        int* out) {
+  const int fmts[3] = {fmt0, fmt1, fmt2}, rows[3] = {rows0, rows1, rows2};
+  if (!out || nmat < 1 || nmat > MT_MATS || cols <= 0 || sms < 1) return ILL_ERR_ARG;
+  for (int i = 0; i < nmat; ++i) {
+    const int bw = fmt_block_weights(fmts[i]);
+    if (!bw || rows[i] <= 0 || cols % bw) return ILL_ERR_ARG;
+  }
+  MtPlan plan;
+  const int rc = mvt_plan(nmat, fmts, rows, cols, n, sms, &plan);
+  if (rc) return rc;
+  const MtParams& p = plan.p;
+  out[0] = p.gw;
+  out[1] = p.groups;
+  out[2] = mt_barrier(p.groups - 1, p.gw);
+  out[3] = p.stages;
+  out[4] = plan.grid;
+  out[5] = (int)plan.smem;
+  return ILL_OK;
+}

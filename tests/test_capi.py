@@ -4,6 +4,8 @@ import ctypes
 import os
 import re
 
+import pytest
+
 from illatio_b200 import _lib, build
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -66,3 +68,26 @@ def test_argument_checks_of_the_chunk_and_peer_entry_points():
     assert s("ill_moe_row_ptrs", 0, 16, 16, 16, 8, 16, None) == 1
     assert s("ill_moe_row_ptrs", 4, 16, 16, 16, 8, 20, None) == 1
     assert s("ill_moe_row_ptrs", 4, 16, 16, 16, 0, 16, None) == 0   # no rows: nothing to do
+
+
+@pytest.mark.parametrize("fmt", [0, 1, 2, (1, 2)])
+@pytest.mark.parametrize("n", [2, 4, 8, 9, 16])
+def test_launches_of_few_tokens_stay_within_a_cta(fmt, n):
+    """Every launch of two to sixteen tokens has barriers (0 to 15), warps and shared memory that a CTA has, over all numbers of blocks a
+    row and the numbers of tiles around whole rounds of 148 SMs: short rows of many rows get up to sixteen groups."""
+    two = isinstance(fmt, tuple)
+    f = fmt if two else (fmt, 0)
+    out, seen = (ctypes.c_int * 6)(), set()
+    for blocks in list(range(1, 42)) + [48, 56, 57, 64, 68, 152, 256, 544]:
+        cols = blocks * (32 if fmt == 0 else 256)
+        for rounds in list(range(1, 20)) + [31, 32, 33, 47, 48, 49, 64, 110]:
+            for rows in (16 * 148 * rounds - 1600, 16 * 148 * rounds, 16 * 148 * rounds + 1):
+                rc = _lib.status("ill_test_few_tokens_plan", 2 if two else 1, f[0], f[1], 0, rows, rows if two else 0, 0, cols, n, 148, out)
+                assert rc in (0, 3)
+                if rc == 0:
+                    warps, groups, barrier, stages, ctas, smem = out
+                    seen.add((warps, groups))
+                    assert warps >= 1 and groups >= 1 and warps * groups <= 16 and 2 <= stages <= 4 and ctas >= 1
+                    assert 0 <= barrier <= 15 and (warps == 1) == (barrier == 0)
+                    assert smem <= 227 * 1024
+    assert (1, 16) in seen

@@ -1,5 +1,7 @@
 """Products of two to sixteen tokens: two or three matrices in one launch (ill_mv_3n) give each matrix's own bits, whatever groups and
 sums the launch deals out; ragged rows, rows at every alignment, Q4_K beside Q6_K; and the product itself against the oracle."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -54,6 +56,31 @@ def test_matrices_in_one_launch_give_each_ones_bits(cuda_lib, fmts, rows, cols, 
     for g, w, r in zip(got, want, rows):
         assert torch.equal(g[:n * r], w)
         assert (g[n * r:] == 7.0).all()
+    assert D.device_status() == 0
+
+
+@pytest.mark.parametrize("fmt,rows,cols,n", [(B.Q4_K, 36000, 768, 4), (B.Q4_K, 37888, 256, 16), (B.Q6_K, 36000, 768, 3), (B.Q8_0, 36001, 576, 8)])
+def test_short_rows_of_many(cuda_lib, fmt, rows, cols, n):
+    """Sixteen groups of one warp a CTA (short rows whose tiles nearly fill the rounds): the bits of launches of some of the rows, which
+    have other groups."""
+    out = (ctypes.c_int * 6)()
+    assert _lib.status("ill_test_few_tokens_plan", 1, fmt, 0, 0, rows, 0, 0, cols, n, 148, out) == 0 and list(out[:3]) == [1, 16, 0]
+    act = dev_act(fmt, np.random.default_rng(rows).standard_normal(n * cols).astype(np.float32))
+    w, keep, ptr = _mat(fmt, rows, cols, 5, 0)
+    xsum = 0 if act.kind == "q8" else act.xsum.data_ptr()
+
+    def mul(row0, count):
+        y = torch.full((n * count + 8,), 7.0, device="cuda")
+        _lib.call("ill_mv", fmt, ptr + row0 * B.row_bytes(fmt, cols), count, cols, act.xq.data_ptr(), act.xs.data_ptr(), xsum, y.data_ptr(), 0, 0, n,
+                  _lib.stream())
+        assert (y[n * count:] == 7.0).all()
+        return y[:n * count].view(n, count)
+
+    got = mul(0, rows)
+    for row0, count in ((0, 1600), (17760, 333), (rows - 1000, 1000)):
+        _lib.call("ill_test_few_tokens_plan", 1, fmt, 0, 0, count, 0, 0, cols, n, 148, out)
+        assert out[1] < 16
+        assert torch.equal(got[:, row0:row0 + count], mul(row0, count))
     assert D.device_status() == 0
 
 
