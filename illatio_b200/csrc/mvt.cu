@@ -344,7 +344,13 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
   const int nsc = p.cols / BW, per_tok = p.cols / 16;
   uint4 sum8[2];            // K formats: eight sums of 16 a load; two loads a thread hold 16 tokens of 8192 columns
   const int nsum8 = FMT == ILL_Q8_0 ? 0 : NTOK * per_tok / 8;
-  auto load_sums = [&](int i) { return i < nsum8 && 8 * i < p.n * per_tok ? ((const uint4*)p.xsum)[i] : make_uint4(0, 0, 0, 0); };
+  const bool sums16 = ((uintptr_t)p.xsum & 15) == 0;  // (the sums lie on eight bytes, if not on sixteen)
+  auto load_sums = [&](int i) {
+    if (i >= nsum8 || 8 * i >= p.n * per_tok) return make_uint4(0, 0, 0, 0);
+    if (sums16) return ((const uint4*)p.xsum)[i];
+    const uint2 a = ((const uint2*)p.xsum)[2 * i], b = ((const uint2*)p.xsum)[2 * i + 1];
+    return make_uint4(a.x, a.y, b.x, b.y);
+  };
 #pragma unroll
   for (int k = 0; k < 2; ++k) sum8[k] = load_sums(tid + k * nthreads);
   for (int tk = cwarp; tk < NTOK; tk += nthreads / 32)  // a warp a token

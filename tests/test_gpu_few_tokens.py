@@ -84,6 +84,33 @@ def test_short_rows_of_many(cuda_lib, fmt, rows, cols, n):
     assert D.device_status() == 0
 
 
+@pytest.mark.parametrize("fmt,cols,n", [(B.Q4_K, 256, 2), (B.Q4_K, 2560, 16), (B.Q6_K, 768, 9), (B.Q4_K, 17408, 5), (B.Q6_K, 17408, 16)])
+def test_sums_of_16_that_lie_on_eight_bytes(cuda_lib, fmt, cols, n):
+    """The sums of 16 need lie on eight bytes only: the bits of sums on sixteen, of one matrix and of two in a launch, and through the
+    operators given an activation of the caller's own."""
+    rows = 33
+    act = dev_act(fmt, np.random.default_rng(cols + n).standard_normal(n * cols).astype(np.float32))
+    buf = torch.empty(act.xsum.numel() + 4, dtype=torch.int16, device="cuda")
+    off = buf[4:]
+    off.copy_(act.xsum)
+    assert act.xsum.data_ptr() % 16 == 0 and off.data_ptr() % 16 == 8
+    mats = [D.upload_gmat(B.synth_matrix(fmt, rows, cols, seed=s), fmt, rows, cols) for s in (1, 2, 3)]
+    other = D.QAct(act.kind, act.xq, act.xs, off)
+    got, want = ([torch.zeros(n * rows, device="cuda") for _ in mats] for _ in range(2))
+    for m, y in zip(mats, want):
+        D.cmat_mul(m, act, y, n)
+    D.cmat_mul(mats[0], other, got[0], n)
+    assert torch.allclose(got[0], want[0], rtol=0, atol=1e-5 * want[0].abs().max().item())
+    if cols < 17408:  # (longer rows' kernel wants Q4_K's sums on sixteen bytes: the product is another's, in another order)
+        assert torch.equal(got[0], want[0])
+        D.qkv_mul(*mats, other, *got, n=n)
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        fa = D.glu_mul(mats[0], mats[1], act, torch.empty_like(want[0]), n, fb=torch.empty_like(want[0]))
+        fo = D.glu_mul(mats[0], mats[1], other, torch.empty_like(want[0]), n, fb=torch.empty_like(want[0]))
+        assert torch.equal(fa, fo)
+    assert D.device_status() == 0
+
+
 @pytest.mark.parametrize("fmt,rows,cols,n", [(B.Q8_0, 50, 1152, 16), (B.Q4_K, 40, 2560, 16), (B.Q4_K, 19, 1280, 3), (B.Q6_K, 40, 5120, 16),
                                              (B.Q6_K, 23, 2304, 2)])
 def test_few_tokens_against_the_oracle(oracle, cuda_lib, fmt, rows, cols, n):
