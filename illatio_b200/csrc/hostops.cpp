@@ -27,7 +27,7 @@ long long g_launches = 0;     // launches made from this module (counted under t
   X(h) X(wq) X(wk) X(wv) X(q) X(k) X(v) X(bq) X(bk) X(bv) X(g) X(u) X(fa) X(fb) X(emb) X(tokens) X(quant_q8) X(rmsnorm_q8) \
   X(cmat_mul) X(glu_mul) X(qkv_mul) X(error) X(vars) X(TC_MIN_TOKENS) X(dk_mv16) X(route) X(dk_shared) X(dk_ffn_tail) X(logits) X(nu) \
   X(mode) X(scale) X(sh_gate) X(sh_up) X(sh_down) X(norm) X(clamp) X(out) X(pool) X(norm2) X(sel) X(shared) X(moe) X(ff) X(gate_fmt) \
-  X(down_fmt) X(gate_bytes) X(n_expert) X(ptrs_all)
+  X(down_fmt) X(gate_bytes) X(ptrs_all) X(slot_ptrs)
 #define DECL(s) PyObject* S_##s;
 NAMES(DECL)
 #undef DECL
@@ -372,14 +372,24 @@ PyObject* dk_shared(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject
   return ret(a[5]);
 } CATCH_ERRORS
 
+// Whether a pool's slot_ptrs() is ExpertPool's own, which reads its ptrs_all: not a subclass's, or an object's with a table elsewhere
+inline bool own_slots(PyObject* pool) {
+  Ref m(PyObject_GetAttr(pool, S_slot_ptrs));
+  return PyMethod_Check(m.p) && PyMethod_GET_SELF(m.p) == pool && PyMethod_GET_FUNCTION(m.p) == slow(S_slot_ptrs);
+}
+
 PyObject* dk_ffn_tail(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) try {
   ARGS("dk_ffn_tail", 5, S_pool, S_norm2, S_sel, S_w, S_clamp, S_shared, S_moe);
   const at::Tensor &x = tensor(a[1]), &sel = tensor(a[2]);
   const long long d = attr_int(a[0], S_d), ff = attr_int(a[0], S_ff), k = sel.numel();
-  if (!plain(x, at::kFloat) || !plain(sel, at::kInt) || x.numel() != d || d % 256 || ff % 256 || k < 1)
+  if (!plain(x, at::kFloat) || !plain(sel, at::kInt) || x.numel() != d || d % 256 || ff % 256 || k < 1 || !own_slots(a[0]))
     return PyObject_Vectorcall(slow(S_dk_ffn_tail), args, nargs, kwnames);
-  const long long gb = attr_int(a[0], S_gate_bytes), ne = attr_int(a[0], S_n_expert);
-  const ill_dptr ptrs = attr_ptr(a[0], S_ptrs_all), sp = ptr(a[2]);
+  const Ref table(PyObject_GetAttr(a[0], S_ptrs_all));
+  const at::Tensor& all = tensor(table.p);
+  if (!plain(all, at::kLong) || all.dim() != 1 || all.device() != sel.device())
+    return PyObject_Vectorcall(slow(S_dk_ffn_tail), args, nargs, kwnames);
+  const long long gb = attr_int(a[0], S_gate_bytes), ne = all.numel();
+  const ill_dptr ptrs = ptr(table.p), sp = ptr(a[2]);
   const ill_stream st = cur_stream();
   const auto f32 = x.options().requires_grad(false);
   Scratch s(x, d + d / 64 + d / 8 + k * (ff + ff / 64 + ff / 8) + 4 * k * d + 8 * 256);

@@ -141,4 +141,5 @@ def _dk_ffn_tail(pool, norm2, sel, w, clamp, shared=None, moe=None):
 # and share a name with one are what it leaves to Python.
 _H = _lib.hostops()
 dk_mv16, route, dk_shared, dk_ffn_tail = (getattr(_H, f) for f in ("dk_mv16", "route", "dk_shared", "dk_ffn_tail"))
-D._SLOW.update({"dk_mv16": _dk_mv16, "route": _route, "dk_shared": _dk_shared, "dk_ffn_tail": _dk_ffn_tail})
+D._SLOW.update({"dk_mv16": _dk_mv16, "route": _route, "dk_shared": _dk_shared, "dk_ffn_tail": _dk_ffn_tail,
+                "slot_ptrs": ExpertPool.slot_ptrs})

@@ -1,5 +1,7 @@
 """The one-token expert products by the router's choice (ill_moe_glu_sel, ill_moe_mv_sel): the bits of the same products given a table
 of the chosen experts' addresses; numbers from the end; a number out of range stays inside the pool and raises the status word."""
+import dataclasses
+
 import numpy as np
 import pytest
 import torch
@@ -70,3 +72,39 @@ def test_native_operators_leave_other_forms_to_python(layer):
     for other in (sel.long(), torch.stack([sel, sel], dim=1)[:, 0]):  # 64-bit numbers, numbers apart
         m2, mid2 = M.dk_ffn_tail(pool, x, other, w, 10.0)
         assert torch.equal(moe, m2) and torch.equal(mid, mid2)
+
+
+class Reversed(M.ExpertPool):
+    def slot_ptrs(self, experts):
+        return self.ptrs_all.flip(0)[experts.long()]
+
+
+class Slots:
+    """A caller's own pool: the experts' addresses by slot_ptrs() alone."""
+
+    def __init__(self, pool):
+        self.d, self.ff, self.gate_fmt, self.down_fmt, self.gate_bytes = pool.d, pool.ff, pool.gate_fmt, pool.down_fmt, pool.gate_bytes
+        self.slot_ptrs = lambda experts: pool.slot_ptrs(experts)
+
+
+@pytest.mark.parametrize("kind", ["subclass", "object", "instance", "longer table", "table apart"])
+def test_a_pool_of_the_callers_own(layer, kind):
+    """The experts' addresses are those that the pool's slot_ptrs() gives."""
+    pool, _ = layer
+    x = torch.randn(pool.d, device="cuda")
+    w = torch.tensor([0.25, 0.75], device="cuda")
+    sel = torch.tensor([1, 3], dtype=torch.int32, device="cuda")
+    own, as_pool = dataclasses.replace(pool), sel
+    if kind == "subclass":
+        own, as_pool = Reversed(**vars(pool)), 4 - sel
+    elif kind == "object":
+        own = Slots(pool)
+    elif kind == "instance":
+        own.slot_ptrs, as_pool = (lambda experts: pool.slot_ptrs(4 - experts)), 4 - sel
+    elif kind == "longer table":
+        own.n_expert = 2
+    else:
+        own.ptrs_all = torch.stack([pool.ptrs_all, pool.ptrs_all + 1], dim=1)[:, 0]
+    want, got = M.dk_ffn_tail(pool, x, as_pool, w, 10.0), M.dk_ffn_tail(own, x, sel, w, 10.0)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert D.device_status() == 0
