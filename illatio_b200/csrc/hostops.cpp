@@ -235,7 +235,9 @@ void mul_any(PyObject* w, PyObject* act, PyObject* y, long long n, PyObject* bia
 // Up to three products of up to 16 tokens that share the activations, in one launch (C null: two); false where that is not to be had
 inline bool mul_3(const Mat& a, const Mat& b, const Mat* c, const Act& x, ill_dptr ya, ill_dptr yb, ill_dptr yc, ill_dptr ba, ill_dptr bb,
                   ill_dptr bc, int n) {
-  // (a Q8_0 matrix takes other activations than the K formats: not with them)
+  // (a Q8_0 matrix takes other activations than the K formats: not with them; a third of no rows, which ill_mv_3n would take for
+  // none, is refused by the product of its own)
+  if (c && c->rows < 1) return false;
   if ((a.type == 0) != (b.type == 0) || a.cols != b.cols || (c && ((c->type == 0) != (a.type == 0) || c->cols != a.cols))) return false;
   const int rc = launch(ill_mv_3n, a.type, b.type, c ? c->type : 0, a.w, b.w, c ? c->w : 0, a.rows, b.rows, c ? c->rows : 0, a.cols, x.xq, x.xs, x.k ? x.xsum : 0, ya, yb,
                         yc, ba, bb, bc, n, cur_stream());

@@ -130,3 +130,16 @@ def test_few_tokens_against_the_oracle(oracle, cuda_lib, fmt, rows, cols, n):
     # whole-number block sums: what differs is the order of at most 152 32-bit additions
     err, _ = rel_errors(y.cpu().numpy().reshape(n, rows), np.stack(want))
     assert err <= 1e-5
+
+
+@pytest.mark.parametrize("fmt", [B.Q8_0, B.Q4_K])
+def test_a_third_matrix_of_no_rows_is_refused(cuda_lib, fmt):
+    """The entry point takes two matrices when the third has neither rows nor an address; the operator's three are three."""
+    cols, n = 256, 4
+    act = dev_act(fmt, np.ones(n * cols, np.float32))
+    m = D.upload_gmat(B.synth_matrix(fmt, 16, cols, seed=1), fmt, 16, cols)
+    none = D.CMat("", fmt, 0, cols, torch.empty(0, dtype=torch.uint8, device="cuda"))
+    y = [torch.zeros(n * 16, device="cuda") for _ in range(3)]
+    with pytest.raises(_lib.IllatioError) as e:
+        D.qkv_mul(m, m, none, act, *y, n=n)
+    assert e.value.code == 1
