@@ -446,9 +446,19 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
   }
 }
 
-template <int FMT, int FMT2, bool AL4>
-static int mvt_launch(const MtParams& p, size_t smem, int grid, cudaStream_t st) {
-  const void* k = p.n <= 8 ? (const void*)mvt_kernel<FMT, FMT2, 1, AL4> : (const void*)mvt_kernel<FMT, FMT2, 2, AL4>;
+// Registers a thread of the kernel, at most: what decides whether an SM holds two CTAs
+static int mt_regs(int fmt, int n) { return fmt == ILL_Q8_0 ? 96 : n <= 8 ? 112 : 128; }
+
+static const void* mt_kernel(int fmt, bool two, bool al4, int n) {
+#define MT_PICK(F, F2, A) (n <= 8 ? (const void*)mvt_kernel<F, F2, 1, A> : (const void*)mvt_kernel<F, F2, 2, A>)
+  if (fmt == ILL_Q8_0) return MT_PICK(ILL_Q8_0, ILL_Q8_0, false);
+  if (fmt == ILL_Q6_K) return MT_PICK(ILL_Q6_K, ILL_Q6_K, false);
+  if (two) return al4 ? MT_PICK(ILL_Q4_K, ILL_Q6_K, true) : MT_PICK(ILL_Q4_K, ILL_Q6_K, false);
+  return al4 ? MT_PICK(ILL_Q4_K, ILL_Q4_K, true) : MT_PICK(ILL_Q4_K, ILL_Q4_K, false);
+#undef MT_PICK
+}
+
+static int mvt_launch(const void* k, const MtParams& p, size_t smem, int grid, cudaStream_t st) {
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e);
@@ -572,9 +582,10 @@ static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n,
   off += (uint32_t)(p.groups * p.gw * p.stages) * p.stage_bytes;
   p.part_off = off;
   off += (uint32_t)p.groups * part_bytes;
-  // (two CTAs an SM where their registers fit too: up to 64 a thread, K formats up to 83 or 128)
-  const int threads = 32 * p.gw * p.groups, most2 = fmt == ILL_Q8_0 ? 512 : n <= 8 ? 384 : 256;
-  const int per_sm = (int)((227u * 1024u) / (off + 1024u)) >= 2 && threads <= most2 ? 2 : 1;
+  // Two CTAs an SM where their shared memory and registers fit: a grid of two an SM that holds one runs in two rounds, each with its
+  // activations to bring (Q8_0 of 16 warps a CTA, 4 tokens: 4096 x 256 4.5 us, 2.7 with one; 17408 x 256 7.6 / 6.4)
+  const int regs = 32 * p.gw * p.groups * mt_regs(fmt, n);
+  const int per_sm = (int)((227u * 1024u) / (off + 1024u)) >= 2 && 2 * regs <= 65536 ? 2 : 1;
   plan->grid = (int)((long long)sms * per_sm < ntiles ? (long long)sms * per_sm : ntiles);
   plan->smem = off;
   plan->fmt = fmt;
@@ -604,15 +615,7 @@ int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
   p.xs = (const float*)(uintptr_t)xs;
   p.xsum = (const int16_t*)(uintptr_t)xsum;
   p.acc = acc;
-  const size_t smem = plan.smem;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (plan.two)
-    return al4 ? mvt_launch<ILL_Q4_K, ILL_Q6_K, true>(p, smem, plan.grid, st) : mvt_launch<ILL_Q4_K, ILL_Q6_K, false>(p, smem, plan.grid, st);
-  switch (plan.fmt) {
-    case ILL_Q8_0: return mvt_launch<ILL_Q8_0, ILL_Q8_0, false>(p, smem, plan.grid, st);
-    case ILL_Q4_K: return al4 ? mvt_launch<ILL_Q4_K, ILL_Q4_K, true>(p, smem, plan.grid, st) : mvt_launch<ILL_Q4_K, ILL_Q4_K, false>(p, smem, plan.grid, st);
-    default: return mvt_launch<ILL_Q6_K, ILL_Q6_K, false>(p, smem, plan.grid, st);
-  }
+  return mvt_launch(mt_kernel(plan.fmt, plan.two, al4, n), p, plan.smem, plan.grid, (cudaStream_t)stream);
 }
 
 }  // namespace ill
@@ -637,5 +640,9 @@ extern "C" int ill_test_few_tokens_plan(int nmat, int fmt0, int fmt1, int fmt2, 
   out[3] = p.stages;
   out[4] = plan.grid;
   out[5] = (int)plan.smem;
+  out[6] = mt_regs(plan.fmt, n);
+  cudaFuncAttributes fa;
+  out[7] = cudaFuncGetAttributes(&fa, mt_kernel(plan.fmt, plan.two, true, n)) == cudaSuccess ? fa.numRegs : 0;
+  (void)cudaGetLastError();
   return ILL_OK;
 }

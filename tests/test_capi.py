@@ -77,7 +77,7 @@ def test_launches_of_few_tokens_stay_within_a_cta(fmt, n):
     row and the numbers of tiles around whole rounds of 148 SMs: short rows of many rows get up to sixteen groups."""
     two = isinstance(fmt, tuple)
     f = fmt if two else (fmt, 0)
-    out, seen = (ctypes.c_int * 6)(), set()
+    out, seen = (ctypes.c_int * 8)(), set()
     for blocks in list(range(1, 42)) + [48, 56, 57, 64, 68, 152, 256, 544]:
         cols = blocks * (32 if fmt == 0 else 256)
         for rounds in list(range(1, 20)) + [31, 32, 33, 47, 48, 49, 64, 110]:
@@ -85,9 +85,10 @@ def test_launches_of_few_tokens_stay_within_a_cta(fmt, n):
                 rc = _lib.status("ill_test_few_tokens_plan", 2 if two else 1, f[0], f[1], 0, rows, rows if two else 0, 0, cols, n, 148, out)
                 assert rc in (0, 3)
                 if rc == 0:
-                    warps, groups, barrier, stages, ctas, smem = out
+                    warps, groups, barrier, stages, ctas, smem, regs, _ = out
                     seen.add((warps, groups))
                     assert warps >= 1 and groups >= 1 and warps * groups <= 16 and 2 <= stages <= 4 and ctas >= 1
                     assert 0 <= barrier <= 15 and (warps == 1) == (barrier == 0)
-                    assert smem <= 227 * 1024
+                    per_sm = 1 if ctas <= 148 else 2
+                    assert ctas <= 296 and per_sm * (smem + 1024) <= 228 * 1024 and per_sm * 32 * warps * groups * regs <= 65536
     assert (1, 16) in seen

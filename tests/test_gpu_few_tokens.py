@@ -63,7 +63,7 @@ def test_matrices_in_one_launch_give_each_ones_bits(cuda_lib, fmts, rows, cols, 
 def test_short_rows_of_many(cuda_lib, fmt, rows, cols, n):
     """Sixteen groups of one warp a CTA (short rows whose tiles nearly fill the rounds): the bits of launches of some of the rows, which
     have other groups."""
-    out = (ctypes.c_int * 6)()
+    out = (ctypes.c_int * 8)()
     assert _lib.status("ill_test_few_tokens_plan", 1, fmt, 0, 0, rows, 0, 0, cols, n, 148, out) == 0 and list(out[:3]) == [1, 16, 0]
     act = dev_act(fmt, np.random.default_rng(rows).standard_normal(n * cols).astype(np.float32))
     w, keep, ptr = _mat(fmt, rows, cols, 5, 0)
@@ -143,3 +143,11 @@ def test_a_third_matrix_of_no_rows_is_refused(cuda_lib, fmt):
     with pytest.raises(_lib.IllatioError) as e:
         D.qkv_mul(m, m, none, act, *y, n=n)
     assert e.value.code == 1
+
+
+@pytest.mark.parametrize("fmts", [(B.Q8_0,), (B.Q4_K,), (B.Q6_K,), (B.Q4_K, B.Q6_K)])
+@pytest.mark.parametrize("n", [8, 16])
+def test_registers_are_what_the_choice_of_ctas_takes_them_for(cuda_lib, fmts, n):
+    out = (ctypes.c_int * 8)()
+    assert _lib.status("ill_test_few_tokens_plan", len(fmts), fmts[0], fmts[-1], 0, 64, 64 if len(fmts) > 1 else 0, 0, 1024, n, 148, out) == 0
+    assert 0 < out[7] <= out[6]  # (registers are given out eight a thread at a time)
