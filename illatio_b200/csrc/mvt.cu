@@ -555,7 +555,9 @@ static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n,
   // Warps a group and groups a CTA, for the least time: the tiles a group takes one after another, times the blocks of its busiest
   // warp, times what a block takes with that many warps an SM (a latency of 24, and 1 a warp).  The rings are as deep as fits (four
   // stages at most, two at least).  Swept over every pair on nine launches of a 0.5B, a 4B and a 27B model at 2, 4 and 16 tokens: the
-  // fastest pair or one within 5 % of it but for a head of 151936 x 2560 at two tokens (10 %).
+  // fastest pair or one within 5 % of it but for a head of 151936 x 2560 at two tokens (10 %).  Short rows have few warps a group: such
+  // a CTA takes groups without a tile up to eight warps, for the activations' sake (1024 x 256, 16 tokens, a warp / eight: Q6_K 4.9 / 3.4
+  // us, Q4_K 4.6 / 2.9; over 1050 shapes of up to 1280 columns 6 % on average, 11 % slower at most, of 2.6 us).
   const uint32_t budget = 226u * 1024u, part_bytes = 2u * p.nsums * ntok * 20 * 4;
   double best = 0;
   for (int gw = p.nsums; gw >= 1; --gw) {
@@ -564,10 +566,12 @@ static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n,
     for (int i = 0; i < (two ? 2 : 1); ++i) most[i] = mt_deal(p.f[i].npieces, gw, sums[i]) * p.f[i].cb;
     const uint32_t ring1 = (uint32_t)gw * p.stage_bytes;
     for (int g = MT_MAX_WARPS / gw; g >= 1; --g) {
-      if (g > 1 && (g - 1) * sms >= ntiles) continue;      // (fewer groups have a tile each already)
+      // (fewer groups have a tile each already, and with eight warps there are enough to bring the activations)
+      if (g > 1 && (g - 1) * sms >= ntiles && (g - 1) * gw >= 8) continue;
       if (off + g * (part_bytes + 2 * ring1) > budget) continue;
       const long long rounds = (ntiles + (long long)g * sms - 1) / ((long long)g * sms);
-      const double a_tile = (double)(tiles[0] * most[0] + tiles[1] * most[1]) / ntiles, cost = rounds * a_tile * (24 + g * gw);
+      const long long busy = (ntiles + sms - 1) / sms;     // groups of a CTA that have a tile, at most
+      const double a_tile = (double)(tiles[0] * most[0] + tiles[1] * most[1]) / ntiles, cost = rounds * a_tile * (24 + (g < busy ? g : busy) * gw);
       if (p.groups && cost >= best) continue;
       best = cost;
       p.groups = g;

@@ -81,7 +81,7 @@ def test_launches_of_few_tokens_stay_within_a_cta(fmt, n):
     for blocks in list(range(1, 42)) + [48, 56, 57, 64, 68, 152, 256, 544]:
         cols = blocks * (32 if fmt == 0 else 256)
         for rounds in list(range(1, 20)) + [31, 32, 33, 47, 48, 49, 64, 110]:
-            for rows in (16 * 148 * rounds - 1600, 16 * 148 * rounds, 16 * 148 * rounds + 1):
+            for rows in (16 * rounds, 16 * 148 * rounds - 1600, 16 * 148 * rounds, 16 * 148 * rounds + 1):
                 rc = _lib.status("ill_test_few_tokens_plan", 2 if two else 1, f[0], f[1], 0, rows, rows if two else 0, 0, cols, n, 148, out)
                 assert rc in (0, 3)
                 if rc == 0:
@@ -89,6 +89,7 @@ def test_launches_of_few_tokens_stay_within_a_cta(fmt, n):
                     seen.add((warps, groups))
                     assert warps >= 1 and groups >= 1 and warps * groups <= 16 and 2 <= stages <= 4 and ctas >= 1
                     assert 0 <= barrier <= 15 and (warps == 1) == (barrier == 0)
+                    assert warps * groups >= 8 or cols > 1280  # (all warps bring the activations)
                     per_sm = 1 if ctas <= 148 else 2
                     assert ctas <= 296 and per_sm * (smem + 1024) <= 228 * 1024 and per_sm * 32 * warps * groups * regs <= 65536
     assert (1, 16) in seen
