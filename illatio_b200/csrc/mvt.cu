@@ -557,7 +557,7 @@ static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n,
   // stages at most, two at least).  Swept over every pair on nine launches of a 0.5B, a 4B and a 27B model at 2, 4 and 16 tokens: the
   // fastest pair or one within 5 % of it but for a head of 151936 x 2560 at two tokens (10 %).  Short rows have few warps a group: such
   // a CTA takes groups without a tile up to eight warps, for the activations' sake (1024 x 256, 16 tokens, a warp / eight: Q6_K 4.9 / 3.4
-  // us, Q4_K 4.6 / 2.9; over 1050 shapes of up to 1280 columns 6 % on average, 11 % slower at most, of 2.6 us).
+  // us, Q4_K 4.6 / 3.1; over 1050 shapes of up to 1280 columns 6 % on average, 11 % slower at most, of 2.6 us).
   const uint32_t budget = 226u * 1024u, part_bytes = 2u * p.nsums * ntok * 20 * 4;
   double best = 0;
   for (int gw = p.nsums; gw >= 1; --gw) {
@@ -629,13 +629,13 @@ using namespace ill;
 extern "C" int ill_test_few_tokens_plan(int nmat, int fmt0, int fmt1, int fmt2, int rows0, int rows1, int rows2, int cols, int n, int sms,
                                         int* out) {
   const int fmts[3] = {fmt0, fmt1, fmt2}, rows[3] = {rows0, rows1, rows2};
-  if (!out || nmat < 1 || nmat > MT_MATS || cols <= 0 || sms < 1) return ILL_ERR_ARG;
+  if (!out || nmat < 1 || nmat > MT_MATS || cols <= 0 || sms < 0) return ILL_ERR_ARG;
   for (int i = 0; i < nmat; ++i) {
     const int bw = fmt_block_weights(fmts[i]);
     if (!bw || rows[i] <= 0 || cols % bw) return ILL_ERR_ARG;
   }
   MtPlan plan;
-  const int rc = mvt_plan(nmat, fmts, rows, cols, n, sms, &plan);
+  const int rc = mvt_plan(nmat, fmts, rows, cols, n, sms ? sms : 148, &plan);
   if (rc) return rc;
   const MtParams& p = plan.p;
   out[0] = p.gw;
@@ -645,8 +645,12 @@ extern "C" int ill_test_few_tokens_plan(int nmat, int fmt0, int fmt1, int fmt2, 
   out[4] = plan.grid;
   out[5] = (int)plan.smem;
   out[6] = mt_regs(plan.fmt, n);
-  cudaFuncAttributes fa;
-  out[7] = cudaFuncGetAttributes(&fa, mt_kernel(plan.fmt, plan.two, true, n)) == cudaSuccess ? fa.numRegs : 0;
-  (void)cudaGetLastError();
+  out[7] = 0;
+  if (!sms) {
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, mt_kernel(plan.fmt, plan.two, true, n));
+    if (e != cudaSuccess) return cuda_fail(e);
+    out[7] = fa.numRegs;
+  }
   return ILL_OK;
 }

@@ -149,5 +149,5 @@ def test_a_third_matrix_of_no_rows_is_refused(cuda_lib, fmt):
 @pytest.mark.parametrize("n", [8, 16])
 def test_registers_are_what_the_choice_of_ctas_takes_them_for(cuda_lib, fmts, n):
     out = (ctypes.c_int * 8)()
-    assert _lib.status("ill_test_few_tokens_plan", len(fmts), fmts[0], fmts[-1], 0, 64, 64 if len(fmts) > 1 else 0, 0, 1024, n, 148, out) == 0
+    assert _lib.status("ill_test_few_tokens_plan", len(fmts), fmts[0], fmts[-1], 0, 64, 64 if len(fmts) > 1 else 0, 0, 1024, n, 0, out) == 0
     assert 0 < out[7] <= out[6]  # (registers are given out eight a thread at a time)
