@@ -16,8 +16,8 @@ unsigned int* device_status_word();
 bool pdl_enabled();
 
 // Launch FN (grid, block, dynamic shared bytes) on ST with ARGS, with the
-// programmatic-dependent-launch attribute when enabled.
-int launch_kernel(const void* fn, dim3 grid, dim3 block, size_t smem, void** args, cudaStream_t st);
+// programmatic-dependent-launch attribute when enabled, in clusters of CLUSTER CTAs.
+int launch_kernel(const void* fn, dim3 grid, dim3 block, size_t smem, void** args, cudaStream_t st, int cluster = 1);
 
 enum { MODE_PLAIN = 0, MODE_GLU = 1, MODE_MOE_GLU = 2,
        MODE_PEERS = 3 /* a plain one-token product whose results go to every rank's buffer, then the ranks meet */ };

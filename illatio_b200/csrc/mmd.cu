@@ -341,15 +341,13 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
 }
 
 // ---- up to sixteen tokens of rows too long for mvt.cu to keep the activations resident ------------------------
-// A 16-row tile's column steps are dealt to eight warps (warp w takes steps w, w + 8, ...) in the four CTAs of a cluster, two each: each
-// warp streams its own steps' weights (its ring of three stages) AND its own steps' activations (two buffers of its own), all
+// A 16-row tile's column steps are dealt to eight warps (warp w takes steps w, w + 8, ...), in one CTA or, two each, in the four CTAs of a
+// cluster: each warp streams its own steps' weights (its ring of three stages) AND its own steps' activations (two buffers of its own), all
 // by 16-byte cp.async of its lanes (Q6_K 5120 x 17408, 4 tokens: 40 us; 59 with a bulk copy a row segment), so the warps
-// never wait for one another until the end, where their partial sums are read from the four CTAs' shared memory in warp order.  A matrix
+// never wait for one another until the end, where their partial sums are read, from the four CTAs' shared memory, in warp order.  A matrix
 // of few rows and many columns (5120 x 17408) thus fills the machine where the chunk kernel above would run two warps a CTA
-// through all 68 steps.  With the eight warps in one CTA, which takes most of an SM's shared memory, 160 tiles were two rounds on 148
-// SMs and 320 three; CTAs of two warps spread over the SMs to a quarter of a tile.  us, one CTA a tile / a cluster, weights cold, launches
-// one behind the other: Q6_K 2560 x 9728, 16 tokens 19.8 / 15.1; 5120 x 17408, 4 tokens 40.6 / 34.7, 16 tokens 47.5 / 41.5; Q4_K
-// 5120 x 17408, 16 tokens 44.0 / 39.2.
+// through all 68 steps.  Eight warps in one CTA take most of an SM's shared memory, so 160 tiles are two rounds on 148
+// SMs and 320 three; CTAs of two warps spread over the SMs to a quarter of a tile, but meet through the cluster (mk_cluster says which).
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
@@ -364,15 +362,16 @@ __device__ __forceinline__ float ld_cluster(const float* p, int rank) {
 
 constexpr int MK_PP = 20;  // floats between the tokens of a partial sum: a fragment's stores lie on different banks
 
-template <int FMT, int NT8, int CTAS /* of a tile */>
-__device__ __forceinline__ void mmk_body(const MdParams& p, u8* smem) {
+template <int FMT, int NT8, int CTAS /* of a tile: a cluster, where more than one */>
+__global__ void __launch_bounds__(MD_THREADS / CTAS, 1) mmk_kernel(const MdParams p) {
+  extern __shared__ __align__(128) u8 smem[];
   constexpr int WARPS = MD_WARPS / CTAS;
   constexpr int TN = 8 * NT8, SB = MdFrag<FMT>::SB, SP = MdFrag<FMT>::SPITCH;
   constexpr bool KQ = FMT != ILL_Q8_0;
   const int tid = threadIdx.x, lane = tid & 31, cwarp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int rank = blockIdx.x % CTAS, tile = blockIdx.x / CTAS, warp = rank * WARPS + cwarp;
+  const int rank = (int)(blockIdx.x % CTAS), warp = rank * WARPS + cwarp;
   const int ntt = (p.n + TN - 1) / TN;
-  const int tok0 = (tile % ntt) * TN, row_base = (tile / ntt) * 16;
+  const int tok0 = (int)(blockIdx.x / CTAS % ntt) * TN, row_base = (int)(blockIdx.x / CTAS / ntt) * 16;
   const int nsteps = p.nsteps;
   u8* xw = smem + (size_t)cwarp * 2 * p.xbuf_bytes;  // this warp's two activation buffers
   u8* ring = smem + p.ring_off + (size_t)cwarp * MD_MAX_STAGES * p.stage_bytes;
@@ -491,17 +490,7 @@ __device__ __forceinline__ void mmk_body(const MdParams& p, u8* smem) {
   }
   if constexpr (CTAS > 1) cluster_sync();  // nobody's partial sums go before everyone has read them
 }
-template <int FMT, int NT8>
-__global__ void __launch_bounds__(MD_THREADS, 1) mmk_kernel(const MdParams p) {
-  extern __shared__ __align__(128) u8 smem[];
-  mmk_body<FMT, NT8, 1>(p, smem);
-}
 constexpr int MK_CTAS = 4;
-template <int FMT, int NT8>
-__global__ void __cluster_dims__(MK_CTAS, 1, 1) __launch_bounds__(MD_THREADS / MK_CTAS) mmk_cluster_kernel(const MdParams p) {
-  extern __shared__ __align__(128) u8 smem[];
-  mmk_body<FMT, NT8, MK_CTAS>(p, smem);
-}
 
 template <int FMT>
 static int mmd_launch(const MdParams& p, int tn, size_t smem, int grid, cudaStream_t st) {
@@ -577,14 +566,27 @@ int mmd_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
 
 template <int FMT>
 static int mmk_launch(const MdParams& p, int tn, int ctas, size_t smem, int grid, cudaStream_t st) {
-  const void* k = tn == 8 ? (const void*)mmk_cluster_kernel<FMT, 1> : (const void*)mmk_cluster_kernel<FMT, 2>;
-  if constexpr (FMT == ILL_Q4_K)
-    if (ctas == 1) k = (const void*)mmk_kernel<FMT, 1>;
+  const void* k = ctas == 1 ? tn == 8 ? (const void*)mmk_kernel<FMT, 1, 1> : (const void*)mmk_kernel<FMT, 2, 1>
+                            : tn == 8 ? (const void*)mmk_kernel<FMT, 1, MK_CTAS> : (const void*)mmk_kernel<FMT, 2, MK_CTAS>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e);
   MdParams pp = p;
   void* args[] = {&pp};
-  return launch_kernel(k, dim3(grid), dim3(32 * MD_WARPS / ctas), smem, args, st);
+  return launch_kernel(k, dim3(grid), dim3(32 * MD_WARPS / ctas), smem, args, st, ctas);
+}
+
+// Whether a tile goes to a cluster of four CTAs and not to one.  Four SMs work on a tile where there are few, up to two sevenths of the
+// SMs, and quarters of a tile fill a last round that is less than 45 % full; else the cluster's meeting, and SMs with CTAs of several
+// tiles, cost more than they give.  Two CTAs a tile of Q4_K fit an SM with up to eight tokens, and with more Q8_0's cluster kernel is the
+// slower: those take clusters for few tiles only.  us, one CTA / a cluster, 17408 columns, weights cold: Q6_K, 16 tokens, 16 tiles
+// 15.2 / 10.6, 36 15.4 / 13.2, 64 15.6 / 18.8, 148 17.8 / 23.5, 149 30.3 / 23.6, 200 32.5 / 31.2, 280 34.3 / 38.1, 310 48.7 / 41.4;
+// Q4_K, 4 tokens, 16 tiles 12.4 / 9.6, 148 12.9 / 19.6, 280 20.6 / 23.1; Q8_0, 16 tokens, 11008 columns, 16 tiles 19.8 / 18.0, 148
+// 22.6 / 40.5, 280 44.2 / 47.1.
+static bool mk_cluster(int fmt, int tn, long long tiles, int sms) {
+  if (tiles <= sms) return 7 * tiles <= 2 * sms;
+  if (fmt == ILL_Q4_K ? tn == 8 : fmt == ILL_Q8_0 && tn == 16) return false;
+  const long long last = (tiles - 1) % sms + 1;
+  return 20 * last <= 9 * sms;
 }
 
 // Up to sixteen tokens with the columns dealt to a CTA's warps (mmk_kernel): for rows of many columns.
@@ -623,8 +625,10 @@ int mmk_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
   p.xsum_off = off;
   if (fmt == ILL_Q4_K) off += (uint32_t)tn * MdFrag<ILL_Q4_K>::SPITCH;
   p.xbuf_bytes = (off + 127) / 128 * 128;
-  // One CTA a tile where two of them fit an SM (Q4_K, up to eight tokens: 5120 x 17408 28 us, a cluster of four 30)
-  const int ctas = fmt == ILL_Q4_K && tn == 8 ? 1 : MK_CTAS, warps = MD_WARPS / ctas;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+  const int ctas = mk_cluster(fmt, tn, (rows + 15) / 16, sms) ? MK_CTAS : 1, warps = MD_WARPS / ctas;
   p.ring_off = 2 * warps * p.xbuf_bytes;
   p.part_off = (uint32_t)((p.ring_off + (size_t)warps * MD_MAX_STAGES * p.stage_bytes + 127) / 128 * 128);
   const size_t smem = p.part_off + (size_t)warps * MK_PP * tn * 4;

@@ -151,3 +151,27 @@ def test_registers_are_what_the_choice_of_ctas_takes_them_for(cuda_lib, fmts, n)
     out = (ctypes.c_int * 8)()
     assert _lib.status("ill_test_few_tokens_plan", len(fmts), fmts[0], fmts[-1], 0, 64, 64 if len(fmts) > 1 else 0, 0, 1024, n, 0, out) == 0
     assert 0 < out[7] <= out[6]  # (registers are given out eight a thread at a time)
+
+
+@pytest.mark.parametrize("fmt", [B.Q8_0, B.Q4_K, B.Q6_K])
+@pytest.mark.parametrize("n", [4, 16])
+def test_long_rows_in_one_cta_and_in_a_cluster(cuda_lib, fmt, n):
+    """Rows too long for their activations to stay in shared memory: a tile of sixteen rows in one CTA (100 tiles: a round of the SMs more
+    than half full; 250) or in a cluster of four (10 tiles; 160), the same bits."""
+    cols, rows = (17408 if n == 4 else 11008), 4000
+    out = (ctypes.c_int * 8)()
+    assert _lib.status("ill_test_few_tokens_plan", 1, fmt, 0, 0, rows, 0, 0, cols, n, 148, out) == 3
+    act = dev_act(fmt, np.random.default_rng(n).standard_normal(n * cols).astype(np.float32))
+    w, keep, ptr = _mat(fmt, rows, cols, 5, 0)
+
+    def mul(row0, count):
+        y = torch.full((n * count + 8,), 7.0, device="cuda")
+        _lib.call("ill_mv", fmt, ptr + row0 * B.row_bytes(fmt, cols), count, cols, act.xq.data_ptr(), act.xs.data_ptr(),
+                  0 if act.kind == "q8" else act.xsum.data_ptr(), y.data_ptr(), 0, 0, n, _lib.stream())
+        assert (y[n * count:] == 7.0).all()
+        return y[:n * count].view(n, count)
+
+    got = mul(0, rows)
+    for row0, count in ((0, 160), (160, 1600), (1440, 2560), (3999, 1)):
+        assert torch.equal(got[:, row0:row0 + count], mul(row0, count))
+    assert D.device_status() == 0
