@@ -23,7 +23,7 @@
 // 512 issue slots a scheduler for 128 x 128 x 32 where the product itself takes 64 cycles (the packed f32x2 forms take two slots
 // each); with the loads of the scales, the hand-overs and the unpacking 830 are executed, at 78 % issue about 1100 cycles.  us, int8
 // mma.sync (the kernel before) / now: 896 x 896 x 777 tokens 14.9 / 11.1, 896 x 4864 x 777 67 / 43, 4864 x 896 x 777 38 / 36,
-// 2048 x 4096 x 64 25 / 20, x 200 60 / 26, x 4096 297 / 288, 4096 x 2048 x 4096 298 / 277, 1536 x 5120 x 8192 548 / 548.
+// 2048 x 4096 x 64 25 / 20, x 200 60 / 26, x 4096 297 / 288, 4096 x 2048 x 4096 298 / 277, 1536 x 5120 x 8192 550 / 570.
 // Measured and taken back: eight drain warps with the next half on its way while one is scaled (NT 128: 309 -> 398); 16 x 256-bit
 // loads of tensor memory, a quarter of the shared memory's traffic (309 -> 319: it was no bound); raw blocks by cp.async of the
 // warps that take them apart (a step 0.5 -> 1.1 us); even shares whatever the rounds (4864 x 896 x 200 13.6 -> 16.3).
@@ -437,6 +437,37 @@ static bool byte_map(CUtensorMap* map, uint64_t base, uint64_t bytes, uint64_t r
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Which tiles: BM tokens each, one after another or (SHARE not 0) in even shares of SHARE columns of 16 tokens
+struct MqDeal {
+  int bm, share, grid;
+};
+static MqDeal mq_deal(int rows, int n, int sms) {
+  MqDeal d = {};
+  const long long ntr = (rows + MQ_ROWS - 1) / MQ_ROWS, cols16 = ntr * ((n + 15) / 16);
+  // Tokens a tile: the rounds of tiles on the SMs times a tile's time a step, us, over 21 matrices at 17 to 8192 tokens.  A step's
+  // hand-overs cost 16 tokens as much as its arithmetic; above 64 tokens a block is a job of its own.  The choice takes the
+  // fastest of them or one that is 0.3 % slower on average, 9 % at most.
+  static const float step_us[8] = {0.63f, 0.79f, 1.14f, 1.27f, 2.02f, 2.10f, 2.34f, 2.38f};
+  float best = 1e30f;
+  long long tiles = 0, rounds = 0;
+  for (int bm = 16; bm <= 128; bm += 16) {
+    const long long count = ntr * ((n + bm - 1) / bm), r = (count + sms - 1) / sms;
+    const float us = (float)r * step_us[bm / 16 - 1];
+    if (us < best) { best = us; d.bm = bm; tiles = count; rounds = r; }
+  }
+  d.grid = (int)(tiles < sms ? tiles : sms);
+  // Even shares instead of a last round that is half empty, for tiles of 64 tokens, three a share at least: the tile more at a share's
+  // ends costs what less than 15 % off the rounds saves.  us, rounds / shares: 9728 x 2560 x 512 tokens (4.1 rounds) 130 / 123, x 400
+  // (3.6) 104 / 97, 17408 x 5120 x 400 (6.4) 352 / 340; where less is to be saved 36000 x 1024 x 300 (9.5) 109 / 115.  Other tiles gain nothing (128 tokens:
+  // 5120 x 1536 x 4096 259 / 273; 32: 151936 x 896 x 32 61 / 61).
+  const long long share = (cols16 + sms - 1) / sms;
+  if (d.bm == 64 && share >= 12 && 1.15 * (double)share < 4.0 * (double)rounds) {
+    d.share = (int)share;
+    d.grid = (int)((cols16 + share - 1) / share);
+  }
+  return d;
+}
+
 // N tokens of a Q8_0 matrix; ILL_ERR_UNSUPPORTED for what it is not written for.
 int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t y, uint64_t bias, int acc, int n, void* stream) {
   if (n < 2 || cols % MQ_STEP || (xq & 15) || (xs & 15) || (w & 1)) return ILL_ERR_UNSUPPORTED;
@@ -453,27 +484,12 @@ int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t
   p.acc = acc;
   p.n = n;
   p.status = device_status_word();
-  const long long ntr = (rows + MQ_ROWS - 1) / MQ_ROWS, ncol = (n + 15) / 16;
-  if (ntr * ncol > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
-  // Tokens a tile: the rounds of tiles on the SMs times a tile's measured time a step, us (2048 rows x 4096 columns, every SM busy).
-  // A step's hand-overs cost 16 tokens as much as its arithmetic; above 64 tokens a block is a job of its own.
-  static const float step_us[8] = {0.54f, 0.71f, 1.09f, 1.27f, 2.06f, 2.08f, 2.41f, 2.43f};
-  float best = 1e30f;
-  long long tiles = 0;
-  for (int bm = 16; bm <= 128; bm += 16) {
-    const long long count = ntr * ((n + bm - 1) / bm), rounds = (count + sms - 1) / sms;
-    const float us = (float)rounds * step_us[bm / 16 - 1];
-    if (us < best) { best = us; p.bm = bm; tiles = count; }
-  }
-  int grid = (int)(tiles < sms ? tiles : sms);
-  if (tiles > 8ll * sms) {
-    // many rounds: even shares instead of a last round that is half empty (1536 x 5120 x 8192 tokens, 11 rounds for 10.4:
-    // 562 -> 543 us; with fewer rounds the tile more at a share's ends costs what it saves)
-    p.bm = 64;
-    p.ncol = (int)ncol;
-    p.share = (int)((ntr * ncol + sms - 1) / sms);
-    grid = (int)((ntr * ncol + p.share - 1) / p.share);
-  }
+  if ((long long)((rows + MQ_ROWS - 1) / MQ_ROWS) * ((n + 15) / 16) > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
+  const MqDeal d = mq_deal(rows, n, sms);
+  p.bm = d.bm;
+  p.ncol = (n + 15) / 16;
+  p.share = d.share;
+  const int grid = d.grid;
   MqMaps maps;
   const uint64_t row_bytes = (uint64_t)cols / 32 * 34;
   if (!byte_map(&maps.x, xq, cols, n, cols, MQ_STEP, p.bm, true)) return cuda_fail(cudaErrorInvalidValue);
@@ -493,3 +509,14 @@ int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t
 }
 
 }  // namespace ill
+
+using namespace ill;
+
+extern "C" int ill_test_q8_chunk_plan(int rows, int n, int sms, int* out) {
+  if (!out || rows < 1 || n < 2 || sms < 1) return ILL_ERR_ARG;
+  const MqDeal d = mq_deal(rows, n, sms);
+  out[0] = d.bm;
+  out[1] = d.share;
+  out[2] = d.grid;
+  return ILL_OK;
+}

@@ -93,3 +93,13 @@ def test_launches_of_few_tokens_stay_within_a_cta(fmt, n):
                     per_sm = 1 if ctas <= 148 else 2
                     assert ctas <= 296 and per_sm * (smem + 1024) <= 228 * 1024 and per_sm * 32 * warps * groups * regs <= 65536
     assert (1, 16) in seen
+
+
+@pytest.mark.parametrize("rows,n,bm,shares", [(151936, 17, 32, False), (151936, 32, 32, False), (151552, 17, 32, False), (9728, 512, 64, True), (9700, 505, 64, True),
+                                              (17300, 399, 64, True), (36000, 300, 64, False), (5120, 3900, 128, False), (4096, 8192, 128, False),
+                                              (151936, 48, 48, False), (896, 777, 48, False)])
+def test_tiles_of_a_q8_0_chunk(rows, n, bm, shares):
+    """Few tokens of many rows keep the tile that their number asks for on both sides of eight rounds; even shares where they save enough."""
+    out = (ctypes.c_int * 3)()
+    assert _lib.status("ill_test_q8_chunk_plan", rows, n, 148, out) == 0
+    assert (out[0], out[1] != 0) == (bm, shares) and 1 <= out[2] <= 148

@@ -25,6 +25,7 @@ def _mat(fmt, rows, cols, seed, off):
 @pytest.mark.parametrize("fmts,rows,cols,n,off", [
     ((B.Q8_0, B.Q8_0, B.Q8_0), (896, 128, 130), 896, 2, 2),
     ((B.Q8_0, B.Q8_0), (17, 1), 32, 16, 0),            # one block a row: one partial sum
+    ((B.Q8_0, B.Q8_0), (128, 128), 128, 2, 0),
     ((B.Q8_0, B.Q8_0), (300, 300), 4864, 9, 0),
     ((B.Q4_K, B.Q4_K, B.Q4_K), (257, 16, 15), 256, 3, 0),
     ((B.Q4_K, B.Q4_K), (2000, 2000), 2560, 16, 0),     # five partial sums

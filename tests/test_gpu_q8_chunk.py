@@ -20,8 +20,11 @@ pytestmark = pytest.mark.gpu
     (896, 1152, 777, 0, False, False),  # tiles of 48
     (384, 512, 1000, 14, True, True),
     (2048, 1024, 300, 0, False, False),
-    (5120, 128, 3900, 0, False, False),  # many rounds: even shares, tiles that end where a tile of rows does
-    (128, 128, 2, 0, False, False),
+    (5120, 128, 3900, 0, False, False),  # many rounds of tiles of 128
+    (9728, 128, 512, 0, False, False),  # even shares, tiles that end where a tile of rows or a share does
+    (9700, 128, 505, 2, True, True),
+    (17300, 256, 399, 0, False, True),
+    (151936, 128, 17, 0, False, False),  # many tiles of rows of few tokens
 ])
 def test_q8_0_chunk_bits(cuda_lib, rows, cols, n, off, acc, bias):
     g = torch.Generator(device="cuda")
