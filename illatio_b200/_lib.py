@@ -37,7 +37,7 @@ SIGNATURES = {
     "ill_test_wait_timeout": (_I, [_L, _P, _S]),
     "ill_test_poll_timeout": (_I, [_L, _c.c_uint32, _c.c_uint32, _P, _S]),
     "ill_test_few_tokens_plan": (_I, [_I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _c.POINTER(_I)]),
-    "ill_test_q8_chunk_plan": (_I, [_I, _I, _I, _c.POINTER(_I)]),
+    "ill_test_q8_chunk_plan": (_I, [_I, _I, _I, _I, _c.POINTER(_I)]),
     "ill_device_status": (_I, [_c.POINTER(_c.c_uint), _S]),
     "ill_quant_q8_0": (_I, [_P, _P, _P, _P, _L, _I, _S]),
     "ill_quant_q8_k": (_I, [_P, _P, _P, _P, _L, _S]),

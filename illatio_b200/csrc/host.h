@@ -40,8 +40,10 @@ int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
 // the same for a chunk of tokens (more than 16): mmd.cu
 int mmd_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum, uint64_t y, uint64_t bias, int acc,
             int n, void* stream);
-// ... of a Q8_0 matrix (mmd_try sends it there): mm_q8.cu
+// ... of a Q8_0 matrix (mmd_try sends it there): mm_q8.cu, which leaves some to mm_q8_i8.cu
 int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t y, uint64_t bias, int acc, int n, void* stream);
+int mm_q8_i8(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t y, uint64_t bias, int acc, int n, int sms, void* stream);
+float mm_q8_i8_step_us(int rows, int n, int sms);  // its estimate for 128 columns
 // up to 16 tokens of rows with many columns, the columns dealt to a CTA's warps: mmd.cu
 int mmk_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum, uint64_t y, uint64_t bias, int acc,
             int n, void* stream);

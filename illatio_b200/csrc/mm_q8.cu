@@ -437,9 +437,10 @@ static bool byte_map(CUtensorMap* map, uint64_t base, uint64_t bytes, uint64_t r
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Which tiles: BM tokens each, one after another or (SHARE not 0) in even shares of SHARE columns of 16 tokens
+// Which tiles: BM tokens each, one after another or (SHARE not 0) in even shares of SHARE columns of 16 tokens; a step's time, us
 struct MqDeal {
   int bm, share, grid;
+  float us;
 };
 static MqDeal mq_deal(int rows, int n, int sms) {
   MqDeal d = {};
@@ -456,6 +457,7 @@ static MqDeal mq_deal(int rows, int n, int sms) {
     if (us < best) { best = us; d.bm = bm; tiles = count; rounds = r; }
   }
   d.grid = (int)(tiles < sms ? tiles : sms);
+  d.us = best;
   // Even shares instead of a last round that is half empty, for tiles of 64 tokens, three a share at least: the tile more at a share's
   // ends costs what less than 15 % off the rounds saves.  us, rounds / shares: 9728 x 2560 x 512 tokens (4.1 rounds) 130 / 123, x 400
   // (3.6) 104 / 97, 17408 x 5120 x 400 (6.4) 352 / 340; where less is to be saved 36000 x 1024 x 300 (9.5) 109 / 115.  Other tiles gain nothing (128 tokens:
@@ -463,9 +465,20 @@ static MqDeal mq_deal(int rows, int n, int sms) {
   const long long share = (cols16 + sms - 1) / sms;
   if (d.bm == 64 && share >= 12 && 1.15 * (double)share < 4.0 * (double)rounds) {
     d.share = (int)share;
+    d.us = 1.10f * step_us[3] * (float)share / 4.0f;
     d.grid = (int)((cols16 + share - 1) / share);
   }
   return d;
+}
+
+// Whether the kernel on mma.sync is the faster one: by the two estimates, with 0.3 us for this kernel's start, and well enough for the
+// estimates' error.  Over 393 products of 21 matrices at 17 to 8192 tokens the choice takes the faster kernel or one within 3 % of it
+// for 358; of rows of 256 columns and more, 25 are slower by more, the most by 15 %.  Up to 32 tokens a tile holds all of them and this
+// kernel has it.  us, this kernel / that: 36000 x 1024 x 80 tokens 39.4 / 29.2, x 160 63.8 / 54.5, 17408 x 5120 x 160 147 / 130, 5120 x
+// 1536 x 512 42.4 / 39.4, 4864 x 896 x 512 26.1 / 24.2, x 777 36 / 38, 896 x 4864 x 777 43 / 67, 2048 x 4096 x 200 26 / 60.
+static bool mq_i8_is_faster(const MqDeal& d, int rows, int cols, int n, int sms) {
+  const float nsteps = (float)(cols / MQ_STEP);
+  return n > 32 && nsteps * mm_q8_i8_step_us(rows, n, sms) < 0.92f * (nsteps * d.us + 0.3f);
 }
 
 // N tokens of a Q8_0 matrix; ILL_ERR_UNSUPPORTED for what it is not written for.
@@ -486,6 +499,7 @@ int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t
   p.status = device_status_word();
   if ((long long)((rows + MQ_ROWS - 1) / MQ_ROWS) * ((n + 15) / 16) > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
   const MqDeal d = mq_deal(rows, n, sms);
+  if (mq_i8_is_faster(d, rows, cols, n, sms)) return mm_q8_i8(w, rows, cols, xq, xs, y, bias, acc, n, sms, stream);
   p.bm = d.bm;
   p.ncol = (n + 15) / 16;
   p.share = d.share;
@@ -512,11 +526,12 @@ int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t
 
 using namespace ill;
 
-extern "C" int ill_test_q8_chunk_plan(int rows, int n, int sms, int* out) {
-  if (!out || rows < 1 || n < 2 || sms < 1) return ILL_ERR_ARG;
+extern "C" int ill_test_q8_chunk_plan(int rows, int cols, int n, int sms, int* out) {
+  if (!out || rows < 1 || cols < MQ_STEP || n < 2 || sms < 1) return ILL_ERR_ARG;
   const MqDeal d = mq_deal(rows, n, sms);
   out[0] = d.bm;
   out[1] = d.share;
   out[2] = d.grid;
+  out[3] = mq_i8_is_faster(d, rows, cols, n, sms);
   return ILL_OK;
 }

@@ -1,5 +1,5 @@
 // The legacy tensor-core path for 8-bit integers (mma.sync m16n8k32 / m16n8k16) and the small loads around it,
-// shared by the several-token product (mvt.cu) and the dense chunk product (mmd.cu).
+// shared by the several-token product (mvt.cu) and the dense chunk products (mmd.cu, mm_q8_i8.cu).
 //
 // Fragment layout, lane = 4 g + t: A (16 rows x K): a0 = row g, k 4t..4t+3; a1 = row g + 8, same k; for k32 a2 / a3
 // the same rows at k + 16.  B (K x 8 columns): b0 = column g, k 4t..4t+3; b1 (k32) at k + 16.  C: c0 / c1 = row g,
@@ -29,6 +29,15 @@ __device__ __forceinline__ void mma_k16_u8(int (&c)[4], uint32_t a0, uint32_t a1
   asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                : "r"(a0), "r"(a1), "r"(b0));
+}
+
+// four 8 x 16-byte matrices of shared memory -> each lane its four bytes of row lane / 4 of each: lane l gives the
+// address of row l % 8 of matrix l / 8.  For a token tile's 64 bytes of quants this is the B fragment of two k32
+// (or four k16) steps: r[0], r[1] = b0, b1 of the first k32 step, r[2], r[3] of the second.
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(p)));
 }
 
 // a 32-bit word at any byte address of shared memory

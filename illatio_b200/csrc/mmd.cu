@@ -15,7 +15,7 @@
 // 33.6 / 19.7, 512 28.4 / 21.9, 2048 65.8 / 62.6; of Q6_K, 512 28.9 / 23.4; 1024 x 5120 of Q6_K, 512 56.3 / 45.1; 9728 x 2560 of Q4_K, 63
 // 56.1 / 45.3.)  Bound now by the chain of one warp's step where few rows and tokens leave a warp or two an SM (1.8 us a step: a
 // block's fragments, then its products), by instruction issue where they do not.
-// This is mmd_kernel, for Q4_K and Q6_K; Q8_0 has a kernel of its own (mm_q8.cu).
+// This is mmd_kernel, for Q4_K and Q6_K; Q8_0 has kernels of its own (mm_q8.cu, mm_q8_i8.cu).
 // Token tiles are the fastest-varying CTA index: the CTAs that share a tile of rows run together and the weights
 // come from HBM once.
 //
@@ -46,15 +46,6 @@ struct MdParams {
   uint32_t xbuf_bytes, xs_off, xsum_off;  // one activation buffer: its size, where its scales and (Q4_K) sums start
   uint32_t ring_off, part_off;
 };
-
-// four 8 x 16-byte matrices of shared memory -> each lane its four bytes of row lane / 4 of each: lane l gives the
-// address of row l % 8 of matrix l / 8.  For a token tile's 64 bytes of quants this is the B fragment of two k32
-// (or four k16) steps: r[0], r[1] = b0, b1 of the first k32 step, r[2], r[3] of the second.
-__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(p)));
-}
 
 // ---- a step's block(s) of 16 rows as tensor-core fragments, and their use against eight tokens ---------------
 // load(): ROW0 / ROW8 = the staged bytes of rows g and g + 8 (g = lane / 4), NB = valid blocks in the step.

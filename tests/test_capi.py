@@ -95,11 +95,13 @@ def test_launches_of_few_tokens_stay_within_a_cta(fmt, n):
     assert (1, 16) in seen
 
 
-@pytest.mark.parametrize("rows,n,bm,shares", [(151936, 17, 32, False), (151936, 32, 32, False), (151552, 17, 32, False), (9728, 512, 64, True), (9700, 505, 64, True),
-                                              (17300, 399, 64, True), (36000, 300, 64, False), (5120, 3900, 128, False), (4096, 8192, 128, False),
-                                              (151936, 48, 48, False), (896, 777, 48, False)])
-def test_tiles_of_a_q8_0_chunk(rows, n, bm, shares):
-    """Few tokens of many rows keep the tile that their number asks for on both sides of eight rounds; even shares where they save enough."""
-    out = (ctypes.c_int * 3)()
-    assert _lib.status("ill_test_q8_chunk_plan", rows, n, 148, out) == 0
-    assert (out[0], out[1] != 0) == (bm, shares) and 1 <= out[2] <= 148
+@pytest.mark.parametrize("rows,cols,n,bm,shares,i8", [
+    (151936, 896, 17, 32, False, False), (151936, 896, 32, 32, False, False), (151552, 896, 17, 32, False, False), (9728, 2560, 512, 64, True, False),
+    (9700, 2560, 505, 64, True, False), (17300, 5120, 399, 64, True, False), (4096, 2048, 8192, 128, False, False), (36000, 1024, 300, 64, False, False),
+    (151936, 896, 80, 80, False, True), (17408, 5120, 160, 64, False, True), (4864, 896, 512, 48, False, True), (896, 4864, 777, 48, False, False)])
+def test_tiles_of_a_q8_0_chunk(rows, cols, n, bm, shares, i8):
+    """Few tokens of many rows keep the tile that their number asks for on both sides of eight rounds; even shares where they save enough;
+    and which of the two kernels takes the chunk."""
+    out = (ctypes.c_int * 4)()
+    assert _lib.status("ill_test_q8_chunk_plan", rows, cols, n, 148, out) == 0
+    assert (out[0], out[1] != 0, bool(out[3])) == (bm, shares, i8) and 1 <= out[2] <= 148

@@ -1,4 +1,4 @@
-"""Q8_0 chunk products on tcgen05 (ill_mv of more than 16 tokens): tiles, ragged edges and rows at every alignment, bit for
+"""Q8_0 chunk products (ill_mv of more than 16 tokens; on tcgen05, some on mma.sync): tiles, ragged edges and rows at every alignment, bit for
 bit against the same sums taken block by block in plain PyTorch: y = y + float(isum) * (d_w * d_x), a rounding a step."""
 import pytest
 import torch
@@ -25,6 +25,14 @@ pytestmark = pytest.mark.gpu
     (9700, 128, 505, 2, True, True),
     (17300, 256, 399, 0, False, True),
     (151936, 128, 17, 0, False, False),  # many tiles of rows of few tokens
+    (127, 384, 29, 0, False, True),
+    (129, 256, 32, 0, True, True),
+    # chunks of the kernel on mma.sync (as the third and fourth, and 128 x 128 below)
+    (128, 128, 64, 0, False, False),
+    (1024, 128, 33, 0, True, True),
+    (20001, 256, 80, 2, False, True),
+    (4864, 896, 511, 4, True, False),
+    (5120, 1536, 301, 10, False, False),
 ])
 def test_q8_0_chunk_bits(cuda_lib, rows, cols, n, off, acc, bias):
     g = torch.Generator(device="cuda")
