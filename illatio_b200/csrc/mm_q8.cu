@@ -444,7 +444,7 @@ struct MqDeal {
 };
 static MqDeal mq_deal(int rows, int n, int sms) {
   MqDeal d = {};
-  const long long ntr = (rows + MQ_ROWS - 1) / MQ_ROWS, cols16 = ntr * ((n + 15) / 16);
+  const long long ntr = (rows + MQ_ROWS - 1) / MQ_ROWS;
   // Tokens a tile: the rounds of tiles on the SMs times a tile's time a step, us, over 21 matrices at 17 to 8192 tokens.  A step's
   // hand-overs cost 16 tokens as much as its arithmetic; above 64 tokens a block is a job of its own.  The choice takes the
   // fastest of them or one that is 0.3 % slower on average, 9 % at most.
@@ -459,14 +459,15 @@ static MqDeal mq_deal(int rows, int n, int sms) {
   d.grid = (int)(tiles < sms ? tiles : sms);
   d.us = best;
   // Even shares instead of a last round that is half empty, for tiles of 64 tokens, three a share at least: the tile more at a share's
-  // ends costs what less than 15 % off the rounds saves.  us, rounds / shares: 9728 x 2560 x 512 tokens (4.1 rounds) 130 / 123, x 400
-  // (3.6) 104 / 97, 17408 x 5120 x 400 (6.4) 352 / 340; where less is to be saved 36000 x 1024 x 300 (9.5) 109 / 115.  Other tiles gain nothing (128 tokens:
-  // 5120 x 1536 x 4096 259 / 273; 32: 151936 x 896 x 32 61 / 61).
-  const long long share = (cols16 + sms - 1) / sms;
-  if (d.bm == 64 && share >= 12 && 1.15 * (double)share < 4.0 * (double)rounds) {
+  // ends costs what less than 13 % off the rounds saves, or 4 % where a share is a third of a tile of rows at most.  us, rounds /
+  // shares: 9728 x 2560 x 512 tokens (4.1 rounds) 130 / 123, x 400 (3.6) 104 / 97, 17408 x 5120 x 400 (6.4) 352 / 340; 896 x 4864 x
+  // 8192 (6.1) 335 / 322, 1536 x 5120 x 8192 (10.4) 570 / 557; where less is to be saved 36000 x 1024 x 300 (9.5) 109 / 115, 5120 x 1536
+  // x 2048 (8.6) 143 / 150.  Other tiles gain nothing (128 tokens: 5120 x 1536 x 4096 259 / 273; 32: 151936 x 896 x 32 61 / 61).
+  const long long ncol = (n + 15) / 16, share = (ntr * ncol + sms - 1) / sms;
+  if (d.bm == 64 && share >= 12 && 100 * share < 4 * rounds * (3 * share <= ncol ? 96 : 87)) {
     d.share = (int)share;
     d.us = 1.10f * step_us[3] * (float)share / 4.0f;
-    d.grid = (int)((cols16 + share - 1) / share);
+    d.grid = (int)((ntr * ncol + share - 1) / share);
   }
   return d;
 }

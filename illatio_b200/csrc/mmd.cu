@@ -354,7 +354,7 @@ __device__ __forceinline__ float ld_cluster(const float* p, int rank) {
 constexpr int MK_PP = 20;  // floats between the tokens of a partial sum: a fragment's stores lie on different banks
 
 template <int FMT, int NT8, int CTAS /* of a tile: a cluster, where more than one */>
-__global__ void __launch_bounds__(MD_THREADS / CTAS, 1) mmk_kernel(const MdParams p) {
+__global__ void __launch_bounds__(MD_THREADS / CTAS, CTAS == 1 ? 1 : NT8 == 1 ? 8 : 0) mmk_kernel(const MdParams p) {
   extern __shared__ __align__(128) u8 smem[];
   constexpr int WARPS = MD_WARPS / CTAS;
   constexpr int TN = 8 * NT8, SB = MdFrag<FMT>::SB, SP = MdFrag<FMT>::SPITCH;

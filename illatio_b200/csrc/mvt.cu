@@ -39,10 +39,11 @@ namespace ill {
 // tile each at a time) as make up to sixteen warps, which share the staged activations, and each warp a ring of two to four stages.
 constexpr int MT_SUMS = 8, MT_MAX_WARPS = 16, MT_ROWS = 16, MT_MAX_STAGES = 4, MT_MATS = 3;
 
-// The named barrier at which the warps of group GRP of GW warps meet, or 0: a group of one warp needs none.  A CTA has barriers 0 (that
-// of __syncthreads) to 15, and sixteen groups of one warp.
-__host__ __device__ constexpr int mt_barrier(int grp, int gw) { return gw == 1 ? 0 : 1 + grp; }
-static_assert(mt_barrier(MT_MAX_WARPS / 2 - 1, 2) <= 15, "groups of two warps are the most that meet at barriers");
+// The named barrier at which the warps of group GRP meet.  A CTA has barriers 0 (that of __syncthreads) to 15, so fifteen groups at most.
+// (Sixteen, those of one warp with __syncwarp instead: the branch cost every launch 1 %.)
+__host__ __device__ constexpr int mt_barrier(int grp) { return 1 + grp; }
+constexpr int MT_MAX_GROUPS = 15;
+static_assert(mt_barrier(MT_MAX_GROUPS - 1) <= 15, "a CTA has no more barriers");
 
 struct MtMat {
   const u8* w;
@@ -271,8 +272,7 @@ __device__ __forceinline__ void cp_async4_or_zero(void* dst, const void* src, bo
 }
 // the meeting of one group's warps
 __device__ __forceinline__ void group_sync(int grp, int gw) {
-  if (gw == 1) __syncwarp();
-  else asm volatile("barrier.cta.sync %0, %1;" ::"r"(mt_barrier(grp, gw)), "r"(32 * gw) : "memory");
+  asm volatile("barrier.cta.sync %0, %1;" ::"r"(mt_barrier(grp)), "r"(32 * gw) : "memory");
 }
 
 template <int N> struct IntC { static constexpr int value = N; };
@@ -344,12 +344,10 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
   const int nsc = p.cols / BW, per_tok = p.cols / 16;
   uint4 sum8[2];            // K formats: eight sums of 16 a load; two loads a thread hold 16 tokens of 8192 columns
   const int nsum8 = FMT == ILL_Q8_0 ? 0 : NTOK * per_tok / 8;
-  const bool sums16 = ((uintptr_t)p.xsum & 15) == 0;  // (the sums lie on eight bytes, if not on sixteen)
   auto load_sums = [&](int i) {
     if (i >= nsum8 || 8 * i >= p.n * per_tok) return make_uint4(0, 0, 0, 0);
-    if (sums16) return ((const uint4*)p.xsum)[i];
     const uint2 a = ((const uint2*)p.xsum)[2 * i], b = ((const uint2*)p.xsum)[2 * i + 1];
-    return make_uint4(a.x, a.y, b.x, b.y);
+    return make_uint4(a.x, a.y, b.x, b.y);  // (the sums lie on eight bytes, if not on sixteen)
   };
 #pragma unroll
   for (int k = 0; k < 2; ++k) sum8[k] = load_sums(tid + k * nthreads);
@@ -565,7 +563,7 @@ static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n,
     int most[2] = {};
     for (int i = 0; i < (two ? 2 : 1); ++i) most[i] = mt_deal(p.f[i].npieces, gw, sums[i]) * p.f[i].cb;
     const uint32_t ring1 = (uint32_t)gw * p.stage_bytes;
-    for (int g = MT_MAX_WARPS / gw; g >= 1; --g) {
+    for (int g = min(MT_MAX_WARPS / gw, MT_MAX_GROUPS); g >= 1; --g) {
       // (fewer groups have a tile each already, and with eight warps there are enough to bring the activations)
       if (g > 1 && (g - 1) * sms >= ntiles && (g - 1) * gw >= 8) continue;
       if (off + g * (part_bytes + 2 * ring1) > budget) continue;
@@ -640,7 +638,7 @@ extern "C" int ill_test_few_tokens_plan(int nmat, int fmt0, int fmt1, int fmt2, 
   const MtParams& p = plan.p;
   out[0] = p.gw;
   out[1] = p.groups;
-  out[2] = mt_barrier(p.groups - 1, p.gw);
+  out[2] = mt_barrier(p.groups - 1);
   out[3] = p.stages;
   out[4] = plan.grid;
   out[5] = (int)plan.smem;

@@ -74,7 +74,7 @@ def test_argument_checks_of_the_chunk_and_peer_entry_points():
 @pytest.mark.parametrize("n", [2, 4, 8, 9, 16])
 def test_launches_of_few_tokens_stay_within_a_cta(fmt, n):
     """Every launch of two to sixteen tokens has barriers (0 to 15), warps and shared memory that a CTA has, over all numbers of blocks a
-    row and the numbers of tiles around whole rounds of 148 SMs: short rows of many rows get up to sixteen groups."""
+    row and the numbers of tiles around whole rounds of 148 SMs: short rows of many rows get up to fifteen groups."""
     two = isinstance(fmt, tuple)
     f = fmt if two else (fmt, 0)
     out, seen = (ctypes.c_int * 8)(), set()
@@ -88,16 +88,17 @@ def test_launches_of_few_tokens_stay_within_a_cta(fmt, n):
                     warps, groups, barrier, stages, ctas, smem, regs, _ = out
                     seen.add((warps, groups))
                     assert warps >= 1 and groups >= 1 and warps * groups <= 16 and 2 <= stages <= 4 and ctas >= 1
-                    assert 0 <= barrier <= 15 and (warps == 1) == (barrier == 0)
+                    assert 1 <= barrier <= 15
                     assert warps * groups >= 8 or cols > 1280  # (all warps bring the activations)
                     per_sm = 1 if ctas <= 148 else 2
                     assert ctas <= 296 and per_sm * (smem + 1024) <= 228 * 1024 and per_sm * 32 * warps * groups * regs <= 65536
-    assert (1, 16) in seen
+    assert (1, 15) in seen
 
 
 @pytest.mark.parametrize("rows,cols,n,bm,shares,i8", [
     (151936, 896, 17, 32, False, False), (151936, 896, 32, 32, False, False), (151552, 896, 17, 32, False, False), (9728, 2560, 512, 64, True, False),
-    (9700, 2560, 505, 64, True, False), (17300, 5120, 399, 64, True, False), (4096, 2048, 8192, 128, False, False), (36000, 1024, 300, 64, False, False),
+    (9700, 2560, 505, 64, True, False), (17300, 5120, 399, 64, True, False), (1536, 5120, 8192, 64, True, False), (5120, 1536, 2048, 64, False, False), (896, 4864, 8192, 64, True, False),
+    (4096, 2048, 8192, 128, False, False), (36000, 1024, 300, 64, False, False),
     (151936, 896, 80, 80, False, True), (17408, 5120, 160, 64, False, True), (4864, 896, 512, 48, False, True), (896, 4864, 777, 48, False, False)])
 def test_tiles_of_a_q8_0_chunk(rows, cols, n, bm, shares, i8):
     """Few tokens of many rows keep the tile that their number asks for on both sides of eight rounds; even shares where they save enough;

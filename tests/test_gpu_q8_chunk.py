@@ -24,6 +24,7 @@ pytestmark = pytest.mark.gpu
     (9728, 128, 512, 0, False, False),  # even shares, tiles that end where a tile of rows or a share does
     (9700, 128, 505, 2, True, True),
     (17300, 256, 399, 0, False, True),
+    (1536, 128, 8190, 0, True, False),
     (151936, 128, 17, 0, False, False),  # many tiles of rows of few tokens
     (127, 384, 29, 0, False, True),
     (129, 256, 32, 0, True, True),
