@@ -57,6 +57,7 @@ struct MqParams {
   const float* bias;
   int acc, n;
   int bm;              // tokens a tile, a multiple of 16; a CTA takes every gridDim.x-th tile -- or, SHARE not 0,
+  int early;           // the next kernel may start before this one ends
   int ncol, share;     // SHARE of the NCOL columns of 16 tokens of all the tiles of rows one after another, in tiles of up to BM
   uint32_t zero;
   unsigned* status;
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) mm_q8_kernel(const __grid_const
   uint32_t* tmem_slot = (uint32_t*)(smem + G::SLOT);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 
-  pdl_launch_dependents();
+  if (p.early) pdl_launch_dependents();
   if (tid == 32) {
     for (int s = 0; s < MQ_NS; ++s) { mbar_init(&full[s], 1 + 4 + 32); mbar_init(&free[s], MQ_DRAIN); }
     for (int b = 0; b < MQ_NACC; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_free[b], MQ_DRAIN); }
@@ -504,6 +505,11 @@ int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t
   p.bm = d.bm;
   p.ncol = (n + 15) / 16;
   p.share = d.share;
+  // What the next kernel's early start gives is a microsecond or two: 896 x 4864 x 777 (43 us) and its like lose 1 % of a chunk
+  // without.  After a long launch, whose CTAs end a tile apart, it costs more: the CTAs of the chain behind it go to whichever SM is
+  // free, not in order, and the large expert products at its end take longer (down product of a shared expert, 5120 x 1536 x 8192 tokens,
+  // 513 us: the layer 8673 us with the early start, 8530 without).
+  p.early = (float)p.nsteps * d.us < 100.0f;
   const int grid = d.grid;
   MqMaps maps;
   const uint64_t row_bytes = (uint64_t)cols / 32 * 34;
