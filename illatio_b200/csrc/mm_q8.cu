@@ -415,7 +415,8 @@ static int mq_launch(const MqMaps& maps, const MqParams& p, int grid, cudaStream
   const void* k = (const void*)mm_q8_kernel<NT>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MqGeom<NT>::SMEM);
   if (e != cudaSuccess) return cuda_fail(e);
-  // the warp groups trade registers after launch: what they ask for together must fit in what the CTA was given
+  // the warp groups trade registers after launch: what they ask for together must fit in what the CTA was given.  (Asked for at each
+  // launch, 0.35 us with the attribute above: an answer kept from the first launch would be one device's, and a failure's for good.)
   cudaFuncAttributes fa;
   e = cudaFuncGetAttributes(&fa, k);
   if (e != cudaSuccess) return cuda_fail(e);

@@ -114,7 +114,8 @@ def test_sums_of_16_that_lie_on_eight_bytes(cuda_lib, fmt, cols, n):
 
 
 @pytest.mark.parametrize("fmt,rows,cols,n", [(B.Q8_0, 50, 1152, 16), (B.Q4_K, 40, 2560, 16), (B.Q4_K, 19, 1280, 3), (B.Q6_K, 40, 5120, 16),
-                                             (B.Q6_K, 23, 2304, 2)])
+                                             (B.Q6_K, 23, 2304, 2), (B.Q8_0, 4864, 896, 16), (B.Q4_K, 2560, 4096, 4),
+                                             (B.Q6_K, 1024, 2560, 9), (B.Q4_K, 2400, 17408, 3), (B.Q6_K, 176, 17408, 16)])
 def test_few_tokens_against_the_oracle(oracle, cuda_lib, fmt, rows, cols, n):
     x = np.random.default_rng(cols).standard_normal(n * cols).astype(np.float32)
     act = dev_act(fmt, x)
