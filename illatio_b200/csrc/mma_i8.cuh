@@ -40,6 +40,10 @@ __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void* p) {
                : "r"(smem_u32(p)));
 }
 
+__device__ __forceinline__ void ldsm4_at(uint32_t (&r)[4], uint32_t a) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+
 // a 32-bit word at any byte address of shared memory
 __device__ __forceinline__ uint32_t lds32u(const u8* p) {
   const uint32_t mis = (uint32_t)(uintptr_t)p & 3u;

@@ -851,10 +851,19 @@ int mv_common(int fmt, int mode, int nmat, const ill_dptr* w, const int* rows, i
   const bool glu = mode == MODE_GLU || mode == MODE_MOE_GLU;
   if ((glu || mode == MODE_PEERS) && n != 1) return ILL_ERR_ARG;
   if (n >= 2 && !glu && nmat == 1 && !ptrs && !x_seg) {
-    // several tokens: the tensor cores' int8 path where it is written (Q8_0, Q4_K, Q6_K; up to 16 tokens with the
-    // activations resident, chunks with them streamed), else the token loop below
+    // several tokens: the tensor cores' int8 path where it is written (up to 16 tokens with the activations resident; Q8_0, Q4_K
+    // and Q6_K also chunks with them streamed), else the token loop below
     int rc_t = ILL_ERR_UNSUPPORTED;
     if (n <= 16) rc_t = mvt_try(1, &fmt, w, rows, cols, xq, xs, xsum, y, bias, acc, n, stream);
+    // (2-bit formats, rows too long for sixteen tokens' activations but not for eight's: half of the tokens at a time)
+    if (rc_t == ILL_ERR_UNSUPPORTED && n > 8 && n <= 16 && (fmt == ILL_Q2_K || fmt == ILL_IQ2_XXS)) {
+      const int h = (n + 1) / 2;
+      rc_t = mvt_try(1, &fmt, w, rows, cols, xq, xs, xsum, y, bias, acc, h, stream);
+      const ill_dptr y2 = y[0] + 4ull * h * rows[0];
+      if (rc_t == ILL_OK)
+        return mvt_try(1, &fmt, w, rows, cols, xq + (ill_dptr)h * cols, xs + 4ull * h * (cols / 256), xsum ? xsum + 2ull * h * (cols / 16) : 0, &y2,
+                       bias, acc, n - h, stream);
+    }
     // a few tokens of rows too long for their activations to stay in shared memory
     if (rc_t == ILL_ERR_UNSUPPORTED && n <= 16) rc_t = mmk_try(fmt, w[0], rows[0], cols, xq, xs, xsum, y[0], bias ? bias[0] : 0, acc, n, stream);
     // a chunk

@@ -24,14 +24,17 @@
 // 142 / 117.  What gave it: one launch; activations that are all asked for before anything is waited for (4 us a launch); the deal;
 // Q4_K's mins against the sums of 16 by two products, its scales four at a time (half the instructions); ldmatrix.
 //
+// The 2-bit formats' blocks are in mtblock.cuh.  us, the token loop of mv.cu (a pass of dp4a a token) / now: Q2_K 151936 x 2560, 4 tokens 236 / 60,
+// 16 tokens 923 / 74; IQ2_XXS 232 / 85 and 768 / 98; 4096 x 4096, 4 tokens 29.5 / 4.6 and 27.2 / 6.3; 512 x 512, 2 tokens 2.9 / 2.1 and 3.1 / 3.1.
+//
 // mma.sync is the legacy tensor path: right here, where N is 8 or 16 and the bound is HBM; the chunk-sized
 // products (hundreds of rows of X an expert) use tcgen05 (mm_id.cu).
 //
 // Replaces mv_q8_n / mm_q8_mma's small-batch use and mv_k's token loop behind CMAT-MUL-N
-// (src/cuda-dense.lisp:220-255; src/cuda/dense.cu:643-885, src/cuda/kquant.cu:169-466) for Q8_0, Q4_K and Q6_K.
-#include "formats.cuh"
+// (src/cuda-dense.lisp:220-255; src/cuda/dense.cu:643-885, src/cuda/kquant.cu:169-466).
 #include "host.h"
-#include "mma_i8.cuh"
+#include "iq2xxs_tables.cuh"
+#include "mtblock.cuh"
 
 namespace ill {
 
@@ -75,21 +78,6 @@ struct MtParams {
   uint32_t xs_off, bs_off, ring_off, part_off;
 };
 
-// The tokens' activations in shared memory.
-struct MtX {
-  const i8* q;        // token t's quants at q + t * stride
-  int stride;
-  const float* s;     // [t][scales a token]
-  const u8* bs;       // K formats, [t][block][32]: the block's sixteen sums of 16 in two bytes each: sum >> 4 (signed), then sum & 15
-  int nsc, nb;
-};
-// B fragments of 64 columns from K on against tokens 8 NT .. 8 NT + 7 (those past the last are staged as zeros): r[0], r[1] the first
-// 32 columns', r[2], r[3] the others'; of k16 products one each
-__device__ __forceinline__ void xfrag(uint32_t (&r)[4], const MtX& x, int nt, int k, int lane) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(x.q + (size_t)(8 * nt + (lane & 7)) * x.stride + k + 16 * (lane >> 3))));
-}
 // sums of 16 times sixteen bytes of the rows' (S0, S8: row g's and g + 8's bytes 4 t ..), each sum split in two int8 halves
 __device__ __forceinline__ void mul_sums(int (&c)[4], uint32_t s0, uint32_t s8, const MtX& x, int nt, int blk, int lane) {
   const u8* b = x.bs + ((size_t)(8 * nt + (lane >> 2)) * x.nb + blk) * 32 + 4 * (lane & 3);
@@ -99,11 +87,6 @@ __device__ __forceinline__ void mul_sums(int (&c)[4], uint32_t s0, uint32_t s8, 
 #pragma unroll
   for (int i = 0; i < 4; ++i) c[i] = 16 * hi[i] + lo[i];
 }
-
-// ---- one block of 16 rows against the tokens: ACC[nt][i] += ... --------------------------------------
-// ROW0 / ROW8: the block's bytes of rows g and g + 8 of the tile (g = lane / 4) in the staged piece; BLK the
-// block's number in the row; NT8 tiles of eight tokens.  Output i of a tile: row g + 8 (i / 2), token 8 nt + 2 (lane % 4) + i % 2.
-template <int FMT, int NT8, bool AL4> struct MtBlock;
 
 template <int NT8, bool AL4> struct MtBlock<ILL_Q8_0, NT8, AL4> {
   __device__ static void run(const u8* row0, const u8* row8, int blk, const MtX& x, int lane, float (&acc)[NT8][4]) {
@@ -263,13 +246,6 @@ template <int NT8, bool AL4> struct MtBlock<ILL_Q6_K, NT8, AL4> {
   }
 };
 
-// 16 / 4 bytes global -> shared, asynchronously, or zeros
-__device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, bool in) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async4_or_zero(void* dst, const void* src, bool in) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 4 : 0) : "memory");
-}
 // the meeting of one group's warps
 __device__ __forceinline__ void group_sync(int grp, int gw) {
   asm volatile("barrier.cta.sync %0, %1;" ::"r"(mt_barrier(grp)), "r"(32 * gw) : "memory");
@@ -312,7 +288,7 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
   auto issue_next = [&]() {  // all lanes: four a row segment, eight rows at a time; a group of cp.async, possibly empty
     if (n_tile < ntiles) {
       auto copy = [&](auto fmt_) {
-        constexpr int F = decltype(fmt_)::value, BB = Fmt<F>::BB, MAXB = F == ILL_Q8_0 ? 8 : F == ILL_Q4_K ? 2 : 1;  // most blocks a piece
+        constexpr int F = decltype(fmt_)::value, BB = Fmt<F>::BB, MAXB = F == ILL_Q8_0 ? 8 : F == ILL_Q6_K ? 1 : 2;  // most blocks a piece
         const MtFmt& f = p.f[F != FMT];
         const int row0 = (n_tile - (n_mi ? p.m[n_mi - 1].tile_end : 0)) * MT_ROWS;
         u8* st = ring + (size_t)i_slot * p.stage_bytes;
@@ -335,6 +311,8 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
     cp_async_commit();
   };
   for (int s = 0; s < stages; ++s) issue_next();  // the weights do not depend on the previous kernel
+  __shared__ uint2 iq_grid[FMT == ILL_IQ2_XXS ? IQ_TABLE_BYTES / 8 : 1];  // (static: the look-ups' addresses start at a constant)
+  if constexpr (FMT == ILL_IQ2_XXS) iq_tables_fill(iq_grid, iq_grid + IQ_COPIES * 256, ill_iq2xxs_grid, ill_ksigns_iq2xs);
   pdl_launch_dependents();
   pdl_wait();
 
@@ -343,7 +321,8 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
   // of gate and up, 2 x 9728 x 2560, of 16 tokens.)
   const int nsc = p.cols / BW, per_tok = p.cols / 16;
   uint4 sum8[2];            // K formats: eight sums of 16 a load; two loads a thread hold 16 tokens of 8192 columns
-  const int nsum8 = FMT == ILL_Q8_0 ? 0 : NTOK * per_tok / 8;
+  constexpr bool SUMS = FMT != ILL_Q8_0 && FMT != ILL_IQ2_XXS;
+  const int nsum8 = SUMS ? NTOK * per_tok / 8 : 0;
   auto load_sums = [&](int i) {
     if (i >= nsum8 || 8 * i >= p.n * per_tok) return make_uint4(0, 0, 0, 0);
     const uint2 a = ((const uint2*)p.xsum)[2 * i], b = ((const uint2*)p.xsum)[2 * i + 1];
@@ -361,20 +340,11 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
     cp_async4_or_zero(xs_s + i, in ? p.xs + i : p.xs, in);
   }
   cp_async_commit();
-  if constexpr (FMT != ILL_Q8_0) {
+  if constexpr (SUMS) {
     // per block 32 bytes: the sixteen sums' high parts (sum >> 4, signed), then their low parts (sum & 15)
     auto store_sums = [&](int i, const uint4& v) {
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};  // two sums each
-      uint32_t hi[2], lo[2];
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        // bits 4..11 of the four 16-bit sums, a byte each; bits 0..3
-        hi[k] = __byte_perm(w[2 * k] >> 4, w[2 * k + 1] >> 4, 0x6420);
-        lo[k] = __byte_perm(w[2 * k], w[2 * k + 1], 0x6420) & 0x0f0f0f0fu;
-      }
       u8* b = smem + p.bs_off + (i >> 1) * 32 + 8 * (i & 1);
-      *(uint2*)b = make_uint2(hi[0], hi[1]);
-      *(uint2*)(b + 16) = make_uint2(lo[0], lo[1]);
+      split_sums(v, *(uint2*)b, *(uint2*)(b + 16));
     };
 #pragma unroll
     for (int k = 0; k < 2; ++k)
@@ -385,6 +355,8 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
   __syncthreads();
   MtX x;
   x.q = xq_s; x.stride = p.x_stride; x.s = xs_s; x.bs = smem + p.bs_off; x.nsc = nsc; x.nb = nb;
+  MtLane xl;  // (the 2-bit formats')
+  xl.set<FMT>(smem_u32(smem), p.x_stride, smem_u32(smem) + p.xs_off, smem_u32(smem) + p.bs_off, nb, FMT == ILL_IQ2_XXS ? smem_u32(iq_grid) : 0u, lane);
 
   int slot = 0, it = 0;
   for (int tile = tile0; tile < ntiles; tile += tile_step, ++it) {
@@ -415,7 +387,11 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
           const u8* s0 = piece + (size_t)g * f.pitch + (((uintptr_t)w + o0) & 15);
           const u8* s8 = piece + (size_t)(g + 8) * f.pitch + (((uintptr_t)w + o8) & 15);
           const int nhere = min(f.cb, nb - pc * f.cb);
-          for (int j = 0; j < nhere; ++j) MtBlock<F, NT8, AL4>::run(s0 + j * BB, s8 + j * BB, pc * f.cb + j, x, lane, acc);
+          if constexpr (F == ILL_Q2_K || F == ILL_IQ2_XXS) {
+            for (int j = 0; j < nhere; ++j) MtBlock<F, NT8, AL4>::run(smem_u32(s0) + j * BB, smem_u32(s8) + j * BB, pc * f.cb + j, xl, lane, acc);
+          } else {
+            for (int j = 0; j < nhere; ++j) MtBlock<F, NT8, AL4>::run(s0 + j * BB, s8 + j * BB, pc * f.cb + j, x, lane, acc);
+          }
         };
         if (TWO && p.m[mi].alt) use(IntC<FMT2>()); else use(IntC<FMT>());
         __syncwarp();
@@ -436,6 +412,7 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
 #pragma unroll
         for (int k = 0; k < MT_SUMS; ++k)
           if (k < nsums) v = __fadd_rn(v, sums[(k * NTOK + tk) * PP + r]);
+        if (FMT == ILL_IQ2_XXS) v *= 0.125f;
         if (p.m[mi].bias) v += p.m[mi].bias[row];
         float* yp = p.m[mi].y + (long long)tk * p.m[mi].rows + row;
         *yp = p.acc ? *yp + v : v;
@@ -445,12 +422,14 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
 }
 
 // Registers a thread of the kernel, at most: what decides whether an SM holds two CTAs
-static int mt_regs(int fmt, int n) { return fmt == ILL_Q8_0 ? 96 : n <= 8 ? 112 : 128; }
+static int mt_regs(int fmt, int n) { return fmt == ILL_Q8_0 ? 96 : n <= 8 && fmt != ILL_IQ2_XXS ? 112 : 128; }
 
 static const void* mt_kernel(int fmt, bool two, bool al4, int n) {
 #define MT_PICK(F, F2, A) (n <= 8 ? (const void*)mvt_kernel<F, F2, 1, A> : (const void*)mvt_kernel<F, F2, 2, A>)
   if (fmt == ILL_Q8_0) return MT_PICK(ILL_Q8_0, ILL_Q8_0, false);
   if (fmt == ILL_Q6_K) return MT_PICK(ILL_Q6_K, ILL_Q6_K, false);
+  if (fmt == ILL_IQ2_XXS) return MT_PICK(ILL_IQ2_XXS, ILL_IQ2_XXS, false);
+  if (fmt == ILL_Q2_K) return al4 ? MT_PICK(ILL_Q2_K, ILL_Q2_K, true) : MT_PICK(ILL_Q2_K, ILL_Q2_K, false);
   if (two) return al4 ? MT_PICK(ILL_Q4_K, ILL_Q6_K, true) : MT_PICK(ILL_Q4_K, ILL_Q6_K, false);
   return al4 ? MT_PICK(ILL_Q4_K, ILL_Q4_K, true) : MT_PICK(ILL_Q4_K, ILL_Q4_K, false);
 #undef MT_PICK
@@ -500,7 +479,6 @@ static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n,
   bool two = false;
   for (int i = 0; i < nmat; ++i) two = two || fmts[i] != fmts[0];
   const int fmt = two ? ILL_Q4_K : fmts[0];
-  if (fmt != ILL_Q8_0 && fmt != ILL_Q4_K && fmt != ILL_Q6_K) return ILL_ERR_UNSUPPORTED;
   for (int i = 0; i < MT_MATS; ++i) {
     if (i < nmat) {
       if (two && fmts[i] != ILL_Q4_K && fmts[i] != ILL_Q6_K) return ILL_ERR_UNSUPPORTED;
@@ -514,10 +492,11 @@ static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n,
     p.m[i].tile_end = (int)ntiles;
   }
   const int bw = fmt_block_weights(fmt), nsc = cols / bw;
+  const uint32_t tables = fmt == ILL_IQ2_XXS ? IQ_TABLE_BYTES : 0u;  // static shared memory
   p.cols = cols;
   p.nblocks = nsc;
   p.n = n;
-  p.x_stride = cols + 16;
+  p.x_stride = mt_x_stride(fmt, cols);
   const uint32_t ntok = n <= 8 ? 8 : 16;  // staged tokens: whole tiles of eight
   uint32_t off = ntok * (uint32_t)p.x_stride;
   off = (off + 15) / 16 * 16;
@@ -532,22 +511,29 @@ static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n,
     // a row's segment: its block's 16-byte aligned span, rows a multiple of 16 bytes apart that is an odd multiple
     // of 16 mod 128 (eight rows x four words then sit on 32 different banks)
     // blocks a piece: about 200-300 bytes a row segment (four lanes' copies), but every sum should get a piece
-    int cb = ft == ILL_Q8_0 ? 8 : ft == ILL_Q4_K ? 2 : 1;
+    int cb = ft == ILL_Q8_0 ? 8 : ft == ILL_Q6_K ? 1 : 2;
     while (cb > 1 && (p.nblocks + cb - 1) / cb < MT_SUMS) cb >>= 1;
-    f.cb = cb;
-    f.npieces = (p.nblocks + cb - 1) / cb;
-    f.pitch = (cb * bb + 15 + 15) / 16 * 16;
-    while ((f.pitch / 16) % 8 % 2 == 0) f.pitch += 16;
-    const uint32_t stage = (uint32_t)(MT_ROWS * f.pitch + 16 + 127) / 128 * 128;
     // Too many tokens of too many columns (no room for eight warps with two stages each): mmd.cu's form, which brings the
-    // activations step by step, is the faster one, and adds a row's blocks in another order
-    if (off + (ft == ILL_Q8_0 ? 0u : ft == ILL_Q4_K ? 16u : 32u) * ntok * (cols / 256) + 16384u + 2u * MT_SUMS * stage > 220u * 1024u)
-      return ILL_ERR_UNSUPPORTED;
+    // activations step by step, is the faster one, and adds a row's blocks in another order.  The 2-bit formats, which have no such form, go
+    // on with a block a piece and six warps (else the token loop of mv.cu; us, 5120 x 17408, 8 tokens: Q2_K 224 / 21, IQ2_XXS 252 / 42).
+    const bool two_bit = ft == ILL_Q2_K || ft == ILL_IQ2_XXS;
+    uint32_t stage;
+    for (;; cb = 1) {
+      f.cb = cb;
+      f.npieces = (p.nblocks + cb - 1) / cb;
+      f.pitch = (cb * bb + 15 + 15) / 16 * 16;
+      while ((f.pitch / 16) % 8 % 2 == 0) f.pitch += 16;
+      stage = (uint32_t)(MT_ROWS * f.pitch + 16 + 127) / 128 * 128;
+      const uint32_t room = off + (ft == ILL_Q8_0 || ft == ILL_IQ2_XXS ? 0u : ft == ILL_Q4_K ? 16u : 32u) * ntok * (cols / 256) +
+                            (two_bit ? 12288u : 16384u) + 2u * (two_bit && cb == 1 ? 6 : MT_SUMS) * stage + tables;
+      if (room <= (two_bit ? 226u : 220u) * 1024u) break;
+      if (!two_bit || cb == 1) return ILL_ERR_UNSUPPORTED;
+    }
     if (stage > p.stage_bytes) p.stage_bytes = stage;
     const int ns = f.npieces < MT_SUMS ? f.npieces : MT_SUMS;
     if (ns > p.nsums) p.nsums = ns;
   }
-  if (fmt != ILL_Q8_0) off += 32u * ntok * (cols / 256);
+  if (fmt != ILL_Q8_0 && fmt != ILL_IQ2_XXS) off += 32u * ntok * (cols / 256);
   off = (off + 127) / 128 * 128;
   p.ring_off = off;
   // Warps a group and groups a CTA, for the least time: the tiles a group takes one after another, times the blocks of its busiest
@@ -556,7 +542,7 @@ static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n,
   // fastest pair or one within 5 % of it but for a head of 151936 x 2560 at two tokens (10 %).  Short rows have few warps a group: such
   // a CTA takes groups without a tile up to eight warps, for the activations' sake (1024 x 256, 16 tokens, a warp / eight: Q6_K 4.9 / 3.4
   // us, Q4_K 4.6 / 3.1; over 1050 shapes of up to 1280 columns 6 % on average, 11 % slower at most, of 2.6 us).
-  const uint32_t budget = 226u * 1024u, part_bytes = 2u * p.nsums * ntok * 20 * 4;
+  const uint32_t budget = 226u * 1024u - tables, part_bytes = 2u * p.nsums * ntok * 20 * 4;
   double best = 0;
   for (int gw = p.nsums; gw >= 1; --gw) {
     u8 sums[2][MT_SUMS];
@@ -587,7 +573,7 @@ static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n,
   // Two CTAs an SM where their shared memory and registers fit: a grid of two an SM that holds one runs in two rounds, each with its
   // activations to bring (Q8_0 of 16 warps a CTA, 4 tokens: 4096 x 256 4.5 us, 2.7 with one; 17408 x 256 7.6 / 6.4)
   const int regs = 32 * p.gw * p.groups * mt_regs(fmt, n);
-  const int per_sm = (int)((227u * 1024u) / (off + 1024u)) >= 2 && 2 * regs <= 65536 ? 2 : 1;
+  const int per_sm = (int)((227u * 1024u) / (off + tables + 1024u)) >= 2 && 2 * regs <= 65536 ? 2 : 1;
   plan->grid = (int)((long long)sms * per_sm < ntiles ? (long long)sms * per_sm : ntiles);
   plan->smem = off;
   plan->fmt = fmt;
@@ -611,7 +597,7 @@ int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
     p.m[i].w = (const u8*)(uintptr_t)w[i];
     p.m[i].y = (float*)(uintptr_t)y[i];
     p.m[i].bias = bias ? (const float*)(uintptr_t)bias[i] : nullptr;
-    if (fmts[i] == ILL_Q4_K) al4 = al4 && (w[i] & 3) == 0;
+    if (fmts[i] == ILL_Q4_K || fmts[i] == ILL_Q2_K) al4 = al4 && (w[i] & 3) == 0;
   }
   p.xq = (const i8*)(uintptr_t)xq;
   p.xs = (const float*)(uintptr_t)xs;
@@ -641,7 +627,7 @@ extern "C" int ill_test_few_tokens_plan(int nmat, int fmt0, int fmt1, int fmt2, 
   out[2] = mt_barrier(p.groups - 1);
   out[3] = p.stages;
   out[4] = plan.grid;
-  out[5] = (int)plan.smem;
+  out[5] = (int)plan.smem + (plan.fmt == ILL_IQ2_XXS ? IQ_TABLE_BYTES : 0);
   out[6] = mt_regs(plan.fmt, n);
   out[7] = 0;
   if (!sms) {
