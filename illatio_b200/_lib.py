@@ -51,6 +51,13 @@ SIGNATURES = {
     "ill_moe_glu": (_I, [_I, _I, _I, _L, _L, _P, _I, _P, _P, _P, _I, _F, _P, _P, _L, _S]),
     "ill_moe_mv_sel": (_I, [_I, _I, _I, _L, _P, _I, _P, _I, _P, _P, _P, _I, _P, _L, _S]),
     "ill_moe_glu_sel": (_I, [_I, _I, _I, _L, _L, _P, _I, _P, _I, _P, _P, _P, _I, _F, _P, _P, _L, _S]),
+    "ill_moe_few_most": (_I, [_I, _I]),
+    "ill_moe_few": (_I, [_I, _I, _I, _L, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _L, _S]),
+    "ill_moe_few2": (_I, [_I, _I, _I, _L, _L, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _P, _L, _S]),
+    "ill_moe_few_glu": (_I, [_I, _I, _I, _L, _L, _P, _P, _P, _I, _L, _P, _P, _P, _P, _F, _P, _P, _L, _S]),
+    "ill_moe_mm_id_over": (_I, [_I, _I, _I, _L, _L, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _P, _L, _I, _S]),
+    "ill_act_f16_over": (_I, [_L, _I, _P, _P, _P, _P, _P, _P, _I, _I, _S]),
+    "ill_swiglu_q8k_both": (_I, [_L, _I, _F, _P, _P, _P, _P, _P, _P, _P, _P, _S]),
     "ill_silu_mul": (_I, [_L, _P, _P, _P, _S]),
     "ill_swiglu_w": (_I, [_L, _I, _F, _P, _P, _P, _P, _S]),
     "ill_moe_sum": (_I, [_I, _I, _L, _P, _P, _P, _P, _S]),

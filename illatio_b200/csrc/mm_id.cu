@@ -72,6 +72,7 @@ struct MmParams {
   unsigned one_count;
   int acc;
   int bm;                      // rows of X a tile of a dense matrix, at most the kernel's NT
+  int over;                    // experts of no more rows than this are left out
 };
 // (DENSE is a template argument of the kernel, so that the experts' launches compile to what they were without it)
 template <bool DENSE> __device__ __forceinline__ unsigned long long mm_ptr(const MmParams& p, int e) {
@@ -888,7 +889,10 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
   pdl_wait();
   int bm = DENSE ? p.bm : NT;
   if constexpr (NT2 != 0) {  // every expert's rows, all loads at once
-    for (int e = tid; e < p.ne; e += G::THREADS) tile_first[e] = min(max(mm_count<DENSE>(p, e), 0), 1 << 22);
+    for (int e = tid; e < p.ne; e += G::THREADS) {
+      const int c = mm_count<DENSE>(p, e);
+      tile_first[e] = c > p.over ? min(c, 1 << 22) : 0;
+    }
     __syncthreads();
   }
   if (warp == 0) {
@@ -906,7 +910,8 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
     int before = 0;
     for (int e0 = 0; e0 < p.ne; e0 += 32) {
       const int e = e0 + lane;
-      const int c = e >= p.ne ? 0 : NT2 ? tile_first[e] : mm_count<DENSE>(p, e);
+      int c = e >= p.ne ? 0 : NT2 ? tile_first[e] : mm_count<DENSE>(p, e);
+      if (!NT2 && !DENSE && c <= p.over) c = 0;
       const int tiles = (c + bm - 1) / bm;
       int incl = tiles;
 #pragma unroll
@@ -945,9 +950,15 @@ __global__ void __launch_bounds__(256) act_f16_kernel(long long rows, int cols, 
                                                       const unsigned* __restrict__ map, __half* __restrict__ xh,
                                                       __half* __restrict__ xe, const u8* __restrict__ sc,
                                                       const u8* __restrict__ wt, float* __restrict__ xd_out,
-                                                      float* __restrict__ w_out, const unsigned* __restrict__ rows_dev) {
+                                                      float* __restrict__ w_out, const unsigned* __restrict__ rows_dev,
+                                                      const unsigned* __restrict__ counts, int ne, int over) {
   pdl_launch_dependents();
   pdl_wait();
+  if (counts) {  // nothing to do unless some expert has more than OVER rows
+    bool any = false;
+    for (int e = threadIdx.x; e < ne; e += blockDim.x) any = any || (int)counts[e] > over;
+    if (!__syncthreads_or(any)) return;
+  }
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // one thread: 16 values
   const int per_row = cols / 16;
   if (gid >= rows * per_row) return;
@@ -1223,7 +1234,7 @@ using namespace ill;
 
 static int act_f16_launch(int64_t rows, int cols, const u8* qp, long long qs, const u8* bp, long long bs, ill_dptr map,
                           ill_dptr xh, ill_dptr xe, const u8* sc, const u8* wt, ill_dptr xd_out, ill_dptr w_out,
-                          ill_stream stream, ill_dptr rows_dev = 0) {
+                          ill_stream stream, ill_dptr rows_dev = 0, ill_dptr counts = 0, int ne = 0, int over = 0) {
   long long nrows = rows;
   const unsigned* mp = (const unsigned*)(uintptr_t)map;
   __half* hp = (__half*)(uintptr_t)xh;
@@ -1231,7 +1242,8 @@ static int act_f16_launch(int64_t rows, int cols, const u8* qp, long long qs, co
   float* xo = (float*)(uintptr_t)xd_out;
   float* wo = (float*)(uintptr_t)w_out;
   const unsigned* rd = (const unsigned*)(uintptr_t)rows_dev;
-  void* args[] = {&nrows, &cols, &qp, &qs, &bp, &bs, &mp, &hp, &ep, &sc, &wt, &xo, &wo, &rd};
+  const unsigned* cn = (const unsigned*)(uintptr_t)counts;
+  void* args[] = {&nrows, &cols, &qp, &qs, &bp, &bs, &mp, &hp, &ep, &sc, &wt, &xo, &wo, &rd, &cn, &ne, &over};
   const long long threads = rows * (cols / 16);
   return launch_kernel((const void*)act_f16_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, args,
                        (cudaStream_t)stream);
@@ -1244,6 +1256,15 @@ extern "C" int ill_act_f16(int64_t rows, int cols, ill_dptr xq, ill_dptr bsums, 
   if (rows == 0) return ILL_OK;
   return act_f16_launch(rows, cols, (const u8*)(uintptr_t)xq, cols, (const u8*)(uintptr_t)bsums, cols / 8, map, xh, xe, nullptr,
                         nullptr, 0, 0, stream);
+}
+
+extern "C" int ill_act_f16_over(int64_t rows, int cols, ill_dptr xq, ill_dptr bsums, ill_dptr map, ill_dptr xh, ill_dptr xe, ill_dptr counts,
+                                int ne, int over, ill_stream stream) {
+  if (rows < 0 || cols <= 0 || cols % 256 || !xq || !xh || (xe && !bsums) || !counts || ne < 1 || over < 0) return ILL_ERR_ARG;
+  if ((xq & 15) || (bsums & 1) || (map & 3) || (xh & 15) || (xe & 15) || (counts & 3)) return ILL_ERR_ALIGN;
+  if (rows == 0) return ILL_OK;
+  return act_f16_launch(rows, cols, (const u8*)(uintptr_t)xq, cols, (const u8*)(uintptr_t)bsums, cols / 8, map, xh, xe, nullptr,
+                        nullptr, 0, 0, stream, 0, counts, ne, over);
 }
 
 extern "C" int64_t ill_ep_row_bytes(int cols) {
@@ -1407,7 +1428,7 @@ static int encode_map(CUtensorMap* map, ill_dptr base, int64_t cols, int64_t row
 static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
                         int64_t total_rows, ill_dptr xh, ill_dptr xe, ill_dptr xd, ill_dptr map, ill_dptr ymap, ill_dptr ypeers,
                         ill_dptr y, int64_t y_stride, ill_stream stream, int64_t add2 = 0, ill_dptr y2 = 0, ill_dptr one_ptr = 0,
-                        int acc = 0);
+                        int acc = 0, int over = 0);
 
 extern "C" int ill_moe_mm_id2(int fmt, int ncols, int nrows, int64_t add, int64_t add2, ill_dptr ptrs, ill_dptr counts,
                               ill_dptr bases, int ne, int64_t total_rows, ill_dptr xh, ill_dptr xe, ill_dptr xd, ill_dptr map,
@@ -1422,6 +1443,14 @@ extern "C" int ill_moe_mm_id(int fmt, int ncols, int nrows, int64_t add, ill_dpt
                              ill_dptr y, int64_t y_stride, ill_stream stream) {
   if (!y) return ILL_ERR_ARG;
   return mm_id_launch(fmt, ncols, nrows, add, ptrs, counts, bases, ne, total_rows, xh, xe, xd, map, ymap, 0, y, y_stride, stream);
+}
+
+extern "C" int ill_moe_mm_id_over(int fmt, int ncols, int nrows, int64_t add, int64_t add2, ill_dptr ptrs, ill_dptr counts, ill_dptr bases,
+                                  int ne, int64_t total_rows, ill_dptr xh, ill_dptr xe, ill_dptr xd, ill_dptr map, ill_dptr y, ill_dptr y2,
+                                  int64_t y_stride, int over, ill_stream stream) {
+  if (!y || (y2 & 15) || (add2 & 3) || over < 0) return ILL_ERR_ARG;
+  return mm_id_launch(fmt, ncols, nrows, add, ptrs, counts, bases, ne, total_rows, xh, xe, xd, map, 0, 0, y, y_stride, stream, add2, y2, 0, 0,
+                      over);
 }
 
 extern "C" int ill_moe_mm_id_peers(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, ill_dptr counts, ill_dptr bases,
@@ -1492,7 +1521,8 @@ static int mm_pick_tile(int fmt, long long rows, long long ntn, int sms) {
 
 static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
                         int64_t total_rows, ill_dptr xh, ill_dptr xe, ill_dptr xd, ill_dptr map, ill_dptr ymap, ill_dptr ypeers,
-                        ill_dptr y, int64_t y_stride, ill_stream stream, int64_t add2, ill_dptr y2, ill_dptr one_ptr, int acc) {
+                        ill_dptr y, int64_t y_stride, ill_stream stream, int64_t add2, ill_dptr y2, ill_dptr one_ptr, int acc,
+                        int over) {
   if (fmt != ILL_IQ2_XXS && fmt != ILL_Q2_K && fmt != ILL_Q4_K && fmt != ILL_Q6_K) return ILL_ERR_UNSUPPORTED;
   const bool km = fmt == ILL_Q2_K || fmt == ILL_Q4_K;  // formats with mins: the sums of 16 of X come along
   if (ncols <= 0 || ncols % 256 || nrows <= 0 || ne <= 0 || ne > 65535 || total_rows < 0 || y_stride < nrows ||
@@ -1534,6 +1564,7 @@ static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptr
   p.one_ptr = one_ptr;
   p.one_count = (unsigned)total_rows;
   p.acc = acc;
+  p.over = over;
   p.status = device_status_word();
   if (ne > MM_MAX_NE) return ILL_ERR_TOO_LARGE;
   int dev = 0, sms = 148;

@@ -15,14 +15,6 @@
 
 namespace ill {
 
-// D4-SIGMOID (src/ds4f.lisp:248-250), each step rounded as written.
-// (One exponential and one division whatever the sign -- 1 / (1 + e^-x) for x >= 0, e^x / (1 + e^x) below, both with
-// e = exp(-|x|) -- so that a warp whose lanes differ in sign does not run both branches one after the other.)
-__device__ __forceinline__ float d4_sigmoid(float x) {
-  const float e = expf(-fabsf(x));
-  return __fdiv_rn(x >= 0.0f ? 1.0f : e, __fadd_rn(1.0f, e));
-}
-
 // MID[r*ff + j] = silu(min(G, c)) * clamp(U, +-c) * W[r]  (src/ds4f.lisp:1016-1019)
 __global__ void __launch_bounds__(256) swiglu_w_kernel(long long n, int ff, float clamp, const float* __restrict__ g,
                                                        const float* __restrict__ u, const float* __restrict__ w,
@@ -304,12 +296,13 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(long long rows, int ro
 // d4_swiglu_w, the Q8_K quantizer and the conversion to the tensor cores' operands in one pass: a warp a
 // 256-wide block of a row's middle values, lane l its elements 8l .. 8l+7.  Every step is the arithmetic of
 // swiglu_w_kernel, quant_q8_k_kernel and act_f16_kernel in turn, so the results are theirs bit for bit; the
-// middle values and their int8 form never go to memory.
+// middle values never go to memory, their int8 form only where XQ asks for it.
 __global__ void __launch_bounds__(256) swiglu_q8k_f16_kernel(long long nblocks, int ff, float clamp,
                                                              const float* __restrict__ g, const float* __restrict__ u,
                                                              const float* __restrict__ w, __half* __restrict__ mh,
                                                              __half* __restrict__ me, float* __restrict__ ms,
-                                                             const unsigned* __restrict__ rows_dev) {
+                                                             const unsigned* __restrict__ rows_dev, i8* __restrict__ xq,
+                                                             int16_t* __restrict__ xsum) {
   pdl_launch_dependents();
   pdl_wait();
   const long long b = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -323,11 +316,7 @@ __global__ void __launch_bounds__(256) swiglu_q8k_f16_kernel(long long nblocks, 
   const float us[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
   float v[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    float gv = gs[j], uv = us[j];
-    if (clamp > 1e-6f) { gv = fminf(gv, clamp); uv = fmaxf(-clamp, fminf(uv, clamp)); }
-    v[j] = __fmul_rn(__fmul_rn(__fmul_rn(gv, d4_sigmoid(gv)), uv), wv);
-  }
+  for (int j = 0; j < 8; ++j) v[j] = d4_middle(gs[j], us[j], wv, clamp);
   // QUANTIZE-Q8K! (src/kquant.lisp:130-167), the quantizer kernels' own routine
   int q[8];
   float d;
@@ -342,9 +331,15 @@ __global__ void __launch_bounds__(256) swiglu_q8k_f16_kernel(long long nblocks, 
   }
   ((uint4*)(mh + b * 256))[lane] = make_uint4(h[0], h[1], h[2], h[3]);
   if (lane == 0) ms[b] = d;
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  if (xq) {  // the int8 form too
+    uint32_t w0, w1;
+    q8k_pack(q, w0, w1);
+    ((uint2*)(xq + b * 256))[lane] = make_uint2(w0, w1);
+    if (!(lane & 1)) xsum[b * 16 + (lane >> 1)] = (int16_t)s;
+  }
   if (me) {
     // the block's sixteen sums of 16 as halves, then 48 zeros (the rest of the 64-wide K step of the mins' product)
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
     __half* e = me + b * 64;
     if (!(lane & 1)) e[lane >> 1] = __float2half_rn((float)s);
     if (lane < 24) ((uint32_t*)(e + 16))[lane] = 0u;
@@ -780,10 +775,10 @@ extern "C" int ill_moe_group_static(int64_t rows, int ne, int nu, ill_dptr sel, 
   return launch_kernel((const void*)group_scatter_kernel, dim3((unsigned)((rows + 255) / 256)), dim3(256), 0, args, st);
 }
 
-extern "C" int ill_swiglu_q8k_f16(int64_t rows, int ff, float clamp, ill_dptr g, ill_dptr u, ill_dptr w, ill_dptr mh,
-                                  ill_dptr me, ill_dptr ms, ill_dptr rows_dev, ill_stream stream) {
+static int swiglu_q8k(int64_t rows, int ff, float clamp, ill_dptr g, ill_dptr u, ill_dptr w, ill_dptr mh, ill_dptr me, ill_dptr ms,
+                      ill_dptr rows_dev, ill_dptr xq, ill_dptr xsum, ill_stream stream) {
   if (rows < 0 || ff <= 0 || ff % 256 || !g || !u || !mh || !ms) return ILL_ERR_ARG;
-  if ((g & 15) || (u & 15) || (w & 3) || (mh & 15) || (me & 15) || (ms & 3) || (rows_dev & 3)) return ILL_ERR_ALIGN;
+  if ((g & 15) || (u & 15) || (w & 3) || (mh & 15) || (me & 15) || (ms & 3) || (rows_dev & 3) || (xq & 15) || (xsum & 7)) return ILL_ERR_ALIGN;
   if (rows == 0) return ILL_OK;
   long long nb = rows * (ff / 256);
   const float* gp = (const float*)(uintptr_t)g;
@@ -793,9 +788,22 @@ extern "C" int ill_swiglu_q8k_f16(int64_t rows, int ff, float clamp, ill_dptr g,
   __half* ep = (__half*)(uintptr_t)me;
   float* sp = (float*)(uintptr_t)ms;
   const unsigned* rd = (const unsigned*)(uintptr_t)rows_dev;
-  void* args[] = {&nb, &ff, &clamp, &gp, &up, &wp, &hp, &ep, &sp, &rd};
+  i8* qp = (i8*)(uintptr_t)xq;
+  int16_t* qs = (int16_t*)(uintptr_t)xsum;
+  void* args[] = {&nb, &ff, &clamp, &gp, &up, &wp, &hp, &ep, &sp, &rd, &qp, &qs};
   return launch_kernel((const void*)swiglu_q8k_f16_kernel, dim3((unsigned)((nb + 7) / 8)), dim3(256), 0, args,
                        (cudaStream_t)stream);
+}
+
+extern "C" int ill_swiglu_q8k_f16(int64_t rows, int ff, float clamp, ill_dptr g, ill_dptr u, ill_dptr w, ill_dptr mh,
+                                  ill_dptr me, ill_dptr ms, ill_dptr rows_dev, ill_stream stream) {
+  return swiglu_q8k(rows, ff, clamp, g, u, w, mh, me, ms, rows_dev, 0, 0, stream);
+}
+
+extern "C" int ill_swiglu_q8k_both(int64_t rows, int ff, float clamp, ill_dptr g, ill_dptr u, ill_dptr w, ill_dptr mh, ill_dptr me,
+                                   ill_dptr ms, ill_dptr xq, ill_dptr xsum, ill_stream stream) {
+  if (!xq || !xsum) return ILL_ERR_ARG;
+  return swiglu_q8k(rows, ff, clamp, g, u, w, mh, me, ms, 0, xq, xsum, stream);
 }
 
 extern "C" int ill_moe_row_ptrs(int ne, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int64_t total_rows, ill_dptr row_ptrs,

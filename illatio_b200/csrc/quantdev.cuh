@@ -11,6 +11,20 @@
 
 namespace ill {
 
+// D4-SIGMOID (src/ds4f.lisp:248-250), each step rounded as written.
+// (One exponential and one division whatever the sign -- 1 / (1 + e^-x) for x >= 0, e^x / (1 + e^x) below, both with
+// e = exp(-|x|) -- so that a warp whose lanes differ in sign does not run both branches one after the other.)
+__device__ __forceinline__ float d4_sigmoid(float x) {
+  const float e = expf(-fabsf(x));
+  return __fdiv_rn(x >= 0.0f ? 1.0f : e, __fadd_rn(1.0f, e));
+}
+
+// The gated middle value of an expert: silu(min(G, c)) * clamp(U, +-c) * W  (src/ds4f.lisp:1016-1019)
+__device__ __forceinline__ float d4_middle(float g, float u, float w, float clamp) {
+  if (clamp > 1e-6f) { g = fminf(g, clamp); u = fmaxf(-clamp, fminf(u, clamp)); }
+  return __fmul_rn(__fmul_rn(__fmul_rn(g, d4_sigmoid(g)), u), w);
+}
+
 // One Q8_0 block: lane l holds element l.
 // lane l's quant of element l of a Q8_0 block, and the scale to store for the block (all lanes)
 __device__ __forceinline__ int q8_0_value(float v, int f16_scale, float& d_out) {

@@ -12,7 +12,7 @@ import torch
 
 from . import _lib
 from . import cuda_dense as D
-from .blocks import Q2_K
+from .blocks import IQ2_XXS, Q2_K
 from .cuda_ds4f import _DENSE_TYPES, ExpertPool, swiglu_w
 
 
@@ -77,6 +77,49 @@ def mm_id(pool, fmt, ncols, nrows, add, sc, xh, xe, xd, rmap, y):
               pool.n_expert, sc.rows, _ptr(xh), _ptr(xe), _ptr(xd), _ptr(rmap), 0, _ptr(y), nrows, _stream())
 
 
+# Rows an expert, on average, up to which the experts with a few rows are taken apart.  us of the routed experts, the chunk product alone /
+# with those apart: 288 experts of Q2_K with skewed popularity, 2 tokens 153 / 123, 64 757 / 467, 512 (a mean of 14) 1420 / 1061, 2048 (57)
+# 2591 / 2172, 8192 (228) 5873 / 5915; 256 experts of IQ2_XXS chosen alike, 64 tokens 1275 / 686, 256 (6) 1650 / 956, 512 (12) 1692 / 1307,
+# 1024 (24: hardly an expert has few) 1755 / 1773, 2048 (48) 1915 / 1906.  Where all 17 to 256 tokens choose the same experts the launches
+# that find nothing to do cost 10 us (64 tokens of six experts 121 / 130).
+FEW_MEAN = 64
+
+
+def few_rows(pool, n, nu):
+    """Rows an expert has, at most, for the products of a few rows an expert to do it in a chunk of N tokens (0: none of the chunk's)."""
+    if n * nu > FEW_MEAN * pool.n_expert or pool.gate_fmt not in (Q2_K, IQ2_XXS) or pool.down_fmt not in (Q2_K, IQ2_XXS):
+        return 0
+    if pool.n_expert > 512:
+        return 0
+    L = _lib.lib()
+    return min(L.ill_moe_few_most(pool.gate_fmt, pool.d), L.ill_moe_few_most(pool.down_fmt, pool.ff))
+
+
+def _few_rows_chunk(pool, n, nu, clamp, sc, shared, most, st):
+    """The chunk's experts that have up to MOST rows by the products for a few rows an expert, the others by the chunk's: the same
+    bits either way.  A token has an expert once, so up to MOST tokens have none of the others."""
+    d, ff, ne = pool.d, pool.ff, pool.n_expert
+    who = (_ptr(pool.ptrs_all), _ptr(sc.counts), _ptr(sc.bases), ne, sc.rows)
+    x, mid = (_ptr(sc.xq.xq), _ptr(sc.xq.xs), _ptr(sc.xq.xsum)), (_ptr(sc.midq.xq), _ptr(sc.midq.xs), _ptr(sc.midq.xsum))
+    if n <= most:
+        _lib.call("ill_moe_few_glu", pool.gate_fmt, d, ff, 0, pool.gate_bytes, *who, *x, _ptr(sc.rmap), float(clamp), _ptr(sc.wrow),
+                  _ptr(sc.mid), ff, st)
+        D.quant_q8(sc.mid, sc.midq)
+    else:
+        _lib.call("ill_act_f16_over", sc.rows, d, x[0], x[2], _ptr(sc.rmap), _ptr(sc.xh), _ptr(sc.xe), _ptr(sc.counts), ne, most, st)
+        _lib.call("ill_moe_few2", pool.gate_fmt, d, ff, 0, pool.gate_bytes, *who, *x, _ptr(sc.rmap), _ptr(sc.g), _ptr(sc.u), ff, st)
+        _lib.call("ill_moe_mm_id_over", pool.gate_fmt, d, ff, 0, pool.gate_bytes, *who, _ptr(sc.xh), _ptr(sc.xe), x[1], _ptr(sc.rmap),
+                  _ptr(sc.g), _ptr(sc.u), ff, most, st)
+        _lib.call("ill_swiglu_q8k_both", sc.rows, ff, float(clamp), _ptr(sc.g), _ptr(sc.u), _ptr(sc.wrow), _ptr(sc.mh), _ptr(sc.me), mid[1],
+                  mid[0], mid[2], st)
+    _lib.call("ill_moe_few", pool.down_fmt, ff, d, 2 * pool.gate_bytes, *who, *mid, 0, _ptr(sc.down), d, st)
+    if n > most:
+        _lib.call("ill_moe_mm_id_over", pool.down_fmt, ff, d, 2 * pool.gate_bytes, 0, *who, _ptr(sc.mh), _ptr(sc.me), mid[1], 0, _ptr(sc.down),
+                  0, d, most, st)
+    _lib.call("ill_moe_sum", d, nu, n, _ptr(sc.down), _ptr(sc.smap), _ptr(shared), _ptr(sc.moe), st)
+    return sc.moe
+
+
 def dk_ffn_routed_chunk(pool, norms, logits, nu, clamp, sc, mode=2, bias=None, scale=1.0, shared=None, fused=True):
     """DK-FFN-ROUTED-CHUNK (src/cuda-ds4f-prefill.lisp:315-356): the chunk's N
     tokens (NORMS [n, d] floats, LOGITS [n, ne] router logits) through their
@@ -88,6 +131,9 @@ def dk_ffn_routed_chunk(pool, norms, logits, nu, clamp, sc, mode=2, bias=None, s
     _lib.call("ill_moe_group", sc.rows, ne, nu, _ptr(sc.sel), _ptr(sc.w), _ptr(sc.group), _ptr(sc.counts),
               _ptr(sc.bases), _ptr(sc.rmap), _ptr(sc.smap), _ptr(sc.wrow), st)
     D.quant_q8(norms, sc.xq)                                       # each token's Q8_K, once
+    most = few_rows(pool, n, nu) if fused else 0
+    if most:
+        return _few_rows_chunk(pool, n, nu, clamp, sc, shared, most, st)
     act_f16(sc.xq, d, sc.rows, sc.rmap, sc.xh, sc.xe)
     if fused:  # gate and up in one launch
         _lib.call("ill_moe_mm_id2", pool.gate_fmt, d, ff, 0, pool.gate_bytes, _ptr(pool.ptrs_all), _ptr(sc.counts), _ptr(sc.bases),

@@ -1,0 +1,107 @@
+"""The experts' products for a few rows an expert (ill_moe_few, ill_moe_few2, ill_moe_few_glu): the bits of the chunk product, experts of
+more rows left to it (ill_moe_mm_id_over)."""
+import pytest
+import torch
+
+from illatio_b200 import _lib
+from illatio_b200 import blocks as B
+from illatio_b200 import cuda_dense as D
+from illatio_b200 import cuda_ds4f as M
+from illatio_b200 import cuda_ds4f_prefill as P
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _need_gpu(cuda_lib):
+    yield
+    assert D.device_status() == 0
+
+
+def _p(t):
+    return t.data_ptr()
+
+
+@pytest.mark.parametrize("fmt,base", [(B.IQ2_XXS, 0), (B.IQ2_XXS, 2), (B.Q2_K, 4)])
+@pytest.mark.parametrize("rows,cols", [(200, 768), (18, 256), (260, 2304), (64, 9216 - 512)])
+@pytest.mark.parametrize("counts", [(0, 1, 8, 9, 3, 0, 16), (17, 15, 16, 2000, 1), (16,), (0, 0, 5)])
+def test_few_rows_have_the_chunk_products_bits(fmt, base, rows, cols, counts):
+    """At the edges of a tile of eight and of the sixteen rows an expert may have, rows that are no multiple of sixteen, one block, an odd
+    number of them, and so many that eight tokens fit only; rows read through a map; nothing written past a row's end."""
+    ne, n = len(counts), sum(counts)
+    most = _lib.lib().ill_moe_few_most(fmt, cols)
+    assert most == (8 if fmt == B.IQ2_XXS and cols > 8192 else 16)
+    nbytes = B.matrix_bytes(fmt, rows, cols)
+    step = (2 * nbytes + 64) // 16 * 16
+    buf = torch.zeros(ne * step + 32, dtype=torch.uint8, device="cuda")
+    for e in range(ne):
+        buf[base + e * step:base + e * step + 2 * nbytes] = B.synth_matrix_torch(fmt, 2 * rows, cols, seed=e + rows)
+    g = torch.Generator(device="cuda").manual_seed(n + cols)
+    tokens = n // 2 + 1
+    act = D.quant_q8(torch.randn(tokens * cols, device="cuda", generator=g), D.make_qact(tokens * cols, "q8k"))
+    tmap = torch.randint(0, tokens, (n,), dtype=torch.int32, device="cuda", generator=g)
+    xh = torch.empty(n, cols, dtype=torch.float16, device="cuda")
+    xe = torch.empty(n, cols // 256, 64, dtype=torch.float16, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    ptrs = torch.tensor([_p(buf) + base + e * step for e in range(ne)], dtype=torch.int64, device="cuda")
+    cnt, bases = torch.tensor(counts, **i32), torch.tensor([sum(counts[:e]) for e in range(ne)], **i32)
+    who = (_p(ptrs), _p(cnt), _p(bases), ne, n)
+    stride = (rows + 3) // 4 * 4 + 4
+    _lib.call("ill_act_f16", n, cols, _p(act.xq), _p(act.xsum), _p(tmap), _p(xh), _p(xe), _lib.stream())
+    want = [torch.full((n, stride), 5.0, device="cuda") for _ in range(2)]
+    _lib.call("ill_moe_mm_id2", fmt, cols, rows, 0, nbytes, *who, _p(xh), _p(xe), _p(act.xs), _p(tmap), _p(want[0]), _p(want[1]), stride, _lib.stream())
+    few = torch.repeat_interleave(cnt <= most, cnt.long())[:, None]
+    x = (_p(act.xq), _p(act.xs), _p(act.xsum), _p(tmap))
+    one, two = torch.full((n, stride), 5.0, device="cuda"), [torch.full((n, stride), 5.0, device="cuda") for _ in range(2)]
+    _lib.call("ill_moe_few", fmt, cols, rows, nbytes, *who, *x, _p(one), stride, _lib.stream())
+    _lib.call("ill_moe_few2", fmt, cols, rows, 0, nbytes, *who, *x, _p(two[0]), _p(two[1]), stride, _lib.stream())
+    assert torch.equal(one, torch.where(few, want[1], 5.0))
+    for a, b in zip(two, want):
+        assert torch.equal(a, torch.where(few, b, 5.0))
+    w = torch.rand(n, device="cuda", generator=g)
+    mid, ref = torch.full((n, stride), 5.0, device="cuda"), torch.empty(n, rows, device="cuda")
+    _lib.call("ill_moe_few_glu", fmt, cols, rows, 0, nbytes, *who, *x, 1.5, _p(w), _p(mid), stride, _lib.stream())
+    if n:
+        a, b = (t[:, :rows].contiguous() for t in want)
+        _lib.call("ill_swiglu_w", n * rows, rows, 1.5, _p(a), _p(b), _p(w), _p(ref), _lib.stream())
+    assert torch.equal(mid[:, :rows], torch.where(few, ref, 5.0)) and (mid[:, rows:] == 5.0).all()
+    # the experts that are left: the operands first as ill_act_f16_over has them, over what was there
+    any_over = max(counts) > most
+    xh2, xe2 = torch.zeros_like(xh), torch.zeros_like(xe)
+    _lib.call("ill_act_f16_over", n, cols, _p(act.xq), _p(act.xsum), _p(tmap), _p(xh2), _p(xe2), _p(cnt), ne, most, _lib.stream())
+    assert torch.equal(xh2, xh if any_over else torch.zeros_like(xh)) and (not any_over or torch.equal(xe2, xe))
+    _lib.call("ill_moe_mm_id_over", fmt, cols, rows, 0, nbytes, *who, _p(xh2), _p(xe2), _p(act.xs), _p(tmap), _p(two[0]), _p(two[1]), stride, most,
+              _lib.stream())
+    assert torch.equal(two[0], want[0]) and torch.equal(two[1], want[1])
+
+
+def test_counts_that_are_not_the_routers_stay_inside_the_buffers():
+    """Numbers of rows past the last row there is, and negative ones: such an expert is left out, or its rows that are there."""
+    fmt, rows, cols, n = B.Q2_K, 48, 512, 10
+    w = B.synth_matrix_torch(fmt, rows, cols, seed=1)
+    act = D.quant_q8(torch.randn(n * cols, device="cuda"), D.make_qact(n * cols, "q8k"))
+    i32 = dict(dtype=torch.int32, device="cuda")
+    ptrs = torch.full((4,), _p(w), dtype=torch.int64, device="cuda")
+    cnt, bases = torch.tensor([4, -3, 9, 16], **i32), torch.tensor([0, 4, 8, 2 ** 31 - 1], **i32)
+    y = torch.full((n + 16, rows), 5.0, device="cuda")
+    _lib.call("ill_moe_few", fmt, cols, rows, 0, _p(ptrs), _p(cnt), _p(bases), 4, n, _p(act.xq), _p(act.xs), _p(act.xsum), 0, _p(y), rows, _lib.stream())
+    assert (y[4:] == 5.0).all() and (y[:4] != 5.0).any(1).all()
+
+
+@pytest.mark.parametrize("n,gate", [(16, B.IQ2_XXS), (17, B.Q2_K), (90, B.IQ2_XXS), (90, B.Q2_K)])
+def test_chunk_driver_with_and_without(n, gate):
+    """The chunk driver with its experts of a few rows apart and with all of them on the chunk product: the same bits.  Twelve experts of
+    which one is chosen by every token."""
+    d, ff, ne, nu = 512, 256, 12, 3
+    pool = M.make_expert_pool(B.synth_matrix(gate, ne * ff, d, seed=1), B.synth_matrix(gate, ne * ff, d, seed=2),
+                              B.synth_matrix(B.Q2_K, ne * d, ff, seed=3), d, ff, ne, gate_fmt=gate)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    norms, logits = torch.randn(n, d, device="cuda", generator=g), torch.randn(n, ne, device="cuda", generator=g)
+    logits[:, 4] += 30.0
+    sc = P.make_chunk_scratch(pool, n, nu)
+    assert P.few_rows(pool, n, nu) == 16
+    got = P.dk_ffn_routed_chunk(pool, norms, logits, nu, 10.0, sc).clone()
+    if n > 16:
+        assert sc.counts.max() > 16 and sc.counts.min() <= 16
+    want = P.dk_ffn_routed_chunk(pool, norms, logits, nu, 10.0, sc, fused=False)
+    assert torch.equal(got, want)
