@@ -19,11 +19,13 @@
 // Tensor memory: three accumulators of 128 columns (a block of 128 tokens, two of 64 or four of 32 a job, so that a hand-over is
 // always about 128 columns' worth), four stages of A.
 //
-// What bounds it: the drain's instructions.  A sum takes a conversion, a multiplication d_w * d_x, one with the sum and an addition,
-// 512 issue slots a scheduler for 128 x 128 x 32 where the product itself takes 64 cycles (the packed f32x2 forms take two slots
-// each); with the loads of the scales, the hand-overs and the unpacking 830 are executed, at 78 % issue about 1100 cycles.  us, int8
-// mma.sync (the kernel before) / now: 896 x 896 x 777 tokens 14.9 / 11.1, 896 x 4864 x 777 67 / 43, 4864 x 896 x 777 38 / 36,
-// 2048 x 4096 x 64 25 / 20, x 200 60 / 26, x 4096 297 / 288, 4096 x 2048 x 4096 298 / 277, 1536 x 5120 x 8192 550 / 570.
+// What bounds it: the drain.  A sum takes a conversion, a multiplication d_w * d_x, one with the sum and an addition.  The three are
+// packed, two sums an instruction: no faster by themselves, but the schedulers have a slot in two left, which the conversions and the
+// rest take (cycles of a scheduler, measured: two scalar multiply-adds and a conversion 3.2, a packed one and a conversion 2.5).  With the
+// loads of the scales, the hand-overs and the unpacking about 1000 cycles for 128 x 128 x 32, where the product itself takes 64.  us,
+// scalar / packed: 896 x 896 x 777 tokens 10.8 / 10.5, 896 x 4864 x 777 43.4 / 41.1, 4864 x 896 x 777 36.1 / 34.2, 2048 x 4096 x 64 20.7 / 20.1, x
+// 200 27.0 / 25.5, x 4096 296 / 274, 4096 x 2048 x 4096 287 / 267, 1536 x 5120 x 8192 561 / 522, 5120 x 1536 x 8192 519 / 484.  (The same with
+// int8 mma.sync, mm_q8_i8.cu: 896 x 4864 x 777 67, 2048 x 4096 x 200 60.)
 // Measured and taken back: eight drain warps with the next half on its way while one is scaled (NT 128: 309 -> 398); 16 x 256-bit
 // loads of tensor memory, a quarter of the shared memory's traffic (309 -> 319: it was no bound); raw blocks by cp.async of the
 // warps that take them apart (a step 0.5 -> 1.1 us); even shares whatever the rounds (4864 x 896 x 200 13.6 -> 16.3).
@@ -60,6 +62,7 @@ struct MqParams {
   int early;           // the next kernel may start before this one ends
   int ncol, share;     // SHARE of the NCOL columns of 16 tokens of all the tiles of rows one after another, in tiles of up to BM
   uint32_t zero;
+  uint64_t neg_zero;   // two of them (mul2_rn)
   unsigned* status;
 };
 struct MqMaps {
@@ -270,9 +273,9 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) mm_q8_kernel(const __grid_const
     uint32_t sph = 0, bph = 0;
     while (ok && tile.next(p)) {
       const int nvalid = tile.nvalid;
-      float out[TW];
+      uint64_t out[TW / 2];    // pairs of fp32
 #pragma unroll
-      for (int i = 0; i < TW; ++i) out[i] = 0.0f;
+      for (int i = 0; i < TW / 2; ++i) out[i] = 0ull;
       for (int st = 0; st < nsteps; ++st) {
         // (complete as soon as the step's first products are: what makes the scales visible here)
         bool lane_ok = mbar_wait(&full[s], sph, p.status, ST_MQ_WAIT + 5);
@@ -298,20 +301,20 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) mm_q8_kernel(const __grid_const
             for (int r = 0; r < 4; ++r) {
               const int blk = j * GB + 8 * r / TW, c = 8 * r % TW;
               const float dw = ws[blk * MQ_ROWS];
+              const uint64_t dw2 = pack2(dw, dw);
 #pragma unroll
               for (int i = 0; i < 8; i += 4) {
-                const float4 dx = *(const float4*)(xs + blk * NT + c + i);
-                out[c + i] = __fadd_rn(out[c + i], __fmul_rn((float)(int)v[r][i], __fmul_rn(dw, dx.x)));
-                out[c + i + 1] = __fadd_rn(out[c + i + 1], __fmul_rn((float)(int)v[r][i + 1], __fmul_rn(dw, dx.y)));
-                out[c + i + 2] = __fadd_rn(out[c + i + 2], __fmul_rn((float)(int)v[r][i + 2], __fmul_rn(dw, dx.z)));
-                out[c + i + 3] = __fadd_rn(out[c + i + 3], __fmul_rn((float)(int)v[r][i + 3], __fmul_rn(dw, dx.w)));
+                const ulonglong2 dx = *(const ulonglong2*)(xs + blk * NT + c + i);
+                uint64_t* o = out + (c + i) / 2;
+                o[0] = add2(o[0], mul2_rn(pack2((float)(int)v[r][i], (float)(int)v[r][i + 1]), mul2(dw2, dx.x), p.neg_zero));
+                o[1] = add2(o[1], mul2_rn(pack2((float)(int)v[r][i + 2], (float)(int)v[r][i + 3]), mul2(dw2, dx.y), p.neg_zero));
               }
             }
           }
         }
         if (!(ok = __all_sync(0xffffffffu, lane_ok))) break;
         // (ZERO is none that the compiler knows: the step's last scales have been used, not only asked for, when it is given back)
-        if (lane == 0) mbar_arrive(free + s + (__float_as_uint(out[TW - 1]) & p.zero));
+        if (lane == 0) mbar_arrive(free + s + ((uint32_t)(out[TW / 2 - 1] >> 32) & p.zero));
         if (++s == MQ_NS) { s = 0; sph ^= 1; }
       }
       const int row = tile.row0 + m;
@@ -328,7 +331,7 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) mm_q8_kernel(const __grid_const
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              float r = out[i0 + i];
+              float r = __uint_as_float((uint32_t)(out[(i0 + i) >> 1] >> (32 * (i & 1))));
               if (p.bias) r += bias;
               if (p.acc) r = old[i] + r;
               if (c0 + i0 + i < nvalid) yp[(long long)(i0 + i) * p.rows] = r;
@@ -499,6 +502,7 @@ int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t
   p.bias = (const float*)(uintptr_t)bias;
   p.acc = acc;
   p.n = n;
+  p.neg_zero = 0x8000000080000000ull;
   p.status = device_status_word();
   if ((long long)((rows + MQ_ROWS - 1) / MQ_ROWS) * ((n + 15) / 16) > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
   const MqDeal d = mq_deal(rows, n, sms);

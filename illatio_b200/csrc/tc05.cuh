@@ -121,11 +121,20 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
+
+// The product rounded by itself, for a sum behind it that rounds again: the assembler joins mul.rn.f32x2 and add.rn.f32x2 to one
+// rounding, and sees through a constant.  NZ: twice -0, which it must not know (A B + -0 is A B, whatever its sign).
+__device__ __forceinline__ uint64_t mul2_rn(uint64_t a, uint64_t b, uint64_t nz) { return fma2(a, b, nz); }
 
 // 16 bytes global -> shared, asynchronously
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {  // both 16-byte aligned
