@@ -38,10 +38,11 @@ bool mv_pick_lanes(int fmt, int units, bool glu, bool big, int* lanes, int* upt)
 int mvt_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum,
             const uint64_t* y, const uint64_t* bias, int acc, int n, void* stream);
 // the same for a chunk of tokens (more than 16): mmd.cu
-int mmd_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum, uint64_t y, uint64_t bias, int acc,
-            int n, void* stream);
-// ... of a Q8_0 matrix (mmd_try sends it there): mm_q8.cu, which leaves some to mm_q8_i8.cu
-int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t y, uint64_t bias, int acc, int n, void* stream);
+int mmd_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum, const uint64_t* y,
+            const uint64_t* bias, int acc, int n, void* stream);
+// ... of Q8_0 matrices (mmd_try sends them there): mm_q8.cu, which leaves some to mm_q8_i8.cu
+int mm_q8_try(int nmat, const uint64_t* w, const int* rows, int cols, uint64_t xq, uint64_t xs, const uint64_t* y, const uint64_t* bias, int acc,
+              int n, void* stream);
 int mm_q8_i8(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t y, uint64_t bias, int acc, int n, int sms, void* stream);
 float mm_q8_i8_step_us(int rows, int n, int sms);  // its estimate for 128 columns
 // up to 16 tokens of rows with many columns, the columns dealt to a CTA's warps: mmd.cu

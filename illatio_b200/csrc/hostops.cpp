@@ -266,8 +266,9 @@ PyObject* qkv_mul(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
       Py_RETURN_NONE;
     }
   }
+  if (n > 1 && !few(n)) return PyObject_Vectorcall(slow(S_qkv_mul), args, nargs, kwnames);  // a chunk
   int left = 0;
-  if (n > 1 && few(n)) {
+  if (n > 1) {
     const Mat q(a[0]), k(a[1]), v(a[2]);
     const Act x(a[3]);
     if (mul_3(q, k, &v, x, ptr(a[4]), ptr(a[5]), ptr(a[6]), OPT_PTR(a[7]), OPT_PTR(a[8]), OPT_PTR(a[9]), (int)n)) left = 3;

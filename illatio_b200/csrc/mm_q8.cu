@@ -34,6 +34,8 @@
 // copies and products in flight end, frees its tensor memory and returns.
 //
 // Replaces mm_q8_mma2 behind CMAT-MUL-N for prefill chunks (src/cuda-dense.lisp:220-255; src/cuda/dense.cu:885-1100).
+#include <string.h>
+
 #include "formats.cuh"
 #include "tc05.cuh"
 #include "host.h"
@@ -49,14 +51,19 @@ constexpr uint32_t MQ_RAW_BYTES = MQ_ROWS * MQ_PITCH, MQ_A_COL = 128 * MQ_NACC;
 constexpr int MQ_REGS_AUX = 32, MQ_REGS_DRAIN = 88, MQ_REGS_UNPACK = 56;
 constexpr int MQ_REGS_SUM = 128 * MQ_REGS_AUX + 32 * (MQ_DRAIN * MQ_REGS_DRAIN + MQ_UNPACK * MQ_REGS_UNPACK);
 
-struct MqParams {
-  int rows, nsteps;
-  int split;           // rows are a multiple of 16 bytes apart only two by two: the even ones and the odd ones have a map each
-  int off[2];          // where the first row's bytes start in the (even, odd) map
-  int cols;
-  const float* xs;
+constexpr int MQ_MATS = 3;
+struct MqMat {         // one of up to three matrices that share the activations
   float* y;
   const float* bias;
+  int rows, rt_end;    // tiles of rows of this one and those before it
+  int off[2];          // where the first row's bytes start in the (even, odd) map
+};
+struct MqParams {
+  MqMat m[MQ_MATS];
+  int nsteps;
+  int split;           // rows are a multiple of 16 bytes apart only two by two: the even ones and the odd ones have a map each
+  int cols;
+  const float* xs;
   int acc, n;
   int bm;              // tokens a tile, a multiple of 16; a CTA takes every gridDim.x-th tile -- or, SHARE not 0,
   int early;           // the next kernel may start before this one ends
@@ -66,7 +73,7 @@ struct MqParams {
   unsigned* status;
 };
 struct MqMaps {
-  CUtensorMap x, w[2];
+  CUtensorMap x, w[MQ_MATS][2];
 };
 
 template <int NT> struct MqGeom {
@@ -93,23 +100,27 @@ __device__ __forceinline__ void mq_cp_async4(void* dst, const void* src) {
 // A CTA's tiles, in order
 struct MqWalk {
   int pos, end, ntr;         // the tile, or column, next; past the last
-  int row0, tok0, nvalid;    // the tile
+  int mi, row0, tok0, nvalid;  // the tile: of which matrix, where
   __device__ __forceinline__ explicit MqWalk(const MqParams& p) {
-    ntr = (p.rows + MQ_ROWS - 1) / MQ_ROWS;
+    ntr = p.m[MQ_MATS - 1].rt_end;
     pos = p.share ? blockIdx.x * p.share : blockIdx.x;
     end = p.share ? min(pos + p.share, ntr * p.ncol) : ntr * ((p.n + p.bm - 1) / p.bm);
+  }
+  __device__ __forceinline__ void at_row_tile(const MqParams& p, int rt) {
+    mi = (rt >= p.m[0].rt_end) + (rt >= p.m[1].rt_end);
+    row0 = (rt - (mi ? p.m[mi - 1].rt_end : 0)) * MQ_ROWS;
   }
   __device__ __forceinline__ bool next(const MqParams& p) {
     if (pos >= end) return false;
     if (p.share) {
       const int rt = pos / p.ncol, col = pos - rt * p.ncol, take = min(min(p.bm / 16, end - pos), p.ncol - col);
-      row0 = rt * MQ_ROWS;
+      at_row_tile(p, rt);
       tok0 = 16 * col;
       nvalid = min(16 * take, p.n - tok0);
       pos += take;
     } else {                 // tiles of rows vary fastest: CTAs running together share X
       const int tt = pos / ntr;
-      row0 = (pos - tt * ntr) * MQ_ROWS;
+      at_row_tile(p, pos - tt * ntr);
       tok0 = tt * p.bm;
       nvalid = min(p.bm, p.n - tok0);
       pos += gridDim.x;
@@ -218,6 +229,8 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) mm_q8_kernel(const __grid_const
       // ---- the weights' raw blocks by TMA (they do not depend on the kernel before)
       int k = 0;
       while (ok && tile.next(p)) {
+        const int off0 = p.m[tile.mi].off[0], off1 = p.m[tile.mi].off[1];
+        const CUtensorMap* maps_w = maps.w[tile.mi];
         for (int st = 0; st < nsteps; ++st, ++k) {
           const int r = k % MQ_NRAW;
           ok = __all_sync(0xffffffffu, mbar_wait(&raw_free[r], ((uint32_t)(k / MQ_NRAW) & 1u) ^ 1u, p.status, ST_MQ_WAIT + 7));
@@ -226,10 +239,10 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) mm_q8_kernel(const __grid_const
             u8* dst = raw + r * MQ_RAW_BYTES;
             mbar_expect_tx(&raw_full[r], MQ_RAW_BYTES);
             if (p.split) {
-              tma_load_2d(dst, &maps.w[0], (p.off[0] + st * MQ_WSTEP) & ~15, tile.row0 / 2, &raw_full[r]);
-              tma_load_2d(dst + MQ_RAW_BYTES / 2, &maps.w[1], (p.off[1] + st * MQ_WSTEP) & ~15, tile.row0 / 2, &raw_full[r]);
+              tma_load_2d(dst, &maps_w[0], (off0 + st * MQ_WSTEP) & ~15, tile.row0 / 2, &raw_full[r]);
+              tma_load_2d(dst + MQ_RAW_BYTES / 2, &maps_w[1], (off1 + st * MQ_WSTEP) & ~15, tile.row0 / 2, &raw_full[r]);
             } else {
-              tma_load_2d(dst, &maps.w[0], (p.off[0] + st * MQ_WSTEP) & ~15, tile.row0, &raw_full[r]);
+              tma_load_2d(dst, &maps_w[0], (off0 + st * MQ_WSTEP) & ~15, tile.row0, &raw_full[r]);
             }
           }
           __syncwarp();
@@ -317,24 +330,25 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) mm_q8_kernel(const __grid_const
         if (lane == 0) mbar_arrive(free + s + ((uint32_t)(out[TW / 2 - 1] >> 32) & p.zero));
         if (++s == MQ_NS) { s = 0; sph ^= 1; }
       }
-      const int row = tile.row0 + m;
-      if (ok && row < p.rows) {
-        const float bias = p.bias ? p.bias[row] : 0.0f;
-        float* yp = p.y + (long long)(tile.tok0 + c0) * p.rows + row;
+      const MqMat& mat = p.m[tile.mi];
+      const int row = tile.row0 + m, rows = mat.rows;
+      if (ok && row < rows) {
+        const float bias = mat.bias ? mat.bias[row] : 0.0f;
+        float* yp = mat.y + (long long)(tile.tok0 + c0) * rows + row;
 #pragma unroll
         for (int i0 = 0; i0 < TW; i0 += 8) {
           if (c0 + i0 < nvalid) {
             float old[8];
             if (p.acc) {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) old[i] = c0 + i0 + i < nvalid ? yp[(long long)(i0 + i) * p.rows] : 0.0f;
+              for (int i = 0; i < 8; ++i) old[i] = c0 + i0 + i < nvalid ? yp[(long long)(i0 + i) * rows] : 0.0f;
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               float r = __uint_as_float((uint32_t)(out[(i0 + i) >> 1] >> (32 * (i & 1))));
-              if (p.bias) r += bias;
+              if (mat.bias) r += bias;
               if (p.acc) r = old[i] + r;
-              if (c0 + i0 + i < nvalid) yp[(long long)(i0 + i) * p.rows] = r;
+              if (c0 + i0 + i < nvalid) yp[(long long)(i0 + i) * rows] = r;
             }
           }
         }
@@ -346,10 +360,10 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) mm_q8_kernel(const __grid_const
     const int q = warp & 3, set = (warp - 4 - MQ_DRAIN) >> 2, row = 32 * q + lane, odd = p.split & row & 1;
     const uint32_t a0 = tmem_base + ((uint32_t)(q * 32) << 16) + MQ_A_COL;
     const u8* mine = raw + (p.split ? odd * (MQ_RAW_BYTES / 2) + (row >> 1) * MQ_PITCH : row * MQ_PITCH);
-    const int off = odd ? p.off[1] : p.off[0];
-    const bool by8 = (off & 7) == 0;                 // (the same for all: rows lie a multiple of eight bytes apart)
     int k = 0;
     while (ok && tile.next(p)) {
+      const int off = p.m[tile.mi].off[odd ? 1 : 0];
+      const bool by8 = (off & 7) == 0;               // (the same for all rows of a matrix: they lie a multiple of eight bytes apart)
       for (int st = 0; st < nsteps; ++st, ++k) {
         if ((k & 1) != set) continue;
         const int s = k % MQ_NS, r = k % MQ_NRAW;
@@ -447,9 +461,8 @@ struct MqDeal {
   int bm, share, grid;
   float us;
 };
-static MqDeal mq_deal(int rows, int n, int sms) {
+static MqDeal mq_deal(long long ntr, int n, int sms) {  // NTR tiles of rows
   MqDeal d = {};
-  const long long ntr = (rows + MQ_ROWS - 1) / MQ_ROWS;
   // Tokens a tile: the rounds of tiles on the SMs times a tile's time a step, us, over 21 matrices at 17 to 8192 tokens.  A step's
   // hand-overs cost 16 tokens as much as its arithmetic; above 64 tokens a block is a job of its own.  The choice takes the
   // fastest of them or one that is 0.3 % slower on average, 9 % at most.
@@ -487,26 +500,56 @@ static bool mq_i8_is_faster(const MqDeal& d, int rows, int cols, int n, int sms)
   return n > 32 && nsteps * mm_q8_i8_step_us(rows, n, sms) < 0.92f * (nsteps * d.us + 0.3f);
 }
 
-// N tokens of a Q8_0 matrix; ILL_ERR_UNSUPPORTED for what it is not written for.
-int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t y, uint64_t bias, int acc, int n, void* stream) {
-  if (n < 2 || cols % MQ_STEP || (xq & 15) || (xs & 15) || (w & 1)) return ILL_ERR_UNSUPPORTED;
+static long long mq_row_tiles(int rows) { return (rows + MQ_ROWS - 1) / MQ_ROWS; }
+
+// Whether one launch of several matrices is faster than one each: by the estimates, with the two microseconds that a launch behind
+// another costs beside its steps.  us, a launch each / one: 896 x 896 and 128 x 896, 17 tokens 11.2 / 5.9, 777 17.7 / 11.2,
+// 2048 26.7 / 19.4; 2 x 1536 x 5120, 64 tokens 49 / 26, 256 62 / 46.
+static bool mq_joint_is_faster(const MqDeal& d, int nmat, const int* rows, int cols, int n, int sms) {
+  const float nsteps = (float)(cols / MQ_STEP);
+  float apart = 0.0f;
+  for (int i = 0; i < nmat; ++i) {
+    const MqDeal one = mq_deal(mq_row_tiles(rows[i]), n, sms);
+    const float us = mq_i8_is_faster(one, rows[i], cols, n, sms) ? mm_q8_i8_step_us(rows[i], n, sms) : one.us;
+    apart += nsteps * us + 2.0f;
+  }
+  return nsteps * d.us + 2.0f < apart;
+}
+
+// N tokens of up to three Q8_0 matrices that share the activations; ILL_ERR_UNSUPPORTED for what it is not written for, and where
+// several are faster one by one.
+int mm_q8_try(int nmat, const uint64_t* w, const int* rows, int cols, uint64_t xq, uint64_t xs, const uint64_t* y, const uint64_t* bias, int acc,
+              int n, void* stream) {
+  if (n < 2 || cols % MQ_STEP || (xq & 15) || (xs & 15) || nmat < 1 || nmat > MQ_MATS) return ILL_ERR_UNSUPPORTED;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   MqParams p = {};
-  p.rows = rows;
+  long long ntr = 0;
+  for (int i = 0; i < MQ_MATS; ++i) {
+    if (i < nmat) {
+      if (w[i] & 1) return ILL_ERR_UNSUPPORTED;
+      p.m[i].rows = rows[i];
+      p.m[i].y = (float*)(uintptr_t)y[i];
+      p.m[i].bias = bias ? (const float*)(uintptr_t)bias[i] : nullptr;
+      ntr += mq_row_tiles(rows[i]);
+    }
+    if (ntr * ((n + 15) / 16) > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
+    p.m[i].rt_end = (int)ntr;
+  }
   p.cols = cols;
   p.nsteps = cols / MQ_STEP;
   p.xs = (const float*)(uintptr_t)xs;
-  p.y = (float*)(uintptr_t)y;
-  p.bias = (const float*)(uintptr_t)bias;
   p.acc = acc;
   p.n = n;
   p.neg_zero = 0x8000000080000000ull;
   p.status = device_status_word();
-  if ((long long)((rows + MQ_ROWS - 1) / MQ_ROWS) * ((n + 15) / 16) > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
-  const MqDeal d = mq_deal(rows, n, sms);
-  if (mq_i8_is_faster(d, rows, cols, n, sms)) return mm_q8_i8(w, rows, cols, xq, xs, y, bias, acc, n, sms, stream);
+  const MqDeal d = mq_deal(ntr, n, sms);
+  if (nmat > 1) {
+    if (!mq_joint_is_faster(d, nmat, rows, cols, n, sms)) return ILL_ERR_UNSUPPORTED;
+  } else if (mq_i8_is_faster(d, rows[0], cols, n, sms)) {
+    return mm_q8_i8(w[0], rows[0], cols, xq, xs, y[0], bias ? bias[0] : 0, acc, n, sms, stream);
+  }
   p.bm = d.bm;
   p.ncol = (n + 15) / 16;
   p.share = d.share;
@@ -521,12 +564,19 @@ int mm_q8_try(uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t
   if (!byte_map(&maps.x, xq, cols, n, cols, MQ_STEP, p.bm, true)) return cuda_fail(cudaErrorInvalidValue);
   // Rows lie a multiple of eight bytes apart; a map's have to lie a multiple of 16.  A row starts OFF bytes after a 16-byte boundary.
   p.split = row_bytes % 16 != 0;
-  for (int i = 0; i < 2; ++i) {
-    const uint64_t base = w + (p.split && i && rows > 1 ? row_bytes : 0), count = p.split ? (rows > 1 ? (rows + 1 - i) / 2 : 1) : rows;
-    p.off[i] = (int)(base & 15);
-    if (!byte_map(&maps.w[i], base & ~15ull, p.off[i] + row_bytes, count, p.split ? 2 * row_bytes : row_bytes, MQ_PITCH,
-                  p.split ? MQ_ROWS / 2 : MQ_ROWS, false))
-      return cuda_fail(cudaErrorInvalidValue);
+  for (int mi = 0; mi < MQ_MATS; ++mi) {
+    if (mi >= nmat) {
+      memcpy(maps.w[mi], maps.w[0], sizeof maps.w[mi]);
+      continue;
+    }
+    for (int i = 0; i < 2; ++i) {
+      const uint64_t base = w[mi] + (p.split && i && rows[mi] > 1 ? row_bytes : 0),
+                     count = p.split ? (rows[mi] > 1 ? (rows[mi] + 1 - i) / 2 : 1) : rows[mi];
+      p.m[mi].off[i] = (int)(base & 15);
+      if (!byte_map(&maps.w[mi][i], base & ~15ull, p.m[mi].off[i] + row_bytes, count, p.split ? 2 * row_bytes : row_bytes, MQ_PITCH,
+                    p.split ? MQ_ROWS / 2 : MQ_ROWS, false))
+        return cuda_fail(cudaErrorInvalidValue);
+    }
   }
   cudaStream_t st = (cudaStream_t)stream;
   if (p.bm <= 32) return mq_launch<32>(maps, p, grid, st);
@@ -540,7 +590,7 @@ using namespace ill;
 
 extern "C" int ill_test_q8_chunk_plan(int rows, int cols, int n, int sms, int* out) {
   if (!out || rows < 1 || cols < MQ_STEP || n < 2 || sms < 1) return ILL_ERR_ARG;
-  const MqDeal d = mq_deal(rows, n, sms);
+  const MqDeal d = mq_deal(mq_row_tiles(rows), n, sms);
   out[0] = d.bm;
   out[1] = d.share;
   out[2] = d.grid;

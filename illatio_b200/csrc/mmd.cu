@@ -218,14 +218,13 @@ template <> struct MdFrag<ILL_Q6_K> {
   }
 };
 
-// MINB = 2 (token tiles of 64): a thread stays within 128 registers and two CTAs share an SM
-template <int FMT, int NT8, int MINB>
-__global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p) {
-  extern __shared__ __align__(128) u8 smem[];
+// A CTA's tile BLOCK of a matrix
+template <int FMT, int NT8>
+__device__ __forceinline__ void md_tile(const MdParams& p, int block, u8* smem) {
   constexpr int TN = 8 * NT8, SB = MdFrag<FMT>::SB, MD_SPITCH = MdFrag<FMT>::SPITCH;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int ntt = (p.n + TN - 1) / TN, nthreads = blockDim.x;  // eight warps, or fewer when the matrix has few rows
-  const int tok0 = (int)(blockIdx.x % ntt) * TN, row_base = (int)(blockIdx.x / ntt) * (nthreads / 2) + warp * 16;
+  const int tok0 = block % ntt * TN, row_base = block / ntt * (nthreads / 2) + warp * 16;
   const int nsteps = p.nsteps, stages = p.stages;
   const bool live = row_base < p.rows;  // a warp whose rows are all past the end only helps to bring the activations
   u8* ring = smem + p.ring_off + (size_t)warp * stages * p.stage_bytes;
@@ -329,6 +328,30 @@ __global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p)
         *yp = p.acc ? *yp + v : v;
       }
     }
+}
+
+// MINB = 2 (token tiles of 64): a thread stays within 128 registers and two CTAs share an SM
+template <int FMT, int NT8, int MINB>
+__global__ void __launch_bounds__(MD_THREADS, MINB) mmd_kernel(const MdParams p) {
+  extern __shared__ __align__(128) u8 smem[];
+  md_tile<FMT, NT8>(p, (int)blockIdx.x, smem);
+}
+
+// Two or three matrices that share the activations (a chunk's K and V), their tiles one matrix after another: alone, 1024 rows of 512
+// tokens are a CTA or two of four warps an SM.  us, a launch each / one, 1024 x 2560
+// of Q4_K and of Q6_K: 17 tokens 31.8 / 16.6, 64 33.8 / 17.4, 256 40.1 / 25.7, 1024 96 / 66.
+constexpr int MD_MATS = 3;
+struct MdJoint {
+  MdParams m[MD_MATS];
+  int first[MD_MATS];   // its first CTA (of matrices that are not there: beyond the last)
+  int q6[MD_MATS];      // Q6_K, not Q4_K
+};
+template <int NT8, int MINB>
+__global__ void __launch_bounds__(MD_THREADS, MINB) mmd_joint_kernel(const __grid_constant__ MdJoint j) {
+  extern __shared__ __align__(128) u8 smem[];
+  const int block = (int)blockIdx.x, i = (block >= j.first[1]) + (block >= j.first[2]);
+  if (j.q6[i]) md_tile<ILL_Q6_K, NT8>(j.m[i], block - j.first[i], smem);
+  else md_tile<ILL_Q4_K, NT8>(j.m[i], block - j.first[i], smem);
 }
 
 // ---- up to sixteen tokens of rows too long for mvt.cu to keep the activations resident ------------------------
@@ -493,30 +516,24 @@ static int mmd_launch(const MdParams& p, int tn, size_t smem, int grid, cudaStre
   return launch_kernel(k, dim3(grid), dim3(32 * p.warps), smem, args, st);
 }
 
-// The chunk product on the tensor cores, for the formats and layouts it is written for; ILL_ERR_UNSUPPORTED
-// otherwise (the caller then takes the token loop of the CUDA-core kernel).
-int mmd_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum, uint64_t y, uint64_t bias, int acc,
-            int n, void* stream) {
-  if (fmt == ILL_Q8_0) return mm_q8_try(w, rows, cols, xq, xs, y, bias, acc, n, stream);
-  if (fmt != ILL_Q4_K && fmt != ILL_Q6_K) return ILL_ERR_UNSUPPORTED;
+// The chunk product on the tensor cores of up to three matrices that share the activations, for the formats and layouts it is written
+// for; ILL_ERR_UNSUPPORTED otherwise (the caller then takes the products one by one, one by the token loop of the CUDA-core kernel).
+int mmd_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int cols, uint64_t xq, uint64_t xs, uint64_t xsum, const uint64_t* y,
+            const uint64_t* bias, int acc, int n, void* stream) {
+  if (fmts[0] == ILL_Q8_0) {
+    for (int i = 1; i < nmat; ++i)
+      if (fmts[i] != ILL_Q8_0) return ILL_ERR_UNSUPPORTED;
+    return mm_q8_try(nmat, w, rows, cols, xq, xs, y, bias, acc, n, stream);
+  }
+  bool q4 = false;
+  for (int i = 0; i < nmat; ++i) {
+    if (fmts[i] != ILL_Q4_K && fmts[i] != ILL_Q6_K) return ILL_ERR_UNSUPPORTED;
+    q4 = q4 || fmts[i] == ILL_Q4_K;
+  }
   if (n < 2) return ILL_ERR_UNSUPPORTED;
   // 16-byte pieces of the activations are copied as they lie: the quants of a step, Q4_K's sixteen sums
   if ((xq & 15) || cols % 256) return ILL_ERR_UNSUPPORTED;
-  if (fmt == ILL_Q4_K && (xsum & 15)) return ILL_ERR_UNSUPPORTED;
-  const int bw = fmt_block_weights(fmt), bb = fmt_block_bytes(fmt);
-  MdParams p = {};
-  p.w = (const u8*)(uintptr_t)w;
-  p.rows = rows;
-  p.cols = cols;
-  p.row_bytes = cols / bw * bb;
-  p.nsteps = cols / 256;
-  p.xq = (const i8*)(uintptr_t)xq;
-  p.xs = (const float*)(uintptr_t)xs;
-  p.xsum = (const int16_t*)(uintptr_t)xsum;
-  p.y = (float*)(uintptr_t)y;
-  p.bias = (const float*)(uintptr_t)bias;
-  p.acc = acc;
-  p.n = n;
+  if (q4 && (xsum & 15)) return ILL_ERR_UNSUPPORTED;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
@@ -524,35 +541,73 @@ int mmd_try(int fmt, uint64_t w, int rows, int cols, uint64_t xq, uint64_t xs, u
   // of 64 keep a thread within 128 registers so that two CTAs share an SM -- measured equal to slower where both
   // fill the machine, so they are for chunks of up to 64 tokens and for matrices with so few rows that tiles of 128
   // would leave the SMs with fewer than eight warps each; 32 below that.
+  long long tiles16 = 0;
+  for (int i = 0; i < nmat; ++i) tiles16 += (rows[i] + 15) / 16;
   int tn = n <= 32 ? 32 : n <= 64 ? 64 : 128;
-  while (tn > 32 && (long long)((rows + 15) / 16) * ((n + tn - 1) / tn) < 8ll * sms) tn >>= 1;
-  // Warps a CTA: eight (128 rows), fewer when that would leave SMs without a CTA (few rows of many columns)
-  p.warps = MD_WARPS;
-  while (p.warps > 1 && (long long)((rows + 16 * p.warps - 1) / (16 * p.warps)) * ((n + tn - 1) / tn) < sms) p.warps >>= 1;
-  // a row's step: its 16-byte aligned span (a block is read from its stage once a step, so the rows' pitch need not
-  // spread them over the banks); 16 bytes after the last row for the unaligned loads' second word
-  p.pitch = (bb + 15 + 15) / 16 * 16;
-  p.stage_bytes = (uint32_t)(16 * p.pitch + 16);
-  uint32_t off = (uint32_t)tn * MD_XPITCH;
-  p.xs_off = off;
-  off += 4u * tn;
-  off = (off + 15) / 16 * 16;
-  p.xsum_off = off;
-  if (fmt == ILL_Q4_K) off += (uint32_t)tn * MdFrag<ILL_Q4_K>::SPITCH;
-  p.xbuf_bytes = (off + 127) / 128 * 128;
-  // stages of weights and activations: four, three where that is all that fits, two where two CTAs share an SM
-  const uint32_t stage = (uint32_t)p.warps * p.stage_bytes + p.xbuf_bytes;
-  p.stages = tn == 64 ? 2 : 226 * 1024 / stage < 4 ? 226 * 1024 / stage : 4;
-  p.ring_off = p.stages * p.xbuf_bytes;
-  const size_t smem = (size_t)p.stages * stage;
+  while (tn > 32 && tiles16 * ((n + tn - 1) / tn) < 8ll * sms) tn >>= 1;
+  // Warps a CTA: eight (128 rows), or four when that would leave SMs without a CTA (few rows of many columns).  (Fewer than four bring
+  // the activations too slowly, 64 to 1536 rows of 1024 to 17408 columns at 17 to 512 tokens: 256 x 2560 x 64 tokens of Q4_K with one, two,
+  // four, eight warps 18.4 / 16.1 / 15.6 / 22.4 us, 1024 x 5120 x 128 35.6 / 33.0 / 30.2 / 43.4, 64 x 17408 x 17 112 / 99 / 97 / 97; four the
+  // fastest of them or within 2 %.)
+  const int ntt = (n + tn - 1) / tn;
+  int warps = MD_WARPS;
+  auto ctas = [&](int m) { return (long long)((rows[m] + 16 * warps - 1) / (16 * warps)) * ntt; };
+  auto all_ctas = [&] {
+    long long c = 0;
+    for (int i = 0; i < nmat; ++i) c += ctas(i);
+    return c;
+  };
+  while (warps > 4 && all_ctas() < sms) warps >>= 1;
+  // Several matrices go in one launch where its CTAs run side by side: two of four warps, or of 64 tokens, fit an SM.  Beyond that the SMs
+  // are full with a launch each (1024 x 2560 of Q4_K and of Q6_K, a launch each / one: 256 tokens 40.1 / 25.7, 512 45.0 / 47.2).
+  if (nmat > 1 && all_ctas() > (long long)sms * (warps <= 4 || tn == 64 ? 2 : 1)) return ILL_ERR_UNSUPPORTED;
+  MdJoint jt = {};
+  size_t smem = 0;
+  for (int i = 0; i < nmat; ++i) {
+    const int bw = fmt_block_weights(fmts[i]), bb = fmt_block_bytes(fmts[i]);
+    MdParams& p = jt.m[i];
+    p.w = (const u8*)(uintptr_t)w[i];
+    p.rows = rows[i];
+    p.cols = cols;
+    p.row_bytes = cols / bw * bb;
+    p.nsteps = cols / 256;
+    p.xq = (const i8*)(uintptr_t)xq;
+    p.xs = (const float*)(uintptr_t)xs;
+    p.xsum = (const int16_t*)(uintptr_t)xsum;
+    p.y = (float*)(uintptr_t)y[i];
+    p.bias = bias ? (const float*)(uintptr_t)bias[i] : nullptr;
+    p.acc = acc;
+    p.n = n;
+    p.warps = warps;
+    // a row's step: its 16-byte aligned span (a block is read from its stage once a step, so the rows' pitch need not
+    // spread them over the banks); 16 bytes after the last row for the unaligned loads' second word
+    p.pitch = (bb + 15 + 15) / 16 * 16;
+    p.stage_bytes = (uint32_t)(16 * p.pitch + 16);
+    uint32_t off = (uint32_t)tn * MD_XPITCH;
+    p.xs_off = off;
+    off += 4u * tn;
+    off = (off + 15) / 16 * 16;
+    p.xsum_off = off;
+    if (fmts[i] == ILL_Q4_K) off += (uint32_t)tn * MdFrag<ILL_Q4_K>::SPITCH;
+    p.xbuf_bytes = (off + 127) / 128 * 128;
+    // stages of weights and activations: four, three where that is all that fits, two where two CTAs share an SM
+    const uint32_t stage = (uint32_t)p.warps * p.stage_bytes + p.xbuf_bytes;
+    p.stages = tn == 64 ? 2 : 226 * 1024 / stage < 4 ? 226 * 1024 / stage : 4;
+    p.ring_off = p.stages * p.xbuf_bytes;
+    if (p.stages * (size_t)stage > smem) smem = p.stages * (size_t)stage;
+    jt.q6[i] = fmts[i] == ILL_Q6_K;
+  }
   if (smem > 226 * 1024) return ILL_ERR_UNSUPPORTED;
-  const long long grid = (long long)((rows + 16 * p.warps - 1) / (16 * p.warps)) * ((n + tn - 1) / tn);
+  const long long grid = all_ctas();
   if (grid > 0x7fffffffll) return ILL_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
-  switch (fmt) {
-    case ILL_Q4_K: return mmd_launch<ILL_Q4_K>(p, tn, smem, (int)grid, st);
-    default: return mmd_launch<ILL_Q6_K>(p, tn, smem, (int)grid, st);
-  }
+  if (nmat == 1) return fmts[0] == ILL_Q4_K ? mmd_launch<ILL_Q4_K>(jt.m[0], tn, smem, (int)grid, st) : mmd_launch<ILL_Q6_K>(jt.m[0], tn, smem, (int)grid, st);
+  for (int i = 1; i < MD_MATS; ++i) jt.first[i] = i < nmat ? jt.first[i - 1] + (int)ctas(i - 1) : 0x7fffffff;
+  const void* k = tn == 32 ? (const void*)mmd_joint_kernel<4, 1> : tn == 64 ? (const void*)mmd_joint_kernel<8, 2> : (const void*)mmd_joint_kernel<16, 1>;
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return cuda_fail(e);
+  void* args[] = {&jt};
+  return launch_kernel(k, dim3((unsigned)grid), dim3(32 * warps), smem, args, st);
 }
 
 template <int FMT>

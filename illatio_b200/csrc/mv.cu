@@ -867,7 +867,7 @@ int mv_common(int fmt, int mode, int nmat, const ill_dptr* w, const int* rows, i
     // a few tokens of rows too long for their activations to stay in shared memory
     if (rc_t == ILL_ERR_UNSUPPORTED && n <= 16) rc_t = mmk_try(fmt, w[0], rows[0], cols, xq, xs, xsum, y[0], bias ? bias[0] : 0, acc, n, stream);
     // a chunk
-    if (rc_t == ILL_ERR_UNSUPPORTED) rc_t = mmd_try(fmt, w[0], rows[0], cols, xq, xs, xsum, y[0], bias ? bias[0] : 0, acc, n, stream);
+    if (rc_t == ILL_ERR_UNSUPPORTED) rc_t = mmd_try(1, &fmt, w, rows, cols, xq, xs, xsum, y, bias, acc, n, stream);
     if (rc_t != ILL_ERR_UNSUPPORTED) return rc_t;
   }
   if (n > MV_MAX_TOK) return ILL_ERR_UNSUPPORTED;  // the token loop below takes 16 at most: the caller splits the chunk
@@ -1003,6 +1003,7 @@ extern "C" int ill_mv_3n(int fmt0, int fmt1, int fmt2, ill_dptr w0, ill_dptr w1,
     if (ys[i] & 3) return ILL_ERR_ALIGN;
   }
   if (xq & 15 || xs & 3 || xsum & 7) return ILL_ERR_ALIGN;
+  if (n > 16) return mmd_try(nmat, fs, ws, rs, cols, xq, xs, xsum, ys, bs, 0, n, stream);
   return mvt_try(nmat, fs, ws, rs, cols, xq, xs, xsum, ys, bs, 0, n, stream);
 }
 

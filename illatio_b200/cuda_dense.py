@@ -127,10 +127,15 @@ def _rmsnorm_q8(x, w, act, d, eps, n=1, h=None, f16_scale=True):
         act._cf = cf
 
 
+def _by_tc(w, act, n, bias):
+    """Whether a product of a chunk goes to the tcgen05 kernel of the K formats."""
+    return ((w.type == 1 or (w.type == 2 and TC_Q6K)) and act.kind == "q8k" and n >= TC_MIN_TOKENS and w.rows >= TC_MIN_ROWS and w.rows % 4 == 0 and bias is None
+            and w.qs.data_ptr() % 16 == 0 and act.xq.numel() == n * w.cols)
+
+
 def _cmat_mul(w, act, y, n=1, bias=None, acc=False):
     """cmat_mul of a chunk, or of a few tokens that have to be split."""
-    if ((w.type == 1 or (w.type == 2 and TC_Q6K)) and act.kind == "q8k" and n >= TC_MIN_TOKENS and w.rows >= TC_MIN_ROWS and w.rows % 4 == 0 and bias is None
-            and w.qs.data_ptr() % 16 == 0 and act.xq.numel() == n * w.cols):
+    if _by_tc(w, act, n, bias):
         # a prefill chunk of a Q4_K / Q6_K matrix: the tcgen05 kernel (the activations' fp16 form is made once per quantization)
         return cmat_mul_tc(w, _chunk_f16_of(act, n, w.cols), y, acc=acc)
     done = 0
@@ -166,9 +171,28 @@ def _side_stream(device):
     return s
 
 
+def chunk_mul_3(mats, act, n):
+    """The products of a chunk of N tokens that share the activations ACT, MATS a list of (matrix, output, bias): two or three in one
+    launch where that is to be had (ill_mv_3n), else one by one; those of the tcgen05 kernel of the K formats by themselves."""
+    joint = [m for m in mats if not _by_tc(m[0], act, n, m[2])]
+    a = joint[0][0] if joint else None
+    if 2 <= len(joint) <= 3 and n > 16 and all(w.cols == a.cols and (w.type == 0) == (a.type == 0) and w.rows > 0 for w, _, _ in joint) and (a.type == 0) == (act.kind == "q8"):
+        w, y, b = ([m[i] for m in joint] + [None] * (3 - len(joint)) for i in range(3))
+        rc = _lib.status("ill_mv_3n", *(m.type if m else 0 for m in w), *(_ptr(m.qs) if m else 0 for m in w), *(m.rows if m else 0 for m in w),
+                         a.cols, _ptr(act.xq), _ptr(act.xs), 0 if act.kind == "q8" else _ptr(act.xsum), *map(_ptr, y), *map(_ptr, b), n, _stream())
+        if rc == 0:
+            mats = [m for m in mats if all(m is not j for j in joint)]
+        elif rc != 3:
+            _lib.fail("ill_mv_3n", rc)
+    for w, y, b in mats:
+        cmat_mul(w, act, y, n, bias=b)
+
+
 def _qkv_mul(wq, wk, wv, act, q, k, v, bq=None, bk=None, bv=None, n=1):
-    """qkv_mul of one token with a V in a format of its own, in a stream that is being captured: Q and K in one
+    """qkv_mul of a chunk; or of one token with a V in a format of its own, in a stream that is being captured: Q and K in one
     launch, V in its own beside it (both read the same activations; in the graph this is a fork and a join)."""
+    if n != 1:
+        return chunk_mul_3([(wq, q, bq), (wk, k, bk), (wv, v, bv)], act, n)
     cur = torch.cuda.current_stream()
     side = _side_stream(cur.device)
     side.wait_stream(cur)

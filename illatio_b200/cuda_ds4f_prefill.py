@@ -214,8 +214,7 @@ def dk_ffn_head_chunk(cur, norm_w, eps, router, sh_gate, sh_up, sh_down, clamp, 
     sg, su = hs.sg[:n], hs.su[:n]
     D.rmsnorm_q8(cur, norm_w, hs.nq, d, eps, n=n, h=norm2, f16_scale=False)     # DK-RMS and DK-Q8MM's quantization of NORM2
     _lib.call("ill_mv_dense", _DENSE_TYPES[router.dtype], _ptr(router), ne, d, _ptr(norm2), _ptr(logits), n, ne, _stream())
-    D.cmat_mul(sh_gate, hs.nq, sg, n)
-    D.cmat_mul(sh_up, hs.nq, su, n)
+    D.chunk_mul_3([(sh_gate, sg, None), (sh_up, su, None)], hs.nq, n)
     _lib.call("ill_swiglu_w", n * hs.ff, hs.ff, float(clamp), _ptr(sg), _ptr(su), 0, _ptr(sg), _stream())
     D.quant_q8(sg, hs.mq, f16_scale=False)
     D.cmat_mul(sh_down, hs.mq, sout, n)
