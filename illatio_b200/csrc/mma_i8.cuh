@@ -106,6 +106,16 @@ __device__ __forceinline__ void copy_segment(u8* dst, const u8* src, uint32_t le
     if (a + 64 * k < end) cp_async16(dst + 16 * t + 64 * k, a + 64 * k);
 }
 
+// The same to the address DST in shared memory, this lane's first piece's (T's).
+template <int NCH>
+__device__ __forceinline__ void copy_segment_at(uint32_t dst, const u8* src, uint32_t len, int t) {
+  const uint32_t lo = (uint32_t)(uintptr_t)src & 15u, end = lo + len;
+  const u8* a = src - lo + 16 * t;
+#pragma unroll
+  for (int k = 0; k < (NCH + 3) / 4; ++k)
+    if (16u * t + 64u * k < end) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 64 * k), "l"(a + 64 * k) : "memory");
+}
+
 // get_scale_min_k4 (src/kquant.lisp:64-72) for group J of the 12 packed bytes at Q
 __device__ __forceinline__ void scale_min_k4(const u8* q, int j, int& sc, int& mn) {
   if (j < 4) { sc = q[j] & 63; mn = q[j + 4] & 63; }

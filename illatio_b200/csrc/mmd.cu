@@ -346,8 +346,8 @@ struct MdJoint {
   int first[MD_MATS];   // its first CTA (of matrices that are not there: beyond the last)
   int q6[MD_MATS];      // Q6_K, not Q4_K
 };
-template <int NT8, int MINB>
-__global__ void __launch_bounds__(MD_THREADS, MINB) mmd_joint_kernel(const __grid_constant__ MdJoint j) {
+template <int NT8, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) mmd_joint_kernel(const __grid_constant__ MdJoint j) {
   extern __shared__ __align__(128) u8 smem[];
   const int block = (int)blockIdx.x, i = (block >= j.first[1]) + (block >= j.first[2]);
   if (j.q6[i]) md_tile<ILL_Q6_K, NT8>(j.m[i], block - j.first[i], smem);
@@ -558,9 +558,12 @@ int mmd_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
     return c;
   };
   while (warps > 4 && all_ctas() < sms) warps >>= 1;
-  // Several matrices go in one launch where its CTAs run side by side: two of four warps, or of 64 tokens, fit an SM.  Beyond that the SMs
-  // are full with a launch each (1024 x 2560 of Q4_K and of Q6_K, a launch each / one: 256 tokens 40.1 / 25.7, 512 45.0 / 47.2).
-  if (nmat > 1 && all_ctas() > (long long)sms * (warps <= 4 || tn == 64 ? 2 : 1)) return ILL_ERR_UNSUPPORTED;
+  // Several matrices go in one launch where its CTAs run side by side: two of four warps, or of 64 tokens, fit an SM, and with two
+  // stages and 128 registers four of four warps (a launch each / two CTAs an SM / four, us: 1024 x 2560 of Q4_K and of Q6_K, 256 tokens
+  // 43 / 25.7 / 34, 512 45.0 / 47.2 / 42.6; 2 x 1024 x 5120 of Q6_K, 512 91 / 91 / 79).  Beyond that the SMs are full with a launch each.
+  if (nmat > 1 && tn == 32 && all_ctas() > sms) warps = 4;
+  const bool four = nmat > 1 && tn == 32 && warps == 4 && all_ctas() > 2ll * sms;
+  if (nmat > 1 && all_ctas() > (long long)sms * (four ? 4 : warps <= 4 || tn == 64 ? 2 : 1)) return ILL_ERR_UNSUPPORTED;
   MdJoint jt = {};
   size_t smem = 0;
   for (int i = 0; i < nmat; ++i) {
@@ -592,7 +595,7 @@ int mmd_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
     p.xbuf_bytes = (off + 127) / 128 * 128;
     // stages of weights and activations: four, three where that is all that fits, two where two CTAs share an SM
     const uint32_t stage = (uint32_t)p.warps * p.stage_bytes + p.xbuf_bytes;
-    p.stages = tn == 64 ? 2 : 226 * 1024 / stage < 4 ? 226 * 1024 / stage : 4;
+    p.stages = tn == 64 || four ? 2 : 226 * 1024 / stage < 4 ? 226 * 1024 / stage : 4;
     p.ring_off = p.stages * p.xbuf_bytes;
     if (p.stages * (size_t)stage > smem) smem = p.stages * (size_t)stage;
     jt.q6[i] = fmts[i] == ILL_Q6_K;
@@ -603,7 +606,8 @@ int mmd_try(int nmat, const int* fmts, const uint64_t* w, const int* rows, int c
   cudaStream_t st = (cudaStream_t)stream;
   if (nmat == 1) return fmts[0] == ILL_Q4_K ? mmd_launch<ILL_Q4_K>(jt.m[0], tn, smem, (int)grid, st) : mmd_launch<ILL_Q6_K>(jt.m[0], tn, smem, (int)grid, st);
   for (int i = 1; i < MD_MATS; ++i) jt.first[i] = i < nmat ? jt.first[i - 1] + (int)ctas(i - 1) : 0x7fffffff;
-  const void* k = tn == 32 ? (const void*)mmd_joint_kernel<4, 1> : tn == 64 ? (const void*)mmd_joint_kernel<8, 2> : (const void*)mmd_joint_kernel<16, 1>;
+  const void* k = four ? (const void*)mmd_joint_kernel<4, 128, 4> : tn == 32 ? (const void*)mmd_joint_kernel<4, MD_THREADS, 1>
+                  : tn == 64 ? (const void*)mmd_joint_kernel<8, MD_THREADS, 2> : (const void*)mmd_joint_kernel<16, MD_THREADS, 1>;
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e);
   void* args[] = {&jt};

@@ -24,8 +24,8 @@
 // 142 / 117.  What gave it: one launch; activations that are all asked for before anything is waited for (4 us a launch); the deal;
 // Q4_K's mins against the sums of 16 by two products, its scales four at a time (half the instructions); ldmatrix.
 //
-// The 2-bit formats' blocks are in mtblock.cuh.  us, the token loop of mv.cu (a pass of dp4a a token) / now: Q2_K 151936 x 2560, 4 tokens 236 / 60,
-// 16 tokens 923 / 74; IQ2_XXS 232 / 85 and 768 / 98; 4096 x 4096, 4 tokens 29.5 / 4.6 and 27.2 / 6.3; 512 x 512, 2 tokens 2.9 / 2.1 and 3.1 / 3.1.
+// The 2-bit formats' blocks are in mtblock.cuh.  us, the token loop of mv.cu (a pass of dp4a a token) / now: Q2_K 151936 x 2560, 4 tokens 236 / 57,
+// 16 tokens 923 / 70; IQ2_XXS 232 / 80 and 768 / 93; 4096 x 4096, 4 tokens 29.5 / 4.5 and 27.2 / 6.1; 512 x 512, 2 tokens 2.9 / 2.1 and 3.1 / 3.1.
 //
 // mma.sync is the legacy tensor path: right here, where N is 8 or 16 and the bound is HBM; the chunk-sized
 // products (hundreds of rows of X an expert) use tcgen05 (mm_id.cu).
@@ -59,6 +59,7 @@ struct MtMat {
 struct MtFmt {
   int row_bytes;
   int cb, npieces;      // blocks a staged piece (a warp's unit of copying); pieces a row
+  uint32_t piece_bytes; // of a row
   int pitch;            // bytes between the rows of a staged piece
   u8 sums[MT_SUMS];     // the partial sums of a group's warp (bits)
 };
@@ -265,39 +266,52 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
   const int tile0 = grp * gridDim.x + blockIdx.x, tile_step = gridDim.x * p.groups;
   i8* xq_s = (i8*)smem;
   float* xs_s = (float*)(smem + p.xs_off);
-  u8* ring = smem + p.ring_off + (size_t)cwarp * stages * p.stage_bytes;
+  const uint32_t ring = smem_u32(smem) + p.ring_off + cwarp * stages * p.stage_bytes;
   const int nb = p.nblocks;
   float* part = (float*)(smem + p.part_off) + (size_t)grp * 2 * p.nsums * NTOK * PP;  // [group][2][sums][tokens][PP]
   const int ntiles = p.m[MT_MATS - 1].tile_end;
 
   auto matrix = [&](int tile) { return (tile >= p.m[0].tile_end) + (tile >= p.m[1].tile_end); };
   auto format = [&](int mi) { return TWO ? p.m[mi].alt : 0; };
-  // this warp's pieces in order: its group's tiles tile0, + tile_step, ...; of each, sum after sum, the pieces of its sums
-  int n_tile = tile0, n_pc = 0, n_mi = 0, i_slot = 0;
+  // this warp's pieces in order: its group's tiles tile0, + tile_step, ...; of each, sum after sum, the pieces of its sums.  What a
+  // tile's pieces share is worked out once a tile: 32-bit offsets from the lane's row are left for a piece.  (722 instructions a block of
+  // Q6_K, 555 now, of which 355 take it apart and multiply it.  A head of 151936 x 2560, 16 tokens 121.8 / 117.4 us, of Q2_K, 4 tokens 60.5 /
+  // 56.6; where latencies bound it nothing: gate and up of 2 x 17408 x 5120, 4 tokens 46.7 / 45.9.)
+  const int g = lane >> 2, t = lane & 3;
+  int n_tile = tile0, n_pc = 0;
   unsigned n_left = 0;
+  const u8* n_src = nullptr;   // the lane's row g of the tile; row g + 8 is N_ROW8 bytes on
+  uint32_t n_row8 = 0, n_dst = ring, n_end = 0;  // where the next stage starts; the end of the ring
+  int n_rows = 0, n_alt = 0;   // rows of the matrix from row g on
   auto at_tile = [&]() {  // on to the first tile from n_tile on that this warp has a sum of
     while (n_tile < ntiles) {
-      n_mi = matrix(n_tile);
-      n_left = p.f[format(n_mi)].sums[wg];
-      if (n_left) { n_pc = __ffs(n_left) - 1; return; }
+      const int mi = matrix(n_tile);
+      const MtFmt& f = p.f[format(mi)];
+      n_left = f.sums[wg];
+      if (n_left) {
+        const int row = (n_tile - (mi ? p.m[mi - 1].tile_end : 0)) * MT_ROWS + g;
+        n_pc = __ffs(n_left) - 1;
+        n_src = p.m[mi].w + (long long)row * f.row_bytes;
+        n_row8 = 8u * (uint32_t)f.row_bytes;
+        n_rows = p.m[mi].rows - row;
+        n_alt = format(mi);
+        return;
+      }
       n_tile += tile_step;
     }
   };
   at_tile();
-  const int g = lane >> 2, t = lane & 3;
+  n_end = ring + stages * p.stage_bytes;
   auto issue_next = [&]() {  // all lanes: four a row segment, eight rows at a time; a group of cp.async, possibly empty
     if (n_tile < ntiles) {
       auto copy = [&](auto fmt_) {
         constexpr int F = decltype(fmt_)::value, BB = Fmt<F>::BB, MAXB = F == ILL_Q8_0 ? 8 : F == ILL_Q6_K ? 1 : 2;  // most blocks a piece
         const MtFmt& f = p.f[F != FMT];
-        const int row0 = (n_tile - (n_mi ? p.m[n_mi - 1].tile_end : 0)) * MT_ROWS;
-        u8* st = ring + (size_t)i_slot * p.stage_bytes;
-        const uint32_t len = (uint32_t)min(f.cb, nb - n_pc * f.cb) * BB;
-        const u8* src = p.m[n_mi].w + (long long)(row0 + g) * f.row_bytes + (long long)n_pc * f.cb * BB;
-#pragma unroll
-        for (int h = 0; h < MT_ROWS; h += 8)
-          if (row0 + h + g < p.m[n_mi].rows)
-            copy_segment<(MAXB * BB + 30) / 16>(st + (size_t)(h + g) * f.pitch, src + (long long)h * f.row_bytes, len, t);
+        const uint32_t off = (uint32_t)n_pc * f.piece_bytes, len = min(f.piece_bytes, (uint32_t)f.row_bytes - off);
+        const uint32_t dst = n_dst + g * f.pitch + 16 * t;
+        const u8* src = n_src + off;
+        if (n_rows > 0) copy_segment_at<(MAXB * BB + 30) / 16>(dst, src, len, t);
+        if (n_rows > 8) copy_segment_at<(MAXB * BB + 30) / 16>(dst + 8 * f.pitch, src + n_row8, len, t);
         n_pc += MT_SUMS;
         if (n_pc >= f.npieces) {
           n_left &= n_left - 1;
@@ -305,8 +319,9 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
           else { n_tile += tile_step; at_tile(); }
         }
       };
-      if (TWO && p.m[n_mi].alt) copy(IntC<FMT2>()); else copy(IntC<FMT>());
-      i_slot = i_slot + 1 == stages ? 0 : i_slot + 1;
+      if (TWO && n_alt) copy(IntC<FMT2>()); else copy(IntC<FMT>());
+      n_dst += p.stage_bytes;
+      if (n_dst == n_end) n_dst = ring;
     }
     cp_async_commit();
   };
@@ -358,12 +373,14 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
   MtLane xl;  // (the 2-bit formats')
   xl.set<FMT>(smem_u32(smem), p.x_stride, smem_u32(smem) + p.xs_off, smem_u32(smem) + p.bs_off, nb, FMT == ILL_IQ2_XXS ? smem_u32(iq_grid) : 0u, lane);
 
-  int slot = 0, it = 0;
+  uint32_t at = ring;          // the stage used next
+  int it = 0;
   for (int tile = tile0; tile < ntiles; tile += tile_step, ++it) {
     const int mi = matrix(tile), row0 = (tile - (mi ? p.m[mi - 1].tile_end : 0)) * MT_ROWS;
     float* sums = part + (size_t)(it & 1) * p.nsums * NTOK * PP;
-    const u8* w = p.m[mi].w;
     const MtFmt& f = p.f[format(mi)];
+    // where the lane's rows start, modulo 16
+    const uint32_t o0 = (uint32_t)(uintptr_t)p.m[mi].w + (uint32_t)(row0 + g) * (uint32_t)f.row_bytes, o8 = o0 + 8u * (uint32_t)f.row_bytes;
     for (unsigned left = f.sums[wg]; left; left &= left - 1) {
       const int sum = __ffs(left) - 1;
       float acc[NT8][4];
@@ -377,23 +394,20 @@ __global__ void __launch_bounds__(32 * MT_MAX_WARPS, 1) mvt_kernel(const __grid_
         else if (stages == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
         else asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncwarp();
-        const u8* piece = ring + (size_t)slot * p.stage_bytes;
-        slot = slot + 1 == stages ? 0 : slot + 1;
         auto use = [&](auto fmt_) {
           constexpr int F = decltype(fmt_)::value, BB = Fmt<F>::BB;
           // a row's segment starts where its block starts inside the 16-byte aligned span that was copied
-          const long long o0 = (long long)(row0 + g) * f.row_bytes + (long long)pc * f.cb * BB;
-          const long long o8 = o0 + 8ll * f.row_bytes;
-          const u8* s0 = piece + (size_t)g * f.pitch + (((uintptr_t)w + o0) & 15);
-          const u8* s8 = piece + (size_t)(g + 8) * f.pitch + (((uintptr_t)w + o8) & 15);
-          const int nhere = min(f.cb, nb - pc * f.cb);
-          if constexpr (F == ILL_Q2_K || F == ILL_IQ2_XXS) {
-            for (int j = 0; j < nhere; ++j) MtBlock<F, NT8, AL4>::run(smem_u32(s0) + j * BB, smem_u32(s8) + j * BB, pc * f.cb + j, xl, lane, acc);
-          } else {
-            for (int j = 0; j < nhere; ++j) MtBlock<F, NT8, AL4>::run(s0 + j * BB, s8 + j * BB, pc * f.cb + j, x, lane, acc);
+          const uint32_t off = (uint32_t)pc * f.piece_bytes;
+          uint32_t s0 = at + g * f.pitch + ((o0 + off) & 15u), s8 = at + (g + 8) * f.pitch + ((o8 + off) & 15u);
+          const int b0 = pc * f.cb, nhere = min(f.cb, nb - b0);
+          for (int j = 0; j < nhere; ++j, s0 += BB, s8 += BB) {
+            if constexpr (F == ILL_Q2_K || F == ILL_IQ2_XXS) MtBlock<F, NT8, AL4>::run(s0, s8, b0 + j, xl, lane, acc);
+            else MtBlock<F, NT8, AL4>::run((const u8*)__cvta_shared_to_generic(s0), (const u8*)__cvta_shared_to_generic(s8), b0 + j, x, lane, acc);
           }
         };
         if (TWO && p.m[mi].alt) use(IntC<FMT2>()); else use(IntC<FMT>());
+        at += p.stage_bytes;
+        if (at == n_end) at = ring;
         __syncwarp();
         issue_next();
       }
@@ -529,6 +543,7 @@ static int mvt_plan(int nmat, const int* fmts, const int* rows, int cols, int n,
       if (room <= (two_bit ? 226u : 220u) * 1024u) break;
       if (!two_bit || cb == 1) return ILL_ERR_UNSUPPORTED;
     }
+    f.piece_bytes = (uint32_t)(f.cb * bb);
     if (stage > p.stage_bytes) p.stage_bytes = stage;
     const int ns = f.npieces < MT_SUMS ? f.npieces : MT_SUMS;
     if (ns > p.nsums) p.nsums = ns;

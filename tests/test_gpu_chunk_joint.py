@@ -23,7 +23,8 @@ def _p(t):
     ((B.Q4_K, B.Q4_K, B.Q6_K), (16, 256, 1), 256, 17, 2, True),
     ((B.Q6_K, B.Q6_K), (1024, 1024), 768, 65, 2, True),
     ((B.Q6_K, B.Q4_K), (1024, 1040), 512, 1024, 0, True),               # tiles of 64 tokens, two CTAs an SM
-    ((B.Q4_K, B.Q6_K), (1024, 1024), 256, 512, 0, False),               # more CTAs than run side by side
+    ((B.Q4_K, B.Q6_K), (1024, 1024), 256, 500, 0, True),                # four CTAs an SM
+    ((B.Q4_K, B.Q6_K), (1024, 1024), 256, 2048, 0, False),              # more CTAs than run side by side
     ((B.Q2_K, B.Q2_K), (64, 64), 256, 20, 0, False),
 ])
 def test_matrices_of_a_chunk_in_one_launch(cuda_lib, fmts, rows, cols, n, off, one):
