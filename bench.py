@@ -339,7 +339,7 @@ def chain_leg(D, B, torch, dev, dims, layers, fmt_main, fmt_alt, seed, peak, nam
            "per_product": {"us_per_token": us_pp, "GBps": m["bytes"] / us_pp / 1e3, "frac_of_hbm": m["bytes"] / us_pp / 1e3 / peak,
                            "launches": launches[0], "how": "one CUDA graph of the token's launches"},
            "one_launch": {"us_per_token": us_one, "GBps": m["bytes"] / us_one / 1e3, "frac_of_hbm": m["bytes"] / us_one / 1e3 / peak,
-                          "launches": 1, "products": plan.n, "how": "ill_decode_run: one cooperative launch, a barrier between dependent products"},
+                          "launches": 1, "products": plan.n, "how": "ill_chain_run: the token's launches recorded once as a CUDA graph, one host call"},
            "parity": {"one_launch_equals_per_product_bits": same}}
     del m, plan, g
     torch.cuda.empty_cache()

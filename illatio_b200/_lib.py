@@ -29,6 +29,10 @@ SIGNATURES = {
     "ill_decode_plan_bytes": (_L, [_I]),
     "ill_decode_plan": (_I, [_c.POINTER(DecodeOp), _I, _P, _L, _c.POINTER(_c.c_int32), _S]),
     "ill_decode_run": (_I, [_P, _c.POINTER(_c.c_int32), _S]),
+    "ill_chain_scratch_bytes": (_L, [_c.POINTER(DecodeOp), _I]),
+    "ill_chain_new": (_I, [_c.POINTER(DecodeOp), _I, _P, _L, _c.POINTER(_c.c_uint64)]),
+    "ill_chain_run": (_I, [_c.c_uint64, _S]),
+    "ill_chain_free": (_I, [_c.c_uint64]),
     "ill_b200_version": (_I, []),
     "ill_error_string": (_c.c_char_p, [_I]),
     "ill_last_cuda_error": (_I, []),

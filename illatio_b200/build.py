@@ -11,7 +11,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libillatio_b200.so")
 HOSTOPS = os.path.join(HERE, "_hostops.so")
-SOURCES = ["lib.cu", "quant.cu", "mv.cu", "moe.cu", "mm_id.cu", "mvf.cu", "decode.cu", "mvt.cu", "mve.cu", "mmd.cu", "mm_q8.cu", "mm_q8_i8.cu"]
+SOURCES = ["lib.cu", "quant.cu", "mv.cu", "moe.cu", "mm_id.cu", "mvf.cu", "decode.cu", "mvt.cu", "mve.cu", "mmd.cu", "mm_q8.cu", "mm_q8_i8.cu", "chain.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC,-fvisibility=hidden", "--expt-relaxed-constexpr",

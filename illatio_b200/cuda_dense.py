@@ -323,25 +323,33 @@ def decode_op(w, x, y, w2=None, norm_w=None, eps=1e-6, bias=None, acc=False, aft
 
 
 class DecodePlan:
-    """A token's chain of products run as ONE launch (ill_decode_plan / ill_decode_run): what CUDA-FORWARD-N
-    (src/cuda-dense.lisp:380-432) issues as a launch per product and per quantization.  OPS: decode_op()s in
-    order.  The plan lives in device memory this object owns; run() enqueues one token on the current stream."""
+    """A token's chain of products enqueued with one call: what CUDA-FORWARD-N (src/cuda-dense.lisp:380-432) issues as a
+    launch per product and per quantization.  OPS: decode_op()s in order.  The plan owns its device memory and the recorded
+    launches (ill_chain_new); run() enqueues one token on the current stream."""
 
     def __init__(self, ops, device="cuda"):
         import ctypes
+        self.chain = ctypes.c_uint64(0)
         self.n = len(ops)
         arr = (_lib.DecodeOp * self.n)(*ops)
         nbytes = _lib.lib().ill_decode_plan_bytes(self.n)
         if nbytes <= 0:
             raise ValueError("a chain holds 1 to 1024 products")
-        self.plan = torch.zeros(nbytes + 128, dtype=torch.uint8, device=device)
-        self.base = (self.plan.data_ptr() + 127) // 128 * 128
-        self.launch = (ctypes.c_int32 * 16)()
-        with torch.cuda.device(self.plan.device):
-            _lib.call("ill_decode_plan", arr, self.n, self.base, nbytes, self.launch, _stream())
+        with torch.cuda.device(device):
+            # (the one-launch form's plan: what it refuses is refused)
+            plan = torch.zeros(nbytes + 128, dtype=torch.uint8, device=device)
+            _lib.call("ill_decode_plan", arr, self.n, (plan.data_ptr() + 127) // 128 * 128, nbytes, (ctypes.c_int32 * 16)(), _stream())
+            nbytes = _lib.lib().ill_chain_scratch_bytes(arr, self.n)
+            self.scratch = torch.empty(nbytes + 128, dtype=torch.uint8, device=device)
+            _lib.call("ill_chain_new", arr, self.n, (self.scratch.data_ptr() + 127) // 128 * 128, nbytes, ctypes.byref(self.chain))
 
     def run(self):
-        _lib.call("ill_decode_run", self.base, self.launch, _stream())
+        _lib.call("ill_chain_run", self.chain, _stream())
+
+    def __del__(self):
+        if getattr(self, "chain", None) and _lib is not None:
+            _lib.status("ill_chain_free", self.chain)
+            self.chain = None
 
 
 def dequant_rows(w, first_row, nrows, out=None):

@@ -2,9 +2,9 @@
 
     python -m illatio_b200.microbench_dense mv   q6_k 151936 5120 4      # ill_mv: FORMAT ROWS COLS TOKENS
     python -m illatio_b200.microbench_dense glu  q4_k 9728 2560           # ill_mv_glu
-    python -m illatio_b200.microbench_dense chain q|qb|head|glu           # ill_decode_run: a chain of products
-                                                                          #   q: 36 Q4_K 4096x2560, no barriers; qb: the same
-                                                                          #   with a barrier after each; head: two Q6_K
+    python -m illatio_b200.microbench_dense chain q|qb|head|glu           # ill_chain_run: a chain of products
+                                                                          #   q: 36 Q4_K 4096x2560 that share activations; qb: the same
+                                                                          #   each behind the one before; head: two Q6_K
                                                                           #   151936x2560; glu: twelve gated Q4_K 9728x2560
 
 Weights are synthetic blocks made on the device (blocks.synth_matrix_torch); a rotation of copies keeps every
