@@ -207,7 +207,13 @@ __device__ __forceinline__ void w_q6k(const uint32_t* ql, const uint32_t* qh, in
 // The tensor maps of X (rows of 64 halves, two K steps a load) and of its sums of 16 for loads of 32, 64, 96 and 128 rows
 struct MmMaps {
   CUtensorMap x[4], e[4];
+  CUtensorMap w[2];  // MM_TMA_W: a dense matrix, and the one beside it, as rows of bytes
 };
+// Whether the raw blocks come by TMA, 128 rows a load: a dense matrix of Q4_K, whose blocks start on 16-byte boundaries (an expert's
+// address is the device's to look up, so it has no map).  Asked for by the lanes that unpack them, the 16-byte pieces took 590 of the
+// 3300 cycles a block that bound the kernel.  us, 512 tokens, before / now: 2 x 9728 x 2560 98 / 91, 4096 x 2560 32 / 30,
+// 2560 x 4096 38.4 / 35.0; 64 tokens x 4096 x 2560 25.2 / 23.6; 2048 x 9728 x 2560 159 / 149.
+template <int FMT, bool DENSE> constexpr bool MM_TMA_W = DENSE && FMT == ILL_Q4_K;
 __device__ __forceinline__ int mm_boxes(int rows) { return max(1, (rows + MM_XBOX - 1) / MM_XBOX); }
 
 // Geometry per format and per NT, the most rows of X a tile has (64, 128 or 256).  A 256-wide block is four K steps; the
@@ -299,11 +305,12 @@ template <int FMT, int NT> struct MmBars {
   uint64_t raw_full[G::DQ_WARPS];   // both warps' copies into a raw buffer landed
   uint64_t raw_empty[G::DQ_WARPS];  // both warps have read it
   uint64_t fin;               // after a time-out: the MMAs issued so far completed
-  __device__ __forceinline__ void init() {
+  // TMA_W: a raw buffer is a block's 128 rows, at [2 set + buffer], filled by one load and read by a set's eight warps
+  __device__ __forceinline__ void init(bool tma_w) {
     for (int s = 0; s < G::NX; ++s) { mbar_init(&xfull[s], 1); mbar_init(&xempty[s], 1); }
     for (int s = 0; s < G::NSLOT; ++s) mbar_init(&afull[s], 4);
     for (int s = 0; s < 8; ++s) mbar_init(&aempty[s], 1);
-    for (int s = 0; s < G::DQ_WARPS; ++s) { mbar_init(&raw_full[s], 64); mbar_init(&raw_empty[s], 2); }
+    for (int s = 0; s < G::DQ_WARPS; ++s) { mbar_init(&raw_full[s], tma_w ? 1 : 64); mbar_init(&raw_empty[s], tma_w ? 8 : 2); }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&efull[s], 1); mbar_init(&eempty[s], 1);
       mbar_init(&mfull[s], 8); mbar_init(&mempty[s], 1);
@@ -320,7 +327,9 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
                                          const uint4* iq_grid, const uint32_t* iq_sgn, uint32_t tmem_base, int warp, int lane) {
   typedef MmGeom<FMT, NT> G;
   constexpr int BB = G::BB, NSLOT = G::NSLOT, NX = G::NX, PITCH = G::PITCH, HALVES = G::HALVES, DC = G::DC;
-  constexpr bool KM = G::KM;
+  constexpr bool KM = G::KM, TMA_W = MM_TMA_W<FMT, DENSE>;
+  constexpr uint32_t W_BYTES = 4 * G::RAW_BYTES;  // a block's 128 rows
+  static_assert(!TMA_W || (PITCH == BB && (NX * G::X_BYTES + 2 * G::E_BYTES + 2 * G::M_BYTES) % 128 == 0 && W_BYTES % 128 == 0), "TMA writes rows of BB bytes");
   // [X ring][KM: sums of 16 x 2, mins x 2] (the X tiles 1024-byte aligned, as the 128-byte swizzle needs), the
   // dequantizing warps' raw blocks, scales
   u8* x_tiles = smem;
@@ -484,7 +493,29 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
       mbar_wait(fin, 0, nullptr, 0, 0, ILL_WAIT_NS / 20);
     }
   } else if (warp < 4) {
-    // ---- warps 2, 3 (LOADERS) bring the raw windows of every block, half of each 32 rows' requests a warp
+    // ---- warps 2, 3 (LOADERS) bring the raw windows of every block, half of each 32 rows' requests a warp; TMA_W: warp 2 its rows
+    if constexpr (TMA_W) {
+      int g_kb = 0;
+      for (int tile = warp == 2 ? (int)blockIdx.x : ntiles; tile < ntiles && ok; tile += gridDim.x) {
+        int expert, row0, nvalid, nt;
+        locate(tile, expert, row0, nvalid, nt);
+        const bool second = nt >= ntn1;
+        if (second) nt -= ntn1;
+        for (int kb = 0; kb < nkb; ++kb, ++g_kb) {
+          const int it = g_kb / G::SETS, at = 2 * (g_kb % G::SETS) + (it & 1);
+          ok = __all_sync(0xffffffffu, mbar_wait(&raw_empty[at], ((uint32_t)(it >> 1) & 1u) ^ 1u, p.status, ST_MM_WAIT_EMPTY + 2));
+          if (!ok) break;
+          if (elect_one()) {
+            mbar_expect_tx(&raw_full[at], W_BYTES);
+            tma_load_2d(raw + at * W_BYTES, &maps.w[second], kb * BB, nt * MM_BN, &raw_full[at]);
+          }
+          __syncwarp();
+        }
+      }
+      if (!ok)  // a wait ran out: the copies that are in flight land before the CTA goes
+        for (int k = max(0, g_kb - 2 * G::SETS); k < g_kb; ++k)
+          mbar_wait(&raw_full[2 * (k % G::SETS) + (k / G::SETS & 1)], (uint32_t)(k / G::SETS >> 1) & 1u, nullptr, 0, 0, ILL_WAIT_NS / 20);
+    }
     if constexpr (G::LOADERS) {
       int g_kb = 0;
       for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
@@ -669,9 +700,11 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(G::REGS_DQ));
     const int wi = warp - (4 + G::DR_WARPS), wq = wi & 3, h = (wi >> 2) & 1, set = wi >> 3, row = 32 * wq + lane;
     const uint32_t lane_base = tmem_base + ((uint32_t)(wq * 32) << 16) + G::A_COL;  // this warp's lanes
-    u8* praw = raw + (set * 4 + wq) * 2 * G::RAW_BYTES;   // the two warps' two buffers
-    uint64_t* rfull = raw_full + (set * 4 + wq) * 2;
-    uint64_t* rempty = raw_empty + (set * 4 + wq) * 2;
+    // the two warps' two buffers (TMA_W: these rows of the set's two)
+    constexpr uint32_t BUF_BYTES = TMA_W ? W_BYTES : G::RAW_BYTES;
+    u8* praw = TMA_W ? raw + set * 2 * W_BYTES + wq * G::RAW_BYTES : raw + (set * 4 + wq) * 2 * G::RAW_BYTES;
+    uint64_t* rfull = raw_full + (TMA_W ? set : set * 4 + wq) * 2;
+    uint64_t* rempty = raw_empty + (TMA_W ? set : set * 4 + wq) * 2;
     const uint4* grid = iq_grid + (lane & 7);
     const uint32_t* sgn = iq_sgn + lane;
     int tile = blockIdx.x, kb = set;               // the block that is fetched next: of the CTA's blocks, every SETS-th
@@ -691,6 +724,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
     };
     auto start = [&]() { return ((uint32_t)(uintptr_t)wrow0 + (uint32_t)lane * (uint32_t)p.row_bytes + (uint32_t)kb * BB) & 15u; };
     auto fetch = [&](int buf) -> uint32_t {        // this warp's part of block kb's windows; where the lane's row starts in its own
+      if (TMA_W) return 0;
       if (!G::LOADERS) mm_fetch<FMT, NT>(wrow0 + (long long)kb * BB, p.row_bytes, rows_here, h, lane, praw + buf * G::RAW_BYTES, &rfull[buf]);
       return start();
     };
@@ -707,12 +741,12 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
       to_block();
       more = tile < ntiles;
       if (more) {
-        if (!G::LOADERS && !__all_sync(0xffffffffu, mbar_wait(&rempty[buf ^ 1], ((uint32_t)(it + 1) >> 1 & 1u) ^ 1u, p.status, ST_MM_WAIT_EMPTY + 2))) { ok = false; break; }
+        if (!G::LOADERS && !TMA_W && !__all_sync(0xffffffffu, mbar_wait(&rempty[buf ^ 1], ((uint32_t)(it + 1) >> 1 & 1u) ^ 1u, p.status, ST_MM_WAIT_EMPTY + 2))) { ok = false; break; }
         o16n = fetch(buf ^ 1);
       }
       if (!__all_sync(0xffffffffu, mbar_wait(&rfull[buf], (uint32_t)(it >> 1) & 1u, p.status, ST_MM_WAIT_FULL + 2))) { ok = false; break; }
       const uint32_t sh = (o16 & 2u) * 8u;         // IQ2_XXS, Q6_K: the block may start in the middle of a word
-      const uint32_t* mine = (const uint32_t*)(praw + buf * G::RAW_BYTES + lane * PITCH);
+      const uint32_t* mine = (const uint32_t*)(praw + buf * BUF_BYTES + lane * PITCH);
       const uint32_t* rw = mine + (o16 >> 2);
       uint32_t dd, m4[2] = {0, 0};                 // d, dmin; Q4_K: the half's scales and mins, Q2_K: its eight scale bytes
       if constexpr (FMT == ILL_IQ2_XXS) dd = rw[0] >> sh;
@@ -865,8 +899,8 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
   // (first tile of each expert, in shared memory).
   pdl_launch_dependents();
   if (tid == 32) {
-    bars->init();
-    if constexpr (NT2 != 0) bars2->init();
+    bars->init(MM_TMA_W<FMT, DENSE>);
+    if constexpr (NT2 != 0) bars2->init(MM_TMA_W<FMT, DENSE>);
     mbar_fence_init();
   }
   if (FMT == ILL_IQ2_XXS) {
@@ -1425,6 +1459,18 @@ static int encode_map(CUtensorMap* map, ill_dptr base, int64_t cols, int64_t row
   return r == CUDA_SUCCESS ? ILL_OK : cuda_fail(cudaErrorInvalidValue);
 }
 
+// A Q4_K matrix's bytes, a block of 128 rows a load (rows past the last: zeros)
+static int encode_raw_map(CUtensorMap* map, ill_dptr base, int ncols, int rows) {
+  EncodeTiledFn enc = encode_tiled_fn();
+  if (!enc) return cuda_fail(cudaErrorNotSupported);
+  const cuuint64_t row_bytes = (cuuint64_t)ncols / 256 * 144;
+  const cuuint64_t dims[2] = {row_bytes, (cuuint64_t)rows}, strides[1] = {row_bytes};
+  const cuuint32_t box[2] = {144, MM_BN}, estr[2] = {1, 1};
+  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)(uintptr_t)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? ILL_OK : cuda_fail(cudaErrorInvalidValue);
+}
+
 static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
                         int64_t total_rows, ill_dptr xh, ill_dptr xe, ill_dptr xd, ill_dptr map, ill_dptr ymap, ill_dptr ypeers,
                         ill_dptr y, int64_t y_stride, ill_stream stream, int64_t add2 = 0, ill_dptr y2 = 0, ill_dptr one_ptr = 0,
@@ -1543,6 +1589,13 @@ static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptr
     if (rc) return rc;
   }
   if (!km) memcpy(maps.e, maps.x, sizeof maps.e);
+  for (int i = 0; i < 2; ++i) {
+    maps.w[i] = maps.x[0];  // (not read)
+    if (one_ptr && fmt == ILL_Q4_K) {
+      const int rc = encode_raw_map(&maps.w[i], one_ptr + (i && y2 ? add2 : 0), ncols, nrows);
+      if (rc) return rc;
+    }
+  }
   MmParams p;
   p.ncols = ncols;
   p.nrows = nrows;
