@@ -245,11 +245,12 @@ template <int FMT, int NT> struct MmGeom {
   static constexpr int NSLOT = (512 - A_COL) / SLOTW;       // a block or two
   static_assert(NSLOT == 4 || NSLOT == 8, "a block's slots are consecutive");
   // Raw blocks: the two warps that unpack them (a block's halves, the same 32 rows) bring their rows' windows -- or, LOADERS,
-  // in IQ2_XXS, whose unpacking bounds the kernel (gate and up of 24576 rows on 256 experts 1360 -> 1301 us; Q6_K was 7 %
-  // slower), the two warps that have no other role, for all -- the CPR 16-byte pieces from the
+  // where the unpacking bounds the kernel: IQ2_XXS (gate and up of 24576 rows on 256 experts 1360 -> 1301 us) and tiles of 128 of
+  // Q2_K (2 x 1536 x 5120 on 64 experts of 128 rows 357 -> 346; tiles of 64 were 15 % slower, Q6_K and Q4_K 7 %), the two warps that
+  // have no other role, for all -- the CPR 16-byte pieces from the
   // boundary at or before the block, PITCH bytes apart (an odd number of 16-byte pieces: 32 rows' words lie in at most four
   // lanes a bank), RPI rows a request, a block of theirs ahead
-  static constexpr bool LOADERS = FMT == ILL_IQ2_XXS;
+  static constexpr bool LOADERS = FMT == ILL_IQ2_XXS || (FMT == ILL_Q2_K && NT == 128);
   static constexpr int CPR = FMT == ILL_Q2_K ? 6 : FMT == ILL_Q4_K ? 9 : FMT == ILL_Q6_K ? 14 : 5;
   static constexpr int PITCH = FMT == ILL_Q2_K ? 112 : FMT == ILL_Q4_K ? 144 : FMT == ILL_Q6_K ? 240 : 80;
   static constexpr int RPI = 32 / CPR;
