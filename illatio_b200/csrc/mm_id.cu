@@ -73,6 +73,7 @@ struct MmParams {
   int acc;
   int bm;                      // rows of X a tile of a dense matrix, at most the kernel's NT
   int over;                    // experts of no more rows than this are left out
+  float neg_zero;              // -0, for mul2_rn
 };
 // (DENSE is a template argument of the kernel, so that the experts' launches compile to what they were without it)
 template <bool DENSE> __device__ __forceinline__ unsigned long long mm_ptr(const MmParams& p, int e) {
@@ -187,10 +188,13 @@ __device__ __forceinline__ void raw_words(const uint32_t* rw, uint32_t sh, uint3
 // integers above 2048, so the product goes to the tensor core in two exact parts: EVEN = (SC - SC % 2) * (q - 32), an
 // even integer of at most 4096, and ODD = (SC % 2) * (q - 32); both are multiplied with the same activations into
 // the same accumulator.
+// EX: of the scale's upper four bits (-8 .. 7) and lower four.
+template <bool EX>
 __device__ __forceinline__ void w_q6k(const uint32_t* ql, const uint32_t* qh, int odd, int qsh, int sc, uint32_t* even, uint32_t* oddp) {
-  const int s0 = sc & 1;
-  uint32_t s2 = small_h2((uint32_t)(sc - s0 + 128));
+  const int s0 = sc & (EX ? 15 : 1);
+  uint32_t s2 = small_h2((uint32_t)((EX ? sc >> 4 : sc - s0) + 128));
   asm("add.rn.f16x2 %0, %0, %1;" : "+r"(s2) : "r"(0xd800d800u));  // - 128
+  const uint32_t l2 = EX ? small_h2((uint32_t)s0) : 0u;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const uint32_t v = ((ql[i] >> (4 * odd)) & 0x0f0f0f0fu) | (((qh[i] >> qsh) & 0x03030303u) << 4);
@@ -199,8 +203,8 @@ __device__ __forceinline__ void w_q6k(const uint32_t* ql, const uint32_t* qh, in
     asm("add.rn.f16x2 %0, %0, %1;" : "+r"(b) : "r"(0xe420e420u));
     even[2 * i] = hmul2(a, s2);
     even[2 * i + 1] = hmul2(b, s2);
-    oddp[2 * i] = s0 ? a : 0u;
-    oddp[2 * i + 1] = s0 ? b : 0u;
+    oddp[2 * i] = EX ? hmul2(a, l2) : s0 ? a : 0u;
+    oddp[2 * i + 1] = EX ? hmul2(b, l2) : s0 ? b : 0u;
   }
 }
 
@@ -223,7 +227,11 @@ __device__ __forceinline__ int mm_boxes(int rows) { return max(1, (rows + MM_XBO
 // Tensor memory, 512 columns (an accumulator's column = a row of X):
 //   D[2] at 0, two accumulators that alternate job by job; KM: the mins' accumulator (two when NT is 64); then the ring
 //   of A slots, a K step each, to the end
-template <int FMT, int NT> struct MmGeom {
+// EX (tiles of up to 64): two accumulators a job, each an integer that fp32 holds, for sums that round once, as int32 would (mm_exact_kernel):
+// Q4_K the block's first and second half of K (at most 128 * 945 * 128 < 2^24), Q6_K the scales' upper and lower four bits (at most
+// 256 * 480 * 128; a block's whole sum reaches 2^27).
+template <int FMT, int NT, bool EX = false> struct MmGeom {
+  static_assert(!EX || (NT == 64 && (FMT == ILL_Q4_K || FMT == ILL_Q6_K)), "tensor memory");
   static constexpr bool KM = FMT == ILL_Q2_K || FMT == ILL_Q4_K;
   static constexpr int BB = FMT == ILL_Q2_K ? 84 : FMT == ILL_Q4_K ? 144 : FMT == ILL_Q6_K ? 210 : 66;
   static constexpr int HALVES = NT > 128 ? 2 : 1;
@@ -240,8 +248,9 @@ template <int FMT, int NT> struct MmGeom {
   static constexpr int REGS_SUM = 128 * REGS_AUX + 32 * (DR_WARPS * REGS_DRAIN + DQ_WARPS * REGS_DQ);
   static constexpr uint32_t SLOTW = FMT == ILL_Q6_K ? 64 : 32;  // columns of an A slot (Q6_K: the even and the odd part)
   static constexpr int NDM = !KM ? 0 : NT < 128 ? 2 : 1;
-  static constexpr uint32_t DM_COL = 2 * DC, A_COL = NT < 128 ? 256 : KM ? 384 : 256;
-  static_assert(DM_COL + NDM * DC <= A_COL, "accumulators and the A ring overlap");
+  static constexpr uint32_t DB = EX ? 2 * DC : DC;          // columns of a job's accumulators
+  static constexpr uint32_t DM_COL = 2 * DB, A_COL = KM && (EX || NT == 128) ? 384 : 256;
+  static_assert(!(NT > 128 && KM) && DM_COL + NDM * DC <= A_COL, "accumulators and the A ring overlap");
   static constexpr int NSLOT = (512 - A_COL) / SLOTW;       // a block or two
   static_assert(NSLOT == 4 || NSLOT == 8, "a block's slots are consecutive");
   // Raw blocks: the two warps that unpack them (a block's halves, the same 32 rows) bring their rows' windows -- or, LOADERS,
@@ -271,6 +280,12 @@ template <int FMT, int NT, int NT2> struct MmSmem {
   static_assert(SMEM <= 227 * 1024, "shared memory of a CTA");
 };
 
+template <int FMT, int FMT2> struct MmExactSmem {
+  static constexpr uint32_t BODY2 = MmGeom<FMT2, 64, true>::BODY, BODY = MmGeom<FMT, 64, true>::BODY > BODY2 ? MmGeom<FMT, 64, true>::BODY : BODY2;
+  static constexpr size_t SMEM = BODY + MM_BARS + 16 + 1024 /* alignment */;
+  static_assert(SMEM <= 227 * 1024, "shared memory of a CTA");
+};
+
 // One of two warps' (H) requests for the windows of a block of ROWS <= 32 rows (the first row's block at SRC) into the buffer DST;
 // FULL gets this warp's 32 arrivals once they have landed.
 template <int FMT, int NT>
@@ -289,8 +304,8 @@ __device__ __forceinline__ void mm_fetch(const u8* src, int row_bytes, int rows,
 }
 
 // The mbarriers of a kernel for tiles of up to NT rows of X
-template <int FMT, int NT> struct MmBars {
-  typedef MmGeom<FMT, NT> G;
+template <int FMT, int NT, bool EX = false> struct MmBars {
+  typedef MmGeom<FMT, NT, EX> G;
   uint64_t xfull[G::NX];      // the X tile landed (TMA)
   uint64_t xempty[G::NX];     // the MMAs that read it completed
   uint64_t afull[G::NSLOT];   // the K step of A is in tensor memory (4 warps)
@@ -322,11 +337,11 @@ template <int FMT, int NT> struct MmBars {
 };
 
 // What a CTA does once its barriers, tables and tensor memory are there and the experts' tiles of up to BM rows of X are counted
-// (TILE_FIRST): tiles blockIdx.x, + gridDim.x, ...
-template <int FMT, bool DENSE, int NT>
-__device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, int bm, u8* smem, MmBars<FMT, NT>* bars, const int* tile_first,
-                                         const uint4* iq_grid, const uint32_t* iq_sgn, uint32_t tmem_base, int warp, int lane) {
-  typedef MmGeom<FMT, NT> G;
+// (TILE_FIRST): tiles CTA, + CTAS, ...
+template <int FMT, bool DENSE, int NT, bool EX = false>
+__device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, int bm, u8* smem, MmBars<FMT, NT, EX>* bars, const int* tile_first,
+                                         const uint4* iq_grid, const uint32_t* iq_sgn, uint32_t tmem_base, int warp, int lane, int cta, int ctas) {
+  typedef MmGeom<FMT, NT, EX> G;
   constexpr int BB = G::BB, NSLOT = G::NSLOT, NX = G::NX, PITCH = G::PITCH, HALVES = G::HALVES, DC = G::DC;
   constexpr bool KM = G::KM, TMA_W = MM_TMA_W<FMT, DENSE>;
   constexpr uint32_t W_BYTES = 4 * G::RAW_BYTES;  // a block's 128 rows
@@ -374,7 +389,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
     // and 1 watch a job's two stages, lane 2 (KM) the tile for its sums of 16: one poll looks at all of them.
     int s = 0, g = 0;                              // stage of the ring; jobs so far
     uint32_t ph = 1;                               // parity that a free stage's barrier has completed (a fresh barrier: 1)
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    for (int tile = cta; tile < ntiles && ok; tile += ctas) {
       int expert, row0, nvalid, nt;
       locate(tile, expert, row0, nvalid, nt);
       for (int kb = 0; kb < nkb && ok; ++kb) {
@@ -426,7 +441,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
                           : lane == 9 ? ST_MM_WAIT_FULL + 4 : lane == 10 ? ST_MM_WAIT_FULL + 3 : ST_MM_WAIT_EPI + 2;
     const uint64_t xdesc0 = umma_desc(x_tiles);
     int s = 0, slot = 0, g = 0, g_kb = 0;          // X stage; first A slot of the block; jobs and blocks so far
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    for (int tile = cta; tile < ntiles && ok; tile += ctas) {
       int expert, row0, nvalid, nt;
       locate(tile, expert, row0, nvalid, nt);
       nvalid = __shfl_sync(0xffffffffu, nvalid, 0);
@@ -438,7 +453,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
           // fp32 accumulate, fp16 A and B, both K-major, M = 128 weight rows, N = the job's rows of X up to 16
           const int nmma = max(16, (rows + 15) & ~15);
           const uint32_t idesc = (1u << 4) | ((uint32_t)(nmma >> 3) << 17) | ((uint32_t)(MM_BN >> 4) << 24);
-          const uint32_t d1 = tmem_base + (uint32_t)(b * DC);
+          const uint32_t d1 = tmem_base + (uint32_t)b * G::DB;
           const uint32_t xstep = mm_boxes(rows) * (MM_XBOX * MM_BK * 2 / 16);  // a K step's tile in a stage
           uint64_t* aem = aempty + 4 * (g_kb & 1);
           BarPoll poll(p.status, code);
@@ -451,10 +466,12 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
             if (elect_one()) {
 #pragma unroll
               for (int k = 0; k < MM_BK / 16; ++k)  // 16 of K: 8 columns of A, 32 bytes inside X's swizzle atom
-                umma_f16_ts(d1, a0 + 8 * k, xdsc + 2 * k, idesc, (i | k) ? 1u : 0u);
-              if constexpr (FMT == ILL_Q6_K) {  // the weights' odd parts against the same activations
+                umma_f16_ts(EX && FMT == ILL_Q4_K ? d1 + (i >> 1) * DC : d1, a0 + 8 * k, xdsc + 2 * k, idesc,
+                            ((EX && FMT == ILL_Q4_K ? i & 1 : i) | k) ? 1u : 0u);
+              if constexpr (FMT == ILL_Q6_K) {  // the weights' odd parts (EX: their other parts) against the same activations
 #pragma unroll
-                for (int k = 0; k < MM_BK / 16; ++k) umma_f16_ts(d1, a0 + 32 + 8 * k, xdsc + 2 * k, idesc, 1u);
+                for (int k = 0; k < MM_BK / 16; ++k)
+                  umma_f16_ts(EX ? d1 + DC : d1, a0 + 32 + 8 * k, xdsc + 2 * k, idesc, EX && !(i | k) ? 0u : 1u);
               }
               if (i & 1) umma_commit(&xempty[s]);
               if (last) umma_commit(&aem[i]);
@@ -497,7 +514,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
     // ---- warps 2, 3 (LOADERS) bring the raw windows of every block, half of each 32 rows' requests a warp; TMA_W: warp 2 its rows
     if constexpr (TMA_W) {
       int g_kb = 0;
-      for (int tile = warp == 2 ? (int)blockIdx.x : ntiles; tile < ntiles && ok; tile += gridDim.x) {
+      for (int tile = warp == 2 ? cta : ntiles; tile < ntiles && ok; tile += ctas) {
         int expert, row0, nvalid, nt;
         locate(tile, expert, row0, nvalid, nt);
         const bool second = nt >= ntn1;
@@ -519,7 +536,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
     }
     if constexpr (G::LOADERS) {
       int g_kb = 0;
-      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+      for (int tile = cta; tile < ntiles && ok; tile += ctas) {
         int expert, row0, nvalid, nt;
         locate(tile, expert, row0, nvalid, nt);
         const bool second = nt >= ntn1;
@@ -554,7 +571,8 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
     const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + 8 * hh;
     int g = 0, d_kb = 0;                           // jobs and blocks drained so far by this CTA
     float* xsw = xsc + (warp - 4) * (HALVES * NP * 32);
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    const uint64_t nz2 = EX ? pack2(p.neg_zero, p.neg_zero) : 0ull;
+    for (int tile = cta; tile < ntiles && ok; tile += ctas) {
       int expert, row0, nvalid, nt;
       locate(tile, expert, row0, nvalid, nt);
       // pairs of fp32: this weight row against the tile's rows of X 128 half + column(0 .. 32 NP - 1)
@@ -598,11 +616,12 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
           }
           const float* xp = xsw + half * NP * 32;
           const int nv = nvalid - 128 * half - 8 * hh;  // columns past the tile's last row of X were not computed
-          const uint32_t td = t0 + b * DC, tm = t0 + G::DM_COL + (G::NDM == 2 ? b * DC : 0);
+          const uint32_t td = t0 + b * G::DB, tm = t0 + G::DM_COL + (G::NDM == 2 ? b * DC : 0);
           // eight columns at a time; in narrow tiles, where the registers allow it, the next eight are on their way meanwhile
-          uint32_t v[PIPE ? 2 : 1][8], w[PIPE ? 2 : 1][8];
+          uint32_t v[PIPE ? 2 : 1][8], w[PIPE ? 2 : 1][8], u[PIPE ? 2 : 1][8];
           if (PIPE && nv > 0) {
             tmem_ld(td, v[0]);
+            if constexpr (EX) tmem_ld(td + DC, u[0]);
             if constexpr (KM) tmem_ld(tm, w[0]);
           }
 #pragma unroll
@@ -614,15 +633,26 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
                 if constexpr (KM) tmem_ld(tm + col, w[0]);
               }
               tmem_ld_wait(v[cur]);
+              if constexpr (EX) tmem_ld_done(u[cur]);
               if constexpr (KM) tmem_ld_done(w[cur]);
               if (PIPE && c + 8 < NP * 32 && nxt < nv) {
                 tmem_ld(td + nxt, v[PIPE ? cur ^ 1 : 0]);
+                if constexpr (EX) tmem_ld(td + DC + nxt, u[PIPE ? cur ^ 1 : 0]);
                 if constexpr (KM) tmem_ld(tm + nxt, w[PIPE ? cur ^ 1 : 0]);
               }
 #pragma unroll
               for (int i = 0; i < 8; i += 4) {
                 const ulonglong2 dx = *(const ulonglong2*)(xp + c + i);
                 uint64_t* o = out + half * NP * 16 + (c + i) / 2;
+                if constexpr (EX) {                // the steps of the int8 kernels, each rounded
+#pragma unroll
+                  for (int k = 0; k < 2; ++k) {
+                    const uint64_t d = k ? dx.y : dx.x, v2 = pack2u(v[cur][i + 2 * k], v[cur][i + 2 * k + 1]), u2 = pack2u(u[cur][i + 2 * k], u[cur][i + 2 * k + 1]);
+                    if constexpr (KM) o[k] = add2(o[k], mul2_rn(mul2(d, dm2), pack2u(w[cur][i + 2 * k], w[cur][i + 2 * k + 1]), nz2));
+                    o[k] = add2(o[k], mul2_rn(mul2(dw2, d), KM ? add2(v2, u2) : fma2(v2, pack2(16.0f, 16.0f), u2), nz2));
+                  }
+                  continue;
+                }
                 if constexpr (KM) {
                   o[0] = fma2(mul2(dx.x, dm2), pack2u(w[cur][i], w[cur][i + 1]), o[0]);
                   o[1] = fma2(mul2(dx.y, dm2), pack2u(w[cur][i + 2], w[cur][i + 3]), o[1]);
@@ -708,7 +738,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
     uint64_t* rempty = raw_empty + (TMA_W ? set : set * 4 + wq) * 2;
     const uint4* grid = iq_grid + (lane & 7);
     const uint32_t* sgn = iq_sgn + lane;
-    int tile = blockIdx.x, kb = set;               // the block that is fetched next: of the CTA's blocks, every SETS-th
+    int tile = cta, kb = set;               // the block that is fetched next: of the CTA's blocks, every SETS-th
     const u8* wrow0 = nullptr;                     // the warp's first row of the tile's matrix
     int rows_here = 0;
     auto at_tile = [&]() {
@@ -721,7 +751,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
       rows_here = min(32, p.nrows - nt * MM_BN - 32 * wq);
     };
     auto to_block = [&]() {                        // on to the tile that block kb falls in
-      while (kb >= nkb && tile < ntiles) { kb -= nkb; tile += gridDim.x; if (kb < nkb) at_tile(); }
+      while (kb >= nkb && tile < ntiles) { kb -= nkb; tile += ctas; if (kb < nkb) at_tile(); }
     };
     auto start = [&]() { return ((uint32_t)(uintptr_t)wrow0 + (uint32_t)lane * (uint32_t)p.row_bytes + (uint32_t)kb * BB) & 15u; };
     auto fetch = [&](int buf) -> uint32_t {        // this warp's part of block kb's windows; where the lane's row starts in its own
@@ -792,7 +822,7 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
 #pragma unroll
             for (int jj = 0; jj < 2; ++jj) {
               uint32_t ev[8], od[8];
-              w_q6k(ql, qh, jj, 2 * (2 * jj + sb), (int)(signed char)((sc[jj] >> (16 * sb + 8 * hf)) & 0xffu), ev, od);
+              w_q6k<EX>(ql, qh, jj, 2 * (2 * jj + sb), (int)(signed char)((sc[jj] >> (16 * sb + 8 * hf)) & 0xffu), ev, od);
               tmem_st8(a0 + G::SLOTW * jj + 16 * sb + 8 * hf, ev);
               tmem_st8(a0 + G::SLOTW * jj + 32 + 16 * sb + 8 * hf, od);
             }
@@ -964,10 +994,56 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   if constexpr (NT2 != 0) {
-    if (__shfl_sync(0xffffffffu, *narrow, 0)) mm_tiles<FMT, DENSE, NT2>(maps, p, NT2, smem, bars2, tile_first, iq_grid, iq_sgn, tmem_base, warp, lane);
-    else mm_tiles<FMT, DENSE, NT>(maps, p, NT, smem, bars, tile_first, iq_grid, iq_sgn, tmem_base, warp, lane);
+    if (__shfl_sync(0xffffffffu, *narrow, 0)) mm_tiles<FMT, DENSE, NT2>(maps, p, NT2, smem, bars2, tile_first, iq_grid, iq_sgn, tmem_base, warp, lane, blockIdx.x, gridDim.x);
+    else mm_tiles<FMT, DENSE, NT>(maps, p, NT, smem, bars, tile_first, iq_grid, iq_sgn, tmem_base, warp, lane, blockIdx.x, gridDim.x);
   } else {
-    mm_tiles<FMT, DENSE, NT>(maps, p, DENSE ? p.bm : NT, smem, bars, tile_first, iq_grid, iq_sgn, tmem_base, warp, lane);
+    mm_tiles<FMT, DENSE, NT>(maps, p, DENSE ? p.bm : NT, smem, bars, tile_first, iq_grid, iq_sgn, tmem_base, warp, lane, blockIdx.x, gridDim.x);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+}
+
+// Two dense matrices of few rows (K and V) against a chunk, with the bits of the int8 kernel of mma.sync: EX's accumulators hold a
+// block's sum exactly, and the drain takes that kernel's float steps.  FMT2 other than FMT: the second matrix (P2) is of another format,
+// and CTAs SPLIT and up take its tiles.  Bound by the unpacking of one block after the other in a CTA (0.75 us a block of Q4_K, 1.57
+// of Q6_K, and 0.0044 a row of X).  us, the int8 kernel's joint launch / this: K and V of 1024 x 2560, 512 tokens, both Q4_K 44 / 19.4, one of
+// Q6_K 48 / 29.5; of 1024 x 5120, both Q6_K 86 / 48.
+template <int FMT, int FMT2>
+__global__ void __launch_bounds__(MmGeom<FMT, 64, true>::THREADS, 1)
+    mm_exact_kernel(const __grid_constant__ MmMaps maps, const MmParams p, const MmParams p2, int split) {
+  typedef MmGeom<FMT, 64, true> G;
+  typedef MmExactSmem<FMT, FMT2> S;
+  constexpr uint32_t TMEM_COLS = 512;
+  static_assert(MmGeom<FMT2, 64, true>::THREADS == G::THREADS, "one launch for both");
+  static_assert(sizeof(MmBars<FMT, 64, true>) <= MM_BARS && sizeof(MmBars<FMT2, 64, true>) <= MM_BARS, "barriers");
+  extern __shared__ __align__(1024) u8 smem_raw[];
+  u8* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  MmBars<FMT, 64, true>* bars = (MmBars<FMT, 64, true>*)(smem + S::BODY);
+  MmBars<FMT2, 64, true>* bars2 = (MmBars<FMT2, 64, true>*)(smem + S::BODY);
+  int* tile_first = (int*)(smem + S::BODY + MM_BARS);
+  uint32_t* tmem_slot = (uint32_t*)(tile_first + 2);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const bool second = FMT2 != FMT && (int)blockIdx.x >= split;
+  pdl_launch_dependents();
+  if (tid == 32) {
+    if (second) bars2->init(MM_TMA_W<FMT2, true>);
+    else bars->init(MM_TMA_W<FMT, true>);
+    mbar_fence_init();
+    tile_first[0] = 0;
+    tile_first[1] = (int)((p.one_count + p.bm - 1) / p.bm);
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
+  pdl_wait();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  if constexpr (FMT2 != FMT) {
+    if (second) mm_tiles<FMT2, true, 64, true>(maps, p2, p2.bm, smem, bars2, tile_first, nullptr, nullptr, tmem_base, warp, lane, blockIdx.x - split, gridDim.x - split);
+    else mm_tiles<FMT, true, 64, true>(maps, p, p.bm, smem, bars, tile_first, nullptr, nullptr, tmem_base, warp, lane, blockIdx.x, split);
+  } else {
+    mm_tiles<FMT, true, 64, true>(maps, p, p.bm, smem, bars, tile_first, nullptr, nullptr, tmem_base, warp, lane, blockIdx.x, gridDim.x);
   }
   tc_fence_before();
   __syncthreads();
@@ -1551,6 +1627,18 @@ static MmVariant mm_variant(int nt) {
   else return mm_one<FMT, false, 128>();
 }
 
+static int mm_ready(const MmVariant& v) {
+  cudaError_t e = cudaFuncSetAttribute(v.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem);
+  if (e != cudaSuccess) return cuda_fail(e);
+  // The warp groups trade registers after launch; what they ask for together must fit in what the
+  // CTA was given, or the drain warps would wait for registers for ever.
+  cudaFuncAttributes fa;
+  e = cudaFuncGetAttributes(&fa, v.k);
+  if (e != cudaSuccess) return cuda_fail(e);
+  if (fa.numRegs / 8 * 8 * v.threads < v.regs_sum) return ILL_ERR_UNSUPPORTED;
+  return ILL_OK;
+}
+
 // Rows of X a tile of a dense matrix: the rounds of tiles on the SMs times a tile's measured time a block of 256 columns, us; tiles
 // of up to 64, of up to 128, and (Q6_K, which has one accumulator a block: with two, draining 256 columns takes longer than it
 // saves) 256 rows.
@@ -1635,15 +1723,88 @@ static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptr
   const long long max_tiles = ((total_rows + least - 1) / least + ne) * ntn;  // an upper bound
   const MmVariant v = fmt == ILL_IQ2_XXS ? mm_variant<ILL_IQ2_XXS>(nt) : fmt == ILL_Q2_K ? mm_variant<ILL_Q2_K>(nt)
                       : fmt == ILL_Q4_K ? mm_variant<ILL_Q4_K>(nt) : mm_variant<ILL_Q6_K>(nt);
-  cudaError_t e = cudaFuncSetAttribute(v.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem);
-  if (e != cudaSuccess) return cuda_fail(e);
-  // The warp groups trade registers after launch; what they ask for together must fit in what the
-  // CTA was given, or the drain warps would wait for registers for ever.
-  cudaFuncAttributes fa;
-  e = cudaFuncGetAttributes(&fa, v.k);
-  if (e != cudaSuccess) return cuda_fail(e);
-  if (fa.numRegs / 8 * 8 * v.threads < v.regs_sum) return ILL_ERR_UNSUPPORTED;
+  const int ready = mm_ready(v);
+  if (ready) return ready;
   void* args[] = {&maps, &p};
   // persistent: a CTA an SM, each walks tiles
   return launch_kernel(v.k, dim3((unsigned)(max_tiles < sms ? max_tiles : sms)), dim3((unsigned)v.threads), v.smem, args, (cudaStream_t)stream);
+}
+
+extern "C" int ill_mm_chunk_exact(int fmt, ill_dptr w, int fmt2, ill_dptr w2, int rows, int cols, ill_dptr xh, ill_dptr xe, ill_dptr xd, int64_t n,
+                                  ill_dptr y, ill_dptr y2, ill_stream stream) {
+  if (fmt == ILL_Q6_K && fmt2 == ILL_Q4_K) {  // the other way round
+    const int f = fmt; fmt = fmt2; fmt2 = f;
+    ill_dptr t = w; w = w2; w2 = t;
+    t = y; y = y2; y2 = t;
+  }
+  if ((fmt != ILL_Q4_K && fmt != ILL_Q6_K) || (fmt2 != ILL_Q4_K && fmt2 != ILL_Q6_K)) return ILL_ERR_UNSUPPORTED;
+  if (!w || !w2 || !y || !y2 || !xh || !xd || (fmt == ILL_Q4_K && !xe) || rows <= 0 || rows % 4 || cols <= 0 || cols % 256 || n < 0 || n > 0x7fffffffll)
+    return ILL_ERR_ARG;
+  if ((xh & 15) || (xe & 15) || (xd & 3) || (y & 15) || (y2 & 15) || (w & (fmt == ILL_Q4_K ? 15 : 3)) || (w2 & (fmt2 == ILL_Q4_K ? 15 : 3)))
+    return ILL_ERR_ALIGN;
+  if (n == 0) return ILL_OK;
+  const bool mixed = fmt != fmt2;
+  MmMaps maps;
+  for (int i = 0; i < 4; ++i) {
+    int rc = encode_map(&maps.x[i], xh, cols, n, false, MM_XBOX * (i + 1));
+    if (rc == ILL_OK && fmt == ILL_Q4_K) rc = encode_map(&maps.e[i], xe, (int64_t)(cols / 256) * 64, n, true, MM_XBOX * (i + 1));
+    if (rc) return rc;
+  }
+  if (fmt != ILL_Q4_K) memcpy(maps.e, maps.x, sizeof maps.e);
+  for (int i = 0; i < 2; ++i) {
+    maps.w[i] = maps.x[0];  // (not read)
+    const int rc = fmt == ILL_Q4_K && !(i && mixed) ? encode_raw_map(&maps.w[i], i ? w2 : w, cols, rows) : ILL_OK;
+    if (rc) return rc;
+  }
+  MmParams p = {}, p2;
+  p.ncols = cols;
+  p.nrows = rows;
+  p.row_bytes = cols / 256 * fmt_block_bytes(fmt);
+  p.xd = (const float*)(uintptr_t)xd;
+  p.total_rows = n;
+  p.y = (float*)(uintptr_t)y;
+  p.y_stride = rows;
+  p.ne = 1;
+  p.one_ptr = w;
+  p.one_count = (unsigned)n;
+  p.neg_zero = -0.0f;
+  p.status = device_status_word();
+  p2 = p;
+  if (mixed) {
+    p2.row_bytes = cols / 256 * fmt_block_bytes(fmt2);
+    p2.y = (float*)(uintptr_t)y2;
+    p2.one_ptr = w2;
+  } else {
+    p.y2 = (float*)(uintptr_t)y2;
+    p.add2 = (long long)(w2 - w);
+  }
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 1) sms = 148;
+  const long long ntn = (rows + MM_BN - 1) / MM_BN;
+  // Rows of X a tile, and the SMs that Q4_K's tiles get beside Q6_K's: the rounds of tiles times a tile's measured time a block, us
+  double best = 1e30;
+  long long grid = 1;
+  int split = 0;
+  for (int b = 16; b <= 64; b += 16) {
+    const long long tiles = (n + b - 1) / b * ntn, all = 2 * tiles, g = all < sms ? all : sms, rounds = (all + g - 1) / g;
+    const double t4 = 0.75 + 0.0044 * b, t6 = 1.57 + 0.0044 * b;
+    // (mixed: Q6_K, the slower, in at least its share of the rounds; a round more of its own leaves Q4_K more SMs)
+    for (long long r = mixed ? 1 : rounds; r <= rounds; ++r) {
+      const long long sp = mixed ? g - (tiles + r - 1) / r : 0;
+      if (mixed && sp < 1) continue;
+      const double a = mixed ? (double)((tiles + sp - 1) / sp) * t4 : 0.0, c = (double)r * (mixed || fmt == ILL_Q6_K ? t6 : t4), us = a > c ? a : c;
+      if (us < best) { best = us; p.bm = p2.bm = b; grid = g; split = (int)sp; }
+    }
+  }
+  typedef MmGeom<ILL_Q4_K, 64, true> G4;
+  typedef MmGeom<ILL_Q6_K, 64, true> G6;
+  const MmVariant v = mixed ? MmVariant{(const void*)mm_exact_kernel<ILL_Q4_K, ILL_Q6_K>, MmExactSmem<ILL_Q4_K, ILL_Q6_K>::SMEM, G4::THREADS,
+                                        G4::REGS_SUM > G6::REGS_SUM ? G4::REGS_SUM : G6::REGS_SUM}
+                      : fmt == ILL_Q4_K ? MmVariant{(const void*)mm_exact_kernel<ILL_Q4_K, ILL_Q4_K>, MmExactSmem<ILL_Q4_K, ILL_Q4_K>::SMEM, G4::THREADS, G4::REGS_SUM}
+                                        : MmVariant{(const void*)mm_exact_kernel<ILL_Q6_K, ILL_Q6_K>, MmExactSmem<ILL_Q6_K, ILL_Q6_K>::SMEM, G6::THREADS, G6::REGS_SUM};
+  const int ready = mm_ready(v);
+  if (ready) return ready;
+  void* args[] = {&maps, &p, &p2, &split};
+  return launch_kernel(v.k, dim3((unsigned)grid), dim3((unsigned)v.threads), v.smem, args, (cudaStream_t)stream);
 }

@@ -171,10 +171,30 @@ def _side_stream(device):
     return s
 
 
+# Two matrices of few rows beside one of the tcgen05 kernel (which wants the activations' fp16 form in this stream in any case) go to the
+# exact form of that kernel: its tiles are 64 rows of X at most, which a chunk's K and V make one round of, and it adds the same integers
+# in the same steps as the int8 kernel.  us, int8 / exact, both of Q4_K | one of Q6_K: 1024 x 2560 of 64 tokens 23.5 / 17.3 | 23.5 / 25.6, of
+# 256 30 / 17 | 33 / 27, of 512 44 / 19 | 48 / 29, of 2048 135 / 54 | 133 / 68; 512 x 2048 of 256 20.5 / 15.3 | 20.5 / 23.5, of 512 25.5 / 15.4 |
+# 27.6 / 23.4; 256 x 2048 of 512 19.4 / 15.4 | 20.5 / 23.6, of 1024 25.5 / 15.4 | 27.6 / 23.6; 128 x 4096 of 2048 41 / 24 | 46 / 38.  A tile of Q6_K
+# takes twice one of Q4_K (two products and two accumulators of every K step), so few of them wait for it.
+EXACT_MIN_Q6K = 1 << 18  # rows times tokens
+
+
+def _exact_takes(w, y, bias, like, act, n):
+    """Whether a matrix beside one of _by_tc's, and in one launch with LIKE, goes to ill_mm_chunk_exact."""
+    return ((w.type == 1 or (w.type == 2 and w.rows * n >= EXACT_MIN_Q6K)) and 0 < w.rows == like.rows and w.rows % 4 == 0 and w.cols == like.cols and bias is None and w.qs.data_ptr() % 16 == 0
+            and y.data_ptr() % 16 == 0 and act.xq.numel() == n * w.cols)
+
+
 def chunk_mul_3(mats, act, n):
     """The products of a chunk of N tokens that share the activations ACT, MATS a list of (matrix, output, bias): two or three in one
-    launch where that is to be had (ill_mv_3n), else one by one; those of the tcgen05 kernel of the K formats by themselves."""
+    launch where that is to be had (ill_mm_chunk_exact, ill_mv_3n), else one by one; those of the tcgen05 kernel of the K formats by themselves."""
     joint = [m for m in mats if not _by_tc(m[0], act, n, m[2])]
+    if len(joint) == 2 < len(mats) and all(_exact_takes(w, y, b, joint[0][0], act, n) for w, y, b in joint):
+        cf, (w, y, _), (w2, y2, _) = _chunk_f16_of(act, n, joint[0][0].cols), *joint
+        _lib.call("ill_mm_chunk_exact", w.type, _ptr(w.qs), w2.type, _ptr(w2.qs), w.rows, w.cols, _ptr(cf.xh), _ptr(cf.xe), _ptr(cf.xd), n, _ptr(y), _ptr(y2),
+                  _stream())
+        mats, joint = [m for m in mats if all(m is not j for j in joint)], []
     a = joint[0][0] if joint else None
     if 2 <= len(joint) <= 3 and n > 16 and all(w.cols == a.cols and (w.type == 0) == (a.type == 0) and w.rows > 0 for w, _, _ in joint) and (a.type == 0) == (act.kind == "q8"):
         w, y, b = ([m[i] for m in joint] + [None] * (3 - len(joint)) for i in range(3))
