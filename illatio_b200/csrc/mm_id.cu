@@ -183,29 +183,31 @@ __device__ __forceinline__ void raw_words(const uint32_t* rw, uint32_t sh, uint3
     prev = next;
   }
 }
-// Q6_K: 16 weights of a K step -- the nibbles at shift 4 ODD of the four words QL, the 2-bit fields at shift QSH of the
-// four words QH -- times their group's signed scale SC.  |SC * (q - 32)| reaches 4064 and fp16 holds only even
-// integers above 2048, so the product goes to the tensor core in two exact parts: EVEN = (SC - SC % 2) * (q - 32), an
-// even integer of at most 4096, and ODD = (SC % 2) * (q - 32); both are multiplied with the same activations into
-// the same accumulator.
-// EX: of the scale's upper four bits (-8 .. 7) and lower four.
-template <bool EX>
-__device__ __forceinline__ void w_q6k(const uint32_t* ql, const uint32_t* qh, int odd, int qsh, int sc, uint32_t* even, uint32_t* oddp) {
-  const int s0 = sc & (EX ? 15 : 1);
-  uint32_t s2 = small_h2((uint32_t)((EX ? sc >> 4 : sc - s0) + 128));
-  asm("add.rn.f16x2 %0, %0, %1;" : "+r"(s2) : "r"(0xd800d800u));  // - 128
-  const uint32_t l2 = EX ? small_h2((uint32_t)s0) : 0u;
+// Q6_K: 16 weights of a K step -- the low (ODD 0) or high nibbles of the four words QL, the 2-bit fields at shift QSH of the
+// four words QH -- times their group's signed scale.  |scale * (q - 32)| reaches 4064 and fp16 holds only even
+// integers above 2048, so the product goes to the tensor core in two exact parts: EVEN = (scale - scale % 2) * (q - 32), an
+// even integer of at most 4096, and ODD = (scale % 2) * (q - 32); both are multiplied with the same activations into
+// the same accumulator.  EX: of the scale's upper four bits (-8 .. 7) and lower four.
+// A nibble in the upper half of its byte, and its 2-bit field in the lower bits of 0x64, are the bits of 1024 + 16 q; times part / 16, less
+// 96 parts, is part * (q - 32) exactly (one rounding).  SE and SO: part / 16, twice (q6k_parts).  (Put together at bit 0,
+// less 1056 and then multiplied, and the half's two K steps stored together: 2560 x 9728, 512 tokens 83 us, now 75; 5120 x 17408 220, now 185.)
+__device__ __forceinline__ void w_q6k(const uint32_t* ql, const uint32_t* qh, int odd, int qsh, uint32_t se, uint32_t so, uint32_t* even, uint32_t* oddp) {
+  const uint32_t be = hmul2(se, 0xe600e600u /* -1536 */), bo = hmul2(so, 0xe600e600u);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const uint32_t v = ((ql[i] >> (4 * odd)) & 0x0f0f0f0fu) | (((qh[i] >> qsh) & 0x03030303u) << 4);
-    uint32_t a = bytes_to_h2_1024(v, 0x4140), b = bytes_to_h2_1024(v, 0x4342);
-    asm("add.rn.f16x2 %0, %0, %1;" : "+r"(a) : "r"(0xe420e420u));  // - 1056: q - 32
-    asm("add.rn.f16x2 %0, %0, %1;" : "+r"(b) : "r"(0xe420e420u));
-    even[2 * i] = hmul2(a, s2);
-    even[2 * i + 1] = hmul2(b, s2);
-    oddp[2 * i] = EX ? hmul2(a, l2) : s0 ? a : 0u;
-    oddp[2 * i + 1] = EX ? hmul2(b, l2) : s0 ? b : 0u;
+    const uint32_t lo = (odd ? ql[i] : ql[i] << 4) & 0xf0f0f0f0u, hi = ((qh[i] >> qsh) & 0x03030303u) | 0x64646464u;
+    const uint32_t a = __byte_perm(lo, hi, 0x5140), b = __byte_perm(lo, hi, 0x7362);
+    even[2 * i] = hfma2(a, se, be);
+    even[2 * i + 1] = hfma2(b, se, be);
+    oddp[2 * i] = hfma2(a, so, bo);
+    oddp[2 * i + 1] = hfma2(b, so, bo);
   }
+}
+// The two parts of four scales, a byte each, the even or upper ones plus 128 or 8
+template <bool EX> __device__ __forceinline__ void q6k_parts(uint32_t sc, uint32_t& e, uint32_t& o) {
+  const uint32_t t = sc ^ 0x80808080u;
+  e = EX ? (t >> 4) & 0x0f0f0f0fu : t & 0xfefefefeu;
+  o = sc & (EX ? 0x0f0f0f0fu : 0x01010101u);
 }
 
 // The tensor maps of X (rows of 64 halves, two K steps a load) and of its sums of 16 for loads of 32, 64, 96 and 128 rows
@@ -244,7 +246,8 @@ template <int FMT, int NT, bool EX = false> struct MmGeom {
   static constexpr int DR_GROUPS = NT == 128 && KM ? 4 : 2, DR_WARPS = 4 * DR_GROUPS;
   static constexpr int THREADS = 32 * (4 + DR_WARPS + DQ_WARPS);
   // registers a thread after the roles part (the sum must fit in what the CTA was launched with: checked by the host)
-  static constexpr int REGS_AUX = 40, REGS_DRAIN = NT > 128 ? 160 : DR_GROUPS == 4 ? 88 : 120, REGS_DQ = 56;
+  static constexpr int REGS_AUX = 40, REGS_DRAIN = FMT == ILL_Q6_K ? (NT > 128 ? 152 : 104) : DR_GROUPS == 4 ? 88 : 120,
+                       REGS_DQ = FMT == ILL_Q6_K ? 64 : 56;
   static constexpr int REGS_SUM = 128 * REGS_AUX + 32 * (DR_WARPS * REGS_DRAIN + DQ_WARPS * REGS_DQ);
   static constexpr uint32_t SLOTW = FMT == ILL_Q6_K ? 64 : 32;  // columns of an A slot (Q6_K: the even and the odd part)
   static constexpr int NDM = !KM ? 0 : NT < 128 ? 2 : 1;
@@ -806,32 +809,37 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
       };
       const uint32_t a0 = lane_base + G::SLOTW * (slot + 2 * h);
       if constexpr (FMT == ILL_Q6_K) {
-        // The half's two K steps together: step jj has the nibbles at shift 4 jj of ql[0 .. 63]; columns 32 sb .. of it go with
-        // the 2-bit fields at shift 2 (2 jj + sb) of qh.  Sixteen weights (a group) at a time.
-        uint32_t sc[2];
+        // Left out for timing, 2560 x 9728 x 64 tokens of 62 us: what follows 19, its second stores 4, the raw copies 6 (one after the
+        // other in a warp; five or six slots in place of four gave nothing, reading the words in pairs neither).
+        // Step jj of the half has the nibbles at shift 4 jj of ql[0 .. 63]; columns 32 sb .. of it go with the 2-bit fields at shift
+        // 2 (2 jj + sb) of qh.  Sixteen weights (a group) at a time.
+        uint32_t sc[2], se[2], so[2], ql[16], qh[8];
         raw_words<2>(rw + 48 + 2 * h, sh, sc);
-        if (!slot_free(2 * h) || !slot_free(2 * h + 1)) break;
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          uint32_t qh[4];
-          raw_words<4>(rw + 32 + 8 * h + 4 * hf, sh, qh);
-#pragma unroll
-          for (int sb = 0; sb < 2; ++sb) {
-            uint32_t ql[4];
-            raw_words<4>(rw + 16 * h + 8 * sb + 4 * hf, sh, ql);
-#pragma unroll
-            for (int jj = 0; jj < 2; ++jj) {
-              uint32_t ev[8], od[8];
-              w_q6k<EX>(ql, qh, jj, 2 * (2 * jj + sb), (int)(signed char)((sc[jj] >> (16 * sb + 8 * hf)) & 0xffu), ev, od);
-              tmem_st8(a0 + G::SLOTW * jj + 16 * sb + 8 * hf, ev);
-              tmem_st8(a0 + G::SLOTW * jj + 32 + 16 * sb + 8 * hf, od);
-            }
-          }
-        }
-        tmem_st_wait();
-        tc_fence_before();
+        raw_words<16>(rw + 16 * h, sh, ql);
+        raw_words<8>(rw + 32 + 8 * h, sh, qh);
         __syncwarp();
-        if (lane == 0) { mbar_arrive(&afull[slot + 2 * h]); mbar_arrive(&afull[slot + 2 * h + 1]); mbar_arrive(&rempty[buf]); }
+        if (lane == 0) mbar_arrive(&rempty[buf]);
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) q6k_parts<EX>(sc[jj], se[jj], so[jj]);
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+#pragma unroll
+          for (int gr = 0; gr < 4; ++gr) {         // 16 weights: columns 32 sb + 16 hf
+            const int sb = gr >> 1, hf = gr & 1;
+            uint32_t ev[8], od[8];
+            // (1024 + part, plus its offset) / 16, less the rest
+            w_q6k(ql + 8 * sb + 4 * hf, qh + 4 * hf, jj, 2 * (2 * jj + sb), hfma2(byte_h2_1024(se[jj], 2 * sb + hf), 0x2c002c00u, EX ? 0xd408d408u : 0xd480d480u),
+                  hfma2(byte_h2_1024(so[jj], 2 * sb + hf), 0x2c002c00u, 0xd400d400u), ev, od);
+            if (gr == 0 && !slot_free(2 * h + jj)) break;
+            tmem_st8(a0 + G::SLOTW * jj + 16 * sb + 8 * hf, ev);
+            tmem_st8(a0 + G::SLOTW * jj + 32 + 16 * sb + 8 * hf, od);
+          }
+          if (!ok) break;
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&afull[slot + 2 * h + jj]);
+        }
       } else {
         uint32_t w[8];
 #pragma unroll
