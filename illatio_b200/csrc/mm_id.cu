@@ -817,8 +817,6 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
         raw_words<2>(rw + 48 + 2 * h, sh, sc);
         raw_words<16>(rw + 16 * h, sh, ql);
         raw_words<8>(rw + 32 + 8 * h, sh, qh);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&rempty[buf]);
 #pragma unroll
         for (int jj = 0; jj < 2; ++jj) q6k_parts<EX>(sc[jj], se[jj], so[jj]);
 #pragma unroll
@@ -838,7 +836,10 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&afull[slot + 2 * h + jj]);
+          if (lane == 0) {
+            mbar_arrive(&afull[slot + 2 * h + jj]);
+            if (jj == 1) mbar_arrive(&rempty[buf]);  // every word has been used: a load that is only asked for may still be under way
+          }
         }
       } else {
         uint32_t w[8];

@@ -71,3 +71,21 @@ def test_qkv_chunks(cuda_lib, fmts, krows, n, off, bias):
     for w, y, bb in zip(ws, want, (None, b, None)):
         D.cmat_mul(w, act, y, n, bias=bb)
     assert all(torch.equal(a, c) for a, c in zip(got, want)) and D.device_status() == 0
+
+
+@pytest.mark.parametrize("fmts", [(Q4, Q6), (Q6, Q6)])
+def test_the_same_bits_every_time(cuda_lib, fmts):
+    """Many tiles a CTA, so that raw blocks, slots and accumulators are reused all the time: sixty launches agree."""
+    rows, cols, n = 1024, 8192, 2048
+    act = _chunk(n, cols, 0)
+    ws = [_matrix(f, rows, cols, 0, seed=i) for i, f in enumerate(fmts)]
+    cf = D.ChunkF16(n, cols).fill(act)
+    want = [_mv(w, act, n) for w in ws]
+    bad = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(60):
+        ys = [torch.full((n * rows,), 7.0, device="cuda") for _ in ws]
+        _lib.call("ill_mm_chunk_exact", fmts[0], ws[0].qs.data_ptr(), fmts[1], ws[1].qs.data_ptr(), rows, cols, cf.xh.data_ptr(), cf.xe.data_ptr(),
+                  cf.xd.data_ptr(), n, ys[0].data_ptr(), ys[1].data_ptr(), _lib.stream())
+        for y, w in zip(ys, want):
+            bad += (y != w).sum()
+    assert bad.item() == 0 and D.device_status() == 0
