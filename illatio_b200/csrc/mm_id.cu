@@ -74,8 +74,13 @@ struct MmParams {
   int bm;                      // rows of X a tile of a dense matrix, at most the kernel's NT
   int over;                    // experts of no more rows than this are left out
   float neg_zero;              // -0, for mul2_rn
+  int tma;                     // the raw blocks come by TMA (mm_tma), of MmMaps::w[WMAP], [WMAP + 1]
+  int wmap;
 };
 // (DENSE is a template argument of the kernel, so that the experts' launches compile to what they were without it)
+template <int FMT, bool DENSE> __device__ __forceinline__ bool mm_tma(const MmParams& p) {
+  if constexpr (!DENSE) return false; else return FMT == ILL_Q4_K || (FMT == ILL_Q6_K && p.tma);
+}
 template <bool DENSE> __device__ __forceinline__ unsigned long long mm_ptr(const MmParams& p, int e) {
   if constexpr (DENSE) return p.one_ptr; else return p.ptrs[e];
 }
@@ -215,11 +220,14 @@ struct MmMaps {
   CUtensorMap x[4], e[4];
   CUtensorMap w[2];  // MM_TMA_W: a dense matrix, and the one beside it, as rows of bytes
 };
-// Whether the raw blocks come by TMA, 128 rows a load: a dense matrix of Q4_K, whose blocks start on 16-byte boundaries (an expert's
-// address is the device's to look up, so it has no map).  Asked for by the lanes that unpack them, the 16-byte pieces took 590 of the
-// 3300 cycles a block that bound the kernel.  us, 512 tokens, before / now: 2 x 9728 x 2560 98 / 91, 4096 x 2560 32 / 30,
-// 2560 x 4096 38.4 / 35.0; 64 tokens x 4096 x 2560 25.2 / 23.6; 2048 x 9728 x 2560 159 / 149.
-template <int FMT, bool DENSE> constexpr bool MM_TMA_W = DENSE && FMT == ILL_Q4_K;
+// Whether the raw blocks may come by TMA, 128 rows of a block at a time: of a dense matrix (an expert's address is the device's to look
+// up, so it has no map).  Q4_K blocks start on 16-byte boundaries: one load.  Q6_K (MmParams::tma: where four rows are a whole number of
+// 16-byte pieces, an even number of blocks a row): the map's rows are four of the matrix's, so that rows 4 i + k start 16-byte aligned up
+// to what k and the block decide; four loads of 32 rows' windows.  Asked for by the lanes that unpack them, the 16-byte pieces took 590 of
+// Q4_K's 3300 cycles a block that bound the kernel.  us, 512 tokens, before / now: Q4_K 2 x 9728 x 2560 98 / 91, 4096 x 2560 32 / 30,
+// 2560 x 4096 38.4 / 35.0; 64 tokens x 4096 x 2560 25.2 / 23.6; 2048 x 9728 x 2560 159 / 149.  Q6_K 2560 x 9728 75 / 67, 5120 x 17408
+// 185 / 181, 5120 x 5120 of 1024 tokens 111 / 99 (also without bank conflicts where the four rows' windows start at four words).
+template <int FMT, bool DENSE> constexpr bool MM_TMA_W = DENSE && (FMT == ILL_Q4_K || FMT == ILL_Q6_K);
 __device__ __forceinline__ int mm_boxes(int rows) { return max(1, (rows + MM_XBOX - 1) / MM_XBOX); }
 
 // Geometry per format and per NT, the most rows of X a tile has (64, 128 or 256).  A 256-wide block is four K steps; the
@@ -324,7 +332,7 @@ template <int FMT, int NT, bool EX = false> struct MmBars {
   uint64_t raw_full[G::DQ_WARPS];   // both warps' copies into a raw buffer landed
   uint64_t raw_empty[G::DQ_WARPS];  // both warps have read it
   uint64_t fin;               // after a time-out: the MMAs issued so far completed
-  // TMA_W: a raw buffer is a block's 128 rows, at [2 set + buffer], filled by one load and read by a set's eight warps
+  // TMA: a raw buffer is a block's 128 rows, at [2 set + buffer], filled by one warp and read by a set's eight warps
   __device__ __forceinline__ void init(bool tma_w) {
     for (int s = 0; s < G::NX; ++s) { mbar_init(&xfull[s], 1); mbar_init(&xempty[s], 1); }
     for (int s = 0; s < G::NSLOT; ++s) mbar_init(&afull[s], 4);
@@ -348,7 +356,8 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
   constexpr int BB = G::BB, NSLOT = G::NSLOT, NX = G::NX, PITCH = G::PITCH, HALVES = G::HALVES, DC = G::DC;
   constexpr bool KM = G::KM, TMA_W = MM_TMA_W<FMT, DENSE>;
   constexpr uint32_t W_BYTES = 4 * G::RAW_BYTES;  // a block's 128 rows
-  static_assert(!TMA_W || (PITCH == BB && (NX * G::X_BYTES + 2 * G::E_BYTES + 2 * G::M_BYTES) % 128 == 0 && W_BYTES % 128 == 0), "TMA writes rows of BB bytes");
+  static_assert(!TMA_W || ((PITCH == BB || FMT == ILL_Q6_K) && (NX * G::X_BYTES + 2 * G::E_BYTES + 2 * G::M_BYTES) % 128 == 0 && G::RAW_BYTES % 128 == 0), "where TMA writes");
+  const bool tma = mm_tma<FMT, DENSE>(p);
   // [X ring][KM: sums of 16 x 2, mins x 2] (the X tiles 1024-byte aligned, as the 128-byte swizzle needs), the
   // dequantizing warps' raw blocks, scales
   u8* x_tiles = smem;
@@ -514,10 +523,10 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
       mbar_wait(fin, 0, nullptr, 0, 0, ILL_WAIT_NS / 20);
     }
   } else if (warp < 4) {
-    // ---- warps 2, 3 (LOADERS) bring the raw windows of every block, half of each 32 rows' requests a warp; TMA_W: warp 2 its rows
+    // ---- warps 2, 3 (LOADERS) bring the raw windows of every block, half of each 32 rows' requests a warp; TMA: warp 2 its rows
     if constexpr (TMA_W) {
       int g_kb = 0;
-      for (int tile = warp == 2 ? cta : ntiles; tile < ntiles && ok; tile += ctas) {
+      for (int tile = warp == 2 && tma ? cta : ntiles; tile < ntiles && ok; tile += ctas) {
         int expert, row0, nvalid, nt;
         locate(tile, expert, row0, nvalid, nt);
         const bool second = nt >= ntn1;
@@ -528,7 +537,14 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
           if (!ok) break;
           if (elect_one()) {
             mbar_expect_tx(&raw_full[at], W_BYTES);
-            tma_load_2d(raw + at * W_BYTES, &maps.w[second], kb * BB, nt * MM_BN, &raw_full[at]);
+            const CUtensorMap* map = &maps.w[p.wmap + (second ? 1 : 0)];
+            if constexpr (FMT == ILL_Q4_K) {
+              tma_load_2d(raw + at * W_BYTES, map, kb * BB, nt * MM_BN, &raw_full[at]);
+            } else {
+#pragma unroll 1
+              for (int k = 0; k < 4; ++k)
+                tma_load_2d(raw + at * W_BYTES + k * G::RAW_BYTES, map, (k * p.row_bytes + kb * BB) & ~15, nt * (MM_BN / 4), &raw_full[at]);
+            }
           }
           __syncwarp();
         }
@@ -734,11 +750,12 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(G::REGS_DQ));
     const int wi = warp - (4 + G::DR_WARPS), wq = wi & 3, h = (wi >> 2) & 1, set = wi >> 3, row = 32 * wq + lane;
     const uint32_t lane_base = tmem_base + ((uint32_t)(wq * 32) << 16) + G::A_COL;  // this warp's lanes
-    // the two warps' two buffers (TMA_W: these rows of the set's two)
-    constexpr uint32_t BUF_BYTES = TMA_W ? W_BYTES : G::RAW_BYTES;
-    u8* praw = TMA_W ? raw + set * 2 * W_BYTES + wq * G::RAW_BYTES : raw + (set * 4 + wq) * 2 * G::RAW_BYTES;
-    uint64_t* rfull = raw_full + (TMA_W ? set : set * 4 + wq) * 2;
-    uint64_t* rempty = raw_empty + (TMA_W ? set : set * 4 + wq) * 2;
+    // this lane's row in the two warps' two buffers (TMA: in the set's two)
+    const uint32_t buf_bytes = tma ? W_BYTES : G::RAW_BYTES;
+    const u8* praw = !tma ? raw + (set * 4 + wq) * 2 * G::RAW_BYTES + lane * PITCH
+                     : FMT == ILL_Q4_K ? raw + set * 2 * W_BYTES + row * PITCH : raw + set * 2 * W_BYTES + (lane & 3) * G::RAW_BYTES + (row >> 2) * PITCH;
+    uint64_t* rfull = raw_full + (tma ? set : set * 4 + wq) * 2;
+    uint64_t* rempty = raw_empty + (tma ? set : set * 4 + wq) * 2;
     const uint4* grid = iq_grid + (lane & 7);
     const uint32_t* sgn = iq_sgn + lane;
     int tile = cta, kb = set;               // the block that is fetched next: of the CTA's blocks, every SETS-th
@@ -758,8 +775,8 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
     };
     auto start = [&]() { return ((uint32_t)(uintptr_t)wrow0 + (uint32_t)lane * (uint32_t)p.row_bytes + (uint32_t)kb * BB) & 15u; };
     auto fetch = [&](int buf) -> uint32_t {        // this warp's part of block kb's windows; where the lane's row starts in its own
-      if (TMA_W) return 0;
-      if (!G::LOADERS) mm_fetch<FMT, NT>(wrow0 + (long long)kb * BB, p.row_bytes, rows_here, h, lane, praw + buf * G::RAW_BYTES, &rfull[buf]);
+      if (!G::LOADERS && !tma)
+        mm_fetch<FMT, NT>(wrow0 + (long long)kb * BB, p.row_bytes, rows_here, h, lane, raw + ((set * 4 + wq) * 2 + buf) * G::RAW_BYTES, &rfull[buf]);
       return start();
     };
     at_tile();
@@ -775,12 +792,12 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
       to_block();
       more = tile < ntiles;
       if (more) {
-        if (!G::LOADERS && !TMA_W && !__all_sync(0xffffffffu, mbar_wait(&rempty[buf ^ 1], ((uint32_t)(it + 1) >> 1 & 1u) ^ 1u, p.status, ST_MM_WAIT_EMPTY + 2))) { ok = false; break; }
+        if (!G::LOADERS && !tma && !__all_sync(0xffffffffu, mbar_wait(&rempty[buf ^ 1], ((uint32_t)(it + 1) >> 1 & 1u) ^ 1u, p.status, ST_MM_WAIT_EMPTY + 2))) { ok = false; break; }
         o16n = fetch(buf ^ 1);
       }
       if (!__all_sync(0xffffffffu, mbar_wait(&rfull[buf], (uint32_t)(it >> 1) & 1u, p.status, ST_MM_WAIT_FULL + 2))) { ok = false; break; }
       const uint32_t sh = (o16 & 2u) * 8u;         // IQ2_XXS, Q6_K: the block may start in the middle of a word
-      const uint32_t* mine = (const uint32_t*)(praw + buf * BUF_BYTES + lane * PITCH);
+      const uint32_t* mine = (const uint32_t*)(praw + (buf ? buf_bytes : 0u));
       const uint32_t* rw = mine + (o16 >> 2);
       uint32_t dd, m4[2] = {0, 0};                 // d, dmin; Q4_K: the half's scales and mins, Q2_K: its eight scale bytes
       if constexpr (FMT == ILL_IQ2_XXS) dd = rw[0] >> sh;
@@ -809,8 +826,8 @@ __device__ __forceinline__ void mm_tiles(const MmMaps& maps, const MmParams& p, 
       };
       const uint32_t a0 = lane_base + G::SLOTW * (slot + 2 * h);
       if constexpr (FMT == ILL_Q6_K) {
-        // Left out for timing, 2560 x 9728 x 64 tokens of 62 us: what follows 19, its second stores 4, the raw copies 6 (one after the
-        // other in a warp; five or six slots in place of four gave nothing, reading the words in pairs neither).
+        // Left out for timing, 2560 x 9728 x 64 tokens of 62 us: what follows 19, its second stores 4, the raw copies 6 where these warps
+        // ask for them (one after the other in a warp; five or six slots in place of four gave nothing, reading the words in pairs neither).
         // Step jj of the half has the nibbles at shift 4 jj of ql[0 .. 63]; columns 32 sb .. of it go with the 2-bit fields at shift
         // 2 (2 jj + sb) of qh.  Sixteen weights (a group) at a time.
         uint32_t sc[2], se[2], so[2], ql[16], qh[8];
@@ -939,8 +956,8 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
   // (first tile of each expert, in shared memory).
   pdl_launch_dependents();
   if (tid == 32) {
-    bars->init(MM_TMA_W<FMT, DENSE>);
-    if constexpr (NT2 != 0) bars2->init(MM_TMA_W<FMT, DENSE>);
+    bars->init(mm_tma<FMT, DENSE>(p));
+    if constexpr (NT2 != 0) bars2->init(mm_tma<FMT, DENSE>(p));
     mbar_fence_init();
   }
   if (FMT == ILL_IQ2_XXS) {
@@ -1015,9 +1032,9 @@ __global__ void __launch_bounds__(MmGeom<FMT, NT>::THREADS, 1) mm_id_kernel(cons
 
 // Two dense matrices of few rows (K and V) against a chunk, with the bits of the int8 kernel of mma.sync: EX's accumulators hold a
 // block's sum exactly, and the drain takes that kernel's float steps.  FMT2 other than FMT: the second matrix (P2) is of another format,
-// and CTAs SPLIT and up take its tiles.  Bound by the unpacking of one block after the other in a CTA (0.75 us a block of Q4_K, 1.57
-// of Q6_K, and 0.0044 a row of X).  us, the int8 kernel's joint launch / this: K and V of 1024 x 2560, 512 tokens, both Q4_K 44 / 19.4, one of
-// Q6_K 48 / 29.5; of 1024 x 5120, both Q6_K 86 / 48.
+// and CTAs SPLIT and up take its tiles.  Bound by the unpacking of one block after the other in a CTA (0.75 us a block of Q4_K, 1.13
+// of Q6_K, and 0.004 a row of X).  us, the int8 kernel's joint launch / this: K and V of 1024 x 2560, 512 tokens, both Q4_K 44 / 19.4, one of
+// Q6_K 48 / 23.4; of 1024 x 5120, both Q6_K 86 / 38.
 template <int FMT, int FMT2>
 __global__ void __launch_bounds__(MmGeom<FMT, 64, true>::THREADS, 1)
     mm_exact_kernel(const __grid_constant__ MmMaps maps, const MmParams p, const MmParams p2, int split) {
@@ -1036,8 +1053,8 @@ __global__ void __launch_bounds__(MmGeom<FMT, 64, true>::THREADS, 1)
   const bool second = FMT2 != FMT && (int)blockIdx.x >= split;
   pdl_launch_dependents();
   if (tid == 32) {
-    if (second) bars2->init(MM_TMA_W<FMT2, true>);
-    else bars->init(MM_TMA_W<FMT, true>);
+    if (second) bars2->init(mm_tma<FMT2, true>(p2));
+    else bars->init(mm_tma<FMT, true>(p));
     mbar_fence_init();
     tile_first[0] = 0;
     tile_first[1] = (int)((p.one_count + p.bm - 1) / p.bm);
@@ -1545,16 +1562,21 @@ static int encode_map(CUtensorMap* map, ill_dptr base, int64_t cols, int64_t row
   return r == CUDA_SUCCESS ? ILL_OK : cuda_fail(cudaErrorInvalidValue);
 }
 
-// A Q4_K matrix's bytes, a block of 128 rows a load (rows past the last: zeros)
-static int encode_raw_map(CUtensorMap* map, ill_dptr base, int ncols, int rows) {
+// A matrix's bytes, 128 rows of a block a load, or (Q6_K) a window of 32 of every fourth row (rows past the last: zeros)
+static int encode_raw_map(CUtensorMap* map, int fmt, ill_dptr base, int ncols, int rows) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return cuda_fail(cudaErrorNotSupported);
-  const cuuint64_t row_bytes = (cuuint64_t)ncols / 256 * 144;
-  const cuuint64_t dims[2] = {row_bytes, (cuuint64_t)rows}, strides[1] = {row_bytes};
-  const cuuint32_t box[2] = {144, MM_BN}, estr[2] = {1, 1};
+  const int each = fmt == ILL_Q4_K ? 1 : 4;
+  const cuuint64_t bytes = (cuuint64_t)ncols / 256 * fmt_block_bytes(fmt) * each;
+  const cuuint64_t dims[2] = {bytes, (cuuint64_t)(rows / each)}, strides[1] = {bytes};
+  const cuuint32_t box[2] = {fmt == ILL_Q4_K ? 144u : 240u, (cuuint32_t)(MM_BN / each)}, estr[2] = {1, 1};
   const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)(uintptr_t)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? ILL_OK : cuda_fail(cudaErrorInvalidValue);
+}
+// Whether encode_raw_map takes a matrix: Q4_K's are 16-byte aligned by contract
+static bool raw_map_takes(int fmt, ill_dptr base, int ncols, int rows) {
+  return fmt == ILL_Q4_K || (fmt == ILL_Q6_K && !(base & 15) && rows % 4 == 0 && ncols % 512 == 0);
 }
 
 static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
@@ -1657,7 +1679,7 @@ static int mm_pick_tile(int fmt, long long rows, long long ntn, int sms) {
   int bm = 16;
   for (int b = 16; b <= (q6 ? 256 : 128); b += 16) {
     const long long tiles = (rows + b - 1) / b * ntn, rounds = (tiles + sms - 1) / sms;
-    const double us = b <= 64 ? (q6 ? 1.5 + 0.0048 * b : 0.82 + 0.0045 * b) : b <= 128 ? (q6 ? 1.5 + 0.0042 * b : 1.05 + 0.0043 * b) : 2.6 + 0.0033 * b;
+    const double us = b <= 64 ? (q6 ? 1.27 + 0.001 * b : 0.82 + 0.0045 * b) : b <= 128 ? (q6 ? 1.13 + 0.0032 * b : 1.05 + 0.0043 * b) : 1.75 + 0.0043 * b;
     if (rounds * us < best) { best = rounds * us; bm = b; }
   }
   return bm;
@@ -1687,14 +1709,17 @@ static int mm_id_launch(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptr
     if (rc) return rc;
   }
   if (!km) memcpy(maps.e, maps.x, sizeof maps.e);
+  const ill_dptr other = one_ptr + (y2 ? add2 : 0);
+  const bool tma = one_ptr && raw_map_takes(fmt, one_ptr, ncols, nrows) && raw_map_takes(fmt, other, ncols, nrows);
   for (int i = 0; i < 2; ++i) {
     maps.w[i] = maps.x[0];  // (not read)
-    if (one_ptr && fmt == ILL_Q4_K) {
-      const int rc = encode_raw_map(&maps.w[i], one_ptr + (i && y2 ? add2 : 0), ncols, nrows);
-      if (rc) return rc;
-    }
+    const int rc = tma ? encode_raw_map(&maps.w[i], fmt, i ? other : one_ptr, ncols, nrows) : ILL_OK;
+    if (rc) return rc;
   }
   MmParams p;
+  p.neg_zero = -0.0f;
+  p.tma = tma;
+  p.wmap = 0;
   p.ncols = ncols;
   p.nrows = nrows;
   p.row_bytes = ncols / 256 * fmt_block_bytes(fmt);
@@ -1760,9 +1785,10 @@ extern "C" int ill_mm_chunk_exact(int fmt, ill_dptr w, int fmt2, ill_dptr w2, in
     if (rc) return rc;
   }
   if (fmt != ILL_Q4_K) memcpy(maps.e, maps.x, sizeof maps.e);
+  const bool tma = raw_map_takes(fmt, w, cols, rows) && (mixed || raw_map_takes(fmt2, w2, cols, rows)), tma2 = mixed && raw_map_takes(fmt2, w2, cols, rows);
   for (int i = 0; i < 2; ++i) {
     maps.w[i] = maps.x[0];  // (not read)
-    const int rc = fmt == ILL_Q4_K && !(i && mixed) ? encode_raw_map(&maps.w[i], i ? w2 : w, cols, rows) : ILL_OK;
+    const int rc = (i && mixed ? tma2 : tma) ? encode_raw_map(&maps.w[i], i ? fmt2 : fmt, i ? w2 : w, cols, rows) : ILL_OK;
     if (rc) return rc;
   }
   MmParams p = {}, p2;
@@ -1777,9 +1803,12 @@ extern "C" int ill_mm_chunk_exact(int fmt, ill_dptr w, int fmt2, ill_dptr w2, in
   p.one_ptr = w;
   p.one_count = (unsigned)n;
   p.neg_zero = -0.0f;
+  p.tma = tma;
   p.status = device_status_word();
   p2 = p;
   if (mixed) {
+    p2.tma = tma2;
+    p2.wmap = 1;
     p2.row_bytes = cols / 256 * fmt_block_bytes(fmt2);
     p2.y = (float*)(uintptr_t)y2;
     p2.one_ptr = w2;
@@ -1797,7 +1826,7 @@ extern "C" int ill_mm_chunk_exact(int fmt, ill_dptr w, int fmt2, ill_dptr w2, in
   int split = 0;
   for (int b = 16; b <= 64; b += 16) {
     const long long tiles = (n + b - 1) / b * ntn, all = 2 * tiles, g = all < sms ? all : sms, rounds = (all + g - 1) / g;
-    const double t4 = 0.75 + 0.0044 * b, t6 = 1.57 + 0.0044 * b;
+    const double t4 = 0.75 + 0.0044 * b, t6 = 1.13 + 0.0035 * b;
     // (mixed: Q6_K, the slower, in at least its share of the rounds; a round more of its own leaves Q4_K more SMs)
     for (long long r = mixed ? 1 : rounds; r <= rounds; ++r) {
       const long long sp = mixed ? g - (tiles + r - 1) / r : 0;

@@ -173,17 +173,17 @@ def _side_stream(device):
 
 # Two matrices of few rows beside one of the tcgen05 kernel (which wants the activations' fp16 form in this stream in any case) go to the
 # exact form of that kernel: its tiles are 64 rows of X at most, which a chunk's K and V make one round of, and it adds the same integers
-# in the same steps as the int8 kernel.  us, int8 / exact, both of Q4_K | one of Q6_K: 1024 x 2560 of 64 tokens 23.5 / 17.3 | 23.5 / 25.6, of
-# 256 30 / 17 | 33 / 27, of 512 44 / 19 | 48 / 29, of 2048 135 / 54 | 133 / 68; 512 x 2048 of 256 20.5 / 15.3 | 20.5 / 23.5, of 512 25.5 / 15.4 |
-# 27.6 / 23.4; 256 x 2048 of 512 19.4 / 15.4 | 20.5 / 23.6, of 1024 25.5 / 15.4 | 27.6 / 23.6; 128 x 4096 of 2048 41 / 24 | 46 / 38.  A tile of Q6_K
-# takes twice one of Q4_K (two products and two accumulators of every K step), so few of them wait for it.
-EXACT_MIN_Q6K = 1 << 18  # rows times tokens
+# in the same steps as the int8 kernel.  us, int8 / exact, both of Q4_K | one of Q6_K: 1024 x 2560 of 64 tokens 23.5 / 17.3 | 23.5 / 21.5, of
+# 256 30 / 17 | 32 / 23, of 512 44 / 19 | 48 / 23, of 2048 135 / 54 | 133 / 64; 1024 x 8192 of 64 53 / 34 | 54 / 48; 256 x 2048 of 64 19.4 / 15.4 |
+# 19.4 / 18.5, of 2048 38 / 17 | 40 / 21; 128 x 4096 of 64 30 / 20 | 30 / 28.  Q6_K of an odd number of blocks, which a TMA load cannot
+# bring: 1024 x 2304 of 64 21.5 / 21.6, of 128 21.5 / 23.5, of 256 29.7 / 23.5.
+EXACT_MIN_Q6K = 1 << 18  # rows times tokens, there
 
 
 def _exact_takes(w, y, bias, like, act, n):
     """Whether a matrix beside one of _by_tc's, and in one launch with LIKE, goes to ill_mm_chunk_exact."""
-    return ((w.type == 1 or (w.type == 2 and w.rows * n >= EXACT_MIN_Q6K)) and 0 < w.rows == like.rows and w.rows % 4 == 0 and w.cols == like.cols and bias is None and w.qs.data_ptr() % 16 == 0
-            and y.data_ptr() % 16 == 0 and act.xq.numel() == n * w.cols)
+    return ((w.type == 1 or (w.type == 2 and (w.cols % 512 == 0 or w.rows * n >= EXACT_MIN_Q6K))) and 0 < w.rows == like.rows and w.rows % 4 == 0
+            and w.cols == like.cols and bias is None and w.qs.data_ptr() % 16 == 0 and y.data_ptr() % 16 == 0 and act.xq.numel() == n * w.cols)
 
 
 def chunk_mul_3(mats, act, n):
