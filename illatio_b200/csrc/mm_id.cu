@@ -22,14 +22,14 @@
 //   warps 4-..  drain the accumulators block by block (tcgen05.ld), scaling each block's integer
 //               sums by the block's float scales; then store the tile (a lane = a weight row, so
 //               the 32 lanes of a warp write 128 contiguous bytes of a row of Y)
-//   the others  bring W_e's raw blocks into shared memory (cp.async) and turn them into the A operand
+//   the others  bring W_e's raw blocks into shared memory (cp.async; or warps 2 and 3 do: LOADERS, MM_TMA_W) and turn them into the A operand
 // The roles' register needs differ widely, so the warp groups trade registers (setmaxnreg).
 // What bounds it: the drain beside the unpacking, by instructions and latency, not the tensor pipe or memory.  Left out for
 // timing: the drain's arithmetic 14-23 % of a launch, its stores 10 %, IQ2_XXS's unpacking 21 %, the X loads, the raw copies
 // and the products' width nothing.  us, with four drain warps, two raw-load warps and 128-row tiles throughout / now, timed in turn:
 // gate and up of 512 tokens x 2 x 9728 x 2560 (Q4_K) 153 / 83, 2560 x 9728 (Q6_K) 123 / 74; 64 tokens on 288 experts (Q2_K), gate and
 // up of 1536 x 5120 1146 / 660, down 671 / 378; 96 rows each on 256 experts, down of 4096 x 2048 (Q2_K) 774 / 682, gate and up of 2048 x
-// 4096 (IQ2_XXS) 1292 / 1274.
+// 4096 (IQ2_XXS) 1292 / 1274.  (Since, by who brings the raw blocks and how Q6_K is unpacked: Q4_K 7 % less, Q6_K 20 %; MM_TMA_W, w_q6k.)
 // Every mbarrier wait is bounded; on a time-out the kernel records a code in the status
 // word, skips what depends on the wait, lets copies and products in flight end, frees its tensor memory and returns.
 //

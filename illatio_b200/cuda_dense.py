@@ -182,7 +182,7 @@ EXACT_MIN_Q6K = 1 << 18  # rows times tokens, there
 
 def _exact_takes(w, y, bias, like, act, n):
     """Whether a matrix beside one of _by_tc's, and in one launch with LIKE, goes to ill_mm_chunk_exact."""
-    return ((w.type == 1 or (w.type == 2 and (w.cols % 512 == 0 or w.rows * n >= EXACT_MIN_Q6K))) and 0 < w.rows == like.rows and w.rows % 4 == 0
+    return ((w.type == 1 or (w.type == 2 and TC_Q6K and (w.cols % 512 == 0 or w.rows * n >= EXACT_MIN_Q6K))) and 0 < w.rows == like.rows and w.rows % 4 == 0
             and w.cols == like.cols and bias is None and w.qs.data_ptr() % 16 == 0 and y.data_ptr() % 16 == 0 and act.xq.numel() == n * w.cols)
 
 
@@ -297,7 +297,8 @@ def tc_takes(w, n):
 # Matrices of fewer rows (K and V, mostly) go to the int8 mma.sync kernel, which is slower there (us, tcgen05 / int8, 512 tokens:
 # 1024 x 2560 of Q4_K 14.0 / 21.6, 1024 x 5120 of Q6_K 37.5 / 45.1) but holds a block's sum in int32: in fp32, exact to 2^24, blocks
 # of near-constant weights and activations lose bits (relative error against 64 bits, tcgen05 / int8: Q6_K 4.9e-7 / 4.3e-8, Q4_K
-# 9.5e-8 / 4.5e-8; ordinary blocks 3.6e-8 both).  It also reads the quants themselves, in any stream and with Y at any float.
+# 9.5e-8 / 4.5e-8; ordinary blocks 3.6e-8 both).  It also reads the quants themselves, in any stream and with Y at any float.  (K and V beside a
+# larger Q: _exact_takes.)
 # Fewer tokens go there for the same reasons, not for speed: 17 / 63 tokens of 4096 x 2560 of Q4_K 13.2 / 13.6 us on tcgen05 and 19.0 /
 # 21.7, of 5120 x 5120 of Q6_K 36.4 / 38.0 and 38.7 / 45.0, and 2 us for the activations' fp16 form once.
 TC_MIN_TOKENS, TC_MIN_ROWS = 64, 2048
