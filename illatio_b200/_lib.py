@@ -59,6 +59,8 @@ SIGNATURES = {
     "ill_moe_few": (_I, [_I, _I, _I, _L, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _L, _S]),
     "ill_moe_few2": (_I, [_I, _I, _I, _L, _L, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _P, _L, _S]),
     "ill_moe_few_glu": (_I, [_I, _I, _I, _L, _L, _P, _P, _P, _I, _L, _P, _P, _P, _P, _F, _P, _P, _L, _S]),
+    "ill_moe_few_all": (_I, [_I, _I, _I, _L, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _L, _S]),
+    "ill_moe_few_glu_all": (_I, [_I, _I, _I, _L, _L, _P, _P, _P, _I, _L, _P, _P, _P, _P, _F, _P, _P, _L, _S]),
     "ill_moe_mm_id_over": (_I, [_I, _I, _I, _L, _L, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _P, _L, _I, _S]),
     "ill_act_f16_over": (_I, [_L, _I, _P, _P, _P, _P, _P, _P, _I, _I, _S]),
     "ill_swiglu_q8k_both": (_I, [_L, _I, _F, _P, _P, _P, _P, _P, _P, _P, _P, _S]),

@@ -11,7 +11,8 @@
 // for up to eight rows and 1180 and 1580 for sixteen, and HBM would take 460 and 360.  Beyond sixteen rows the chunk kernel's tile of 64
 // costs less than a second pass.  Bound by instruction issue: about 300 (Q2_K) and 540 (IQ2_XXS) a block of sixteen weight rows, the
 // logic (unpacking, look-ups) at half rate, 57 % and 67 % of the issue slots taken by the sixteen warps that 128 registers allow (twenty
-// of 96 registers: slower).  us of the routed experts, before / now: 64 tokens on 288 experts of Q2_K 757 / 467 (gate and up 475 / 268),
+// of 96 registers: slower).  An expert of more rows is left to the chunk kernel, or (ALL: no other launch follows) taken in passes of
+// sixteen.  us of the routed experts, before / now: 64 tokens on 288 experts of Q2_K 757 / 467 (gate and up 475 / 268),
 // on 256 of IQ2_XXS and Q2_K 1275 / 686; 2 tokens 153 / 123 and 145 / 115.
 //
 // Replaces d4_mv_iq2_xxs / d4_mv_q2_k with COUNTS / BASES (src/cuda/ds4f.cu:769-902) behind DK-FFN-SMALL
@@ -23,7 +24,8 @@
 
 namespace ill {
 
-constexpr int ME_WARPS = 16, ME_ROWS = 16, ME_MAX_STAGES = 4, ME_CB = 4 /* blocks a staged piece, at most */, ME_MAX_NE = 1024;
+constexpr int ME_WARPS = 16, ME_ROWS = 16, ME_MAX_STAGES = 4, ME_CB = 4 /* blocks a staged piece, at most */, ME_MAX_NE = 1024,
+              ME_LINE = 0x3fffffff;  // the line's length, at most
 
 struct MeParams {
   const unsigned long long* ptrs;
@@ -43,7 +45,8 @@ struct MeParams {
   float* y2;                   // two matrices, results apart: that of up
   const float* weights;        // ... or gated: a row's weight
   float clamp;
-  int most;                    // rows an expert of this launch has, at most: 8 or 16
+  int most;                    // rows that are taken at a time: 8 or 16
+  int all;                     // an expert with more rows is taken in passes of that many, not left out
   int pitch, stages;           // bytes between the rows of a staged piece; stages a warp
   uint32_t stage_bytes, xs_off, bs_off, ring_off, first_off /* where each expert's tiles start on the line; its end */;
   int x_stride;
@@ -76,25 +79,27 @@ __global__ void __launch_bounds__(32 * ME_WARPS, 1) mve_kernel(const __grid_cons
   // rows of an expert that is this launch's, and all of whose rows are there
   auto count = [&](int e) {
     const unsigned c = p.counts[e];
-    return c <= (unsigned)p.most && (long long)p.bases[e] + c <= p.total_rows ? (int)c : 0;
+    return (p.all || c <= (unsigned)p.most) && (long long)p.bases[e] + c <= p.total_rows ? (int)c : 0;
   };
+  const int pass_cost = ntr * me_cost(p.most);  // of a pass that is not an expert's last
   for (int e = tid; e < p.ne; e += nthreads) {
-    const int c = count(e);
-    first[e] = c ? ntr * me_cost(c) : 0;
+    const int c = count(e), passes = max(c - 1, 0) / p.most;
+    first[e] = c ? passes * pass_cost + ntr * me_cost(c - passes * p.most) : 0;
   }
   __syncthreads();
   if (warp == 0) {
     int before = 0;
     for (int e0 = 0; e0 < p.ne; e0 += 32) {
-      const int e = e0 + lane, c = e < p.ne ? first[e] : 0;
-      int incl = c;
+      const int e = e0 + lane;
+      int incl = e < p.ne ? first[e] : 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
+      for (int o = 1; o < 32; o <<= 1) {  // (what passes ME_LINE is of counts that add up to more rows than there are)
         const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
+        if (lane >= o) incl = min(incl + v, ME_LINE);
       }
-      if (e < p.ne) first[e] = before + incl - c;
-      before += __shfl_sync(0xffffffffu, incl, 31);
+      const int excl = __shfl_up_sync(0xffffffffu, incl, 1);
+      if (e < p.ne) first[e] = min(before + (lane ? excl : 0), ME_LINE);
+      before = min(before + __shfl_sync(0xffffffffu, incl, 31), ME_LINE);
     }
     if (lane == 0) first[p.ne] = before;
   }
@@ -102,18 +107,21 @@ __global__ void __launch_bounds__(32 * ME_WARPS, 1) mve_kernel(const __grid_cons
   const long long line = first[p.ne];
   const int lo = (int)(line * blockIdx.x / gridDim.x), hi = (int)(line * (blockIdx.x + 1) / gridDim.x);
 
-  // The CTA's experts in order: of each, the tiles that start in LO .. HI
+  // The CTA's experts in order, pass by pass: of each, the tiles that start in LO .. HI
   struct Seg {
-    int e, row0, n;     // the expert, its first row, its rows
-    int t0, t1;         // the CTA's tiles of it
+    int e, pass, row0, n;  // the expert, the pass, its first row, its rows
+    int t0, t1;            // the CTA's tiles of it
+    int end;               // where it ends on the line
     const u8* w;
   };
   auto fill = [&](Seg& s) {
-    s.row0 = (int)p.bases[s.e];
-    s.n = count(s.e);
-    const int cost = me_cost(s.n), at = first[s.e];
+    const int done = s.pass * p.most;
+    s.row0 = (int)p.bases[s.e] + done;
+    s.n = min(count(s.e) - done, p.most);
+    const int cost = me_cost(s.n), at = first[s.e] + s.pass * pass_cost;
     s.t0 = at >= lo ? 0 : (lo - at + cost - 1) / cost;
     s.t1 = min(ntr, (hi - at + cost - 1) / cost);
+    s.end = at + ntr * cost;
     s.w = (const u8*)(uintptr_t)after_wait(p.ptrs)[s.e] + p.add;
   };
   auto begin = [&](Seg& s) -> bool {  // the one that LO lies in: the last that starts there or before (one without rows ends where it starts)
@@ -124,13 +132,18 @@ __global__ void __launch_bounds__(32 * ME_WARPS, 1) mve_kernel(const __grid_cons
       if (first[m] <= lo) a = m; else b = m - 1;
     }
     s.e = a;
+    s.pass = (lo - first[a]) / pass_cost;
     fill(s);
     return true;
   };
   auto next = [&](Seg& s) -> bool {
-    const int end = first[s.e + 1];
+    const int end = s.end;
     if (end >= hi) return false;
-    do ++s.e; while (first[s.e + 1] <= end);  // (the line's end is beyond END)
+    ++s.pass;
+    if (first[s.e + 1] <= end) {
+      do ++s.e; while (first[s.e + 1] <= end);  // (the line's end is beyond END)
+      s.pass = 0;
+    }
     fill(s);
     return true;
   };
@@ -318,7 +331,7 @@ extern "C" int ill_moe_few_most(int fmt, int ncols) {
   return me_plan(fmt, ncols, 1, &p, &smem) == ILL_OK ? p.most : 0;
 }
 
-static int moe_few(int fmt, int ncols, int nrows, int64_t add, int64_t add2, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
+static int moe_few(bool all, int fmt, int ncols, int nrows, int64_t add, int64_t add2, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
                    int64_t total_rows, ill_dptr xq, ill_dptr xs, ill_dptr xsum, ill_dptr map, float clamp, ill_dptr weights, ill_dptr y,
                    ill_dptr y2, int64_t y_stride, ill_stream stream) {
   if (fmt != ILL_Q2_K && fmt != ILL_IQ2_XXS) return ILL_ERR_UNSUPPORTED;
@@ -328,7 +341,7 @@ static int moe_few(int fmt, int ncols, int nrows, int64_t add, int64_t add2, ill
   if ((ptrs & 7) || (counts & 3) || (bases & 3) || (xq & 15) || (xs & 3) || (xsum & 7) || (map & 3) || (weights & 3) || (y & 3) || (y2 & 3))
     return ILL_ERR_ALIGN;
   const long long ntr = (nrows + ME_ROWS - 1) / ME_ROWS, experts = ne < total_rows ? ne : total_rows;  // with rows, at most
-  if (ne > ME_MAX_NE || 3 * ntr * ne > 0x3fffffff) return ILL_ERR_TOO_LARGE;
+  if (ne > ME_MAX_NE || 3 * ntr * ne > ME_LINE || (all && total_rows > 8 * (ME_LINE / (3 * ntr) - ne))) return ILL_ERR_TOO_LARGE;
   if (total_rows == 0) return ILL_OK;
   MeParams p = {};
   size_t smem = 0;
@@ -339,6 +352,7 @@ static int moe_few(int fmt, int ncols, int nrows, int64_t add, int64_t add2, ill
   p.bases = (const unsigned*)(uintptr_t)bases;
   p.map = (const unsigned*)(uintptr_t)map;
   p.ne = ne;
+  p.all = all;
   p.total_rows = total_rows;
   p.add = add;
   p.up_add = add2 - add;
@@ -367,20 +381,34 @@ static int moe_few(int fmt, int ncols, int nrows, int64_t add, int64_t add2, ill
 extern "C" int ill_moe_few(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
                            int64_t total_rows, ill_dptr xq, ill_dptr xs, ill_dptr xsum, ill_dptr map, ill_dptr y, int64_t y_stride,
                            ill_stream stream) {
-  return moe_few(fmt, ncols, nrows, add, add, ptrs, counts, bases, ne, total_rows, xq, xs, xsum, map, 0.0f, 0, y, 0, y_stride, stream);
+  return moe_few(false, fmt, ncols, nrows, add, add, ptrs, counts, bases, ne, total_rows, xq, xs, xsum, map, 0.0f, 0, y, 0, y_stride, stream);
 }
 
 extern "C" int ill_moe_few2(int fmt, int ncols, int nrows, int64_t add, int64_t add2, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
                             int64_t total_rows, ill_dptr xq, ill_dptr xs, ill_dptr xsum, ill_dptr map, ill_dptr y, ill_dptr y2,
                             int64_t y_stride, ill_stream stream) {
   if (!y2) return ILL_ERR_ARG;
-  return moe_few(fmt, ncols, nrows, add, add2, ptrs, counts, bases, ne, total_rows, xq, xs, xsum, map, 0.0f, 0, y, y2, y_stride, stream);
+  return moe_few(false, fmt, ncols, nrows, add, add2, ptrs, counts, bases, ne, total_rows, xq, xs, xsum, map, 0.0f, 0, y, y2, y_stride, stream);
 }
 
 extern "C" int ill_moe_few_glu(int fmt, int ncols, int nrows, int64_t gate_add, int64_t up_add, ill_dptr ptrs, ill_dptr counts,
                                ill_dptr bases, int ne, int64_t total_rows, ill_dptr xq, ill_dptr xs, ill_dptr xsum, ill_dptr map,
                                float clamp, ill_dptr weights, ill_dptr mid, int64_t mid_stride, ill_stream stream) {
   if (!weights) return ILL_ERR_ARG;
-  return moe_few(fmt, ncols, nrows, gate_add, up_add, ptrs, counts, bases, ne, total_rows, xq, xs, xsum, map, clamp, weights, mid, 0, mid_stride,
+  return moe_few(false, fmt, ncols, nrows, gate_add, up_add, ptrs, counts, bases, ne, total_rows, xq, xs, xsum, map, clamp, weights, mid, 0, mid_stride,
                  stream);
+}
+
+extern "C" int ill_moe_few_all(int fmt, int ncols, int nrows, int64_t add, ill_dptr ptrs, ill_dptr counts, ill_dptr bases, int ne,
+                               int64_t total_rows, ill_dptr xq, ill_dptr xs, ill_dptr xsum, ill_dptr map, ill_dptr y, int64_t y_stride,
+                               ill_stream stream) {
+  return moe_few(true, fmt, ncols, nrows, add, add, ptrs, counts, bases, ne, total_rows, xq, xs, xsum, map, 0.0f, 0, y, 0, y_stride, stream);
+}
+
+extern "C" int ill_moe_few_glu_all(int fmt, int ncols, int nrows, int64_t gate_add, int64_t up_add, ill_dptr ptrs, ill_dptr counts,
+                                   ill_dptr bases, int ne, int64_t total_rows, ill_dptr xq, ill_dptr xs, ill_dptr xsum, ill_dptr map,
+                                   float clamp, ill_dptr weights, ill_dptr mid, int64_t mid_stride, ill_stream stream) {
+  if (!weights) return ILL_ERR_ARG;
+  return moe_few(true, fmt, ncols, nrows, gate_add, up_add, ptrs, counts, bases, ne, total_rows, xq, xs, xsum, map, clamp, weights, mid, 0,
+                 mid_stride, stream);
 }

@@ -97,14 +97,16 @@ def few_rows(pool, n, nu):
 
 def _few_rows_chunk(pool, n, nu, clamp, sc, shared, most, st):
     """The chunk's experts that have up to MOST rows by the products for a few rows an expert, the others by the chunk's: the same
-    bits either way.  A token has an expert once, so up to MOST tokens have none of the others."""
+    bits either way.  Up to MOST tokens have none of the others unless the router gives a token one expert again (scores that are all NaN or
+    -inf: expert 0 for every slot that is left), so they go to the former alone, which then takes that expert in passes."""
     d, ff, ne = pool.d, pool.ff, pool.n_expert
     who = (_ptr(pool.ptrs_all), _ptr(sc.counts), _ptr(sc.bases), ne, sc.rows)
     x, mid = (_ptr(sc.xq.xq), _ptr(sc.xq.xs), _ptr(sc.xq.xsum)), (_ptr(sc.midq.xq), _ptr(sc.midq.xs), _ptr(sc.midq.xsum))
     if n <= most:
-        _lib.call("ill_moe_few_glu", pool.gate_fmt, d, ff, 0, pool.gate_bytes, *who, *x, _ptr(sc.rmap), float(clamp), _ptr(sc.wrow),
+        _lib.call("ill_moe_few_glu_all", pool.gate_fmt, d, ff, 0, pool.gate_bytes, *who, *x, _ptr(sc.rmap), float(clamp), _ptr(sc.wrow),
                   _ptr(sc.mid), ff, st)
         D.quant_q8(sc.mid, sc.midq)
+        _lib.call("ill_moe_few_all", pool.down_fmt, ff, d, 2 * pool.gate_bytes, *who, *mid, 0, _ptr(sc.down), d, st)
     else:
         _lib.call("ill_act_f16_over", sc.rows, d, x[0], x[2], _ptr(sc.rmap), _ptr(sc.xh), _ptr(sc.xe), _ptr(sc.counts), ne, most, st)
         _lib.call("ill_moe_few2", pool.gate_fmt, d, ff, 0, pool.gate_bytes, *who, *x, _ptr(sc.rmap), _ptr(sc.g), _ptr(sc.u), ff, st)
@@ -112,8 +114,7 @@ def _few_rows_chunk(pool, n, nu, clamp, sc, shared, most, st):
                   _ptr(sc.g), _ptr(sc.u), ff, most, st)
         _lib.call("ill_swiglu_q8k_both", sc.rows, ff, float(clamp), _ptr(sc.g), _ptr(sc.u), _ptr(sc.wrow), _ptr(sc.mh), _ptr(sc.me), mid[1],
                   mid[0], mid[2], st)
-    _lib.call("ill_moe_few", pool.down_fmt, ff, d, 2 * pool.gate_bytes, *who, *mid, 0, _ptr(sc.down), d, st)
-    if n > most:
+        _lib.call("ill_moe_few", pool.down_fmt, ff, d, 2 * pool.gate_bytes, *who, *mid, 0, _ptr(sc.down), d, st)
         _lib.call("ill_moe_mm_id_over", pool.down_fmt, ff, d, 2 * pool.gate_bytes, 0, *who, _ptr(sc.mh), _ptr(sc.me), mid[1], 0, _ptr(sc.down),
                   0, d, most, st)
     _lib.call("ill_moe_sum", d, nu, n, _ptr(sc.down), _ptr(sc.smap), _ptr(shared), _ptr(sc.moe), st)

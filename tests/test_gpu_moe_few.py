@@ -105,3 +105,79 @@ def test_chunk_driver_with_and_without(n, gate):
         assert sc.counts.max() > 16 and sc.counts.min() <= 16
     want = P.dk_ffn_routed_chunk(pool, norms, logits, nu, 10.0, sc, fused=False)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("n,d", [(4, 512), (16, 512), (4, 7168)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_a_router_that_gives_a_token_one_expert_again(n, d, masked):
+    """Scores that are NaN, or -inf by a mask that leaves fewer than NU experts: the router takes expert 0 for each of the slots that are
+    left, which then has more rows than a launch for a few takes at a time.  The other tokens' rows are theirs, bit for bit, and none
+    is what the scratch held before.  (7168 columns of IQ2_XXS: eight rows at a time.)"""
+    ff, ne, nu = 256, 12, 8
+    pool = M.make_expert_pool(B.synth_matrix(B.IQ2_XXS, ne * ff, d, seed=1), B.synth_matrix(B.IQ2_XXS, ne * ff, d, seed=2),
+                              B.synth_matrix(B.Q2_K, ne * d, ff, seed=3), d, ff, ne, gate_fmt=B.IQ2_XXS)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    norms, logits = torch.randn(n, d, device="cuda", generator=g), torch.randn(n, ne, device="cuda", generator=g)
+    healthy, bias = torch.ones(n, dtype=torch.bool, device="cuda"), None
+    if masked:
+        bias = torch.full((ne,), float("-inf"), device="cuda")
+        bias[[2, 5, 7]] = 0.0
+    else:
+        logits[:, 0] += 30.0     # the healthy ones choose expert 0 too
+        logits[1] = logits[n - 1] = float("nan")
+        healthy[1] = healthy[n - 1] = False
+    sc = P.make_chunk_scratch(pool, n, nu)
+    most = P.few_rows(pool, n, nu)
+    assert most == (16 if d == 512 else 8)
+    want = P.dk_ffn_routed_chunk(pool, norms, logits, nu, 10.0, sc, bias=bias, fused=False).clone()
+    assert int(sc.counts[0]) > most
+    for t in (sc.mid, sc.down, sc.g, sc.u, sc.moe):
+        t.fill_(1e30)
+    got = P.dk_ffn_routed_chunk(pool, norms, logits, nu, 10.0, sc, bias=bias)
+    assert torch.isfinite(want[healthy]).all() and torch.equal(got[healthy], want[healthy])
+
+
+@pytest.mark.parametrize("fmt,cols", [(B.IQ2_XXS, 512), (B.Q2_K, 768), (B.Q2_K, 9216)])
+@pytest.mark.parametrize("counts", [(17, 0, 16, 33, 1), (40,), (0, 8, 9, 64, 0, 25)])
+def test_all_experts_in_passes(fmt, cols, counts):
+    """ill_moe_few_all and ill_moe_few_glu_all: experts of more rows than a pass has (16; 8 of 9216 columns), at the edges of a pass and
+    beside experts of few and of none: the chunk product's bits."""
+    rows, ne, n = 200, len(counts), sum(counts)
+    nbytes = B.matrix_bytes(fmt, rows, cols)
+    step = (2 * nbytes + 15) // 16 * 16
+    buf = torch.zeros(ne * step, dtype=torch.uint8, device="cuda")
+    for e in range(ne):
+        buf[e * step:e * step + 2 * nbytes] = B.synth_matrix_torch(fmt, 2 * rows, cols, seed=e + rows)
+    g = torch.Generator(device="cuda").manual_seed(n + cols)
+    act = D.quant_q8(torch.randn(n * cols, device="cuda", generator=g), D.make_qact(n * cols, "q8k"))
+    tmap = torch.randint(0, n, (n,), dtype=torch.int32, device="cuda", generator=g)
+    xh, xe = torch.empty(n, cols, dtype=torch.float16, device="cuda"), torch.empty(n, cols // 256, 64, dtype=torch.float16, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    ptrs = torch.tensor([_p(buf) + e * step for e in range(ne)], dtype=torch.int64, device="cuda")
+    cnt, bases = torch.tensor(counts, **i32), torch.tensor([sum(counts[:e]) for e in range(ne)], **i32)
+    who, x = (_p(ptrs), _p(cnt), _p(bases), ne, n), (_p(act.xq), _p(act.xs), _p(act.xsum), _p(tmap))
+    _lib.call("ill_act_f16", n, cols, x[0], x[2], _p(tmap), _p(xh), _p(xe), _lib.stream())
+    want = [torch.empty(n, rows, device="cuda") for _ in range(2)]
+    _lib.call("ill_moe_mm_id2", fmt, cols, rows, 0, nbytes, *who, _p(xh), _p(xe), x[1], _p(tmap), _p(want[0]), _p(want[1]), rows, _lib.stream())
+    w = torch.rand(n, device="cuda", generator=g)
+    got, mid, ref = (torch.full((n, rows), 5.0, device="cuda") for _ in range(3))
+    _lib.call("ill_moe_few_all", fmt, cols, rows, nbytes, *who, *x, _p(got), rows, _lib.stream())
+    _lib.call("ill_moe_few_glu_all", fmt, cols, rows, 0, nbytes, *who, *x, 1.5, _p(w), _p(mid), rows, _lib.stream())
+    _lib.call("ill_swiglu_w", n * rows, rows, 1.5, _p(want[0]), _p(want[1]), _p(w), _p(ref), _lib.stream())
+    assert torch.equal(got, want[1]) and torch.equal(mid, ref)
+
+
+def test_counts_past_the_rows_there_are_in_passes():
+    """Counts that add up to more rows than there are (experts that share rows): each expert's results, in some order, and nothing else."""
+    fmt, rows, cols, n, ne = B.Q2_K, 48, 512, 40, 3
+    w = B.synth_matrix_torch(fmt, rows, cols, seed=1)
+    act = D.quant_q8(torch.randn(n * cols, device="cuda"), D.make_qact(n * cols, "q8k"))
+    i32 = dict(dtype=torch.int32, device="cuda")
+    ptrs = torch.full((ne,), _p(w), dtype=torch.int64, device="cuda")
+    cnt, bases = torch.tensor([40, 40, 41], **i32), torch.zeros(ne, **i32)
+    y, one = torch.full((n + 16, rows), 5.0, device="cuda"), torch.empty(n, rows, device="cuda")
+    _lib.call("ill_moe_few_all", fmt, cols, rows, 0, _p(ptrs), _p(cnt), _p(bases), ne, n, _p(act.xq), _p(act.xs), _p(act.xsum), 0, _p(y), rows, _lib.stream())
+    for t in range(0, n, 8):
+        _lib.call("ill_moe_few", fmt, cols, rows, 0, _p(ptrs), _p(torch.tensor([8], **i32)), _p(bases), 1, 8, _p(act.xq) + t * cols, _p(act.xs) + 4 * t * (cols // 256),
+                  _p(act.xsum) + 2 * t * (cols // 16), 0, _p(one) + 4 * t * rows, rows, _lib.stream())
+    assert torch.equal(y[:n], one) and (y[n:] == 5.0).all()
