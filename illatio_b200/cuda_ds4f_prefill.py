@@ -85,19 +85,24 @@ def mm_id(pool, fmt, ncols, nrows, add, sc, xh, xe, xd, rmap, y):
 FEW_MEAN = 64
 
 
+def _few_limits(pool):
+    """Rows an expert has, at most, for the products of a few rows an expert to do it: of gate and up, of down."""
+    most = _lib.lib().ill_moe_few_most
+    return most(pool.gate_fmt, pool.d), most(pool.down_fmt, pool.ff)
+
+
 def few_rows(pool, n, nu):
-    """Rows an expert has, at most, for the products of a few rows an expert to do it in a chunk of N tokens (0: none of the chunk's)."""
+    """Rows an expert has, at most, for the products of a few rows an expert to do all of it in a chunk of N tokens (0: none of the chunk's)."""
     if n * nu > FEW_MEAN * pool.n_expert or pool.gate_fmt not in (Q2_K, IQ2_XXS) or pool.down_fmt not in (Q2_K, IQ2_XXS):
         return 0
     if pool.n_expert > 512:
         return 0
-    L = _lib.lib()
-    return min(L.ill_moe_few_most(pool.gate_fmt, pool.d), L.ill_moe_few_most(pool.down_fmt, pool.ff))
+    return min(_few_limits(pool))
 
 
 def _few_rows_chunk(pool, n, nu, clamp, sc, shared, most, st):
-    """The chunk's experts that have up to MOST rows by the products for a few rows an expert, the others by the chunk's: the same
-    bits either way.  Up to MOST tokens have none of the others unless the router gives a token one expert again (scores that are all NaN or
+    """The chunk's experts that have a few rows by the products for those, up to each product's limit (of which MOST is the smaller),
+    the others by the chunk's: the same bits either way.  Up to MOST tokens have none of the others unless the router gives a token one expert again (scores that are all NaN or
     -inf: expert 0 for every slot that is left), so they go to the former alone, which then takes that expert in passes."""
     d, ff, ne = pool.d, pool.ff, pool.n_expert
     who = (_ptr(pool.ptrs_all), _ptr(sc.counts), _ptr(sc.bases), ne, sc.rows)
@@ -108,15 +113,16 @@ def _few_rows_chunk(pool, n, nu, clamp, sc, shared, most, st):
         D.quant_q8(sc.mid, sc.midq)
         _lib.call("ill_moe_few_all", pool.down_fmt, ff, d, 2 * pool.gate_bytes, *who, *mid, 0, _ptr(sc.down), d, st)
     else:
-        _lib.call("ill_act_f16_over", sc.rows, d, x[0], x[2], _ptr(sc.rmap), _ptr(sc.xh), _ptr(sc.xe), _ptr(sc.counts), ne, most, st)
+        gate_most, down_most = _few_limits(pool)
+        _lib.call("ill_act_f16_over", sc.rows, d, x[0], x[2], _ptr(sc.rmap), _ptr(sc.xh), _ptr(sc.xe), _ptr(sc.counts), ne, gate_most, st)
         _lib.call("ill_moe_few2", pool.gate_fmt, d, ff, 0, pool.gate_bytes, *who, *x, _ptr(sc.rmap), _ptr(sc.g), _ptr(sc.u), ff, st)
         _lib.call("ill_moe_mm_id_over", pool.gate_fmt, d, ff, 0, pool.gate_bytes, *who, _ptr(sc.xh), _ptr(sc.xe), x[1], _ptr(sc.rmap),
-                  _ptr(sc.g), _ptr(sc.u), ff, most, st)
+                  _ptr(sc.g), _ptr(sc.u), ff, gate_most, st)
         _lib.call("ill_swiglu_q8k_both", sc.rows, ff, float(clamp), _ptr(sc.g), _ptr(sc.u), _ptr(sc.wrow), _ptr(sc.mh), _ptr(sc.me), mid[1],
                   mid[0], mid[2], st)
         _lib.call("ill_moe_few", pool.down_fmt, ff, d, 2 * pool.gate_bytes, *who, *mid, 0, _ptr(sc.down), d, st)
         _lib.call("ill_moe_mm_id_over", pool.down_fmt, ff, d, 2 * pool.gate_bytes, 0, *who, _ptr(sc.mh), _ptr(sc.me), mid[1], 0, _ptr(sc.down),
-                  0, d, most, st)
+                  0, d, down_most, st)
     _lib.call("ill_moe_sum", d, nu, n, _ptr(sc.down), _ptr(sc.smap), _ptr(shared), _ptr(sc.moe), st)
     return sc.moe
 

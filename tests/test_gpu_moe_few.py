@@ -181,3 +181,20 @@ def test_counts_past_the_rows_there_are_in_passes():
         _lib.call("ill_moe_few", fmt, cols, rows, 0, _p(ptrs), _p(torch.tensor([8], **i32)), _p(bases), 1, 8, _p(act.xq) + t * cols, _p(act.xs) + 4 * t * (cols // 256),
                   _p(act.xsum) + 2 * t * (cols // 16), 0, _p(one) + 4 * t * rows, rows, _lib.stream())
     assert torch.equal(y[:n], one) and (y[n:] == 5.0).all()
+
+
+def test_chunk_driver_with_limits_that_differ():
+    """Eight rows of 7168 columns of IQ2_XXS for gate and up, sixteen for down: experts between them, and of fewer and more."""
+    d, ff, ne, nu, n = 7168, 256, 12, 3, 40
+    pool = M.make_expert_pool(B.synth_matrix(B.IQ2_XXS, ne * ff, d, seed=1), B.synth_matrix(B.IQ2_XXS, ne * ff, d, seed=2),
+                              B.synth_matrix(B.Q2_K, ne * d, ff, seed=3), d, ff, ne, gate_fmt=B.IQ2_XXS)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    norms, logits = torch.randn(n, d, device="cuda", generator=g), torch.randn(n, ne, device="cuda", generator=g)
+    logits[:, 4] += 30.0
+    sc = P.make_chunk_scratch(pool, n, nu)
+    want = P.dk_ffn_routed_chunk(pool, norms, logits, nu, 10.0, sc, fused=False).clone()
+    c = sc.counts
+    assert ((c > 8) & (c <= 16)).any() and (c > 16).any() and (c <= 8).any()
+    for t in (sc.down, sc.g, sc.u, sc.moe):
+        t.fill_(1e30)
+    assert torch.equal(P.dk_ffn_routed_chunk(pool, norms, logits, nu, 10.0, sc), want)
