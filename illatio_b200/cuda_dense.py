@@ -343,6 +343,31 @@ def decode_op(w, x, y, w2=None, norm_w=None, eps=1e-6, bias=None, acc=False, aft
     return op
 
 
+class _Chain:
+    """Recorded launches (ill_chain_new) and the scratch that they go through, given back with the last plan that has them: copies of a
+    plan share them, and no other process can have them."""
+
+    def __init__(self, arr, n, device):
+        import ctypes
+        self.handle = ctypes.c_uint64(0)
+        nbytes = _lib.lib().ill_chain_scratch_bytes(arr, n)
+        self.scratch = torch.empty(nbytes + 128, dtype=torch.uint8, device=device)
+        _lib.call("ill_chain_new", arr, n, (self.scratch.data_ptr() + 127) // 128 * 128, nbytes, ctypes.byref(self.handle))
+
+    def __del__(self):
+        if self.handle and _lib is not None:
+            _lib.status("ill_chain_free", self.handle)
+
+    def __copy__(self):
+        return self
+
+    def __deepcopy__(self, memo):
+        return self
+
+    def __reduce__(self):
+        raise TypeError("a plan's recorded launches belong to this process")
+
+
 class DecodePlan:
     """A token's chain of products enqueued with one call: what CUDA-FORWARD-N (src/cuda-dense.lisp:380-432) issues as a
     launch per product and per quantization.  OPS: decode_op()s in order.  The plan owns its device memory and the recorded
@@ -350,7 +375,6 @@ class DecodePlan:
 
     def __init__(self, ops, device="cuda"):
         import ctypes
-        self.chain = ctypes.c_uint64(0)
         self.n = len(ops)
         arr = (_lib.DecodeOp * self.n)(*ops)
         nbytes = _lib.lib().ill_decode_plan_bytes(self.n)
@@ -360,17 +384,10 @@ class DecodePlan:
             # (the one-launch form's plan: what it refuses is refused)
             plan = torch.zeros(nbytes + 128, dtype=torch.uint8, device=device)
             _lib.call("ill_decode_plan", arr, self.n, (plan.data_ptr() + 127) // 128 * 128, nbytes, (ctypes.c_int32 * 16)(), _stream())
-            nbytes = _lib.lib().ill_chain_scratch_bytes(arr, self.n)
-            self.scratch = torch.empty(nbytes + 128, dtype=torch.uint8, device=device)
-            _lib.call("ill_chain_new", arr, self.n, (self.scratch.data_ptr() + 127) // 128 * 128, nbytes, ctypes.byref(self.chain))
+            self.chain = _Chain(arr, self.n, device)
 
     def run(self):
-        _lib.call("ill_chain_run", self.chain, _stream())
-
-    def __del__(self):
-        if getattr(self, "chain", None) and _lib is not None:
-            _lib.status("ill_chain_free", self.chain)
-            self.chain = None
+        _lib.call("ill_chain_run", self.chain.handle, _stream())
 
 
 def dequant_rows(w, first_row, nrows, out=None):
