@@ -349,7 +349,7 @@ class _Chain:
 
     def __init__(self, arr, n, device):
         import ctypes
-        self.handle = ctypes.c_uint64(0)
+        self.handle, self.stream = ctypes.c_uint64(0), _stream()
         nbytes = _lib.lib().ill_chain_scratch_bytes(arr, n)
         self.scratch = torch.empty(nbytes + 128, dtype=torch.uint8, device=device)
         _lib.call("ill_chain_new", arr, n, (self.scratch.data_ptr() + 127) // 128 * 128, nbytes, ctypes.byref(self.handle))
@@ -357,6 +357,12 @@ class _Chain:
     def __del__(self):
         if self.handle and _lib is not None:
             _lib.status("ill_chain_free", self.handle)
+
+    def run(self):
+        st = _stream()
+        _lib.call("ill_chain_run", self.handle, st)
+        if st != self.stream:  # the scratch is this stream's too: not given out anew before what runs here is through
+            self.scratch.record_stream(torch.cuda.current_stream())
 
     def __copy__(self):
         return self
@@ -370,8 +376,9 @@ class _Chain:
 
 class DecodePlan:
     """A token's chain of products enqueued with one call: what CUDA-FORWARD-N (src/cuda-dense.lisp:380-432) issues as a
-    launch per product and per quantization.  OPS: decode_op()s in order.  The plan owns its device memory and the recorded
-    launches (ill_chain_new); run() enqueues one token on the current stream."""
+    launch per product and per quantization.  OPS: decode_op()s in order.  The plan owns its scratch and the recorded
+    launches (ill_chain_new); run() enqueues one token on the current stream, any stream of the device.  It may go while a token is
+    on its way, but not before a recording of the caller's that run() went into, nor before the buffers that OPS names."""
 
     def __init__(self, ops, device="cuda"):
         import ctypes
@@ -387,7 +394,7 @@ class DecodePlan:
             self.chain = _Chain(arr, self.n, device)
 
     def run(self):
-        _lib.call("ill_chain_run", self.chain.handle, _stream())
+        self.chain.run()
 
 
 def dequant_rows(w, first_row, nrows, out=None):

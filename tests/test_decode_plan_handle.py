@@ -39,3 +39,18 @@ def test_copies_of_a_plan_share_its_launches(freed):
 def test_a_plan_does_not_outlive_its_process(freed):
     with pytest.raises(TypeError):
         pickle.dumps(D.DecodePlan([_lib.DecodeOp()], device="cpu"))
+
+
+def test_scratch_is_held_for_a_stream_of_another_run(freed, monkeypatch):
+    plan, held = D.DecodePlan([_lib.DecodeOp()], device="cpu"), []
+
+    class Scratch(torch.Tensor):
+        def record_stream(self, stream):
+            held.append(stream)
+    plan.chain.scratch = plan.chain.scratch.as_subclass(Scratch)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: "another")
+    plan.run()
+    assert held == []
+    monkeypatch.setattr(D, "_stream", lambda: 7)
+    plan.run()
+    assert held == ["another"]

@@ -96,6 +96,26 @@ def test_into_a_recording_and_in_another_stream():
     torch.cuda.synchronize()
 
 
+def test_scratch_of_a_plan_that_runs_in_another_stream():
+    """The plan goes while a token waits in a stream that is not the one it was made in: its scratch is not given out meanwhile."""
+    m = Layer(B.Q4_K, B.Q6_K)
+    plan = D.DecodePlan(m.ops)
+    want = m.state(plan.run)
+    m.h.copy_(m.x0)
+    torch.cuda.synchronize()
+    side, busy = torch.cuda.Stream(), torch.cuda.Event()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)
+        plan.run()
+        busy.record()
+    at, size = plan.chain.scratch.data_ptr(), plan.chain.scratch.numel()
+    del plan
+    others = [torch.empty(size, dtype=torch.uint8, device="cuda") for _ in range(3)]
+    assert not busy.query() and all(t.data_ptr() != at for t in others)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip([m.h, *m.out], want))
+
+
 def test_what_a_chain_refuses():
     m = Layer(B.Q4_K, B.Q6_K)
     n = len(m.ops)
