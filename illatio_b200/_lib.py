@@ -27,6 +27,7 @@ class DecodeOp(_c.Structure):
 
 SIGNATURES = {
     "ill_decode_plan_bytes": (_L, [_I]),
+    "ill_decode_check": (_I, [_c.POINTER(DecodeOp), _I]),
     "ill_decode_plan": (_I, [_c.POINTER(DecodeOp), _I, _P, _L, _c.POINTER(_c.c_int32), _S]),
     "ill_decode_run": (_I, [_P, _c.POINTER(_c.c_int32), _S]),
     "ill_chain_scratch_bytes": (_L, [_c.POINTER(DecodeOp), _I]),

@@ -509,11 +509,8 @@ extern "C" int64_t ill_decode_plan_bytes(int nops) {
   return 128 + (int64_t)nops * (int64_t)sizeof(DecOp);
 }
 
-extern "C" int ill_decode_plan(const ill_decode_op* ops, int nops, ill_dptr plan, int64_t plan_bytes, int32_t* launch,
-                               ill_stream stream) {
-  if (!ops || !launch || nops < 1 || nops > DEC_MAX_OPS || !plan) return ILL_ERR_ARG;
-  if (plan & 127) return ILL_ERR_ALIGN;
-  if (plan_bytes < ill_decode_plan_bytes(nops)) return ILL_ERR_TOO_LARGE;
+// The list as the kernel walks it (DEV_OPS 0: only whether it can be run) and the launch
+static int plan_list(const ill_decode_op* ops, int nops, DecOp* dev_ops, int32_t* launch) {
   int dev = 0, sms = 0, smem_max = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -540,14 +537,12 @@ extern "C" int ill_decode_plan(const ill_decode_op* ops, int nops, ill_dptr plan
   if ((int)fixed + DEC_WARPS * 8192 > budget) return ILL_ERR_TOO_LARGE;
   const int ring = (int)((((uint32_t)budget - fixed) / DEC_WARPS) & ~127u);
   const int limit = ring / 2 - 32;  // a tile's bytes at most: the next one fits beside it
-  std::vector<DecOp> dev_ops((size_t)nops);
   long long groups = 0;
   int meetings = 0;
   const long long gwarps = (long long)sms * DEC_WARPS;
   for (int i = 0; i < nops; ++i) {
     const ill_decode_op& o = ops[i];
-    DecOp& d = dev_ops[(size_t)i];
-    d = DecOp();
+    DecOp d = DecOp();
     const int bw = fmt_block_weights(o.fmt), bb = fmt_block_bytes(o.fmt), uw = (o.fmt == ILL_Q8_0 || o.fmt == ILL_IQ2_XXS) ? 32 : 64;
     const bool glu = o.kind == ILL_OP_GLU;
     d.w = (const u8*)(uintptr_t)o.w;
@@ -615,14 +610,8 @@ extern "C" int ill_decode_plan(const ill_decode_op* ops, int nops, ill_dptr plan
     d.restage = (!pv || d.after || pv->x != o.x || pv->norm_w != o.norm_w || pv->eps != o.eps || pv->cols != o.cols || pv->fmt != o.fmt ||
                  (o.fmt == ILL_Q8_0 && (pv->f16_scale != 0) != (o.f16_scale != 0)))
                     ? 1 : 0;
+    if (dev_ops) dev_ops[i] = d;
   }
-  unsigned char head[128] = {0};
-  cudaStream_t st = (cudaStream_t)stream;
-  e = cudaMemcpyAsync((void*)(uintptr_t)plan, head, sizeof head, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync((void*)(uintptr_t)(plan + 128), dev_ops.data(), (size_t)nops * sizeof(DecOp), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the host copy of the list is released on return
-  if (e != cudaSuccess) return cuda_fail(e);
   const uint32_t smem = fixed + (uint32_t)ring * DEC_WARPS;
   e = cudaFuncSetAttribute(decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e);
@@ -640,6 +629,32 @@ extern "C" int ill_decode_plan(const ill_decode_op* ops, int nops, ill_dptr plan
   launch[DL_MEETINGS] = meetings;
   launch[DL_EPOCH] = 0;   // arrivals at the barrier so far (the count in PLAN starts at 0 with it)
   launch[DL_MAGIC] = DL_MAGIC_VALUE;
+  return ILL_OK;
+}
+
+extern "C" int ill_decode_check(const ill_decode_op* ops, int nops) {
+  if (!ops || nops < 1 || nops > DEC_MAX_OPS) return ILL_ERR_ARG;
+  int32_t launch[DL_WORDS];
+  return plan_list(ops, nops, nullptr, launch);
+}
+
+extern "C" int ill_decode_plan(const ill_decode_op* ops, int nops, ill_dptr plan, int64_t plan_bytes, int32_t* launch,
+                               ill_stream stream) {
+  if (!ops || !launch || nops < 1 || nops > DEC_MAX_OPS || !plan) return ILL_ERR_ARG;
+  if (plan & 127) return ILL_ERR_ALIGN;
+  if (plan_bytes < ill_decode_plan_bytes(nops)) return ILL_ERR_TOO_LARGE;
+  std::vector<DecOp> dev_ops((size_t)nops);
+  int32_t words[DL_WORDS];  // (LAUNCH is written once all is well)
+  const int rc = plan_list(ops, nops, dev_ops.data(), words);
+  if (rc) return rc;
+  unsigned char head[128] = {0};
+  cudaStream_t st = (cudaStream_t)stream;
+  cudaError_t e = cudaMemcpyAsync((void*)(uintptr_t)plan, head, sizeof head, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync((void*)(uintptr_t)(plan + 128), dev_ops.data(), (size_t)nops * sizeof(DecOp), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the host copy of the list is released on return
+  if (e != cudaSuccess) return cuda_fail(e);
+  for (int i = 0; i < DL_WORDS; ++i) launch[i] = words[i];
   return ILL_OK;
 }
 

@@ -381,16 +381,15 @@ class DecodePlan:
     on its way, but not before a recording of the caller's that run() went into, nor before the buffers that OPS names."""
 
     def __init__(self, ops, device="cuda"):
-        import ctypes
         self.n = len(ops)
         arr = (_lib.DecodeOp * self.n)(*ops)
-        nbytes = _lib.lib().ill_decode_plan_bytes(self.n)
-        if nbytes <= 0:
+        if _lib.lib().ill_decode_plan_bytes(self.n) <= 0:
             raise ValueError("a chain holds 1 to 1024 products")
         with torch.cuda.device(device):
-            # (the one-launch form's plan: what it refuses is refused)
-            plan = torch.zeros(nbytes + 128, dtype=torch.uint8, device=device)
-            _lib.call("ill_decode_plan", arr, self.n, (plan.data_ptr() + 127) // 128 * 128, nbytes, (ctypes.c_int32 * 16)(), _stream())
+            # (what the one-launch form refuses is refused.  The code in an error is that of its entry point.)
+            rc = _lib.status("ill_decode_check", arr, self.n)
+            if rc:
+                _lib.fail("ill_decode_plan", rc)
             self.chain = _Chain(arr, self.n, device)
 
     def run(self):

@@ -19,7 +19,12 @@ def freed(monkeypatch):
         if name == "ill_chain_new":
             args[-1]._obj.value = 5
     monkeypatch.setattr(D._lib, "call", call)
-    monkeypatch.setattr(D._lib, "status", lambda name, *args: out.append((name, args[0].value)))
+
+    def status(name, *args):
+        if name == "ill_chain_free":
+            out.append((name, args[0].value))
+        return 0
+    monkeypatch.setattr(D._lib, "status", status)
     monkeypatch.setattr(D, "_stream", lambda: 0)
     monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
     return out

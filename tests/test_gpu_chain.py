@@ -116,6 +116,46 @@ def test_scratch_of_a_plan_that_runs_in_another_stream():
     assert all(torch.equal(a, b) for a, b in zip([m.h, *m.out], want))
 
 
+def test_a_plan_is_made_beside_what_runs():
+    """Without waiting for the stream, and with no memory but its scratch."""
+    m = Layer(B.Q4_K, B.Q6_K)
+    D.DecodePlan(m.ops)
+    torch.cuda.synchronize()
+    busy, before = torch.cuda.Event(), torch.cuda.memory_allocated()
+    torch.cuda._sleep(200_000_000)
+    busy.record()
+    plan = D.DecodePlan(m.ops)
+    assert not busy.query()
+    assert torch.cuda.memory_allocated() - before <= (plan.chain.scratch.numel() + 511) // 512 * 512
+    torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("change", ["", "cols 500", "cols 32768", "cols 33024", "rows 0", "w 8", "kind 7", "fmt 9", "w2 16", "x 4", "y 2", "1024", "many"])
+def test_the_check_refuses_what_the_one_launch_does(change):
+    w = _mat(B.Q4_K, 16, 512, 1)
+    op = D.decode_op(w, torch.zeros(512, device="cuda"), torch.zeros(16, device="cuda"))
+    ops = [op]
+    if change == "1024":
+        ops = [op] * 1024
+    elif change == "many":        # does not fit beside so many columns
+        ops = [op] * 900
+        op.cols = 32768
+    elif change:
+        k, v = change.split()
+        setattr(op, k, getattr(op, k) + int(v) if k in ("w", "x", "y") else int(v))
+    n = len(ops)
+    arr, nbytes, launch = (_lib.DecodeOp * n)(*ops), _lib.lib().ill_decode_plan_bytes(n), (ctypes.c_int32 * 16)()
+    buf = torch.zeros(nbytes + 128, dtype=torch.uint8, device="cuda")
+    rc = _lib.status("ill_decode_plan", arr, n, (buf.data_ptr() + 127) // 128 * 128, nbytes, launch, _lib.stream())
+    assert _lib.status("ill_decode_check", arr, n) == rc and (rc == 0) == (change in ("", "cols 32768", "1024")) and bool(launch[9]) == (rc == 0)
+    if rc:
+        with pytest.raises(_lib.IllatioError) as e:
+            D.DecodePlan(ops)
+        assert e.value.code == rc
+    with pytest.raises(ValueError):
+        D.DecodePlan([op] * 1025)
+
+
 def test_what_a_chain_refuses():
     m = Layer(B.Q4_K, B.Q6_K)
     n = len(m.ops)
