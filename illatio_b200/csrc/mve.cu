@@ -62,11 +62,11 @@ __device__ __forceinline__ void cp_async16_at(uint32_t dst, const void* src) {
 
 template <int N> struct MeN { static constexpr int value = N; };
 
-template <int FMT, bool TWO, bool AL4>
+template <int FMT, bool TWO>
 __global__ void __launch_bounds__(32 * ME_WARPS, 1) mve_kernel(const __grid_constant__ MeParams p) {
   extern __shared__ __align__(128) u8 smem[];
   constexpr int BB = Fmt<FMT>::BB, MATS = TWO ? 2 : 1;
-  constexpr bool SUMS = FMT == ILL_Q2_K;
+  constexpr bool SUMS = FMT == ILL_Q2_K, AL4 = FMT == ILL_Q2_K;  // (Q2_K: 84-byte blocks from a word on; IQ2_XXS: 66-byte ones, on two bytes)
   int* first = (int*)(smem + p.first_off);  // where each expert's tiles start on the line; its end
   __shared__ uint2 iq_grid[FMT == ILL_IQ2_XXS ? IQ_TABLE_BYTES / 8 : 1];  // (static: the look-ups' addresses start at a constant)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -340,6 +340,7 @@ static int moe_few(bool all, int fmt, int ncols, int nrows, int64_t add, int64_t
   if (!ptrs || !counts || !bases || !xq || !xs || !y || (fmt == ILL_Q2_K && !xsum)) return ILL_ERR_ARG;
   if ((ptrs & 7) || (counts & 3) || (bases & 3) || (xq & 15) || (xs & 3) || (xsum & 7) || (map & 3) || (weights & 3) || (y & 3) || (y2 & 3))
     return ILL_ERR_ALIGN;
+  if ((add | add2) & (fmt == ILL_Q2_K ? 3 : 1)) return ILL_ERR_ALIGN;
   const long long ntr = (nrows + ME_ROWS - 1) / ME_ROWS, experts = ne < total_rows ? ne : total_rows;  // with rows, at most
   if (ne > ME_MAX_NE || 3 * ntr * ne > ME_LINE || (all && total_rows > 8 * (ME_LINE / (3 * ntr) - ne))) return ILL_ERR_TOO_LARGE;
   if (total_rows == 0) return ILL_OK;
@@ -367,11 +368,9 @@ static int moe_few(bool all, int fmt, int ncols, int nrows, int64_t add, int64_t
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-  // (Q2_K's words: a block's 84 bytes keep the alignment that the matrix has, which is a multiple of four where ADD is one)
-  const bool two = weights || y2, al4 = ((add | add2) & 3) == 0;
-  const void* k = fmt == ILL_IQ2_XXS ? (two ? (const void*)mve_kernel<ILL_IQ2_XXS, true, false> : (const void*)mve_kernel<ILL_IQ2_XXS, false, false>)
-                  : al4 ? (two ? (const void*)mve_kernel<ILL_Q2_K, true, true> : (const void*)mve_kernel<ILL_Q2_K, false, true>)
-                        : (two ? (const void*)mve_kernel<ILL_Q2_K, true, false> : (const void*)mve_kernel<ILL_Q2_K, false, false>);
+  const bool two = weights || y2;
+  const void* k = fmt == ILL_IQ2_XXS ? (two ? (const void*)mve_kernel<ILL_IQ2_XXS, true> : (const void*)mve_kernel<ILL_IQ2_XXS, false>)
+                                     : (two ? (const void*)mve_kernel<ILL_Q2_K, true> : (const void*)mve_kernel<ILL_Q2_K, false>);
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e);
   void* args[] = {&p};

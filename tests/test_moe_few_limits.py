@@ -25,3 +25,17 @@ def test_each_product_leaves_the_other_what_it_does_not_take(monkeypatch, gate, 
     over = [(a[0], a[1], a[-2]) for name, a in seen if name == "ill_moe_mm_id_over"]
     assert few == over == [(gate, d, limits[0]), (B.Q2_K, ff, limits[1])]
     assert [a[-2] for name, a in seen if name == "ill_act_f16_over"] == [limits[0]]
+
+
+@pytest.mark.parametrize("fmt,step", [(B.Q2_K, 4), (B.IQ2_XXS, 2)])
+def test_a_matrix_off_its_boundary_is_refused(fmt, step):
+    """(A matrix on its boundary gets past the checks: no rows, no launch.)"""
+    P_ = 0x10000
+    who, x = (P_, P_, P_, 4, 0), (P_, P_, P_, P_)
+    for add, rc in ((0, 0), (step, 0), (step // 2, 2), (1, 2), (step + 1, 2)):
+        for form in ("ill_moe_few", "ill_moe_few_all"):
+            assert _lib.status(form, fmt, 512, 16, add, *who, *x, P_, 16, 0) == rc, (form, add)
+        for a, b in ((add, 0), (0, add)):
+            assert _lib.status("ill_moe_few2", fmt, 512, 16, a, b, *who, *x, P_, P_, 16, 0) == rc
+            for form in ("ill_moe_few_glu", "ill_moe_few_glu_all"):
+                assert _lib.status(form, fmt, 512, 16, a, b, *who, *x, 1.0, P_, P_, 16, 0) == rc
