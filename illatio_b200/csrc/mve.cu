@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(32 * ME_WARPS, 1) mve_kernel(const __grid_cons
   };
   const int pass_cost = ntr * me_cost(p.most);  // of a pass that is not an expert's last
   for (int e = tid; e < p.ne; e += nthreads) {
-    const int c = count(e), passes = max(c - 1, 0) / p.most;
+    const int c = count(e), passes = max(c - 1, 0) >> (p.most == 16 ? 4 : 3);
     first[e] = c ? passes * pass_cost + ntr * me_cost(c - passes * p.most) : 0;
   }
   __syncthreads();
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(32 * ME_WARPS, 1) mve_kernel(const __grid_cons
       if (first[m] <= lo) a = m; else b = m - 1;
     }
     s.e = a;
-    s.pass = (lo - first[a]) / pass_cost;
+    s.pass = p.all ? (lo - first[a]) / pass_cost : 0;
     fill(s);
     return true;
   };
