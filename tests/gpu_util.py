@@ -1,7 +1,10 @@
 """Helpers shared by the GPU parity tests."""
+import ctypes
+
 import numpy as np
 import torch
 
+from illatio_b200 import _lib
 from illatio_b200 import blocks as B
 from illatio_b200 import cuda_dense as D
 
@@ -46,3 +49,13 @@ def sum_terms(oracle, fmt, w, rows, cols, act_host, n=1):
     xf = np.abs(xq.astype(np.float64) * np.repeat(xs.astype(np.float64), per)).reshape(n, cols)
     wf = np.abs(oracle.dequant(fmt, w, rows, cols).astype(np.float64))
     return xf @ wf.T
+
+
+def one_launch(ops):
+    """A function that runs the chain OPS as the one cooperative launch (ill_decode_plan / ill_decode_run)."""
+    n = len(ops)
+    arr, nbytes, launch = (_lib.DecodeOp * n)(*ops), _lib.lib().ill_decode_plan_bytes(n), (ctypes.c_int32 * 16)()
+    buf = torch.zeros(nbytes + 128, dtype=torch.uint8, device="cuda")
+    base = (buf.data_ptr() + 127) // 128 * 128
+    _lib.call("ill_decode_plan", arr, n, base, nbytes, launch, _lib.stream())
+    return lambda: (_lib.call("ill_decode_run", base, launch, _lib.stream()), buf)

@@ -9,6 +9,8 @@ from illatio_b200 import _lib
 from illatio_b200 import blocks as B
 from illatio_b200 import cuda_dense as D
 
+from gpu_util import one_launch
+
 pytestmark = pytest.mark.gpu
 EPS = 1e-6
 
@@ -54,15 +56,6 @@ class Layer:
         run()
         torch.cuda.synchronize()
         return [t.clone() for t in [self.h, *self.out]]
-
-
-def one_launch(ops):
-    n = len(ops)
-    arr, nbytes, launch = (_lib.DecodeOp * n)(*ops), _lib.lib().ill_decode_plan_bytes(n), (ctypes.c_int32 * 16)()
-    buf = torch.zeros(nbytes + 128, dtype=torch.uint8, device="cuda")
-    base = (buf.data_ptr() + 127) // 128 * 128
-    _lib.call("ill_decode_plan", arr, n, base, nbytes, launch, _lib.stream())
-    return lambda: (_lib.call("ill_decode_run", base, launch, _lib.stream()), buf)
 
 
 @pytest.mark.parametrize("main,alt,big", [(B.Q4_K, B.Q6_K, 0), (B.Q8_0, B.Q8_0, 0), (B.IQ2_XXS, B.Q2_K, 0), (B.Q6_K, B.Q4_K, 0), (B.Q4_K, B.Q6_K, 36000)])

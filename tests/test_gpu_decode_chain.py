@@ -1,7 +1,7 @@
-"""A token's chain of products in one launch (ill_decode_plan / ill_decode_run) against the same chain issued
-product by product (ill_rmsnorm_q8, ill_quant_q8_k / ill_quant_q8_0, ill_mv, ill_mv_glu): the same bits, since a
-row's arithmetic and the quantizers are shared; and the per-product path is what the other tests hold against
-the CPU oracle.  One chain is also checked against the oracle directly.
+"""A token's chain of products, as recorded launches (DecodePlan) and in one launch (ill_decode_plan / ill_decode_run), against the same
+chain issued product by product (ill_rmsnorm_q8, ill_quant_q8_k / ill_quant_q8_0, ill_mv, ill_mv_glu): the same bits.  The recorded
+launches are those; the one launch is a kernel of its own that shares a row's arithmetic and the quantizers.  The per-product path is what
+the other tests hold against the CPU oracle; one chain is also checked against the oracle directly.
 """
 import numpy as np
 import pytest
@@ -9,10 +9,11 @@ import torch
 
 from illatio_b200 import blocks as B
 from illatio_b200 import cuda_dense as D
-from gpu_util import to_dev
+from gpu_util import one_launch, to_dev
 
 pytestmark = pytest.mark.gpu
 EPS = 1e-6
+FORMS = {"recorded": lambda ops: D.DecodePlan(ops).run, "one launch": one_launch}
 
 
 @pytest.fixture(autouse=True)
@@ -90,25 +91,27 @@ class Model:
     ((2560, 4096, 1024, 9728, 151936), 2, B.Q4_K, B.Q6_K),   # the 4B model's shapes and its whole head
     ((1024, 2048, 512, 2048, 2000), 2, B.IQ2_XXS, B.Q2_K),   # the 2-bit formats
 ])
-def test_chain_equals_per_product_path(dims, layers, fmt_main, fmt_alt):
+@pytest.mark.parametrize("form", FORMS)
+def test_chain_equals_per_product_path(form, dims, layers, fmt_main, fmt_alt):
     m = Model(*dims, layers, fmt_main, fmt_alt, seed=3)
     x0 = torch.randn(dims[0], device="cuda", generator=torch.Generator(device="cuda").manual_seed(9))
     m.h.copy_(x0)
     m.per_product()
     want = m.state()
-    plan = D.DecodePlan(m.ops())
-    for _ in range(2):   # the plan and its barrier serve any number of tokens
+    run = FORMS[form](m.ops())
+    for _ in range(2):   # the launches, and the plan with its barrier, serve any number of tokens
         for t in (m.q, m.k, m.v, m.fa, m.logits):
             t.fill_(-3.0)
         m.h.copy_(x0)
-        plan.run()
+        run()
         torch.cuda.synchronize()
         for name, a, b in zip("h q k v fa logits".split(), m.state(), want):
             assert torch.isfinite(a).all(), name
             assert torch.equal(a, b), "%s differs: %g" % (name, (a - b).abs().max().item())
 
 
-def test_chain_against_the_oracle(oracle):
+@pytest.mark.parametrize("form", FORMS)
+def test_chain_against_the_oracle(oracle, form):
     """rmsnorm -> gated Q4_K product -> Q6_K product added into h, each step against the CPU routines."""
     hidden, ffn = 768, 1280
     rng = np.random.default_rng(5)
@@ -119,9 +122,8 @@ def test_chain_against_the_oracle(oracle):
     h, fa = to_dev(h0), torch.empty(ffn, device="cuda")
     G, U, DN = (D.upload_gmat(m, f, r, c) for m, f, r, c in ((g, B.Q4_K, ffn, hidden), (u, B.Q4_K, ffn, hidden), (dn, B.Q6_K, hidden, ffn)))
     nwd = to_dev(nw)   # the plan keeps addresses only: every buffer it names must outlive it
-    plan = D.DecodePlan([D.decode_op(G, h, fa, w2=U, norm_w=nwd, eps=EPS, after=False),
-                         D.decode_op(DN, fa, h, acc=True, after=True)])
-    plan.run()
+    run = FORMS[form]([D.decode_op(G, h, fa, w2=U, norm_w=nwd, eps=EPS, after=False), D.decode_op(DN, fa, h, acc=True, after=True)])
+    run()
     torch.cuda.synchronize()
     act = oracle.quantize_q8k(oracle.rmsnorm(h0, nw, EPS))
     gv = oracle.matvec(B.Q4_K, g, ffn, hidden, act)[0].astype(np.float64)
@@ -135,16 +137,18 @@ def test_chain_against_the_oracle(oracle):
 
 def test_long_rows_are_taken_in_runs_of_columns():
     """Rows too long to fit a tile whole (and for ill_mv to keep in registers): 17408 columns, Q6_K and Q8_0.
-    The chain takes such a row in runs of columns and carries its sum; against ill_mv, whose order of additions
-    differs for such rows, to fp32 reassociation."""
+    The one launch takes such a row in runs of columns and carries its sum; against ill_mv, whose order of additions
+    differs for such rows, to fp32 reassociation.  The recorded launches are ill_mv."""
     for fmt in (B.Q6_K, B.Q8_0, B.Q4_K):
         w = _mat(fmt, 300, 17408, 1)
         x = torch.randn(17408, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
-        y, want = torch.zeros(300, device="cuda"), torch.zeros(300, device="cuda")
-        D.DecodePlan([D.decode_op(w, x, y, after=False)]).run()
+        y, z, want = (torch.zeros(300, device="cuda") for _ in range(3))
+        runs = [one_launch([D.decode_op(w, x, y, after=False)]), FORMS["recorded"]([D.decode_op(w, x, z, after=False)])]
+        for run in runs:
+            run()
         D.cmat_mul(w, D.quant_q8(x, D.make_qact(17408, D.matrix_act_kind(w))), want, 1)
         torch.cuda.synchronize()
-        assert ((y - want).abs().max() / want.abs().max()).item() < 1e-5
+        assert ((y - want).abs().max() / want.abs().max()).item() < 1e-5 and torch.equal(z, want)
 
 
 def test_plan_refuses_what_it_cannot_run():

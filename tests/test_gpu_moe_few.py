@@ -1,5 +1,6 @@
 """The experts' products for a few rows an expert (ill_moe_few, ill_moe_few2, ill_moe_few_glu): the bits of the chunk product, experts of
 more rows left to it (ill_moe_mm_id_over)."""
+import numpy as np
 import pytest
 import torch
 
@@ -177,8 +178,9 @@ def test_counts_past_the_rows_there_are_in_passes():
     cnt, bases = torch.tensor([40, 40, 41], **i32), torch.zeros(ne, **i32)
     y, one = torch.full((n + 16, rows), 5.0, device="cuda"), torch.empty(n, rows, device="cuda")
     _lib.call("ill_moe_few_all", fmt, cols, rows, 0, _p(ptrs), _p(cnt), _p(bases), ne, n, _p(act.xq), _p(act.xs), _p(act.xsum), 0, _p(y), rows, _lib.stream())
+    eight = torch.tensor([8], **i32)
     for t in range(0, n, 8):
-        _lib.call("ill_moe_few", fmt, cols, rows, 0, _p(ptrs), _p(torch.tensor([8], **i32)), _p(bases), 1, 8, _p(act.xq) + t * cols, _p(act.xs) + 4 * t * (cols // 256),
+        _lib.call("ill_moe_few", fmt, cols, rows, 0, _p(ptrs), _p(eight), _p(bases), 1, 8, _p(act.xq) + t * cols, _p(act.xs) + 4 * t * (cols // 256),
                   _p(act.xsum) + 2 * t * (cols // 16), 0, _p(one) + 4 * t * rows, rows, _lib.stream())
     assert torch.equal(y[:n], one) and (y[n:] == 5.0).all()
 
@@ -198,3 +200,35 @@ def test_chunk_driver_with_limits_that_differ():
     for t in (sc.down, sc.g, sc.u, sc.moe):
         t.fill_(1e30)
     assert torch.equal(P.dk_ffn_routed_chunk(pool, norms, logits, nu, 10.0, sc), want)
+
+
+def test_block_sums_past_24_bits(oracle):
+    """IQ2_XXS's block sums reach 2.6 times 2^24: whole numbers of 32 bits here, each sum rounded once (three roundings a block: the sum, the
+    product of the scales, theirs), where the chunk product adds in fp32.  One block a row of the largest scale and codebook entry."""
+    fmt, rows, cols, n = B.IQ2_XXS, 32, 256, 5
+    rng = np.random.default_rng(1)
+    base = B.synth_matrix(fmt, 256, cols, seed=1).reshape(256, 66).copy()
+    base[:, :2] = np.frombuffer(np.float16(1.0).tobytes(), np.uint8)
+    base[:, 2:].reshape(256, 8, 8)[:, :, 4:] = np.frombuffer(np.uint32(0xf0000000).tobytes(), np.uint8)  # no signs, the scale 31
+    base[:, 2:].reshape(256, 8, 8)[:, :, :4] = np.arange(256, dtype=np.uint8)[:, None, None]
+    sums = oracle.dequant(fmt, base.reshape(-1), 256, cols).astype(np.float64).sum(1)
+    block = base[sums.argmax()].copy()
+    w = np.repeat(block[None], rows, 0)
+    w[:, 2:].reshape(rows, 8, 8)[:, :, 4] ^= rng.integers(0, 4, (rows, 8), dtype=np.uint8)  # some signs
+    wf = oracle.dequant(fmt, w.reshape(-1), rows, cols).astype(np.float64)
+    act = D.quant_q8(torch.full((n * cols,), 0.7, device="cuda") * (1 + torch.rand(n * cols, device="cuda") / 64), D.make_qact(n * cols, "q8k"))
+    q, d = act.xq.cpu().numpy().astype(np.float64).reshape(n, cols), act.xs.cpu().numpy().astype(np.float64)
+    want = (q @ wf.T) * d[:, None]
+    assert np.abs(q @ wf.T).max() * 8 > 2 ** 24
+    i32 = dict(dtype=torch.int32, device="cuda")
+    dw = torch.as_tensor(w.reshape(-1)).cuda()
+    ptrs, cnt, bases = torch.tensor([_p(dw)], dtype=torch.int64, device="cuda"), torch.tensor([n], **i32), torch.tensor([0], **i32)
+    who = (_p(ptrs), _p(cnt), _p(bases), 1, n)
+    y, chunk = torch.empty(n, rows, device="cuda"), torch.empty(n, rows, device="cuda")
+    xh = torch.empty(n, cols, dtype=torch.float16, device="cuda")
+    _lib.call("ill_moe_few", fmt, cols, rows, 0, *who, _p(act.xq), _p(act.xs), _p(act.xsum), 0, _p(y), rows, _lib.stream())
+    _lib.call("ill_act_f16", n, cols, _p(act.xq), _p(act.xsum), 0, _p(xh), 0, _lib.stream())
+    _lib.call("ill_moe_mm_id", fmt, cols, rows, 0, *who, _p(xh), 0, _p(act.xs), 0, 0, _p(chunk), rows, _lib.stream())
+    err, err_chunk = (np.abs(t.cpu().numpy() - want).max() / np.abs(want).max() for t in (y, chunk))
+    assert err <= 3 * 2.0 ** -24, err
+    assert err <= err_chunk <= (3 + 16 * 2) * 2.0 ** -24, err_chunk  # sixteen additions of 16 columns, each off by up to 2 past 2^24
