@@ -310,8 +310,31 @@ def chain_per_product(D, m, acts):
     return n + 2
 
 
+def one_launch_of(ops, torch, dev):
+    """A function that runs the chain OPS as the one cooperative launch (ill_decode_plan / ill_decode_run)."""
+    import ctypes
+    from illatio_b200 import _lib
+    n = len(ops)
+    arr, nbytes, launch = (_lib.DecodeOp * n)(*ops), _lib.lib().ill_decode_plan_bytes(n), (ctypes.c_int32 * 16)()
+    buf = torch.zeros(nbytes + 128, dtype=torch.uint8, device=dev)
+    base = (buf.data_ptr() + 127) // 128 * 128
+    _lib.call("ill_decode_plan", arr, n, base, nbytes, launch, _lib.stream())
+    return lambda: (_lib.call("ill_decode_run", base, launch, _lib.stream()), buf)
+
+
+def graph_launches(fn, torch):
+    """How many launches FN puts into a CUDA graph."""
+    import ctypes
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        fn()
+    n = ctypes.c_size_t(0)
+    rc = ctypes.CDLL("libcudart.so.12").cudaGraphGetNodes(ctypes.c_void_p(g.raw_cuda_graph()), None, ctypes.byref(n))
+    return n.value if rc == 0 else None
+
+
 def chain_leg(D, B, torch, dev, dims, layers, fmt_main, fmt_alt, seed, peak, name):
-    """A token's chain both ways, timed; and that the two give the same logits."""
+    """A token's chain three ways, timed; and that they give the same logits."""
     m = build_chain_model(D, B, torch, dev, dims, layers, fmt_main, fmt_alt, seed)
     hidden, qdim, kvdim, ffn, vocab = dims
     acts = {(k, kind): D.make_qact(n, kind, device=dev) for k, n in (("h", hidden), ("q", qdim), ("fa", ffn)) for kind in ("q8", "q8k")}
@@ -322,26 +345,37 @@ def chain_leg(D, B, torch, dev, dims, layers, fmt_main, fmt_alt, seed, peak, nam
         launches[0] = chain_per_product(D, m, acts) + 1
     plan = D.DecodePlan(chain_ops(D, m), device=dev)
 
-    def one_launch():
+    coop = one_launch_of(chain_ops(D, m), torch, dev)
+
+    def recorded():
         m["h"].copy_(m["x0"])
         plan.run()
+
+    def one_launch():
+        m["h"].copy_(m["x0"])
+        coop()
     per_product()
     torch.cuda.synchronize()
     want = m["logits"].clone()
-    m["logits"].zero_()
-    one_launch()
-    torch.cuda.synchronize()
-    same = bool(torch.equal(m["logits"], want)) and bool(torch.isfinite(want).all())
+
+    def same(fn):
+        m["logits"].zero_()
+        fn()
+        torch.cuda.synchronize()
+        return bool(torch.equal(m["logits"], want)) and bool(torch.isfinite(want).all())
+    parity = {"recorded_launches_equal_per_product_bits": same(recorded), "one_launch_equals_per_product_bits": same(one_launch)}
     g = graph_of(per_product, torch)
-    us_pp = time_us(g.replay, 10, torch)
-    us_one = time_us(one_launch, 10, torch)
+
+    def timed(fn, **kw):
+        us = time_us(fn, 10, torch)
+        return {"us_per_token": us, "GBps": m["bytes"] / us / 1e3, "frac_of_hbm": m["bytes"] / us / 1e3 / peak, **kw}
     out = {"workload": name, "weight_MB": m["bytes"] / 1e6,
-           "per_product": {"us_per_token": us_pp, "GBps": m["bytes"] / us_pp / 1e3, "frac_of_hbm": m["bytes"] / us_pp / 1e3 / peak,
-                           "launches": launches[0], "how": "one CUDA graph of the token's launches"},
-           "one_launch": {"us_per_token": us_one, "GBps": m["bytes"] / us_one / 1e3, "frac_of_hbm": m["bytes"] / us_one / 1e3 / peak,
-                          "launches": 1, "products": plan.n, "how": "ill_chain_run: the token's launches recorded once as a CUDA graph, one host call"},
-           "parity": {"one_launch_equals_per_product_bits": same}}
-    del m, plan, g
+           "per_product": timed(g.replay, launches=launches[0], how="one CUDA graph of the token's launches"),
+           "recorded_launches": timed(recorded, launches=graph_launches(plan.run, torch), products=plan.n,
+                                      how="ill_chain_run: the token's launches recorded once as a CUDA graph, one host call"),
+           "one_launch": timed(one_launch, launches=1, products=plan.n, how="ill_decode_run: one cooperative launch"),
+           "parity": parity}
+    del m, plan, coop, g
     torch.cuda.empty_cache()
     return out
 
