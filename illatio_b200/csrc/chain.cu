@@ -5,7 +5,9 @@
 // before it ends (programmatic dependent launch, which a graph keeps), take three to four: us a token, that kernel / this: 36 layers
 // of a 4B model (Q4_K, Q6_K) and its head 2360 / 1515, 24 of a 0.5B one (Q8_0) 1120 / 463, one layer and the head 101 / 55.
 // The products and quantizers are the stand-alone ones (ill_mv, ill_mv_3, ill_mv_glu, ill_quant_q8_*, ill_rmsnorm_q8), so the results are
-// theirs and the chain kernel's, bit for bit.
+// theirs, bit for bit, and the chain kernel's where that takes a row whole (decode.cu).
+// In a recording of the caller's, products of two formats go one behind the other: the fork (issue's SIDE) needs a stream and events that
+// would be that recording's.
 //
 // Replaces the launches of CUDA-FORWARD-N (src/cuda-dense.lisp:380-432).
 #include <new>

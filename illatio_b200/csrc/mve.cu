@@ -4,7 +4,7 @@
 // A persistent CTA of sixteen warps an SM.  The experts' tiles of 16 weight rows (or of gate's and up's) lie one after another on a line,
 // a tile as long as it takes (me_cost), and every CTA has an even share of the line.  It stages an expert's activations, read where the
 // tokens' quants lie, and its warps take that expert's tiles, all blocks of a row in order: the chunk kernel's order (mm_id.cu), and
-// its bits.  Weights: 16-byte cp.async into a ring a warp, four lanes a row segment, on across tiles and experts.
+// its bits while a block's sum stays under 2^24 (IQ2_XXS's can reach 2.6 times that: int32 holds it, the chunk kernel's fp32 rounds).  Weights: 16-byte cp.async into a ring a warp, four lanes a row segment, on across tiles and experts.
 //
 // Why not the chunk kernel: its block of 128 weight rows goes through raw bytes, fp16 operands in tensor memory, a product and a drain, a
 // chain of about 1700 cycles whatever the rows of X; here a block of 128 x 256 weights takes 970 (Q2_K) and 1370 (IQ2_XXS) cycles an SM

@@ -294,11 +294,10 @@ def tc_takes(w, n):
             and w.qs.data_ptr() % 16 == 0)
 
 
-# Matrices of fewer rows (K and V, mostly) go to the int8 mma.sync kernel, which is slower there (us, tcgen05 / int8, 512 tokens:
-# 1024 x 2560 of Q4_K 14.0 / 21.6, 1024 x 5120 of Q6_K 37.5 / 45.1) but holds a block's sum in int32: in fp32, exact to 2^24, blocks
+# Matrices of fewer rows that are not K and V beside a larger Q (those: _exact_takes) go to the int8 mma.sync kernel, which is slower there
+# (us, tcgen05 / int8, 512 tokens: 1024 x 2560 of Q4_K 14.0 / 21.6, 1024 x 5120 of Q6_K 37.5 / 45.1) but holds a block's sum in int32: in fp32, exact to 2^24, blocks
 # of near-constant weights and activations lose bits (relative error against 64 bits, tcgen05 / int8: Q6_K 4.9e-7 / 4.3e-8, Q4_K
-# 9.5e-8 / 4.5e-8; ordinary blocks 3.6e-8 both).  It also reads the quants themselves, in any stream and with Y at any float.  (K and V beside a
-# larger Q: _exact_takes.)
+# 9.5e-8 / 4.5e-8; ordinary blocks 3.6e-8 both).  It also reads the quants themselves, in any stream and with Y at any float.
 # Fewer tokens go there for the same reasons, not for speed: 17 / 63 tokens of 4096 x 2560 of Q4_K 13.2 / 13.6 us on tcgen05 and 19.0 /
 # 21.7, of 5120 x 5120 of Q6_K 36.4 / 38.0 and 38.7 / 45.0, and 2 us for the activations' fp16 form once.
 TC_MIN_TOKENS, TC_MIN_ROWS = 64, 2048

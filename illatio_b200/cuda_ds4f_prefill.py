@@ -102,7 +102,8 @@ def few_rows(pool, n, nu):
 
 def _few_rows_chunk(pool, n, nu, clamp, sc, shared, most, st):
     """The chunk's experts that have a few rows by the products for those, up to each product's limit (of which MOST is the smaller),
-    the others by the chunk's: the same bits either way.  Up to MOST tokens have none of the others unless the router gives a token one expert again (scores that are all NaN or
+    the others by the chunk's: the same bits either way but for IQ2_XXS blocks whose whole-number sum passes 2^24, which the former
+    holds exactly.  Up to MOST tokens have none of the others unless the router gives a token one expert again (scores that are all NaN or
     -inf: expert 0 for every slot that is left), so they go to the former alone, which then takes that expert in passes."""
     d, ff, ne = pool.d, pool.ff, pool.n_expert
     who = (_ptr(pool.ptrs_all), _ptr(sc.counts), _ptr(sc.bases), ne, sc.rows)
@@ -164,9 +165,10 @@ def dk_ffn_small(pool, norms, logits, nu, clamp, sc, **kw):
     """DK-FFN-SMALL (src/cuda-ds4f-spec.lisp:31-132): the routed experts for a few tokens at once -- several decode
     sequences, or the positions of a speculative run -- with the rows grouped by expert so that an expert's weights
     are read once for all of its tokens.  The reference multiplies with its matvec kernels given COUNTS / BASES
-    (src/cuda/ds4f.cu:769-772); here the grouping and the products are the chunk driver's: the tcgen05 kernel takes
-    tiles of as few as 16 rows, and for the 2-bit expert formats it is the faster of the two forms (their matvecs
-    are bound by instructions, not by the bytes they read).  Same arguments and result as dk_ffn_routed_chunk."""
+    (src/cuda/ds4f.cu:769-772); here the grouping and the products are the chunk driver's, which for the 2-bit expert
+    formats has a kernel for the experts of a few rows (few_rows): an expert's weights are unpacked once for up to
+    sixteen of them, where a matvec, bound by instructions and not by the bytes it reads, unpacks them for each.
+    Same arguments and result as dk_ffn_routed_chunk."""
     return dk_ffn_routed_chunk(pool, norms, logits, nu, clamp, sc, **kw)
 
 
