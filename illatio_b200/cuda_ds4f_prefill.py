@@ -82,8 +82,8 @@ def mm_id(pool, fmt, ncols, nrows, add, sc, xh, xe, xd, rmap, y):
 # 1420 / 1061, 2048 (57) 2591 / 2172, 8192 (228) 5873 / 5915.  Logits with an expert's own normal deviate added, times 0, 0.5, 1 and 2: 256
 # experts of IQ2_XXS, 512 tokens (12) 1684 / 1260, 1594 / 1170, 1142 / 879, 674 / 591; 1024 (24) 1746 / 1795, 1793 / 1531, 1510 / 1233, 982 / 874;
 # 2048 (48) 1928 / 1912, 2152 / 1928, 1969 / 1722, 1402 / 1342; 160 of Q2_K, 512 (26) 874 / 913, 1011 / 897, 945 / 727, 589 / 539.  It loses where
-# hardly an expert has few rows: 3 to 4 % at a mean of 24 to 26 that all experts share alike (a warp's tile of the few takes 15 us
-# however few they are), and the 5 to 9 us of launches that find nothing to do where all tokens choose the same experts (64 tokens of six 111 / 116).
+# hardly an expert has few rows: 3 to 4 % at a mean of 24 to 26 that all experts share alike (a warp's tile of gate and up of 5120 columns
+# takes 23 us however few experts there are, of down of 1536 columns 7), and the 5 to 9 us of launches that find nothing to do where all tokens choose the same experts (64 tokens of six 111 / 116).
 FEW_MEAN = 64
 
 
