@@ -348,7 +348,8 @@ class _Chain:
 
     def __init__(self, arr, n, device):
         import ctypes
-        self.handle, self.stream = ctypes.c_uint64(0), _stream()
+        self.handle = ctypes.c_uint64(0)  # (first: __del__ looks at it whatever fails)
+        self.stream = _stream()
         nbytes = _lib.lib().ill_chain_scratch_bytes(arr, n)
         self.scratch = torch.empty(nbytes + 128, dtype=torch.uint8, device=device)
         _lib.call("ill_chain_new", arr, n, (self.scratch.data_ptr() + 127) // 128 * 128, nbytes, ctypes.byref(self.handle))
